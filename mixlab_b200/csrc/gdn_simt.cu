@@ -16,18 +16,25 @@
 //
 // Kernels:
 //   gdn_prep_kernel        one CTA per (chunk, b*H+h): gam, T, w, u, P -> workspace
-//   gdn_state_fwd_kernel   one CTA per (32-column slab of Dv, b*H+h), sequential over
+//   gdn_state_fwd_kernel   one CTA per (16-column slab of Dv, b*H+h), sequential over
 //                          chunks: v_new, out, state (columns of Dv are independent)
 //   gdn_state_bwd_kernel   same mapping, reverse over chunks: dv_new, dS
 //   gdn_chunk_bwd_kernel   one CTA per chunk: dq, dk, dv, dbeta, dgate
 //   gdn_recurrent_fwd_kernel  token-by-token recurrence (chunk <= 1,
 //                          gated_delta_scan_naive, gpu/ir.cpp:2314-2350)
+//
+// All products are register-tiled over shared-memory tiles of 64 rows (a chunk, zero-padded) and issue packed
+// two-wide FMAs: a chain of fp32 sums either way, with half the issue slots, which the shared-memory loads need.
+#include <initializer_list>
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace mxb {
 
 struct GdnP {
   int B, T, H, K, V, C, n, gate_is_log, save;
+  int vecK, vecV;  // rows of Dk / Dv elements can be read and written four elements at a time
   const void *q, *k, *v;
   const float *beta, *gate, *h0;
   void* out;
@@ -37,8 +44,9 @@ struct GdnP {
   void *dq, *dk, *dv;
   float *dbeta, *dgate, *dh0;
   // workspace, all fp32, indexed by ci = (b*H+h)*n + chunk
+  int* status;  // 256-byte header, always zero on this path
   float *gam;   // [C]
-  float *Tm;    // [C,C]
+  float *Tm;    // [C,C]  (written when the forward saves for the backward)
   float *w;     // [C,K]
   float *u;     // [C,V]
   float *P;     // [C,C]
@@ -46,538 +54,1127 @@ struct GdnP {
   float *vn;    // [C,V]
   float *dhs;   // [V,K]  dS at chunk end, transposed
   float *dvn;   // [C,V]
-  float *dqi, *dw, *dkt;  // [C,K]
+  float *e;     // [C,V]  T^T dv_new
+  float *z;     // [C,K]  T^T dw
 };
-
-// out(i,j, sum_{kk in [lo(i,j), hi(i,j))} a(i,kk) b(kk,j)); consecutive threads walk j.
-template <typename FA, typename FB, typename FL, typename FH, typename FO>
-__device__ __forceinline__ void cta_gemm_r(int M, int N, FA a, FB b, FL lo, FH hi, FO out) {
-  for (int idx = threadIdx.x; idx < M * N; idx += blockDim.x) {
-    const int i = idx / N, j = idx - i * N;
-    float acc = 0.f;
-    const int h = hi(i, j);
-    for (int kk = lo(i, j); kk < h; ++kk) acc = fmaf(a(i, kk), b(kk, j), acc);
-    out(i, j, acc);
-  }
-}
-template <typename FA, typename FB, typename FO>
-__device__ __forceinline__ void cta_gemm(int M, int N, int Kd, FA a, FB b, FO out) {
-  cta_gemm_r(M, N, a, b, [](int, int) { return 0; }, [Kd](int, int) { return Kd; }, out);
-}
-// Row-mapped variant: warp w owns rows w, w+nw, ...; lanes walk j.  elem(i,j,acc)
-// returns a value that is summed over the row and handed to row(i,sum) by lane 0.
-template <typename FA, typename FB, typename FL, typename FH, typename FE, typename FR>
-__device__ __forceinline__ void cta_gemm_rows(int M, int N, FA a, FB b, FL lo, FH hi, FE elem, FR row) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int i = warp; i < M; i += nw) {
-    float part = 0.f;
-    for (int j = lane; j < N; j += 32) {
-      float acc = 0.f;
-      const int h = hi(i, j);
-      for (int kk = lo(i, j); kk < h; ++kk) acc = fmaf(a(i, kk), b(kk, j), acc);
-      part += elem(i, j, acc);
-    }
-    part = warp_sum(part);
-    if (lane == 0) row(i, part);
-  }
-}
 
 __device__ __forceinline__ float log_gate(float g, int gate_is_log) {
   return gate_is_log ? fmaxf(g, kLogGateFloor) : logf(fmaxf(g, kGateFloor));
 }
 
-// ------------------------------------------------------------------ prep
+// ---------------------------------------------------------- tiles and products
+namespace simt {
+constexpr int R = 64;    // tile rows: a chunk, zero-padded
+constexpr int LD = 68;   // pitch of [64][64] matrices: rows 16 bytes apart modulo 128, so that eight rows read at the
+                         // same column fall into different banks
+constexpr int KB = 32;   // contraction elements staged per step
+constexpr int LB = KB + 4;
+
+using f2 = unsigned long long;  // two packed floats
+__device__ __forceinline__ f2 pack2(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void fma2(f2& d, f2 a, f2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float sum2(f2 v) {
+  const float2 t = unpack2(v);
+  return t.x + t.y;
+}
+__device__ __forceinline__ ulonglong2 lds2x2(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+
+// Four consecutive elements col .. col+3 of a row of n (zeros past the end).
 template <typename IO>
-__global__ void __launch_bounds__(256) gdn_prep_kernel(GdnP p) {
-  extern __shared__ float smem[];
-  const int C = p.C, K = p.K, V = p.V, ldk = K + 1, ldc = C + 1;
-  float* ks = smem;            // [C][ldk]
-  float* Am = ks + C * ldk;    // [C][ldc]
-  float* Tm = Am + C * ldc;    // [C][ldc]
-  float* gam = Tm + C * ldc;   // [C]
-  float* bet = gam + C;        // [C]
-  float* bd = bet + C;         // [C] beta * E(gam)
-  const int tid = threadIdx.x, c = blockIdx.x, bh = blockIdx.y;
-  const int b = bh / p.H, h = bh % p.H, t0 = c * C;
+__device__ __forceinline__ float4 ld4(const IO* row, int col, int n, bool vec);
+template <>
+__device__ __forceinline__ float4 ld4<float>(const float* row, int col, int n, bool vec) {
+  if (col >= n) return make_float4(0.f, 0.f, 0.f, 0.f);
+  if (vec) return *reinterpret_cast<const float4*>(row + col);
+  return make_float4(row[col], col + 1 < n ? row[col + 1] : 0.f, col + 2 < n ? row[col + 2] : 0.f, col + 3 < n ? row[col + 3] : 0.f);
+}
+template <>
+__device__ __forceinline__ float4 ld4<__nv_bfloat16>(const __nv_bfloat16* row, int col, int n, bool vec) {
+  if (col >= n) return make_float4(0.f, 0.f, 0.f, 0.f);
+  if (vec) {
+    const uint2 w = *reinterpret_cast<const uint2*>(row + col);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+  return make_float4(to_f32(row[col]), col + 1 < n ? to_f32(row[col + 1]) : 0.f, col + 2 < n ? to_f32(row[col + 2]) : 0.f,
+                     col + 3 < n ? to_f32(row[col + 3]) : 0.f);
+}
+template <typename IO>
+__device__ __forceinline__ void st4(IO* row, int col, int n, bool vec, float4 x) {
+  if (col >= n) return;
+  if (vec) {
+    if constexpr (sizeof(IO) == 4) {
+      *reinterpret_cast<float4*>(row + col) = x;
+    } else {
+      __nv_bfloat162 a = __floats2bfloat162_rn(x.x, x.y), b = __floats2bfloat162_rn(x.z, x.w);
+      *reinterpret_cast<uint2*>(row + col) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+    }
+    return;
+  }
+  row[col] = from_f32<IO>(x.x);
+  if (col + 1 < n) row[col + 1] = from_f32<IO>(x.y);
+  if (col + 2 < n) row[col + 2] = from_f32<IO>(x.z);
+  if (col + 3 < n) row[col + 3] = from_f32<IO>(x.w);
+}
+__device__ __forceinline__ float4 scale4(float4 x, float s) { return make_float4(x.x * s, x.y * s, x.z * s, x.w * s); }
+__device__ __forceinline__ float dot4(float4 a, float4 b, float s) {
+  return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
+}
+
+__device__ __forceinline__ void cp_async16(float* dst, const void* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async4(float* dst, const void* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 4 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Rows 0 .. 63 of n elements -> shared tile with the given pitch; rows past `rows` become zero.  float32 rows travel
+// asynchronously (the caller commits and waits), bf16 rows are widened on the way.  256 threads.
+template <typename IO, typename F>
+__device__ __forceinline__ void stage_rows(float* dst, int pitch, int rows, int n, bool vec, const IO* any, F rowptr) {
+  if constexpr (sizeof(IO) == 4) {
+    if (vec) {
+      const int n4 = n >> 2;
+      for (int u = threadIdx.x; u < R * 32; u += 256) {  // 32 units of four cover the widest row (128)
+        const int i = u >> 5, c4 = u & 31;
+        if (c4 < n4) cp_async16(dst + i * pitch + 4 * c4, i < rows ? rowptr(i) + 4 * c4 : any, i < rows);
+      }
+    } else {
+      for (int u = threadIdx.x; u < R * 128; u += 256) {
+        const int i = u >> 7, c = u & 127;
+        if (c < n) cp_async4(dst + i * pitch + c, i < rows ? rowptr(i) + c : any, i < rows);
+      }
+    }
+  } else {
+    for (int u = threadIdx.x; u < R * 32; u += 256) {
+      const int i = u >> 5, c = 4 * (u & 31);
+      if (c < n) *reinterpret_cast<float4*>(dst + i * pitch + c) = i < rows ? ld4(rowptr(i), c, n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+}
+
+// acc[r][c] += sum_k A[ty + 16 r][k] B[tx + 16 c][k]: both operands contiguous along the contraction, the two halves
+// of an accumulator take its even and odd elements.
+__device__ __forceinline__ void tile_nt(f2 (&acc)[4][4], const float* A, int lda, const float* B, int ldb, int kd) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll 4
+  for (int k = 0; k < kd; k += 4) {
+    ulonglong2 a[4], b[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) a[r] = lds2x2(A + (ty + 16 * r) * lda + k);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) b[c] = lds2x2(B + (tx + 16 * c) * ldb + k);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        fma2(acc[r][c], a[r].x, b[c].x);
+        fma2(acc[r][c], a[r].y, b[c].y);
+      }
+  }
+}
+// acc[r][2 g + s] += sum_k A[4 ty + r][k] B[k][64 g + 4 tx + 2 s, +1].  AT: A is stored transposed, [k][i].
+template <int NG, bool AT>
+__device__ __forceinline__ void tile_nn(f2 (&acc)[4][2 * NG], const float* A, int lda, const float* B, int ldb, int kd) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll 2
+  for (int k = 0; k < kd; k += 4) {
+    float a[4][4];  // [row][k]
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float4 t = AT ? *reinterpret_cast<const float4*>(A + (k + r) * lda + 4 * ty)
+                          : *reinterpret_cast<const float4*>(A + (4 * ty + r) * lda + k);
+      if (AT) { a[0][r] = t.x; a[1][r] = t.y; a[2][r] = t.z; a[3][r] = t.w; }
+      else { a[r][0] = t.x; a[r][1] = t.y; a[r][2] = t.z; a[r][3] = t.w; }
+    }
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      ulonglong2 b[NG];
+#pragma unroll
+      for (int g = 0; g < NG; ++g) b[g] = lds2x2(B + (k + kk) * ldb + 64 * g + 4 * tx);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const f2 aa = pack2(a[r][kk], a[r][kk]);
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+          fma2(acc[r][2 * g], aa, b[g].x);
+          fma2(acc[r][2 * g + 1], aa, b[g].y);
+        }
+      }
+    }
+  }
+}
+template <int N>
+__device__ __forceinline__ void clear(f2 (&acc)[4][N]) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < N; ++c) acc[r][c] = 0ull;
+}
+template <int NG>
+__device__ __forceinline__ float4 acc4(const f2 (&acc)[4][2 * NG], int r, int g) {
+  const float2 a = unpack2(acc[r][2 * g]), b = unpack2(acc[r][2 * g + 1]);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+// Sum over the 16 threads that share the rows of a tile.
+__device__ __forceinline__ float row_sum(float v) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Streaming buffers of the products whose operands come from global memory: two stages of KB contraction elements,
+// the next stage's elements in registers while the current one is multiplied.
+constexpr int kStageA = R * LB;      // [64][LB]
+constexpr int kStageB = KB * 128;    // [KB][128], or [64][LB] for the products along rows
+constexpr int kStageFloats = 2 * (kStageA + kStageB);
+static_assert(kStageB >= R * LB, "row blocks fit the stage of the wide operand");
+
+// acc += A B^T over kd elements; la(i, k), lb(j, k) give elements k .. k+3 of row i of A, row j of B.
+template <typename FA, typename FB>
+__device__ __forceinline__ void stream_nt(f2 (&acc)[4][4], float* stage, int kd, FA la, FB lb) {
+  float4 ra[2], rb[2];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int u = threadIdx.x + 256 * m, i = u >> 3, c = 4 * (u & 7);
+      ra[m] = la(i, k0 + c);
+      rb[m] = lb(i, k0 + c);
+    }
+  };
+  auto put = [&](int buf) {
+    float* sA = stage + buf * kStageA;
+    float* sB = stage + 2 * kStageA + buf * kStageB;
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int u = threadIdx.x + 256 * m, i = u >> 3, c = 4 * (u & 7);
+      *reinterpret_cast<float4*>(sA + i * LB + c) = ra[m];
+      *reinterpret_cast<float4*>(sB + i * LB + c) = rb[m];
+    }
+  };
+  fetch(0);
+  __syncthreads();  // whoever used the stages before is done
+  put(0);
+  __syncthreads();
+  int buf = 0;
+  for (int k0 = 0; k0 < kd; k0 += KB, buf ^= 1) {
+    const bool more = k0 + KB < kd;
+    if (more) fetch(k0 + KB);
+    tile_nt(acc, stage + buf * kStageA, LB, stage + 2 * kStageA + buf * kStageB, LB, KB);
+    if (more) put(buf ^ 1);
+    __syncthreads();
+  }
+}
+// acc += A B over kd elements, B streamed: lb(k, j) gives elements j .. j+3 of row k.  A streamed (AM = 0, la(i, k)),
+// or a [64][64] matrix in shared memory as it is (AM = 1) or transposed (AM = 2), pitch LD.
+template <int NG, int AM, typename FA, typename FB>
+__device__ __forceinline__ void stream_nn(f2 (&acc)[4][2 * NG], float* stage, int kd, const float* As, FA la, FB lb) {
+  constexpr int NB = 2 * NG;  // units of four per thread in a KB x 64 NG block
+  float4 ra[2], rb[NB];
+  auto fetch = [&](int k0) {
+    if (AM == 0) {
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int u = threadIdx.x + 256 * m;
+        ra[m] = la(u >> 3, k0 + 4 * (u & 7));
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < NB; ++m) {
+      const int u = threadIdx.x + 256 * m;
+      rb[m] = lb(k0 + u / (16 * NG), 4 * (u % (16 * NG)));
+    }
+  };
+  auto put = [&](int buf) {
+    if (AM == 0) {
+      float* sA = stage + buf * kStageA;
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int u = threadIdx.x + 256 * m;
+        *reinterpret_cast<float4*>(sA + (u >> 3) * LB + 4 * (u & 7)) = ra[m];
+      }
+    }
+    float* sB = stage + 2 * kStageA + buf * kStageB;
+#pragma unroll
+    for (int m = 0; m < NB; ++m) *reinterpret_cast<float4*>(sB + 4 * (threadIdx.x + 256 * m)) = rb[m];
+  };
+  fetch(0);
+  __syncthreads();
+  put(0);
+  __syncthreads();
+  int buf = 0;
+  for (int k0 = 0; k0 < kd; k0 += KB, buf ^= 1) {
+    const bool more = k0 + KB < kd;
+    if (more) fetch(k0 + KB);
+    const float* sB = stage + 2 * kStageA + buf * kStageB;
+    if (AM == 0) tile_nn<NG, false>(acc, stage + buf * kStageA, LB, sB, 64 * NG, KB);
+    else if (AM == 1) tile_nn<NG, false>(acc, As + k0, LD, sB, 64 * NG, KB);
+    else tile_nn<NG, true>(acc, As + k0 * LD, LD, sB, 64 * NG, KB);
+    if (more) put(buf ^ 1);
+    __syncthreads();
+  }
+}
+struct NoA { __device__ float4 operator()(int, int) const { return make_float4(0.f, 0.f, 0.f, 0.f); } };
+}  // namespace simt
+
+// ------------------------------------------------------------------ prep
+// One chunk: 64 x 64 x (2 Dk + Dv + Dk) multiply-adds and a triangular inverse, all operands through the streaming
+// stages; 70 KB of shared memory, three CTAs per SM.
+constexpr int kPrepF32Smem = (simt::kStageFloats + simt::R * simt::LD + 3 * simt::R) * 4;
+
+template <typename IO>
+__global__ void __launch_bounds__(256, 2) gdn_prep_kernel(GdnP p) {
+  using namespace simt;
+  extern __shared__ __align__(16) float smem[];
+  float* stage = smem;
+  float* Am = stage + kStageFloats;  // [64][LD]  A, then T in place
+  float* gam = Am + R * LD;
+  float* bet = gam + R;
+  float* bd = bet + R;  // beta * E(gam)
+  const int C = p.C, K = p.K, V = p.V;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31;
+  const int c = blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H, t0 = c * C;
+  const int imax = min(C, p.T - t0);
   const size_t ci = (size_t)bh * p.n + c;
   const IO* q = static_cast<const IO*>(p.q);
   const IO* k = static_cast<const IO*>(p.k);
   const IO* v = static_cast<const IO*>(p.v);
   auto row = [&](int i) { return ((size_t)(b * p.T + t0 + i) * p.H + h); };
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto ldq = [&](int i, int x) { return i < imax ? ld4(q + row(i) * K, x, K, p.vecK) : zero; };
+  auto ldk = [&](int i, int x) { return i < imax ? ld4(k + row(i) * K, x, K, p.vecK) : zero; };
+  auto ldv = [&](int i, int x) { return i < imax ? ld4(v + row(i) * V, x, V, p.vecV) : zero; };
 
-  if (tid < C) {
-    const bool ok = t0 + tid < p.T;
-    bet[tid] = ok ? p.beta[row(tid)] : 0.f;
-    gam[tid] = ok ? log_gate(p.gate[row(tid)], p.gate_is_log) : 0.f;
-  }
-  for (int idx = tid; idx < C * K; idx += blockDim.x) {
-    const int i = idx / K, kk = idx - i * K;
-    ks[i * ldk + kk] = (t0 + i < p.T) ? to_f32(k[row(i) * K + kk]) : 0.f;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    float acc = 0.f;
-    for (int i = 0; i < C; ++i) { acc += gam[i]; gam[i] = acc; }
-  }
-  __syncthreads();
-  if (tid < C) {
-    bd[tid] = bet[tid] * exp_nonpos_precise(gam[tid]);
-    p.gam[ci * C + tid] = gam[tid];
-  }
-  cta_gemm(C, C, K, [&](int i, int kk) { return ks[i * ldk + kk]; },
-           [&](int kk, int j) { return ks[j * ldk + kk]; },
-           [&](int i, int j, float acc) {
-             Am[i * ldc + j] = (i > j) ? -bet[i] * acc * exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
-           });
-  __syncthreads();
-  // T = (I - A)^-1, one thread per column, forward substitution over rows.
-  if (tid < C) {
-    const int col = tid;
-    for (int i = 0; i < C; ++i) {
-      float s = (i == col) ? 1.f : 0.f;
-      for (int j = col; j < i; ++j) s = fmaf(Am[i * ldc + j], Tm[j * ldc + col], s);
-      Tm[i * ldc + col] = (i < col) ? 0.f : s;
+  if (c == 0 && bh == 0 && tid < 64) p.status[tid] = 0;
+  if (tid < 32) {  // inclusive cumulative sum of the log gate, two elements per lane
+    const int i0 = 2 * lane, i1 = i0 + 1;
+    const float g0 = i0 < imax ? log_gate(p.gate[row(i0)], p.gate_is_log) : 0.f;
+    const float g1 = i1 < imax ? log_gate(p.gate[row(i1)], p.gate_is_log) : 0.f;
+    float s = g0 + g1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float t = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += t;
     }
+    const float b0 = i0 < imax ? p.beta[row(i0)] : 0.f, b1 = i1 < imax ? p.beta[row(i1)] : 0.f;
+    gam[i0] = s - g1; gam[i1] = s;
+    bet[i0] = b0; bet[i1] = b1;
+    bd[i0] = b0 * exp_nonpos_precise(s - g1); bd[i1] = b1 * exp_nonpos_precise(s);
+    if (i0 < C) p.gam[ci * C + i0] = s - g1;
+    if (i1 < C) p.gam[ci * C + i1] = s;
   }
-  __syncthreads();
-  for (int idx = tid; idx < C * C; idx += blockDim.x) {
-    const int i = idx / C, j = idx - i * C;
-    p.Tm[ci * C * C + idx] = Tm[i * ldc + j];
+  {
+    f2 acc[4][4];
+    clear(acc);
+    stream_nt(acc, stage, K, ldk, ldk);  // (its barriers also publish gam, bet, bd)
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int i = ty + 16 * r, j = tx + 16 * x;
+        Am[i * LD + j] = (i > j) ? -bet[i] * sum2(acc[r][x]) * exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
+      }
+    clear(acc);
+    stream_nt(acc, stage, K, ldq, ldk);
+    float* P = p.P + ci * C * C;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int i = ty + 16 * r, j = tx + 16 * x;
+        if (i < C && j < C) P[i * C + j] = (i >= j) ? sum2(acc[r][x]) * exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
+      }
   }
-  auto lo0 = [](int, int) { return 0; };
-  auto hi_i = [](int i, int) { return i + 1; };
-  // u = T (v beta)
-  cta_gemm_r(C, V, [&](int i, int m) { return Tm[i * ldc + m]; },
-             [&](int m, int j) { return (t0 + m < p.T) ? to_f32(v[row(m) * V + j]) * bet[m] : 0.f; },
-             lo0, hi_i, [&](int i, int j, float acc) { p.u[(ci * C + i) * V + j] = acc; });
-  // w = T (k beta E(gam))
-  cta_gemm_r(C, K, [&](int i, int m) { return Tm[i * ldc + m]; },
-             [&](int m, int kk) { return ks[m * ldk + kk] * bd[m]; },
-             lo0, hi_i, [&](int i, int kk, float acc) { p.w[(ci * C + i) * K + kk] = acc; });
-  // P = (q k^T) * Gamma * [i>=j]
-  cta_gemm(C, C, K,
-           [&](int i, int kk) { return (t0 + i < p.T) ? to_f32(q[row(i) * K + kk]) : 0.f; },
-           [&](int kk, int j) { return ks[j * ldk + kk]; },
-           [&](int i, int j, float acc) {
-             p.P[ci * C * C + i * C + j] = (i >= j) ? acc * exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
-           });
+  // T = (I - A)^-1 in place: the two 32 x 32 diagonal blocks by forward substitution (thread = block and column, the
+  // column in registers), then the off-diagonal block T21 = T22 (A21 T11) as two 32^3 products over all threads.
+  {
+    float Tc[32];
+    const int cc = tid & 31, r0 = 32 * ((tid >> 5) & 1);
+    if (tid < R) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float* arow = Am + (r0 + i) * LD + r0;
+        float s0 = (i == cc) ? 1.f : 0.f, s1 = 0.f;
+#pragma unroll
+        for (int j = 0; j + 1 < i; j += 2) {
+          s0 = fmaf(arow[j], Tc[j], s0);
+          s1 = fmaf(arow[j + 1], Tc[j + 1], s1);
+        }
+        if (i & 1) s0 = fmaf(arow[i - 1], Tc[i - 1], s0);
+        Tc[i] = (i < cc) ? 0.f : s0 + s1;
+      }
+    }
+    __syncthreads();
+    if (tid < R) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) Am[(r0 + i) * LD + r0 + cc] = Tc[i];
+    }
+    __syncthreads();
+    const int i2 = tid >> 3, jb = (tid & 7) * 4;
+    float4 x = zero;
+#pragma unroll 8
+    for (int m = 0; m < 32; ++m) {  // X = A21 T11 -> the unused upper-right block
+      const float a = Am[(32 + i2) * LD + m];
+      const float4 t = *reinterpret_cast<const float4*>(Am + m * LD + jb);
+      x = make_float4(fmaf(a, t.x, x.x), fmaf(a, t.y, x.y), fmaf(a, t.z, x.z), fmaf(a, t.w, x.w));
+    }
+    *reinterpret_cast<float4*>(Am + i2 * LD + 32 + jb) = x;
+    __syncthreads();
+    float4 y = zero;
+#pragma unroll 8
+    for (int m = 0; m < 32; ++m) {  // T21 = T22 X -> over A21
+      const float a = Am[(32 + i2) * LD + 32 + m];
+      const float4 t = *reinterpret_cast<const float4*>(Am + m * LD + 32 + jb);
+      y = make_float4(fmaf(a, t.x, y.x), fmaf(a, t.y, y.y), fmaf(a, t.z, y.z), fmaf(a, t.w, y.w));
+    }
+    *reinterpret_cast<float4*>(Am + (32 + i2) * LD + jb) = y;
+    __syncthreads();
+    *reinterpret_cast<float4*>(Am + i2 * LD + 32 + jb) = zero;  // the upper-right block of T
+    __syncthreads();
+  }
+  if (p.save)
+    for (int u = tid; u < R * R; u += 256) {
+      const int i = u >> 6, j = u & 63;
+      if (i < C && j < C) p.Tm[ci * C * C + i * C + j] = Am[i * LD + j];
+    }
+  // u = T (v beta), w = T (k beta E(gam)): a block of columns at a time
+  auto product = [&](auto ng, int n, int vec, float* dst, auto ld, const float* scale) {
+    constexpr int NG = decltype(ng)::value;
+    for (int j0 = 0; j0 < n; j0 += 64 * NG) {
+      f2 acc[4][2 * NG];
+      clear(acc);
+      stream_nn<NG, 1>(acc, stage, R, Am, NoA{}, [&](int m, int x) { return scale4(ld(m, j0 + x), scale[m]); });
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int g = 0; g < NG; ++g)
+          if (4 * ty + r < C) st4(dst + (ci * C + 4 * ty + r) * n, j0 + 64 * g + 4 * tx, n, vec, acc4<NG>(acc, r, g));
+    }
+  };
+  if (V <= 64) product(std::integral_constant<int, 1>{}, V, p.vecV, p.u, ldv, bet);
+  else product(std::integral_constant<int, 2>{}, V, p.vecV, p.u, ldv, bet);
+  if (K <= 64) product(std::integral_constant<int, 1>{}, K, p.vecK, p.w, ldk, bd);
+  else product(std::integral_constant<int, 2>{}, K, p.vecK, p.w, ldk, bd);
 }
 
 // ------------------------------------------------------------ state forward
-template <typename IO>
+// The sequential pass: latency and arithmetic of one chunk, chunk after chunk.  A CTA owns 16 columns of the state, so
+// that a few (batch, head) pairs still spread over many SMs.  The tiles of the next chunk travel (cp.async) as soon as
+// their buffer has been read: w and q behind the first barrier, k and P behind the second.
+//   [w;q] S      thread = rows ty, ty + 32 of both x columns tx, tx + 8
+//   P v_new      the same rows and columns
+//   (k r)^T v_new  thread = KT state rows x 2 columns, the state itself stays in registers
+template <int KP>
+constexpr int state_fwd_smem() {
+  return 4 * (192 * (KP + 4) + simt::R * simt::LD + 16 * (KP + 4) + 16 * simt::LD + simt::R * 32 + 2 * (2 * simt::R + 4));
+}
+template <typename IO, int KP>
 __global__ void __launch_bounds__(256) gdn_state_fwd_kernel(GdnP p) {
-  extern __shared__ float smem[];
+  using namespace simt;
+  constexpr int LK = KP + 4, KT = KP / 32;
+  extern __shared__ __align__(16) float smem[];
+  float* Wq = smem;              // [128][LK] w rows, then q rows
+  float* Ks = Wq + 128 * LK;     // [64][LK]
+  float* Ps = Ks + R * LK;       // [64][LD]
+  float* St = Ps + R * LD;       // [16][LK]  S^T
+  float* Vt = St + 16 * LK;      // [16][LD]  v_new^T
+  float* Vd = Vt + 16 * LD;      // [64][32]  r_i v_new, every element twice
+  float* sc = Vd + R * 32;       // x2 [64] E(gam), [64] E(gam_last - gam), E(gam_last)
+  constexpr int kSc = 2 * R + 4;
   const int C = p.C, K = p.K, V = p.V;
-  float* S = smem;            // [K][33]
-  float* vn = S + K * 33;     // [C][32]
-  float* vr = vn + C * 32;    // [C][32]  r_i * v_new
-  float* dd = vr + C * 32;    // [C] E(gam)
-  float* rr = dd + C;         // [C] E(gam_last - gam)
-  const int tid = threadIdx.x, j = tid & 31, rg = tid >> 5;
-  const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
-  const int jv = blockIdx.x * 32 + j;
-  const bool jok = jv < V;
+  const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3, kk0 = ty * KT;
+  const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H, j0 = blockIdx.x * 16;
   const IO* q = static_cast<const IO*>(p.q);
   const IO* k = static_cast<const IO*>(p.k);
   IO* out = static_cast<IO*>(p.out);
-
-  for (int kk = rg; kk < K; kk += 8)
-    S[kk * 33 + j] = (p.h0 && jok) ? p.h0[((size_t)bh * K + kk) * V + jv] : 0.f;
+  auto row = [&](int c, int i) { return ((size_t)(b * p.T + c * C + i) * p.H + h); };
+  auto load_wq = [&](int c) {
+    if (c < p.n) {
+      const float* w = p.w + ((size_t)bh * p.n + c) * C * K;
+      stage_rows(Wq, LK, C, K, p.vecK, w, [&](int i) { return w + i * K; });
+      stage_rows(Wq + R * LK, LK, min(C, p.T - c * C), K, p.vecK, q, [&](int i) { return q + row(c, i) * K; });
+    }
+    cp_commit();
+  };
+  auto load_kp = [&](int c) {
+    if (c < p.n) {
+      stage_rows(Ks, LK, min(C, p.T - c * C), K, p.vecK, k, [&](int i) { return k + row(c, i) * K; });
+      const float* P = p.P + ((size_t)bh * p.n + c) * C * C;
+      if (C == R) {
+        for (int u = tid; u < R * 16; u += 256) cp_async16(Ps + (u >> 4) * LD + 4 * (u & 15), P + 4 * u, true);
+      } else {
+        for (int u = tid; u < C * C; u += 256) cp_async4(Ps + (u / C) * LD + u % C, P + u, true);
+      }
+    }
+    cp_commit();
+  };
+  auto scalars = [&](int c) {  // decay factors of chunk c, buffer c & 1
+    float* s = sc + (c & 1) * kSc;
+    if (tid < R) {
+      const float* gam = p.gam + ((size_t)bh * p.n + c) * C;
+      const float gl = gam[C - 1], g = tid < C ? gam[tid] : gl;
+      s[tid] = exp_nonpos_precise(g);
+      s[R + tid] = exp_nonpos_precise(gl - g);
+      if (tid == 0) s[2 * R] = exp_nonpos_precise(gl);
+    }
+  };
+  for (int u = tid; u < 192 * LK; u += 256) Wq[u] = 0.f;  // rows and columns that no copy reaches
+  for (int u = tid; u < R * LD; u += 256) Ps[u] = 0.f;
+  f2 S[2][KT / 2];  // state rows kk0 .. , columns j0 + 2 tx and + 1
+#pragma unroll
+  for (int y = 0; y < 2; ++y)
+#pragma unroll
+    for (int x = 0; x < KT / 2; ++x) {
+      const int jv = j0 + 2 * tx + y, kk = kk0 + 2 * x;
+      const float* src = p.h0 ? p.h0 + ((size_t)bh * K + kk) * V + jv : nullptr;
+      S[y][x] = pack2(src && jv < V && kk < K ? src[0] : 0.f, src && jv < V && kk + 1 < K ? src[V] : 0.f);
+    }
+  scalars(0);
   __syncthreads();
+  load_wq(0);
+  load_kp(0);
+#pragma unroll
+  for (int y = 0; y < 2; ++y)
+#pragma unroll
+    for (int x = 0; x < KT / 2; ++x) *reinterpret_cast<f2*>(St + (2 * tx + y) * LK + kk0 + 2 * x) = S[y][x];
 
   for (int c = 0; c < p.n; ++c) {
     const size_t ci = (size_t)bh * p.n + c;
-    const int t0 = c * C;
-    auto row = [&](int i) { return ((size_t)(b * p.T + t0 + i) * p.H + h); };
-    const float* gam = p.gam + ci * C;
-    const float glast = gam[C - 1];
-    if (tid < C) {
-      dd[tid] = exp_nonpos_precise(gam[tid]);
-      rr[tid] = exp_nonpos_precise(glast - gam[tid]);
-    }
+    const float* s = sc + (c & 1) * kSc;
+    const int imax = min(C, p.T - c * C);
     if (p.save) {  // state at chunk start, transposed [V][K]
-      for (int idx = tid; idx < 32 * K; idx += blockDim.x) {
-        const int jj = idx / K, kk = idx - jj * K;
-        const int col = blockIdx.x * 32 + jj;
-        if (col < V) p.hs[(ci * V + col) * K + kk] = S[kk * 33 + jj];
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int x = 0; x < KT / 2; ++x) {
+          const int jv = j0 + 2 * tx + y, kk = kk0 + 2 * x;
+          const float2 t = unpack2(S[y][x]);
+          float* dst = p.hs + (ci * V + jv) * K + kk;
+          if (jv < V && kk < K) dst[0] = t.x;
+          if (jv < V && kk + 1 < K) dst[1] = t.y;
+        }
+    }
+    float un[2][2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const int i = ty + 32 * r, jv = j0 + tx + 8 * y;
+        un[r][y] = (i < C && jv < V) ? p.u[(ci * C + i) * V + jv] : 0.f;
+      }
+    cp_wait<1>();
+    __syncthreads();  // w, q and the state are in place
+    f2 acc[4][2];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = 0ull;
+#pragma unroll 4
+    for (int x = 0; x < KP; x += 4) {
+      const ulonglong2 s0 = lds2x2(St + tx * LK + x), s1 = lds2x2(St + (tx + 8) * LK + x);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const ulonglong2 a = lds2x2(Wq + (ty + 32 * r) * LK + x);
+        fma2(acc[r][0], a.x, s0.x);
+        fma2(acc[r][1], a.x, s1.x);
+        fma2(acc[r][0], a.y, s0.y);
+        fma2(acc[r][1], a.y, s1.y);
       }
     }
-    __syncthreads();
-    // v_new = u - w S
-    const float* w = p.w + ci * C * K;
-    for (int i = rg; i < C; i += 8) {
-      float acc = 0.f;
-      for (int kk = 0; kk < K; ++kk) acc = fmaf(w[i * K + kk], S[kk * 33 + j], acc);
-      const float val = jok ? p.u[(ci * C + i) * V + jv] - acc : 0.f;
-      vn[i * 32 + j] = val;
-      vr[i * 32 + j] = val * rr[i];
-      if (p.save && jok) p.vn[(ci * C + i) * V + jv] = val;
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {  // v_new = u - w S
+        const int i = ty + 32 * r, j = tx + 8 * y;
+        const float val = un[r][y] - sum2(acc[r][y]);
+        Vt[j * LD + i] = val;
+        const float vr = val * s[R + i];
+        *reinterpret_cast<f2*>(Vd + i * 32 + 2 * j) = pack2(vr, vr);
+        if (p.save && i < C && j0 + j < V) p.vn[(ci * C + i) * V + j0 + j] = val;
+      }
+    cp_wait<0>();
+    __syncthreads();  // v_new, k and P are in place; w and q have been read
+    load_wq(c + 1);
+    {  // o = E(gam) (q S) + P v_new
+      f2 o[2][2];
+      o[0][0] = o[0][1] = o[1][0] = o[1][1] = 0ull;
+#pragma unroll 4
+      for (int m = 0; m < 32; m += 4) {
+        const ulonglong2 v0 = lds2x2(Vt + tx * LD + m), v1 = lds2x2(Vt + (tx + 8) * LD + m);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const ulonglong2 a = lds2x2(Ps + (ty + 32 * r) * LD + m);
+          fma2(o[r][0], a.x, v0.x);
+          fma2(o[r][1], a.x, v1.x);
+          fma2(o[r][0], a.y, v0.y);
+          fma2(o[r][1], a.y, v1.y);
+        }
+      }
+#pragma unroll 4
+      for (int m = 32; m < 64; m += 4) {  // P is lower triangular: only the upper rows have these columns
+        const ulonglong2 v0 = lds2x2(Vt + tx * LD + m), v1 = lds2x2(Vt + (tx + 8) * LD + m);
+        const ulonglong2 a = lds2x2(Ps + (ty + 32) * LD + m);
+        fma2(o[1][0], a.x, v0.x);
+        fma2(o[1][1], a.x, v1.x);
+        fma2(o[1][0], a.y, v0.y);
+        fma2(o[1][1], a.y, v1.y);
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          const int i = ty + 32 * r, jv = j0 + tx + 8 * y;
+          if (i < imax && jv < V) out[row(c, i) * V + jv] = from_f32<IO>(fmaf(s[i], sum2(acc[2 + r][y]), sum2(o[r][y])));
+        }
     }
-    __syncthreads();
-    // o = E(gam) (q S) + P v_new
-    const float* P = p.P + ci * C * C;
-    for (int i = rg; i < C; i += 8) {
-      if (t0 + i >= p.T) continue;
-      float acc = 0.f;
-      const IO* qi = q + row(i) * K;
-      for (int kk = 0; kk < K; ++kk) acc = fmaf(to_f32(qi[kk]), S[kk * 33 + j], acc);
-      acc *= dd[i];
-      for (int m = 0; m <= i; ++m) acc = fmaf(P[i * C + m], vn[m * 32 + j], acc);
-      if (jok) out[row(i) * V + jv] = from_f32<IO>(acc);
+    {  // S <- S E(gam_last) + (k r)^T v_new
+      const f2 L = pack2(s[2 * R], s[2 * R]);
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int x = 0; x < KT / 2; ++x) S[y][x] = mul2(S[y][x], L);
+#pragma unroll 8
+      for (int i = 0; i < R; ++i) {
+        const ulonglong2 vv = lds2x2(Vd + i * 32 + 4 * tx);
+#pragma unroll
+        for (int x = 0; x < KT / 2; ++x) {
+          const f2 kx = *reinterpret_cast<const f2*>(Ks + i * LK + kk0 + 2 * x);
+          fma2(S[0][x], kx, vv.x);
+          fma2(S[1][x], kx, vv.y);
+        }
+      }
     }
-    __syncthreads();
-    // S <- S E(gam_last) + (k r)^T v_new
-    const float L = exp_nonpos_precise(glast);
-    const int imax = min(C, p.T - t0);
-    for (int kk = rg; kk < K; kk += 8) {
-      float acc = S[kk * 33 + j] * L;
-      for (int i = 0; i < imax; ++i) acc = fmaf(to_f32(k[row(i) * K + kk]), vr[i * 32 + j], acc);
-      S[kk * 33 + j] = acc;
-    }
-    __syncthreads();
+    if (c + 1 < p.n) scalars(c + 1);
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+      for (int x = 0; x < KT / 2; ++x) *reinterpret_cast<f2*>(St + (2 * tx + y) * LK + kk0 + 2 * x) = S[y][x];
+    __syncthreads();  // k, P and v_new have been read
+    load_kp(c + 1);
   }
-  if (p.hT && jok)
-    for (int kk = rg; kk < K; kk += 8) p.hT[((size_t)bh * K + kk) * V + jv] = S[kk * 33 + j];
+  if (p.hT) {
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+      for (int x = 0; x < KT / 2; ++x) {
+        const int jv = j0 + 2 * tx + y, kk = kk0 + 2 * x;
+        const float2 t = unpack2(S[y][x]);
+        float* dst = p.hT + ((size_t)bh * K + kk) * V + jv;
+        if (jv < V && kk < K) dst[0] = t.x;
+        if (jv < V && kk + 1 < K) dst[V] = t.y;
+      }
+  }
 }
 
 // ----------------------------------------------------------- state backward
-template <typename IO>
+// The same slabs in reverse:  dv_new = P^T dO + r (k dS);  dS <- E(gam_last) dS + (q E(gam))^T dO - w^T dv_new.
+// k and P of the next chunk travel behind the first barrier, q and w behind the second.
+template <int KP>
+constexpr int state_bwd_smem() {
+  return 4 * (192 * (KP + 4) + simt::R * simt::LD + 16 * (KP + 4) + 16 * simt::LD + 3 * simt::R * 32 + 2 * (2 * simt::R + 4));
+}
+template <typename IO, int KP>
 __global__ void __launch_bounds__(256) gdn_state_bwd_kernel(GdnP p) {
-  extern __shared__ float smem[];
+  using namespace simt;
+  constexpr int LK = KP + 4, KT = KP / 32;
+  extern __shared__ __align__(16) float smem[];
+  float* Ks = smem;              // [64][LK]
+  float* Qs = Ks + R * LK;       // [64][LK]
+  float* Ws = Qs + R * LK;       // [64][LK]
+  float* Pt = Ws + R * LK;       // [64][LD]  P^T
+  float* St = Pt + R * LD;       // [16][LK]  dS^T
+  float* Ot = St + 16 * LK;      // [16][LD]  dO^T
+  float* Vd = Ot + 16 * LD;      // [64][32]  -dv_new, every element twice
+  float* Od = Vd + R * 32;       // x2 [64][32]  E(gam_i) dO, every element twice
+  float* sc = Od + 2 * R * 32;   // x2 [64] E(gam), [64] E(gam_last - gam), E(gam_last)
+  constexpr int kSc = 2 * R + 4;
   const int C = p.C, K = p.K, V = p.V;
-  float* dS = smem;            // [K][33]
-  float* dOs = dS + K * 33;    // [C][32]
-  float* dOd = dOs + C * 32;   // [C][32]  E(gam_i) dO
-  float* dvs = dOd + C * 32;   // [C][32]  dv_new
-  float* dd = dvs + C * 32;
-  float* rr = dd + C;
-  const int tid = threadIdx.x, j = tid & 31, rg = tid >> 5;
-  const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
-  const int jv = blockIdx.x * 32 + j;
-  const bool jok = jv < V;
+  const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3, kk0 = ty * KT;
+  const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H, j0 = blockIdx.x * 16;
   const IO* q = static_cast<const IO*>(p.q);
   const IO* k = static_cast<const IO*>(p.k);
   const IO* dO = static_cast<const IO*>(p.dO);
-
-  for (int kk = rg; kk < K; kk += 8)
-    dS[kk * 33 + j] = (p.dhT_in && jok) ? p.dhT_in[((size_t)bh * K + kk) * V + jv] : 0.f;
+  auto row = [&](int c, int i) { return ((size_t)(b * p.T + c * C + i) * p.H + h); };
+  auto load_kp = [&](int c) {
+    if (c >= 0) {
+      stage_rows(Ks, LK, min(C, p.T - c * C), K, p.vecK, k, [&](int i) { return k + row(c, i) * K; });
+      const float* P = p.P + ((size_t)bh * p.n + c) * C * C;
+      for (int u = tid; u < C * C; u += 256) {
+        const int m = C == R ? u >> 6 : u / C, i = u - m * C;
+        cp_async4(Pt + i * LD + m, P + u, true);
+      }
+    }
+    cp_commit();
+  };
+  auto load_qw = [&](int c) {
+    if (c >= 0) {
+      const float* w = p.w + ((size_t)bh * p.n + c) * C * K;
+      stage_rows(Qs, LK, min(C, p.T - c * C), K, p.vecK, q, [&](int i) { return q + row(c, i) * K; });
+      stage_rows(Ws, LK, C, K, p.vecK, w, [&](int i) { return w + i * K; });
+    }
+    cp_commit();
+  };
+  auto scalars = [&](int c) {
+    float* s = sc + (c & 1) * kSc;
+    if (tid < R) {
+      const float* gam = p.gam + ((size_t)bh * p.n + c) * C;
+      const float gl = gam[C - 1], g = tid < C ? gam[tid] : gl;
+      s[tid] = exp_nonpos_precise(g);
+      s[R + tid] = exp_nonpos_precise(gl - g);
+      if (tid == 0) s[2 * R] = exp_nonpos_precise(gl);
+    }
+  };
+  float o[2][2];  // this thread's elements of dO, fetched a chunk ahead
+  auto fetch_o = [&](int c) {
+    const int imax = min(C, p.T - c * C);
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const int i = ty + 32 * r, jv = j0 + tx + 8 * y;
+        o[r][y] = (i < imax && jv < V) ? to_f32(dO[row(c, i) * V + jv]) : 0.f;
+      }
+  };
+  // the scaling with E(gam) reads the factor itself: the chunk's scalars are being written by other threads
+  auto put_o = [&](int c) {
+    const float* gam = p.gam + ((size_t)bh * p.n + c) * C;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int i = ty + 32 * r;
+      const float di = exp_nonpos_precise(gam[min(i, C - 1)]);
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const int j = tx + 8 * y;
+        Ot[j * LD + i] = o[r][y];
+        const float x = o[r][y] * di;
+        *reinterpret_cast<f2*>(Od + (c & 1) * R * 32 + i * 32 + 2 * j) = pack2(x, x);
+      }
+    }
+  };
+  for (int u = tid; u < 192 * LK + R * LD; u += 256) Ks[u] = 0.f;  // rows and columns that no copy reaches
+  f2 S[2][KT / 2];
+#pragma unroll
+  for (int y = 0; y < 2; ++y)
+#pragma unroll
+    for (int x = 0; x < KT / 2; ++x) {
+      const int jv = j0 + 2 * tx + y, kk = kk0 + 2 * x;
+      const float* src = p.dhT_in ? p.dhT_in + ((size_t)bh * K + kk) * V + jv : nullptr;
+      S[y][x] = pack2(src && jv < V && kk < K ? src[0] : 0.f, src && jv < V && kk + 1 < K ? src[V] : 0.f);
+    }
+  scalars(p.n - 1);
+  fetch_o(p.n - 1);
   __syncthreads();
+  load_kp(p.n - 1);
+  load_qw(p.n - 1);
+  put_o(p.n - 1);
+#pragma unroll
+  for (int y = 0; y < 2; ++y)
+#pragma unroll
+    for (int x = 0; x < KT / 2; ++x) *reinterpret_cast<f2*>(St + (2 * tx + y) * LK + kk0 + 2 * x) = S[y][x];
 
   for (int c = p.n - 1; c >= 0; --c) {
     const size_t ci = (size_t)bh * p.n + c;
-    const int t0 = c * C;
-    auto row = [&](int i) { return ((size_t)(b * p.T + t0 + i) * p.H + h); };
-    const float* gam = p.gam + ci * C;
-    const float glast = gam[C - 1];
-    const int imax = min(C, p.T - t0);
-    if (tid < C) {
-      dd[tid] = exp_nonpos_precise(gam[tid]);
-      rr[tid] = exp_nonpos_precise(glast - gam[tid]);
-    }
-    for (int idx = tid; idx < 32 * K; idx += blockDim.x) {  // dS at chunk end, transposed
-      const int jj = idx / K, kk = idx - jj * K;
-      const int col = blockIdx.x * 32 + jj;
-      if (col < V) p.dhs[(ci * V + col) * K + kk] = dS[kk * 33 + jj];
-    }
-    __syncthreads();
-    for (int i = rg; i < C; i += 8) {
-      const float x = (i < imax && jok) ? to_f32(dO[row(i) * V + jv]) : 0.f;
-      dOs[i * 32 + j] = x;
-      dOd[i * 32 + j] = x * dd[i];
-    }
-    __syncthreads();
-    // dv_new = P^T dO + (k r) dS
-    const float* P = p.P + ci * C * C;
-    for (int i = rg; i < C; i += 8) {
-      float acc = 0.f;
-      if (i < imax) {
-        const IO* ki = k + row(i) * K;
-        for (int kk = 0; kk < K; ++kk) acc = fmaf(to_f32(ki[kk]), dS[kk * 33 + j], acc);
-        acc *= rr[i];
+    const float* s = sc + (c & 1) * kSc;
+    // dS at chunk end, transposed [V][K]
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+      for (int x = 0; x < KT / 2; ++x) {
+        const int jv = j0 + 2 * tx + y, kk = kk0 + 2 * x;
+        const float2 t = unpack2(S[y][x]);
+        float* dst = p.dhs + (ci * V + jv) * K + kk;
+        if (jv < V && kk < K) dst[0] = t.x;
+        if (jv < V && kk + 1 < K) dst[1] = t.y;
       }
-      for (int m = i; m < C; ++m) acc = fmaf(P[m * C + i], dOs[m * 32 + j], acc);
-      dvs[i * 32 + j] = acc;
-      if (jok) p.dvn[(ci * C + i) * V + jv] = acc;
+    if (c > 0) fetch_o(c - 1);
+    cp_wait<1>();
+    __syncthreads();  // k, P, dO and dS are in place
+    f2 acc[2][2], po[2][2];
+    acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0ull;
+    po[0][0] = po[0][1] = po[1][0] = po[1][1] = 0ull;
+#pragma unroll 4
+    for (int x = 0; x < KP; x += 4) {  // k dS
+      const ulonglong2 s0 = lds2x2(St + tx * LK + x), s1 = lds2x2(St + (tx + 8) * LK + x);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const ulonglong2 a = lds2x2(Ks + (ty + 32 * r) * LK + x);
+        fma2(acc[r][0], a.x, s0.x);
+        fma2(acc[r][1], a.x, s1.x);
+        fma2(acc[r][0], a.y, s0.y);
+        fma2(acc[r][1], a.y, s1.y);
+      }
     }
-    __syncthreads();
-    // dS <- E(gam_last) dS + (q E(gam))^T dO - w^T dv_new
-    const float L = exp_nonpos_precise(glast);
-    const float* w = p.w + ci * C * K;
-    for (int kk = rg; kk < K; kk += 8) {
-      float acc = dS[kk * 33 + j] * L;
-      for (int i = 0; i < imax; ++i) acc = fmaf(to_f32(q[row(i) * K + kk]), dOd[i * 32 + j], acc);
-      for (int i = 0; i < C; ++i) acc = fmaf(-w[i * K + kk], dvs[i * 32 + j], acc);
-      dS[kk * 33 + j] = acc;
+#pragma unroll 4
+    for (int m = 0; m < 32; m += 4) {  // P^T dO (upper triangular: the lower rows start at their half)
+      const ulonglong2 v0 = lds2x2(Ot + tx * LD + m), v1 = lds2x2(Ot + (tx + 8) * LD + m);
+      const ulonglong2 a = lds2x2(Pt + ty * LD + m);
+      fma2(po[0][0], a.x, v0.x);
+      fma2(po[0][1], a.x, v1.x);
+      fma2(po[0][0], a.y, v0.y);
+      fma2(po[0][1], a.y, v1.y);
     }
-    __syncthreads();
+#pragma unroll 4
+    for (int m = 32; m < 64; m += 4) {
+      const ulonglong2 v0 = lds2x2(Ot + tx * LD + m), v1 = lds2x2(Ot + (tx + 8) * LD + m);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const ulonglong2 a = lds2x2(Pt + (ty + 32 * r) * LD + m);
+        fma2(po[r][0], a.x, v0.x);
+        fma2(po[r][1], a.x, v1.x);
+        fma2(po[r][0], a.y, v0.y);
+        fma2(po[r][1], a.y, v1.y);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const int i = ty + 32 * r, j = tx + 8 * y;
+        const float val = fmaf(s[R + i], sum2(acc[r][y]), sum2(po[r][y]));
+        *reinterpret_cast<f2*>(Vd + i * 32 + 2 * j) = pack2(-val, -val);
+        if (i < C && j0 + j < V) p.dvn[(ci * C + i) * V + j0 + j] = val;
+      }
+    cp_wait<0>();
+    __syncthreads();  // dv_new, q and w are in place; k, P and dO have been read
+    load_kp(c - 1);
+    const float* od = Od + (c & 1) * R * 32;
+    const f2 L = pack2(s[2 * R], s[2 * R]);
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+      for (int x = 0; x < KT / 2; ++x) S[y][x] = mul2(S[y][x], L);
+#pragma unroll 4
+    for (int i = 0; i < R; ++i) {
+      const ulonglong2 oo = lds2x2(od + i * 32 + 4 * tx), vv = lds2x2(Vd + i * 32 + 4 * tx);
+#pragma unroll
+      for (int x = 0; x < KT / 2; ++x) {
+        const f2 qx = *reinterpret_cast<const f2*>(Qs + i * LK + kk0 + 2 * x);
+        const f2 wx = *reinterpret_cast<const f2*>(Ws + i * LK + kk0 + 2 * x);
+        fma2(S[0][x], qx, oo.x);
+        fma2(S[1][x], qx, oo.y);
+        fma2(S[0][x], wx, vv.x);
+        fma2(S[1][x], wx, vv.y);
+      }
+    }
+    if (c > 0) {
+      scalars(c - 1);
+      put_o(c - 1);
+    }
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+      for (int x = 0; x < KT / 2; ++x) *reinterpret_cast<f2*>(St + (2 * tx + y) * LK + kk0 + 2 * x) = S[y][x];
+    __syncthreads();  // q, w and dv_new have been read
+    load_qw(c - 1);
   }
-  if (p.dh0 && jok)
-    for (int kk = rg; kk < K; kk += 8) p.dh0[((size_t)bh * K + kk) * V + jv] = dS[kk * 33 + j];
+  if (p.dh0) {
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+      for (int x = 0; x < KT / 2; ++x) {
+        const int jv = j0 + 2 * tx + y, kk = kk0 + 2 * x;
+        const float2 t = unpack2(S[y][x]);
+        float* dst = p.dh0 + ((size_t)bh * K + kk) * V + jv;
+        if (jv < V && kk < K) dst[0] = t.x;
+        if (jv < V && kk + 1 < K) dst[V] = t.y;
+      }
+  }
 }
 
 // ----------------------------------------------------------- chunk backward
-template <typename IO>
-__global__ void __launch_bounds__(256) gdn_chunk_bwd_kernel(GdnP p) {
-  extern __shared__ float smem[];
-  const int C = p.C, K = p.K, V = p.V, ldc = C + 1;
-  const int lds = (K > V ? K : V) + 1;
-  float* stage = smem;             // [C][lds]
-  float* Tm = stage + C * lds;     // [C][ldc]
-  float* G = Tm + C * ldc;         // Gamma (lower incl.)
-  float* X1 = G + C * ldc;         // dP*Gamma
-  float* X2 = X1 + C * ldc;        // scratch / dT / dA
-  float* X3 = X2 + C * ldc;        // k k^T
-  float* X4 = X3 + C * ldc;        // scratch / T^T dT / symmetric M
-  float* gam = X4 + C * ldc;
-  float* bet = gam + C;
-  float* dd = bet + C;
-  float* rr = dd + C;
-  float* dgam = rr + C;
-  float* dbet = dgam + C;
-  float* rs1 = dbet + C;          // [C] per-row scratch sums
-  float* rs2 = rs1 + C;
-  float* red = rs2 + C;           // [32]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// One CTA per chunk, everything that is not the sequential pass.  With e = T^T dv_new and z = T^T dw = -e S0^T
+// (dw = -dv_new S0^T is never formed):
+//   dPG = tril(dO v_new^T) Gamma                       dq = E(gam) dO S0^T + dPG k
+//   Y = e (v beta)^T + z (k beta E(gam))^T             M = -tril(Y T^T, -1) Gamma,  Mb = beta_i M
+//   dk = r (v_new dS^T) + dPG^T q + (Mb + Mb^T) k + beta E(gam) z            dv = beta e
+//   dbeta = e.v + E(gam) (k.z) + sum_j M_ij (k_i.k_j)
+//   dgam_i = q_i.dq_i - k_i.dk_i + 2 beta_i (E(gam_i) (k_i.z_i) + sum_j M_ij (k_i.k_j)),
+//   dgam_last += L <dS,S0> + sum_i r_i k_i.(v_new dS^T)_i
+// (the row and column sums over Gamma of the P and A terms are the parts of q.dq and k.dk that come from dPG and Mb).
+// Three 64 x 64 matrices live in shared memory, every wide operand is streamed; e and z make a round trip through the
+// workspace (L2).  105 KB: two CTAs per SM.
+constexpr int kChunkF32Smem = (simt::kStageFloats + 3 * simt::R * simt::LD + 9 * simt::R + 16) * 4;
+static_assert(2 * (kChunkF32Smem + 1024) <= 228 * 1024, "two CTAs per SM");
+
+template <typename IO, int NGK>
+__global__ void __launch_bounds__(256, 2) gdn_chunk_bwd_kernel(GdnP p) {
+  using namespace simt;
+  extern __shared__ __align__(16) float smem[];
+  float* stage = smem;
+  float* Tm = stage + kStageFloats;  // [64][LD] T
+  float* X1 = Tm + R * LD;           // dP Gamma
+  float* X2 = X1 + R * LD;           // Y, then Mb + Mb^T
+  float* gam = X2 + R * LD;
+  float* bet = gam + R;
+  float* dd = bet + R;
+  float* rr = dd + R;
+  float* bd = rr + R;
+  float* rs = bd + R;    // row sums of M (k k^T)
+  float* dbe = rs + R;   // dbeta
+  float* dg = dbe + R;   // dgam
+  float* rho = dg + R;   // k_i . dkp_i
+  float* red = rho + R;  // [8]
+  const int C = p.C, K = p.K, V = p.V;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31, warp = tid >> 5;
   const int c = blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H, t0 = c * C;
   const size_t ci = (size_t)bh * p.n + c;
   const int imax = min(C, p.T - t0);
-  const IO* q = static_cast<const IO*>(p.q);
-  const IO* k = static_cast<const IO*>(p.k);
-  const IO* v = static_cast<const IO*>(p.v);
-  const IO* dO = static_cast<const IO*>(p.dO);
   auto row = [&](int i) { return ((size_t)(b * p.T + t0 + i) * p.H + h); };
-  auto ldq = [&](int i, int kk) { return i < imax ? to_f32(q[row(i) * K + kk]) : 0.f; };
-  auto ldk = [&](int i, int kk) { return i < imax ? to_f32(k[row(i) * K + kk]) : 0.f; };
-  auto ldv = [&](int i, int jj) { return i < imax ? to_f32(v[row(i) * V + jj]) : 0.f; };
-  auto lddo = [&](int i, int jj) { return i < imax ? to_f32(dO[row(i) * V + jj]) : 0.f; };
-  const float* hs = p.hs + ci * V * K;
-  const float* dhs = p.dhs + ci * V * K;
-  const float* vn = p.vn + ci * C * V;
-  const float* dvn = p.dvn + ci * C * V;
-  float* dqi = p.dqi + ci * C * K;
-  float* dw = p.dw + ci * C * K;
-  float* dkt = p.dkt + ci * C * K;
-  auto lo0 = [](int, int) { return 0; };
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const IO *q = static_cast<const IO*>(p.q), *k = static_cast<const IO*>(p.k);
+  const IO *v = static_cast<const IO*>(p.v), *dO = static_cast<const IO*>(p.dO);
+  auto ldq = [&](int i, int x) { return i < imax ? ld4(q + row(i) * K, x, K, p.vecK) : zero; };
+  auto ldk = [&](int i, int x) { return i < imax ? ld4(k + row(i) * K, x, K, p.vecK) : zero; };
+  auto ldv = [&](int i, int x) { return i < imax ? ld4(v + row(i) * V, x, V, p.vecV) : zero; };
+  auto ldo = [&](int i, int x) { return i < imax ? ld4(dO + row(i) * V, x, V, p.vecV) : zero; };
+  const float *hs = p.hs + ci * V * K, *dhs = p.dhs + ci * V * K;
+  const float *vn = p.vn + ci * C * V, *dvn = p.dvn + ci * C * V;
+  float *e = p.e + ci * C * V, *z = p.z + ci * C * K;
+  auto lde = [&](int i, int x) { return i < C ? ld4(e + i * V, x, V, p.vecV) : zero; };
+  auto ldz = [&](int i, int x) { return i < C ? ld4(z + i * K, x, K, p.vecK) : zero; };
+  auto ldvn = [&](int i, int x) { return i < C ? ld4(vn + i * V, x, V, p.vecV) : zero; };
+  auto lddvn = [&](int i, int x) { return i < C ? ld4(dvn + i * V, x, V, p.vecV) : zero; };
+  auto ldhs = [&](int j, int x) { return j < V ? ld4(hs + (size_t)j * K, x, K, p.vecK) : zero; };
+  auto lddhs = [&](int j, int x) { return j < V ? ld4(dhs + (size_t)j * K, x, K, p.vecK) : zero; };
 
-  if (tid < C) {
-    gam[tid] = p.gam[ci * C + tid];
-    bet[tid] = (tid < imax) ? p.beta[row(tid)] : 0.f;
-    dgam[tid] = 0.f;
-    dbet[tid] = 0.f;
+  if (tid < R) {
+    const float gl = p.gam[ci * C + C - 1], g = tid < C ? p.gam[ci * C + tid] : gl;
+    const float bt = tid < imax ? p.beta[row(tid)] : 0.f, d = exp_nonpos_precise(g);
+    gam[tid] = g;
+    bet[tid] = bt;
+    dd[tid] = d;
+    rr[tid] = exp_nonpos_precise(gl - g);
+    bd[tid] = bt * d;
   }
-  __syncthreads();
-  const float glast = gam[C - 1];
-  const float L = exp_nonpos_precise(glast);
-  if (tid < C) {
-    dd[tid] = exp_nonpos_precise(gam[tid]);
-    rr[tid] = exp_nonpos_precise(glast - gam[tid]);
+  for (int u = tid; u < R * R; u += 256) {
+    const int i = u >> 6, j = u & 63;
+    Tm[i * LD + j] = (i < C && j < C) ? p.Tm[ci * C * C + i * C + j] : 0.f;
   }
-  for (int idx = tid; idx < C * C; idx += blockDim.x) {
-    const int i = idx / C, j = idx - i * C;
-    Tm[i * ldc + j] = p.Tm[ci * C * C + idx];
-    G[i * ldc + j] = (i >= j) ? exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
-  }
-  // ---- A: contractions with the two states (operands straight from global) ----
-  cta_gemm(C, K, V, [&](int i, int jj) { return lddo(i, jj); },
-           [&](int jj, int kk) { return hs[jj * K + kk]; },
-           [&](int i, int kk, float acc) { dqi[i * K + kk] = acc; });
-  cta_gemm(C, K, V, [&](int i, int jj) { return dvn[i * V + jj]; },
-           [&](int jj, int kk) { return hs[jj * K + kk]; },
-           [&](int i, int kk, float acc) { dw[i * K + kk] = -acc; });
-  cta_gemm(C, K, V, [&](int i, int jj) { return vn[i * V + jj]; },
-           [&](int jj, int kk) { return dhs[jj * K + kk]; },
-           [&](int i, int kk, float acc) { dkt[i * K + kk] = acc; });
-  {  // L <dS_end, S_start>
+  {  // <dS, S0>
     float part = 0.f;
-    for (int idx = tid; idx < V * K; idx += blockDim.x) part = fmaf(hs[idx], dhs[idx], part);
+    if (p.vecK) {
+      for (int u = 4 * tid; u < V * K; u += 1024)
+        part = dot4(*reinterpret_cast<const float4*>(hs + u), *reinterpret_cast<const float4*>(dhs + u), part);
+    } else {
+      for (int u = tid; u < V * K; u += 256) part = fmaf(hs[u], dhs[u], part);
+    }
     part = warp_sum(part);
     if (lane == 0) red[warp] = part;
   }
-  // stage <- v_new
-  for (int idx = tid; idx < C * V; idx += blockDim.x) {
-    const int i = idx / V, jj = idx - i * V;
-    stage[i * lds + jj] = vn[idx];
-  }
-  __syncthreads();
-  if (tid == 0) {
-    float s = 0.f;
-    for (int wv = 0; wv < (int)(blockDim.x >> 5); ++wv) s += red[wv];
-    dgam[C - 1] += L * s;
-  }
-  // ---- B: dP * Gamma ----
-  cta_gemm_r(C, C, [&](int i, int jj) { return lddo(i, jj); },
-             [&](int jj, int j) { return stage[j * lds + jj]; }, lo0,
-             [&](int i, int j) { return (i >= j) ? V : 0; },
-             [&](int i, int j, float acc) { X1[i * ldc + j] = acc * G[i * ldc + j]; });
-  __syncthreads();
-  // ---- C: stage <- k ; q k^T, k k^T, dq, partial dk ----
-  for (int idx = tid; idx < C * K; idx += blockDim.x) {
-    const int i = idx / K, kk = idx - i * K;
-    stage[i * lds + kk] = ldk(i, kk);
-  }
-  __syncthreads();
-  cta_gemm_r(C, C, [&](int i, int kk) { return ldq(i, kk); },
-             [&](int kk, int j) { return stage[j * lds + kk]; }, lo0,
-             [&](int i, int j) { return (i >= j) ? K : 0; },
-             [&](int i, int j, float acc) { X2[i * ldc + j] = acc * X1[i * ldc + j]; });
-  cta_gemm_r(C, C, [&](int i, int kk) { return stage[i * lds + kk]; },
-             [&](int kk, int j) { return stage[j * lds + kk]; }, lo0,
-             [&](int i, int j) { return (i > j) ? K : 0; },
-             [&](int i, int j, float acc) { X3[i * ldc + j] = acc; });
-  // row reductions that read dqi / dkt before dkt is overwritten
-  for (int i = warp; i < C; i += (blockDim.x >> 5)) {
-    float s1 = 0.f, s2 = 0.f;
-    for (int kk = lane; kk < K; kk += 32) {
-      s1 = fmaf(ldq(i, kk), dqi[i * K + kk], s1);
-      s2 = fmaf(stage[i * lds + kk], dkt[i * K + kk], s2);
-    }
-    s1 = warp_sum(s1);
-    s2 = warp_sum(s2);
-    if (lane == 0) {
-      rs1[i] = dd[i] * s1;  // dgam_i contribution from (q E(gam)) S
-      rs2[i] = rr[i] * s2;  // rho_i
-    }
-  }
-  __syncthreads();
-  if (tid < C) {
-    float s = 0.f;
-    for (int j = 0; j <= tid; ++j) s += X2[tid * ldc + j];
-    for (int m = tid; m < C; ++m) s -= X2[m * ldc + tid];
-    dgam[tid] += s + rs1[tid] - rs2[tid];
-  }
-  __syncthreads();
-  if (tid == 0) {
-    float s = 0.f;
-    for (int i = 0; i < C; ++i) s += rs2[i];
-    dgam[C - 1] += s;
-  }
-  __syncthreads();
-  // dq = E(gam) dqi + (dP Gamma) k      (final)
+  // ---- e = T^T dv_new, dv = beta e, e.v ----
   {
-    IO* dq = static_cast<IO*>(p.dq);
-    cta_gemm_r(C, K, [&](int i, int j) { return X1[i * ldc + j]; },
-               [&](int j, int kk) { return stage[j * lds + kk]; }, lo0,
-               [&](int i, int) { return i + 1; },
-               [&](int i, int kk, float acc) {
-                 if (i < imax) dq[row(i) * K + kk] = from_f32<IO>(fmaf(dd[i], dqi[i * K + kk], acc));
-               });
-  }
-  // dk partial = (dP Gamma)^T q + r dkt     (kept in dkt)
-  cta_gemm_r(C, K, [&](int i, int m) { return X1[m * ldc + i]; },
-             [&](int m, int kk) { return ldq(m, kk); },
-             [](int i, int) { return i; }, [C](int, int) { return C; },
-             [&](int i, int kk, float acc) { dkt[i * K + kk] = fmaf(rr[i], dkt[i * K + kk], acc); });
-  __syncthreads();
-  // ---- D: dT = du (v beta)^T + dw (k beta E(gam))^T  (strictly lower part is all that is used)
-  for (int idx = tid; idx < C * V; idx += blockDim.x) {
-    const int i = idx / V, jj = idx - i * V;
-    stage[i * lds + jj] = ldv(i, jj) * bet[i];
-  }
-  __syncthreads();
-  cta_gemm(C, C, V, [&](int i, int jj) { return dvn[i * V + jj]; },
-           [&](int jj, int j) { return stage[j * lds + jj]; },
-           [&](int i, int j, float acc) { X2[i * ldc + j] = acc; });
-  __syncthreads();
-  for (int idx = tid; idx < C * K; idx += blockDim.x) {
-    const int i = idx / K, kk = idx - i * K;
-    stage[i * lds + kk] = ldk(i, kk) * bet[i] * dd[i];
-  }
-  __syncthreads();
-  cta_gemm(C, C, K, [&](int i, int kk) { return dw[i * K + kk]; },
-           [&](int kk, int j) { return stage[j * lds + kk]; },
-           [&](int i, int j, float acc) { X2[i * ldc + j] += acc; });
-  __syncthreads();
-  // X4 = T^T dT ;  dA = (X4 T^T) strictly lower -> X2
-  cta_gemm_r(C, C, [&](int i, int m) { return Tm[m * ldc + i]; },
-             [&](int m, int j) { return X2[m * ldc + j]; },
-             [](int i, int) { return i; }, [C](int, int) { return C; },
-             [&](int i, int j, float acc) { X4[i * ldc + j] = acc; });
-  __syncthreads();
-  cta_gemm_r(C, C, [&](int i, int m) { return X4[i * ldc + m]; },
-             [&](int m, int j) { return Tm[j * ldc + m]; }, lo0,
-             [&](int i, int j) { return (i > j) ? j + 1 : 0; },
-             [&](int i, int j, float acc) { X2[i * ldc + j] = (i > j) ? acc : 0.f; });
-  // stage <- k again (X2 is not read until after the next barrier)
-  for (int idx = tid; idx < C * K; idx += blockDim.x) {
-    const int i = idx / K, kk = idx - i * K;
-    stage[i * lds + kk] = ldk(i, kk);
-  }
-  __syncthreads();
-  // ---- E: M = -dA Gamma ; Mb = beta_i M ; dbeta, dgam from A ; X4 <- Mb + Mb^T
-  for (int idx = tid; idx < C * C; idx += blockDim.x) {
-    const int i = idx / C, j = idx - i * C;
-    if (i > j) {
-      const float M = -X2[i * ldc + j] * G[i * ldc + j];
-      X2[i * ldc + j] = M * X3[i * ldc + j];  // M * (k_i.k_j)
-      const float mb = M * bet[i];
-      X4[i * ldc + j] = mb;
-      X4[j * ldc + i] = mb;
-    } else if (i == j) {
-      X2[i * ldc + i] = 0.f;
-      X4[i * ldc + i] = 0.f;
-    }
-  }
-  __syncthreads();
-  if (tid < C) {
-    float rs = 0.f, cs = 0.f;
-    for (int j = 0; j < tid; ++j) rs += X2[tid * ldc + j];
-    for (int m = tid + 1; m < C; ++m) cs += bet[m] * X2[m * ldc + tid];
-    dbet[tid] += rs;
-    dgam[tid] += bet[tid] * rs - cs;
-  }
-  // dv = beta (T^T du) ; dbeta += v . (T^T du)
-  {
+    float vd[4] = {0.f, 0.f, 0.f, 0.f};
     IO* dv = static_cast<IO*>(p.dv);
-    cta_gemm_rows(C, V, [&](int i, int m) { return Tm[m * ldc + i]; },
-                  [&](int m, int jj) { return dvn[m * V + jj]; },
-                  [](int i, int) { return i; }, [C](int, int) { return C; },
-                  [&](int i, int jj, float acc) {
-                    if (i < imax) dv[row(i) * V + jj] = from_f32<IO>(bet[i] * acc);
-                    return ldv(i, jj) * acc;
-                  },
-                  [&](int i, float s) { rs1[i] = s; });
+    auto product = [&](auto ng, int j0) {
+      constexpr int NG = decltype(ng)::value;
+      f2 acc[4][2 * NG];
+      clear(acc);
+      stream_nn<NG, 2>(acc, stage, R, Tm, NoA{}, [&](int m, int x) { return lddvn(m, j0 + x); });
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+          const int i = 4 * ty + r, j = j0 + 64 * g + 4 * tx;
+          const float4 x = acc4<NG>(acc, r, g);
+          if (i < C) st4(e + i * V, j, V, p.vecV, x);
+          if (i < imax) {
+            vd[r] = dot4(x, ldv(i, j), vd[r]);
+            st4(dv + row(i) * V, j, V, p.vecV, scale4(x, bet[i]));
+          }
+        }
+    };
+    if (V <= 64) product(std::integral_constant<int, 1>{}, 0);
+    else
+      for (int j0 = 0; j0 < V; j0 += 128) product(std::integral_constant<int, 2>{}, j0);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      vd[r] = row_sum(vd[r]);
+      if (tx == 0) dbe[4 * ty + r] = vd[r];
+    }
   }
-  // z = T^T dw ; dk = partial + beta E(gam) z + (Mb + Mb^T) k ; k.z row sums
+  // ---- dP Gamma ----
   {
-    IO* dk = static_cast<IO*>(p.dk);
-    const int nw = blockDim.x >> 5;
-    for (int i = warp; i < C; i += nw) {
-      float part = 0.f;
-      for (int kk = lane; kk < K; kk += 32) {
-        float z = 0.f;
-        for (int m = i; m < C; ++m) z = fmaf(Tm[m * ldc + i], dw[m * K + kk], z);
-        float acc = 0.f;
-        for (int jx = 0; jx < C; ++jx) acc = fmaf(X4[i * ldc + jx], stage[jx * lds + kk], acc);
-        if (i < imax) dk[row(i) * K + kk] = from_f32<IO>(dkt[i * K + kk] + bet[i] * dd[i] * z + acc);
-        part = fmaf(stage[i * lds + kk], z, part);
+    f2 acc[4][4];
+    clear(acc);
+    stream_nt(acc, stage, V, ldo, ldvn);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int i = ty + 16 * r, j = tx + 16 * x;
+        X1[i * LD + j] = (i >= j) ? sum2(acc[r][x]) * exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
       }
-      part = warp_sum(part);
-      if (lane == 0) rs2[i] = part;  // k_i . z_i
+  }
+  // ---- dq = E(gam) dO S0^T + dPG k ----
+  {
+    f2 acc[4][2 * NGK];
+    clear(acc);
+    stream_nn<NGK, 0>(acc, stage, V, nullptr, ldo, ldhs);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const f2 s = pack2(dd[4 * ty + r], dd[4 * ty + r]);
+#pragma unroll
+      for (int x = 0; x < 2 * NGK; ++x) acc[r][x] = mul2(acc[r][x], s);
+    }
+    stream_nn<NGK, 1>(acc, stage, R, X1, NoA{}, ldk);
+    IO* dq = static_cast<IO*>(p.dq);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = 4 * ty + r;
+      float qd = 0.f;
+#pragma unroll
+      for (int g = 0; g < NGK; ++g) {
+        const int j = 64 * g + 4 * tx;
+        const float4 x = acc4<NGK>(acc, r, g);
+        qd = dot4(x, ldq(i, j), qd);
+        if (i < imax) st4(dq + row(i) * K, j, K, p.vecK, x);
+      }
+      qd = row_sum(qd);
+      if (tx == 0) dg[i] = qd;
+    }
+  }
+  // ---- z = -e S0^T, k.z ----
+  {
+    f2 acc[4][2 * NGK];
+    clear(acc);
+    stream_nn<NGK, 0>(acc, stage, V, nullptr, lde, ldhs);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = 4 * ty + r;
+      float kz = 0.f;
+#pragma unroll
+      for (int g = 0; g < NGK; ++g) {
+        const int j = 64 * g + 4 * tx;
+        const float4 x = scale4(acc4<NGK>(acc, r, g), -1.f);
+        kz = dot4(x, ldk(i, j), kz);
+        if (i < C) st4(z + i * K, j, K, p.vecK, x);
+      }
+      kz = row_sum(kz);
+      if (tx == 0) {
+        dbe[i] += dd[i] * kz;
+        dg[i] += 2.f * bd[i] * kz;
+      }
+    }
+    __syncthreads();  // e and z are complete
+  }
+  // ---- Y = e (v beta)^T + z (k beta E(gam))^T, dA = tril(Y T^T, -1), M ----
+  {
+    f2 acc[4][4];
+    clear(acc);
+    stream_nt(acc, stage, V, lde, [&](int m, int x) { return scale4(ldv(m, x), bet[m]); });
+    stream_nt(acc, stage, K, ldz, [&](int m, int x) { return scale4(ldk(m, x), bd[m]); });
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) X2[(ty + 16 * r) * LD + tx + 16 * x] = sum2(acc[r][x]);
+    f2 kk[4][4];
+    clear(kk);
+    stream_nt(kk, stage, K, ldk, ldk);  // its barriers publish Y
+    clear(acc);
+    tile_nt(acc, X2, LD, Tm, LD, R);
+    __syncthreads();  // Y has been read
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = ty + 16 * r;
+      float sum = 0.f;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int j = tx + 16 * x;
+        if (i > j) {
+          const float M = -sum2(acc[r][x]) * exp_nonpos_precise(gam[i] - gam[j]);
+          sum = fmaf(M, sum2(kk[r][x]), sum);
+          X2[i * LD + j] = bet[i] * M;
+          X2[j * LD + i] = bet[i] * M;
+        } else if (i == j) {
+          X2[i * LD + i] = 0.f;
+        }
+      }
+      sum = row_sum(sum);
+      if (tx == 0) rs[i] = sum;
+    }
+  }
+  // ---- dk ----
+  {
+    f2 acc[4][2 * NGK];
+    clear(acc);
+    stream_nn<NGK, 0>(acc, stage, V, nullptr, ldvn, lddhs);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = 4 * ty + r;
+      const f2 s = pack2(rr[i], rr[i]);
+      float kp = 0.f;
+#pragma unroll
+      for (int g = 0; g < NGK; ++g) {
+        acc[r][2 * g] = mul2(acc[r][2 * g], s);
+        acc[r][2 * g + 1] = mul2(acc[r][2 * g + 1], s);
+        kp = dot4(acc4<NGK>(acc, r, g), ldk(i, 64 * g + 4 * tx), kp);
+      }
+      kp = row_sum(kp);
+      if (tx == 0) rho[i] = kp;
+    }
+    stream_nn<NGK, 2>(acc, stage, R, X1, NoA{}, ldq);
+    stream_nn<NGK, 1>(acc, stage, R, X2, NoA{}, ldk);
+    IO* dk = static_cast<IO*>(p.dk);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = 4 * ty + r;
+      float kd = 0.f;
+#pragma unroll
+      for (int g = 0; g < NGK; ++g) {
+        const int j = 64 * g + 4 * tx;
+        const float4 a = acc4<NGK>(acc, r, g), zz = ldz(i, j);
+        const float4 x = make_float4(fmaf(bd[i], zz.x, a.x), fmaf(bd[i], zz.y, a.y), fmaf(bd[i], zz.z, a.z), fmaf(bd[i], zz.w, a.w));
+        kd = dot4(x, ldk(i, j), kd);
+        if (i < imax) st4(dk + row(i) * K, j, K, p.vecK, x);
+      }
+      kd = row_sum(kd);
+      if (tx == 0) {
+        dbe[i] += rs[i];
+        dg[i] += 2.f * bet[i] * rs[i] - kd;
+      }
     }
   }
   __syncthreads();
-  if (tid < C) {
-    const float vdu = rs1[tid];
-    const float kz = rs2[tid];
-    dbet[tid] += vdu + dd[tid] * kz;
-    dgam[tid] += bet[tid] * dd[tid] * kz;
-  }
-  __syncthreads();
-  if (tid == 0) {  // dg = reverse cumulative sum of dgam within the chunk
-    float acc = 0.f;
-    for (int i = C - 1; i >= 0; --i) { acc += dgam[i]; dgam[i] = acc; }
+  if (tid < 32) {  // dg = reverse cumulative sum of dgam within the chunk: one warp, two rows per lane
+    float base = 0.f;
+    for (int x = 0; x < 8; ++x) base += red[x];
+    base = exp_nonpos_precise(gam[R - 1]) * base + warp_sum(rho[tid] + rho[tid + 32]);
+    const int ra = R - 1 - 2 * tid, rb = ra - 1;
+    float a = dg[ra], bq = dg[rb];
+    warp_rcumsum64(a, bq, tid);
+    __syncwarp();
+    dg[ra] = base + a;
+    dg[rb] = base + bq;
   }
   __syncthreads();
   if (tid < imax) {
-    p.dbeta[row(tid)] = dbet[tid];
-    float dg = dgam[tid];
+    p.dbeta[row(tid)] = dbe[tid];
+    float x = dg[tid];
     const float gin = p.gate[row(tid)];
     if (p.gate_is_log) {
-      if (gin < kLogGateFloor) dg = 0.f;
+      if (gin < kLogGateFloor) x = 0.f;
     } else {
-      dg = (gin > kGateFloor) ? dg / gin : 0.f;
+      x = (gin > kGateFloor) ? x / gin : 0.f;
     }
-    p.dgate[row(tid)] = dg;
+    p.dgate[row(tid)] = x;
   }
 }
 
@@ -636,7 +1233,7 @@ __global__ void __launch_bounds__(256) gdn_recurrent_fwd_kernel(GdnP p) {
 static size_t carve(GdnP& p, void* ws, bool bwd) {
   Carver cv(ws);
   const size_t nc = (size_t)p.B * p.H * p.n, C = p.C, K = p.K, V = p.V;
-  cv.take<int>(64);  // device status header (always zero on this path)
+  p.status = cv.take<int>(64);  // device status header (always zero on this path)
   p.gam = cv.take<float>(nc * C);
   p.Tm = cv.take<float>(nc * C * C);
   p.w = cv.take<float>(nc * C * K);
@@ -647,9 +1244,8 @@ static size_t carve(GdnP& p, void* ws, bool bwd) {
     p.vn = cv.take<float>(nc * C * V);
     p.dhs = cv.take<float>(nc * V * K);
     p.dvn = cv.take<float>(nc * C * V);
-    p.dqi = cv.take<float>(nc * C * K);
-    p.dw = cv.take<float>(nc * C * K);
-    p.dkt = cv.take<float>(nc * C * K);
+    p.e = cv.take<float>(nc * C * V);
+    p.z = cv.take<float>(nc * C * K);
   }
   return cv.bytes();
 }
@@ -686,30 +1282,59 @@ static mxb_status set_smem(KernelT kern, size_t bytes) {
   return MXB_OK;
 }
 
+// Rows can be moved four elements at a time where the width is a multiple of four and every tensor of that width is
+// aligned to four elements (the workspace always is).
+template <typename IO>
+static bool vec_ok(int width, std::initializer_list<const void*> tensors) {
+  uintptr_t bits = 0;
+  for (const void* t : tensors) bits |= reinterpret_cast<uintptr_t>(t);
+  return width % 4 == 0 && bits % (4 * sizeof(IO)) == 0;
+}
+
+template <typename IO, int KP>
+static mxb_status run_state_fwd(const GdnP& p, cudaStream_t st) {
+  constexpr int sm = state_fwd_smem<KP>();
+  if (set_smem(gdn_state_fwd_kernel<IO, KP>, sm) != MXB_OK) return MXB_ERR_CUDA;
+  MXB_LAUNCH("gdn_state_fwd_kernel", st, (gdn_state_fwd_kernel<IO, KP><<<dim3((p.V + 15) / 16, p.B * p.H), 256, sm, st>>>(p)));
+  return check_launch("gdn_state_fwd_kernel");
+}
+template <typename IO, int KP>
+static mxb_status run_state_bwd(const GdnP& p, cudaStream_t st) {
+  constexpr int sm = state_bwd_smem<KP>();
+  if (set_smem(gdn_state_bwd_kernel<IO, KP>, sm) != MXB_OK) return MXB_ERR_CUDA;
+  MXB_LAUNCH("gdn_state_bwd_kernel", st, (gdn_state_bwd_kernel<IO, KP><<<dim3((p.V + 15) / 16, p.B * p.H), 256, sm, st>>>(p)));
+  return check_launch("gdn_state_bwd_kernel");
+}
+template <typename IO, int NGK>
+static mxb_status run_chunk_bwd(const GdnP& p, cudaStream_t st) {
+  if (set_smem(gdn_chunk_bwd_kernel<IO, NGK>, kChunkF32Smem) != MXB_OK) return MXB_ERR_CUDA;
+  MXB_LAUNCH("gdn_chunk_bwd_kernel", st,
+             (gdn_chunk_bwd_kernel<IO, NGK><<<dim3(p.n, p.B * p.H), 256, kChunkF32Smem, st>>>(p)));
+  return check_launch("gdn_chunk_bwd_kernel");
+}
+
 template <typename IO>
 static mxb_status run_fwd(GdnP& p, bool chunked, cudaStream_t st) {
-  const int C = p.C, K = p.K, V = p.V;
-  dim3 gslab((V + 31) / 32, p.B * p.H);
+  const int K = p.K, V = p.V;
   if (!chunked) {
+    dim3 gslab((V + 31) / 32, p.B * p.H);
     size_t sm = sizeof(float) * (K * 33 + 2 * K + 512);
     if (set_smem(gdn_recurrent_fwd_kernel<IO>, sm) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_recurrent_fwd_kernel", st, (gdn_recurrent_fwd_kernel<IO><<<gslab, 256, sm, st>>>(p)));
     return check_launch("gdn_recurrent_fwd_kernel");
   }
-  size_t sm1 = sizeof(float) * (C * (K + 1) + 2 * C * (C + 1) + 3 * C);
-  if (set_smem(gdn_prep_kernel<IO>, sm1) != MXB_OK) return MXB_ERR_CUDA;
-  MXB_LAUNCH("gdn_prep_kernel", st, (gdn_prep_kernel<IO><<<dim3(p.n, p.B * p.H), 256, sm1, st>>>(p)));
+  p.vecK = vec_ok<IO>(K, {p.q, p.k, p.dq, p.dk});
+  p.vecV = vec_ok<IO>(V, {p.v, p.dO, p.dv});
+  if (set_smem(gdn_prep_kernel<IO>, kPrepF32Smem) != MXB_OK) return MXB_ERR_CUDA;
+  MXB_LAUNCH("gdn_prep_kernel", st, (gdn_prep_kernel<IO><<<dim3(p.n, p.B * p.H), 256, kPrepF32Smem, st>>>(p)));
   mxb_status s = check_launch("gdn_prep_kernel");
   if (s != MXB_OK) return s;
-  size_t sm2 = sizeof(float) * (K * 33 + 2 * C * 32 + 2 * C);
-  if (set_smem(gdn_state_fwd_kernel<IO>, sm2) != MXB_OK) return MXB_ERR_CUDA;
-  MXB_LAUNCH("gdn_state_fwd_kernel", st, (gdn_state_fwd_kernel<IO><<<gslab, 256, sm2, st>>>(p)));
-  return check_launch("gdn_state_fwd_kernel");
+  return K <= 64 ? run_state_fwd<IO, 64>(p, st) : run_state_fwd<IO, 128>(p, st);
 }
 
 template <typename IO>
 static mxb_status run_bwd(GdnP& p, bool recompute, cudaStream_t st) {
-  const int C = p.C, K = p.K, V = p.V;
+  const int K = p.K, V = p.V;
   p.save = 1;
   mxb_status s = MXB_OK;
   if (recompute) {
@@ -723,17 +1348,11 @@ static mxb_status run_bwd(GdnP& p, bool recompute, cudaStream_t st) {
     p.hT = keep_hT;
     if (s != MXB_OK) return s;
   }
-  dim3 gslab((V + 31) / 32, p.B * p.H);
-  size_t sm3 = sizeof(float) * (K * 33 + 3 * C * 32 + 2 * C);
-  if (set_smem(gdn_state_bwd_kernel<IO>, sm3) != MXB_OK) return MXB_ERR_CUDA;
-  MXB_LAUNCH("gdn_state_bwd_kernel", st, (gdn_state_bwd_kernel<IO><<<gslab, 256, sm3, st>>>(p)));
-  s = check_launch("gdn_state_bwd_kernel");
+  p.vecK = vec_ok<IO>(K, {p.q, p.k, p.dq, p.dk});
+  p.vecV = vec_ok<IO>(V, {p.v, p.dO, p.dv});
+  s = K <= 64 ? run_state_bwd<IO, 64>(p, st) : run_state_bwd<IO, 128>(p, st);
   if (s != MXB_OK) return s;
-  const int lds = (K > V ? K : V) + 1;
-  size_t sm4 = sizeof(float) * (C * lds + 6 * C * (C + 1) + 8 * C + 32);
-  if (set_smem(gdn_chunk_bwd_kernel<IO>, sm4) != MXB_OK) return MXB_ERR_CUDA;
-  MXB_LAUNCH("gdn_chunk_bwd_kernel", st, (gdn_chunk_bwd_kernel<IO><<<dim3(p.n, p.B * p.H), 256, sm4, st>>>(p)));
-  return check_launch("gdn_chunk_bwd_kernel");
+  return K <= 64 ? run_chunk_bwd<IO, 1>(p, st) : run_chunk_bwd<IO, 2>(p, st);
 }
 
 mxb_status gdn_simt_fwd(const mxb_gdn_desc* d, const void* q, const void* k, const void* v,
@@ -745,7 +1364,6 @@ mxb_status gdn_simt_fwd(const mxb_gdn_desc* d, const void* q, const void* k, con
   if (chunked) {
     p.save = (d->flags & MXB_GDN_SAVE_FOR_BWD) ? 1 : 0;
     carve(p, ws, p.save != 0);
-    if (cudaMemsetAsync(ws, 0, 256, st) != cudaSuccess) return MXB_ERR_CUDA;
   }
   return d->io_dtype == MXB_F32 ? run_fwd<float>(p, chunked, st) : run_fwd<__nv_bfloat16>(p, chunked, st);
 }
@@ -758,7 +1376,6 @@ mxb_status gdn_simt_bwd(const mxb_gdn_desc* d, const void* q, const void* k, con
   p.q = q; p.k = k; p.v = v; p.beta = beta; p.gate = gate; p.h0 = h0;
   p.dO = dO; p.dhT_in = dhT; p.dq = dq; p.dk = dk; p.dv = dv; p.dbeta = dbeta; p.dgate = dgate; p.dh0 = dh0;
   carve(p, ws, true);
-  if (cudaMemsetAsync(ws, 0, 256, st) != cudaSuccess) return MXB_ERR_CUDA;
   // saved intermediates exist only for the chunked forward
   const bool recompute = !(d->flags & MXB_GDN_BWD_USE_SAVED) || d->chunk <= 1;
   return d->io_dtype == MXB_F32 ? run_bwd<float>(p, recompute, st) : run_bwd<__nv_bfloat16>(p, recompute, st);
