@@ -16,7 +16,7 @@
 //
 // Kernels:
 //   gdn_prep_kernel        one CTA per (chunk, b*H+h): gam, T, w, u, P -> workspace
-//   gdn_state_fwd_kernel   one CTA per (16-column slab of Dv, b*H+h), sequential over
+//   gdn_state_fwd_kernel   one CTA per (slab of 4, 8 or 16 columns of Dv, b*H+h), sequential over
 //                          chunks: v_new, out, state (columns of Dv are independent)
 //   gdn_state_bwd_kernel   same mapping, reverse over chunks: dv_new, dS
 //   gdn_chunk_bwd_kernel   one CTA per chunk: dq, dk, dv, dbeta, dgate
@@ -29,6 +29,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace mxb {
 
@@ -50,6 +51,7 @@ struct GdnP {
   float *w;     // [C,K]
   float *u;     // [C,V]
   float *P;     // [C,C]
+  float *Pt;    // [C,C]  P^T (written when the forward saves for the backward)
   float *hs;    // [V,K]  state at chunk start, transposed
   float *vn;    // [C,V]
   float *dhs;   // [V,K]  dS at chunk end, transposed
@@ -134,43 +136,6 @@ __device__ __forceinline__ void st4(IO* row, int col, int n, bool vec, float4 x)
 __device__ __forceinline__ float4 scale4(float4 x, float s) { return make_float4(x.x * s, x.y * s, x.z * s, x.w * s); }
 __device__ __forceinline__ float dot4(float4 a, float4 b, float s) {
   return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
-}
-
-__device__ __forceinline__ void cp_async16(float* dst, const void* src, bool ok) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async4(float* dst, const void* src, bool ok) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 4 : 0)
-               : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Rows 0 .. 63 of n elements -> shared tile with the given pitch; rows past `rows` become zero.  float32 rows travel
-// asynchronously (the caller commits and waits), bf16 rows are widened on the way.  256 threads.
-template <typename IO, typename F>
-__device__ __forceinline__ void stage_rows(float* dst, int pitch, int rows, int n, bool vec, const IO* any, F rowptr) {
-  if constexpr (sizeof(IO) == 4) {
-    if (vec) {
-      const int n4 = n >> 2;
-      for (int u = threadIdx.x; u < R * 32; u += 256) {  // 32 units of four cover the widest row (128)
-        const int i = u >> 5, c4 = u & 31;
-        if (c4 < n4) cp_async16(dst + i * pitch + 4 * c4, i < rows ? rowptr(i) + 4 * c4 : any, i < rows);
-      }
-    } else {
-      for (int u = threadIdx.x; u < R * 128; u += 256) {
-        const int i = u >> 7, c = u & 127;
-        if (c < n) cp_async4(dst + i * pitch + c, i < rows ? rowptr(i) + c : any, i < rows);
-      }
-    }
-  } else {
-    for (int u = threadIdx.x; u < R * 32; u += 256) {
-      const int i = u >> 5, c = 4 * (u & 31);
-      if (c < n) *reinterpret_cast<float4*>(dst + i * pitch + c) = i < rows ? ld4(rowptr(i), c, n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
 }
 
 // acc[r][c] += sum_k A[ty + 16 r][k] B[tx + 16 c][k]: both operands contiguous along the contraction, the two halves
@@ -396,14 +361,23 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(GdnP p) {
       }
     clear(acc);
     stream_nt(acc, stage, K, ldq, ldk);
-    float* P = p.P + ci * C * C;
+    // P leaves row by row, and transposed for the backward; the tile goes over the streaming stage, which has been read
+    constexpr int LP = R + 1;
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
         const int i = ty + 16 * r, j = tx + 16 * x;
-        if (i < C && j < C) P[i * C + j] = (i >= j) ? sum2(acc[r][x]) * exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
+        stage[i * LP + j] = (i >= j) ? sum2(acc[r][x]) * exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
       }
+    __syncthreads();
+    for (int u = tid; u < R * R; u += 256) {
+      const int i = u >> 6, j = u & 63;
+      if (i < C && j < C) {
+        p.P[ci * C * C + i * C + j] = stage[i * LP + j];
+        if (p.save) p.Pt[ci * C * C + i * C + j] = stage[j * LP + i];
+      }
+    }
   }
   // T = (I - A)^-1 in place: the two 32 x 32 diagonal blocks by forward substitution (thread = block and column, the
   // column in registers), then the off-diagonal block T21 = T22 (A21 T11) as two 32^3 products over all threads.
@@ -477,425 +451,411 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(GdnP p) {
   else product(std::integral_constant<int, 2>{}, K, p.vecK, p.w, ldk, bd);
 }
 
-// ------------------------------------------------------------ state forward
-// The sequential pass: latency and arithmetic of one chunk, chunk after chunk.  A CTA owns 16 columns of the state, so
-// that a few (batch, head) pairs still spread over many SMs.  The tiles of the next chunk travel (cp.async) as soon as
-// their buffer has been read: w and q behind the first barrier, k and P behind the second.
-//   [w;q] S      thread = rows ty, ty + 32 of both x columns tx, tx + 8
-//   P v_new      the same rows and columns
-//   (k r)^T v_new  thread = KT state rows x 2 columns, the state itself stays in registers
-template <int KP>
-constexpr int state_fwd_smem() {
-  return 4 * (192 * (KP + 4) + simt::R * simt::LD + 16 * (KP + 4) + 16 * simt::LD + simt::R * 32 + 2 * (2 * simt::R + 4));
-}
-template <typename IO, int KP>
-__global__ void __launch_bounds__(256) gdn_state_fwd_kernel(GdnP p) {
+// ------------------------------------------------------------ state passes
+// The sequential passes: one chunk after the other, so the time of a chunk is what counts.  A CTA owns W columns of
+// the state (columns are independent), W as small as still fits the CTAs on the SMs at once.  What bounds a chunk is
+// the shared-memory bandwidth of the products, so every thread computes 4 x 4 outputs (eight loaded values per sixteen
+// multiply-adds) over a part of the contraction, and the parts (32 / W of them for 128 rows) are added through shared
+// memory in a fixed order.  One output per thread and 16-column slabs, operands by one cp.async per 16 bytes:
+// 8.2 us a chunk at Dk = 64 (6.6 k of 16.4 k cycles went into issuing the copies); now every row is one bulk copy,
+// issued by one thread as soon as the tile it replaces has been read.
+//
+// A thread's 4 x 4 outputs of a product along rows: rows ty + NR r, columns tx + NCG c.
+template <int W, int NR>
+struct SlabMap {
+  static constexpr int NCG = W / 4;             // column groups
+  static constexpr int PER = NR * NCG;          // threads that share a part of the contraction
+  static constexpr int PITCH = W == 16 ? 20 : W + 1;  // of a row of partial sums (few bank conflicts both ways)
+};
+// part[s][ty + NR r][tx + NCG c] = sum over the s-th part of the contraction of A[row][k] B[col][k]; `t` < SP * PER
+template <int W, int NR, int SP>
+__device__ __forceinline__ void slab_nt(float* part, const float* A, int lda, const float* B, int ldb, int kd, int t) {
   using namespace simt;
-  constexpr int LK = KP + 4, KT = KP / 32;
+  using M = SlabMap<W, NR>;
+  const int tx = t % M::NCG, ty = (t / M::NCG) % NR, s = t / M::PER;
+  const int len = kd / SP, k0 = s * len;
+  f2 acc[4][4];
+  clear(acc);
+  const float* a0 = A + ty * lda + k0;
+  const float* b0 = B + tx * ldb + k0;
+#pragma unroll 2
+  for (int k = 0; k < len; k += 4) {
+    ulonglong2 a[4], b[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) a[r] = lds2x2(a0 + NR * r * lda + k);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) b[c] = lds2x2(b0 + M::NCG * c * ldb + k);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        fma2(acc[r][c], a[r].x, b[c].x);
+        fma2(acc[r][c], a[r].y, b[c].y);
+      }
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      part[s * 4 * NR * M::PITCH + (ty + NR * r) * M::PITCH + tx + M::NCG * c] = sum2(acc[r][c]);
+}
+// part[s][4 tx + c][kk] = sum over the s-th part of the 64 rows i of A[i][kk] B[i][4 tx + c]; t < 128
+template <int W, int KP>
+__device__ __forceinline__ void slab_tn(float* part, const float* A, const float* B, int t) {
+  using namespace simt;
+  constexpr int LK = KP + 4, NCG = W / 4, PER = NCG * (KP / 4), SP = 128 / PER, LEN = R / SP;
+  const int tx = t % NCG, kg = (t / NCG) % (KP / 4), s = t / PER;
+  f2 acc[4][2];  // [column][pair of state rows]
+  clear(acc);
+  const float* a0 = A + s * LEN * LK + 4 * kg;
+  const float* b0 = B + s * LEN * W + 4 * tx;
+#pragma unroll 4
+  for (int i = 0; i < LEN; ++i) {
+    const ulonglong2 a = lds2x2(a0 + i * LK);
+    const float4 b = *reinterpret_cast<const float4*>(b0 + i * W);
+    const f2 bb[4] = {pack2(b.x, b.x), pack2(b.y, b.y), pack2(b.z, b.z), pack2(b.w, b.w)};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      fma2(acc[c][0], a.x, bb[c]);
+      fma2(acc[c][1], a.y, bb[c]);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    *reinterpret_cast<ulonglong2*>(part + (s * W + 4 * tx + c) * LK + 4 * kg) = make_ulonglong2(acc[c][0], acc[c][1]);
+}
+constexpr int kSlabScalars = 2 * simt::R + 4;  // E(gam), E(gam_last - gam), E(gam_last)
+
+// A tile of 64 rows of n elements, rows past `rows` zero, by the threads themselves (bf16 rows are widened).
+template <typename IO, typename F>
+__device__ __forceinline__ void slab_copy(float* dst, int pitch, int rows, int n, int vec, F rowptr) {
+  for (int u = threadIdx.x; u < simt::R * 32; u += 256) {
+    const int i = u >> 5, c = 4 * (u & 31);
+    if (c < n)
+      *reinterpret_cast<float4*>(dst + i * pitch + c) = i < rows ? simt::ld4(rowptr(i), c, n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+// The same by one bulk copy per row, completing on `bar`, where rows are float32 and 16-byte multiples (vec); thread
+// t0 + i issues row i.  The caller has told the barrier how many bytes to expect.
+template <typename IO>
+__device__ __forceinline__ bool bulk_rows(int vec) { return sizeof(IO) == 4 && vec; }
+template <typename IO, typename F>
+__device__ __forceinline__ void slab_load(float* dst, int pitch, int rows, int n, int vec, uint64_t* bar, int t0, F rowptr) {
+  if (!bulk_rows<IO>(vec)) return slab_copy<IO>(dst, pitch, rows, n, vec, rowptr);
+  const int i = threadIdx.x - t0;
+  if (i >= 0 && i < rows) tc::bulk_load(tc::smem_u32(dst + i * pitch), rowptr(i), n * 4, bar);
+  if (rows < simt::R)
+    for (int u = threadIdx.x; u < (simt::R - rows) * 32; u += 256)
+      if (4 * (u & 31) < n) *reinterpret_cast<float4*>(dst + (rows + (u >> 5)) * pitch + 4 * (u & 31)) = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+// A [C][C] matrix of the workspace into a [64][LD] tile (what lies outside stays zero from the start).
+__device__ __forceinline__ void slab_square(float* dst, const float* src, int C, bool bulk, uint64_t* bar, int t0) {
+  if (bulk) {
+    const int i = threadIdx.x - t0;
+    if (i >= 0 && i < simt::R) tc::bulk_load(tc::smem_u32(dst + i * simt::LD), src + i * simt::R, simt::R * 4, bar);
+  } else {
+    for (int u = threadIdx.x; u < C * C; u += 256) dst[(u / C) * simt::LD + u % C] = src[u];
+  }
+}
+
+// Floats of the partial sums: 128 rows of W columns in 32 / W parts (the products of the second step need less).
+template <int W>
+constexpr int kSlabPart = 32 / W * 128 * SlabMap<W, 16>::PITCH;
+template <int W, int KP>
+constexpr int state_fwd_smem() {
+  return 4 * (192 * (KP + 4) + simt::R * simt::LD + W * (KP + 4) + W * simt::LD + simt::R * W + 2 * kSlabScalars + kSlabPart<W>) + 64;
+}
+template <int W, int KP>
+constexpr int state_bwd_smem() {
+  return 4 * (192 * (KP + 4) + simt::R * simt::LD + W * (KP + 4) + W * simt::LD + 2 * simt::R * W + 2 * kSlabScalars + kSlabPart<W>) + 64;
+}
+// Decay factors of one chunk from its in-chunk cumulative log decay g (lane's own) and gl (the last).
+__device__ __forceinline__ void slab_scalars(float* s, float g, float gl) {
+  const int tid = threadIdx.x;
+  if (tid < simt::R) {
+    s[tid] = exp_nonpos_precise(g);
+    s[simt::R + tid] = exp_nonpos_precise(gl - g);
+    if (tid == 0) s[2 * simt::R] = exp_nonpos_precise(gl);
+  }
+}
+// State slab (transposed, pitch LK) <-> [K][V] tensor columns j0 .. j0+W-1.
+template <int W, int KP>
+__device__ __forceinline__ void slab_state_in(float* St, const float* src, int K, int V, int j0) {
+  for (int u = threadIdx.x; u < W * KP; u += 256) {
+    const int j = u % W, kk = u / W;
+    St[j * (KP + 4) + kk] = (src && kk < K && j0 + j < V) ? src[(size_t)kk * V + j0 + j] : 0.f;
+  }
+}
+template <int W, int KP>
+__device__ __forceinline__ void slab_state_out(const float* St, float* dst, int K, int V, int j0) {
+  for (int u = threadIdx.x; u < W * KP; u += 256) {
+    const int j = u % W, kk = u / W;
+    if (kk < K && j0 + j < V) dst[(size_t)kk * V + j0 + j] = St[j * (KP + 4) + kk];
+  }
+}
+// The same slab as rows of the transposed states [V][K] kept per chunk.
+template <int W, int KP>
+__device__ __forceinline__ void slab_state_keep(const float* St, float* dst, int K, int V, int vec, int j0) {
+  for (int u = threadIdx.x; u < W * KP / 4; u += 256) {
+    const int j = u / (KP / 4), kk = 4 * (u % (KP / 4));
+    if (j0 + j < V) simt::st4(dst + (size_t)(j0 + j) * K, kk, K, vec, *reinterpret_cast<const float4*>(St + j * (KP + 4) + kk));
+  }
+}
+// State <- L state + partial sums (NP of them), and the copy kept for chunk kernels where `keep` is not null.
+template <int W, int KP, int NP>
+__device__ __forceinline__ void slab_state_step(float* St, const float* part, float L, float* keep, int K, int V, int vec, int j0) {
+  constexpr int LK = KP + 4;
+  for (int u = threadIdx.x; u < W * KP / 4; u += 256) {
+    const int j = u / (KP / 4), kk = 4 * (u % (KP / 4));
+    float4* own = reinterpret_cast<float4*>(St + j * LK + kk);
+    float4 x = simt::scale4(*own, L);
+#pragma unroll
+    for (int s = 0; s < NP; ++s) {
+      const float4 t = *reinterpret_cast<const float4*>(part + (s * W + j) * LK + kk);
+      x = make_float4(x.x + t.x, x.y + t.y, x.z + t.z, x.w + t.w);
+    }
+    *own = x;
+    if (keep && j0 + j < V) simt::st4(keep + (size_t)(j0 + j) * K, kk, K, vec, x);
+  }
+}
+template <int W>
+__device__ __forceinline__ float slab_sum(const float* part, int rows, int row, int col) {
+  float v = 0.f;
+#pragma unroll
+  for (int s = 0; s < 32 / W; ++s) v += part[(s * rows + row) * SlabMap<W, 16>::PITCH + col];
+  return v;
+}
+
+// v_new = u - w S;  o = E(gam) (q S) + P v_new;  S <- E(gam_last) S + (k r)^T v_new
+template <typename IO, int W, int KP>
+__global__ void __launch_bounds__(256, 1) gdn_state_fwd_kernel(GdnP p) {
+  using namespace simt;
+  constexpr int LK = KP + 4, SP = 32 / W, SPK = 2048 / (W * KP), PITCH = SlabMap<W, 16>::PITCH;
   extern __shared__ __align__(16) float smem[];
   float* Wq = smem;              // [128][LK] w rows, then q rows
   float* Ks = Wq + 128 * LK;     // [64][LK]
   float* Ps = Ks + R * LK;       // [64][LD]
-  float* St = Ps + R * LD;       // [16][LK]  S^T
-  float* Vt = St + 16 * LK;      // [16][LD]  v_new^T
-  float* Vd = Vt + 16 * LD;      // [64][32]  r_i v_new, every element twice
-  float* sc = Vd + R * 32;       // x2 [64] E(gam), [64] E(gam_last - gam), E(gam_last)
-  constexpr int kSc = 2 * R + 4;
+  float* St = Ps + R * LD;       // [W][LK]  S^T
+  float* Vt = St + W * LK;       // [W][LD]  v_new^T
+  float* Vr = Vt + W * LD;       // [64][W]  r_i v_new
+  float* sc = Vr + R * W;        // x2 decay factors of a chunk
+  float* part = sc + 2 * kSlabScalars;
+  float* partK = part + SP * R * PITCH;  // beside the 64 rows of P v_new
+  uint64_t* bar = reinterpret_cast<uint64_t*>(part + kSlabPart<W>);  // [0] w, q; [1] k, P
   const int C = p.C, K = p.K, V = p.V;
-  const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3, kk0 = ty * KT;
-  const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H, j0 = blockIdx.x * 16;
+  const int tid = threadIdx.x;
+  const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H, j0 = blockIdx.x * W;
   const IO* q = static_cast<const IO*>(p.q);
   const IO* k = static_cast<const IO*>(p.k);
   IO* out = static_cast<IO*>(p.out);
   auto row = [&](int c, int i) { return ((size_t)(b * p.T + c * C + i) * p.H + h); };
+  const bool bulkK = bulk_rows<IO>(p.vecK), bulkP = C == R;
   auto load_wq = [&](int c) {
-    if (c < p.n) {
-      const float* w = p.w + ((size_t)bh * p.n + c) * C * K;
-      stage_rows(Wq, LK, C, K, p.vecK, w, [&](int i) { return w + i * K; });
-      stage_rows(Wq + R * LK, LK, min(C, p.T - c * C), K, p.vecK, q, [&](int i) { return q + row(c, i) * K; });
-    }
-    cp_commit();
+    if (c >= p.n) return;
+    const float* w = p.w + ((size_t)bh * p.n + c) * C * K;
+    const int rows = min(C, p.T - c * C);
+    if (bulkK && tid == 0) tc::mbar_expect_tx(bar, (C + rows) * K * 4);
+    if (bulkK) slab_load<float>(Wq, LK, C, K, p.vecK, bar, 0, [&](int i) { return w + i * K; });
+    else slab_copy<float>(Wq, LK, C, K, p.vecK, [&](int i) { return w + i * K; });
+    slab_load<IO>(Wq + R * LK, LK, rows, K, p.vecK, bar, 64, [&](int i) { return q + row(c, i) * K; });
   };
   auto load_kp = [&](int c) {
-    if (c < p.n) {
-      stage_rows(Ks, LK, min(C, p.T - c * C), K, p.vecK, k, [&](int i) { return k + row(c, i) * K; });
-      const float* P = p.P + ((size_t)bh * p.n + c) * C * C;
-      if (C == R) {
-        for (int u = tid; u < R * 16; u += 256) cp_async16(Ps + (u >> 4) * LD + 4 * (u & 15), P + 4 * u, true);
-      } else {
-        for (int u = tid; u < C * C; u += 256) cp_async4(Ps + (u / C) * LD + u % C, P + u, true);
-      }
-    }
-    cp_commit();
+    if (c >= p.n) return;
+    const float* P = p.P + ((size_t)bh * p.n + c) * C * C;
+    const int rows = min(C, p.T - c * C);
+    if ((bulkK || bulkP) && tid == 0) tc::mbar_expect_tx(bar + 1, (bulkK ? rows * K * 4 : 0) + (bulkP ? R * R * 4 : 0));
+    slab_load<IO>(Ks, LK, rows, K, p.vecK, bar + 1, 128, [&](int i) { return k + row(c, i) * K; });
+    slab_square(Ps, P, C, bulkP, bar + 1, 192);
   };
-  auto scalars = [&](int c) {  // decay factors of chunk c, buffer c & 1
-    float* s = sc + (c & 1) * kSc;
-    if (tid < R) {
-      const float* gam = p.gam + ((size_t)bh * p.n + c) * C;
-      const float gl = gam[C - 1], g = tid < C ? gam[tid] : gl;
-      s[tid] = exp_nonpos_precise(g);
-      s[R + tid] = exp_nonpos_precise(gl - g);
-      if (tid == 0) s[2 * R] = exp_nonpos_precise(gl);
-    }
-  };
-  for (int u = tid; u < 192 * LK; u += 256) Wq[u] = 0.f;  // rows and columns that no copy reaches
-  for (int u = tid; u < R * LD; u += 256) Ps[u] = 0.f;
-  f2 S[2][KT / 2];  // state rows kk0 .. , columns j0 + 2 tx and + 1
-#pragma unroll
-  for (int y = 0; y < 2; ++y)
-#pragma unroll
-    for (int x = 0; x < KT / 2; ++x) {
-      const int jv = j0 + 2 * tx + y, kk = kk0 + 2 * x;
-      const float* src = p.h0 ? p.h0 + ((size_t)bh * K + kk) * V + jv : nullptr;
-      S[y][x] = pack2(src && jv < V && kk < K ? src[0] : 0.f, src && jv < V && kk + 1 < K ? src[V] : 0.f);
-    }
-  scalars(0);
+  if (tid == 0) {
+    tc::mbar_init(bar, 1);
+    tc::mbar_init(bar + 1, 1);
+    tc::mbar_fence_init();
+  }
+  for (int u = tid; u < 192 * LK + R * LD; u += 256) Wq[u] = 0.f;  // rows and columns that no copy reaches
+  slab_state_in<W, KP>(St, p.h0 ? p.h0 + (size_t)bh * K * V : nullptr, K, V, j0);
+  const float* gam = p.gam + (size_t)bh * p.n * C;
+  float gl = gam[C - 1], g = tid < C ? gam[tid] : gl;
+  slab_scalars(sc, g, gl);
+  tc::fence_async_smem();
   __syncthreads();
   load_wq(0);
   load_kp(0);
-#pragma unroll
-  for (int y = 0; y < 2; ++y)
-#pragma unroll
-    for (int x = 0; x < KT / 2; ++x) *reinterpret_cast<f2*>(St + (2 * tx + y) * LK + kk0 + 2 * x) = S[y][x];
+  if (p.save) slab_state_keep<W, KP>(St, p.hs + (size_t)bh * p.n * V * K, K, V, p.vecK, j0);
 
+  bool ok = true;
   for (int c = 0; c < p.n; ++c) {
     const size_t ci = (size_t)bh * p.n + c;
-    const float* s = sc + (c & 1) * kSc;
+    const float* s = sc + (c & 1) * kSlabScalars;
     const int imax = min(C, p.T - c * C);
-    if (p.save) {  // state at chunk start, transposed [V][K]
+    float un[W / 4], oq[W / 4];  // this thread's elements of u (fetched ahead of their use) and of E(gam) q S
 #pragma unroll
-      for (int y = 0; y < 2; ++y)
-#pragma unroll
-        for (int x = 0; x < KT / 2; ++x) {
-          const int jv = j0 + 2 * tx + y, kk = kk0 + 2 * x;
-          const float2 t = unpack2(S[y][x]);
-          float* dst = p.hs + (ci * V + jv) * K + kk;
-          if (jv < V && kk < K) dst[0] = t.x;
-          if (jv < V && kk + 1 < K) dst[1] = t.y;
-        }
+    for (int x = 0; x < W / 4; ++x) {
+      const int i = (tid + 256 * x) / W, jv = j0 + (tid + 256 * x) % W;
+      un[x] = (i < C && jv < V) ? p.u[(ci * C + i) * V + jv] : 0.f;
     }
-    float un[2][2];
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-      for (int y = 0; y < 2; ++y) {
-        const int i = ty + 32 * r, jv = j0 + tx + 8 * y;
-        un[r][y] = (i < C && jv < V) ? p.u[(ci * C + i) * V + jv] : 0.f;
-      }
-    cp_wait<1>();
-    __syncthreads();  // w, q and the state are in place
-    f2 acc[4][2];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = 0ull;
-#pragma unroll 4
-    for (int x = 0; x < KP; x += 4) {
-      const ulonglong2 s0 = lds2x2(St + tx * LK + x), s1 = lds2x2(St + (tx + 8) * LK + x);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const ulonglong2 a = lds2x2(Wq + (ty + 32 * r) * LK + x);
-        fma2(acc[r][0], a.x, s0.x);
-        fma2(acc[r][1], a.x, s1.x);
-        fma2(acc[r][0], a.y, s0.y);
-        fma2(acc[r][1], a.y, s1.y);
-      }
+    if (c + 1 < p.n) {
+      gl = gam[(c + 2) * C - 1];
+      g = tid < C ? gam[(c + 1) * C + tid] : gl;
     }
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-      for (int y = 0; y < 2; ++y) {  // v_new = u - w S
-        const int i = ty + 32 * r, j = tx + 8 * y;
-        const float val = un[r][y] - sum2(acc[r][y]);
-        Vt[j * LD + i] = val;
-        const float vr = val * s[R + i];
-        *reinterpret_cast<f2*>(Vd + i * 32 + 2 * j) = pack2(vr, vr);
-        if (p.save && i < C && j0 + j < V) p.vn[(ci * C + i) * V + j0 + j] = val;
-      }
-    cp_wait<0>();
-    __syncthreads();  // v_new, k and P are in place; w and q have been read
+    if (bulkK) ok = tc::mbar_wait(bar, c & 1);
+    ok = __syncthreads_and(ok);  // w, q, the state and the decay factors are in place
+    if (!ok) break;
+    slab_nt<W, 32, SP>(part, Wq, LK, St, LK, KP, tid);
+    tc::fence_async_smem();
+    __syncthreads();
     load_wq(c + 1);
-    {  // o = E(gam) (q S) + P v_new
-      f2 o[2][2];
-      o[0][0] = o[0][1] = o[1][0] = o[1][1] = 0ull;
-#pragma unroll 4
-      for (int m = 0; m < 32; m += 4) {
-        const ulonglong2 v0 = lds2x2(Vt + tx * LD + m), v1 = lds2x2(Vt + (tx + 8) * LD + m);
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          const ulonglong2 a = lds2x2(Ps + (ty + 32 * r) * LD + m);
-          fma2(o[r][0], a.x, v0.x);
-          fma2(o[r][1], a.x, v1.x);
-          fma2(o[r][0], a.y, v0.y);
-          fma2(o[r][1], a.y, v1.y);
-        }
-      }
-#pragma unroll 4
-      for (int m = 32; m < 64; m += 4) {  // P is lower triangular: only the upper rows have these columns
-        const ulonglong2 v0 = lds2x2(Vt + tx * LD + m), v1 = lds2x2(Vt + (tx + 8) * LD + m);
-        const ulonglong2 a = lds2x2(Ps + (ty + 32) * LD + m);
-        fma2(o[1][0], a.x, v0.x);
-        fma2(o[1][1], a.x, v1.x);
-        fma2(o[1][0], a.y, v0.y);
-        fma2(o[1][1], a.y, v1.y);
-      }
-#pragma unroll
-      for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int y = 0; y < 2; ++y) {
-          const int i = ty + 32 * r, jv = j0 + tx + 8 * y;
-          if (i < imax && jv < V) out[row(c, i) * V + jv] = from_f32<IO>(fmaf(s[i], sum2(acc[2 + r][y]), sum2(o[r][y])));
-        }
+    for (int x = 0; x < W / 4; ++x) {
+      const int i = (tid + 256 * x) / W, j = (tid + 256 * x) % W;
+      const float val = un[x] - slab_sum<W>(part, 128, i, j);
+      oq[x] = s[i] * slab_sum<W>(part, 128, R + i, j);
+      Vt[j * LD + i] = val;
+      Vr[i * W + j] = val * s[R + i];
+      if (p.save && i < C && j0 + j < V) p.vn[(ci * C + i) * V + j0 + j] = val;
     }
-    {  // S <- S E(gam_last) + (k r)^T v_new
-      const f2 L = pack2(s[2 * R], s[2 * R]);
-#pragma unroll
-      for (int y = 0; y < 2; ++y)
-#pragma unroll
-        for (int x = 0; x < KT / 2; ++x) S[y][x] = mul2(S[y][x], L);
-#pragma unroll 8
-      for (int i = 0; i < R; ++i) {
-        const ulonglong2 vv = lds2x2(Vd + i * 32 + 4 * tx);
-#pragma unroll
-        for (int x = 0; x < KT / 2; ++x) {
-          const f2 kx = *reinterpret_cast<const f2*>(Ks + i * LK + kk0 + 2 * x);
-          fma2(S[0][x], kx, vv.x);
-          fma2(S[1][x], kx, vv.y);
-        }
-      }
-    }
-    if (c + 1 < p.n) scalars(c + 1);
-#pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-      for (int x = 0; x < KT / 2; ++x) *reinterpret_cast<f2*>(St + (2 * tx + y) * LK + kk0 + 2 * x) = S[y][x];
-    __syncthreads();  // k, P and v_new have been read
+    if (bulkK || bulkP) ok = tc::mbar_wait(bar + 1, c & 1);
+    ok = __syncthreads_and(ok);  // v_new, k and P are in place
+    if (!ok) break;
+    if (tid < 128) slab_nt<W, 16, SP>(part, Ps, LD, Vt, LD, R, tid);
+    else slab_tn<W, KP>(partK, Ks, Vr, tid - 128);
+    tc::fence_async_smem();
+    __syncthreads();
     load_kp(c + 1);
+#pragma unroll
+    for (int x = 0; x < W / 4; ++x) {
+      const int i = (tid + 256 * x) / W, j = (tid + 256 * x) % W;
+      if (i < imax && j0 + j < V) out[row(c, i) * V + j0 + j] = from_f32<IO>(oq[x] + slab_sum<W>(part, R, i, j));
+    }
+    slab_state_step<W, KP, SPK>(St, partK, s[2 * R], p.save && c + 1 < p.n ? p.hs + (ci + 1) * V * K : nullptr, K, V, p.vecK, j0);
+    slab_scalars(sc + ((c + 1) & 1) * kSlabScalars, g, gl);
   }
-  if (p.hT) {
-#pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-      for (int x = 0; x < KT / 2; ++x) {
-        const int jv = j0 + 2 * tx + y, kk = kk0 + 2 * x;
-        const float2 t = unpack2(S[y][x]);
-        float* dst = p.hT + ((size_t)bh * K + kk) * V + jv;
-        if (jv < V && kk < K) dst[0] = t.x;
-        if (jv < V && kk + 1 < K) dst[V] = t.y;
-      }
+  if (!ok && tid == 0) atomicExch(p.status, 5);
+  if (p.hT && ok) {
+    __syncthreads();
+    slab_state_out<W, KP>(St, p.hT + (size_t)bh * K * V, K, V, j0);
   }
 }
 
-// ----------------------------------------------------------- state backward
-// The same slabs in reverse:  dv_new = P^T dO + r (k dS);  dS <- E(gam_last) dS + (q E(gam))^T dO - w^T dv_new.
-// k and P of the next chunk travel behind the first barrier, q and w behind the second.
-template <int KP>
-constexpr int state_bwd_smem() {
-  return 4 * (192 * (KP + 4) + simt::R * simt::LD + 16 * (KP + 4) + 16 * simt::LD + 3 * simt::R * 32 + 2 * (2 * simt::R + 4));
-}
-template <typename IO, int KP>
-__global__ void __launch_bounds__(256) gdn_state_bwd_kernel(GdnP p) {
+// dv_new = P^T dO + r (k dS);  dS <- E(gam_last) dS + (q E(gam))^T dO - w^T dv_new, chunks in reverse.
+template <typename IO, int W, int KP>
+__global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p) {
   using namespace simt;
-  constexpr int LK = KP + 4, KT = KP / 32;
+  constexpr int LK = KP + 4, SP = 32 / W, SPK = 2048 / (W * KP), PITCH = SlabMap<W, 16>::PITCH;
   extern __shared__ __align__(16) float smem[];
   float* Ks = smem;              // [64][LK]
   float* Qs = Ks + R * LK;       // [64][LK]
   float* Ws = Qs + R * LK;       // [64][LK]
   float* Pt = Ws + R * LK;       // [64][LD]  P^T
-  float* St = Pt + R * LD;       // [16][LK]  dS^T
-  float* Ot = St + 16 * LK;      // [16][LD]  dO^T
-  float* Vd = Ot + 16 * LD;      // [64][32]  -dv_new, every element twice
-  float* Od = Vd + R * 32;       // x2 [64][32]  E(gam_i) dO, every element twice
-  float* sc = Od + 2 * R * 32;   // x2 [64] E(gam), [64] E(gam_last - gam), E(gam_last)
-  constexpr int kSc = 2 * R + 4;
+  float* St = Pt + R * LD;       // [W][LK]   dS^T
+  float* Ot = St + W * LK;       // [W][LD]   dO^T
+  float* Od = Ot + W * LD;       // [64][W]   E(gam_i) dO
+  float* Vn = Od + R * W;        // [64][W]   -dv_new
+  float* sc = Vn + R * W;        // x2 decay factors of a chunk
+  float* part = sc + 2 * kSlabScalars;
+  float* partP = part + SP * R * PITCH;        // P^T dO beside k dS
+  float* partW = part + SPK * W * LK;          // w^T dv_new beside q^T dO
+  uint64_t* bar = reinterpret_cast<uint64_t*>(part + kSlabPart<W>);  // [0] k, P^T; [1] q, w
+  static_assert(2 * SPK * W * LK <= kSlabPart<W>, "partial sums of the second step");
   const int C = p.C, K = p.K, V = p.V;
-  const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3, kk0 = ty * KT;
-  const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H, j0 = blockIdx.x * 16;
+  const int tid = threadIdx.x;
+  const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H, j0 = blockIdx.x * W;
   const IO* q = static_cast<const IO*>(p.q);
   const IO* k = static_cast<const IO*>(p.k);
   const IO* dO = static_cast<const IO*>(p.dO);
   auto row = [&](int c, int i) { return ((size_t)(b * p.T + c * C + i) * p.H + h); };
+  const bool bulkK = bulk_rows<IO>(p.vecK), bulkP = C == R;
   auto load_kp = [&](int c) {
-    if (c >= 0) {
-      stage_rows(Ks, LK, min(C, p.T - c * C), K, p.vecK, k, [&](int i) { return k + row(c, i) * K; });
-      const float* P = p.P + ((size_t)bh * p.n + c) * C * C;
-      for (int u = tid; u < C * C; u += 256) {
-        const int m = C == R ? u >> 6 : u / C, i = u - m * C;
-        cp_async4(Pt + i * LD + m, P + u, true);
-      }
-    }
-    cp_commit();
+    if (c < 0) return;
+    const float* P = p.Pt + ((size_t)bh * p.n + c) * C * C;
+    const int rows = min(C, p.T - c * C);
+    if ((bulkK || bulkP) && tid == 0) tc::mbar_expect_tx(bar, (bulkK ? rows * K * 4 : 0) + (bulkP ? R * R * 4 : 0));
+    slab_load<IO>(Ks, LK, rows, K, p.vecK, bar, 0, [&](int i) { return k + row(c, i) * K; });
+    slab_square(Pt, P, C, bulkP, bar, 64);
   };
   auto load_qw = [&](int c) {
-    if (c >= 0) {
-      const float* w = p.w + ((size_t)bh * p.n + c) * C * K;
-      stage_rows(Qs, LK, min(C, p.T - c * C), K, p.vecK, q, [&](int i) { return q + row(c, i) * K; });
-      stage_rows(Ws, LK, C, K, p.vecK, w, [&](int i) { return w + i * K; });
-    }
-    cp_commit();
+    if (c < 0) return;
+    const float* w = p.w + ((size_t)bh * p.n + c) * C * K;
+    const int rows = min(C, p.T - c * C);
+    if (bulkK && tid == 0) tc::mbar_expect_tx(bar + 1, (C + rows) * K * 4);
+    slab_load<IO>(Qs, LK, rows, K, p.vecK, bar + 1, 128, [&](int i) { return q + row(c, i) * K; });
+    if (bulkK) slab_load<float>(Ws, LK, C, K, p.vecK, bar + 1, 192, [&](int i) { return w + i * K; });
+    else slab_copy<float>(Ws, LK, C, K, p.vecK, [&](int i) { return w + i * K; });
   };
-  auto scalars = [&](int c) {
-    float* s = sc + (c & 1) * kSc;
-    if (tid < R) {
-      const float* gam = p.gam + ((size_t)bh * p.n + c) * C;
-      const float gl = gam[C - 1], g = tid < C ? gam[tid] : gl;
-      s[tid] = exp_nonpos_precise(g);
-      s[R + tid] = exp_nonpos_precise(gl - g);
-      if (tid == 0) s[2 * R] = exp_nonpos_precise(gl);
-    }
-  };
-  float o[2][2];  // this thread's elements of dO, fetched a chunk ahead
-  auto fetch_o = [&](int c) {
-    const int imax = min(C, p.T - c * C);
+  const float* gam = p.gam + (size_t)bh * p.n * C;
+  // this thread's elements of dO and the log decay of their rows, fetched a chunk ahead
+  float o[W / 4], go[W / 4], gl, g;
+  auto fetch = [&](int c) {
+    const int rows = min(C, p.T - c * C);
+    gl = gam[(c + 1) * C - 1];
+    g = tid < C ? gam[c * C + tid] : gl;
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-      for (int y = 0; y < 2; ++y) {
-        const int i = ty + 32 * r, jv = j0 + tx + 8 * y;
-        o[r][y] = (i < imax && jv < V) ? to_f32(dO[row(c, i) * V + jv]) : 0.f;
-      }
-  };
-  // the scaling with E(gam) reads the factor itself: the chunk's scalars are being written by other threads
-  auto put_o = [&](int c) {
-    const float* gam = p.gam + ((size_t)bh * p.n + c) * C;
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const int i = ty + 32 * r;
-      const float di = exp_nonpos_precise(gam[min(i, C - 1)]);
-#pragma unroll
-      for (int y = 0; y < 2; ++y) {
-        const int j = tx + 8 * y;
-        Ot[j * LD + i] = o[r][y];
-        const float x = o[r][y] * di;
-        *reinterpret_cast<f2*>(Od + (c & 1) * R * 32 + i * 32 + 2 * j) = pack2(x, x);
-      }
+    for (int x = 0; x < W / 4; ++x) {
+      const int i = (tid + 256 * x) / W, jv = j0 + (tid + 256 * x) % W;
+      o[x] = (i < rows && jv < V) ? to_f32(dO[row(c, i) * V + jv]) : 0.f;
+      go[x] = gam[c * C + min(i, C - 1)];
     }
   };
+  auto put = [&](int c) {
+    slab_scalars(sc + (c & 1) * kSlabScalars, g, gl);
+#pragma unroll
+    for (int x = 0; x < W / 4; ++x) {
+      const int i = (tid + 256 * x) / W, j = (tid + 256 * x) % W;
+      Ot[j * LD + i] = o[x];
+      Od[i * W + j] = o[x] * exp_nonpos_precise(go[x]);
+    }
+  };
+  if (tid == 0) {
+    tc::mbar_init(bar, 1);
+    tc::mbar_init(bar + 1, 1);
+    tc::mbar_fence_init();
+  }
   for (int u = tid; u < 192 * LK + R * LD; u += 256) Ks[u] = 0.f;  // rows and columns that no copy reaches
-  f2 S[2][KT / 2];
-#pragma unroll
-  for (int y = 0; y < 2; ++y)
-#pragma unroll
-    for (int x = 0; x < KT / 2; ++x) {
-      const int jv = j0 + 2 * tx + y, kk = kk0 + 2 * x;
-      const float* src = p.dhT_in ? p.dhT_in + ((size_t)bh * K + kk) * V + jv : nullptr;
-      S[y][x] = pack2(src && jv < V && kk < K ? src[0] : 0.f, src && jv < V && kk + 1 < K ? src[V] : 0.f);
-    }
-  scalars(p.n - 1);
-  fetch_o(p.n - 1);
+  slab_state_in<W, KP>(St, p.dhT_in ? p.dhT_in + (size_t)bh * K * V : nullptr, K, V, j0);
+  fetch(p.n - 1);
+  put(p.n - 1);
+  tc::fence_async_smem();
   __syncthreads();
   load_kp(p.n - 1);
   load_qw(p.n - 1);
-  put_o(p.n - 1);
-#pragma unroll
-  for (int y = 0; y < 2; ++y)
-#pragma unroll
-    for (int x = 0; x < KT / 2; ++x) *reinterpret_cast<f2*>(St + (2 * tx + y) * LK + kk0 + 2 * x) = S[y][x];
+  slab_state_keep<W, KP>(St, p.dhs + ((size_t)bh * p.n + p.n - 1) * V * K, K, V, p.vecK, j0);
 
+  bool ok = true;
   for (int c = p.n - 1; c >= 0; --c) {
     const size_t ci = (size_t)bh * p.n + c;
-    const float* s = sc + (c & 1) * kSc;
-    // dS at chunk end, transposed [V][K]
-#pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-      for (int x = 0; x < KT / 2; ++x) {
-        const int jv = j0 + 2 * tx + y, kk = kk0 + 2 * x;
-        const float2 t = unpack2(S[y][x]);
-        float* dst = p.dhs + (ci * V + jv) * K + kk;
-        if (jv < V && kk < K) dst[0] = t.x;
-        if (jv < V && kk + 1 < K) dst[1] = t.y;
-      }
-    if (c > 0) fetch_o(c - 1);
-    cp_wait<1>();
-    __syncthreads();  // k, P, dO and dS are in place
-    f2 acc[2][2], po[2][2];
-    acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0ull;
-    po[0][0] = po[0][1] = po[1][0] = po[1][1] = 0ull;
-#pragma unroll 4
-    for (int x = 0; x < KP; x += 4) {  // k dS
-      const ulonglong2 s0 = lds2x2(St + tx * LK + x), s1 = lds2x2(St + (tx + 8) * LK + x);
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const ulonglong2 a = lds2x2(Ks + (ty + 32 * r) * LK + x);
-        fma2(acc[r][0], a.x, s0.x);
-        fma2(acc[r][1], a.x, s1.x);
-        fma2(acc[r][0], a.y, s0.y);
-        fma2(acc[r][1], a.y, s1.y);
-      }
-    }
-#pragma unroll 4
-    for (int m = 0; m < 32; m += 4) {  // P^T dO (upper triangular: the lower rows start at their half)
-      const ulonglong2 v0 = lds2x2(Ot + tx * LD + m), v1 = lds2x2(Ot + (tx + 8) * LD + m);
-      const ulonglong2 a = lds2x2(Pt + ty * LD + m);
-      fma2(po[0][0], a.x, v0.x);
-      fma2(po[0][1], a.x, v1.x);
-      fma2(po[0][0], a.y, v0.y);
-      fma2(po[0][1], a.y, v1.y);
-    }
-#pragma unroll 4
-    for (int m = 32; m < 64; m += 4) {
-      const ulonglong2 v0 = lds2x2(Ot + tx * LD + m), v1 = lds2x2(Ot + (tx + 8) * LD + m);
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const ulonglong2 a = lds2x2(Pt + (ty + 32 * r) * LD + m);
-        fma2(po[r][0], a.x, v0.x);
-        fma2(po[r][1], a.x, v1.x);
-        fma2(po[r][0], a.y, v0.y);
-        fma2(po[r][1], a.y, v1.y);
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-      for (int y = 0; y < 2; ++y) {
-        const int i = ty + 32 * r, j = tx + 8 * y;
-        const float val = fmaf(s[R + i], sum2(acc[r][y]), sum2(po[r][y]));
-        *reinterpret_cast<f2*>(Vd + i * 32 + 2 * j) = pack2(-val, -val);
-        if (i < C && j0 + j < V) p.dvn[(ci * C + i) * V + j0 + j] = val;
-      }
-    cp_wait<0>();
-    __syncthreads();  // dv_new, q and w are in place; k, P and dO have been read
+    const float* s = sc + (c & 1) * kSlabScalars;
+    const uint32_t ph = (p.n - 1 - c) & 1;
+    if (c > 0) fetch(c - 1);
+    if (bulkK || bulkP) ok = tc::mbar_wait(bar, ph);
+    ok = __syncthreads_and(ok);  // k, P^T, dO, dS and the decay factors are in place
+    if (!ok) break;
+    if (tid < 128) slab_nt<W, 16, SP>(part, Ks, LK, St, LK, KP, tid);
+    else slab_nt<W, 16, SP>(partP, Pt, LD, Ot, LD, R, tid - 128);
+    tc::fence_async_smem();
+    __syncthreads();
     load_kp(c - 1);
-    const float* od = Od + (c & 1) * R * 32;
-    const f2 L = pack2(s[2 * R], s[2 * R]);
 #pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-      for (int x = 0; x < KT / 2; ++x) S[y][x] = mul2(S[y][x], L);
-#pragma unroll 4
-    for (int i = 0; i < R; ++i) {
-      const ulonglong2 oo = lds2x2(od + i * 32 + 4 * tx), vv = lds2x2(Vd + i * 32 + 4 * tx);
-#pragma unroll
-      for (int x = 0; x < KT / 2; ++x) {
-        const f2 qx = *reinterpret_cast<const f2*>(Qs + i * LK + kk0 + 2 * x);
-        const f2 wx = *reinterpret_cast<const f2*>(Ws + i * LK + kk0 + 2 * x);
-        fma2(S[0][x], qx, oo.x);
-        fma2(S[1][x], qx, oo.y);
-        fma2(S[0][x], wx, vv.x);
-        fma2(S[1][x], wx, vv.y);
-      }
+    for (int x = 0; x < W / 4; ++x) {
+      const int i = (tid + 256 * x) / W, j = (tid + 256 * x) % W;
+      const float val = fmaf(s[R + i], slab_sum<W>(part, R, i, j), slab_sum<W>(partP, R, i, j));
+      Vn[i * W + j] = -val;
+      if (i < C && j0 + j < V) p.dvn[(ci * C + i) * V + j0 + j] = val;
     }
-    if (c > 0) {
-      scalars(c - 1);
-      put_o(c - 1);
-    }
-#pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-      for (int x = 0; x < KT / 2; ++x) *reinterpret_cast<f2*>(St + (2 * tx + y) * LK + kk0 + 2 * x) = S[y][x];
-    __syncthreads();  // q, w and dv_new have been read
+    if (bulkK) ok = tc::mbar_wait(bar + 1, ph);
+    ok = __syncthreads_and(ok);  // dv_new, q and w are in place
+    if (!ok) break;
+    if (tid < 128) slab_tn<W, KP>(part, Qs, Od, tid);
+    else slab_tn<W, KP>(partW, Ws, Vn, tid - 128);
+    tc::fence_async_smem();
+    __syncthreads();
     load_qw(c - 1);
+    slab_state_step<W, KP, 2 * SPK>(St, part, s[2 * R], c > 0 ? p.dhs + (ci - 1) * V * K : nullptr, K, V, p.vecK, j0);
+    if (c > 0) put(c - 1);
   }
-  if (p.dh0) {
-#pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-      for (int x = 0; x < KT / 2; ++x) {
-        const int jv = j0 + 2 * tx + y, kk = kk0 + 2 * x;
-        const float2 t = unpack2(S[y][x]);
-        float* dst = p.dh0 + ((size_t)bh * K + kk) * V + jv;
-        if (jv < V && kk < K) dst[0] = t.x;
-        if (jv < V && kk + 1 < K) dst[V] = t.y;
-      }
+  if (!ok && tid == 0) atomicExch(p.status, 5);
+  if (p.dh0 && ok) {
+    __syncthreads();
+    slab_state_out<W, KP>(St, p.dh0 + (size_t)bh * K * V, K, V, j0);
   }
 }
 
@@ -1240,6 +1200,7 @@ static size_t carve(GdnP& p, void* ws, bool bwd) {
   p.u = cv.take<float>(nc * C * V);
   p.P = cv.take<float>(nc * C * C);
   if (bwd) {
+    p.Pt = cv.take<float>(nc * C * C);
     p.hs = cv.take<float>(nc * V * K);
     p.vn = cv.take<float>(nc * C * V);
     p.dhs = cv.take<float>(nc * V * K);
@@ -1291,19 +1252,35 @@ static bool vec_ok(int width, std::initializer_list<const void*> tensors) {
   return width % 4 == 0 && bits % (4 * sizeof(IO)) == 0;
 }
 
-template <typename IO, int KP>
-static mxb_status run_state_fwd(const GdnP& p, cudaStream_t st) {
-  constexpr int sm = state_fwd_smem<KP>();
-  if (set_smem(gdn_state_fwd_kernel<IO, KP>, sm) != MXB_OK) return MXB_ERR_CUDA;
-  MXB_LAUNCH("gdn_state_fwd_kernel", st, (gdn_state_fwd_kernel<IO, KP><<<dim3((p.V + 15) / 16, p.B * p.H), 256, sm, st>>>(p)));
+// Columns of a state CTA: the narrowest slab whose CTAs are on the 148 SMs at once (a chunk takes less time the narrower
+// the slab is), 16 where even those come in several rounds: per column the wide slab is the cheapest.
+static int slab_columns(const GdnP& p) {
+  for (int w = 4; w < 16; w *= 2)
+    if ((size_t)p.B * p.H * ((p.V + w - 1) / w) <= 148) return w;
+  return 16;
+}
+template <typename IO, int W, int KP>
+static mxb_status run_state(const GdnP& p, bool bwd, cudaStream_t st) {
+  const dim3 grid((p.V + W - 1) / W, p.B * p.H);
+  if (bwd) {
+    constexpr int sm = state_bwd_smem<W, KP>();
+    if (set_smem(gdn_state_bwd_kernel<IO, W, KP>, sm) != MXB_OK) return MXB_ERR_CUDA;
+    MXB_LAUNCH("gdn_state_bwd_kernel", st, (gdn_state_bwd_kernel<IO, W, KP><<<grid, 256, sm, st>>>(p)));
+    return check_launch("gdn_state_bwd_kernel");
+  }
+  constexpr int sm = state_fwd_smem<W, KP>();
+  if (set_smem(gdn_state_fwd_kernel<IO, W, KP>, sm) != MXB_OK) return MXB_ERR_CUDA;
+  MXB_LAUNCH("gdn_state_fwd_kernel", st, (gdn_state_fwd_kernel<IO, W, KP><<<grid, 256, sm, st>>>(p)));
   return check_launch("gdn_state_fwd_kernel");
 }
-template <typename IO, int KP>
-static mxb_status run_state_bwd(const GdnP& p, cudaStream_t st) {
-  constexpr int sm = state_bwd_smem<KP>();
-  if (set_smem(gdn_state_bwd_kernel<IO, KP>, sm) != MXB_OK) return MXB_ERR_CUDA;
-  MXB_LAUNCH("gdn_state_bwd_kernel", st, (gdn_state_bwd_kernel<IO, KP><<<dim3((p.V + 15) / 16, p.B * p.H), 256, sm, st>>>(p)));
-  return check_launch("gdn_state_bwd_kernel");
+template <typename IO>
+static mxb_status run_state(const GdnP& p, bool bwd, cudaStream_t st) {
+  const bool narrow = p.K <= 64;
+  switch (slab_columns(p)) {
+    case 4: return narrow ? run_state<IO, 4, 64>(p, bwd, st) : run_state<IO, 4, 128>(p, bwd, st);
+    case 8: return narrow ? run_state<IO, 8, 64>(p, bwd, st) : run_state<IO, 8, 128>(p, bwd, st);
+    default: return narrow ? run_state<IO, 16, 64>(p, bwd, st) : run_state<IO, 16, 128>(p, bwd, st);
+  }
 }
 template <typename IO, int NGK>
 static mxb_status run_chunk_bwd(const GdnP& p, cudaStream_t st) {
@@ -1329,7 +1306,7 @@ static mxb_status run_fwd(GdnP& p, bool chunked, cudaStream_t st) {
   MXB_LAUNCH("gdn_prep_kernel", st, (gdn_prep_kernel<IO><<<dim3(p.n, p.B * p.H), 256, kPrepF32Smem, st>>>(p)));
   mxb_status s = check_launch("gdn_prep_kernel");
   if (s != MXB_OK) return s;
-  return K <= 64 ? run_state_fwd<IO, 64>(p, st) : run_state_fwd<IO, 128>(p, st);
+  return run_state<IO>(p, false, st);
 }
 
 template <typename IO>
@@ -1350,7 +1327,7 @@ static mxb_status run_bwd(GdnP& p, bool recompute, cudaStream_t st) {
   }
   p.vecK = vec_ok<IO>(K, {p.q, p.k, p.dq, p.dk});
   p.vecV = vec_ok<IO>(V, {p.v, p.dO, p.dv});
-  s = K <= 64 ? run_state_bwd<IO, 64>(p, st) : run_state_bwd<IO, 128>(p, st);
+  s = run_state<IO>(p, true, st);
   if (s != MXB_OK) return s;
   return K <= 64 ? run_chunk_bwd<IO, 1>(p, st) : run_chunk_bwd<IO, 2>(p, st);
 }
