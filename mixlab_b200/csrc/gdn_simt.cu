@@ -25,6 +25,9 @@
 //
 // All products are register-tiled over shared-memory tiles of 64 rows (a chunk, zero-padded) and issue packed
 // two-wide FMAs: a chain of fp32 sums either way, with half the issue slots, which the shared-memory loads need.
+#include <cuda.h>
+
+#include <cstring>
 #include <initializer_list>
 #include <type_traits>
 
@@ -33,8 +36,12 @@
 
 namespace mxb {
 
+// [B,T,H,D] float32 -> tensor map with boxes of 32 columns x 64 rows, 128-byte swizzle; false if it cannot be made.
+bool make_tma_map_f32(CUtensorMap* m, const void* base, int B, int T, int H, int D);
+
 struct GdnP {
   int B, T, H, K, V, C, n, gate_is_log, save;
+  int tma;         // the state passes fetch their tiles with the copy engine (float32, Dk % 4 == 0, chunks of 64)
   int vecK, vecV;  // rows of Dk / Dv elements can be read and written four elements at a time
   const void *q, *k, *v;
   const float *beta, *gate, *h0;
@@ -457,8 +464,9 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(GdnP p) {
 // the shared-memory bandwidth of the products, so every thread computes 4 x 4 outputs (eight loaded values per sixteen
 // multiply-adds) over a part of the contraction, and the parts (32 / W of them for 128 rows) are added through shared
 // memory in a fixed order.  One output per thread and 16-column slabs, operands by one cp.async per 16 bytes:
-// 8.2 us a chunk at Dk = 64 (6.6 k of 16.4 k cycles went into issuing the copies); now every row is one bulk copy,
-// issued by one thread as soon as the tile it replaces has been read.
+// 8.2 us a chunk at Dk = 64 (6.6 k of 16.4 k cycles went into issuing the copies; one bulk copy per row still took
+// its warp 2.2 k); now a tile is two or four tensor copies issued by one thread as soon as the tile it replaces has
+// been read.
 //
 // A thread's 4 x 4 outputs of a product along rows: rows ty + NR r, columns tx + NCG c.
 template <int W, int NR>
@@ -467,24 +475,31 @@ struct SlabMap {
   static constexpr int PER = NR * NCG;          // threads that share a part of the contraction
   static constexpr int PITCH = W == 16 ? 20 : W + 1;  // of a row of partial sums (few bank conflicts both ways)
 };
+// The operand tiles that travel (w, q, k, P) lie as the copy engine writes boxes of 32 floats with 128-byte swizzle:
+// slabs of 32 columns, the 16-byte unit within a row XORed with the row's position in its group of eight, so that
+// eight rows read at the same column, or eight units of one row, come from different banks.  Unit u of row i:
+template <int ROWS>
+__device__ __forceinline__ int slab_unit(int i, int u) { return (u >> 3) * (ROWS * 32) + i * 32 + (((u & 7) ^ (i & 7)) << 2); }
+
 // part[s][ty + NR r][tx + NCG c] = sum over the s-th part of the contraction of A[row][k] B[col][k]; `t` < SP * PER
-template <int W, int NR, int SP>
-__device__ __forceinline__ void slab_nt(float* part, const float* A, int lda, const float* B, int ldb, int kd, int t) {
+template <int W, int NR, int SP, int ROWS, int KD>
+__device__ __forceinline__ void slab_nt(float* part, const float* A, const float* B, int ldb, int t) {
   using namespace simt;
   using M = SlabMap<W, NR>;
   const int tx = t % M::NCG, ty = (t / M::NCG) % NR, s = t / M::PER;
-  const int len = kd / SP, k0 = s * len;
+  constexpr int LEN = KD / SP / 4;  // units of four per part
   f2 acc[4][4];
   clear(acc);
-  const float* a0 = A + ty * lda + k0;
-  const float* b0 = B + tx * ldb + k0;
+  const float* b0 = B + tx * ldb;
 #pragma unroll 2
-  for (int k = 0; k < len; k += 4) {
+  for (int x = 0; x < LEN; ++x) {
+    const int u = s * LEN + x;
+    const float* a0 = A + slab_unit<ROWS>(ty, u);  // (the rows of a thread are a multiple of eight apart)
     ulonglong2 a[4], b[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) a[r] = lds2x2(a0 + NR * r * lda + k);
+    for (int r = 0; r < 4; ++r) a[r] = lds2x2(a0 + NR * 32 * r);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) b[c] = lds2x2(b0 + M::NCG * c * ldb + k);
+    for (int c = 0; c < 4; ++c) b[c] = lds2x2(b0 + M::NCG * c * ldb + 4 * u);
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -500,18 +515,17 @@ __device__ __forceinline__ void slab_nt(float* part, const float* A, int lda, co
       part[s * 4 * NR * M::PITCH + (ty + NR * r) * M::PITCH + tx + M::NCG * c] = sum2(acc[r][c]);
 }
 // part[s][4 tx + c][kk] = sum over the s-th part of the 64 rows i of A[i][kk] B[i][4 tx + c]; t < 128
-template <int W, int KP>
+template <int W, int KP, int ROWS>
 __device__ __forceinline__ void slab_tn(float* part, const float* A, const float* B, int t) {
   using namespace simt;
   constexpr int LK = KP + 4, NCG = W / 4, PER = NCG * (KP / 4), SP = 128 / PER, LEN = R / SP;
   const int tx = t % NCG, kg = (t / NCG) % (KP / 4), s = t / PER;
   f2 acc[4][2];  // [column][pair of state rows]
   clear(acc);
-  const float* a0 = A + s * LEN * LK + 4 * kg;
   const float* b0 = B + s * LEN * W + 4 * tx;
 #pragma unroll 4
   for (int i = 0; i < LEN; ++i) {
-    const ulonglong2 a = lds2x2(a0 + i * LK);
+    const ulonglong2 a = lds2x2(A + slab_unit<ROWS>(s * LEN + i, kg));
     const float4 b = *reinterpret_cast<const float4*>(b0 + i * W);
     const f2 bb[4] = {pack2(b.x, b.x), pack2(b.y, b.y), pack2(b.z, b.z), pack2(b.w, b.w)};
 #pragma unroll
@@ -526,35 +540,25 @@ __device__ __forceinline__ void slab_tn(float* part, const float* A, const float
 }
 constexpr int kSlabScalars = 2 * simt::R + 4;  // E(gam), E(gam_last - gam), E(gam_last)
 
-// A tile of 64 rows of n elements, rows past `rows` zero, by the threads themselves (bf16 rows are widened).
-template <typename IO, typename F>
-__device__ __forceinline__ void slab_copy(float* dst, int pitch, int rows, int n, int vec, F rowptr) {
-  for (int u = threadIdx.x; u < simt::R * 32; u += 256) {
-    const int i = u >> 5, c = 4 * (u & 31);
-    if (c < n)
-      *reinterpret_cast<float4*>(dst + i * pitch + c) = i < rows ? simt::ld4(rowptr(i), c, n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+// Tensor maps of the tiles: boxes of 32 columns x 64 rows; rows past the end of a sequence and columns past Dk arrive as
+// zeros.
+struct alignas(64) SlabMaps {
+  CUtensorMap w, q, k, P;  // P: the transposed matrices in the backward
+};
+// Rows 0 .. 63 of a tile of KP columns by the threads themselves (bf16 rows are widened), zeros past `rows` and n.
+template <typename IO, int KP, int ROWS, typename F>
+__device__ __forceinline__ void slab_copy(float* dst, int rows, int n, int vec, F rowptr) {
+  for (int u = threadIdx.x; u < simt::R * (KP / 4); u += 256) {
+    const int i = u / (KP / 4), c4 = u % (KP / 4);
+    *reinterpret_cast<float4*>(dst + slab_unit<ROWS>(i, c4)) =
+        i < rows ? simt::ld4(rowptr(i), 4 * c4, n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
-// The same by one bulk copy per row, completing on `bar`, where rows are float32 and 16-byte multiples (vec); thread
-// t0 + i issues row i.  The caller has told the barrier how many bytes to expect.
-template <typename IO>
-__device__ __forceinline__ bool bulk_rows(int vec) { return sizeof(IO) == 4 && vec; }
-template <typename IO, typename F>
-__device__ __forceinline__ void slab_load(float* dst, int pitch, int rows, int n, int vec, uint64_t* bar, int t0, F rowptr) {
-  if (!bulk_rows<IO>(vec)) return slab_copy<IO>(dst, pitch, rows, n, vec, rowptr);
-  const int i = threadIdx.x - t0;
-  if (i >= 0 && i < rows) tc::bulk_load(tc::smem_u32(dst + i * pitch), rowptr(i), n * 4, bar);
-  if (rows < simt::R)
-    for (int u = threadIdx.x; u < (simt::R - rows) * 32; u += 256)
-      if (4 * (u & 31) < n) *reinterpret_cast<float4*>(dst + (rows + (u >> 5)) * pitch + 4 * (u & 31)) = make_float4(0.f, 0.f, 0.f, 0.f);
-}
-// A [C][C] matrix of the workspace into a [64][LD] tile (what lies outside stays zero from the start).
-__device__ __forceinline__ void slab_square(float* dst, const float* src, int C, bool bulk, uint64_t* bar, int t0) {
-  if (bulk) {
-    const int i = threadIdx.x - t0;
-    if (i >= 0 && i < simt::R) tc::bulk_load(tc::smem_u32(dst + i * simt::LD), src + i * simt::R, simt::R * 4, bar);
-  } else {
-    for (int u = threadIdx.x; u < C * C; u += 256) dst[(u / C) * simt::LD + u % C] = src[u];
+// A [C][C] matrix of the workspace (what lies outside stays zero from the start).
+__device__ __forceinline__ void slab_square(float* dst, const float* src, int C) {
+  for (int u = threadIdx.x; u < C * C; u += 256) {
+    const int i = u / C, j = u % C;
+    dst[slab_unit<simt::R>(i, j >> 2) + (j & 3)] = src[u];
   }
 }
 
@@ -563,11 +567,11 @@ template <int W>
 constexpr int kSlabPart = 32 / W * 128 * SlabMap<W, 16>::PITCH;
 template <int W, int KP>
 constexpr int state_fwd_smem() {
-  return 4 * (192 * (KP + 4) + simt::R * simt::LD + W * (KP + 4) + W * simt::LD + simt::R * W + 2 * kSlabScalars + kSlabPart<W>) + 64;
+  return 4 * (192 * KP + simt::R * simt::R + W * (KP + 4) + W * simt::LD + simt::R * W + 2 * kSlabScalars + kSlabPart<W>) + 64 + 1024;
 }
 template <int W, int KP>
 constexpr int state_bwd_smem() {
-  return 4 * (192 * (KP + 4) + simt::R * simt::LD + W * (KP + 4) + W * simt::LD + 2 * simt::R * W + 2 * kSlabScalars + kSlabPart<W>) + 64;
+  return 4 * (192 * KP + simt::R * simt::R + W * (KP + 4) + W * simt::LD + 2 * simt::R * W + 2 * kSlabScalars + kSlabPart<W>) + 64 + 1024;
 }
 // Decay factors of one chunk from its in-chunk cumulative log decay g (lane's own) and gl (the last).
 __device__ __forceinline__ void slab_scalars(float* s, float g, float gl) {
@@ -628,14 +632,15 @@ __device__ __forceinline__ float slab_sum(const float* part, int rows, int row, 
 
 // v_new = u - w S;  o = E(gam) (q S) + P v_new;  S <- E(gam_last) S + (k r)^T v_new
 template <typename IO, int W, int KP>
-__global__ void __launch_bounds__(256, 1) gdn_state_fwd_kernel(GdnP p) {
+__global__ void __launch_bounds__(256, 1) gdn_state_fwd_kernel(GdnP p, const __grid_constant__ SlabMaps maps) {
   using namespace simt;
   constexpr int LK = KP + 4, SP = 32 / W, SPK = 2048 / (W * KP), PITCH = SlabMap<W, 16>::PITCH;
-  extern __shared__ __align__(16) float smem[];
-  float* Wq = smem;              // [128][LK] w rows, then q rows
-  float* Ks = Wq + 128 * LK;     // [64][LK]
-  float* Ps = Ks + R * LK;       // [64][LD]
-  float* St = Ps + R * LD;       // [W][LK]  S^T
+  extern __shared__ float smem_raw[];
+  float* Wq = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(smem_raw) + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u));
+                                 // slabs of [128 rows][32]: w rows, then q rows
+  float* Ks = Wq + 128 * KP;     // slabs of [64][32]
+  float* Ps = Ks + R * KP;       // slabs of [64][32]
+  float* St = Ps + R * R;        // [W][LK]  S^T
   float* Vt = St + W * LK;       // [W][LD]  v_new^T
   float* Vr = Vt + W * LD;       // [64][W]  r_i v_new
   float* sc = Vr + R * W;        // x2 decay factors of a chunk
@@ -649,30 +654,43 @@ __global__ void __launch_bounds__(256, 1) gdn_state_fwd_kernel(GdnP p) {
   const IO* k = static_cast<const IO*>(p.k);
   IO* out = static_cast<IO*>(p.out);
   auto row = [&](int c, int i) { return ((size_t)(b * p.T + c * C + i) * p.H + h); };
-  const bool bulkK = bulk_rows<IO>(p.vecK), bulkP = C == R;
+  const bool tma = p.tma;
   auto load_wq = [&](int c) {
     if (c >= p.n) return;
-    const float* w = p.w + ((size_t)bh * p.n + c) * C * K;
-    const int rows = min(C, p.T - c * C);
-    if (bulkK && tid == 0) tc::mbar_expect_tx(bar, (C + rows) * K * 4);
-    if (bulkK) slab_load<float>(Wq, LK, C, K, p.vecK, bar, 0, [&](int i) { return w + i * K; });
-    else slab_copy<float>(Wq, LK, C, K, p.vecK, [&](int i) { return w + i * K; });
-    slab_load<IO>(Wq + R * LK, LK, rows, K, p.vecK, bar, 64, [&](int i) { return q + row(c, i) * K; });
+    if (tma) {  // one thread per tensor issues, in different warps
+      if (tid == 0) {
+        tc::mbar_expect_tx(bar, 128 * KP * 4);
+        for (int x = 0; x < KP / 32; ++x) tc::tma_load_4d(tc::smem_u32(Wq + x * 4096), &maps.w, 32 * x, 0, (bh * p.n + c) * R, 0, bar);
+      } else if (tid == 32) {
+        for (int x = 0; x < KP / 32; ++x) tc::tma_load_4d(tc::smem_u32(Wq + x * 4096 + 2048), &maps.q, 32 * x, h, c * R, b, bar);
+      }
+    } else {
+      const float* w = p.w + ((size_t)bh * p.n + c) * C * K;
+      slab_copy<float, KP, 128>(Wq, C, K, p.vecK, [&](int i) { return w + i * K; });
+      slab_copy<IO, KP, 128>(Wq + 2048, min(C, p.T - c * C), K, p.vecK, [&](int i) { return q + row(c, i) * K; });
+    }
   };
   auto load_kp = [&](int c) {
     if (c >= p.n) return;
-    const float* P = p.P + ((size_t)bh * p.n + c) * C * C;
-    const int rows = min(C, p.T - c * C);
-    if ((bulkK || bulkP) && tid == 0) tc::mbar_expect_tx(bar + 1, (bulkK ? rows * K * 4 : 0) + (bulkP ? R * R * 4 : 0));
-    slab_load<IO>(Ks, LK, rows, K, p.vecK, bar + 1, 128, [&](int i) { return k + row(c, i) * K; });
-    slab_square(Ps, P, C, bulkP, bar + 1, 192);
+    if (tma) {
+      if (tid == 64) {
+        tc::mbar_expect_tx(bar + 1, R * (KP + R) * 4);
+        for (int x = 0; x < KP / 32; ++x) tc::tma_load_4d(tc::smem_u32(Ks + x * 2048), &maps.k, 32 * x, h, c * R, b, bar + 1);
+      } else if (tid == 96) {
+        for (int x = 0; x < 2; ++x) tc::tma_load_4d(tc::smem_u32(Ps + x * 2048), &maps.P, 32 * x, 0, (bh * p.n + c) * R, 0, bar + 1);
+      }
+    } else {
+      slab_copy<IO, KP, R>(Ks, min(C, p.T - c * C), K, p.vecK, [&](int i) { return k + row(c, i) * K; });
+      slab_square(Ps, p.P + ((size_t)bh * p.n + c) * C * C, C);
+    }
   };
   if (tid == 0) {
     tc::mbar_init(bar, 1);
     tc::mbar_init(bar + 1, 1);
     tc::mbar_fence_init();
   }
-  for (int u = tid; u < 192 * LK + R * LD; u += 256) Wq[u] = 0.f;  // rows and columns that no copy reaches
+  if (C < R)
+    for (int u = tid; u < R * R; u += 256) Ps[u] = 0.f;
   slab_state_in<W, KP>(St, p.h0 ? p.h0 + (size_t)bh * K * V : nullptr, K, V, j0);
   const float* gam = p.gam + (size_t)bh * p.n * C;
   float gl = gam[C - 1], g = tid < C ? gam[tid] : gl;
@@ -698,10 +716,10 @@ __global__ void __launch_bounds__(256, 1) gdn_state_fwd_kernel(GdnP p) {
       gl = gam[(c + 2) * C - 1];
       g = tid < C ? gam[(c + 1) * C + tid] : gl;
     }
-    if (bulkK) ok = tc::mbar_wait(bar, c & 1);
+    if (tma) ok = tc::mbar_wait(bar, c & 1);
     ok = __syncthreads_and(ok);  // w, q, the state and the decay factors are in place
     if (!ok) break;
-    slab_nt<W, 32, SP>(part, Wq, LK, St, LK, KP, tid);
+    slab_nt<W, 32, SP, 128, KP>(part, Wq, St, LK, tid);
     tc::fence_async_smem();
     __syncthreads();
     load_wq(c + 1);
@@ -714,11 +732,11 @@ __global__ void __launch_bounds__(256, 1) gdn_state_fwd_kernel(GdnP p) {
       Vr[i * W + j] = val * s[R + i];
       if (p.save && i < C && j0 + j < V) p.vn[(ci * C + i) * V + j0 + j] = val;
     }
-    if (bulkK || bulkP) ok = tc::mbar_wait(bar + 1, c & 1);
+    if (tma) ok = tc::mbar_wait(bar + 1, c & 1);
     ok = __syncthreads_and(ok);  // v_new, k and P are in place
     if (!ok) break;
-    if (tid < 128) slab_nt<W, 16, SP>(part, Ps, LD, Vt, LD, R, tid);
-    else slab_tn<W, KP>(partK, Ks, Vr, tid - 128);
+    if (tid < 128) slab_nt<W, 16, SP, R, R>(part, Ps, Vt, LD, tid);
+    else slab_tn<W, KP, R>(partK, Ks, Vr, tid - 128);
     tc::fence_async_smem();
     __syncthreads();
     load_kp(c + 1);
@@ -739,15 +757,16 @@ __global__ void __launch_bounds__(256, 1) gdn_state_fwd_kernel(GdnP p) {
 
 // dv_new = P^T dO + r (k dS);  dS <- E(gam_last) dS + (q E(gam))^T dO - w^T dv_new, chunks in reverse.
 template <typename IO, int W, int KP>
-__global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p) {
+__global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p, const __grid_constant__ SlabMaps maps) {
   using namespace simt;
   constexpr int LK = KP + 4, SP = 32 / W, SPK = 2048 / (W * KP), PITCH = SlabMap<W, 16>::PITCH;
-  extern __shared__ __align__(16) float smem[];
-  float* Ks = smem;              // [64][LK]
-  float* Qs = Ks + R * LK;       // [64][LK]
-  float* Ws = Qs + R * LK;       // [64][LK]
-  float* Pt = Ws + R * LK;       // [64][LD]  P^T
-  float* St = Pt + R * LD;       // [W][LK]   dS^T
+  extern __shared__ float smem_raw[];
+  float* Ks = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(smem_raw) + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u));
+                                 // slabs of [64][32], the four tiles
+  float* Qs = Ks + R * KP;
+  float* Ws = Qs + R * KP;
+  float* Pt = Ws + R * KP;       // P^T
+  float* St = Pt + R * R;        // [W][LK]   dS^T
   float* Ot = St + W * LK;       // [W][LD]   dO^T
   float* Od = Ot + W * LD;       // [64][W]   E(gam_i) dO
   float* Vn = Od + R * W;        // [64][W]   -dv_new
@@ -764,23 +783,35 @@ __global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p) {
   const IO* k = static_cast<const IO*>(p.k);
   const IO* dO = static_cast<const IO*>(p.dO);
   auto row = [&](int c, int i) { return ((size_t)(b * p.T + c * C + i) * p.H + h); };
-  const bool bulkK = bulk_rows<IO>(p.vecK), bulkP = C == R;
+  const bool tma = p.tma;
   auto load_kp = [&](int c) {
     if (c < 0) return;
-    const float* P = p.Pt + ((size_t)bh * p.n + c) * C * C;
-    const int rows = min(C, p.T - c * C);
-    if ((bulkK || bulkP) && tid == 0) tc::mbar_expect_tx(bar, (bulkK ? rows * K * 4 : 0) + (bulkP ? R * R * 4 : 0));
-    slab_load<IO>(Ks, LK, rows, K, p.vecK, bar, 0, [&](int i) { return k + row(c, i) * K; });
-    slab_square(Pt, P, C, bulkP, bar, 64);
+    if (tma) {
+      if (tid == 0) {
+        tc::mbar_expect_tx(bar, R * (KP + R) * 4);
+        for (int x = 0; x < KP / 32; ++x) tc::tma_load_4d(tc::smem_u32(Ks + x * 2048), &maps.k, 32 * x, h, c * R, b, bar);
+      } else if (tid == 32) {
+        for (int x = 0; x < 2; ++x) tc::tma_load_4d(tc::smem_u32(Pt + x * 2048), &maps.P, 32 * x, 0, (bh * p.n + c) * R, 0, bar);
+      }
+    } else {
+      slab_copy<IO, KP, R>(Ks, min(C, p.T - c * C), K, p.vecK, [&](int i) { return k + row(c, i) * K; });
+      slab_square(Pt, p.Pt + ((size_t)bh * p.n + c) * C * C, C);
+    }
   };
   auto load_qw = [&](int c) {
     if (c < 0) return;
-    const float* w = p.w + ((size_t)bh * p.n + c) * C * K;
-    const int rows = min(C, p.T - c * C);
-    if (bulkK && tid == 0) tc::mbar_expect_tx(bar + 1, (C + rows) * K * 4);
-    slab_load<IO>(Qs, LK, rows, K, p.vecK, bar + 1, 128, [&](int i) { return q + row(c, i) * K; });
-    if (bulkK) slab_load<float>(Ws, LK, C, K, p.vecK, bar + 1, 192, [&](int i) { return w + i * K; });
-    else slab_copy<float>(Ws, LK, C, K, p.vecK, [&](int i) { return w + i * K; });
+    if (tma) {
+      if (tid == 64) {
+        tc::mbar_expect_tx(bar + 1, 2 * R * KP * 4);
+        for (int x = 0; x < KP / 32; ++x) tc::tma_load_4d(tc::smem_u32(Qs + x * 2048), &maps.q, 32 * x, h, c * R, b, bar + 1);
+      } else if (tid == 96) {
+        for (int x = 0; x < KP / 32; ++x) tc::tma_load_4d(tc::smem_u32(Ws + x * 2048), &maps.w, 32 * x, 0, (bh * p.n + c) * R, 0, bar + 1);
+      }
+    } else {
+      const float* w = p.w + ((size_t)bh * p.n + c) * C * K;
+      slab_copy<IO, KP, R>(Qs, min(C, p.T - c * C), K, p.vecK, [&](int i) { return q + row(c, i) * K; });
+      slab_copy<float, KP, R>(Ws, C, K, p.vecK, [&](int i) { return w + i * K; });
+    }
   };
   const float* gam = p.gam + (size_t)bh * p.n * C;
   // this thread's elements of dO and the log decay of their rows, fetched a chunk ahead
@@ -810,7 +841,8 @@ __global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p) {
     tc::mbar_init(bar + 1, 1);
     tc::mbar_fence_init();
   }
-  for (int u = tid; u < 192 * LK + R * LD; u += 256) Ks[u] = 0.f;  // rows and columns that no copy reaches
+  if (C < R)
+    for (int u = tid; u < R * R; u += 256) Pt[u] = 0.f;
   slab_state_in<W, KP>(St, p.dhT_in ? p.dhT_in + (size_t)bh * K * V : nullptr, K, V, j0);
   fetch(p.n - 1);
   put(p.n - 1);
@@ -826,11 +858,11 @@ __global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p) {
     const float* s = sc + (c & 1) * kSlabScalars;
     const uint32_t ph = (p.n - 1 - c) & 1;
     if (c > 0) fetch(c - 1);
-    if (bulkK || bulkP) ok = tc::mbar_wait(bar, ph);
+    if (tma) ok = tc::mbar_wait(bar, ph);
     ok = __syncthreads_and(ok);  // k, P^T, dO, dS and the decay factors are in place
     if (!ok) break;
-    if (tid < 128) slab_nt<W, 16, SP>(part, Ks, LK, St, LK, KP, tid);
-    else slab_nt<W, 16, SP>(partP, Pt, LD, Ot, LD, R, tid - 128);
+    if (tid < 128) slab_nt<W, 16, SP, R, KP>(part, Ks, St, LK, tid);
+    else slab_nt<W, 16, SP, R, R>(partP, Pt, Ot, LD, tid - 128);
     tc::fence_async_smem();
     __syncthreads();
     load_kp(c - 1);
@@ -841,11 +873,11 @@ __global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p) {
       Vn[i * W + j] = -val;
       if (i < C && j0 + j < V) p.dvn[(ci * C + i) * V + j0 + j] = val;
     }
-    if (bulkK) ok = tc::mbar_wait(bar + 1, ph);
+    if (tma) ok = tc::mbar_wait(bar + 1, ph);
     ok = __syncthreads_and(ok);  // dv_new, q and w are in place
     if (!ok) break;
-    if (tid < 128) slab_tn<W, KP>(part, Qs, Od, tid);
-    else slab_tn<W, KP>(partW, Ws, Vn, tid - 128);
+    if (tid < 128) slab_tn<W, KP, R>(part, Qs, Od, tid);
+    else slab_tn<W, KP, R>(partW, Ws, Vn, tid - 128);
     tc::fence_async_smem();
     __syncthreads();
     load_qw(c - 1);
@@ -1260,17 +1292,23 @@ static int slab_columns(const GdnP& p) {
   return 16;
 }
 template <typename IO, int W, int KP>
-static mxb_status run_state(const GdnP& p, bool bwd, cudaStream_t st) {
+static mxb_status run_state(GdnP p, bool bwd, cudaStream_t st) {
+  SlabMaps maps;
+  std::memset(&maps, 0, sizeof maps);
+  const int rows = p.B * p.H * p.n * p.C;
+  p.tma = sizeof(IO) == 4 && p.C == simt::R && make_tma_map_f32(&maps.q, p.q, p.B, p.T, p.H, p.K) &&
+          make_tma_map_f32(&maps.k, p.k, p.B, p.T, p.H, p.K) && make_tma_map_f32(&maps.w, p.w, 1, rows, 1, p.K) &&
+          make_tma_map_f32(&maps.P, bwd ? p.Pt : p.P, 1, rows, 1, simt::R);
   const dim3 grid((p.V + W - 1) / W, p.B * p.H);
   if (bwd) {
     constexpr int sm = state_bwd_smem<W, KP>();
     if (set_smem(gdn_state_bwd_kernel<IO, W, KP>, sm) != MXB_OK) return MXB_ERR_CUDA;
-    MXB_LAUNCH("gdn_state_bwd_kernel", st, (gdn_state_bwd_kernel<IO, W, KP><<<grid, 256, sm, st>>>(p)));
+    MXB_LAUNCH("gdn_state_bwd_kernel", st, (gdn_state_bwd_kernel<IO, W, KP><<<grid, 256, sm, st>>>(p, maps)));
     return check_launch("gdn_state_bwd_kernel");
   }
   constexpr int sm = state_fwd_smem<W, KP>();
   if (set_smem(gdn_state_fwd_kernel<IO, W, KP>, sm) != MXB_OK) return MXB_ERR_CUDA;
-  MXB_LAUNCH("gdn_state_fwd_kernel", st, (gdn_state_fwd_kernel<IO, W, KP><<<grid, 256, sm, st>>>(p)));
+  MXB_LAUNCH("gdn_state_fwd_kernel", st, (gdn_state_fwd_kernel<IO, W, KP><<<grid, 256, sm, st>>>(p, maps)));
   return check_launch("gdn_state_fwd_kernel");
 }
 template <typename IO>

@@ -730,16 +730,23 @@ static EncodeTiledFn encode_tiled_fn() {
 }
 // [B,T,H,D] bf16 as a 4-d tensor (D, H, T, B) with boxes of 64 columns x 64 time steps, 128-byte swizzle
 // (D a multiple of 8: rows are 16-byte multiples; columns past D and rows past T are zero-filled by the copy engine
-// on loads and clipped on stores).  Shared with the Mamba-3 kernels.
-bool make_tma_map_bthd(CUtensorMap* m, const void* base, int B, int T, int H, int D) {
+// on loads and clipped on stores); float32 tensors: boxes of 32 columns.  Shared with the other kernels.
+static bool make_tma_map(CUtensorMap* m, CUtensorMapDataType type, int size, const void* base, int B, int T, int H, int D) {
   EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || D % 8 || D <= 0) return false;
+  if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || D * size % 16 || D <= 0) return false;
+  const cuuint64_t row = (cuuint64_t)D * size;
   const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)T, (cuuint64_t)B};
-  const cuuint64_t strides[3] = {(cuuint64_t)D * 2, (cuuint64_t)H * D * 2, (cuuint64_t)T * H * D * 2};
-  const cuuint32_t box[4] = {64, 1, 64, 1}, estr[4] = {1, 1, 1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+  const cuuint64_t strides[3] = {row, H * row, T * (H * row)};
+  const cuuint32_t box[4] = {128u / size, 1, 64, 1}, estr[4] = {1, 1, 1, 1};
+  return fn(m, type, 4, const_cast<void*>(base), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+bool make_tma_map_bthd(CUtensorMap* m, const void* base, int B, int T, int H, int D) {
+  return make_tma_map(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, B, T, H, D);
+}
+bool make_tma_map_f32(CUtensorMap* m, const void* base, int B, int T, int H, int D) {
+  return make_tma_map(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, B, T, H, D);
 }
 
 static bool g_tc_use_tma = true;
