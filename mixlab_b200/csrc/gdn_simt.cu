@@ -42,6 +42,7 @@ bool make_tma_map_f32(CUtensorMap* m, const void* base, int B, int T, int H, int
 struct GdnP {
   int B, T, H, K, V, C, n, gate_is_log, save;
   int tma;         // the state passes fetch their tiles with the copy engine (float32, Dk % 4 == 0, chunks of 64)
+  int vtma;        // the same for v (Dv % 4 == 0)
   int vecK, vecV;  // rows of Dk / Dv elements can be read and written four elements at a time
   const void *q, *k, *v;
   const float *beta, *gate, *h0;
@@ -58,7 +59,6 @@ struct GdnP {
   float *w;     // [C,K]
   float *u;     // [C,V]
   float *P;     // [C,C]
-  float *Pt;    // [C,C]  P^T (written when the forward saves for the backward)
   float *hs;    // [V,K]  state at chunk start, transposed
   float *vn;    // [C,V]
   float *dhs;   // [V,K]  dS at chunk end, transposed
@@ -309,155 +309,6 @@ __device__ __forceinline__ void stream_nn(f2 (&acc)[4][2 * NG], float* stage, in
 struct NoA { __device__ float4 operator()(int, int) const { return make_float4(0.f, 0.f, 0.f, 0.f); } };
 }  // namespace simt
 
-// ------------------------------------------------------------------ prep
-// One chunk: 64 x 64 x (2 Dk + Dv + Dk) multiply-adds and a triangular inverse, all operands through the streaming
-// stages; 70 KB of shared memory, three CTAs per SM.
-constexpr int kPrepF32Smem = (simt::kStageFloats + simt::R * simt::LD + 3 * simt::R) * 4;
-
-template <typename IO>
-__global__ void __launch_bounds__(256, 2) gdn_prep_kernel(GdnP p) {
-  using namespace simt;
-  extern __shared__ __align__(16) float smem[];
-  float* stage = smem;
-  float* Am = stage + kStageFloats;  // [64][LD]  A, then T in place
-  float* gam = Am + R * LD;
-  float* bet = gam + R;
-  float* bd = bet + R;  // beta * E(gam)
-  const int C = p.C, K = p.K, V = p.V;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31;
-  const int c = blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H, t0 = c * C;
-  const int imax = min(C, p.T - t0);
-  const size_t ci = (size_t)bh * p.n + c;
-  const IO* q = static_cast<const IO*>(p.q);
-  const IO* k = static_cast<const IO*>(p.k);
-  const IO* v = static_cast<const IO*>(p.v);
-  auto row = [&](int i) { return ((size_t)(b * p.T + t0 + i) * p.H + h); };
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto ldq = [&](int i, int x) { return i < imax ? ld4(q + row(i) * K, x, K, p.vecK) : zero; };
-  auto ldk = [&](int i, int x) { return i < imax ? ld4(k + row(i) * K, x, K, p.vecK) : zero; };
-  auto ldv = [&](int i, int x) { return i < imax ? ld4(v + row(i) * V, x, V, p.vecV) : zero; };
-
-  if (c == 0 && bh == 0 && tid < 64) p.status[tid] = 0;
-  if (tid < 32) {  // inclusive cumulative sum of the log gate, two elements per lane
-    const int i0 = 2 * lane, i1 = i0 + 1;
-    const float g0 = i0 < imax ? log_gate(p.gate[row(i0)], p.gate_is_log) : 0.f;
-    const float g1 = i1 < imax ? log_gate(p.gate[row(i1)], p.gate_is_log) : 0.f;
-    float s = g0 + g1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float t = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= o) s += t;
-    }
-    const float b0 = i0 < imax ? p.beta[row(i0)] : 0.f, b1 = i1 < imax ? p.beta[row(i1)] : 0.f;
-    gam[i0] = s - g1; gam[i1] = s;
-    bet[i0] = b0; bet[i1] = b1;
-    bd[i0] = b0 * exp_nonpos_precise(s - g1); bd[i1] = b1 * exp_nonpos_precise(s);
-    if (i0 < C) p.gam[ci * C + i0] = s - g1;
-    if (i1 < C) p.gam[ci * C + i1] = s;
-  }
-  {
-    f2 acc[4][4];
-    clear(acc);
-    stream_nt(acc, stage, K, ldk, ldk);  // (its barriers also publish gam, bet, bd)
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const int i = ty + 16 * r, j = tx + 16 * x;
-        Am[i * LD + j] = (i > j) ? -bet[i] * sum2(acc[r][x]) * exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
-      }
-    clear(acc);
-    stream_nt(acc, stage, K, ldq, ldk);
-    // P leaves row by row, and transposed for the backward; the tile goes over the streaming stage, which has been read
-    constexpr int LP = R + 1;
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const int i = ty + 16 * r, j = tx + 16 * x;
-        stage[i * LP + j] = (i >= j) ? sum2(acc[r][x]) * exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
-      }
-    __syncthreads();
-    for (int u = tid; u < R * R; u += 256) {
-      const int i = u >> 6, j = u & 63;
-      if (i < C && j < C) {
-        p.P[ci * C * C + i * C + j] = stage[i * LP + j];
-        if (p.save) p.Pt[ci * C * C + i * C + j] = stage[j * LP + i];
-      }
-    }
-  }
-  // T = (I - A)^-1 in place: the two 32 x 32 diagonal blocks by forward substitution (thread = block and column, the
-  // column in registers), then the off-diagonal block T21 = T22 (A21 T11) as two 32^3 products over all threads.
-  {
-    float Tc[32];
-    const int cc = tid & 31, r0 = 32 * ((tid >> 5) & 1);
-    if (tid < R) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float* arow = Am + (r0 + i) * LD + r0;
-        float s0 = (i == cc) ? 1.f : 0.f, s1 = 0.f;
-#pragma unroll
-        for (int j = 0; j + 1 < i; j += 2) {
-          s0 = fmaf(arow[j], Tc[j], s0);
-          s1 = fmaf(arow[j + 1], Tc[j + 1], s1);
-        }
-        if (i & 1) s0 = fmaf(arow[i - 1], Tc[i - 1], s0);
-        Tc[i] = (i < cc) ? 0.f : s0 + s1;
-      }
-    }
-    __syncthreads();
-    if (tid < R) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) Am[(r0 + i) * LD + r0 + cc] = Tc[i];
-    }
-    __syncthreads();
-    const int i2 = tid >> 3, jb = (tid & 7) * 4;
-    float4 x = zero;
-#pragma unroll 8
-    for (int m = 0; m < 32; ++m) {  // X = A21 T11 -> the unused upper-right block
-      const float a = Am[(32 + i2) * LD + m];
-      const float4 t = *reinterpret_cast<const float4*>(Am + m * LD + jb);
-      x = make_float4(fmaf(a, t.x, x.x), fmaf(a, t.y, x.y), fmaf(a, t.z, x.z), fmaf(a, t.w, x.w));
-    }
-    *reinterpret_cast<float4*>(Am + i2 * LD + 32 + jb) = x;
-    __syncthreads();
-    float4 y = zero;
-#pragma unroll 8
-    for (int m = 0; m < 32; ++m) {  // T21 = T22 X -> over A21
-      const float a = Am[(32 + i2) * LD + 32 + m];
-      const float4 t = *reinterpret_cast<const float4*>(Am + m * LD + 32 + jb);
-      y = make_float4(fmaf(a, t.x, y.x), fmaf(a, t.y, y.y), fmaf(a, t.z, y.z), fmaf(a, t.w, y.w));
-    }
-    *reinterpret_cast<float4*>(Am + (32 + i2) * LD + jb) = y;
-    __syncthreads();
-    *reinterpret_cast<float4*>(Am + i2 * LD + 32 + jb) = zero;  // the upper-right block of T
-    __syncthreads();
-  }
-  if (p.save)
-    for (int u = tid; u < R * R; u += 256) {
-      const int i = u >> 6, j = u & 63;
-      if (i < C && j < C) p.Tm[ci * C * C + i * C + j] = Am[i * LD + j];
-    }
-  // u = T (v beta), w = T (k beta E(gam)): a block of columns at a time
-  auto product = [&](auto ng, int n, int vec, float* dst, auto ld, const float* scale) {
-    constexpr int NG = decltype(ng)::value;
-    for (int j0 = 0; j0 < n; j0 += 64 * NG) {
-      f2 acc[4][2 * NG];
-      clear(acc);
-      stream_nn<NG, 1>(acc, stage, R, Am, NoA{}, [&](int m, int x) { return scale4(ld(m, j0 + x), scale[m]); });
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int g = 0; g < NG; ++g)
-          if (4 * ty + r < C) st4(dst + (ci * C + 4 * ty + r) * n, j0 + 64 * g + 4 * tx, n, vec, acc4<NG>(acc, r, g));
-    }
-  };
-  if (V <= 64) product(std::integral_constant<int, 1>{}, V, p.vecV, p.u, ldv, bet);
-  else product(std::integral_constant<int, 2>{}, V, p.vecV, p.u, ldv, bet);
-  if (K <= 64) product(std::integral_constant<int, 1>{}, K, p.vecK, p.w, ldk, bd);
-  else product(std::integral_constant<int, 2>{}, K, p.vecK, p.w, ldk, bd);
-}
-
 // ------------------------------------------------------------ state passes
 // The sequential passes: one chunk after the other, so the time of a chunk is what counts.  A CTA owns W columns of
 // the state (columns are independent), W as small as still fits the CTAs on the SMs at once.  What bounds a chunk is
@@ -543,7 +394,7 @@ constexpr int kSlabScalars = 2 * simt::R + 4;  // E(gam), E(gam_last - gam), E(g
 // Tensor maps of the tiles: boxes of 32 columns x 64 rows; rows past the end of a sequence and columns past Dk arrive as
 // zeros.
 struct alignas(64) SlabMaps {
-  CUtensorMap w, q, k, P;  // P: the transposed matrices in the backward
+  CUtensorMap w, q, k, P;  // P: v in the prep kernel
 };
 // Rows 0 .. 63 of a tile of KP columns by the threads themselves (bf16 rows are widened), zeros past `rows` and n.
 template <typename IO, int KP, int ROWS, typename F>
@@ -562,6 +413,258 @@ __device__ __forceinline__ void slab_square(float* dst, const float* src, int C)
   }
 }
 
+// ------------------------------------------------------------------ prep
+// One chunk, a chain of dependent steps: copies -> [k;q] k^T -> triangular inverse -> (T beta) v, (T beta)(E(gam) k).
+// k, q and v are requested at once and stay in shared memory in the swizzled layout of their copies, k is scaled in
+// place beside the inverse; 82 KB, two CTAs per SM.  (Streaming every product's operands in steps of 32 exposed the
+// latency of global memory a dozen times: 18.8 us for 32 chunks of 64 / 64 columns on an empty GPU.)
+template <int KP>
+struct PrepF32 {
+  static constexpr int VC = 128;                         // columns of v at a time
+  static constexpr int kv = KP == 64 ? simt::R * VC : 0; // floats of v's own tile; 128 columns of v go over q
+  static constexpr int smem = 4 * (2 * simt::R * KP + kv + simt::R * simt::LD + 4 * simt::R) + 64 + 1024;
+};
+
+// acc[r][2 g + s] += sum_{m < 4 ty + 4} A[4 ty + r][m] B[m][64 g + 4 tx + 2 s, +1], A lower triangular, B swizzled
+template <int NG>
+__device__ __forceinline__ void prep_product(simt::f2 (&acc)[4][2 * NG], const float* A, const float* B) {
+  using namespace simt;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+#pragma unroll 2
+  for (int m = 0; m < 4 * ty + 4; m += 4) {
+    float a[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float4 t = *reinterpret_cast<const float4*>(A + (4 * ty + r) * LD + m);
+      a[r][0] = t.x; a[r][1] = t.y; a[r][2] = t.z; a[r][3] = t.w;
+    }
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+      ulonglong2 b[NG];
+#pragma unroll
+      for (int g = 0; g < NG; ++g) b[g] = lds2x2(B + slab_unit<R>(m + y, 16 * g + tx));
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const f2 aa = pack2(a[r][y], a[r][y]);
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+          fma2(acc[r][2 * g], aa, b[g].x);
+          fma2(acc[r][2 * g + 1], aa, b[g].y);
+        }
+      }
+    }
+  }
+}
+
+template <typename IO, int KP>
+__global__ void __launch_bounds__(256, 2) gdn_prep_kernel(GdnP p, const __grid_constant__ SlabMaps maps) {
+  using namespace simt;
+  extern __shared__ float smem_raw[];
+  float* Ks = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(smem_raw) + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u));
+  float* Qs = Ks + R * KP;
+  float* Vs = KP == 64 ? Qs + R * KP : Qs;  // 128 columns of v
+  float* Am = Qs + R * KP + PrepF32<KP>::kv;  // [64][LD]  A, then T, then T diag(beta)
+  float* gam = Am + R * LD;
+  float* bet = gam + R;
+  float* dd = bet + R;  // E(gam)
+  uint64_t* bar = reinterpret_cast<uint64_t*>(dd + 2 * R);  // [0] k, q; [1] v
+  const int C = p.C, K = p.K, V = p.V;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31;
+  const int c = blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H, t0 = c * C;
+  const int imax = min(C, p.T - t0);
+  const size_t ci = (size_t)bh * p.n + c;
+  const IO* q = static_cast<const IO*>(p.q);
+  const IO* k = static_cast<const IO*>(p.k);
+  const IO* v = static_cast<const IO*>(p.v);
+  auto row = [&](int i) { return ((size_t)(b * p.T + t0 + i) * p.H + h); };
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const bool tma = p.tma, vtma = p.vtma;
+  auto load_v = [&](int j0) {  // columns j0 .. of v; columns past Dv are not read by anyone
+    if (vtma) {
+      if (tid == 0) {
+        const int nx = min(4, (V - j0 + 31) / 32);
+        tc::mbar_expect_tx(bar + 1, nx * R * 32 * 4);
+        for (int x = 0; x < nx; ++x) tc::tma_load_4d(tc::smem_u32(Vs + x * 2048), &maps.P, j0 + 32 * x, h, t0, b, bar + 1);
+      }
+    } else {
+      for (int u = tid; u < R * 32; u += 256) {
+        const int i = u >> 5, c4 = u & 31;
+        *reinterpret_cast<float4*>(Vs + slab_unit<R>(i, c4)) = i < imax ? ld4(v + row(i) * V, j0 + 4 * c4, V, p.vecV) : zero;
+      }
+    }
+  };
+  if (tid == 0) {
+    tc::mbar_init(bar, 1);
+    tc::mbar_init(bar + 1, 1);
+    tc::mbar_fence_init();
+    if (tma) {
+      tc::mbar_expect_tx(bar, 2 * R * KP * 4);
+      for (int x = 0; x < KP / 32; ++x) {
+        tc::tma_load_4d(tc::smem_u32(Ks + x * 2048), &maps.k, 32 * x, h, t0, b, bar);
+        tc::tma_load_4d(tc::smem_u32(Qs + x * 2048), &maps.q, 32 * x, h, t0, b, bar);
+      }
+    }
+  }
+  if (!tma) {
+    slab_copy<IO, KP, R>(Ks, imax, K, p.vecK, [&](int i) { return k + row(i) * K; });
+    slab_copy<IO, KP, R>(Qs, imax, K, p.vecK, [&](int i) { return q + row(i) * K; });
+  }
+  if (KP == 64) load_v(0);
+  if (c == 0 && bh == 0 && tid >= 64 && tid < 128) p.status[tid - 64] = 0;
+  if (tid >= 32 && tid < 64) {  // inclusive cumulative sum of the log gate, two elements per lane
+    const int i0 = 2 * lane, i1 = i0 + 1;
+    const float g0 = i0 < imax ? log_gate(p.gate[row(i0)], p.gate_is_log) : 0.f;
+    const float g1 = i1 < imax ? log_gate(p.gate[row(i1)], p.gate_is_log) : 0.f;
+    const float b0 = i0 < imax ? p.beta[row(i0)] : 0.f, b1 = i1 < imax ? p.beta[row(i1)] : 0.f;
+    float s = g0 + g1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float t = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += t;
+    }
+    gam[i0] = s - g1; gam[i1] = s;
+    bet[i0] = b0; bet[i1] = b1;
+    dd[i0] = exp_nonpos_precise(s - g1); dd[i1] = exp_nonpos_precise(s);
+    if (i0 < C) p.gam[ci * C + i0] = s - g1;
+    if (i1 < C) p.gam[ci * C + i1] = s;
+  }
+  __syncthreads();
+  bool ok = !tma || tc::mbar_wait(bar, 0);
+  {  // k k^T and q k^T: rows ty + 16 r of both, columns tx + 16 x, lower 16 x 16 blocks only
+    f2 acc[8][4];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) acc[r][x] = 0ull;
+#pragma unroll 2
+    for (int u = 0; u < KP / 4; ++u) {
+      const float* a0 = Ks + slab_unit<R>(ty, u);
+      const float* b0 = Ks + slab_unit<R>(tx, u);
+      ulonglong2 bb[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) bb[x] = lds2x2(b0 + 16 * 32 * x);
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const ulonglong2 a = lds2x2(a0 + (r >> 2) * R * KP + 16 * 32 * (r & 3));
+#pragma unroll
+        for (int x = 0; x <= (r & 3); ++x) {
+          fma2(acc[r][x], a.x, bb[x].x);
+          fma2(acc[r][x], a.y, bb[x].y);
+        }
+      }
+    }
+    float* P = p.P + ci * C * C;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int i = ty + 16 * r, j = tx + 16 * x;
+        const float e = x <= r ? exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
+        Am[i * LD + j] = (i > j) ? -bet[i] * sum2(acc[r][x]) * e : 0.f;
+        if (i < C && j < C) P[i * C + j] = (i >= j) ? sum2(acc[4 + r][x]) * e : 0.f;
+      }
+  }
+  tc::fence_async_smem();
+  __syncthreads();  // A is in place, q has been read
+  if (KP != 64) load_v(0);
+  // T = (I - A)^-1 in place: the two 32 x 32 diagonal blocks by forward substitution (thread = block and column, the
+  // column in registers) while the other threads scale k to E(gam) k, then the off-diagonal block T21 = T22 (A21 T11)
+  // as two 32^3 products over all threads.
+  {
+    float Tc[32];
+    const int cc = tid & 31, r0 = 32 * ((tid >> 5) & 1);
+    if (tid < R) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float* arow = Am + (r0 + i) * LD + r0;
+        float s0 = (i == cc) ? 1.f : 0.f, s1 = 0.f;
+#pragma unroll
+        for (int j = 0; j + 1 < i; j += 2) {
+          s0 = fmaf(arow[j], Tc[j], s0);
+          s1 = fmaf(arow[j + 1], Tc[j + 1], s1);
+        }
+        if (i & 1) s0 = fmaf(arow[i - 1], Tc[i - 1], s0);
+        Tc[i] = (i < cc) ? 0.f : s0 + s1;
+      }
+    } else {
+      for (int u = tid - R; u < R * (KP / 4); u += 192) {
+        const int i = u / (KP / 4);
+        float4* x = reinterpret_cast<float4*>(Ks + slab_unit<R>(i, u % (KP / 4)));
+        *x = scale4(*x, dd[i]);
+      }
+    }
+    __syncthreads();
+    if (tid < R) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) Am[(r0 + i) * LD + r0 + cc] = Tc[i];
+    }
+    __syncthreads();
+    const int i2 = tid >> 3, jb = (tid & 7) * 4;
+    float4 x = zero;
+#pragma unroll 8
+    for (int m = 0; m < 32; ++m) {  // X = A21 T11 -> the unused upper-right block
+      const float a = Am[(32 + i2) * LD + m];
+      const float4 t = *reinterpret_cast<const float4*>(Am + m * LD + jb);
+      x = make_float4(fmaf(a, t.x, x.x), fmaf(a, t.y, x.y), fmaf(a, t.z, x.z), fmaf(a, t.w, x.w));
+    }
+    *reinterpret_cast<float4*>(Am + i2 * LD + 32 + jb) = x;
+    __syncthreads();
+    float4 y = zero;
+#pragma unroll 8
+    for (int m = 0; m < 32; ++m) {  // T21 = T22 X -> over A21
+      const float a = Am[(32 + i2) * LD + 32 + m];
+      const float4 t = *reinterpret_cast<const float4*>(Am + m * LD + 32 + jb);
+      y = make_float4(fmaf(a, t.x, y.x), fmaf(a, t.y, y.y), fmaf(a, t.z, y.z), fmaf(a, t.w, y.w));
+    }
+    __syncthreads();
+    *reinterpret_cast<float4*>(Am + (32 + i2) * LD + jb) = y;
+    *reinterpret_cast<float4*>(Am + i2 * LD + 32 + jb) = zero;  // the upper-right block of T
+    __syncthreads();
+  }
+  for (int u = tid; u < R * R; u += 256) {  // T leaves for the backward; its columns are scaled by beta
+    const int i = u >> 6, j = u & 63;
+    const float t = Am[i * LD + j];
+    if (p.save && i < C && j < C) p.Tm[ci * C * C + i * C + j] = t;
+    Am[i * LD + j] = t * bet[j];
+  }
+  __syncthreads();
+  {  // w
+    constexpr int NG = KP / 64;
+    f2 acc[4][2 * NG];
+    clear(acc);
+    prep_product<NG>(acc, Am, Ks);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int g = 0; g < NG; ++g)
+        if (4 * ty + r < C) st4(p.w + (ci * C + 4 * ty + r) * K, 64 * g + 4 * tx, K, p.vecK, acc4<NG>(acc, r, g));
+  }
+  for (int j0 = 0, it = 0; j0 < V; j0 += 128, ++it) {  // u
+    if (it > 0) {
+      tc::fence_async_smem();
+      __syncthreads();
+      load_v(j0);
+    }
+    if (vtma) ok = tc::mbar_wait(bar + 1, it & 1) && ok;
+    else __syncthreads();
+    auto product = [&](auto ng) {
+      constexpr int NG = decltype(ng)::value;
+      f2 acc[4][2 * NG];
+      clear(acc);
+      prep_product<NG>(acc, Am, Vs);
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int g = 0; g < NG; ++g)
+          if (4 * ty + r < C) st4(p.u + (ci * C + 4 * ty + r) * V, j0 + 64 * g + 4 * tx, V, p.vecV, acc4<NG>(acc, r, g));
+    };
+    if (V - j0 <= 64) product(std::integral_constant<int, 1>{});
+    else product(std::integral_constant<int, 2>{});
+  }
+  if (!ok && tid == 0) atomicExch(p.status, 5);
+}
+
+// ----------------------------------------------------------- state passes: slabs
 // Floats of the partial sums: 128 rows of W columns in 32 / W parts (the products of the second step need less).
 template <int W>
 constexpr int kSlabPart = 32 / W * 128 * SlabMap<W, 16>::PITCH;
@@ -571,7 +674,7 @@ constexpr int state_fwd_smem() {
 }
 template <int W, int KP>
 constexpr int state_bwd_smem() {
-  return 4 * (192 * KP + simt::R * simt::R + W * (KP + 4) + W * simt::LD + 2 * simt::R * W + 2 * kSlabScalars + kSlabPart<W>) + 64 + 1024;
+  return 4 * (192 * KP + simt::R * simt::R + W * (KP + 4) + 3 * simt::R * W + 2 * kSlabScalars + kSlabPart<W>) + 64 + 1024;
 }
 // Decay factors of one chunk from its in-chunk cumulative log decay g (lane's own) and gl (the last).
 __device__ __forceinline__ void slab_scalars(float* s, float g, float gl) {
@@ -765,17 +868,17 @@ __global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p, const __g
                                  // slabs of [64][32], the four tiles
   float* Qs = Ks + R * KP;
   float* Ws = Qs + R * KP;
-  float* Pt = Ws + R * KP;       // P^T
-  float* St = Pt + R * R;        // [W][LK]   dS^T
-  float* Ot = St + W * LK;       // [W][LD]   dO^T
-  float* Od = Ot + W * LD;       // [64][W]   E(gam_i) dO
+  float* Ps = Ws + R * KP;
+  float* St = Ps + R * R;        // [W][LK]   dS^T
+  float* Os = St + W * LK;       // [64][W]   dO
+  float* Od = Os + R * W;        // [64][W]   E(gam_i) dO
   float* Vn = Od + R * W;        // [64][W]   -dv_new
   float* sc = Vn + R * W;        // x2 decay factors of a chunk
   float* part = sc + 2 * kSlabScalars;
   float* partP = part + SP * R * PITCH;        // P^T dO beside k dS
   float* partW = part + SPK * W * LK;          // w^T dv_new beside q^T dO
-  uint64_t* bar = reinterpret_cast<uint64_t*>(part + kSlabPart<W>);  // [0] k, P^T; [1] q, w
-  static_assert(2 * SPK * W * LK <= kSlabPart<W>, "partial sums of the second step");
+  uint64_t* bar = reinterpret_cast<uint64_t*>(part + kSlabPart<W>);  // [0] k, P; [1] q, w
+  static_assert(2 * SPK * W * LK <= kSlabPart<W> && SP * (R * PITCH + W * LD) <= kSlabPart<W>, "partial sums of both steps");
   const int C = p.C, K = p.K, V = p.V;
   const int tid = threadIdx.x;
   const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H, j0 = blockIdx.x * W;
@@ -791,11 +894,11 @@ __global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p, const __g
         tc::mbar_expect_tx(bar, R * (KP + R) * 4);
         for (int x = 0; x < KP / 32; ++x) tc::tma_load_4d(tc::smem_u32(Ks + x * 2048), &maps.k, 32 * x, h, c * R, b, bar);
       } else if (tid == 32) {
-        for (int x = 0; x < 2; ++x) tc::tma_load_4d(tc::smem_u32(Pt + x * 2048), &maps.P, 32 * x, 0, (bh * p.n + c) * R, 0, bar);
+        for (int x = 0; x < 2; ++x) tc::tma_load_4d(tc::smem_u32(Ps + x * 2048), &maps.P, 32 * x, 0, (bh * p.n + c) * R, 0, bar);
       }
     } else {
       slab_copy<IO, KP, R>(Ks, min(C, p.T - c * C), K, p.vecK, [&](int i) { return k + row(c, i) * K; });
-      slab_square(Pt, p.Pt + ((size_t)bh * p.n + c) * C * C, C);
+      slab_square(Ps, p.P + ((size_t)bh * p.n + c) * C * C, C);
     }
   };
   auto load_qw = [&](int c) {
@@ -832,7 +935,7 @@ __global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p, const __g
 #pragma unroll
     for (int x = 0; x < W / 4; ++x) {
       const int i = (tid + 256 * x) / W, j = (tid + 256 * x) % W;
-      Ot[j * LD + i] = o[x];
+      Os[i * W + j] = o[x];
       Od[i * W + j] = o[x] * exp_nonpos_precise(go[x]);
     }
   };
@@ -842,7 +945,7 @@ __global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p, const __g
     tc::mbar_fence_init();
   }
   if (C < R)
-    for (int u = tid; u < R * R; u += 256) Pt[u] = 0.f;
+    for (int u = tid; u < R * R; u += 256) Ps[u] = 0.f;
   slab_state_in<W, KP>(St, p.dhT_in ? p.dhT_in + (size_t)bh * K * V : nullptr, K, V, j0);
   fetch(p.n - 1);
   put(p.n - 1);
@@ -859,17 +962,20 @@ __global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p, const __g
     const uint32_t ph = (p.n - 1 - c) & 1;
     if (c > 0) fetch(c - 1);
     if (tma) ok = tc::mbar_wait(bar, ph);
-    ok = __syncthreads_and(ok);  // k, P^T, dO, dS and the decay factors are in place
+    ok = __syncthreads_and(ok);  // k, P, dO, dS and the decay factors are in place
     if (!ok) break;
     if (tid < 128) slab_nt<W, 16, SP, R, KP>(part, Ks, St, LK, tid);
-    else slab_nt<W, 16, SP, R, R>(partP, Pt, Ot, LD, tid - 128);
+    else slab_tn<W, R, R>(partP, Ps, Os, tid - 128);
     tc::fence_async_smem();
     __syncthreads();
     load_kp(c - 1);
 #pragma unroll
     for (int x = 0; x < W / 4; ++x) {
       const int i = (tid + 256 * x) / W, j = (tid + 256 * x) % W;
-      const float val = fmaf(s[R + i], slab_sum<W>(part, R, i, j), slab_sum<W>(partP, R, i, j));
+      float val = 0.f;
+#pragma unroll
+      for (int y = 0; y < SP; ++y) val += partP[(y * W + j) * LD + i];  // (P^T dO lies column by column)
+      val = fmaf(s[R + i], slab_sum<W>(part, R, i, j), val);
       Vn[i * W + j] = -val;
       if (i < C && j0 + j < V) p.dvn[(ci * C + i) * V + j0 + j] = val;
     }
@@ -1232,7 +1338,6 @@ static size_t carve(GdnP& p, void* ws, bool bwd) {
   p.u = cv.take<float>(nc * C * V);
   p.P = cv.take<float>(nc * C * C);
   if (bwd) {
-    p.Pt = cv.take<float>(nc * C * C);
     p.hs = cv.take<float>(nc * V * K);
     p.vn = cv.take<float>(nc * C * V);
     p.dhs = cv.take<float>(nc * V * K);
@@ -1284,6 +1389,19 @@ static bool vec_ok(int width, std::initializer_list<const void*> tensors) {
   return width % 4 == 0 && bits % (4 * sizeof(IO)) == 0;
 }
 
+template <typename IO, int KP>
+static mxb_status run_prep(GdnP p, cudaStream_t st) {
+  SlabMaps maps;
+  std::memset(&maps, 0, sizeof maps);
+  p.tma = sizeof(IO) == 4 && p.C == simt::R && make_tma_map_f32(&maps.q, p.q, p.B, p.T, p.H, p.K) &&
+          make_tma_map_f32(&maps.k, p.k, p.B, p.T, p.H, p.K);
+  p.vtma = sizeof(IO) == 4 && p.C == simt::R && make_tma_map_f32(&maps.P, p.v, p.B, p.T, p.H, p.V);
+  constexpr int sm = PrepF32<KP>::smem;
+  if (set_smem(gdn_prep_kernel<IO, KP>, sm) != MXB_OK) return MXB_ERR_CUDA;
+  MXB_LAUNCH("gdn_prep_kernel", st, (gdn_prep_kernel<IO, KP><<<dim3(p.n, p.B * p.H), 256, sm, st>>>(p, maps)));
+  return check_launch("gdn_prep_kernel");
+}
+
 // Columns of a state CTA: the narrowest slab whose CTAs are on the 148 SMs at once (a chunk takes less time the narrower
 // the slab is), 16 where even those come in several rounds: per column the wide slab is the cheapest.
 static int slab_columns(const GdnP& p) {
@@ -1298,7 +1416,7 @@ static mxb_status run_state(GdnP p, bool bwd, cudaStream_t st) {
   const int rows = p.B * p.H * p.n * p.C;
   p.tma = sizeof(IO) == 4 && p.C == simt::R && make_tma_map_f32(&maps.q, p.q, p.B, p.T, p.H, p.K) &&
           make_tma_map_f32(&maps.k, p.k, p.B, p.T, p.H, p.K) && make_tma_map_f32(&maps.w, p.w, 1, rows, 1, p.K) &&
-          make_tma_map_f32(&maps.P, bwd ? p.Pt : p.P, 1, rows, 1, simt::R);
+          make_tma_map_f32(&maps.P, p.P, 1, rows, 1, simt::R);
   const dim3 grid((p.V + W - 1) / W, p.B * p.H);
   if (bwd) {
     constexpr int sm = state_bwd_smem<W, KP>();
@@ -1340,9 +1458,7 @@ static mxb_status run_fwd(GdnP& p, bool chunked, cudaStream_t st) {
   }
   p.vecK = vec_ok<IO>(K, {p.q, p.k, p.dq, p.dk});
   p.vecV = vec_ok<IO>(V, {p.v, p.dO, p.dv});
-  if (set_smem(gdn_prep_kernel<IO>, kPrepF32Smem) != MXB_OK) return MXB_ERR_CUDA;
-  MXB_LAUNCH("gdn_prep_kernel", st, (gdn_prep_kernel<IO><<<dim3(p.n, p.B * p.H), 256, kPrepF32Smem, st>>>(p)));
-  mxb_status s = check_launch("gdn_prep_kernel");
+  mxb_status s = K <= 64 ? run_prep<IO, 64>(p, st) : run_prep<IO, 128>(p, st);
   if (s != MXB_OK) return s;
   return run_state<IO>(p, false, st);
 }
