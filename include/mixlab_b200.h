@@ -102,8 +102,7 @@ enum {
                                    CUDA-core kernels (a cross-check of the two backwards) */
   MXB_GDN_SAVE_FOR_BWD = 4,     /* forward: also keep the per-chunk states and v_new in the
                                    workspace, which must then have the BACKWARD size */
-  MXB_GDN_DECODE_REGISTER_KERNEL = 16, /* decode step: use the register-resident kernel even where
-                                          the bulk-copy pipelined kernel covers the shape */
+  MXB_GDN_DECODE_REGISTER_KERNEL = 16, /* accepted; the register-resident kernel is the only decode kernel */
   MXB_GDN_NO_TMA = 32,          /* tensor-core path: stage k, q, v of the prep kernel with cp.async instead
                                    of TMA tensor copies (a cross-check of the two staging paths) */
   MXB_GDN_F32_IO_BF16_OPERANDS = 64, /* io_dtype MXB_F32 only: round q, k, v (and d_out) to bf16, run the

@@ -27,6 +27,18 @@ mxb_status check_launch(const char* what) {
   return MXB_ERR_CUDA;
 }
 
+mxb_status allow_smem(const void* kernel, int bytes, std::atomic<uint64_t>& done) {
+  if (bytes <= 48 * 1024) return MXB_OK;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (e == cudaSuccess && (done.load(std::memory_order_relaxed) & bit)) return MXB_OK;
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) { set_last_cuda_error((int)e); return MXB_ERR_CUDA; }
+  done.fetch_or(bit, std::memory_order_relaxed);
+  return MXB_OK;
+}
+
 // ---- per-launch event tracing -------------------------------------------
 struct TraceRec { const char* name; cudaEvent_t e0, e1; };
 static std::atomic<bool> g_trace_on{false};

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/mixlab_b200.h"
 
 namespace mxb {
@@ -101,6 +103,15 @@ void trace_end(cudaStream_t st);
     ::mxb::trace_end(st);           \
     ::mxb::note_launch();           \
   } while (0)
+
+// Opts a kernel in to more than 48 KB of dynamic shared memory, once per device and kernel (the attribute belongs to the
+// device's context): done is the caller's record, one bit per device.
+mxb_status allow_smem(const void* kernel, int bytes, std::atomic<uint64_t>& done);
+#define MXB_ALLOW_SMEM(bytes, ...)                                              \
+  ([&]() -> mxb_status {                                                        \
+    static std::atomic<uint64_t> done{0};                                       \
+    return ::mxb::allow_smem(reinterpret_cast<const void*>(__VA_ARGS__), bytes, done); \
+  }())
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 

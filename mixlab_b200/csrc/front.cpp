@@ -1,0 +1,502 @@
+// Native half of the torch front end (mixlab_b200/ops.py): checks every operand, allocates the results, keeps the
+// per-device workspace and calls the C ABI.  The C ABI sees only pointers, so a wrong operand would otherwise be read
+// out of bounds or as the wrong type.
+//
+// What bounds a small call is this host work: in Python the checks, the ctypes conversions and the allocations of one
+// decode step took 17 us beside a kernel of 5 us, those of a short scan 30 us.
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/extension.h>
+
+#include <map>
+#include <optional>
+#include <string>
+#include <vector>
+
+#include "../../include/mixlab_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using Opt = std::optional<Tensor>;
+using Shape = at::IntArrayRef;
+
+namespace {
+
+// ------------------------------------------------------------------ the C ABI
+#define MXB_FUNCTIONS(X)                                                                                              \
+  X(mxb_gdn_fwd_workspace_bytes) X(mxb_gdn_bwd_workspace_bytes) X(mxb_gdn_fwd) X(mxb_gdn_bwd) X(mxb_gdn_decode_step)  \
+  X(mxb_gdn_block_workspace_bytes) X(mxb_gdn_block_pre_fwd) X(mxb_gdn_block_pre_bwd) X(mxb_gdn_block_post_fwd)        \
+  X(mxb_gdn_block_post_bwd) X(mxb_mamba3_fwd_workspace_bytes) X(mxb_mamba3_bwd_workspace_bytes) X(mxb_mamba3_fwd)     \
+  X(mxb_mamba3_bwd) X(mxb_mamba3_block_workspace_bytes) X(mxb_mamba3_block_conv_fwd) X(mxb_mamba3_block_conv_bwd)     \
+  X(mxb_mamba3_block_bc_fwd) X(mxb_mamba3_block_bc_bwd) X(mxb_mamba3_block_post_fwd) X(mxb_mamba3_block_post_bwd)
+struct Abi {
+#define X(name) decltype(&::name) name = nullptr;
+  MXB_FUNCTIONS(X)
+#undef X
+} abi;
+
+void open_library(const std::string& path) {
+  void* h = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  if (!h) throw py::import_error(dlerror());
+#define X(name)                                                     \
+  abi.name = reinterpret_cast<decltype(abi.name)>(dlsym(h, #name)); \
+  if (!abi.name) throw py::import_error("missing export " #name);
+  MXB_FUNCTIONS(X)
+#undef X
+}
+
+// ------------------------------------------------------------------ operands
+[[noreturn]] void not_cuda() { throw py::value_error("mixlab_b200 operators take CUDA tensors only (no CPU fallback)"); }
+
+int32_t io_code(const Tensor& t) {
+  if (t.scalar_type() == at::kFloat) return MXB_F32;
+  if (t.scalar_type() == at::kBFloat16) return MXB_BF16;
+  throw py::type_error(std::string("unsupported dtype ") + c10::toString(t.scalar_type()) + " (float32 or bfloat16)");
+}
+
+std::string text(Shape s) {
+  std::string r = "(";
+  for (size_t i = 0; i < s.size(); ++i) r += (i ? ", " : "") + std::to_string(s[i]);
+  return r + ")";
+}
+
+void check(const Tensor& t, Shape shape, at::ScalarType dtype, at::Device dev, const char* name) {
+  if (!t.is_cuda()) not_cuda();
+  if (t.sizes() != shape) throw py::value_error(std::string(name) + ": shape " + text(t.sizes()) + ", expected " + text(shape));
+  if (t.scalar_type() != dtype)
+    throw py::type_error(std::string(name) + ": dtype " + c10::toString(t.scalar_type()) + ", expected " + c10::toString(dtype));
+  if (t.device() != dev) throw py::value_error(std::string(name) + ": on " + t.device().str() + ", expected " + dev.str());
+  if (!t.is_contiguous()) throw py::value_error(std::string(name) + ": tensor must be contiguous");
+}
+void check(const Opt& t, Shape shape, at::ScalarType dtype, at::Device dev, const char* name) {
+  if (t) check(*t, shape, dtype, dev, name);
+}
+
+template <typename T = void>
+T* ptr(const Tensor& t) { return static_cast<T*>(t.data_ptr()); }
+template <typename T = void>
+T* ptr(const Opt& t) { return t ? static_cast<T*>(t->data_ptr()) : nullptr; }
+
+Tensor make(Shape shape, at::ScalarType dtype, at::Device dev) {
+  return at::detail::empty_cuda(shape, dtype, dev, std::nullopt);
+}
+Tensor like(const Tensor& t) { return make(t.sizes(), t.scalar_type(), t.device()); }
+constexpr at::ScalarType F = at::kFloat;
+
+// A call on the device of `t`: that device is current, its current stream is the one to launch on.
+struct On {
+  c10::cuda::CUDAGuard guard;
+  at::Device dev;
+  void* stream;
+  explicit On(const Tensor& t)
+      : guard((t.is_cuda() ? (void)0 : not_cuda(), t.device())), dev(t.device()), stream(c10::cuda::getCurrentCUDAStream(dev.index()).stream()) {}
+};
+
+template <typename Fn, typename... A>
+void call(const char* what, Fn fn, A... args) {
+  mxb_status s;
+  {
+    py::gil_scoped_release nogil;  // a launch can block while the stream's queue is full
+    s = fn(args...);
+  }
+  if (s != MXB_OK) py::module_::import("mixlab_b200._lib").attr("check")(s, what);  // raises MxbError
+}
+
+// ------------------------------------------------------------------ workspace
+// One cached byte buffer per device, grown to the largest size asked for.  `saved` describes the forward call whose
+// intermediates it holds; any other use of the buffer clears it, so that a backward with use_saved=True cannot consume
+// overwritten tiles.  Guarded by the interpreter lock.
+struct Token {
+  int kind = 0;  // 0: nothing saved
+  void* stream = nullptr;
+  int64_t extra[4] = {};
+  struct Operand {
+    const void* data;
+    std::vector<int64_t> shape;
+    at::ScalarType dtype;
+    bool operator==(const Operand& o) const { return data == o.data && dtype == o.dtype && shape == o.shape; }
+  };
+  std::vector<Operand> operands;
+  bool operator==(const Token& o) const {
+    return kind == o.kind && stream == o.stream && std::equal(extra, extra + 4, o.extra) && operands == o.operands;
+  }
+};
+struct Workspace {
+  Tensor buf;
+  Token saved;
+};
+std::map<int, Workspace>& workspaces() {
+  static auto* m = new std::map<int, Workspace>;  // never destroyed: the allocator may be gone by then
+  return *m;
+}
+Tensor workspace(size_t nbytes, int device) {
+  Workspace& w = workspaces()[device];
+  w.saved.kind = 0;
+  if (!w.buf.defined() || static_cast<size_t>(w.buf.numel()) < nbytes) {
+    w.buf = Tensor();
+    w.buf = make({static_cast<int64_t>(nbytes < 256 ? 256 : nbytes)}, at::kByte, at::Device(at::kCUDA, device));
+  }
+  return w.buf;
+}
+Token token(int kind, void* stream, std::initializer_list<const Tensor*> ts, std::initializer_list<int64_t> extra) {
+  Token t;
+  t.kind = kind;
+  t.stream = stream;
+  std::copy(extra.begin(), extra.end(), t.extra);
+  t.operands.reserve(ts.size());
+  for (const Tensor* x : ts) t.operands.push_back({x->data_ptr(), x->sizes().vec(), x->scalar_type()});
+  return t;
+}
+// The workspace of a use_saved backward, which still has to hold what the forward described by `want` left in it.
+Tensor saved_workspace(const Token& want, size_t nbytes, int device, const char* what) {
+  Workspace& w = workspaces()[device];
+  if (!(w.saved == want))
+    throw std::runtime_error(std::string(what) + ": use_saved=True needs the immediately preceding save_for_backward forward on "
+                             "the same tensors, stream and device (the cached workspace has been reused since, or never held them)");
+  if (static_cast<size_t>(w.buf.numel()) < nbytes)
+    throw std::runtime_error(std::string(what) + ": the cached workspace was reallocated after the forward saved into it");
+  return w.buf;
+}
+
+// ------------------------------------------------------------------ gated delta rule
+mxb_gdn_desc gdn_desc(const Tensor& q, const Tensor& v, int64_t chunk, bool gate_is_log, int64_t flags) {
+  if (q.dim() != 4 || v.dim() != 4) throw py::value_error("q, k must be [B,T,H,Dk] and v [B,T,H,Dv]");
+  return {(int32_t)q.size(0), (int32_t)q.size(1), (int32_t)q.size(2), (int32_t)q.size(3), (int32_t)v.size(3), (int32_t)chunk,
+          io_code(q), gate_is_log ? 1 : 0, (int32_t)flags};
+}
+void check_gdn(const mxb_gdn_desc& d, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta, const Tensor& gate) {
+  const auto dev = q.device();
+  const auto io = q.scalar_type();
+  const int64_t kd[] = {d.B, d.T, d.H, d.Dk}, vd[] = {d.B, d.T, d.H, d.Dv};
+  check(q, kd, io, dev, "q");
+  check(k, kd, io, dev, "k");
+  check(v, vd, io, dev, "v");
+  check(beta, Shape(kd, 3), F, dev, "beta");
+  check(gate, Shape(kd, 3), F, dev, "gate");
+}
+Token gdn_token(const On& on, const mxb_gdn_desc& d, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta,
+                const Tensor& gate) {
+  // the flag bits that choose a kernel family choose the layout of what a forward saves
+  return token(1, on.stream, {&q, &k, &v, &beta, &gate},
+               {d.chunk, d.gate_is_log, d.flags & ~(MXB_GDN_SAVE_FOR_BWD | MXB_GDN_BWD_USE_SAVED)});
+}
+
+py::object gdn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta, const Tensor& gate, int64_t chunk,
+                       bool gate_is_log, const Opt& h0, bool want_final, int64_t flags, bool save) {
+  On on(q);
+  const mxb_gdn_desc d = gdn_desc(q, v, chunk, gate_is_log, save ? flags | MXB_GDN_SAVE_FOR_BWD : flags);
+  check_gdn(d, q, k, v, beta, gate);
+  const int64_t sd[] = {d.B, d.H, d.Dk, d.Dv};
+  check(h0, sd, F, on.dev, "h0");
+  Tensor out = like(v), hT;
+  if (want_final) hT = make(sd, F, on.dev);
+  Tensor ws = workspace(abi.mxb_gdn_fwd_workspace_bytes(&d), on.dev.index());
+  call("mxb_gdn_fwd", abi.mxb_gdn_fwd, &d, ptr(q), ptr(k), ptr(v), ptr<float>(beta), ptr<float>(gate), ptr<float>(h0), ptr(out),
+       want_final ? ptr<float>(hT) : nullptr, ptr(ws), (size_t)ws.numel(), on.stream);
+  if (save) workspaces()[on.dev.index()].saved = gdn_token(on, d, q, k, v, beta, gate);
+  return want_final ? py::object(py::make_tuple(out, hT)) : py::cast(out);
+}
+
+py::dict gdn_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta, const Tensor& gate, const Tensor& d_out,
+                      int64_t chunk, bool gate_is_log, const Opt& h0, const Opt& d_final, int64_t flags, bool use_saved) {
+  On on(q);
+  const mxb_gdn_desc d = gdn_desc(q, v, chunk, gate_is_log, use_saved ? flags | MXB_GDN_BWD_USE_SAVED : flags);
+  check_gdn(d, q, k, v, beta, gate);
+  const int64_t sd[] = {d.B, d.H, d.Dk, d.Dv};
+  check(d_out, v.sizes(), q.scalar_type(), on.dev, "d_out");
+  check(h0, sd, F, on.dev, "h0");
+  check(d_final, sd, F, on.dev, "d_final_state");
+  const size_t nws = abi.mxb_gdn_bwd_workspace_bytes(&d);
+  Tensor ws = use_saved ? saved_workspace(gdn_token(on, d, q, k, v, beta, gate), nws, on.dev.index(), "gated_delta_scan_backward")
+                        : workspace(nws, on.dev.index());
+  Tensor dq = like(q), dk = like(k), dv = like(v), db = like(beta), dg = like(gate);
+  Opt dh0;
+  if (h0) dh0 = like(*h0);
+  call("mxb_gdn_bwd", abi.mxb_gdn_bwd, &d, ptr(q), ptr(k), ptr(v), ptr<float>(beta), ptr<float>(gate), ptr<float>(h0), ptr(d_out),
+       ptr<float>(d_final), ptr(dq), ptr(dk), ptr(dv), ptr<float>(db), ptr<float>(dg), ptr<float>(dh0), ptr(ws), (size_t)ws.numel(),
+       on.stream);
+  py::dict r;
+  r["dq"] = dq; r["dk"] = dk; r["dv"] = dv; r["dbeta"] = db; r["dgate"] = dg; r["dh0"] = dh0;
+  return r;
+}
+
+Tensor gdn_decode(const Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta, const Tensor& gate,
+                  bool gate_is_log, const Opt& out_, int64_t flags) {
+  On on(state);
+  if (!q.is_cuda()) not_cuda();
+  if (state.dim() != 4) throw py::value_error("state must be [N,H,Dk,Dv]");
+  const int64_t N = state.size(0), H = state.size(1), K = state.size(2), V = state.size(3);
+  const mxb_gdn_desc d{(int32_t)N, 1, (int32_t)H, (int32_t)K, (int32_t)V, 0, io_code(q), gate_is_log ? 1 : 0, (int32_t)flags};
+  const auto io = q.scalar_type();
+  const int64_t kd[] = {N, H, K}, vd[] = {N, H, V};
+  check(state, state.sizes(), F, on.dev, "state");
+  check(q, kd, io, on.dev, "q");
+  check(k, kd, io, on.dev, "k");
+  check(v, vd, io, on.dev, "v");
+  check(beta, Shape(kd, 2), F, on.dev, "beta");
+  check(gate, Shape(kd, 2), F, on.dev, "gate");
+  check(out_, vd, io, on.dev, "out");
+  Tensor out = out_ ? *out_ : like(v);
+  call("mxb_gdn_decode_step", abi.mxb_gdn_decode_step, &d, ptr<float>(state), ptr(q), ptr(k), ptr(v), ptr<float>(beta),
+       ptr<float>(gate), ptr(out), on.stream);
+  return out;
+}
+
+// ------------------------------------------------------------------ gated_deltanet block stages
+struct BlockArgs {
+  mxb_gdn_desc d;
+  int64_t kd[3], vd[3], hd[3];
+};
+BlockArgs check_block_pre(const On& on, const Tensor& qp, const Tensor& kp, const Tensor& vp, const Tensor& cq, const Tensor& ck,
+                          const Tensor& cv, const Tensor& a, const Tensor& b, const Tensor& al, const Tensor& bias, int64_t H,
+                          int64_t Dk, int64_t Dv, bool gate_is_log) {
+  if (qp.dim() != 3) throw py::value_error("q_proj must be [B,T,H*Dk]");
+  const int64_t B = qp.size(0), T = qp.size(1);
+  BlockArgs r{{(int32_t)B, (int32_t)T, (int32_t)H, (int32_t)Dk, (int32_t)Dv, 64, io_code(qp), gate_is_log ? 1 : 0, 0},
+              {B, T, H * Dk}, {B, T, H * Dv}, {B, T, H}};
+  const auto io = qp.scalar_type();
+  const int64_t wk[] = {4, H * Dk}, wv[] = {4, H * Dv};
+  check(qp, r.kd, io, on.dev, "q_proj");
+  check(kp, r.kd, io, on.dev, "k_proj");
+  check(vp, r.vd, io, on.dev, "v_proj");
+  check(cq, wk, F, on.dev, "conv_q");
+  check(ck, wk, F, on.dev, "conv_k");
+  check(cv, wv, F, on.dev, "conv_v");
+  check(a, r.hd, F, on.dev, "a_raw");
+  check(b, r.hd, F, on.dev, "b_raw");
+  check(al, Shape(&H, 1), F, on.dev, "a_log");
+  check(bias, Shape(&H, 1), F, on.dev, "dt_bias");
+  return r;
+}
+py::tuple gdn_block_pre(const Tensor& qp, const Tensor& kp, const Tensor& vp, const Tensor& cq, const Tensor& ck, const Tensor& cv,
+                        const Tensor& a, const Tensor& b, const Tensor& al, const Tensor& bias, int64_t H, int64_t Dk, int64_t Dv,
+                        bool gate_is_log) {
+  On on(qp);
+  BlockArgs x = check_block_pre(on, qp, kp, vp, cq, ck, cv, a, b, al, bias, H, Dk, Dv, gate_is_log);
+  const int64_t k4[] = {x.d.B, x.d.T, H, Dk}, v4[] = {x.d.B, x.d.T, H, Dv};
+  const auto io = qp.scalar_type();
+  Tensor q = make(k4, io, on.dev), k = make(k4, io, on.dev), v = make(v4, io, on.dev), beta = make(x.hd, F, on.dev), gate = make(x.hd, F, on.dev);
+  call("mxb_gdn_block_pre_fwd", abi.mxb_gdn_block_pre_fwd, &x.d, ptr(qp), ptr(kp), ptr(vp), ptr<float>(cq), ptr<float>(ck), ptr<float>(cv),
+       ptr<float>(a), ptr<float>(b), ptr<float>(al), ptr<float>(bias), ptr(q), ptr(k), ptr(v), ptr<float>(beta), ptr<float>(gate), on.stream);
+  return py::make_tuple(q, k, v, beta, gate);
+}
+py::dict gdn_block_pre_backward(const Tensor& qp, const Tensor& kp, const Tensor& vp, const Tensor& cq, const Tensor& ck,
+                                const Tensor& cv, const Tensor& a, const Tensor& b, const Tensor& al, const Tensor& bias, int64_t H,
+                                int64_t Dk, int64_t Dv, const Tensor& dq, const Tensor& dk, const Tensor& dv, const Tensor& dbeta,
+                                const Tensor& dgate, bool gate_is_log) {
+  On on(qp);
+  BlockArgs x = check_block_pre(on, qp, kp, vp, cq, ck, cv, a, b, al, bias, H, Dk, Dv, gate_is_log);
+  const int64_t k4[] = {x.d.B, x.d.T, H, Dk}, v4[] = {x.d.B, x.d.T, H, Dv};
+  const auto io = qp.scalar_type();
+  check(dq, k4, io, on.dev, "dq");
+  check(dk, k4, io, on.dev, "dk");
+  check(dv, v4, io, on.dev, "dv");
+  check(dbeta, x.hd, F, on.dev, "dbeta");
+  check(dgate, x.hd, F, on.dev, "dgate");
+  Tensor dqp = like(qp), dkp = like(kp), dvp = like(vp), dcq = like(cq), dck = like(ck), dcv = like(cv), da = like(a), db = like(b),
+         dal = like(al), dbias = like(bias);
+  Tensor ws = workspace(abi.mxb_gdn_block_workspace_bytes(&x.d), on.dev.index());
+  call("mxb_gdn_block_pre_bwd", abi.mxb_gdn_block_pre_bwd, &x.d, ptr(qp), ptr(kp), ptr(vp), ptr<float>(cq), ptr<float>(ck), ptr<float>(cv),
+       ptr<float>(a), ptr<float>(b), ptr<float>(al), ptr<float>(bias), ptr(dq), ptr(dk), ptr(dv), ptr<float>(dbeta), ptr<float>(dgate),
+       ptr(dqp), ptr(dkp), ptr(dvp), ptr<float>(dcq), ptr<float>(dck), ptr<float>(dcv), ptr<float>(da), ptr<float>(db), ptr<float>(dal),
+       ptr<float>(dbias), ptr(ws), (size_t)ws.numel(), on.stream);
+  py::dict r;
+  r["dq_proj"] = dqp; r["dk_proj"] = dkp; r["dv_proj"] = dvp; r["dconv_q"] = dcq; r["dconv_k"] = dck; r["dconv_v"] = dcv;
+  r["da_raw"] = da; r["db_raw"] = db; r["da_log"] = dal; r["ddt_bias"] = dbias;
+  return r;
+}
+mxb_gdn_desc check_block_post(const On& on, const Tensor& o, const Tensor& z, const Tensor& w) {
+  if (o.dim() != 4) throw py::value_error("o must be [B,T,H,Dv]");
+  const int64_t B = o.size(0), T = o.size(1), H = o.size(2), Dv = o.size(3), zd[] = {B, T, H * Dv};
+  const mxb_gdn_desc d{(int32_t)B, (int32_t)T, (int32_t)H, 8, (int32_t)Dv, 64, io_code(o), 0, 0};
+  check(o, o.sizes(), o.scalar_type(), on.dev, "o");
+  check(z, zd, o.scalar_type(), on.dev, "z");
+  check(w, Shape(&Dv, 1), F, on.dev, "o_norm");
+  return d;
+}
+Tensor gdn_block_post(const Tensor& o, const Tensor& z, const Tensor& w) {
+  On on(o);
+  const mxb_gdn_desc d = check_block_post(on, o, z, w);
+  Tensor y = like(z);
+  call("mxb_gdn_block_post_fwd", abi.mxb_gdn_block_post_fwd, &d, ptr(o), ptr(z), ptr<float>(w), ptr(y), on.stream);
+  return y;
+}
+py::dict gdn_block_post_backward(const Tensor& o, const Tensor& z, const Tensor& w, const Tensor& dy) {
+  On on(o);
+  const mxb_gdn_desc d = check_block_post(on, o, z, w);
+  check(dy, z.sizes(), o.scalar_type(), on.dev, "dy");
+  Tensor d_o = like(o), dz = like(z), dw = like(w);
+  Tensor ws = workspace(abi.mxb_gdn_block_workspace_bytes(&d), on.dev.index());
+  call("mxb_gdn_block_post_bwd", abi.mxb_gdn_block_post_bwd, &d, ptr(o), ptr(z), ptr<float>(w), ptr(dy), ptr(d_o), ptr(dz), ptr<float>(dw),
+       ptr(ws), (size_t)ws.numel(), on.stream);
+  py::dict r;
+  r["do"] = d_o; r["dz"] = dz; r["do_norm"] = dw;
+  return r;
+}
+
+// ------------------------------------------------------------------ Mamba-3 scan
+mxb_mamba3_desc check_mamba3(const On& on, const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta,
+                             const Tensor& a_log, const Tensor& b, const Tensor& c, int64_t nheads, int64_t flags) {
+  if (x.dim() != 3 || b.dim() != 4) throw py::value_error("x must be [B,T,D] and b, c [B,T,G,N]");
+  const int64_t B = x.size(0), T = x.size(1), D = x.size(2), G = b.size(2), N = b.size(3);
+  const mxb_mamba3_desc d{(int32_t)B, (int32_t)T, (int32_t)D, (int32_t)N, (int32_t)G, (int32_t)nheads, io_code(x), (int32_t)flags};
+  const auto io = x.scalar_type();
+  const int64_t per[] = {B, T, nheads > 0 ? nheads : D, N / 2}, al[] = {nheads > 0 ? nheads : D, N}, gn[] = {B, T, G, N};
+  check(x, x.sizes(), io, on.dev, "x");
+  check(dt, Shape(per, 3), F, on.dev, "dt");
+  check(lam, Shape(per, 3), F, on.dev, "lambda");
+  check(theta, Shape(per, nheads > 0 ? 3 : 4), F, on.dev, "theta");
+  check(a_log, Shape(al, nheads > 0 ? 1 : 2), F, on.dev, "a_log");
+  check(b, gn, io, on.dev, "b");
+  check(c, gn, io, on.dev, "c");
+  return d;
+}
+Tensor mamba3_forward(const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta, const Tensor& a_log, const Tensor& b,
+                      const Tensor& c, int64_t nheads, int64_t flags, bool save) {
+  On on(x);
+  const mxb_mamba3_desc d = check_mamba3(on, x, dt, lam, theta, a_log, b, c, nheads, save ? flags | MXB_MAMBA3_SAVE_FOR_BWD : flags);
+  Tensor y = like(x);
+  Tensor ws = workspace(abi.mxb_mamba3_fwd_workspace_bytes(&d), on.dev.index());
+  call("mxb_mamba3_fwd", abi.mxb_mamba3_fwd, &d, ptr(x), ptr<float>(dt), ptr<float>(lam), ptr<float>(theta), ptr<float>(a_log), ptr(b), ptr(c),
+       ptr(y), ptr(ws), (size_t)ws.numel(), on.stream);
+  if (save) workspaces()[on.dev.index()].saved = token(2, on.stream, {&x, &dt, &lam, &theta, &a_log, &b, &c}, {nheads});
+  return y;
+}
+py::dict mamba3_backward(const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta, const Tensor& a_log, const Tensor& b,
+                         const Tensor& c, const Tensor& dy, int64_t nheads, int64_t flags, bool use_saved) {
+  On on(x);
+  const mxb_mamba3_desc d = check_mamba3(on, x, dt, lam, theta, a_log, b, c, nheads, use_saved ? flags | MXB_MAMBA3_BWD_USE_SAVED : flags);
+  check(dy, x.sizes(), x.scalar_type(), on.dev, "dy");
+  const size_t nws = abi.mxb_mamba3_bwd_workspace_bytes(&d);
+  Tensor ws = use_saved ? saved_workspace(token(2, on.stream, {&x, &dt, &lam, &theta, &a_log, &b, &c}, {nheads}), nws, on.dev.index(),
+                                          "mamba3_selective_scan_backward")
+                        : workspace(nws, on.dev.index());
+  Tensor dx = like(x), ddt = like(dt), dlam = like(lam), dth = like(theta), dal = like(a_log), db = like(b), dc = like(c);
+  call("mxb_mamba3_bwd", abi.mxb_mamba3_bwd, &d, ptr(x), ptr<float>(dt), ptr<float>(lam), ptr<float>(theta), ptr<float>(a_log), ptr(b), ptr(c),
+       ptr(dy), ptr(dx), ptr<float>(ddt), ptr<float>(dlam), ptr<float>(dth), ptr<float>(dal), ptr(db), ptr(dc), ptr(ws), (size_t)ws.numel(),
+       on.stream);
+  py::dict r;
+  r["dx"] = dx; r["ddt"] = ddt; r["dlambda"] = dlam; r["dtheta"] = dth; r["da_log"] = dal; r["db"] = db; r["dc"] = dc;
+  return r;
+}
+
+// ------------------------------------------------------------------ Mamba-3 block stages
+mxb_mamba3_desc m3_rows(const Tensor& x) {
+  if (x.dim() != 3) throw py::value_error("expected a [B,T,D] tensor");
+  return {(int32_t)x.size(0), (int32_t)x.size(1), (int32_t)x.size(2), 8, 1, 0, io_code(x), 0};
+}
+mxb_mamba3_desc check_conv(const On& on, const Tensor& x, const Tensor& w) {
+  const mxb_mamba3_desc d = m3_rows(x);
+  const int64_t wd[] = {d.D, w.dim() ? w.size(-1) : 0};
+  check(x, x.sizes(), x.scalar_type(), on.dev, "x");
+  check(w, wd, F, on.dev, "w");
+  return d;
+}
+Tensor mamba3_block_conv(const Tensor& x, const Tensor& w) {
+  On on(x);
+  const mxb_mamba3_desc d = check_conv(on, x, w);
+  Tensor y = like(x);
+  call("mxb_mamba3_block_conv_fwd", abi.mxb_mamba3_block_conv_fwd, &d, (int32_t)w.size(1), ptr(x), ptr<float>(w), ptr(y), on.stream);
+  return y;
+}
+py::dict mamba3_block_conv_backward(const Tensor& x, const Tensor& w, const Tensor& dy) {
+  On on(x);
+  const mxb_mamba3_desc d = check_conv(on, x, w);
+  check(dy, x.sizes(), x.scalar_type(), on.dev, "dy");
+  Tensor dx = like(x), dw = like(w);
+  Tensor ws = workspace(abi.mxb_mamba3_block_workspace_bytes(&d), on.dev.index());
+  call("mxb_mamba3_block_conv_bwd", abi.mxb_mamba3_block_conv_bwd, &d, (int32_t)w.size(1), ptr(x), ptr<float>(w), ptr(dy), ptr(dx),
+       ptr<float>(dw), ptr(ws), (size_t)ws.numel(), on.stream);
+  py::dict r;
+  r["dx"] = dx; r["dw"] = dw;
+  return r;
+}
+mxb_mamba3_desc check_bc(const On& on, const Tensor& bp, const Tensor& cp, const Tensor& bs, const Tensor& cs, int64_t G, int64_t N) {
+  if (bp.dim() != 3) throw py::value_error("b_proj must be [B,T,G*N]");
+  const int64_t gn[] = {bp.size(0), bp.size(1), G * N};
+  const mxb_mamba3_desc d{(int32_t)gn[0], (int32_t)gn[1], 8, (int32_t)N, (int32_t)G, 0, io_code(bp), 0};
+  check(bp, gn, bp.scalar_type(), on.dev, "b_proj");
+  check(cp, gn, bp.scalar_type(), on.dev, "c_proj");
+  check(bs, Shape(&N, 1), F, on.dev, "b_scale");
+  check(cs, Shape(&N, 1), F, on.dev, "c_scale");
+  return d;
+}
+py::tuple mamba3_block_bc(const Tensor& bp, const Tensor& cp, const Tensor& bs, const Tensor& cs, const Tensor& bb, const Tensor& cb,
+                          int64_t G, int64_t N, double eps) {
+  On on(bp);
+  const mxb_mamba3_desc d = check_bc(on, bp, cp, bs, cs, G, N);
+  const int64_t gn = G * N, o4[] = {d.B, d.T, G, N};
+  check(bb, Shape(&gn, 1), F, on.dev, "b_bias");
+  check(cb, Shape(&gn, 1), F, on.dev, "c_bias");
+  Tensor b = make(o4, bp.scalar_type(), on.dev), c = make(o4, bp.scalar_type(), on.dev);
+  call("mxb_mamba3_block_bc_fwd", abi.mxb_mamba3_block_bc_fwd, &d, (float)eps, ptr(bp), ptr(cp), ptr<float>(bs), ptr<float>(cs),
+       ptr<float>(bb), ptr<float>(cb), ptr(b), ptr(c), on.stream);
+  return py::make_tuple(b, c);
+}
+py::dict mamba3_block_bc_backward(const Tensor& bp, const Tensor& cp, const Tensor& bs, const Tensor& cs, const Tensor& db,
+                                  const Tensor& dc, int64_t G, int64_t N, double eps) {
+  On on(bp);
+  const mxb_mamba3_desc d = check_bc(on, bp, cp, bs, cs, G, N);
+  const int64_t gn = G * N, o4[] = {d.B, d.T, G, N};
+  check(db, o4, bp.scalar_type(), on.dev, "db");
+  check(dc, o4, bp.scalar_type(), on.dev, "dc");
+  Tensor dbp = like(bp), dcp = like(cp), dbs = like(bs), dcs = like(cs), dbb = make(Shape(&gn, 1), F, on.dev), dcb = make(Shape(&gn, 1), F, on.dev);
+  Tensor ws = workspace(abi.mxb_mamba3_block_workspace_bytes(&d), on.dev.index());
+  call("mxb_mamba3_block_bc_bwd", abi.mxb_mamba3_block_bc_bwd, &d, (float)eps, ptr(bp), ptr(cp), ptr<float>(bs), ptr<float>(cs), ptr(db),
+       ptr(dc), ptr(dbp), ptr(dcp), ptr<float>(dbs), ptr<float>(dcs), ptr<float>(dbb), ptr<float>(dcb), ptr(ws), (size_t)ws.numel(),
+       on.stream);
+  py::dict r;
+  r["db_proj"] = dbp; r["dc_proj"] = dcp; r["db_scale"] = dbs; r["dc_scale"] = dcs; r["db_bias"] = dbb; r["dc_bias"] = dcb;
+  return r;
+}
+mxb_mamba3_desc check_post(const On& on, const Tensor& y, const Tensor& z, const Tensor& w) {
+  const mxb_mamba3_desc d = m3_rows(y);
+  const int64_t D = d.D;
+  check(y, y.sizes(), y.scalar_type(), on.dev, "y");
+  check(z, y.sizes(), y.scalar_type(), on.dev, "z");
+  check(w, Shape(&D, 1), F, on.dev, "post_norm");
+  return d;
+}
+Tensor mamba3_block_post(const Tensor& y, const Tensor& z, const Tensor& w, double eps) {
+  On on(y);
+  const mxb_mamba3_desc d = check_post(on, y, z, w);
+  Tensor out = like(y);
+  call("mxb_mamba3_block_post_fwd", abi.mxb_mamba3_block_post_fwd, &d, (float)eps, ptr(y), ptr(z), ptr<float>(w), ptr(out), on.stream);
+  return out;
+}
+py::dict mamba3_block_post_backward(const Tensor& y, const Tensor& z, const Tensor& w, const Tensor& dout, double eps) {
+  On on(y);
+  const mxb_mamba3_desc d = check_post(on, y, z, w);
+  check(dout, y.sizes(), y.scalar_type(), on.dev, "dout");
+  Tensor dy = like(y), dz = like(z), dw = like(w);
+  Tensor ws = workspace(abi.mxb_mamba3_block_workspace_bytes(&d), on.dev.index());
+  call("mxb_mamba3_block_post_bwd", abi.mxb_mamba3_block_post_bwd, &d, (float)eps, ptr(y), ptr(z), ptr<float>(w), ptr(dout), ptr(dy), ptr(dz),
+       ptr<float>(dw), ptr(ws), (size_t)ws.numel(), on.stream);
+  py::dict r;
+  r["dy"] = dy; r["dz"] = dz; r["dpost_norm"] = dw;
+  return r;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_front, m) {
+  m.def("open", &open_library);
+  m.def("workspace", &workspace);
+  m.def("gdn_forward", &gdn_forward);
+  m.def("gdn_backward", &gdn_backward);
+  m.def("gdn_decode", &gdn_decode);
+  m.def("gdn_block_pre", &gdn_block_pre);
+  m.def("gdn_block_pre_backward", &gdn_block_pre_backward);
+  m.def("gdn_block_post", &gdn_block_post);
+  m.def("gdn_block_post_backward", &gdn_block_post_backward);
+  m.def("mamba3_forward", &mamba3_forward);
+  m.def("mamba3_backward", &mamba3_backward);
+  m.def("mamba3_block_conv", &mamba3_block_conv);
+  m.def("mamba3_block_conv_backward", &mamba3_block_conv_backward);
+  m.def("mamba3_block_bc", &mamba3_block_bc);
+  m.def("mamba3_block_bc_backward", &mamba3_block_bc_backward);
+  m.def("mamba3_block_post", &mamba3_block_post);
+  m.def("mamba3_block_post_backward", &mamba3_block_post_backward);
+}

@@ -1371,15 +1371,6 @@ bool gdn_simt_supported(const mxb_gdn_desc* d) {
   return d->Dk >= 1 && d->Dv >= 1 && d->Dk <= 128 && d->Dv <= 256;
 }
 
-template <typename KernelT>
-static mxb_status set_smem(KernelT kern, size_t bytes) {
-  if (bytes > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) { set_last_cuda_error((int)e); return MXB_ERR_CUDA; }
-  }
-  return MXB_OK;
-}
-
 // Rows can be moved four elements at a time where the width is a multiple of four and every tensor of that width is
 // aligned to four elements (the workspace always is).
 template <typename IO>
@@ -1397,7 +1388,7 @@ static mxb_status run_prep(GdnP p, cudaStream_t st) {
           make_tma_map_f32(&maps.k, p.k, p.B, p.T, p.H, p.K);
   p.vtma = sizeof(IO) == 4 && p.C == simt::R && make_tma_map_f32(&maps.P, p.v, p.B, p.T, p.H, p.V);
   constexpr int sm = PrepF32<KP>::smem;
-  if (set_smem(gdn_prep_kernel<IO, KP>, sm) != MXB_OK) return MXB_ERR_CUDA;
+  if (MXB_ALLOW_SMEM(sm, gdn_prep_kernel<IO, KP>) != MXB_OK) return MXB_ERR_CUDA;
   MXB_LAUNCH("gdn_prep_kernel", st, (gdn_prep_kernel<IO, KP><<<dim3(p.n, p.B * p.H), 256, sm, st>>>(p, maps)));
   return check_launch("gdn_prep_kernel");
 }
@@ -1420,12 +1411,12 @@ static mxb_status run_state(GdnP p, bool bwd, cudaStream_t st) {
   const dim3 grid((p.V + W - 1) / W, p.B * p.H);
   if (bwd) {
     constexpr int sm = state_bwd_smem<W, KP>();
-    if (set_smem(gdn_state_bwd_kernel<IO, W, KP>, sm) != MXB_OK) return MXB_ERR_CUDA;
+    if (MXB_ALLOW_SMEM(sm, gdn_state_bwd_kernel<IO, W, KP>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_state_bwd_kernel", st, (gdn_state_bwd_kernel<IO, W, KP><<<grid, 256, sm, st>>>(p, maps)));
     return check_launch("gdn_state_bwd_kernel");
   }
   constexpr int sm = state_fwd_smem<W, KP>();
-  if (set_smem(gdn_state_fwd_kernel<IO, W, KP>, sm) != MXB_OK) return MXB_ERR_CUDA;
+  if (MXB_ALLOW_SMEM(sm, gdn_state_fwd_kernel<IO, W, KP>) != MXB_OK) return MXB_ERR_CUDA;
   MXB_LAUNCH("gdn_state_fwd_kernel", st, (gdn_state_fwd_kernel<IO, W, KP><<<grid, 256, sm, st>>>(p, maps)));
   return check_launch("gdn_state_fwd_kernel");
 }
@@ -1440,7 +1431,7 @@ static mxb_status run_state(const GdnP& p, bool bwd, cudaStream_t st) {
 }
 template <typename IO, int NGK>
 static mxb_status run_chunk_bwd(const GdnP& p, cudaStream_t st) {
-  if (set_smem(gdn_chunk_bwd_kernel<IO, NGK>, kChunkF32Smem) != MXB_OK) return MXB_ERR_CUDA;
+  if (MXB_ALLOW_SMEM(kChunkF32Smem, gdn_chunk_bwd_kernel<IO, NGK>) != MXB_OK) return MXB_ERR_CUDA;
   MXB_LAUNCH("gdn_chunk_bwd_kernel", st,
              (gdn_chunk_bwd_kernel<IO, NGK><<<dim3(p.n, p.B * p.H), 256, kChunkF32Smem, st>>>(p)));
   return check_launch("gdn_chunk_bwd_kernel");
@@ -1452,7 +1443,7 @@ static mxb_status run_fwd(GdnP& p, bool chunked, cudaStream_t st) {
   if (!chunked) {
     dim3 gslab((V + 31) / 32, p.B * p.H);
     size_t sm = sizeof(float) * (K * 33 + 2 * K + 512);
-    if (set_smem(gdn_recurrent_fwd_kernel<IO>, sm) != MXB_OK) return MXB_ERR_CUDA;
+    if (MXB_ALLOW_SMEM((int)sm, gdn_recurrent_fwd_kernel<IO>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_recurrent_fwd_kernel", st, (gdn_recurrent_fwd_kernel<IO><<<gslab, 256, sm, st>>>(p)));
     return check_launch("gdn_recurrent_fwd_kernel");
   }

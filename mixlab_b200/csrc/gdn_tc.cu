@@ -77,6 +77,8 @@ __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid
     return (uint32_t)(c8 >> 3) * 16384u + (uint32_t)i * 128u + (uint32_t)(((c8 & 7) ^ (i & 7)) << 4);
   };
 
+  // The first CTA clears the status header: whoever raises it has waited in vain for far longer than this takes.
+  if (c == 0 && bh == 0 && tid < 64) p.status[tid] = 0;
   // prologue latencies side by side: warp 0 allocates TMEM, warp 1 reads the gates, one thread of warp 2
   // initialises the barriers and issues the copies that complete on them
   if (tid == 64) {
@@ -704,13 +706,6 @@ size_t gdn_tc_workspace_bytes(const mxb_gdn_desc* d, bool bwd) {
   return own > simt ? own : simt;
 }
 
-template <typename KernelT>
-static mxb_status tc_set_smem(KernelT kern, int bytes) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e != cudaSuccess) { set_last_cuda_error((int)e); return MXB_ERR_CUDA; }
-  return MXB_OK;
-}
-
 mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st);
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).
@@ -753,8 +748,6 @@ static bool g_tc_use_tma = true;
 void gdn_tc_set_tma(bool on) { g_tc_use_tma = on; }
 
 mxb_status tc_run_fwd(TcP& p, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(p.status, 0, 256, st);
-  if (e != cudaSuccess) { set_last_cuda_error((int)e); return MXB_ERR_CUDA; }
   PrepMaps maps;
   std::memset(&maps, 0, sizeof maps);
   // heads narrower than the tiles exist only through the copy engine (the per-thread staging addresses full rows)
@@ -764,22 +757,22 @@ mxb_status tc_run_fwd(TcP& p, cudaStream_t st) {
                    make_tma_map_bthd(&maps.o, p.out, p.B, p.T, p.H, p.Dv);
   if (narrow && !tma) return MXB_ERR_UNSUPPORTED;
   if (tma) {
-    if (tc_set_smem(gdn_tc_prep_kernel<true>, kPrepSmem) != MXB_OK) return MXB_ERR_CUDA;
+    if (MXB_ALLOW_SMEM(kPrepSmem, gdn_tc_prep_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_prep_kernel", st,
                (gdn_tc_prep_kernel<true><<<dim3(p.n, p.B * p.H), 128, kPrepSmem, st>>>(p, maps)));
   } else {
-    if (tc_set_smem(gdn_tc_prep_kernel<false>, kPrepSmem) != MXB_OK) return MXB_ERR_CUDA;
+    if (MXB_ALLOW_SMEM(kPrepSmem, gdn_tc_prep_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_prep_kernel", st,
                (gdn_tc_prep_kernel<false><<<dim3(p.n, p.B * p.H), 128, kPrepSmem, st>>>(p, maps)));
   }
   mxb_status s = check_launch("gdn_tc_prep_kernel");
   if (s != MXB_OK) return s;
   if (tma) {
-    if (tc_set_smem(gdn_tc_state_fwd_kernel<true>, kStateFwdSmem) != MXB_OK) return MXB_ERR_CUDA;
+    if (MXB_ALLOW_SMEM(kStateFwdSmem, gdn_tc_state_fwd_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_state_fwd_kernel", st,
                (gdn_tc_state_fwd_kernel<true><<<dim3(p.B * p.H), 256, kStateFwdSmem, st>>>(p, maps)));
   } else {
-    if (tc_set_smem(gdn_tc_state_fwd_kernel<false>, kStateFwdSmem) != MXB_OK) return MXB_ERR_CUDA;
+    if (MXB_ALLOW_SMEM(kStateFwdSmem, gdn_tc_state_fwd_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_state_fwd_kernel", st,
                (gdn_tc_state_fwd_kernel<false><<<dim3(p.B * p.H), 256, kStateFwdSmem, st>>>(p, maps)));
   }

@@ -722,13 +722,6 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
 // ------------------------------------------------------------------ host
 mxb_status tc_run_fwd(TcP& p, cudaStream_t st);
 
-template <typename KernelT>
-static mxb_status bwd_set_smem(KernelT kern, int bytes) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e != cudaSuccess) { set_last_cuda_error((int)e); return MXB_ERR_CUDA; }
-  return MXB_OK;
-}
-
 // Forward recompute (saving per-chunk states and v_new), reverse state pass, per-chunk pass.
 mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st) {
   p.save = 1;
@@ -751,11 +744,11 @@ mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st) {
                    make_tma_map_bthd(&maps.dO, p.dO, p.B, p.T, p.H, p.Dv);
   if (narrow && !tma) return MXB_ERR_UNSUPPORTED;
   if (tma) {
-    if (bwd_set_smem(gdn_tc_state_bwd_kernel<true>, kStateBwdSmem) != MXB_OK) return MXB_ERR_CUDA;
+    if (MXB_ALLOW_SMEM(kStateBwdSmem, gdn_tc_state_bwd_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_state_bwd_kernel", st,
                (gdn_tc_state_bwd_kernel<true><<<dim3(p.B * p.H), 256, kStateBwdSmem, st>>>(p, maps)));
   } else {
-    if (bwd_set_smem(gdn_tc_state_bwd_kernel<false>, kStateBwdSmem) != MXB_OK) return MXB_ERR_CUDA;
+    if (MXB_ALLOW_SMEM(kStateBwdSmem, gdn_tc_state_bwd_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_state_bwd_kernel", st,
                (gdn_tc_state_bwd_kernel<false><<<dim3(p.B * p.H), 256, kStateBwdSmem, st>>>(p, maps)));
   }
@@ -772,7 +765,7 @@ mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st) {
   if (!(make_tma_map_bthd(&maps.dq, p.dq, p.B, p.T, p.H, p.Dk) && make_tma_map_bthd(&maps.dk, p.dk, p.B, p.T, p.H, p.Dk) &&
         make_tma_map_bthd(&maps.dv, p.dv, p.B, p.T, p.H, p.Dv)))
     return MXB_ERR_UNSUPPORTED;
-  if (bwd_set_smem(gdn_tc_chunk_bwd_kernel, kChunkBwdSmem) != MXB_OK) return MXB_ERR_CUDA;
+  if (MXB_ALLOW_SMEM(kChunkBwdSmem, gdn_tc_chunk_bwd_kernel) != MXB_OK) return MXB_ERR_CUDA;
   MXB_LAUNCH("gdn_tc_chunk_bwd_kernel", st,
              (gdn_tc_chunk_bwd_kernel<<<dim3(p.B * p.H, p.n), 256, kChunkBwdSmem, st>>>(p, maps)));
   return check_launch("gdn_tc_chunk_bwd_kernel");

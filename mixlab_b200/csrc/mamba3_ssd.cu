@@ -284,6 +284,7 @@ __global__ void __launch_bounds__(kScalThreads) m3s_scalars_kernel(SsdP p) {
   const int head = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const size_t base = ((size_t)b * p.NH + head) * p.T;
   const int per = (p.T + kScalThreads - 1) / kScalThreads, lo = tid * per, hi = min(p.T, lo + per);
+  if (head == 0 && b == 0 && tid < 64) p.status[tid] = 0;  // (the kernels behind this one raise it)
   // Batches of kScalBatch steps: all loads of a batch are issued before its first store (a store in between would
   // pin the order, since the compiler cannot prove the arrays distinct, and every step would pay a full memory latency).
   double acc = 0.0;
@@ -1082,13 +1083,6 @@ size_t mamba3_ssd_workspace_bytes(const mxb_mamba3_desc* d, bool bwd) {
   return carve_ssd(p, nullptr, bwd);
 }
 
-template <typename KernelT>
-static mxb_status ssd_smem(KernelT k, size_t bytes) {
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) { set_last_cuda_error((int)e); return MXB_ERR_CUDA; }
-  return MXB_OK;
-}
-
 bool make_tma_map_bthd(CUtensorMap* m, const void* base, int B, int T, int H, int D);
 
 // Tensor maps for the token-indexed operands of the chunk kernels (dy only in the backward); false when one
@@ -1111,11 +1105,11 @@ static mxb_status ssd_state_pass(SsdP& p, int mode, cudaStream_t st) {
   const bool tma = !p.no_tma && make_tma_map_bthd(&maps.r, mode == 0 ? p.b : p.c, p.B, p.T, p.G, m3s::N) &&
                    make_tma_map_bthd(&maps.x, mode == 0 ? p.x : p.dy, p.B, p.T, p.NH, m3s::P);
   if (tma) {
-    if (ssd_smem(m3s::m3s_state_pass_kernel<true>, m3s::kPassSmem) != MXB_OK) return MXB_ERR_CUDA;
+    if (MXB_ALLOW_SMEM(m3s::kPassSmem, m3s::m3s_state_pass_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("m3s_state_pass_kernel", st,
                (m3s::m3s_state_pass_kernel<true><<<dim3(p.NH, p.B), 256, m3s::kPassSmem, st>>>(p, mode, maps)));
   } else {
-    if (ssd_smem(m3s::m3s_state_pass_kernel<false>, m3s::kPassSmem) != MXB_OK) return MXB_ERR_CUDA;
+    if (MXB_ALLOW_SMEM(m3s::kPassSmem, m3s::m3s_state_pass_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("m3s_state_pass_kernel", st,
                (m3s::m3s_state_pass_kernel<false><<<dim3(p.NH, p.B), 256, m3s::kPassSmem, st>>>(p, mode, maps)));
   }
@@ -1124,7 +1118,6 @@ static mxb_status ssd_state_pass(SsdP& p, int mode, cudaStream_t st) {
 
 static mxb_status ssd_forward(SsdP& p, cudaStream_t st) {
   const dim3 gc(p.n, p.NH, p.B);
-  if (cudaMemsetAsync(p.status, 0, 256, st) != cudaSuccess) return MXB_ERR_CUDA;
   MXB_LAUNCH("m3s_scalars_kernel", st, (m3s::m3s_scalars_kernel<<<dim3(p.NH, p.B), m3s::kScalThreads, 0, st>>>(p)));
   MXB_LAUNCH("m3s_chunk_scalars_kernel", st, (m3s::m3s_chunk_scalars_kernel<<<gc, 64, 0, st>>>(p)));
   mxb_status ps = ssd_state_pass(p, 0, st);
@@ -1132,10 +1125,10 @@ static mxb_status ssd_forward(SsdP& p, cudaStream_t st) {
   if (p.y) {
     m3s::ChunkMaps maps;
     if (ssd_chunk_maps(p, maps)) {
-      if (ssd_smem(m3s::m3s_chunk_out_kernel<true>, m3s::kOutSmem) != MXB_OK) return MXB_ERR_CUDA;
+      if (MXB_ALLOW_SMEM(m3s::kOutSmem, m3s::m3s_chunk_out_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
       MXB_LAUNCH("m3s_chunk_out_kernel", st, (m3s::m3s_chunk_out_kernel<true><<<gc, 128, m3s::kOutSmem, st>>>(p, maps)));
     } else {
-      if (ssd_smem(m3s::m3s_chunk_out_kernel<false>, m3s::kOutSmem) != MXB_OK) return MXB_ERR_CUDA;
+      if (MXB_ALLOW_SMEM(m3s::kOutSmem, m3s::m3s_chunk_out_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
       MXB_LAUNCH("m3s_chunk_out_kernel", st, (m3s::m3s_chunk_out_kernel<false><<<gc, 128, m3s::kOutSmem, st>>>(p, maps)));
     }
   }
@@ -1163,9 +1156,8 @@ mxb_status mamba3_ssd_bwd(const mxb_mamba3_desc* d, const void* x, const float* 
   p.ddt = ddt; p.dlam = dlam; p.dtheta = dtheta; p.da_log = da_log;
   carve_ssd(p, ws, true);
   p.y = nullptr;  // the forward recompute stops at the chunk states
-  if (d->flags & MXB_MAMBA3_BWD_USE_SAVED) {  // dt, lambda, phi, the chunk decays and H0 are still in place
-    if (cudaMemsetAsync(p.status, 0, 256, st) != cudaSuccess) return MXB_ERR_CUDA;
-  } else {
+  // with saved intermediates dt, lambda, phi, the chunk decays and H0 are still in place
+  if (!(d->flags & MXB_MAMBA3_BWD_USE_SAVED)) {
     mxb_status s = ssd_forward(p, st);
     if (s != MXB_OK) return s;
   }
@@ -1174,10 +1166,10 @@ mxb_status mamba3_ssd_bwd(const mxb_mamba3_desc* d, const void* x, const float* 
   if (ps != MXB_OK) return ps;
   m3s::ChunkMaps maps;
   if (ssd_chunk_maps(p, maps)) {
-    if (ssd_smem(m3s::m3s_chunk_grad_kernel<true>, m3s::kGradSmem) != MXB_OK) return MXB_ERR_CUDA;
+    if (MXB_ALLOW_SMEM(m3s::kGradSmem, m3s::m3s_chunk_grad_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("m3s_chunk_grad_kernel", st, (m3s::m3s_chunk_grad_kernel<true><<<gc, 256, m3s::kGradSmem, st>>>(p, maps)));
   } else {
-    if (ssd_smem(m3s::m3s_chunk_grad_kernel<false>, m3s::kGradSmem) != MXB_OK) return MXB_ERR_CUDA;
+    if (MXB_ALLOW_SMEM(m3s::kGradSmem, m3s::m3s_chunk_grad_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("m3s_chunk_grad_kernel", st, (m3s::m3s_chunk_grad_kernel<false><<<gc, 256, m3s::kGradSmem, st>>>(p, maps)));
   }
   MXB_LAUNCH("m3s_final_kernel", st, (m3s::m3s_final_kernel<<<dim3(p.NH, p.B), m3s::kScalThreads, 0, st>>>(p)));
