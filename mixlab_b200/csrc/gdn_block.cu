@@ -7,20 +7,19 @@
 // and their backward passes.  All of it is an HBM stream: every element is read once (plus a 3-step halo of the
 // convolution) and written once, in 16-byte pieces.
 //
-// Work split: a row is one (batch, step, head) vector of D <= 128 channels; a thread owns 8 consecutive channels
-// (one 16-byte bf16 unit), so 16 lanes cover a row and the row reductions are 4 shuffles.  For the convolution a
-// lane group walks kRun consecutive steps of one (batch, head) with the previous three inputs in registers.
+// Work split: a row is one (batch, step, head) vector of D <= 128 channels; as many lanes as it needs (a power of two)
+// cover it with 4 channels each (convolution stages) or 8 (output stage).
 // Sums over (batch, step) - convolution weight, norm weight, A_log, dt_bias gradients - go through per-CTA partial
 // rows in the workspace and a fixed-order second pass (no atomics).
+#include <type_traits>
+
 #include "common.cuh"
+#include "packed.cuh"
 
 namespace mxb {
 namespace blk {
 
 using bf16 = __nv_bfloat16;
-constexpr int kRun = 16;      // steps per lane group (3 more are recomputed as halo in the backward)
-constexpr int kGroups = 8;    // lane groups per CTA (128 threads)
-constexpr int kTile = kRun * kGroups;
 
 struct BlockP {
   int B, T, H, Dk, Dv, gate_is_log;
@@ -55,14 +54,6 @@ __device__ __forceinline__ void store8<bf16>(bf16* p, const float (&e)[8]) {
   for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(e[2 * i], e[2 * i + 1]);
   *reinterpret_cast<uint4*>(p) = v;
 }
-// sum over the 16 lanes of a group.  The mask names only the caller's half of the warp: the two lane groups of a
-// warp may run different numbers of loop iterations, so neither may wait for the other.
-__device__ __forceinline__ float group_sum(float v) {
-  const unsigned mask = 0xffffu << (threadIdx.x & 16);
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
-  return v;
-}
 __device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 // sigmoid for the streams: bf16 I/O takes tanh.approx (one MUFU op, relative error ~5e-4, far below the rounding
 // of the stored result); fp32 I/O takes exp + reciprocal (a few ulp)
@@ -89,61 +80,150 @@ struct PreArgs {
   float* dwp[3];         // backward: per-CTA partial rows [B*ntiles][4][H*D]
 };
 
-// ------------------------------------------------------------------ pre: forward
-// grid (3 * ntiles, H, B) x 128.  blockIdx.x / ntiles selects q, k or v.
+// Four channels of a step as they come from memory, and widened to two packed pairs.
 template <typename IO>
-__global__ void __launch_bounds__(128) gdn_block_pre_fwd_kernel(BlockP p, PreArgs<IO> a, int ntiles) {
-  const int which = blockIdx.x / ntiles, tile = blockIdx.x % ntiles;
-  const int h = blockIdx.y, b = blockIdx.z;
+struct Raw4 { uint2 v; };
+template <>
+struct Raw4<float> { float4 v; };
+__device__ __forceinline__ void load_raw(Raw4<bf16>& r, const bf16* p, bool ok) {
+  r.v = ok ? __ldg(reinterpret_cast<const uint2*>(p)) : make_uint2(0u, 0u);
+}
+__device__ __forceinline__ void load_raw(Raw4<float>& r, const float* p, bool ok) {
+  r.v = ok ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+__device__ __forceinline__ void widen(f2 (&e)[2], const Raw4<bf16>& r) {
+  e[0] = pack2(__uint_as_float(r.v.x << 16), __uint_as_float(r.v.x & 0xffff0000u));
+  e[1] = pack2(__uint_as_float(r.v.y << 16), __uint_as_float(r.v.y & 0xffff0000u));
+}
+__device__ __forceinline__ void widen(f2 (&e)[2], const Raw4<float>& r) {
+  e[0] = pack2(r.v.x, r.v.y);
+  e[1] = pack2(r.v.z, r.v.w);
+}
+__device__ __forceinline__ void store_pairs(bf16* p, const f2 (&e)[2]) {
+  const float2 a = unpack2(e[0]), b = unpack2(e[1]);
+  __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(b.x, b.y);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+}
+__device__ __forceinline__ void store_pairs(float* p, const f2 (&e)[2]) {
+  const float2 a = unpack2(e[0]), b = unpack2(e[1]);
+  *reinterpret_cast<float4*>(p) = make_float4(a.x, a.y, b.x, b.y);
+}
+template <typename IO>
+__device__ __forceinline__ f2 sigmoid_pair(f2 x) {
+  const float2 a = unpack2(x);
+  return pack2(sigmoid_io<IO>(a.x), sigmoid_io<IO>(a.y));
+}
+template <>
+__device__ __forceinline__ f2 sigmoid_pair<bf16>(f2 x) {
+  float2 a = unpack2(mul2(x, dup2(0.5f)));
+  asm("tanh.approx.f32 %0, %0;" : "+f"(a.x));
+  asm("tanh.approx.f32 %0, %0;" : "+f"(a.y));
+  return mad2(pack2(a.x, a.y), dup2(0.5f), dup2(0.5f));
+}
+// Row sums of four steps at once over the LPR lanes of a row: lane l ends up with the sum of step l & 3.  Halving
+// exchanges: 3 + log2(LPR / 4) shuffles instead of 4 log2(LPR).
+template <int LPR>
+__device__ __forceinline__ float row_sums4(const float (&v)[4]) {
+  const int l = threadIdx.x;
+  const bool b0 = l & 1, b1 = l & 2;
+  const float u0 = (b0 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[1], 1);
+  const float u1 = (b0 ? v[3] : v[2]) + __shfl_xor_sync(0xffffffffu, b0 ? v[2] : v[3], 1);
+  float s = (b1 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, b1 ? u0 : u1, 2);
+#pragma unroll
+  for (int o = 4; o < LPR; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+// A value that lane l holds for step l & 3, for step s.
+__device__ __forceinline__ float of_step(float v, int s) { return __shfl_sync(0xffffffffu, v, (threadIdx.x & 28) | s); }
+
+// Thread map of the convolution stages: a CTA of 256 threads covers 64 x 4 channels of consecutive heads (LPR lanes per
+// row of a head; one contiguous piece of a time step) and four runs of `run` consecutive steps.  Steps go in batches
+// of four, the loads of the next batch in flight behind the arithmetic of the current one; the previous three inputs
+// (and, backward, the previous three ds) stay in registers.
+constexpr int kPreRuns = 4;
+struct PreMap {
+  int head, ch, t0;
+  bool act;
+  template <int LPR>
+  static __device__ __forceinline__ PreMap make(int H, int D, int run) {
+    const int seg = threadIdx.x & 63, l = seg & (LPR - 1);
+    PreMap m;
+    m.head = blockIdx.x * (64 / LPR) + seg / LPR;
+    m.act = m.head < H && 4 * l < D;
+    m.ch = m.head * D + 4 * l;
+    m.t0 = (blockIdx.y * kPreRuns + (threadIdx.x >> 6)) * run;
+    return m;
+  }
+};
+
+// ------------------------------------------------------------------ pre: forward
+// grid (head blocks, time tiles, streams x B)
+template <typename IO, int LPR>
+__global__ void __launch_bounds__(256) gdn_block_pre_fwd_kernel(BlockP p, PreArgs<IO> a, int run, int first) {
+  const int which = first + blockIdx.z / p.B, b = blockIdx.z % p.B;
   const int D = which == 2 ? p.Dv : p.Dk, C = p.H * D;
-  const int lane16 = threadIdx.x & 15, grp = threadIdx.x >> 4;
-  const bool act = lane16 * 8 < D;
-  const int ch = h * D + lane16 * 8;  // first of this thread's 8 channels
-  const int t0 = tile * kTile + grp * kRun;
-  const IO* x = a.x[which] + (size_t)b * p.T * C + ch;
-  IO* y = a.y[which] + (size_t)b * p.T * C + ch;
-  float w[4][8];  // zero for the lanes beyond D: their zero results take part in the row sums
+  const PreMap m = PreMap::make<LPR>(p.H, D, run);
+  const IO* x = a.x[which] + (size_t)b * p.T * C + m.ch;
+  IO* y = a.y[which] + (size_t)b * p.T * C + m.ch;
+  f2 w[4][2];  // zero for the lanes beyond D: their zero results take part in the row sums
 #pragma unroll
-  for (int tap = 0; tap < 4; ++tap)
-#pragma unroll
-    for (int c = 0; c < 8; ++c) w[tap][c] = 0.f;
-  if (act) {
-#pragma unroll
-    for (int tap = 0; tap < 4; ++tap) load8<float>(a.w[which] + tap * C + ch, w[tap]);
+  for (int tap = 0; tap < 4; ++tap) {
+    Raw4<float> r;
+    load_raw(r, a.w[which] + tap * C + m.ch, m.act);
+    widen(w[tap], r);
   }
-  const float scale = which == 0 ? 1.f / (float)D : rsqrtf((float)D);  // q: 1/dk, k: 1/sqrt(dk)
-  float x1[8], x2[8], x3[8];  // inputs of the previous three steps
+  const float inv_d = 1.f / (float)D, scale = which == 0 ? inv_d : rsqrtf((float)D);  // q: 1/dk, k: 1/sqrt(dk)
+  auto fetch = [&](Raw4<IO>& r, int t) { load_raw(r, x + (size_t)t * C, m.act && t >= 0 && t < p.T); };
+  f2 xx[7][2];  // inputs of the steps t-3 .. t+3
 #pragma unroll
-  for (int c = 0; c < 8; ++c) x1[c] = x2[c] = x3[c] = 0.f;
-  if (act) {
-    if (t0 - 1 >= 0 && t0 - 1 < p.T) load8<IO>(x + (size_t)(t0 - 1) * C, x1);
-    if (t0 - 2 >= 0 && t0 - 2 < p.T) load8<IO>(x + (size_t)(t0 - 2) * C, x2);
-    if (t0 - 3 >= 0 && t0 - 3 < p.T) load8<IO>(x + (size_t)(t0 - 3) * C, x3);
+  for (int k = 0; k < 3; ++k) {
+    Raw4<IO> r;
+    fetch(r, m.t0 - 3 + k);
+    widen(xx[k], r);
   }
+  Raw4<IO> nx[4];
 #pragma unroll
-  for (int r = 0; r < kRun; ++r) {
-    const int t = t0 + r;
-    const bool in = act && t < p.T;  // t < T is uniform over the 16 lanes of a group
-    float x0[8], s[8];
+  for (int s = 0; s < 4; ++s) fetch(nx[s], m.t0 + s);
+  for (int r0 = 0; r0 < run; r0 += 4) {
+    const int t = m.t0 + r0;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) x0[c] = 0.f;
-    if (in) load8<IO>(x + (size_t)t * C, x0);
-    float ss = 0.f;
+    for (int s = 0; s < 4; ++s) widen(xx[3 + s], nx[s]);
+    if (r0 + 4 < run) {
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const float acc = w[0][c] * x0[c] + w[1][c] * x1[c] + w[2][c] * x2[c] + w[3][c] * x3[c];
-      s[c] = acc * sigmoid_io<IO>(acc);  // rows past T are computed on zero-filled inputs and not stored
-      ss = fmaf(s[c], s[c], ss);
+      for (int s = 0; s < 4; ++s) fetch(nx[s], t + 4 + s);
+    }
+    f2 sv[4][2];
+    float ss[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      f2 sq = 0ull;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        f2 acc = mul2(w[0][c], xx[s + 3][c]);
+        fma2(acc, w[1][c], xx[s + 2][c]);
+        fma2(acc, w[2][c], xx[s + 1][c]);
+        fma2(acc, w[3][c], xx[s][c]);
+        sv[s][c] = mul2(acc, sigmoid_pair<IO>(acc));
+        fma2(sq, sv[s][c], sv[s][c]);
+      }
+      ss[s] = sum2(sq);
     }
     if (which < 2) {
-      ss = group_sum(ss);
-      const float rn = rsqrtf(ss / (float)D + 1e-6f) * scale;
+      const float rn = rsqrtf(fmaf(row_sums4<LPR>(ss), inv_d, 1e-6f)) * scale;
 #pragma unroll
-      for (int c = 0; c < 8; ++c) s[c] *= rn;
+      for (int s = 0; s < 4; ++s) {
+        const f2 f = dup2(of_step(rn, s));
+        sv[s][0] = mul2(sv[s][0], f);
+        sv[s][1] = mul2(sv[s][1], f);
+      }
     }
-    if (in) store8<IO>(y + (size_t)t * C, s);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) { x3[c] = x2[c]; x2[c] = x1[c]; x1[c] = x0[c]; }
+    for (int s = 0; s < 4; ++s)
+      if (m.act && t + s < p.T) store_pairs(y + (size_t)(t + s) * C, sv[s]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) xx[k][c] = xx[k + 4][c];
   }
 }
 
@@ -163,157 +243,171 @@ __global__ void __launch_bounds__(256) gdn_block_gate_fwd_kernel(BlockP p, const
 }
 
 // ------------------------------------------------------------------ pre: backward
-// Same split as the forward.  A lane group recomputes the convolution of its run and of the three steps after it
-// (their ds feeds dx of the run), keeps the last four ds in registers and emits dx three steps behind.
-// The backward keeps 4 channels per thread (a warp covers a row): its per-thread state - weights, weight-gradient
-// accumulators, three previous inputs and three previous ds per channel - would otherwise take ~180 registers and
-// leave two CTAs per SM.
-constexpr int kBwdGroups = 4;                   // warps per CTA, one run each
-constexpr int kBwdTile = kRun * kBwdGroups;
-template <typename IO>
-__device__ __forceinline__ void load4(const IO* p, float (&e)[4]);
-template <>
-__device__ __forceinline__ void load4<float>(const float* p, float (&e)[4]) {
-  const float4 a = __ldg(reinterpret_cast<const float4*>(p));
-  e[0] = a.x; e[1] = a.y; e[2] = a.z; e[3] = a.w;
-}
-template <>
-__device__ __forceinline__ void load4<bf16>(const bf16* p, float (&e)[4]) {
-  const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-  e[0] = __low2float(h[0]); e[1] = __high2float(h[0]); e[2] = __low2float(h[1]); e[3] = __high2float(h[1]);
-}
-template <typename IO>
-__device__ __forceinline__ void store4(IO* p, const float (&e)[4]);
-template <>
-__device__ __forceinline__ void store4<float>(float* p, const float (&e)[4]) {
-  *reinterpret_cast<float4*>(p) = make_float4(e[0], e[1], e[2], e[3]);
-}
-template <>
-__device__ __forceinline__ void store4<bf16>(bf16* p, const float (&e)[4]) {
-  uint2 v;
-  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
-  h[0] = __floats2bfloat162_rn(e[0], e[1]);
-  h[1] = __floats2bfloat162_rn(e[2], e[3]);
-  *reinterpret_cast<uint2*>(p) = v;
-}
-
-template <typename IO>
-__global__ void __launch_bounds__(128) gdn_block_pre_bwd_kernel(BlockP p, PreArgs<IO> a, int ntiles) {
-  __shared__ float red[kBwdGroups][4][128];
-  const int which = blockIdx.x / ntiles, tile = blockIdx.x % ntiles;
-  const int h = blockIdx.y, b = blockIdx.z;
+// Same map as the forward.  A run recomputes the convolution of its steps and of the three steps after it (their ds
+// feeds dx of the run) and emits dx three steps behind.  Bound: HBM (nine tensors) and, close behind, issue: about
+// 17 instructions per element with packed arithmetic (40 and half of the lanes idle at 64 channels before: 760 us for
+// 16 x 2048 x 16 heads of 64 bf16 channels).
+template <typename IO, int LPR>
+__global__ void __launch_bounds__(256, 2) gdn_block_pre_bwd_kernel(BlockP p, PreArgs<IO> a, int run, int first) {
+  __shared__ float red[kPreRuns][4][256];
+  const int which = first + blockIdx.z / p.B, b = blockIdx.z % p.B;
   const int D = which == 2 ? p.Dv : p.Dk, C = p.H * D;
-  const int lane32 = threadIdx.x & 31, grp = threadIdx.x >> 5;
-  const bool act = lane32 * 4 < D;
-  const int ch = h * D + lane32 * 4;
-  const int t0 = tile * kBwdTile + grp * kRun;
-  const IO* x = a.x[which] + (size_t)b * p.T * C + ch;
-  const IO* dy = a.dy[which] + (size_t)b * p.T * C + ch;
-  IO* dx = a.dx[which] + (size_t)b * p.T * C + ch;
-  float w[4][4], dw[4][4];
+  const PreMap m = PreMap::make<LPR>(p.H, D, run);
+  const IO* x = a.x[which] + (size_t)b * p.T * C + m.ch;
+  const IO* dy = a.dy[which] + (size_t)b * p.T * C + m.ch;
+  IO* dx = a.dx[which] + (size_t)b * p.T * C + m.ch;
+  f2 w[4][2], dw[4][2];
 #pragma unroll
-  for (int tap = 0; tap < 4; ++tap)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) { w[tap][c] = 0.f; dw[tap][c] = 0.f; }
-  if (act) {
-#pragma unroll
-    for (int tap = 0; tap < 4; ++tap) load4<float>(a.w[which] + tap * C + ch, w[tap]);
+  for (int tap = 0; tap < 4; ++tap) {
+    Raw4<float> r;
+    load_raw(r, a.w[which] + tap * C + m.ch, m.act);
+    widen(w[tap], r);
+    dw[tap][0] = dw[tap][1] = 0ull;
   }
-  const float scale = which == 0 ? 1.f / (float)D : rsqrtf((float)D);
-  float x1[4], x2[4], x3[4], d1[4], d2[4], d3[4];  // previous inputs; previous three ds
+  const float inv_d = 1.f / (float)D, scale = which == 0 ? inv_d : rsqrtf((float)D);
+  auto fetch = [&](Raw4<IO>& r, const IO* src, int t) { load_raw(r, src + (size_t)t * C, m.act && t >= 0 && t < p.T); };
+  f2 xx[7][2], dd[7][2];  // inputs and ds of the steps t-3 .. t+3
 #pragma unroll
-  for (int c = 0; c < 4; ++c) x1[c] = x2[c] = x3[c] = d1[c] = d2[c] = d3[c] = 0.f;
-  if (act) {
-    if (t0 - 1 >= 0 && t0 - 1 < p.T) load4<IO>(x + (size_t)(t0 - 1) * C, x1);
-    if (t0 - 2 >= 0 && t0 - 2 < p.T) load4<IO>(x + (size_t)(t0 - 2) * C, x2);
-    if (t0 - 3 >= 0 && t0 - 3 < p.T) load4<IO>(x + (size_t)(t0 - 3) * C, x3);
+  for (int k = 0; k < 3; ++k) {
+    Raw4<IO> r;
+    fetch(r, x, m.t0 - 3 + k);
+    widen(xx[k], r);
+    dd[k][0] = dd[k][1] = 0ull;
   }
+  Raw4<IO> nx[4], ng[4];
 #pragma unroll
-  for (int r = 0; r < kRun + 3; ++r) {
-    const int t = t0 + r;
-    const bool in = act && t < p.T;
-    float x0[4], g[4], ds[4];
+  for (int s = 0; s < 4; ++s) {
+    fetch(nx[s], x, m.t0 + s);
+    fetch(ng[s], dy, m.t0 + s);
+  }
+  for (int r0 = 0; r0 < run + 4; r0 += 4) {  // the last batch is the halo: three steps, no weight gradient
+    const int t = m.t0 + r0;
+    const bool halo = r0 == run;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) { x0[c] = 0.f; g[c] = 0.f; }
-    if (in) { load4<IO>(x + (size_t)t * C, x0); load4<IO>(dy + (size_t)t * C, g); }
+    for (int s = 0; s < 4; ++s) widen(xx[3 + s], nx[s]);
+    f2 g[4][2];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) widen(g[s], ng[s]);
+    if (!halo) {
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        if (s == 3 && r0 + 4 == run) break;  // the halo's fourth step is not needed (it reuses what is there)
+        fetch(nx[s], x, t + 4 + s);
+        fetch(ng[s], dy, t + 4 + s);
+      }
+    }
     // one sigmoid per element gives SiLU and its derivative; rows past T have zero dy, hence zero ds
-    float sv[4], dsl[4], ss = 0.f, dot = 0.f;
+    f2 sv[4][2], dsl[4][2];
+    float ss[4], dot[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const float acc = w[0][c] * x0[c] + w[1][c] * x1[c] + w[2][c] * x2[c] + w[3][c] * x3[c];
-      const float sg = sigmoid_io<IO>(acc);
-      sv[c] = acc * sg;
-      dsl[c] = fmaf(sv[c], 1.f - sg, sg);  // sg (1 + acc (1 - sg))
-      ss = fmaf(sv[c], sv[c], ss);
-      dot = fmaf(sv[c], g[c], dot);
-    }
-    if (which < 2) {  // y = s rn scale: ds_c = scale rn (g_c - s_c rn^2 dot / D)
-      ss = warp_sum(ss);
-      dot = warp_sum(dot);
-      const float rn = rsqrtf(ss / (float)D + 1e-6f);
-      const float k2 = rn * rn * dot / (float)D;
+    for (int s = 0; s < 4; ++s) {
+      f2 sq = 0ull, sg_dot = 0ull;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) g[c] = scale * rn * (g[c] - sv[c] * k2);
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) ds[c] = g[c] * dsl[c];
-    if (r < kRun) {  // this step belongs to the run: its share of the weight gradient
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        dw[0][c] = fmaf(x0[c], ds[c], dw[0][c]);
-        dw[1][c] = fmaf(x1[c], ds[c], dw[1][c]);
-        dw[2][c] = fmaf(x2[c], ds[c], dw[2][c]);
-        dw[3][c] = fmaf(x3[c], ds[c], dw[3][c]);
+      for (int c = 0; c < 2; ++c) {
+        f2 acc = mul2(w[0][c], xx[s + 3][c]);
+        fma2(acc, w[1][c], xx[s + 2][c]);
+        fma2(acc, w[2][c], xx[s + 1][c]);
+        fma2(acc, w[3][c], xx[s][c]);
+        const f2 sg = sigmoid_pair<IO>(acc);
+        sv[s][c] = mul2(acc, sg);
+        dsl[s][c] = mad2(sv[s][c], mad2(sg, dup2(-1.f), dup2(1.f)), sg);  // sg (1 + acc (1 - sg))
+        fma2(sq, sv[s][c], sv[s][c]);
+        fma2(sg_dot, sv[s][c], g[s][c]);
       }
+      ss[s] = sum2(sq);
+      dot[s] = sum2(sg_dot);
     }
-    if (r >= 3) {  // dx of step t-3 is complete: w0 ds[t-3] + w1 ds[t-2] + w2 ds[t-1] + w3 ds[t]
-      const int to = t - 3;
-      if (act && to < p.T) {
-        float o[4];
+    if (which < 2) {  // y = s rn scale: gradient at s = scale rn (g - s rn^2 dot / D)
+      const float rn = rsqrtf(fmaf(row_sums4<LPR>(ss), inv_d, 1e-6f));
+      const float fa = scale * rn, fb = -fa * rn * rn * (row_sums4<LPR>(dot) * inv_d);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) o[c] = w[0][c] * d3[c] + w[1][c] * d2[c] + w[2][c] * d1[c] + w[3][c] * ds[c];
-        store4<IO>(dx + (size_t)to * C, o);
+      for (int s = 0; s < 4; ++s) {
+        const f2 f0 = dup2(of_step(fa, s)), f1 = dup2(of_step(fb, s));
+#pragma unroll
+        for (int c = 0; c < 2; ++c) g[s][c] = mad2(f1, sv[s][c], mul2(f0, g[s][c]));
       }
     }
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      x3[c] = x2[c]; x2[c] = x1[c]; x1[c] = x0[c];
-      d3[c] = d2[c]; d2[c] = d1[c]; d1[c] = ds[c];
+    for (int s = 0; s < 4; ++s)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) dd[3 + s][c] = mul2(g[s][c], dsl[s][c]);
+    if (!halo) {
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+#pragma unroll
+        for (int tap = 0; tap < 4; ++tap)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) fma2(dw[tap][c], xx[s + 3 - tap][c], dd[3 + s][c]);
     }
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {  // dx of step t+s-3: w0 ds[t+s-3] + ... + w3 ds[t+s]
+      const int r = r0 + s - 3;
+      if (r >= 0 && r < run && m.act && t + s - 3 < p.T) {
+        f2 o[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          o[c] = mul2(w[0][c], dd[s][c]);
+          fma2(o[c], w[1][c], dd[s + 1][c]);
+          fma2(o[c], w[2][c], dd[s + 2][c]);
+          fma2(o[c], w[3][c], dd[s + 3][c]);
+        }
+        store_pairs(dx + (size_t)(t + s - 3) * C, o);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        xx[k][c] = xx[k + 4][c];
+        dd[k][c] = dd[k + 4][c];
+      }
   }
-  // weight-gradient partial of this CTA: sum over its lane groups in a fixed order
+  // weight-gradient partial of this CTA: its four runs added in a fixed order
+  const int seg = threadIdx.x & 63, rid = threadIdx.x >> 6;
 #pragma unroll
-  for (int tap = 0; tap < 4; ++tap)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) red[grp][tap][lane32 * 4 + c] = dw[tap][c];
+  for (int tap = 0; tap < 4; ++tap) {
+    const float2 lo = unpack2(dw[tap][0]), hi = unpack2(dw[tap][1]);
+    *reinterpret_cast<float4*>(&red[rid][tap][4 * seg]) = make_float4(lo.x, lo.y, hi.x, hi.y);
+  }
   __syncthreads();
-  float* dst = a.dwp[which] + ((size_t)(b * ntiles + tile) * 4) * C + h * D;
-  for (int i = threadIdx.x; i < 4 * D; i += 128) {
-    const int tap = i / D, c = i % D;
-    float s = 0.f;
+  if (m.act) {  // thread = tap rid, its own four channels
+    float4 s = *reinterpret_cast<const float4*>(&red[0][rid][4 * seg]);
 #pragma unroll
-    for (int g2 = 0; g2 < kBwdGroups; ++g2) s += red[g2][tap][c];
-    dst[(size_t)tap * C + c] = s;
+    for (int k = 1; k < kPreRuns; ++k) {
+      const float4 v = *reinterpret_cast<const float4*>(&red[k][rid][4 * seg]);
+      s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
+    }
+    *reinterpret_cast<float4*>(a.dwp[which] + (((size_t)b * gridDim.y + blockIdx.y) * 4 + rid) * C + m.ch) = s;
   }
 }
 
 // out[j] = sum over rows of part[row][j] in a fixed order: a CTA owns 32 columns, its 8 warps take every 8th row
-// (coalesced 128-byte reads, 8 loads in flight per column), then the 8 slices are added in order.  grid ceil(n / 32)
-__global__ void __launch_bounds__(256) gdn_block_colsum_kernel(const float* __restrict__ part, int rows, int n,
-                                                               float* __restrict__ out) {
+// (coalesced 128-byte reads, 8 loads in flight per column), then the 8 slices are added in order.  Up to five matrices
+// per launch, segment s starting at block first[s].
+struct ColSums {
+  const float* part[5];
+  float* out[5];
+  int rows[5], n[5], first[6], count;
+};
+__global__ void __launch_bounds__(256) gdn_block_colsum_kernel(ColSums c) {
   __shared__ float red[8][32];
-  const int j = blockIdx.x * 32 + (threadIdx.x & 31), slice = threadIdx.x >> 5;
+  int g = 0;
+  while (g + 1 < c.count && (int)blockIdx.x >= c.first[g + 1]) ++g;
+  const int n = c.n[g], rows = c.rows[g];
+  const int j = (blockIdx.x - c.first[g]) * 32 + (threadIdx.x & 31), slice = threadIdx.x >> 5;
+  const float* part = c.part[g];
   float s = 0.f;
-  if (j < n)
+  if (j < n) {
+#pragma unroll 8
     for (int r = slice; r < rows; r += 8) s += part[(size_t)r * n + j];
+  }
   red[slice][threadIdx.x & 31] = s;
   __syncthreads();
   if (threadIdx.x < 32 && j < n) {
     float t = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) t += red[k][threadIdx.x];
-    out[j] = t;
+    c.out[g][j] = t;
   }
 }
 
@@ -357,7 +451,7 @@ __global__ void __launch_bounds__(256) gdn_block_gate_bwd_kernel(BlockP p, const
 
 // The same with every (b, t, h) element on its own thread, coalesced, for head counts that divide 256: a thread's
 // head is then tid % H for every element it touches.  Per-CTA partial sums [2][G][H] -> fixed-order second pass.
-constexpr int kGatePerCta = 256 * 16;
+constexpr int kGatePerCta = 256 * 8;
 __global__ void __launch_bounds__(256) gdn_block_gate_bwd_flat_kernel(BlockP p, const float* __restrict__ a_raw,
                                                                       const float* __restrict__ b_raw,
                                                                       const float* __restrict__ a_log,
@@ -396,51 +490,70 @@ __global__ void __launch_bounds__(256) gdn_block_gate_bwd_flat_kernel(BlockP p, 
 }
 
 // ------------------------------------------------------------------ post
-// y = o rsqrt(mean(o^2) + 1e-5) o_norm SiLU(z); rows = (b, t, h), D = Dv; 8 rows per CTA pass
-template <typename IO>
+// y = o rsqrt(mean(o^2) + 1e-5) o_norm SiLU(z); rows = (b, t, h), D = Dv.  A thread owns 8 channels, LPR lanes a row
+// (with 16 lanes for every width, half of them idled at 64 channels: 60 us instead of 36 for 16 x 2048 x 16 rows);
+// two rows per pass, so that the loads of both are in flight.
+template <int LPR>
+__device__ __forceinline__ float lane_sum(float v) {
+#pragma unroll
+  for (int o = LPR / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+template <typename IO, int LPR>
 __global__ void __launch_bounds__(128) gdn_block_post_fwd_kernel(BlockP p, const IO* __restrict__ o,
                                                                  const IO* __restrict__ z,
                                                                  const float* __restrict__ wn, IO* __restrict__ y) {
-  const int D = p.Dv, lane16 = threadIdx.x & 15, grp = threadIdx.x >> 4;
-  const bool act = lane16 * 8 < D;
-  const size_t rows = (size_t)p.B * p.T * p.H;
+  constexpr int kRows = 128 / LPR;  // rows of a CTA
+  const int D = p.Dv, l = threadIdx.x % LPR;
+  const bool act = l * 8 < D;
+  const size_t rows = (size_t)p.B * p.T * p.H, step = (size_t)gridDim.x * kRows;
   float w[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (act) load8<float>(wn + lane16 * 8, w);
-  for (size_t row = (size_t)blockIdx.x * kGroups + grp; row < rows; row += (size_t)gridDim.x * kGroups) {
-    const size_t off = row * D + lane16 * 8;
-    float ov[8], zv[8];
+  if (act) load8<float>(wn + l * 8, w);
+  for (size_t first = (size_t)blockIdx.x * kRows; first < rows; first += 2 * step) {
+    float ov[2][8], zv[2][8];
+    bool in[2];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) ov[c] = zv[c] = 0.f;
-    if (act) { load8<IO>(o + off, ov); load8<IO>(z + off, zv); }
-    float ss = 0.f;
+    for (int u = 0; u < 2; ++u) {
+      const size_t row = first + u * step + threadIdx.x / LPR;
+      in[u] = act && row < rows;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) ss = fmaf(ov[c], ov[c], ss);
-    ss = group_sum(ss);
-    const float rn = rsqrtf(ss / (float)D + 1e-5f);
+      for (int c = 0; c < 8; ++c) ov[u][c] = zv[u][c] = 0.f;
+      if (in[u]) { load8<IO>(o + row * D + l * 8, ov[u]); load8<IO>(z + row * D + l * 8, zv[u]); }
+    }
 #pragma unroll
-    for (int c = 0; c < 8; ++c) ov[c] = ov[c] * rn * w[c] * zv[c] * sigmoid_io<IO>(zv[c]);
-    if (act) store8<IO>(y + off, ov);
+    for (int u = 0; u < 2; ++u) {
+      const size_t row = first + u * step + threadIdx.x / LPR;
+      float ss = 0.f;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) ss = fmaf(ov[u][c], ov[u][c], ss);
+      const float rn = rsqrtf(lane_sum<LPR>(ss) / (float)D + 1e-5f);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) ov[u][c] = ov[u][c] * rn * w[c] * zv[u][c] * sigmoid_io<IO>(zv[u][c]);
+      if (in[u]) store8<IO>(y + row * D + l * 8, ov[u]);
+    }
   }
 }
 
-template <typename IO>
+template <typename IO, int LPR>
 __global__ void __launch_bounds__(128) gdn_block_post_bwd_kernel(BlockP p, const IO* __restrict__ o,
                                                                  const IO* __restrict__ z,
                                                                  const float* __restrict__ wn,
                                                                  const IO* __restrict__ dy, IO* __restrict__ d_o,
                                                                  IO* __restrict__ dz, float* __restrict__ dwp) {
-  __shared__ float red[kGroups][128];
-  const int D = p.Dv, lane16 = threadIdx.x & 15, grp = threadIdx.x >> 4;
-  const bool act = lane16 * 8 < D;
-  const size_t rows = (size_t)p.B * p.T * p.H;
+  constexpr int kRows = 128 / LPR;
+  __shared__ float red[kRows][8 * LPR];
+  const int D = p.Dv, l = threadIdx.x % LPR;
+  const bool act = l * 8 < D;
+  const size_t rows = (size_t)p.B * p.T * p.H, step = (size_t)gridDim.x * kRows;
   float w[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, dw[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (act) load8<float>(wn + lane16 * 8, w);
-  for (size_t row = (size_t)blockIdx.x * kGroups + grp; row < rows; row += (size_t)gridDim.x * kGroups) {
-    const size_t off = row * D + lane16 * 8;
+  if (act) load8<float>(wn + l * 8, w);
+  for (size_t first = (size_t)blockIdx.x * kRows; first < rows; first += step) {
+    const size_t row = first + threadIdx.x / LPR, off = row * D + l * 8;
+    const bool in = act && row < rows;
     float ov[8], zv[8], gv[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) ov[c] = zv[c] = gv[c] = 0.f;
-    if (act) { load8<IO>(o + off, ov); load8<IO>(z + off, zv); load8<IO>(dy + off, gv); }
+    if (in) { load8<IO>(o + off, ov); load8<IO>(z + off, zv); load8<IO>(dy + off, gv); }
     float ss = 0.f, dot = 0.f, g[8], sz[8], dsz[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
@@ -451,10 +564,8 @@ __global__ void __launch_bounds__(128) gdn_block_post_bwd_kernel(BlockP p, const
       ss = fmaf(ov[c], ov[c], ss);
       dot = fmaf(ov[c], g[c], dot);
     }
-    ss = group_sum(ss);
-    dot = group_sum(dot);
-    const float rn = rsqrtf(ss / (float)D + 1e-5f);
-    const float k2 = rn * rn * dot / (float)D;
+    const float rn = rsqrtf(lane_sum<LPR>(ss) / (float)D + 1e-5f);
+    const float k2 = rn * rn * lane_sum<LPR>(dot) / (float)D;
     float dzv[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
@@ -463,15 +574,15 @@ __global__ void __launch_bounds__(128) gdn_block_post_bwd_kernel(BlockP p, const
       dzv[c] = gv[c] * w[c] * on * dsz[c];
       g[c] = rn * (g[c] - ov[c] * k2);
     }
-    if (act) { store8<IO>(d_o + off, g); store8<IO>(dz + off, dzv); }
+    if (in) { store8<IO>(d_o + off, g); store8<IO>(dz + off, dzv); }
   }
 #pragma unroll
-  for (int c = 0; c < 8; ++c) red[grp][lane16 * 8 + c] = dw[c];
+  for (int c = 0; c < 8; ++c) red[threadIdx.x / LPR][l * 8 + c] = dw[c];
   __syncthreads();
   for (int c = threadIdx.x; c < D; c += 128) {
     float s = 0.f;
 #pragma unroll
-    for (int g2 = 0; g2 < kGroups; ++g2) s += red[g2][c];
+    for (int g2 = 0; g2 < kRows; ++g2) s += red[g2][c];
     dwp[(size_t)blockIdx.x * D + c] = s;
   }
 }
@@ -489,12 +600,28 @@ static BlockP make_blk(const mxb_gdn_desc* d) {
 bool gdn_block_supported(const mxb_gdn_desc* d) {
   return d->Dk % 8 == 0 && d->Dv % 8 == 0 && d->Dk <= 128 && d->Dv <= 128 && d->Dk > 0 && d->Dv > 0;
 }
-static int blk_tiles(const mxb_gdn_desc* d) { return (d->T + blk::kTile - 1) / blk::kTile; }
-static int blk_bwd_tiles(const mxb_gdn_desc* d) { return (d->T + blk::kBwdTile - 1) / blk::kBwdTile; }
+// Lanes per row: the power of two that covers D / per channels.
+static int blk_lanes(int D, int per) {
+  int l = per == 4 ? 4 : 1;
+  while (l * per < D) l *= 2;
+  return l;
+}
+// Steps per run: 32 (a halo of three steps is recomputed per run in the backward) while that still gives two CTAs per
+// SM, shorter runs for smaller problems, where the length of the chain is what counts.
+static int blk_run(const mxb_gdn_desc* d) {
+  const int hk = 64 / blk_lanes(d->Dk, 4);
+  for (int run = 32; run > 4; run /= 2)
+    if ((size_t)3 * d->B * ((d->H + hk - 1) / hk) * ((d->T + 4 * run - 1) / (4 * run)) >= 2 * 148) return run;
+  return 4;
+}
+static int blk_tiles(const mxb_gdn_desc* d) {
+  const int tile = blk::kPreRuns * blk_run(d);
+  return (d->T + tile - 1) / tile;
+}
 static int blk_post_ctas(const mxb_gdn_desc* d) {
-  const size_t rows = (size_t)d->B * d->T * d->H;
-  const size_t want = (rows + blk::kGroups - 1) / blk::kGroups;
-  return (int)(want < 148 * 16 ? want : 148 * 16);
+  const size_t rows = (size_t)d->B * d->T * d->H, per = 128 / blk_lanes(d->Dv, 8);
+  const size_t want = (rows + per - 1) / per;
+  return (int)(want < 148 * 8 ? want : 148 * 8);
 }
 static int blk_gate_ctas(const mxb_gdn_desc* d) {
   const size_t n = (size_t)d->B * d->T * d->H;
@@ -502,11 +629,32 @@ static int blk_gate_ctas(const mxb_gdn_desc* d) {
 }
 // backward partial rows: conv weights of q, k, v and the per-head gate sums; or the norm weight
 size_t gdn_block_workspace_bytes(const mxb_gdn_desc* d) {
-  const size_t rows = (size_t)d->B * blk_bwd_tiles(d);
+  const size_t rows = (size_t)d->B * blk_tiles(d);
   const size_t pre = rows * 4 * ((size_t)2 * d->H * d->Dk + (size_t)d->H * d->Dv) * sizeof(float);
   const size_t post = (size_t)blk_post_ctas(d) * d->Dv * sizeof(float);
   const size_t gate = 2 * (size_t)blk_gate_ctas(d) * d->H * sizeof(float);
   return (pre + gate > post ? pre + gate : post) + 256;
+}
+
+// call(LPR) with the lane count as a compile-time constant
+template <typename F>
+static void with_lanes(int lanes, F&& call) {
+  switch (lanes) {
+    case 1: call(std::integral_constant<int, 1>{}); break;
+    case 2: call(std::integral_constant<int, 2>{}); break;
+    case 4: call(std::integral_constant<int, 4>{}); break;
+    case 8: call(std::integral_constant<int, 8>{}); break;
+    case 16: call(std::integral_constant<int, 16>{}); break;
+    default: call(std::integral_constant<int, 32>{}); break;
+  }
+}
+// The convolution kernels over q, k (streams 0, 1) and v (2): one launch where the lane counts agree, two otherwise.
+template <typename F>
+static void blk_streams(const mxb_gdn_desc* d, F&& launch) {
+  const int lk = blk_lanes(d->Dk, 4), lv = blk_lanes(d->Dv, 4), nt = blk_tiles(d);
+  auto grid = [&](int lanes, int streams) { return dim3((d->H + 64 / lanes - 1) / (64 / lanes), nt, streams * d->B); };
+  launch(lk, grid(lk, lk == lv ? 3 : 2), 0);
+  if (lk != lv) launch(lv, grid(lv, 1), 2);
 }
 
 template <typename IO>
@@ -519,9 +667,14 @@ static mxb_status blk_pre_fwd(const mxb_gdn_desc* d, const void* qp, const void*
   a.x[0] = static_cast<const IO*>(qp); a.x[1] = static_cast<const IO*>(kp); a.x[2] = static_cast<const IO*>(vp);
   a.w[0] = cq; a.w[1] = ck; a.w[2] = cv;
   a.y[0] = static_cast<IO*>(q); a.y[1] = static_cast<IO*>(k); a.y[2] = static_cast<IO*>(v);
-  const int nt = blk_tiles(d);
-  MXB_LAUNCH("gdn_block_pre_fwd_kernel", st,
-             (blk::gdn_block_pre_fwd_kernel<IO><<<dim3(3 * nt, d->H, d->B), 128, 0, st>>>(p, a, nt)));
+  const int run = blk_run(d);
+  blk_streams(d, [&](int lanes, dim3 grid, int first) {
+    with_lanes(lanes, [&](auto lpr) {
+      constexpr int LPR = decltype(lpr)::value;
+      if constexpr (LPR >= 4)
+        MXB_LAUNCH("gdn_block_pre_fwd_kernel", st, (blk::gdn_block_pre_fwd_kernel<IO, LPR><<<grid, 256, 0, st>>>(p, a, run, first)));
+    });
+  });
   const size_t n = (size_t)d->B * d->T * d->H;
   const int gb = (int)((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8);
   MXB_LAUNCH("gdn_block_gate_fwd_kernel", st,
@@ -550,34 +703,40 @@ static mxb_status blk_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void*
   a.w[0] = cq; a.w[1] = ck; a.w[2] = cv;
   a.dy[0] = static_cast<const IO*>(dq); a.dy[1] = static_cast<const IO*>(dk); a.dy[2] = static_cast<const IO*>(dv);
   a.dx[0] = static_cast<IO*>(dqp); a.dx[1] = static_cast<IO*>(dkp); a.dx[2] = static_cast<IO*>(dvp);
-  const int nt = blk_bwd_tiles(d);
-  const size_t rows = (size_t)d->B * nt, Ck = (size_t)d->H * d->Dk, Cv = (size_t)d->H * d->Dv;
+  const int run = blk_run(d);
+  const size_t rows = (size_t)d->B * blk_tiles(d), Ck = (size_t)d->H * d->Dk, Cv = (size_t)d->H * d->Dv;
   float* base = reinterpret_cast<float*>(static_cast<char*>(ws) + 256);
   a.dwp[0] = base; a.dwp[1] = base + rows * 4 * Ck; a.dwp[2] = base + rows * 8 * Ck;
-  MXB_LAUNCH("gdn_block_pre_bwd_kernel", st,
-             (blk::gdn_block_pre_bwd_kernel<IO><<<dim3(3 * nt, d->H, d->B), 128, 0, st>>>(p, a, nt)));
-  float* outs[3] = {dcq, dck, dcv};
-  for (int w = 0; w < 3; ++w) {
-    const int n = (int)(4 * (w == 2 ? Cv : Ck));
-    MXB_LAUNCH("gdn_block_colsum_kernel", st,
-               (blk::gdn_block_colsum_kernel<<<(n + 31) / 32, 256, 0, st>>>(a.dwp[w], (int)rows, n, outs[w])));
-  }
+  blk_streams(d, [&](int lanes, dim3 grid, int first) {
+    with_lanes(lanes, [&](auto lpr) {
+      constexpr int LPR = decltype(lpr)::value;
+      if constexpr (LPR >= 4)
+        MXB_LAUNCH("gdn_block_pre_bwd_kernel", st, (blk::gdn_block_pre_bwd_kernel<IO, LPR><<<grid, 256, 0, st>>>(p, a, run, first)));
+    });
+  });
+  blk::ColSums c{};
+  auto sum = [&](const float* part, int nrows, int n, float* out) {
+    c.part[c.count] = part; c.out[c.count] = out; c.rows[c.count] = nrows; c.n[c.count] = n;
+    c.first[c.count + 1] = c.first[c.count] + (n + 31) / 32;
+    ++c.count;
+  };
+  sum(a.dwp[0], (int)rows, (int)(4 * Ck), dcq);
+  sum(a.dwp[1], (int)rows, (int)(4 * Ck), dck);
+  sum(a.dwp[2], (int)rows, (int)(4 * Cv), dcv);
   if (256 % d->H == 0) {
     const int gc = blk_gate_ctas(d);
     float* gpart = base + rows * 4 * (2 * Ck + Cv);
     MXB_LAUNCH("gdn_block_gate_bwd_flat_kernel", st,
                (blk::gdn_block_gate_bwd_flat_kernel<<<gc, 256, 0, st>>>(p, a_raw, b_raw, a_log, dt_bias, dbeta, dgate,
                                                                        da_raw, db_raw, gpart)));
-    MXB_LAUNCH("gdn_block_colsum_kernel", st,
-               (blk::gdn_block_colsum_kernel<<<(d->H + 31) / 32, 256, 0, st>>>(gpart, gc, d->H, da_log)));
-    MXB_LAUNCH("gdn_block_colsum_kernel", st,
-               (blk::gdn_block_colsum_kernel<<<(d->H + 31) / 32, 256, 0, st>>>(gpart + (size_t)gc * d->H, gc, d->H,
-                                                                                 ddt_bias)));
+    sum(gpart, gc, d->H, da_log);
+    sum(gpart + (size_t)gc * d->H, gc, d->H, ddt_bias);
   } else {
     MXB_LAUNCH("gdn_block_gate_bwd_kernel", st,
                (blk::gdn_block_gate_bwd_kernel<<<d->H, 256, 0, st>>>(p, a_raw, b_raw, a_log, dt_bias, dbeta, dgate,
                                                                       da_raw, db_raw, da_log, ddt_bias)));
   }
+  MXB_LAUNCH("gdn_block_colsum_kernel", st, (blk::gdn_block_colsum_kernel<<<c.first[c.count], 256, 0, st>>>(c)));
   return check_launch("gdn_block_pre_bwd");
 }
 mxb_status gdn_block_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void* kp, const void* vp, const float* cq,
@@ -598,21 +757,29 @@ static mxb_status blk_post(const mxb_gdn_desc* d, const void* o, const void* z, 
                            const void* dy, void* d_o, void* dz, float* dwn, void* ws, cudaStream_t st) {
   BlockP p = make_blk(d);
   const int ctas = blk_post_ctas(d);
+  const int lanes = blk_lanes(d->Dv, 8);
   if (!dy) {
-    MXB_LAUNCH("gdn_block_post_fwd_kernel", st,
-               (blk::gdn_block_post_fwd_kernel<IO><<<ctas, 128, 0, st>>>(p, static_cast<const IO*>(o),
-                                                                         static_cast<const IO*>(z), wn,
-                                                                         static_cast<IO*>(y))));
+    with_lanes(lanes, [&](auto lpr) {
+      constexpr int LPR = decltype(lpr)::value;
+      if constexpr (LPR <= 16)
+        MXB_LAUNCH("gdn_block_post_fwd_kernel", st,
+                   (blk::gdn_block_post_fwd_kernel<IO, LPR><<<ctas, 128, 0, st>>>(
+                       p, static_cast<const IO*>(o), static_cast<const IO*>(z), wn, static_cast<IO*>(y))));
+    });
     return check_launch("gdn_block_post_fwd");
   }
   float* part = reinterpret_cast<float*>(static_cast<char*>(ws) + 256);
-  MXB_LAUNCH("gdn_block_post_bwd_kernel", st,
-             (blk::gdn_block_post_bwd_kernel<IO><<<ctas, 128, 0, st>>>(p, static_cast<const IO*>(o),
-                                                                       static_cast<const IO*>(z), wn,
-                                                                       static_cast<const IO*>(dy), static_cast<IO*>(d_o),
-                                                                       static_cast<IO*>(dz), part)));
-  MXB_LAUNCH("gdn_block_colsum_kernel", st,
-             (blk::gdn_block_colsum_kernel<<<(d->Dv + 31) / 32, 256, 0, st>>>(part, ctas, d->Dv, dwn)));
+  with_lanes(lanes, [&](auto lpr) {
+    constexpr int LPR = decltype(lpr)::value;
+    if constexpr (LPR <= 16)
+      MXB_LAUNCH("gdn_block_post_bwd_kernel", st,
+                 (blk::gdn_block_post_bwd_kernel<IO, LPR><<<ctas, 128, 0, st>>>(
+                     p, static_cast<const IO*>(o), static_cast<const IO*>(z), wn, static_cast<const IO*>(dy),
+                     static_cast<IO*>(d_o), static_cast<IO*>(dz), part)));
+  });
+  blk::ColSums c{};
+  c.part[0] = part; c.out[0] = dwn; c.rows[0] = ctas; c.n[0] = d->Dv; c.count = 1; c.first[1] = (d->Dv + 31) / 32;
+  MXB_LAUNCH("gdn_block_colsum_kernel", st, (blk::gdn_block_colsum_kernel<<<c.first[1], 256, 0, st>>>(c)));
   return check_launch("gdn_block_post_bwd");
 }
 mxb_status gdn_block_post(const mxb_gdn_desc* d, const void* o, const void* z, const float* wn, void* y, const void* dy,

@@ -32,6 +32,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "packed.cuh"
 #include "tcgen05.cuh"
 
 namespace mxb {
@@ -79,27 +80,6 @@ constexpr int LD = 68;   // pitch of [64][64] matrices: rows 16 bytes apart modu
 constexpr int KB = 32;   // contraction elements staged per step
 constexpr int LB = KB + 4;
 
-using f2 = unsigned long long;  // two packed floats
-__device__ __forceinline__ f2 pack2(float a, float b) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(f2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ void fma2(f2& d, f2 a, f2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ float sum2(f2 v) {
-  const float2 t = unpack2(v);
-  return t.x + t.y;
-}
 __device__ __forceinline__ ulonglong2 lds2x2(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
 
 // Four consecutive elements col .. col+3 of a row of n (zeros past the end).
@@ -427,7 +407,7 @@ struct PrepF32 {
 
 // acc[r][2 g + s] += sum_{m < 4 ty + 4} A[4 ty + r][m] B[m][64 g + 4 tx + 2 s, +1], A lower triangular, B swizzled
 template <int NG>
-__device__ __forceinline__ void prep_product(simt::f2 (&acc)[4][2 * NG], const float* A, const float* B) {
+__device__ __forceinline__ void prep_product(f2 (&acc)[4][2 * NG], const float* A, const float* B) {
   using namespace simt;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 #pragma unroll 2
