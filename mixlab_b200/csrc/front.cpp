@@ -353,6 +353,10 @@ mxb_mamba3_desc check_mamba3(const On& on, const Tensor& x, const Tensor& dt, co
   check(c, gn, io, on.dev, "c");
   return d;
 }
+Token mamba3_token(const On& on, const mxb_mamba3_desc& d, const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta,
+                   const Tensor& a_log, const Tensor& b, const Tensor& c) {
+  return token(2, on.stream, {&x, &dt, &lam, &theta, &a_log, &b, &c}, {d.nheads, d.flags & ~(MXB_MAMBA3_SAVE_FOR_BWD | MXB_MAMBA3_BWD_USE_SAVED)});
+}
 Tensor mamba3_forward(const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta, const Tensor& a_log, const Tensor& b,
                       const Tensor& c, int64_t nheads, int64_t flags, bool save) {
   On on(x);
@@ -361,7 +365,7 @@ Tensor mamba3_forward(const Tensor& x, const Tensor& dt, const Tensor& lam, cons
   Tensor ws = workspace(abi.mxb_mamba3_fwd_workspace_bytes(&d), on.dev.index());
   call("mxb_mamba3_fwd", abi.mxb_mamba3_fwd, &d, ptr(x), ptr<float>(dt), ptr<float>(lam), ptr<float>(theta), ptr<float>(a_log), ptr(b), ptr(c),
        ptr(y), ptr(ws), (size_t)ws.numel(), on.stream);
-  if (save) workspaces()[on.dev.index()].saved = token(2, on.stream, {&x, &dt, &lam, &theta, &a_log, &b, &c}, {nheads});
+  if (save) workspaces()[on.dev.index()].saved = mamba3_token(on, d, x, dt, lam, theta, a_log, b, c);
   return y;
 }
 py::dict mamba3_backward(const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta, const Tensor& a_log, const Tensor& b,
@@ -370,8 +374,7 @@ py::dict mamba3_backward(const Tensor& x, const Tensor& dt, const Tensor& lam, c
   const mxb_mamba3_desc d = check_mamba3(on, x, dt, lam, theta, a_log, b, c, nheads, use_saved ? flags | MXB_MAMBA3_BWD_USE_SAVED : flags);
   check(dy, x.sizes(), x.scalar_type(), on.dev, "dy");
   const size_t nws = abi.mxb_mamba3_bwd_workspace_bytes(&d);
-  Tensor ws = use_saved ? saved_workspace(token(2, on.stream, {&x, &dt, &lam, &theta, &a_log, &b, &c}, {nheads}), nws, on.dev.index(),
-                                          "mamba3_selective_scan_backward")
+  Tensor ws = use_saved ? saved_workspace(mamba3_token(on, d, x, dt, lam, theta, a_log, b, c), nws, on.dev.index(), "mamba3_selective_scan_backward")
                         : workspace(nws, on.dev.index());
   Tensor dx = like(x), ddt = like(dt), dlam = like(lam), dth = like(theta), dal = like(a_log), db = like(b), dc = like(c);
   call("mxb_mamba3_bwd", abi.mxb_mamba3_bwd, &d, ptr(x), ptr<float>(dt), ptr<float>(lam), ptr<float>(theta), ptr<float>(a_log), ptr(b), ptr(c),

@@ -1,0 +1,868 @@
+// Mamba-3 selective scan, per-channel layout, window-parallel: forward and backward for problems whose (batch, channel)
+// pairs cannot fill the GPU with walks over the whole sequence (mamba3.cu has the recurrence and the serial walk).
+//
+// A walker owns one (batch, channel, window of 8 steps).  Every carried quantity is linear in what crosses a window
+// boundary, so the walk splits into local walks and scans over the windows:
+//   prepare   softplus(dt), sigmoid(lambda) of every (step, channel), window sums of dt theta and dt
+//   scan      angle at each window start
+//   local     walks from a zero state (forward) and from a zero dh (reverse; backward only)
+//   scan      H <- exp(A sum dt) H + local: state at each window start; the same for dh, in reverse
+//   walk      forward: the true walk writes y;  backward: replay into shared memory, then the true reverse walk with
+//             window-local angle-gradient sums
+//   scan, fix reverse scan of those sums; the later windows' sums are added to ddt and dtheta
+//
+// What bounds it: instruction issue (a sine, a cosine and two exponentials per state pair and pass).  So everything
+// that belongs to a (step, channel) is computed once and not by every lane and pass; the two states of a pair and two
+// pairs per lane go through packed arithmetic; a pass keeps sine, cosine and decay in shared memory for its reverse
+// half; rows of dB, dC are added over the channels of a warp by halving exchanges and over the warps once per window.
+// Scans run 16 segments of windows side by side.  2 x 1024 x 128 channels of 16 states, forward + backward:
+// 310 -> 93 us of kernels; 4096 x 448 channels: 1.79 -> 0.59 ms.
+//
+// Every sum has a fixed order: the same inputs give the same bits.
+#include <algorithm>
+
+#include "mamba3.cuh"
+#include "packed.cuh"
+
+namespace mxb {
+namespace m3w {
+
+constexpr int W = kM3WinSteps;
+
+// sin, cos of two angles in [-pi, pi] (a little more is fine): reduction by the nearest multiple of pi/2 in two parts
+// (Cody and Waite), Taylor polynomials of degree 9 and 10 on [-pi/4, pi/4].  Truncation is below 2e-9; the largest
+// error over 4 million angles against double precision is 6.9e-8 (1.4 ulp of the result).
+__device__ __forceinline__ void sincos2(f2 x, f2& sn, f2& cs) {
+  const f2 magic = dup2(12582912.f), minus = dup2(-12582912.f);  // 1.5 * 2^23: rounds to the nearest integer
+  const f2 kf = mad2(x, dup2(0.63661977236758134f), magic);
+  const f2 k = add2(kf, minus);
+  f2 r = mad2(k, dup2(-1.5707963705062866f), x);   // pi/2 rounded to float, and what is left of it
+  r = mad2(k, dup2(4.3711390001862426e-8f), r);
+  const f2 r2 = mul2(r, r);
+  f2 ps = dup2(2.7557319223985893e-6f);
+  ps = mad2(ps, r2, dup2(-1.9841269841269841e-4f));
+  ps = mad2(ps, r2, dup2(8.3333333333333333e-3f));
+  ps = mad2(ps, r2, dup2(-1.6666666666666667e-1f));
+  ps = mad2(mul2(ps, r2), r, r);
+  f2 pc = dup2(-2.7557319223985888e-7f);
+  pc = mad2(pc, r2, dup2(2.4801587301587302e-5f));
+  pc = mad2(pc, r2, dup2(-1.3888888888888889e-3f));
+  pc = mad2(pc, r2, dup2(4.1666666666666667e-2f));
+  pc = mad2(pc, r2, dup2(-0.5f));
+  pc = mad2(pc, r2, dup2(1.f));
+  const float2 s = unpack2(ps), c = unpack2(pc), q = unpack2(kf);
+  auto quadrant = [](float s, float c, float q, float& so, float& co) {
+    const int k = __float_as_int(q);  // the low bits of the rounded sum are the multiple of pi/2
+    const float a = (k & 1) ? c : s, b = (k & 1) ? s : c;
+    so = __int_as_float(__float_as_int(a) ^ ((k & 2) << 30));
+    co = __int_as_float(__float_as_int(b) ^ (((k + 1) & 2) << 30));
+  };
+  float s0, c0, s1, c1;
+  quadrant(s.x, c.x, q.x, s0, c0);
+  quadrant(s.y, c.y, q.y, s1, c1);
+  sn = pack2(s0, s1);
+  cs = pack2(c0, c1);
+}
+// Two angles wrapped to [-pi, pi] (m3_wrap, packed).
+__device__ __forceinline__ f2 wrap2(f2 x) {
+  const f2 k = add2(mad2(x, dup2(0.15915494309189535f), dup2(12582912.f)), dup2(-12582912.f));
+  return mad2(k, dup2(-1.9353071795864769e-3f), mad2(k, dup2(-6.28125f), x));
+}
+__device__ __forceinline__ f2 neg2(f2 v) { return v ^ 0x8000000080000000ull; }
+__device__ __forceinline__ f2 exp2p(f2 a, float dt) {  // exp(dt a), both halves
+  const float2 t = unpack2(a);
+  return pack2(expf(dt * t.x), expf(dt * t.y));
+}
+
+// One walker: the lanes of one channel in one window.  A lane owns PR state pairs kp = sl PR + r in units of two; a
+// packed value holds the same quantity of both pairs of a unit, even and odd states apart, so that the rotations are
+// plain packed multiply-adds.  Whatever a window needs from global memory is requested before the first step: per-step
+// scalars by the lane that owns the step (handed round by shuffles), theta into registers, the rows of b and c into
+// shared memory, where all channels of the CTA read them.  Steps past the end of the sequence read as zeros, which
+// leaves state and gradients untouched; only their results are not stored.
+template <typename IO, int PR, int LPC>
+struct Walker {
+  static constexpr int CPW = 32 / LPC;             // channels per warp
+  static constexpr int OWN = (W + LPC - 1) / LPC;  // steps whose scalars a lane holds
+  static constexpr int UN = PR / 2;                // units of two pairs
+  static constexpr int NP = PR * LPC;              // pairs per row, padded
+  static constexpr int kRows = 2 * W + 1;          // rows in shared memory: b of ts-1 .. ts+W-1, then c of ts ..
+  const M3P& p;
+  const M3Idx ix;
+  const int lane, sl, wc, d, b, w, ts, base;
+  const size_t row0;
+  float* rows;  // [kRows][2 (even, odd)][NP]
+  __device__ Walker(const M3P& p_, float* rows_)
+      : p(p_), ix(p_), lane(threadIdx.x & 31), sl(lane % LPC), wc((threadIdx.x >> 5) * CPW + lane / LPC),
+        d(blockIdx.x * ((blockDim.x >> 5) * CPW) + wc), b(blockIdx.z), w(blockIdx.y), ts(w * W), base(lane / LPC * LPC),
+        row0((size_t)b * p_.T + ts), rows(rows_) {}
+  __device__ bool act(int r) const { return sl * PR + r < p.Kp; }
+  __device__ bool in(int s) const { return ts + s < p.T; }
+  __device__ size_t wrow() const { return ((size_t)b * p.nW + w) * p.D + d; }
+  __device__ size_t chan(int s) const { return ix.chan(row0 + s, d); }
+  // per-step scalars: own(f)[o] = f(step sl + LPC o) for the steps inside the sequence; of(v, s): step s's value
+  template <typename F>
+  __device__ void own(float (&v)[OWN], F f) const {
+#pragma unroll
+    for (int o = 0; o < OWN; ++o) {
+      const int s = sl + LPC * o;
+      v[o] = s < W && in(s) ? f(s) : 0.f;
+    }
+  }
+  __device__ float of(const float (&v)[OWN], int s) const { return __shfl_sync(0xffffffffu, v[s / LPC], base + s % LPC); }
+  __device__ void stage(bool with_c) const {
+    const IO *B = static_cast<const IO*>(p.b), *C = static_cast<const IO*>(p.c);
+    const int n = with_c ? kRows : W + 1;
+    const int d0 = blockIdx.x * ((blockDim.x >> 5) * CPW);  // any channel of the CTA: they share a group
+    for (int u = threadIdx.x; u < n * NP; u += blockDim.x) {
+      const int i = u / NP, kp = u - i * NP, t = i <= W ? ts - 1 + i : ts + i - W - 1;
+      float e = 0.f, o = 0.f;
+      if (kp < p.Kp && t >= 0 && t < p.T) {
+        const IO* src = (i <= W ? B : C) + ix.grp((size_t)b * p.T + t, d0, 2 * kp);
+        e = to_f32(src[0]);
+        o = to_f32(src[1]);
+      }
+      rows[i * 2 * NP + kp] = e;
+      rows[i * 2 * NP + NP + kp] = o;
+    }
+  }
+  // row i of the staged rows in the frame of the angles: (c e + s o, c o - s e)
+  __device__ void rotated(int i, int u, f2 sn, f2 cs, f2& v0, f2& v1) const {
+    const f2 e = *reinterpret_cast<const f2*>(rows + i * 2 * NP + sl * PR + 2 * u);
+    const f2 o = *reinterpret_cast<const f2*>(rows + i * 2 * NP + NP + sl * PR + 2 * u);
+    v0 = mad2(sn, o, mul2(cs, e));
+    v1 = mad2(neg2(sn), e, mul2(cs, o));
+  }
+  __device__ void rot_b(int s, int u, f2 sn, f2 cs, f2& v0, f2& v1) const { rotated(s + 1, u, sn, cs, v0, v1); }  // step ts + s
+  __device__ void rot_c(int s, int u, f2 sn, f2 cs, f2& v0, f2& v1) const { rotated(W + 1 + s, u, sn, cs, v0, v1); }
+  // one value per pair, from a row of Kp
+  __device__ f2 two(const float* s, int u) const {
+    s += sl * PR + 2 * u;
+    if (p.vec) {
+      if (!act(2 * u)) return 0ull;
+      const float2 x = *reinterpret_cast<const float2*>(s);
+      return pack2(x.x, x.y);
+    }
+    return pack2(act(2 * u) ? s[0] : 0.f, act(2 * u + 1) ? s[1] : 0.f);
+  }
+  __device__ void put_two(float* s, int u, f2 v) const {
+    const float2 x = unpack2(v);
+    s += sl * PR + 2 * u;
+    if (p.vec) {
+      if (act(2 * u)) *reinterpret_cast<float2*>(s) = x;
+      return;
+    }
+    if (act(2 * u)) s[0] = x.x;
+    if (act(2 * u + 1)) s[1] = x.y;
+  }
+  __device__ void thetas(f2 (&th)[W][UN]) const {
+    const size_t stride = p.NH > 0 ? p.NH : (size_t)p.D * p.Kp;
+    const float* src = p.theta + ix.theta(row0, d, 0);
+#pragma unroll
+    for (int s = 0; s < W; ++s)
+#pragma unroll
+      for (int u = 0; u < UN; ++u) th[s][u] = !in(s) ? 0ull : p.NH > 0 ? dup2(src[s * stride]) : two(src + s * stride, u);
+  }
+  // a row of N states: even (v0) and odd (v1) states of a unit
+  __device__ void states(const float* s, int u, f2& v0, f2& v1) const {
+    s += 2 * (sl * PR + 2 * u);
+    if (p.vec) {
+      const float4 x = act(2 * u) ? *reinterpret_cast<const float4*>(s) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v0 = pack2(x.x, x.z);
+      v1 = pack2(x.y, x.w);
+      return;
+    }
+    v0 = pack2(act(2 * u) ? s[0] : 0.f, act(2 * u + 1) ? s[2] : 0.f);
+    v1 = pack2(act(2 * u) ? s[1] : 0.f, act(2 * u + 1) ? s[3] : 0.f);
+  }
+  __device__ void put_states(float* s, int u, f2 v0, f2 v1) const {
+    const float2 x = unpack2(v0), y = unpack2(v1);
+    s += 2 * (sl * PR + 2 * u);
+    if (p.vec) {
+      if (act(2 * u)) *reinterpret_cast<float4*>(s) = make_float4(x.x, y.x, x.y, y.y);
+      return;
+    }
+    if (act(2 * u)) { s[0] = x.x; s[1] = y.x; }
+    if (act(2 * u + 1)) { s[2] = x.y; s[3] = y.y; }
+  }
+  __device__ void rates(f2 (&A)[PR]) const {  // A[2 u]: even states of unit u, A[2 u + 1]: odd
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+      float a[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) a[x] = act(2 * u + x / 2) ? -expf(p.a_log[ix.alog(d, 2 * (sl * PR + 2 * u) + x)]) : 0.f;
+      A[2 * u] = pack2(a[0], a[2]);
+      A[2 * u + 1] = pack2(a[1], a[3]);
+    }
+  }
+  // rotated b of the step before the window, at the window's start angle
+  __device__ void before(const f2 (&phi)[UN], f2 (&pb)[PR]) const {
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+      f2 sn, cs;
+      sincos2(phi[u], sn, cs);
+      rot_b(-1, u, sn, cs, pb[2 * u], pb[2 * u + 1]);
+    }
+  }
+};
+template <typename IO, int PR, int LPC>
+constexpr int kRowBytes = (2 * W + 1) * 2 * PR * LPC * 4;
+
+// ------------------------------------------------------------------ prepare
+template <typename IO, int PR, int LPC>
+__global__ void __launch_bounds__(256) m3w_prepare_kernel(M3P p) {
+  using K = Walker<IO, PR, LPC>;
+  const K k(p, nullptr);
+  f2 th[W][K::UN], ph[K::UN];
+  k.thetas(th);
+  const bool store = p.NH == 0 || k.d % k.ix.cph == 0;
+  float dts[K::OWN];
+  k.own(dts, [&](int s) {
+    const size_t i = k.chan(s);
+    const float v = m3_softplus(p.dt[i]);
+    if (store) {
+      p.dtv[i] = v;
+      p.lamv[i] = m3_sigmoid(p.lam[i]);
+    }
+    return v;
+  });
+  float sum = 0.f;
+#pragma unroll
+  for (int u = 0; u < K::UN; ++u) ph[u] = 0ull;
+#pragma unroll
+  for (int s = 0; s < W; ++s) {
+    const float dt = k.of(dts, s);
+    sum += dt;
+#pragma unroll
+    for (int u = 0; u < K::UN; ++u) ph[u] = mad2(dup2(dt), th[s][u], ph[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < K::UN; ++u) k.put_two(p.ck_phi + k.wrow() * p.Kp, u, ph[u]);
+  if (k.sl == 0) p.dtsum[k.wrow()] = sum;
+}
+
+// -------------------------------------------------------------------- scans
+// 32 chains x 16 segments of windows per CTA: every segment is folded, the folds of the earlier segments give what
+// enters it, and the segment is walked again to write.  Loads in batches ahead of the stores.
+//   kPhase  ck_phi: window sums -> wrapped angle at each window start
+//   kState  ck_h: local end states -> state at each window start
+//   kDh     dhk: local dh -> dh entering each window from later steps; upk: local -> true `up` of its first step
+//   kAngle  ang: window sums -> sum over all later windows
+enum { kPhase, kState, kDh, kAngle };
+constexpr int kSegs = 16, kBatch = 8;
+template <int MODE>
+__device__ __forceinline__ void scan_chain(const M3P& p, int chains) {
+  __shared__ float s_add[kSegs][32], s_dt[kSegs][32];
+  const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5, b = blockIdx.y;
+  const int i = blockIdx.x * 32 + lane;
+  const bool in = i < chains;
+  const bool linear = MODE == kState || MODE == kDh;
+  const int per = (p.nW + kSegs - 1) / kSegs, lo = min(p.nW, seg * per), hi = min(p.nW, lo + per);
+  float* buf = MODE == kPhase ? p.ck_phi : MODE == kState ? p.ck_h : MODE == kDh ? p.dhk : p.ang;
+  const int d = linear ? i / p.N : 0;
+  const M3Idx ix(p);
+  const float A = linear && in ? -expf(p.a_log[ix.alog(d, i % p.N)]) : 0.f;
+  auto win = [&](int x) { return MODE == kDh || MODE == kAngle ? p.nW - 1 - x : x; };  // x-th window in walking order
+  auto at = [&](int w) { return ((size_t)b * p.nW + w) * chains + i; };
+  float run = 0.f, dts = 0.f;
+  for (int x0 = lo; x0 < hi; x0 += kBatch) {
+    float loc[kBatch], dec[kBatch];
+#pragma unroll
+    for (int x = 0; x < kBatch; ++x) {
+      const bool ok = in && x0 + x < hi;
+      loc[x] = ok ? buf[at(win(x0 + x))] : 0.f;
+      dec[x] = ok && linear ? p.dtsum[((size_t)b * p.nW + win(x0 + x)) * p.D + d] : 0.f;
+    }
+#pragma unroll
+    for (int x = 0; x < kBatch; ++x) {
+      if (linear) run = fmaf(expf(A * dec[x]), run, loc[x]);
+      else run = MODE == kPhase ? m3_wrap(run + loc[x]) : run + loc[x];
+      dts += dec[x];
+    }
+  }
+  s_add[seg][lane] = run;
+  s_dt[seg][lane] = dts;
+  __syncthreads();
+  run = 0.f;
+  for (int s = 0; s < seg; ++s) {
+    if (linear) run = fmaf(expf(A * s_dt[s][lane]), run, s_add[s][lane]);
+    else run = MODE == kPhase ? m3_wrap(run + s_add[s][lane]) : run + s_add[s][lane];
+  }
+  for (int x0 = lo; x0 < hi; x0 += kBatch) {
+    float loc[kBatch], dec[kBatch], up[kBatch], dt0[kBatch];
+#pragma unroll
+    for (int x = 0; x < kBatch; ++x) {
+      const bool ok = in && x0 + x < hi;
+      const int w = win(x0 + x);
+      loc[x] = ok ? buf[at(w)] : 0.f;
+      dec[x] = ok && linear ? p.dtsum[((size_t)b * p.nW + w) * p.D + d] : 0.f;
+      if (MODE == kDh) {
+        up[x] = ok ? p.upk[at(w)] : 0.f;
+        dt0[x] = ok ? p.dtv[ix.chan((size_t)b * p.T + (size_t)w * W, d)] : 0.f;
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < kBatch; ++x) {
+      if (in && x0 + x < hi) {
+        const int w = win(x0 + x);
+        buf[at(w)] = run;
+        if (MODE == kDh) p.upk[at(w)] = fmaf(expf(A * (dec[x] - dt0[x])), run, up[x]);
+      }
+      if (linear) run = fmaf(expf(A * dec[x]), run, loc[x]);
+      else run = MODE == kPhase ? m3_wrap(run + loc[x]) : run + loc[x];
+    }
+  }
+}
+__global__ void __launch_bounds__(32 * kSegs) m3w_phase_scan_kernel(M3P p) { scan_chain<kPhase>(p, p.D * p.Kp); }
+__global__ void __launch_bounds__(32 * kSegs) m3w_angle_scan_kernel(M3P p) { scan_chain<kAngle>(p, p.D * p.Kp); }
+// blockIdx.z: 0 the states, 1 dh (first: the one to start with)
+__global__ void __launch_bounds__(32 * kSegs) m3w_linear_scan_kernel(M3P p, int first) {
+  if (first + (int)blockIdx.z == 0) scan_chain<kState>(p, p.D * p.N);
+  else scan_chain<kDh>(p, p.D * p.N);
+}
+
+// -------------------------------------------------------------- local walks
+// Forward from a zero state (leaves the end state in ck_h) and, with DH, back with dh alone:
+//   up_t = dh_t + dy_t Crot_t,  dh_{t-1} = alpha_t up_t
+// (leaves the dh that leaves the window at its start in dhk and the up of its first step in upk).  Sine, cosine and
+// decay of a step wait in shared memory for the way back.
+template <typename IO, int PR, int LPC, bool FWD, bool DH>
+__global__ void __launch_bounds__(256) m3w_local_kernel(M3P p) {
+  using K = Walker<IO, PR, LPC>;
+  constexpr int UN = K::UN;
+  extern __shared__ f2 hist[];  // [W][2 PR][threads], then the rows
+  const K k(p, reinterpret_cast<float*>(hist + (DH ? W * 2 * PR * blockDim.x : 0)));
+  auto slot = [&](int s, int x) -> f2& { return hist[(s * (2 * PR) + x) * blockDim.x + threadIdx.x]; };
+  const IO *X = static_cast<const IO*>(p.x), *DY = static_cast<const IO*>(p.dy);
+  f2 th[W][UN], A[PR], phi[UN];
+  k.thetas(th);
+  float dts[K::OWN], lams[K::OWN], xs[K::OWN], dys[K::OWN], px = 0.f;
+  k.own(dts, [&](int s) { return p.dtv[k.chan(s)]; });
+  if (FWD) {
+    k.own(lams, [&](int s) { return p.lamv[k.chan(s)]; });
+    k.own(xs, [&](int s) { return to_f32(X[(k.row0 + s) * p.D + k.d]); });
+    if (k.ts > 0) px = to_f32(X[(k.row0 - 1) * p.D + k.d]);
+  }
+  if (DH) k.own(dys, [&](int s) { return to_f32(DY[(k.row0 + s) * p.D + k.d]); });
+  k.stage(DH);
+#pragma unroll
+  for (int u = 0; u < UN; ++u) phi[u] = k.two(p.ck_phi + k.wrow() * p.Kp, u);
+  k.rates(A);
+  __syncthreads();
+  f2 h[PR], pb[PR];
+  if (FWD) {
+#pragma unroll
+    for (int r = 0; r < PR; ++r) h[r] = 0ull;
+    k.before(phi, pb);
+  }
+#pragma unroll
+  for (int s = 0; s < W; ++s) {
+    const float dt = k.of(dts, s);
+    f2 gx = 0ull, bx = 0ull;
+    if (FWD) {
+      const float lam = k.of(lams, s), x = k.of(xs, s);
+      gx = dup2(lam * dt * x);
+      bx = dup2((1.f - lam) * dt * px);
+      px = x;
+    }
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+      f2 sn, cs;
+      phi[u] = wrap2(mad2(dup2(dt), th[s][u], phi[u]));
+      sincos2(phi[u], sn, cs);
+      const f2 al0 = exp2p(A[2 * u], dt), al1 = exp2p(A[2 * u + 1], dt);
+      if (DH) {
+        slot(s, 2 * u) = al0;
+        slot(s, 2 * u + 1) = al1;
+        slot(s, PR + 2 * u) = sn;
+        slot(s, PR + 2 * u + 1) = cs;
+      }
+      if (FWD) {
+        f2 b0, b1;
+        k.rot_b(s, u, sn, cs, b0, b1);
+        h[2 * u] = mad2(al0, mad2(bx, pb[2 * u], h[2 * u]), mul2(gx, b0));
+        h[2 * u + 1] = mad2(al1, mad2(bx, pb[2 * u + 1], h[2 * u + 1]), mul2(gx, b1));
+        pb[2 * u] = b0;
+        pb[2 * u + 1] = b1;
+      }
+    }
+  }
+  if (FWD) {
+#pragma unroll
+    for (int u = 0; u < UN; ++u) k.put_states(p.ck_h + k.wrow() * p.N, u, h[2 * u], h[2 * u + 1]);
+  }
+  if (DH) {
+    f2 dh[PR], up[PR];
+#pragma unroll
+    for (int r = 0; r < PR; ++r) dh[r] = up[r] = 0ull;
+#pragma unroll
+    for (int s = W - 1; s >= 0; --s) {
+      const f2 dy = dup2(k.of(dys, s));
+#pragma unroll
+      for (int u = 0; u < UN; ++u) {
+        f2 c0, c1;
+        k.rot_c(s, u, slot(s, PR + 2 * u), slot(s, PR + 2 * u + 1), c0, c1);
+        up[2 * u] = mad2(dy, c0, dh[2 * u]);
+        up[2 * u + 1] = mad2(dy, c1, dh[2 * u + 1]);
+        dh[2 * u] = mul2(slot(s, 2 * u), up[2 * u]);
+        dh[2 * u + 1] = mul2(slot(s, 2 * u + 1), up[2 * u + 1]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+      k.put_states(p.dhk + k.wrow() * p.N, u, dh[2 * u], dh[2 * u + 1]);
+      k.put_states(p.upk + k.wrow() * p.N, u, up[2 * u], up[2 * u + 1]);
+    }
+  }
+}
+
+// ------------------------------------------------------------ forward walk
+template <typename IO, int PR, int LPC>
+__global__ void __launch_bounds__(256) m3w_out_kernel(M3P p) {
+  using K = Walker<IO, PR, LPC>;
+  constexpr int UN = K::UN;
+  extern __shared__ f2 hist[];
+  const K k(p, reinterpret_cast<float*>(hist));
+  const IO* X = static_cast<const IO*>(p.x);
+  IO* Y = static_cast<IO*>(p.y);
+  f2 th[W][UN], A[PR], h[PR], phi[UN], pb[PR];
+  k.thetas(th);
+  float dts[K::OWN], lams[K::OWN], xs[K::OWN];
+  k.own(dts, [&](int s) { return p.dtv[k.chan(s)]; });
+  k.own(lams, [&](int s) { return p.lamv[k.chan(s)]; });
+  k.own(xs, [&](int s) { return to_f32(X[(k.row0 + s) * p.D + k.d]); });
+  float px = k.ts > 0 ? to_f32(X[(k.row0 - 1) * p.D + k.d]) : 0.f;
+  k.stage(true);
+#pragma unroll
+  for (int u = 0; u < UN; ++u) {
+    phi[u] = k.two(p.ck_phi + k.wrow() * p.Kp, u);
+    k.states(p.ck_h + k.wrow() * p.N, u, h[2 * u], h[2 * u + 1]);
+  }
+  k.rates(A);
+  __syncthreads();
+  k.before(phi, pb);
+  float ys[K::OWN];
+#pragma unroll
+  for (int s = 0; s < W; ++s) {
+    const float dt = k.of(dts, s), lam = k.of(lams, s), x = k.of(xs, s);
+    const f2 gx = dup2(lam * dt * x), bx = dup2((1.f - lam) * dt * px);
+    px = x;
+    f2 part = 0ull;
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+      f2 sn, cs, b0, b1, c0, c1;
+      phi[u] = wrap2(mad2(dup2(dt), th[s][u], phi[u]));
+      sincos2(phi[u], sn, cs);
+      k.rot_b(s, u, sn, cs, b0, b1);
+      k.rot_c(s, u, sn, cs, c0, c1);
+      h[2 * u] = mad2(exp2p(A[2 * u], dt), mad2(bx, pb[2 * u], h[2 * u]), mul2(gx, b0));
+      h[2 * u + 1] = mad2(exp2p(A[2 * u + 1], dt), mad2(bx, pb[2 * u + 1], h[2 * u + 1]), mul2(gx, b1));
+      part = mad2(h[2 * u], c0, part);
+      part = mad2(h[2 * u + 1], c1, part);
+      pb[2 * u] = b0;
+      pb[2 * u + 1] = b1;
+    }
+    const float y = group_sum<LPC>(sum2(part));
+    if (k.sl == s % LPC) ys[s / LPC] = y;
+  }
+#pragma unroll
+  for (int o = 0; o < K::OWN; ++o) {
+    const int s = k.sl + LPC * o;
+    if (s < W && k.in(s)) Y[(k.row0 + s) * p.D + k.d] = from_f32<IO>(ys[o]);
+  }
+}
+
+// ----------------------------------------------------------- backward walk
+// Sums of N = 4 PR values over the channels of a warp: each exchange halves the values a lane still carries, the
+// channel's bit choosing the half it keeps.  On return v[0 .. N / CPW) of channel c are the sums of the values first ..
+template <int N, int CPW, int LPC>
+__device__ __forceinline__ int sum_channels(float (&v)[N], int ch) {
+  int first = 0;
+#pragma unroll
+  for (int m = CPW / 2, n = N / 2; m > 0; m /= 2, n /= 2) {
+    const bool up = (ch & m) != 0;
+#pragma unroll
+    for (int x = 0; x < n; ++x) {
+      const float send = up ? v[x] : v[x + n], keep = up ? v[x + n] : v[x];
+      v[x] = keep + __shfl_xor_sync(0xffffffffu, send, m * LPC);
+    }
+    if (up) first += n;
+  }
+  return first;
+}
+// Sums of four values over the lanes of a channel: lane sl ends up with that of value sl & 3.
+template <int LPC>
+__device__ __forceinline__ float sum_lanes4(float a, float b, float c, float d, int sl) {
+  const bool b0 = sl & 1, b1 = sl & 2;
+  const float u0 = (b0 ? b : a) + __shfl_xor_sync(0xffffffffu, b0 ? a : b, 1);
+  const float u1 = (b0 ? d : c) + __shfl_xor_sync(0xffffffffu, b0 ? c : d, 1);
+  float v = (b1 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, b1 ? u0 : u1, 2);
+#pragma unroll
+  for (int o = 4; o < LPC; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+template <int PR, int LPC>
+struct GradSmem {  // bytes per thread, per warp and fixed
+  static constexpr int kThread = W * 3 * PR * 8, kWarp = W * 2 * 2 * PR * LPC * 4 + W * (32 / LPC) * 5 * 4;
+};
+// grid (D / channels of a CTA, windows, B)
+template <typename IO, int PR, int LPC>
+__global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
+  using K = Walker<IO, PR, LPC>;
+  constexpr int UN = K::UN, CPW = K::CPW, KEEP = 4 * PR / CPW > 0 ? 4 * PR / CPW : 1, NR = 2 * K::NP;
+  static_assert(4 * PR >= CPW, "a lane keeps at least one sum");
+  extern __shared__ f2 hist[];  // [W][3 PR][threads]: h after the step, decay, sine / cosine
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5;
+  float* red = reinterpret_cast<float*>(hist + (size_t)W * 3 * PR * blockDim.x);  // [W][warps][2 (dB, dC)][NR]
+  float* fin = red + (size_t)W * warps * 2 * NR;                                  // [W][channels][4]
+  float* fin5 = fin + W * warps * CPW * 4;                                        // [W][channels]
+  const K k(p, fin5 + W * warps * CPW);
+  auto slot = [&](int s, int x) -> f2& { return hist[(s * (3 * PR) + x) * blockDim.x + threadIdx.x]; };
+  const IO *X = static_cast<const IO*>(p.x), *DY = static_cast<const IO*>(p.dy);
+  const bool per_head = p.NH > 0;
+  f2 th[W][UN], A[PR], h[PR], pb[PR], phi[UN], dh[PR], pgb[PR];
+  k.thetas(th);
+  float dts[K::OWN], lams[K::OWN], xs[K::OWN], dys[K::OWN];
+  k.own(dts, [&](int s) { return p.dtv[k.chan(s)]; });
+  k.own(lams, [&](int s) { return p.lamv[k.chan(s)]; });
+  k.own(xs, [&](int s) { return to_f32(X[(k.row0 + s) * p.D + k.d]); });
+  k.own(dys, [&](int s) { return to_f32(DY[(k.row0 + s) * p.D + k.d]); });
+  const float px0 = k.ts > 0 ? to_f32(X[(k.row0 - 1) * p.D + k.d]) : 0.f;
+  const bool more = k.in(W);  // a window follows: its first step sends something back to this one's last
+  float dt_e = 0.f, bf_e = 0.f;
+  if (more) {
+    dt_e = p.dtv[k.chan(W)];
+    bf_e = (1.f - p.lamv[k.chan(W)]) * dt_e;
+  }
+  k.stage(true);
+#pragma unroll
+  for (int u = 0; u < UN; ++u) {
+    phi[u] = k.two(p.ck_phi + k.wrow() * p.Kp, u);
+    k.states(p.ck_h + k.wrow() * p.N, u, h[2 * u], h[2 * u + 1]);
+    k.states(p.dhk + k.wrow() * p.N, u, dh[2 * u], dh[2 * u + 1]);
+    pgb[2 * u] = pgb[2 * u + 1] = 0ull;
+    if (more) k.states(p.upk + (k.wrow() + p.D) * p.N, u, pgb[2 * u], pgb[2 * u + 1]);
+  }
+  k.rates(A);
+  __syncthreads();
+  k.before(phi, pb);
+  f2 hs[PR], pbs[PR];  // state and rotated b before the window's first step
+#pragma unroll
+  for (int r = 0; r < PR; ++r) {
+    hs[r] = h[r];
+    pbs[r] = pb[r];
+  }
+  // ---- replay, keeping state, decay, sine and cosine of every step ----
+  float px = px0;
+#pragma unroll
+  for (int s = 0; s < W; ++s) {
+    const float dt = k.of(dts, s), lam = k.of(lams, s), x = k.of(xs, s);
+    const f2 gx = dup2(lam * dt * x), bx = dup2((1.f - lam) * dt * px);
+    px = x;
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+      f2 sn, cs, b0, b1;
+      phi[u] = wrap2(mad2(dup2(dt), th[s][u], phi[u]));
+      sincos2(phi[u], sn, cs);
+      k.rot_b(s, u, sn, cs, b0, b1);
+      const f2 al0 = exp2p(A[2 * u], dt), al1 = exp2p(A[2 * u + 1], dt);
+      h[2 * u] = mad2(al0, mad2(bx, pb[2 * u], h[2 * u]), mul2(gx, b0));
+      h[2 * u + 1] = mad2(al1, mad2(bx, pb[2 * u + 1], h[2 * u + 1]), mul2(gx, b1));
+      pb[2 * u] = b0;
+      pb[2 * u + 1] = b1;
+      slot(s, 2 * u) = h[2 * u];
+      slot(s, 2 * u + 1) = h[2 * u + 1];
+      slot(s, PR + 2 * u) = al0;
+      slot(s, PR + 2 * u + 1) = al1;
+      slot(s, 2 * PR + 2 * u) = sn;
+      slot(s, 2 * PR + 2 * u + 1) = cs;
+    }
+  }
+  // ---- what the first step of the next window sends back (pgb holds its `up`) ----
+  f2 dal[PR], carry[UN];
+  f2 pend = 0ull;  // contribution of step t+1 to dx_t (lane partial)
+#pragma unroll
+  for (int u = 0; u < UN; ++u) {
+    carry[u] = 0ull;
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      const int r = 2 * u + y;
+      dal[r] = 0ull;
+      if (more) {
+        const f2 v = mul2(pgb[r], mul2(dup2(bf_e), exp2p(A[r], dt_e)));
+        pend = mad2(pb[r], v, pend);
+        pgb[r] = mul2(dup2(px), v);
+      }
+    }
+  }
+  // ---- reverse: pb = rotated b of the step, q = that of the step before ----
+#pragma unroll
+  for (int s = W - 1; s >= 0; --s) {
+    const float dt = k.of(dts, s), lam = k.of(lams, s), x = k.of(xs, s), dy = k.of(dys, s);
+    const float xprev = s > 0 ? k.of(xs, s > 0 ? s - 1 : 0) : px0;
+    const float bf = (1.f - lam) * dt;
+    const f2 dy2 = dup2(dy), gx = dup2(lam * dt * x), bx = dup2(bf * xprev), dt2 = dup2(dt);
+    f2 s_bu = 0ull, s_qv = 0ull, s_a = 0ull, s_ca = 0ull;
+    float rows[4 * PR];  // this lane's values of dB (first half) and dC of the step
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+      const f2 sn = slot(s, 2 * PR + 2 * u), cs = slot(s, 2 * PR + 2 * u + 1), nsn = neg2(sn);
+      f2 q[2], c[2], gb[2], gc[2];
+      if (s > 0) k.rot_b(s - 1, u, slot(s - 1, 2 * PR + 2 * u), slot(s - 1, 2 * PR + 2 * u + 1), q[0], q[1]);
+      else { q[0] = pbs[2 * u]; q[1] = pbs[2 * u + 1]; }
+      k.rot_c(s, u, sn, cs, c[0], c[1]);
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const int r = 2 * u + y;
+        const f2 hb = s > 0 ? slot(s - 1, r) : hs[r];
+        const f2 up = mad2(dy2, c[y], dh[r]);
+        const f2 v = mul2(slot(s, PR + r), up);
+        s_bu = mad2(pb[r], up, s_bu);
+        s_qv = mad2(q[y], v, s_qv);
+        gb[y] = mad2(gx, up, pgb[r]);
+        gc[y] = mul2(dy2, slot(s, r));
+        const f2 wv = mul2(A[r], mul2(v, mad2(bx, q[y], hb)));
+        s_a = add2(s_a, wv);
+        dal[r] = mad2(dt2, wv, dal[r]);
+        pgb[r] = mul2(bx, v);
+        dh[r] = v;
+      }
+      // rotation adjoint: rows of dB and dC, and the angle gradient of the pairs
+      const float2 be = unpack2(mad2(nsn, gb[1], mul2(cs, gb[0]))), bo = unpack2(mad2(sn, gb[0], mul2(cs, gb[1])));
+      const float2 ce = unpack2(mad2(nsn, gc[1], mul2(cs, gc[0]))), co = unpack2(mad2(sn, gc[0], mul2(cs, gc[1])));
+      float* rb = rows + 4 * u;
+      float* rc = rows + 2 * PR + 4 * u;
+      rb[0] = be.x; rb[1] = bo.x; rb[2] = be.y; rb[3] = bo.y;
+      rc[0] = ce.x; rc[1] = co.x; rc[2] = ce.y; rc[3] = co.y;
+      f2 turn = mad2(pb[2 * u + 1], gb[0], mul2(c[1], gc[0]));
+      turn = add2(turn, neg2(mad2(pb[2 * u], gb[1], mul2(c[0], gc[1]))));
+      carry[u] = add2(carry[u], turn);
+      pb[2 * u] = q[0];
+      pb[2 * u + 1] = q[1];
+      s_a = mad2(carry[u], th[s][u], s_a);
+      if (per_head) s_ca = add2(s_ca, carry[u]);
+      else if (k.in(s)) k.put_two(p.dtheta + ((k.row0 + s) * p.D + k.d) * p.Kp, u, mul2(carry[u], dt2));
+    }
+    const float v = sum_lanes4<LPC>(sum2(s_bu), sum2(s_qv), sum2(s_a), sum2(pend), k.sl);
+    if (k.sl < 4) fin[(s * warps * CPW + k.wc) * 4 + k.sl] = v;
+    if (per_head) {
+      const float t = group_sum<LPC>(sum2(s_ca));
+      if (k.sl == 0) fin5[s * warps * CPW + k.wc] = t;
+    }
+    pend = mul2(dup2(bf), s_qv);
+    const int first = sum_channels<4 * PR, CPW, LPC>(rows, k.lane / LPC);
+    float* dst = red + (size_t)(s * warps + warp) * 2 * NR;
+#pragma unroll
+    for (int y = 0; y < KEEP; ++y) {
+      const int v2 = first + y;  // value of this lane: dB for v2 < 2 PR, then dC
+      dst[(v2 >= 2 * PR ? NR : 0) + k.sl * 2 * PR + v2 % (2 * PR)] = rows[y];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < UN; ++u) k.put_two(p.ang + k.wrow() * p.Kp, u, carry[u]);
+  // da_log: d/d a_log = d/dA * A  (A = -exp(a_log)); the closed form above already carries A
+  if (per_head) {
+    f2 sum = 0ull;
+#pragma unroll
+    for (int r = 0; r < PR; ++r) sum = add2(sum, dal[r]);
+    const float v = group_sum<LPC>(sum2(sum));
+    if (k.sl == 0) p.dal_part[k.wrow()] = v;
+  } else {
+#pragma unroll
+    for (int u = 0; u < UN; ++u) k.put_states(p.dal_part + k.wrow() * p.N, u, dal[2 * u], dal[2 * u + 1]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int o = 0; o < K::OWN; ++o) {  // the lane that owns a step finishes its scalars: dx, ddt, dlambda
+    const int s = k.sl + LPC * o;
+    const float xp = __shfl_sync(0xffffffffu, o > 0 && k.sl == LPC - 1 ? xs[o > 0 ? o - 1 : 0] : xs[o], (k.sl == 0 ? k.base + LPC - 1 : k.lane - 1));
+    if (s < W && k.in(s)) {
+      const float4 f = *reinterpret_cast<const float4*>(fin + (s * warps * CPW + k.wc) * 4);  // b.up, q.v, rest, dx of later step
+      const float dt = dts[o], lam = lams[o], x = xs[o], xprev = s == 0 ? px0 : xp;
+      const size_t i = (k.row0 + s) * p.D + k.d, ci = k.chan(s);
+      static_cast<IO*>(p.dx)[i] = from_f32<IO>(fmaf(lam * dt, f.x, f.w));
+      const float dsp = (f.z + (1.f - lam) * xprev * f.y + lam * x * f.x) * m3_sigmoid(p.dt[ci]);
+      const float dlam = dt * (x * f.x - xprev * f.y) * lam * (1.f - lam);
+      if (per_head) {  // per channel; m3_head_sum_kernel adds the channels of a head
+        const size_t btd = (size_t)p.B * p.T * p.D;
+        p.hd[i] = dsp;
+        p.hd[btd + i] = dlam;
+        p.hd[2 * btd + i] = fin5[s * warps * CPW + k.wc] * dt;
+      } else {
+        p.ddt[ci] = dsp;
+        p.dlam[ci] = dlam;
+      }
+    }
+  }
+  __syncthreads();
+  const int g = k.d / k.ix.cpg, slice = (k.d % k.ix.cpg) / (warps * CPW), steps = min(W, p.T - k.ts);
+  for (int i = threadIdx.x; i < steps * 2 * p.N; i += blockDim.x) {
+    const int s = i / (2 * p.N), v = i - s * 2 * p.N, which = v >= p.N, n = v - which * p.N;
+    const float* src = red + (size_t)s * warps * 2 * NR + which * NR + n;
+    float acc = 0.f;
+    for (int y = 0; y < warps; ++y) acc += src[(size_t)y * 2 * NR];
+    (which ? p.pc32 : p.pb32)[(((k.row0 + s) * p.G + g) * p.S + slice) * p.N + n] = acc;
+  }
+}
+
+// The angle gradient reaches every earlier step: the later windows' sums are added to ddt and dtheta of each step
+// (the walks used only the sums inside their own window).
+template <typename IO, int PR, int LPC>
+__global__ void __launch_bounds__(256) m3w_fix_kernel(M3P p) {
+  using K = Walker<IO, PR, LPC>;
+  constexpr int UN = K::UN;
+  const K k(p, nullptr);
+  if (k.w == p.nW - 1) return;  // nothing comes after the last window (every other one is whole)
+  const bool per_head = p.NH > 0;
+  const size_t stride = (size_t)p.D * p.Kp;
+  float* dst = p.dtheta + (k.row0 * p.D + k.d) * p.Kp;
+  f2 off[UN], th[W][UN], dth[W][UN];
+#pragma unroll
+  for (int u = 0; u < UN; ++u) off[u] = k.two(p.ang + k.wrow() * p.Kp, u);
+  k.thetas(th);
+  if (!per_head) {
+#pragma unroll
+    for (int s = 0; s < W; ++s)
+#pragma unroll
+      for (int u = 0; u < UN; ++u) dth[s][u] = k.two(dst + s * stride, u);
+  }
+  float dts[K::OWN], raw[K::OWN], add[K::OWN];
+  k.own(dts, [&](int s) { return p.dtv[k.chan(s)]; });
+  k.own(raw, [&](int s) { return p.dt[k.chan(s)]; });
+#pragma unroll
+  for (int s = 0; s < W; ++s) {
+    const f2 dt = dup2(k.of(dts, s));
+    f2 acc = 0ull;
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+      acc = mad2(off[u], th[s][u], acc);
+      if (!per_head) k.put_two(dst + s * stride, u, mad2(off[u], dt, dth[s][u]));
+    }
+    const float v = group_sum<LPC>(sum2(acc));
+    if (k.sl == s % LPC) add[s / LPC] = v;
+  }
+  float o = 0.f;
+  if (per_head) {
+    f2 sum = 0ull;
+#pragma unroll
+    for (int u = 0; u < UN; ++u) sum = add2(sum, off[u]);
+    o = group_sum<LPC>(sum2(sum));
+  }
+#pragma unroll
+  for (int x = 0; x < K::OWN; ++x) {
+    const int s = k.sl + LPC * x;
+    if (s < W) {
+      const float dsp = add[x] * m3_sigmoid(raw[x]);
+      if (per_head) {
+        const size_t btd = (size_t)p.B * p.T * p.D, i = (k.row0 + s) * p.D + k.d;
+        p.hd[i] += dsp;
+        p.hd[2 * btd + i] += o * dts[x];
+      } else {
+        p.ddt[k.chan(s)] += dsp;
+      }
+    }
+  }
+}
+}  // namespace m3w
+
+// --------------------------------------------------------------------- host
+using namespace m3w;
+
+// Lanes per channel: two pairs per lane (four beyond 64 pairs), at least four lanes; a warp's channels share a group.
+M3WinShape m3w_shape(const M3P& p) {
+  const int pr = p.Kp > 64 ? 4 : 2;
+  M3WinShape s{4, 1};
+  while (s.lanes < 32 && (s.lanes * pr < p.Kp || p.D / p.G % (32 / s.lanes) != 0)) s.lanes *= 2;
+  const int per_group = p.D / p.G / (32 / s.lanes), cap = pr == 4 ? 4 : 8;
+  for (int w = 1; w <= cap; ++w)
+    if (per_group % w == 0) s.warps = w;
+  return s;
+}
+
+#define M3W_DISPATCH(lanes, Kp, call)                                       \
+  do {                                                                      \
+    if ((Kp) > 64) { constexpr int PRV = 4, LPCV = 32; call; }              \
+    else if ((lanes) == 4) { constexpr int PRV = 2, LPCV = 4; call; }       \
+    else if ((lanes) == 8) { constexpr int PRV = 2, LPCV = 8; call; }       \
+    else if ((lanes) == 16) { constexpr int PRV = 2, LPCV = 16; call; }     \
+    else { constexpr int PRV = 2, LPCV = 32; call; }                        \
+  } while (0)
+
+struct M3WGrid {
+  M3WinShape shape;
+  dim3 walk;
+  int threads;
+};
+static M3WGrid m3w_grid(const M3P& p) {
+  M3WGrid g{m3w_shape(p), {}, 0};
+  g.threads = 32 * g.shape.warps;
+  g.walk = dim3((p.D + g.shape.warps * (32 / g.shape.lanes) - 1) / (g.shape.warps * (32 / g.shape.lanes)), p.nW, p.B);
+  return g;
+}
+static dim3 chain_grid(const M3P& p, int chains, int kinds) { return dim3((chains + 31) / 32, p.B, kinds); }
+
+template <typename IO, int PR, int LPC, bool FWD, bool DH>
+static mxb_status launch_local(const M3P& p, const M3WGrid& g, cudaStream_t st) {
+  constexpr int per_thread = DH ? W * 2 * PR * 8 : 0, rows = kRowBytes<IO, PR, LPC>;
+  const int sm = per_thread * g.threads + rows;
+  if (MXB_ALLOW_SMEM(per_thread * (PR == 4 ? 128 : 256) + rows, m3w_local_kernel<IO, PR, LPC, FWD, DH>) != MXB_OK) return MXB_ERR_CUDA;
+  MXB_LAUNCH("m3w_local_kernel", st, (m3w_local_kernel<IO, PR, LPC, FWD, DH><<<g.walk, g.threads, sm, st>>>(p)));
+  return MXB_OK;
+}
+template <typename IO, int PR, int LPC>
+static mxb_status launch_grad(const M3P& p, const M3WGrid& g, cudaStream_t st) {
+  constexpr int per_warp = 32 * GradSmem<PR, LPC>::kThread + GradSmem<PR, LPC>::kWarp, rows = kRowBytes<IO, PR, LPC>;
+  if (MXB_ALLOW_SMEM((PR == 4 ? 4 : 8) * per_warp + rows, m3w_grad_kernel<IO, PR, LPC>) != MXB_OK) return MXB_ERR_CUDA;
+  const int sm = g.shape.warps * per_warp + rows;
+  MXB_LAUNCH("m3w_grad_kernel", st, (m3w_grad_kernel<IO, PR, LPC><<<g.walk, g.threads, sm, st>>>(p)));
+  return MXB_OK;
+}
+template <typename IO>
+static mxb_status prepare(const M3P& p, const M3WGrid& g, cudaStream_t st) {
+  M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_prepare_kernel", st, (m3w_prepare_kernel<IO, PRV, LPCV><<<g.walk, g.threads, 0, st>>>(p))));
+  MXB_LAUNCH("m3w_phase_scan_kernel", st, (m3w_phase_scan_kernel<<<chain_grid(p, p.D * p.Kp, 1), 32 * kSegs, 0, st>>>(p)));
+  return check_launch("mamba3 window preparation");
+}
+
+template <typename IO>
+static mxb_status forward(const M3P& p, cudaStream_t st) {
+  const M3WGrid g = m3w_grid(p);
+  mxb_status s = prepare<IO>(p, g, st);
+  if (s != MXB_OK) return s;
+  M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_local<IO, PRV, LPCV, true, false>(p, g, st)));
+  if (s != MXB_OK) return s;
+  MXB_LAUNCH("m3w_linear_scan_kernel", st, (m3w_linear_scan_kernel<<<chain_grid(p, p.D * p.N, 1), 32 * kSegs, 0, st>>>(p, 0)));
+  M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_out_kernel", st, (m3w_out_kernel<IO, PRV, LPCV><<<g.walk, g.threads, kRowBytes<IO, PRV, LPCV>, st>>>(p))));
+  return check_launch("mamba3 window-parallel forward");
+}
+// have_states: angles and states at the window starts (and dtv, lamv) are those a forward on the same inputs left.
+template <typename IO>
+static mxb_status backward(const M3P& p, bool have_states, cudaStream_t st) {
+  const M3WGrid g = m3w_grid(p);
+  mxb_status s = MXB_OK;
+  if (have_states) {
+    M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_local<IO, PRV, LPCV, false, true>(p, g, st)));
+  } else {
+    s = prepare<IO>(p, g, st);
+    if (s == MXB_OK) M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_local<IO, PRV, LPCV, true, true>(p, g, st)));
+  }
+  if (s != MXB_OK) return s;
+  const int first = have_states ? 1 : 0;
+  MXB_LAUNCH("m3w_linear_scan_kernel", st,
+             (m3w_linear_scan_kernel<<<chain_grid(p, p.D * p.N, 2 - first), 32 * kSegs, 0, st>>>(p, first)));
+  M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_grad<IO, PRV, LPCV>(p, g, st)));
+  if (s != MXB_OK) return s;
+  MXB_LAUNCH("m3w_angle_scan_kernel", st, (m3w_angle_scan_kernel<<<chain_grid(p, p.D * p.Kp, 1), 32 * kSegs, 0, st>>>(p)));
+  M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_fix_kernel", st, (m3w_fix_kernel<IO, PRV, LPCV><<<g.walk, g.threads, 0, st>>>(p))));
+  return check_launch("mamba3 window-parallel backward");
+}
+
+mxb_status m3w_forward(const M3P& p, bool f32, cudaStream_t st) {
+  return f32 ? forward<float>(p, st) : forward<__nv_bfloat16>(p, st);
+}
+mxb_status m3w_backward(const M3P& p, bool f32, bool have_states, cudaStream_t st) {
+  return f32 ? backward<float>(p, have_states, st) : backward<__nv_bfloat16>(p, have_states, st);
+}
+
+}  // namespace mxb
