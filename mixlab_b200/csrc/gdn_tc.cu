@@ -199,89 +199,19 @@ __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  // T = (I - A)^-1 in fp32, in place over A.  The two 32 x 32 diagonal blocks by forward substitution
-  // (thread = block and column, the column in registers), then the off-diagonal block
-  // T21 = T22 (A21 T11) as two small fp32 products over all 128 threads.
-  {
-    float Tc[32];
-    const int blk = (tid >> 5) & 1, cc = tid & 31, r0 = 32 * blk;
-    if (ok && tid < C) {
+  // The other half of the CTA meanwhile turns k into diag(d) k in place (its product with itself is done), so that
+  // w = (T diag beta)(diag(d) k) needs no second scaled copy of T.
+  invert_unit_lower(Am, ok, [&](int i) {
+    const float di = dd[i];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float* arow = Am + (r0 + i) * LDA + r0;
-        float s0 = (i == cc) ? 1.f : 0.f, s1 = 0.f;
-#pragma unroll
-        for (int j = 0; j + 1 < i; j += 2) {
-          s0 = fmaf(arow[j], Tc[j], s0);
-          s1 = fmaf(arow[j + 1], Tc[j + 1], s1);
-        }
-        if (i & 1) s0 = fmaf(arow[i - 1], Tc[i - 1], s0);
-        Tc[i] = (i < cc) ? 0.f : s0 + s1;
-      }
-    } else if (ok) {
-      // the other half of the CTA meanwhile turns k into diag(d) k in place (its product with itself is done), so
-      // that w = (T diag beta)(diag(d) k) needs no second scaled copy of T
-      const int i = tid - C;
-      const float di = dd[i];
-#pragma unroll
-      for (int c8 = 0; c8 < 16; ++c8) {
-        uint4* unit = reinterpret_cast<uint4*>(Akq + kq_unit(i, c8));
-        *unit = tc::scale_bf16x8(*unit, di);
-      }
+    for (int c8 = 0; c8 < 16; ++c8) {
+      uint4* unit = reinterpret_cast<uint4*>(Akq + kq_unit(i, c8));
+      *unit = tc::scale_bf16x8(*unit, di);
     }
-    __syncthreads();  // every thread has read its block of A
-    if (ok && tid < C) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) Am[(r0 + i) * LDA + r0 + cc] = Tc[i];
-    }
-    __syncthreads();
-    const int i2 = tid >> 2, jb = (tid & 3) * 8;  // row i2 of the lower-left block, 8 of its columns
-    {  // X = A21 T11 -> the unused upper-right block
-      float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-      for (int k = 0; k < 32; ++k) {
-        const float a = Am[(32 + i2) * LDA + k];
-        const float4 t0 = *reinterpret_cast<const float4*>(Am + k * LDA + jb);
-        const float4 t1 = *reinterpret_cast<const float4*>(Am + k * LDA + jb + 4);
-        x[0] = fmaf(a, t0.x, x[0]); x[1] = fmaf(a, t0.y, x[1]); x[2] = fmaf(a, t0.z, x[2]); x[3] = fmaf(a, t0.w, x[3]);
-        x[4] = fmaf(a, t1.x, x[4]); x[5] = fmaf(a, t1.y, x[5]); x[6] = fmaf(a, t1.z, x[6]); x[7] = fmaf(a, t1.w, x[7]);
-      }
-      *reinterpret_cast<float4*>(Am + i2 * LDA + 32 + jb) = make_float4(x[0], x[1], x[2], x[3]);
-      *reinterpret_cast<float4*>(Am + i2 * LDA + 32 + jb + 4) = make_float4(x[4], x[5], x[6], x[7]);
-    }
-    __syncthreads();
-    {  // T21 = T22 X -> over A21 (nothing reads A21 any more)
-      float y[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-      for (int k = 0; k < 32; ++k) {
-        const float a = Am[(32 + i2) * LDA + 32 + k];
-        const float4 t0 = *reinterpret_cast<const float4*>(Am + k * LDA + 32 + jb);
-        const float4 t1 = *reinterpret_cast<const float4*>(Am + k * LDA + 32 + jb + 4);
-        y[0] = fmaf(a, t0.x, y[0]); y[1] = fmaf(a, t0.y, y[1]); y[2] = fmaf(a, t0.z, y[2]); y[3] = fmaf(a, t0.w, y[3]);
-        y[4] = fmaf(a, t1.x, y[4]); y[5] = fmaf(a, t1.y, y[5]); y[6] = fmaf(a, t1.z, y[6]); y[7] = fmaf(a, t1.w, y[7]);
-      }
-      *reinterpret_cast<float4*>(Am + (32 + i2) * LDA + jb) = make_float4(y[0], y[1], y[2], y[3]);
-      *reinterpret_cast<float4*>(Am + (32 + i2) * LDA + jb + 4) = make_float4(y[4], y[5], y[6], y[7]);
-    }
-    __syncthreads();
-    // the T image and the bf16 operand tile T diag(beta); the upper triangle (it holds X) reads as zero.  Both go
-    // over the fp32 matrix: every thread first reads all its rows, then a barrier, then writes.
+  });
+  {  // the T image and the bf16 operand tile T diag(beta) go over the fp32 matrix: read everything, barrier, write
     uint4 timg[4], tbimg[4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int u = tid + 128 * m, i = urow8(u), c8 = ucol8(u);
-      const float4 a0 = *reinterpret_cast<const float4*>(Am + i * LDA + 8 * c8);
-      const float4 a1 = *reinterpret_cast<const float4*>(Am + i * LDA + 8 * c8 + 4);
-      float e[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, eb[8];
-#pragma unroll
-      for (int y = 0; y < 8; ++y) {
-        const int mm = 8 * c8 + y;
-        e[y] = (mm <= i) ? e[y] : 0.f;
-        eb[y] = e[y] * bet[mm];
-      }
-      timg[m] = pack8f(e);
-      tbimg[m] = pack8f(eb);
-    }
+    load_inverse_images(Am, bet, timg, tbimg);
     __syncthreads();
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
@@ -671,15 +601,19 @@ bool gdn_tc_supported(const mxb_gdn_desc* d) {
   return d->io_dtype == MXB_BF16 && width_ok(d->Dk) && width_ok(d->Dv) && d->chunk >= C;
 }
 
+// Heads of exactly 64 columns have kernels of their own (gdn_tc64.cu); every other width up to 128 rides on 128-wide tiles.
+static bool is64(const TcP& p) { return p.Dk == 64 && p.Dv == 64; }
+
 static size_t carve_tc(TcP& p, void* ws, bool bwd) {
   Carver cv(ws);
-  const size_t nc = (size_t)p.B * p.H * p.n;
+  const size_t nc = (size_t)p.B * p.H * p.n, KD = is64(p) ? 64 : tcg::KD;  // width of the tiles
   p.status = cv.take<int>(64);
   p.gam = cv.take<float>(nc * C);
   p.Tm = cv.take<bf16>(nc * C * C);
   p.w = cv.take<bf16>(nc * C * KD);
   p.u = cv.take<bf16>(nc * C * KD);
   p.P = cv.take<bf16>(nc * C * C);
+  if (is64(p)) p.Pt = cv.take<bf16>(nc * C * C);
   if (bwd) {
     p.hs = cv.take<bf16>(nc * KD * KD);
     p.vn = cv.take<bf16>(nc * C * KD);
@@ -707,6 +641,7 @@ size_t gdn_tc_workspace_bytes(const mxb_gdn_desc* d, bool bwd) {
 }
 
 mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st);
+mxb_status tc64_run_fwd(TcP& p, cudaStream_t st);
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -748,6 +683,7 @@ static bool g_tc_use_tma = true;
 void gdn_tc_set_tma(bool on) { g_tc_use_tma = on; }
 
 mxb_status tc_run_fwd(TcP& p, cudaStream_t st) {
+  if (is64(p)) return tc64_run_fwd(p, st);
   PrepMaps maps;
   std::memset(&maps, 0, sizeof maps);
   // heads narrower than the tiles exist only through the copy engine (the per-thread staging addresses full rows)

@@ -39,6 +39,7 @@ struct TcP {
   bf16* w;       // [C][KD]
   bf16* u;       // [C][KD]
   bf16* P;       // [C][C]
+  bf16* Pt;      // [C][C]    P^T (64-wide kernels only)
   // Everything below is stored as the byte image of the blocked shared-memory operand tile it is read into.
   bf16* hs;      // [KD][KD]  state at chunk start   (backward only)
   bf16* vn;      // [C][KD]
@@ -121,6 +122,89 @@ __device__ __forceinline__ void ld_acc64(uint32_t taddr, int warp, float (&f)[64
   for (int i = 0; i < 32; ++i) {
     f[i] = __uint_as_float(r0[i]);
     f[32 + i] = __uint_as_float(r1[i]);
+  }
+}
+// T = (I - A)^-1 in fp32, in place over the strictly lower triangular [64][LDA] matrix A; 128 threads, `other(t)` is run
+// by threads 64 + t beside the first step.  The two 32 x 32 diagonal blocks by forward substitution (thread = block and
+// column, the column in registers), then the off-diagonal block T21 = T22 (A21 T11) as two small products: 4 x 2 outputs
+// per thread, a warp's share cut so that it skips the zero triangle (one row of 8 outputs per thread over the full
+// contraction read 2.4 times as much shared memory, which is what bounds the prep kernels).  The upper-right block is
+// left with A21 T11, the rest of T is exact.  Ends without a barrier behind the last stores.
+template <typename F>
+__device__ __forceinline__ void invert_unit_lower(float* Am, bool ok, F other) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  float Tc[32];
+  const int r0 = 32 * (warp & 1);
+  if (ok && tid < C) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const float* arow = Am + (r0 + i) * LDA + r0;
+      float s0 = (i == lane) ? 1.f : 0.f, s1 = 0.f;
+#pragma unroll
+      for (int j = 0; j + 1 < i; j += 2) {
+        s0 = fmaf(arow[j], Tc[j], s0);
+        s1 = fmaf(arow[j + 1], Tc[j + 1], s1);
+      }
+      if (i & 1) s0 = fmaf(arow[i - 1], Tc[i - 1], s0);
+      Tc[i] = (i < lane) ? 0.f : s0 + s1;
+    }
+  } else if (ok) {
+    other(tid - C);
+  }
+  __syncthreads();  // every thread has read its block of A
+  if (ok && tid < C) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) Am[(r0 + i) * LDA + r0 + lane] = Tc[i];
+  }
+  __syncthreads();
+  auto product = [&](const float* a, const float* b, int k0, int k1, int row0, int rstep, float* out) {
+    float x[4][2] = {};
+#pragma unroll 2
+    for (int k = k0; k < k1; k += 4) {
+      float4 av[4];
+      float2 bv[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) av[r] = *reinterpret_cast<const float4*>(a + (row0 + rstep * r) * LDA + k);
+#pragma unroll
+      for (int y = 0; y < 4; ++y) bv[y] = *reinterpret_cast<const float2*>(b + (k + y) * LDA);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        x[r][0] = fmaf(av[r].x, bv[0].x, x[r][0]); x[r][1] = fmaf(av[r].x, bv[0].y, x[r][1]);
+        x[r][0] = fmaf(av[r].y, bv[1].x, x[r][0]); x[r][1] = fmaf(av[r].y, bv[1].y, x[r][1]);
+        x[r][0] = fmaf(av[r].z, bv[2].x, x[r][0]); x[r][1] = fmaf(av[r].z, bv[2].y, x[r][1]);
+        x[r][0] = fmaf(av[r].w, bv[3].x, x[r][0]); x[r][1] = fmaf(av[r].w, bv[3].y, x[r][1]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) *reinterpret_cast<float2*>(out + (row0 + rstep * r) * LDA) = make_float2(x[r][0], x[r][1]);
+  };
+  {  // X = A21 T11 -> the unused upper-right block; a warp takes eight columns, T11 is zero above its diagonal
+    const int j = 8 * warp + 2 * (lane & 3);
+    product(Am + 32 * LDA, Am + j, 8 * warp, 32, lane >> 2, 8, Am + 32 + j);
+  }
+  __syncthreads();
+  {  // T21 = T22 X -> over A21 (nothing reads A21 any more); a warp takes eight rows
+    const int j = 2 * (lane & 15);
+    product(Am + 32 * LDA + 32, Am + 32 + j, 0, 8 * warp + 8, 8 * warp + (lane >> 4), 2, Am + 32 * LDA + j);
+  }
+  __syncthreads();
+}
+// This thread's units of the bf16 operand images of T and T diag(beta) (the upper triangle reads as zero).
+__device__ __forceinline__ void load_inverse_images(const float* Am, const float* bet, uint4 (&timg)[4], uint4 (&tbimg)[4]) {
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const int u = threadIdx.x + 128 * m, i = urow8(u), c8 = ucol8(u);
+    const float4 a0 = *reinterpret_cast<const float4*>(Am + i * LDA + 8 * c8);
+    const float4 a1 = *reinterpret_cast<const float4*>(Am + i * LDA + 8 * c8 + 4);
+    float e[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, eb[8];
+#pragma unroll
+    for (int y = 0; y < 8; ++y) {
+      const int mm = 8 * c8 + y;
+      e[y] = (mm <= i) ? e[y] : 0.f;
+      eb[y] = e[y] * bet[mm];
+    }
+    timg[m] = make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]), tc::pack_bf16(e[4], e[5]), tc::pack_bf16(e[6], e[7]));
+    tbimg[m] = make_uint4(tc::pack_bf16(eb[0], eb[1]), tc::pack_bf16(eb[2], eb[3]), tc::pack_bf16(eb[4], eb[5]), tc::pack_bf16(eb[6], eb[7]));
   }
 }
 }  // namespace tcg

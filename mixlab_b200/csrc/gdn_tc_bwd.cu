@@ -721,6 +721,7 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
 
 // ------------------------------------------------------------------ host
 mxb_status tc_run_fwd(TcP& p, cudaStream_t st);
+mxb_status tc64_run_bwd(const TcP& p, cudaStream_t st);
 
 // Forward recompute (saving per-chunk states and v_new), reverse state pass, per-chunk pass.
 mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st) {
@@ -736,6 +737,7 @@ mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st) {
     p.hT = keep_hT;
     if (s != MXB_OK) return s;
   }
+  if (p.Dk == 64 && p.Dv == 64) return tc64_run_bwd(p, st);
   RowMaps maps;
   std::memset(&maps, 0, sizeof maps);
   const bool narrow = p.Dk != KD || p.Dv != KD;  // narrower heads exist only through the copy engine
