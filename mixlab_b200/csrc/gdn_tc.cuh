@@ -4,6 +4,8 @@
 
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "umma_tiles.cuh"
 
@@ -125,50 +127,54 @@ __device__ __forceinline__ void ld_acc64(uint32_t taddr, int warp, float (&f)[64
   }
 }
 // T = (I - A)^-1 in fp32, in place over the strictly lower triangular [64][LDA] matrix A; 128 threads, `other(t)` is run
-// by threads 64 + t beside the first step.  The two 32 x 32 diagonal blocks by forward substitution (thread = block and
-// column, the column in registers), then the off-diagonal block T21 = T22 (A21 T11) as two small products: 4 x 2 outputs
-// per thread, a warp's share cut so that it skips the zero triangle (one row of 8 outputs per thread over the full
-// contraction read 2.4 times as much shared memory, which is what bounds the prep kernels).  The upper-right block is
-// left with A21 T11, the rest of T is exact.  Ends without a barrier behind the last stores.
+// by threads 64 + t beside the first step.  The four 16 x 16 diagonal blocks by forward substitution (thread = block and
+// column, the column in registers), then pairs of blocks are joined twice, T21 = T22 (A21 T11): 16-wide for both halves
+// side by side, then 32-wide.  The products take 2 x 2 and 4 x 2 outputs per thread and skip the zero triangle: shared
+// memory is what bounds the prep kernels (two 32-step substitutions and one row of 8 outputs per thread took 4.1 k + 2.2 k
+// cycles of a CTA's 18 k).  The upper-right blocks are left with A21 T11, nobody reads them.  Ends with a barrier.
 template <typename F>
 __device__ __forceinline__ void invert_unit_lower(float* Am, bool ok, F other) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  float Tc[32];
-  const int r0 = 32 * (warp & 1);
-  if (ok && tid < C) {
+  {
+    float Tc[16];
+    const int r0 = 16 * (tid >> 4), col = tid & 15;
+    if (ok && tid < C) {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float* arow = Am + (r0 + i) * LDA + r0;
-      float s0 = (i == lane) ? 1.f : 0.f, s1 = 0.f;
+      for (int i = 0; i < 16; ++i) {
+        const float* arow = Am + (r0 + i) * LDA + r0;
+        float s0 = (i == col) ? 1.f : 0.f, s1 = 0.f;
 #pragma unroll
-      for (int j = 0; j + 1 < i; j += 2) {
-        s0 = fmaf(arow[j], Tc[j], s0);
-        s1 = fmaf(arow[j + 1], Tc[j + 1], s1);
+        for (int j = 0; j + 1 < i; j += 2) {
+          s0 = fmaf(arow[j], Tc[j], s0);
+          s1 = fmaf(arow[j + 1], Tc[j + 1], s1);
+        }
+        if (i & 1) s0 = fmaf(arow[i - 1], Tc[i - 1], s0);
+        Tc[i] = (i < col) ? 0.f : s0 + s1;
       }
-      if (i & 1) s0 = fmaf(arow[i - 1], Tc[i - 1], s0);
-      Tc[i] = (i < lane) ? 0.f : s0 + s1;
+    } else if (ok) {
+      other(tid - C);
     }
-  } else if (ok) {
-    other(tid - C);
-  }
-  __syncthreads();  // every thread has read its block of A
-  if (ok && tid < C) {
+    __syncthreads();  // every thread has read its block of A
+    if (ok && tid < C) {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) Am[(r0 + i) * LDA + r0 + lane] = Tc[i];
+      for (int i = 0; i < 16; ++i) Am[(r0 + i) * LDA + r0 + col] = Tc[i];
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  auto product = [&](const float* a, const float* b, int k0, int k1, int row0, int rstep, float* out) {
-    float x[4][2] = {};
+  // out[row0 + rstep r][0, 1] = sum over k in [k0, k1) of a[row0 + rstep r][k] b[k][0, 1]
+  auto product = [&](auto rows, const float* a, const float* b, int k0, int k1, int row0, int rstep, float* out) {
+    constexpr int R = decltype(rows)::value;
+    float x[R][2] = {};
 #pragma unroll 2
     for (int k = k0; k < k1; k += 4) {
-      float4 av[4];
+      float4 av[R];
       float2 bv[4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) av[r] = *reinterpret_cast<const float4*>(a + (row0 + rstep * r) * LDA + k);
+      for (int r = 0; r < R; ++r) av[r] = *reinterpret_cast<const float4*>(a + (row0 + rstep * r) * LDA + k);
 #pragma unroll
       for (int y = 0; y < 4; ++y) bv[y] = *reinterpret_cast<const float2*>(b + (k + y) * LDA);
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
+      for (int r = 0; r < R; ++r) {
         x[r][0] = fmaf(av[r].x, bv[0].x, x[r][0]); x[r][1] = fmaf(av[r].x, bv[0].y, x[r][1]);
         x[r][0] = fmaf(av[r].y, bv[1].x, x[r][0]); x[r][1] = fmaf(av[r].y, bv[1].y, x[r][1]);
         x[r][0] = fmaf(av[r].z, bv[2].x, x[r][0]); x[r][1] = fmaf(av[r].z, bv[2].y, x[r][1]);
@@ -176,16 +182,26 @@ __device__ __forceinline__ void invert_unit_lower(float* Am, bool ok, F other) {
       }
     }
 #pragma unroll
-    for (int r = 0; r < 4; ++r) *reinterpret_cast<float2*>(out + (row0 + rstep * r) * LDA) = make_float2(x[r][0], x[r][1]);
+    for (int r = 0; r < R; ++r) *reinterpret_cast<float2*>(out + (row0 + rstep * r) * LDA) = make_float2(x[r][0], x[r][1]);
   };
+  {  // the two 32 x 32 diagonal blocks: half a CTA each, rows g, g + 8, two columns
+    const std::integral_constant<int, 2> two;
+    float* M = Am + 32 * (tid >> 6) * (LDA + 1);
+    const int t = tid & 63, g = t >> 3, j = 2 * (t & 7);
+    product(two, M + 16 * LDA, M + j, 0, 16, g, 8, M + 16 + j);
+    __syncthreads();
+    product(two, M + 16 * LDA + 16, M + 16 + j, 0, 16, g, 8, M + 16 * LDA + j);
+    __syncthreads();
+  }
+  const std::integral_constant<int, 4> four;
   {  // X = A21 T11 -> the unused upper-right block; a warp takes eight columns, T11 is zero above its diagonal
     const int j = 8 * warp + 2 * (lane & 3);
-    product(Am + 32 * LDA, Am + j, 8 * warp, 32, lane >> 2, 8, Am + 32 + j);
+    product(four, Am + 32 * LDA, Am + j, 8 * warp, 32, lane >> 2, 8, Am + 32 + j);
   }
   __syncthreads();
   {  // T21 = T22 X -> over A21 (nothing reads A21 any more); a warp takes eight rows
     const int j = 2 * (lane & 15);
-    product(Am + 32 * LDA + 32, Am + 32 + j, 0, 8 * warp + 8, 8 * warp + (lane >> 4), 2, Am + 32 * LDA + j);
+    product(four, Am + 32 * LDA + 32, Am + 32 + j, 0, 8 * warp + 8, 8 * warp + (lane >> 4), 2, Am + 32 * LDA + j);
   }
   __syncthreads();
 }

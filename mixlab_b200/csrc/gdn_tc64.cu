@@ -43,18 +43,19 @@ __device__ __forceinline__ void scale_rows(uint8_t* tile, const float* s, int nt
 }
 
 // ------------------------------------------------------------------ prep
-// Four CTAs per SM (128 TMEM columns, 51 KB).  [k;q] (swizzled boxes) -> v takes the place of q -> u and w leave over
-// v and k; the fp32 matrix holds A, T and, once it is dead, the bf16 T image and T diag(beta).
-constexpr int kPrepSmem = 3 * kTile + C * LDA * 4 + 3 * C * 4 + 64 + 1024;
-static_assert(4 * (kPrepSmem + 1024) <= 228 * 1024, "four CTAs per SM");
+// A chain of dependent steps (prep kernel of gdn_tc.cu); six CTAs per SM overlap theirs (64 TMEM columns, 36 KB).  [k;q]
+// (swizzled boxes) -> the P^T image, then v, then u over q, w over k; the fp32 matrix holds A, T and, once it is dead, the
+// bf16 T image and T diag(beta).
+constexpr int kPrepSmem = 2 * kTile + C * LDA * 4 + 3 * C * 4 + 64 + 1024;
+static_assert(6 * (kPrepSmem + 1024) <= 228 * 1024, "six CTAs per SM");
 
-__global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+__global__ void __launch_bounds__(128, 6) gdn_tc_prep_kernel(TcP p, const __grid_constant__ RowMaps maps) {
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
   uint8_t* Xk = sm;             // k, then d k, then the w image
-  uint8_t* Xq = Xk + kTile;     // q, then v, then the u image
-  uint8_t* Xpt = Xq + kTile;    // P^T image
-  float* Am = reinterpret_cast<float*>(Xpt + kTile);  // [64][LDA]  A, then T in place
+  uint8_t* Xq = Xk + kTile;     // q, then the P^T image, then v, then the u image
+  uint8_t* Xpt = Xq;
+  float* Am = reinterpret_cast<float*>(Xq + kTile);  // [64][LDA]  A, then T in place
   uint8_t* Tt = reinterpret_cast<uint8_t*>(Am);       // T image
   uint8_t* Tb = Tt + kTile;                           // T diag(beta)
   float* gam = Am + C * LDA;
@@ -78,7 +79,7 @@ __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid
     tc::tma_load_4d(tc::smem_u32(Xq), &maps.q, 0, h, t0, b, &mbar[1]);
   }
   if (warp == 0) {
-    tc::tmem_alloc(tslot, 128);
+    tc::tmem_alloc(tslot, 64);
     tc::tmem_relinquish();
   }
   if (warp == 1) {  // in-chunk inclusive cumulative sum of the log gate: two elements per lane
@@ -110,10 +111,6 @@ __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid
   }
   if (ok) ok = tc::mbar_wait(mbar, 0);
   tc::fence_after_sync();
-  if (tid == 64) {  // q is dead: v takes its place (needed long after the solve)
-    tc::mbar_expect_tx(&mbar[2], kTile);
-    tc::tma_load_4d(tc::smem_u32(Xq), &maps.v, 0, h, t0, b, &mbar[2]);
-  }
   if (ok) {
     const int i = tid & 63;
     const float gi = gam[i], bi = bet[i];
@@ -153,9 +150,12 @@ __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  if (ok && tid == 96) {
+  if (ok && tid == 96) {  // P^T leaves, then v takes its place (needed long after the solve)
     tc::bulk_store(p.Pt + ci * C * C, tc::smem_u32(Xpt), kTile);
     tc::bulk_commit();
+    tc::bulk_wait_read<0>();
+    tc::mbar_expect_tx(&mbar[2], kTile);
+    tc::tma_load_4d(tc::smem_u32(Xq), &maps.v, 0, h, t0, b, &mbar[2]);
   }
   invert_unit_lower(Am, ok, [&](int t) {  // the other half of the CTA: k <- diag(d) k
     uint4* unit = reinterpret_cast<uint4*>(Xk);
@@ -176,46 +176,45 @@ __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  // [w | u] = (T beta) [d k | v]: one product of 128 columns
-  if (ok && tid == 0) {
-    tc::issue_gemm(taddr, tc::kmajor_tile(Tb, C), tc::mnmajor_sw128_tile(Xk, kTile), 64, 128, C, false);
-    tc::mma_commit(mbar);
-    if (p.save) {
-      tc::bulk_store(p.Tm + ci * C * C, tc::smem_u32(Tt), kTile);
+  // w = (T beta)(d k), then u = (T beta) v through the same accumulator columns
+  const int ir = 16 * warp + (lane & 15);  // M=64: row m sits in TMEM lane (m%16) + 32*(m/16)
+  for (int which = 0; which < 2; ++which) {
+    uint8_t* X = which ? Xq : Xk;
+    if (ok && tid == 0) {
+      tc::issue_gemm(taddr, tc::kmajor_tile(Tb, C), tc::mnmajor_sw128_tile(X, kTile), 64, W, C, false);
+      tc::mma_commit(mbar);
+      if (which) tc::bulk_store(p.w + ci * C * W, tc::smem_u32(Xk), kTile);
+      else if (p.save) tc::bulk_store(p.Tm + ci * C * C, tc::smem_u32(Tt), kTile);
       tc::bulk_commit();
     }
-  }
-  if (ok) ok = tc::mbar_wait(mbar, 1);
-  tc::fence_after_sync();
-  if (ok) {  // M=64: row m sits in TMEM lane (m%16) + 32*(m/16)
-    const int ir = 16 * warp + (lane & 15);
-    for (int c0 = 0; c0 < 128; c0 += 32) {
-      float f[32];
-      ld_acc32(taddr, warp, c0, f);
-      if (lane < 16) {
+    if (ok) ok = tc::mbar_wait(mbar, 1 ^ which);
+    tc::fence_after_sync();
+    if (ok) {
+      for (int c0 = 0; c0 < 64; c0 += 32) {
+        float f[32];
+        ld_acc32(taddr, warp, c0, f);
+        if (lane < 16) {
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          const int c8 = ((c0 & 63) >> 3) + x;
-          if (c0 < 64) sts16(Xk, sw_unit(ir, c8), pack8(&f[8 * x]));              // w, swizzled
-          else sts16(Xq, tc::kmajor_unit(ir, c8, W), pack8(&f[8 * x]));           // u, un-swizzled
+          for (int x = 0; x < 4; ++x)  // the w image is swizzled, the u image is not
+            sts16(X, which ? tc::kmajor_unit(ir, (c0 >> 3) + x, W) : sw_unit(ir, (c0 >> 3) + x), pack8(&f[8 * x]));
         }
       }
     }
-  } else if (tid == 0) {
-    atomicExch(p.status, 1);
+    tc::fence_async_smem();
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
   }
-  tc::fence_async_smem();
-  tc::fence_before_sync();
-  __syncthreads();
-  if (tid == 0 && ok) {
-    tc::bulk_store(p.w + ci * C * W, tc::smem_u32(Xk), kTile);
-    tc::bulk_store(p.u + ci * C * W, tc::smem_u32(Xq), kTile);
-    tc::bulk_commit();
+  if (!ok && tid == 0) atomicExch(p.status, 1);
+  if (tid == 0) {
+    if (ok) {
+      tc::bulk_store(p.u + ci * C * W, tc::smem_u32(Xq), kTile);
+      tc::bulk_commit();
+    }
+    tc::bulk_wait_read<0>();  // shared memory must outlive the copies
   }
-  if (tid == 0 || tid == 96) tc::bulk_wait_read<0>();  // shared memory must outlive the copies
-  tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(taddr, 128);
+  if (warp == 0) tc::tmem_dealloc(taddr, 64);
 }
 
 // ------------------------------------------------------------ state forward
