@@ -305,27 +305,36 @@ __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid
 // barrier of their group, like the images: no thread spends issue slots on copies (four cp.async per thread and
 // group cost every thread ~1.6 k and ~1.1 k cycles per chunk, on the critical path between an MMA and its epilogue).
 // TMA = false: the same rows by cp.async into the same swizzled positions.
-constexpr int kStateFwdSmem = 2 * 32768 + 32768 + 2 * 16384 + 16384 + 16384 + 2 * 16384 + 2 * 16384 + 2 * C * 4 + 128 + 1024;
+//
+// NV: columns of the state per CTA.  128 (all of them) where the (batch, head) pairs fill the GPU; 64 otherwise: a
+// chunk's chain of products and epilogues is then half as wide (columns of the state are independent; w, q, k and P are
+// read by both CTAs, the second time from L2).
+template <int NV>
+constexpr int kStateFwdSmem = 2 * 32768 + 256 * NV + 2 * 16384 + 128 * NV + 128 * NV + 2 * 16384 + 2 * 128 * NV + 2 * C * 4 + 128 + 1024;
 
-template <bool TMA>
+template <bool TMA, int NV>
 __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+  static_assert(NV == KD || TMA, "the per-thread staging moves whole rows");
+  constexpr int NC = NV / 2;                   // columns per thread
+  constexpr int NST = NV == KD ? 1 : 16;       // pieces of a state image in the workspace (rows of eight, NV columns)
+  const int col0 = blockIdx.y * NV;
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
   uint8_t* A1 = sm;                 // x2 [128: w rows 0-63, q rows 64-127][128 kk], two swizzled slabs of 64 columns
-  uint8_t* Sop = A1 + 2 * 32768;    // [128 kk][128 j]   bf16 copy of the state
-  uint8_t* A2 = Sop + 32768;        // x2 [128: zero rows 0-63, P rows 64-127][64 m]
-  uint8_t* Vn = A2 + 2 * 16384;     // [64 i][128 j]     v_new
-  uint8_t* Ot = Vn + 16384;         // [64 i][128 j]     output tile on its way out (two swizzled slabs)
-  uint8_t* A3 = Ot + 16384;         // x2 [64 i][128 kk] k, then diag(E(gam_last-gam_i)) k  (A = k^T), swizzled slabs
-  uint8_t* Ut = A3 + 2 * 16384;     // x2 [64 i][128 j]  u
-  float* dd = reinterpret_cast<float*>(Ut + 2 * 16384);
+  uint8_t* Sop = A1 + 2 * 32768;    // [128 kk][NV j]    bf16 copy of the state
+  uint8_t* A2 = Sop + 256 * NV;       // x2 [128: zero rows 0-63, P rows 64-127][64 m]
+  uint8_t* Vn = A2 + 2 * 16384;     // [64 i][NV j]      v_new
+  uint8_t* Ot = Vn + 128 * NV;      // [64 i][NV j]      output tile on its way out (swizzled slabs of 64 columns)
+  uint8_t* A3 = Ot + 128 * NV;       // x2 [64 i][128 kk] k, then diag(E(gam_last-gam_i)) k  (A = k^T), swizzled slabs
+  uint8_t* Ut = A3 + 2 * 16384;     // x2 [64 i][NV j]   u
+  float* dd = reinterpret_cast<float*>(Ut + 2 * 128 * NV);
   float* rr = dd + C;
   // [0] MMA completion; per buffer: [1 + buf] w image and q rows, [3 + buf] u image, [5 + buf] P image and k rows landed
   uint64_t* mbar = reinterpret_cast<uint64_t*>(rr + C);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int kk = tid & 127, half = tid >> 7, j0 = 64 * half;
+  const int kk = tid & 127, half = tid >> 7, j0 = NC * half;
   const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
   const uint32_t sA1b = tc::smem_u32(A1), sA2b = tc::smem_u32(A2), sA3b = tc::smem_u32(A3), sUb = tc::smem_u32(Ut);
   const uint32_t sOt = tc::smem_u32(Ot);
@@ -362,8 +371,10 @@ __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __gr
   auto issue_U = [&](int c) {
     if (c < p.n && tid == 64) {
       const size_t ci = (size_t)bh * p.n + c;
-      tc::mbar_expect_tx(&mbar[3 + (c & 1)], 16384);
-      tc::bulk_load(sUb + (c & 1) * 16384, p.u + ci * C * KD, 16384, &mbar[3 + (c & 1)]);
+      tc::mbar_expect_tx(&mbar[3 + (c & 1)], 128 * NV);
+      for (int g = 0; g < (NST + 1) / 2; ++g)  // this CTA's columns of each group of eight rows
+        tc::bulk_load(sUb + (c & 1) * 128 * NV + g * 16 * NV, p.u + ci * C * KD + g * 8 * KD + 8 * col0, 256 * NV / (NST + (NST & 1)),
+                      &mbar[3 + (c & 1)]);
     }
     if (!TMA) tc::cp_async_commit();  // (empty: keeps the group count of the schedule below)
   };
@@ -403,17 +414,17 @@ __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __gr
     issue_U(c);
     issue_PK(c);
   }
-  float S[64];  // state row kk, columns j0 .. j0+63 (zero outside the true Dk x Dv state)
+  float S[NC];  // state row kk, columns col0 + j0 .. (zero outside the true Dk x Dv state)
   if (p.h0) {
-    const float4* src = reinterpret_cast<const float4*>(p.h0 + ((size_t)bh * p.Dk + kk) * p.Dv + j0);
+    const float4* src = reinterpret_cast<const float4*>(p.h0 + ((size_t)bh * p.Dk + kk) * p.Dv + col0 + j0);
 #pragma unroll
-    for (int x = 0; x < 16; ++x) {
-      const float4 t4 = (kk < p.Dk && j0 + 4 * x < p.Dv) ? __ldg(src + x) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int x = 0; x < NC / 4; ++x) {
+      const float4 t4 = (kk < p.Dk && col0 + j0 + 4 * x < p.Dv) ? __ldg(src + x) : make_float4(0.f, 0.f, 0.f, 0.f);
       S[4 * x] = t4.x; S[4 * x + 1] = t4.y; S[4 * x + 2] = t4.z; S[4 * x + 3] = t4.w;
     }
   } else {
 #pragma unroll
-    for (int x = 0; x < 64; ++x) S[x] = 0.f;
+    for (int x = 0; x < NC; ++x) S[x] = 0.f;
   }
   for (int u = tid; u < 2 * 64 * 8; u += 256)  // the zero rows of both [0;P] tiles
     sts16(A2 + (u >> 9) * 16384, tc::kmajor_unit((u >> 3) & 63, u & 7, C), zero16());
@@ -435,7 +446,7 @@ __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __gr
     uint8_t* A1c = A1 + buf * 32768;
     uint8_t* A2c = A2 + buf * 16384;
     uint8_t* A3c = A3 + buf * 16384;
-    uint8_t* Utc = Ut + buf * 16384;
+    uint8_t* Utc = Ut + buf * 128 * NV;
     const float glast = gl_nxt, g = g_nxt;
     if (c + 1 < p.n) {
       g_nxt = p.gam[(ci + 1) * C + (tid & 63)];
@@ -447,12 +458,12 @@ __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __gr
       rr[tid] = exp_nonpos(glast - g);
     }
 #pragma unroll
-    for (int c8 = 0; c8 < 8; ++c8) {  // state as the MMA operand (and saved for the backward)
+    for (int c8 = 0; c8 < NC / 8; ++c8) {  // state as the MMA operand (and saved for the backward)
       const uint4 val = make_uint4(tc::pack_bf16(S[8 * c8], S[8 * c8 + 1]), tc::pack_bf16(S[8 * c8 + 2], S[8 * c8 + 3]),
                                    tc::pack_bf16(S[8 * c8 + 4], S[8 * c8 + 5]), tc::pack_bf16(S[8 * c8 + 6], S[8 * c8 + 7]));
-      sts16(Sop, tc::mnmajor_unit(kk, 8 * half + c8, KD), val);
+      sts16(Sop, tc::mnmajor_unit(kk, NC / 8 * half + c8, NV), val);
     }
-    if (tid == 0) tc::bulk_wait_read<0>();  // the previous chunk's v_new image has left its tile
+    if (tid < NST) tc::bulk_wait_read<0>();  // the previous chunk's v_new image has left its tile
     if (!TMA) tc::cp_async_wait<5>();  // group A of this chunk has landed (q rows; the images on the barrier)
     if (ok) ok = tc::mbar_wait(&mbar[1 + buf], lph);
     tc::fence_async_smem();
@@ -461,16 +472,16 @@ __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __gr
     if (!ok) break;              // threads leave the loop together
     tc::fence_after_sync();
     if (tid == 0) {  // D1 = [w;q] S
-      tc::issue_gemm(taddr, tc::kmajor_sw128_tile(A1c, 16384), tc::mnmajor_tile(Sop, KD), 128, KD, KD, false);
+      tc::issue_gemm(taddr, tc::kmajor_sw128_tile(A1c, 16384), tc::mnmajor_tile(Sop, NV), 128, NV, KD, false);
       tc::mma_commit(mbar);
-      if (p.save) {  // the state at chunk start, saved for the backward as the byte image of the operand tile
-        tc::bulk_store(p.hs + ci * KD * KD, tc::smem_u32(Sop), 32768);
-        tc::bulk_commit();
-      }
+    }
+    if (p.save && tid < NST) {  // the state at chunk start, saved for the backward as the byte image of the operand tile
+      tc::bulk_store(p.hs + ci * KD * KD + tid * 8 * KD + 8 * col0, tc::smem_u32(Sop) + tid * 16 * NV, 256 * NV / NST);
+      tc::bulk_commit();
     }
     if (TMA && tid == kOutThread && c > 0) {  // the previous chunk's output tile (complete since the barrier above)
-      for (int sl = 0; sl < 2; ++sl)  // a slab that lies wholly past the true width is not stored at all
-        if (64 * sl < p.Dv) tc::tma_store_4d(&maps.o, sOt + sl * 8192, 64 * sl, h, t0 - C, b);
+      for (int sl = 0; sl < NV / 64; ++sl)  // a slab that lies wholly past the true width is not stored at all
+        if (col0 + 64 * sl < p.Dv) tc::tma_store_4d(&maps.o, sOt + sl * 8192, col0 + 64 * sl, h, t0 - C, b);
       tc::bulk_commit();
     }
     // In the shadow of the MMA: k <- diag(r) k in place, so that the state update contracts it with v_new itself
@@ -488,30 +499,30 @@ __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __gr
     tc::fence_after_sync();
     issue_A(c + 2);
     if (ok) ok = tc::mbar_wait(&mbar[3 + buf], lph);  // u image of this chunk
-    float f[64];  // accumulator row; rows 64-127 keep E(gam_i) (q S) here until P v_new arrives
+    float f[NC];  // accumulator row; rows 64-127 keep E(gam_i) (q S) here until P v_new arrives
     if (ok) {
       const int i = kk & 63;
-      ld_acc64(taddr + j0, warp, f);
+      ld_accN(taddr + j0, warp, f);
       if (kk < 64) {  // v_new = u - w S
 #pragma unroll
-        for (int x = 0; x < 8; ++x) {
-          const int c8 = 8 * half + x;
-          const uint4 uu = *reinterpret_cast<const uint4*>(Utc + tc::kmajor_unit(i, c8, KD));
+        for (int x = 0; x < NC / 8; ++x) {
+          const int c8 = NC / 8 * half + x;
+          const uint4 uu = *reinterpret_cast<const uint4*>(Utc + tc::kmajor_unit(i, c8, NV));
           float e[8];
           tc::unpack_bf16(uu.x, e[0], e[1]); tc::unpack_bf16(uu.y, e[2], e[3]);
           tc::unpack_bf16(uu.z, e[4], e[5]); tc::unpack_bf16(uu.w, e[6], e[7]);
 #pragma unroll
           for (int y = 0; y < 8; ++y) e[y] -= f[8 * x + y];
-          sts16(Vn, tc::mnmajor_unit(i, c8, KD), make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]),
+          sts16(Vn, tc::mnmajor_unit(i, c8, NV), make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]),
                                                             tc::pack_bf16(e[4], e[5]), tc::pack_bf16(e[6], e[7])));
         }
       } else {
         const float di = dd[i];
 #pragma unroll
-        for (int jj = 0; jj < 64; ++jj) f[jj] *= di;
+        for (int jj = 0; jj < NC; ++jj) f[jj] *= di;
       }
     }
-    if (tid == 0) tc::bulk_wait_read<0>();  // the state image has left its tile
+    if (tid < NST) tc::bulk_wait_read<0>();  // the state image has left its tile
     if (TMA && tid == kOutThread) tc::bulk_wait_read<0>();  // the previous output tile has left its tile
     tc::fence_async_smem();
     tc::fence_before_sync();
@@ -520,13 +531,13 @@ __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __gr
     issue_U(c + 2);  // u has been consumed by every thread
     if (ok && tid == 0) {
       // D2 = [0;P] v_new          D3 = (r k)^T v_new
-      tc::issue_gemm(taddr + 128, tc::kmajor_tile(A2c, C), tc::mnmajor_tile(Vn, KD), 128, KD, C, false);
-      tc::issue_gemm(taddr + 256, tc::mnmajor_sw128_tile(A3c, 8192), tc::mnmajor_tile(Vn, KD), 128, KD, C, false);
+      tc::issue_gemm(taddr + 128, tc::kmajor_tile(A2c, C), tc::mnmajor_tile(Vn, NV), 128, NV, C, false);
+      tc::issue_gemm(taddr + 256, tc::mnmajor_sw128_tile(A3c, 8192), tc::mnmajor_tile(Vn, NV), 128, NV, C, false);
       tc::mma_commit(mbar);
-      if (p.save) {
-        tc::bulk_store(p.vn + ci * C * KD, tc::smem_u32(Vn), 16384);
-        tc::bulk_commit();
-      }
+    }
+    if (ok && p.save && tid < (NST + 1) / 2) {
+      tc::bulk_store(p.vn + ci * C * KD + tid * 8 * KD + 8 * col0, tc::smem_u32(Vn) + tid * 16 * NV, 256 * NV / (NST + (NST & 1)));
+      tc::bulk_commit();
     }
     if (ok) {
       ok = tc::mbar_wait(mbar, ph);
@@ -536,13 +547,13 @@ __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __gr
     issue_PK(c + 2);
     if (ok) {
       const int i = kk & 63;
-      float a[64];
+      float a[NC];
       if (kk >= 64) {  // out = E(gam)(q S) + P v_new      (warp-uniform branch)
-        ld_acc64(taddr + 128 + j0, warp, a);
+        ld_accN(taddr + 128 + j0, warp, a);
         if (TMA) {     // into the swizzled output tile; one thread hands it to the copy engine after the next barrier
 #pragma unroll
-          for (int x = 0; x < 8; ++x)
-            sts16(Ot, tc::sw128_unit(i, 8 * half + x),
+          for (int x = 0; x < NC / 8; ++x)
+            sts16(Ot, tc::sw128_unit(i, NC / 8 * half + x),
                   make_uint4(tc::pack_bf16(f[8 * x] + a[8 * x], f[8 * x + 1] + a[8 * x + 1]),
                              tc::pack_bf16(f[8 * x + 2] + a[8 * x + 2], f[8 * x + 3] + a[8 * x + 3]),
                              tc::pack_bf16(f[8 * x + 4] + a[8 * x + 4], f[8 * x + 5] + a[8 * x + 5]),
@@ -550,16 +561,16 @@ __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __gr
         } else if (i < imax) {
           uint4* dst = reinterpret_cast<uint4*>(p.out + grow(c, i) * KD + j0);
 #pragma unroll
-          for (int x = 0; x < 8; ++x)
+          for (int x = 0; x < NC / 8; ++x)
             dst[x] = make_uint4(tc::pack_bf16(f[8 * x] + a[8 * x], f[8 * x + 1] + a[8 * x + 1]),
                                 tc::pack_bf16(f[8 * x + 2] + a[8 * x + 2], f[8 * x + 3] + a[8 * x + 3]),
                                 tc::pack_bf16(f[8 * x + 4] + a[8 * x + 4], f[8 * x + 5] + a[8 * x + 5]),
                                 tc::pack_bf16(f[8 * x + 6] + a[8 * x + 6], f[8 * x + 7] + a[8 * x + 7]));
         }
       }
-      ld_acc64(taddr + 256 + j0, warp, a);  // S <- E(gam_last) S + (r k)^T v_new
+      ld_accN(taddr + 256 + j0, warp, a);  // S <- E(gam_last) S + (r k)^T v_new
 #pragma unroll
-      for (int jj = 0; jj < 64; ++jj) S[jj] = fmaf(L, S[jj], a[jj]);
+      for (int jj = 0; jj < NC; ++jj) S[jj] = fmaf(L, S[jj], a[jj]);
     }
     tc::fence_before_sync();
   }
@@ -568,19 +579,19 @@ __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __gr
     tc::fence_async_smem();
     __syncthreads();
     if (ok && tid == kOutThread) {
-      for (int sl = 0; sl < 2; ++sl)
-        if (64 * sl < p.Dv) tc::tma_store_4d(&maps.o, sOt + sl * 8192, 64 * sl, h, (p.n - 1) * C, b);
+      for (int sl = 0; sl < NV / 64; ++sl)
+        if (col0 + 64 * sl < p.Dv) tc::tma_store_4d(&maps.o, sOt + sl * 8192, col0 + 64 * sl, h, (p.n - 1) * C, b);
       tc::bulk_commit();
     }
     if (tid == kOutThread) tc::bulk_wait_read<0>();
   }
-  if (tid == 0) tc::bulk_wait_read<0>();  // shared memory must outlive the copies
+  if (tid < NST) tc::bulk_wait_read<0>();  // shared memory must outlive the copies
   if (!ok && tid == 0) atomicExch(p.status, 2);
   if (ok && p.hT && kk < p.Dk) {
-    float4* dst = reinterpret_cast<float4*>(p.hT + ((size_t)bh * p.Dk + kk) * p.Dv + j0);
+    float4* dst = reinterpret_cast<float4*>(p.hT + ((size_t)bh * p.Dk + kk) * p.Dv + col0 + j0);
 #pragma unroll
-    for (int x = 0; x < 16; ++x)
-      if (j0 + 4 * x < p.Dv) dst[x] = make_float4(S[4 * x], S[4 * x + 1], S[4 * x + 2], S[4 * x + 3]);
+    for (int x = 0; x < NC / 4; ++x)
+      if (col0 + j0 + 4 * x < p.Dv) dst[x] = make_float4(S[4 * x], S[4 * x + 1], S[4 * x + 2], S[4 * x + 3]);
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -703,15 +714,18 @@ mxb_status tc_run_fwd(TcP& p, cudaStream_t st) {
   }
   mxb_status s = check_launch("gdn_tc_prep_kernel");
   if (s != MXB_OK) return s;
-  if (tma) {
-    if (MXB_ALLOW_SMEM(kStateFwdSmem, gdn_tc_state_fwd_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
+  auto state = [&](auto tma_v, auto nv) {
+    constexpr bool TMA = decltype(tma_v)::value;
+    constexpr int NV = decltype(nv)::value;
+    if (MXB_ALLOW_SMEM(kStateFwdSmem<NV>, gdn_tc_state_fwd_kernel<TMA, NV>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_state_fwd_kernel", st,
-               (gdn_tc_state_fwd_kernel<true><<<dim3(p.B * p.H), 256, kStateFwdSmem, st>>>(p, maps)));
-  } else {
-    if (MXB_ALLOW_SMEM(kStateFwdSmem, gdn_tc_state_fwd_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
-    MXB_LAUNCH("gdn_tc_state_fwd_kernel", st,
-               (gdn_tc_state_fwd_kernel<false><<<dim3(p.B * p.H), 256, kStateFwdSmem, st>>>(p, maps)));
-  }
+               (gdn_tc_state_fwd_kernel<TMA, NV><<<dim3(p.B * p.H, (p.Dv + NV - 1) / NV), 256, kStateFwdSmem<NV>, st>>>(p, maps)));
+    return MXB_OK;
+  };
+  if (!tma) s = state(std::false_type{}, std::integral_constant<int, KD>{});
+  else if (tc_split_columns(p)) s = state(std::true_type{}, std::integral_constant<int, 64>{});
+  else s = state(std::true_type{}, std::integral_constant<int, KD>{});
+  if (s != MXB_OK) return s;
   return check_launch("gdn_tc_state_fwd_kernel");
 }
 

@@ -113,6 +113,11 @@ __device__ __forceinline__ void for_acc2x32(uint32_t taddr, int warp, int c0, F&
   for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(r1[i]);
   process(c0 + 32, f);
 }
+// The sequential passes of 128-wide heads take half of the state's columns per CTA where that still puts every CTA on an
+// SM of its own: the chain of a chunk is what counts then, not the bytes (16 heads, 24 chunks: 65 -> 56 us
+// forward).
+inline bool tc_split_columns(const TcP& p) { return p.Dv > 64 && 2 * p.B * p.H <= 148; }
+
 // Loads 64 fp32 accumulator columns [0, 64) at taddr of this thread's TMEM lane: both loads in flight, one wait.
 __device__ __forceinline__ void ld_acc64(uint32_t taddr, int warp, float (&f)[64]) {
   uint32_t r0[32], r1[32];
@@ -126,6 +131,8 @@ __device__ __forceinline__ void ld_acc64(uint32_t taddr, int warp, float (&f)[64
     f[32 + i] = __uint_as_float(r1[i]);
   }
 }
+__device__ __forceinline__ void ld_accN(uint32_t taddr, int warp, float (&f)[64]) { ld_acc64(taddr, warp, f); }
+__device__ __forceinline__ void ld_accN(uint32_t taddr, int warp, float (&f)[32]) { ld_acc32(taddr, warp, 0, f); }
 // T = (I - A)^-1 in fp32, in place over the strictly lower triangular [64][LDA] matrix A; 128 threads, `other(t)` is run
 // by threads 64 + t beside the first step.  The four 16 x 16 diagonal blocks by forward substitution (thread = block and
 // column, the column in registers), then pairs of blocks are joined twice, T21 = T22 (A21 T11): 16-wide for both halves

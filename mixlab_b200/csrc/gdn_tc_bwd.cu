@@ -37,28 +37,34 @@ namespace mxb {
 // TMA = true: the k, dO and q rows arrive as tensor-map boxes (128-byte swizzle, two 8 KB slabs of 64 columns per
 // tile) issued by one thread on the barrier of group A; TMA = false: by cp.async into the same swizzled positions
 // (twelve copies per thread and chunk).  The w image is stored in the same swizzled layout by the prep kernel.
+// NV: columns of dS per CTA, as in the forward pass.
+template <int NV>
 constexpr int kStateBwdSmem =
-    2 * 16384 + 32768 + 2 * 8192 + 2 * 16384 + 2 * 16384 + 2 * 16384 + 16384 + 3 * C * 4 + 128 + 1024;
+    2 * 16384 + 256 * NV + 2 * 8192 + 2 * 128 * NV + 2 * 16384 + 2 * 16384 + 128 * NV + 3 * C * 4 + 128 + 1024;
 
-template <bool TMA>
+template <bool TMA, int NV>
 __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+  static_assert(NV == KD || TMA, "the per-thread staging moves whole rows");
+  constexpr int NC = NV / 2;                   // columns per thread
+  constexpr int NST = NV == KD ? 1 : 16;       // pieces of a state image in the workspace (rows of eight, NV columns)
+  const int col0 = blockIdx.y * NV;
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
   uint8_t* Ak = sm;                  // x2 [64 i][128 kk]   k  (swizzled slabs)
-  uint8_t* dSop = Ak + 2 * 16384;    // [128 kk][128 j]     bf16 copy of dS
-  uint8_t* Pt = dSop + 32768;        // x2 [64 m][64 i]     P   (A = P^T: contraction over rows)
-  uint8_t* dOop = Pt + 2 * 8192;     // x2 [64 m][128 j]    dO (swizzled slabs)
-  uint8_t* Aq = dOop + 2 * 16384;    // x2 [64 i][128 kk]   q, then diag(E(gam)) q (swizzled slabs)   (A = q^T)
+  uint8_t* dSop = Ak + 2 * 16384;    // [128 kk][NV j]      bf16 copy of dS
+  uint8_t* Pt = dSop + 256 * NV;        // x2 [64 m][64 i]     P   (A = P^T: contraction over rows)
+  uint8_t* dOop = Pt + 2 * 8192;     // x2 [64 m][NV j]     dO (swizzled slabs)
+  uint8_t* Aq = dOop + 2 * 128 * NV;    // x2 [64 i][128 kk]   q, then diag(E(gam)) q (swizzled slabs)   (A = q^T)
   uint8_t* Aw = Aq + 2 * 16384;      // x2 [64 i][128 kk]   w image (swizzled slabs)                  (A = w^T)
-  uint8_t* Bd = Aw + 2 * 16384;      // [64 i][128 j]       -dv_new
-  float* rr = reinterpret_cast<float*>(Bd + 16384);
+  uint8_t* Bd = Aw + 2 * 16384;      // [64 i][NV j]        -dv_new
+  float* rr = reinterpret_cast<float*>(Bd + 128 * NV);
   float* ddn = rr + C;               // x2 E(gam) of the chunk whose q is scaled next (buffer = chunk & 1)
   // [0] MMA completion; per buffer: [1 + buf] group A landed, [3 + buf] w image landed
   uint64_t* mbar = reinterpret_cast<uint64_t*>(ddn + 2 * C);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int kk = tid & 127, half = tid >> 7, j0 = 64 * half;
+  const int kk = tid & 127, half = tid >> 7, j0 = NC * half;
   const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
   const uint32_t sAk = tc::smem_u32(Ak), sPt = tc::smem_u32(Pt), sdO = tc::smem_u32(dOop), sAq = tc::smem_u32(Aq);
   const uint32_t sAw = tc::smem_u32(Aw);
@@ -82,12 +88,12 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
       }
       if (tid == 32) {  // P is a byte image of its operand tile: one bulk copy, completing on the group's barrier
         uint64_t* mb = &mbar[1 + (c & 1)];
-        tc::mbar_expect_tx(mb, TMA ? 8192 + 3 * 16384 : 8192);
+        tc::mbar_expect_tx(mb, TMA ? 8192 + 2 * 16384 + 128 * NV : 8192);
         tc::bulk_load(sPt + (c & 1) * 8192, p.P + ci * C * C, 8192, mb);
         if (TMA) {
           for (int sl = 0; sl < 2; ++sl) {
             tc::tma_load_4d(sAk + o16 + sl * 8192, &maps.k, 64 * sl, h, c * C, b, mb);
-            tc::tma_load_4d(sdO + o16 + sl * 8192, &maps.dO, 64 * sl, h, c * C, b, mb);
+            if (sl < NV / 64) tc::tma_load_4d(sdO + (c & 1) * 128 * NV + sl * 8192, &maps.dO, col0 + 64 * sl, h, c * C, b, mb);
             tc::tma_load_4d(sAq + o16 + sl * 8192, &maps.q, 64 * sl, h, c * C, b, mb);
           }
         }
@@ -126,17 +132,17 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
     issue_A(c);
     issue_B(c);
   }
-  float dS[64];  // row kk of dS, columns j0 .. j0+63
+  float dS[NC];  // row kk of dS, columns col0 + j0 ..
   if (p.dhT_in) {
-    const float4* src = reinterpret_cast<const float4*>(p.dhT_in + ((size_t)bh * p.Dk + kk) * p.Dv + j0);
+    const float4* src = reinterpret_cast<const float4*>(p.dhT_in + ((size_t)bh * p.Dk + kk) * p.Dv + col0 + j0);
 #pragma unroll
-    for (int x = 0; x < 16; ++x) {
-      const float4 t4 = (kk < p.Dk && j0 + 4 * x < p.Dv) ? __ldg(src + x) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int x = 0; x < NC / 4; ++x) {
+      const float4 t4 = (kk < p.Dk && col0 + j0 + 4 * x < p.Dv) ? __ldg(src + x) : make_float4(0.f, 0.f, 0.f, 0.f);
       dS[4 * x] = t4.x; dS[4 * x + 1] = t4.y; dS[4 * x + 2] = t4.z; dS[4 * x + 3] = t4.w;
     }
   } else {
 #pragma unroll
-    for (int x = 0; x < 64; ++x) dS[x] = 0.f;
+    for (int x = 0; x < NC; ++x) dS[x] = 0.f;
   }
   // in-chunk cumulative log decay: this chunk's, and the next (earlier) one's fetched a chunk early
   const size_t gbase = (size_t)bh * p.n * C;
@@ -176,12 +182,12 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
       if (c > 0) ddn[(buf ^ 1) * C + tid] = exp_nonpos(g_cur);  // for the next chunk's q
     }
 #pragma unroll
-    for (int c8 = 0; c8 < 8; ++c8) {  // dS at chunk end: MMA operand + saved for the chunk kernel
+    for (int c8 = 0; c8 < NC / 8; ++c8) {  // dS at chunk end: MMA operand + saved for the chunk kernel
       const uint4 val = make_uint4(tc::pack_bf16(dS[8 * c8], dS[8 * c8 + 1]), tc::pack_bf16(dS[8 * c8 + 2], dS[8 * c8 + 3]),
                                    tc::pack_bf16(dS[8 * c8 + 4], dS[8 * c8 + 5]), tc::pack_bf16(dS[8 * c8 + 6], dS[8 * c8 + 7]));
-      sts16(dSop, tc::mnmajor_unit(kk, 8 * half + c8, KD), val);
+      sts16(dSop, tc::mnmajor_unit(kk, NC / 8 * half + c8, NV), val);
     }
-    if (tid == 0) tc::bulk_wait_read<0>();  // the previous chunk's -dv_new image has left its tile
+    if (tid < NST) tc::bulk_wait_read<0>();  // the previous chunk's -dv_new image has left its tile
     // group A of this chunk was waited for when its q was scaled (previous iteration / prologue)
     tc::fence_async_smem();
     tc::fence_before_sync();
@@ -189,13 +195,15 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
     if (!ok) break;              // threads leave the loop together
     tc::fence_after_sync();
     if (tid == 0) {
-      tc::issue_gemm(taddr, tc::kmajor_sw128_tile(Ak + buf * 16384, 8192), tc::mnmajor_tile(dSop, KD), 64, KD, KD, false);  // k dS
-      tc::issue_gemm(taddr + 128, tc::mnmajor_tile(Pt + buf * 8192, C), tc::mnmajor_sw128_tile(dOop + buf * 16384, 8192), 64, KD,
+      tc::issue_gemm(taddr, tc::kmajor_sw128_tile(Ak + buf * 16384, 8192), tc::mnmajor_tile(dSop, NV), 64, NV, KD, false);  // k dS
+      tc::issue_gemm(taddr + 128, tc::mnmajor_tile(Pt + buf * 8192, C), tc::mnmajor_sw128_tile(dOop + buf * 128 * NV, 8192), 64, NV,
                      C, false);                                                                                           // P^T dO
-      tc::issue_gemm(taddr + 256, tc::mnmajor_sw128_tile(Aq + buf * 16384, 8192), tc::mnmajor_sw128_tile(dOop + buf * 16384, 8192),
-                     128, KD, C, false);                                                                                  // (d q)^T dO
+      tc::issue_gemm(taddr + 256, tc::mnmajor_sw128_tile(Aq + buf * 16384, 8192), tc::mnmajor_sw128_tile(dOop + buf * 128 * NV, 8192),
+                     128, NV, C, false);                                                                                  // (d q)^T dO
       tc::mma_commit(mbar);
-      tc::bulk_store(p.dhs + ci * KD * KD, tc::smem_u32(dSop), 32768);  // dS at chunk end, as the operand-tile image
+    }
+    if (tid < NST) {  // dS at chunk end, as the operand-tile image
+      tc::bulk_store(p.dhs + ci * KD * KD + tid * 8 * KD + 8 * col0, tc::smem_u32(dSop) + tid * 16 * NV, 256 * NV / NST);
       tc::bulk_commit();
     }
     if (ok) ok = tc::mbar_wait(mbar, ph);
@@ -205,7 +213,7 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
     if (ok) {
       const int i = 16 * (warp & 3) + (lane & 15);  // M=64 accumulators: row i in TMEM lane (i%16) + 32*(i/16)
       const float ri = rr[i];
-      for (int c0 = 0; c0 < 64; c0 += 32) {
+      for (int c0 = 0; c0 < NC; c0 += 32) {
         float fa[32], fb[32];
         ld_acc32(taddr + j0, warp, c0, fa);
         ld_acc32(taddr + 128 + j0, warp, c0, fb);
@@ -215,23 +223,25 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
             float e[8];
 #pragma unroll
             for (int y = 0; y < 8; ++y) e[y] = -fmaf(ri, fa[8 * x + y], fb[8 * x + y]);
-            const int c8 = 8 * half + (c0 >> 3) + x;
-            sts16(Bd, tc::kmajor_unit(i, c8, KD), make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]),
+            const int c8 = NC / 8 * half + (c0 >> 3) + x;
+            sts16(Bd, tc::kmajor_unit(i, c8, NV), make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]),
                                                              tc::pack_bf16(e[4], e[5]), tc::pack_bf16(e[6], e[7])));
           }
         }
       }
     }
-    if (tid == 0) tc::bulk_wait_read<0>();  // the dS image has left its tile
+    if (tid < NST) tc::bulk_wait_read<0>();  // the dS image has left its tile
     if (ok) ok = tc::mbar_wait(&mbar[3 + buf], lph);  // w image of this chunk
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     if (ok && tid == 0) {  // ... - w^T dv_new
-      tc::issue_gemm(taddr + 256, tc::mnmajor_sw128_tile(Aw + buf * 16384, 8192), tc::mnmajor_tile(Bd, KD), 128, KD, C, true);
+      tc::issue_gemm(taddr + 256, tc::mnmajor_sw128_tile(Aw + buf * 16384, 8192), tc::mnmajor_tile(Bd, NV), 128, NV, C, true);
       tc::mma_commit(mbar);
-      tc::bulk_store(p.dvn + ci * C * KD, tc::smem_u32(Bd), 16384);  // -dv_new as the operand-tile image
+    }
+    if (ok && tid < (NST + 1) / 2) {  // -dv_new as the operand-tile image
+      tc::bulk_store(p.dvn + ci * C * KD + tid * 8 * KD + 8 * col0, tc::smem_u32(Bd) + tid * 16 * NV, 256 * NV / (NST + (NST & 1)));
       tc::bulk_commit();
     }
     if (c > 0) {  // in the shadow of the MMA: the next chunk's q (its group landed a chunk ago)
@@ -246,21 +256,21 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
     tc::fence_after_sync();
     issue_B(c - 2);
     if (ok) {
-      float a[64];
-      ld_acc64(taddr + 256 + j0, warp, a);
+      float a[NC];
+      ld_accN(taddr + 256 + j0, warp, a);
 #pragma unroll
-      for (int jj = 0; jj < 64; ++jj) dS[jj] = fmaf(L, dS[jj], a[jj]);
+      for (int jj = 0; jj < NC; ++jj) dS[jj] = fmaf(L, dS[jj], a[jj]);
     }
     tc::fence_before_sync();
   }
   if (!TMA) tc::cp_async_wait<0>();
-  if (tid == 0) tc::bulk_wait_read<0>();  // shared memory must outlive the copies
+  if (tid < NST) tc::bulk_wait_read<0>();  // shared memory must outlive the copies
   if (!ok && tid == 0) atomicExch(p.status, 3);
   if (ok && p.dh0 && kk < p.Dk) {
-    float4* dst = reinterpret_cast<float4*>(p.dh0 + ((size_t)bh * p.Dk + kk) * p.Dv + j0);
+    float4* dst = reinterpret_cast<float4*>(p.dh0 + ((size_t)bh * p.Dk + kk) * p.Dv + col0 + j0);
 #pragma unroll
-    for (int x = 0; x < 16; ++x)
-      if (j0 + 4 * x < p.Dv) dst[x] = make_float4(dS[4 * x], dS[4 * x + 1], dS[4 * x + 2], dS[4 * x + 3]);
+    for (int x = 0; x < NC / 4; ++x)
+      if (col0 + j0 + 4 * x < p.Dv) dst[x] = make_float4(dS[4 * x], dS[4 * x + 1], dS[4 * x + 2], dS[4 * x + 3]);
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -745,15 +755,18 @@ mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st) {
                    make_tma_map_bthd(&maps.q, p.q, p.B, p.T, p.H, p.Dk) && make_tma_map_bthd(&maps.v, p.v, p.B, p.T, p.H, p.Dv) &&
                    make_tma_map_bthd(&maps.dO, p.dO, p.B, p.T, p.H, p.Dv);
   if (narrow && !tma) return MXB_ERR_UNSUPPORTED;
-  if (tma) {
-    if (MXB_ALLOW_SMEM(kStateBwdSmem, gdn_tc_state_bwd_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
+  auto state = [&](auto tma_v, auto nv) {
+    constexpr bool TMA = decltype(tma_v)::value;
+    constexpr int NV = decltype(nv)::value;
+    if (MXB_ALLOW_SMEM(kStateBwdSmem<NV>, gdn_tc_state_bwd_kernel<TMA, NV>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_state_bwd_kernel", st,
-               (gdn_tc_state_bwd_kernel<true><<<dim3(p.B * p.H), 256, kStateBwdSmem, st>>>(p, maps)));
-  } else {
-    if (MXB_ALLOW_SMEM(kStateBwdSmem, gdn_tc_state_bwd_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
-    MXB_LAUNCH("gdn_tc_state_bwd_kernel", st,
-               (gdn_tc_state_bwd_kernel<false><<<dim3(p.B * p.H), 256, kStateBwdSmem, st>>>(p, maps)));
-  }
+               (gdn_tc_state_bwd_kernel<TMA, NV><<<dim3(p.B * p.H, (p.Dv + NV - 1) / NV), 256, kStateBwdSmem<NV>, st>>>(p, maps)));
+    return MXB_OK;
+  };
+  if (!tma) s = state(std::false_type{}, std::integral_constant<int, KD>{});
+  else if (tc_split_columns(p)) s = state(std::true_type{}, std::integral_constant<int, 64>{});
+  else s = state(std::true_type{}, std::integral_constant<int, KD>{});
+  if (s != MXB_OK) return s;
   s = check_launch("gdn_tc_state_bwd_kernel");
   if (s != MXB_OK) return s;
   // The chunk kernel is fed and drained by the copy engine only (also under MXB_GDN_NO_TMA, which selects the
