@@ -543,6 +543,7 @@ mxb_status mxb_mamba3_block_post_bwd(const mxb_mamba3_desc* d, float eps, const 
 }
 
 // ---------------------------------------------------------------- host ctx
+constexpr int kHostSlots = 4;  // slices in flight at most
 struct mxb_host_ctx {
   int device;
   char* arena;
@@ -550,8 +551,8 @@ struct mxb_host_ctx {
   cudaStream_t stream;           // kernels of the even slices
   cudaStream_t stream2;          // kernels of the odd slices (small slices do not fill the GPU: let two overlap)
   cudaStream_t s_h2d, s_d2h;     // copy engines, one per direction
-  cudaEvent_t h2d_done[2], comp_done[2], d2h_done[2];
-  cudaEvent_t do_done[2], fwd_done[2];  // dO uploaded / forward finished: the forward need not wait for dO, nor out for the backward
+  cudaEvent_t h2d_done[kHostSlots], comp_done[kHostSlots], d2h_done[kHostSlots];
+  cudaEvent_t do_done[kHostSlots], fwd_done[kHostSlots];  // dO uploaded / forward finished: the forward need not wait for dO, nor out for the backward
   cudaEvent_t bg_up;                    // beta and gate of the whole batch uploaded
 };
 
@@ -578,7 +579,7 @@ mxb_status mxb_host_ctx_create(int device, size_t arena_bytes, mxb_host_ctx** ou
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->s_h2d, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->s_d2h, cudaStreamNonBlocking);
-  for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
+  for (int i = 0; i < kHostSlots && e == cudaSuccess; ++i) {
     e = cudaEventCreateWithFlags(&c->h2d_done[i], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->comp_done[i], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->d2h_done[i], cudaEventDisableTiming);
@@ -599,7 +600,7 @@ void mxb_host_ctx_destroy(mxb_host_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   cudaDeviceSynchronize();
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < kHostSlots; ++i) {
     if (c->h2d_done[i]) cudaEventDestroy(c->h2d_done[i]);
     if (c->comp_done[i]) cudaEventDestroy(c->comp_done[i]);
     if (c->d2h_done[i]) cudaEventDestroy(c->d2h_done[i]);
@@ -627,11 +628,41 @@ __global__ void __launch_bounds__(256) head_scatter_kernel(const float* __restri
     full[(i / Hs) * H + h0 + (i % Hs)] = compact[i];
 }
 
-// The batch is cut into slices; slice i+1 is uploaded and slice i-1 downloaded while slice i computes (two device
-// slots per tensor, two copy streams, two kernel streams, events between them).  A slice is one sequence, or - when
-// the batch has few sequences - a group of heads of one sequence, moved by strided copies: the first upload and the
-// last download are the part of the traffic nothing overlaps, so slices are kept to about a sixteenth of the batch.
-// beta and gate (and their gradients) are small: they cross once for the whole batch.
+// The batch is cut into slices; later slices are uploaded and earlier ones downloaded while slice i computes (device
+// slots per tensor, two copy streams, two kernel streams, events between them).  A slice is some sequences, or - when
+// the batch has few - a group of heads of one sequence, moved by strided copies.  beta and gate (and their gradients)
+// are small: they cross once for the whole batch.
+//
+// Bound by the PCIe link, 64 MB each way in 1.36 ms when both directions run.  Besides that a call takes the first
+// upload and the last download (one slice, which nothing overlaps), one slice's chain of kernels, and about 11 us per
+// copy when both directions run (the strided row width makes no difference down to 512 bytes): with S slices of 4
+// copies, bytes / (S * 49 GB/s) + S * 44 us, least near S = sqrt(bytes / 2.25 MB).  More slices than that lost at
+// every size (2 x 2048 x 16 heads of 128: 2, 4, 8 slices 2161, 1852, 1980 us; 4 x 1024 x 16: 4, 8, 16 slices 1868,
+// 1855, 2500; 2 x 700 x 16: 2, 4, 8 slices 756, 793, 988; 1 x 200 x 8: 1, 2 slices 156, 181).
+struct HostSlicing {
+  int per, nsplit;  // sequences per slice; head groups per sequence (one sequence per slice then)
+};
+static HostSlicing host_slicing(const mxb_gdn_desc* d, size_t es) {
+  const double bytes = 2.0 * d->B * d->T * d->H * ((double)d->Dk + d->Dv) * es;
+  int want = 1;
+  while (want < 16 && (want + 1.0) * (want + 1.0) * 2.25e6 <= bytes) ++want;
+  HostSlicing h{(d->B + want - 1) / want, 1};
+  // Head groups in halves, or in rows of a host page at least: with a quarter of a page per row every slice's copies
+  // touch every page again, which some hosts translate slowly (1 x 4096 x 16 heads of 128, two and four groups: 2185
+  // and 2014 us on one host, 2350 and 2709 on another).
+  const size_t row = (size_t)d->H * (d->Dk < d->Dv ? d->Dk : d->Dv) * es;
+  while (d->B * 2 * h.nsplit <= want && d->H % (2 * h.nsplit) == 0 && (h.nsplit == 1 || row / (2 * h.nsplit) >= 4096))
+    h.nsplit *= 2;
+  return h;
+}
+// The next finer slicing, for an arena that cannot hold the slots of `h`; false when there is none.
+static bool host_slice_finer(const mxb_gdn_desc* d, HostSlicing* h) {
+  if (h->per > 1) { h->per /= 2; return true; }
+  if (d->H % (2 * h->nsplit)) return false;
+  h->nsplit *= 2;
+  return true;
+}
+
 static mxb_status host_gdn_pipeline(mxb_host_ctx* c, const mxb_gdn_desc* d, const void* q, const void* k,
                                     const void* v, const float* beta, const float* gate, void* out,
                                     const void* d_out, void* dq, void* dk, void* dv, float* dbeta, float* dgate) {
@@ -643,72 +674,75 @@ static mxb_status host_gdn_pipeline(mxb_host_ctx* c, const mxb_gdn_desc* d, cons
   if (bwd && (!dq || !dk || !dv || !dbeta || !dgate)) return MXB_ERR_INVALID_ARGUMENT;
   MXB_CUDA_TRY(cudaSetDevice(c->device));
   const size_t es = d->io_dtype == MXB_F32 ? 4 : 2;
-  // sequences per slice (MXB_HOST_SLICE_SEQS overrides the default of 1) and head groups per sequence
-  // (MXB_HOST_HEAD_SPLIT overrides; by default doubled until there are 16 slices, while a group's rows stay >= 1 KB)
-  int per = 1, nsplit = 1;
-  bool per_set = false;
-  if (const char* ev = std::getenv("MXB_HOST_SLICE_SEQS")) { per = std::atoi(ev); per_set = true; }
-  if (per < 1) per = 1;
-  if (per > d->B) per = d->B;
-  if (const char* ev = std::getenv("MXB_HOST_HEAD_SPLIT")) {
-    nsplit = std::atoi(ev);
-    if (nsplit < 1 || d->H % nsplit) nsplit = 1;
-  } else if (!per_set) {
-    const size_t dmin = (size_t)(d->Dk < d->Dv ? d->Dk : d->Dv) * es;
-    while (d->B * nsplit < 16 && d->H % (2 * nsplit) == 0 && (size_t)(d->H / (2 * nsplit)) * dmin >= 1024) nsplit *= 2;
+  // MXB_HOST_SLICE_SEQS and MXB_HOST_HEAD_SPLIT override the slicing
+  HostSlicing cut = host_slicing(d, es);
+  const char *ev_seqs = std::getenv("MXB_HOST_SLICE_SEQS"), *ev_split = std::getenv("MXB_HOST_HEAD_SPLIT");
+  if (ev_seqs || ev_split) cut = {1, 1};
+  if (ev_seqs) cut.per = std::atoi(ev_seqs);
+  if (cut.per < 1) cut.per = 1;
+  if (cut.per > d->B) cut.per = d->B;
+  if (ev_split) {
+    cut.nsplit = std::atoi(ev_split);
+    if (cut.nsplit < 1 || d->H % cut.nsplit) cut.nsplit = 1;
   }
-  if (nsplit > 1) per = 1;
-  const int Hs = d->H / nsplit;  // heads of the largest slice
+  if (cut.nsplit > 1) cut.per = 1;
+  const size_t nfull = (size_t)d->B * d->T * d->H;  // beta, gate and their gradients, whole batch
+  mxb_gdn_desc df = *d, db = *d;
+  if (bwd) {  // keep the forward intermediates in the arena for the backward that follows
+    df.flags |= MXB_GDN_SAVE_FOR_BWD;
+    db.flags |= MXB_GDN_BWD_USE_SAVED;
+  }
+  float *f_beta = nullptr, *f_gate = nullptr, *f_dbeta = nullptr, *f_dgate = nullptr;
+  char *i_q[kHostSlots], *i_k[kHostSlots], *i_v[kHostSlots], *i_do[kHostSlots];
+  char *o_out[kHostSlots], *o_q[kHostSlots], *o_k[kHostSlots], *o_v[kHostSlots], *wss[kHostSlots];
+  float *i_b[kHostSlots], *i_g[kHostSlots], *o_b[kHostSlots], *o_g[kHostSlots];
+  size_t ws_bytes = 0;
+  int nslots = kHostSlots, nslices = 0;
+  // Up to four slots, so that a slice whose chain of kernels is longer than its copies does not hold back the uploads
+  // behind it; as many as the arena holds, and finer slices where it cannot hold two.
+  for (;;) {
+    const int nsplit = cut.nsplit, Hs = d->H / nsplit;
+    nslices = nsplit > 1 ? d->B * nsplit : (d->B + cut.per - 1) / cut.per;
+    if (nslots > nslices) nslots = nslices < 2 ? 2 : nslices;
+    df.B = db.B = cut.per;
+    df.H = db.H = Hs;
+    const size_t ws_f = mxb_gdn_fwd_workspace_bytes(&df), ws_b = bwd ? mxb_gdn_bwd_workspace_bytes(&db) : 0;
+    ws_bytes = ws_f > ws_b ? ws_f : ws_b;
+    const size_t ns = (size_t)cut.per * d->T * Hs, nk = ns * d->Dk, nv = ns * d->Dv;  // slot capacities
+    Carver cv(c->arena);
+    f_beta = cv.take<float>(nfull);
+    f_gate = cv.take<float>(nfull);
+    f_dbeta = bwd ? cv.take<float>(nfull) : nullptr;
+    f_dgate = bwd ? cv.take<float>(nfull) : nullptr;
+    for (int sl = 0; sl < nslots; ++sl) {
+      i_q[sl] = cv.take<char>(nk * es); i_k[sl] = cv.take<char>(nk * es); i_v[sl] = cv.take<char>(nv * es);
+      o_out[sl] = cv.take<char>(nv * es);
+      i_b[sl] = i_g[sl] = o_b[sl] = o_g[sl] = nullptr;
+      if (nsplit > 1) { i_b[sl] = cv.take<float>(ns); i_g[sl] = cv.take<float>(ns); }
+      i_do[sl] = o_q[sl] = o_k[sl] = o_v[sl] = nullptr;
+      if (bwd) {
+        i_do[sl] = cv.take<char>(nv * es);
+        o_q[sl] = cv.take<char>(nk * es); o_k[sl] = cv.take<char>(nk * es); o_v[sl] = cv.take<char>(nv * es);
+        if (nsplit > 1) { o_b[sl] = cv.take<float>(ns); o_g[sl] = cv.take<float>(ns); }
+      }
+      wss[sl] = cv.take<char>(ws_bytes);
+    }
+    if (cv.bytes() <= c->arena_bytes) break;
+    if (nslots > 2) { --nslots; continue; }
+    if (ev_seqs || ev_split || !host_slice_finer(d, &cut)) return MXB_ERR_WORKSPACE;
+    nslots = kHostSlots;
+  }
+  const int per = cut.per, nsplit = cut.nsplit, Hs = d->H / nsplit;
+  // per-sequence element counts of a slice's tensors
+  const size_t sk = (size_t)d->T * Hs * d->Dk, sv = (size_t)d->T * Hs * d->Dv;
   struct Slice { int b0, nb, h0, hs; };
   std::vector<Slice> slices;
   if (nsplit > 1) {
-    // equal head groups: cutting the last group finer (to shorten the download that overlaps nothing) was slower,
-    // every extra slice pays the latency of the sequential state passes once more
     for (int b0 = 0; b0 < d->B; ++b0)
       for (int g = 0; g < nsplit; ++g) slices.push_back({b0, 1, g * Hs, Hs});
   } else {
     for (int b0 = 0; b0 < d->B; b0 += per) slices.push_back({b0, b0 + per <= d->B ? per : d->B - b0, 0, d->H});
   }
-  const int nslices = (int)slices.size();
-  // per-sequence element counts of a slice's tensors
-  const size_t sk = (size_t)d->T * Hs * d->Dk, sv = (size_t)d->T * Hs * d->Dv, ss = (size_t)d->T * Hs;
-  mxb_gdn_desc d1 = *d;
-  d1.B = per;
-  d1.H = Hs;
-  mxb_gdn_desc df = d1, db = d1;
-  // The slices' kernels stage their operands with per-thread copies where they have such a variant: this call is
-  // bound by the two PCIe copy streams, which ran slower beside kernels fed by the tensor-copy engine.
-  df.flags |= MXB_GDN_NO_TMA;
-  db.flags |= MXB_GDN_NO_TMA;
-  if (bwd) {  // keep the forward intermediates in the arena for the backward that follows
-    df.flags |= MXB_GDN_SAVE_FOR_BWD;
-    db.flags |= MXB_GDN_BWD_USE_SAVED;
-  }
-  const size_t ws_f = mxb_gdn_fwd_workspace_bytes(&df), ws_b = bwd ? mxb_gdn_bwd_workspace_bytes(&db) : 0;
-  const size_t ws_bytes = ws_f > ws_b ? ws_f : ws_b;
-  const size_t nk = sk * per, nv = sv * per, ns = ss * per;  // slot capacities
-  const size_t nfull = (size_t)d->B * d->T * d->H;           // beta, gate and their gradients, whole batch
-  Carver cv(c->arena);
-  char *i_q[2], *i_k[2], *i_v[2], *i_do[2], *o_out[2], *o_q[2], *o_k[2], *o_v[2];
-  float *i_b[2], *i_g[2], *o_b[2], *o_g[2];
-  float* f_beta = cv.take<float>(nfull);
-  float* f_gate = cv.take<float>(nfull);
-  float* f_dbeta = bwd ? cv.take<float>(nfull) : nullptr;
-  float* f_dgate = bwd ? cv.take<float>(nfull) : nullptr;
-  for (int sl = 0; sl < 2; ++sl) {
-    i_q[sl] = cv.take<char>(nk * es); i_k[sl] = cv.take<char>(nk * es); i_v[sl] = cv.take<char>(nv * es);
-    o_out[sl] = cv.take<char>(nv * es);
-    i_b[sl] = i_g[sl] = o_b[sl] = o_g[sl] = nullptr;
-    if (nsplit > 1) { i_b[sl] = cv.take<float>(ns); i_g[sl] = cv.take<float>(ns); }
-    i_do[sl] = o_q[sl] = o_k[sl] = o_v[sl] = nullptr;
-    if (bwd) {
-      i_do[sl] = cv.take<char>(nv * es);
-      o_q[sl] = cv.take<char>(nk * es); o_k[sl] = cv.take<char>(nk * es); o_v[sl] = cv.take<char>(nv * es);
-      if (nsplit > 1) { o_b[sl] = cv.take<float>(ns); o_g[sl] = cv.take<float>(ns); }
-    }
-  }
-  char* wss[2] = {cv.take<char>(ws_bytes), cv.take<char>(ws_bytes)};  // one workspace per slot
-  if (cv.bytes() > c->arena_bytes) return MXB_ERR_WORKSPACE;
   auto hp = [](const void* base, size_t off) { return static_cast<const char*>(base) + off; };
   auto hpw = [](void* base, size_t off) { return static_cast<char*>(base) + off; };
   const cudaMemcpyKind H2D = cudaMemcpyHostToDevice, D2H = cudaMemcpyDeviceToHost;
@@ -727,7 +761,7 @@ static mxb_status host_gdn_pipeline(mxb_host_ctx* c, const mxb_gdn_desc* d, cons
   MXB_CUDA_TRY(cudaMemcpyAsync(f_gate, gate, nfull * 4, H2D, c->s_h2d));
   MXB_CUDA_TRY(cudaEventRecord(c->bg_up, c->s_h2d));
   for (int bi = 0; bi < nslices; ++bi) {
-    const int sl = bi & 1;
+    const int sl = bi % nslots;
     const int b0 = slices[bi].b0, nb = slices[bi].nb, h0 = slices[bi].h0, hs = slices[bi].hs;
     const size_t ck = sk * nb * es, cvb = sv * nb * es;   // bytes of this slice (contiguous slices only)
     // element offsets of the slice's first row in the full tensors
@@ -735,7 +769,7 @@ static mxb_status host_gdn_pipeline(mxb_host_ctx* c, const mxb_gdn_desc* d, cons
     const size_t os_ = (size_t)b0 * d->T * d->H;
     df.B = db.B = nb;
     df.H = db.H = hs;
-    if (bi >= 2) MXB_CUDA_TRY(cudaStreamWaitEvent(c->s_h2d, c->comp_done[sl], 0));  // slot inputs consumed
+    if (bi >= nslots) MXB_CUDA_TRY(cudaStreamWaitEvent(c->s_h2d, c->comp_done[sl], 0));  // slot inputs consumed
     MXB_CUDA_TRY(up(i_q[sl], q, ok_, ck, d->Dk, hs));
     MXB_CUDA_TRY(up(i_k[sl], k, ok_, ck, d->Dk, hs));
     MXB_CUDA_TRY(up(i_v[sl], v, ov_, cvb, d->Dv, hs));
@@ -744,11 +778,11 @@ static mxb_status host_gdn_pipeline(mxb_host_ctx* c, const mxb_gdn_desc* d, cons
       MXB_CUDA_TRY(up(i_do[sl], d_out, ov_, cvb, d->Dv, hs));
       MXB_CUDA_TRY(cudaEventRecord(c->do_done[sl], c->s_h2d));
     }
-    cudaStream_t kst = sl ? c->stream2 : c->stream;
+    cudaStream_t kst = (bi & 1) ? c->stream2 : c->stream;
     char* ws = wss[sl];
     MXB_CUDA_TRY(cudaStreamWaitEvent(kst, c->h2d_done[sl], 0));
     if (bi < 2) MXB_CUDA_TRY(cudaStreamWaitEvent(kst, c->bg_up, 0));
-    if (bi >= 2) MXB_CUDA_TRY(cudaStreamWaitEvent(kst, c->d2h_done[sl], 0));  // slot outputs drained
+    if (bi >= nslots) MXB_CUDA_TRY(cudaStreamWaitEvent(kst, c->d2h_done[sl], 0));  // slot outputs drained
     const float *sb = f_beta + os_, *sg = f_gate + os_;
     float *sdb = bwd ? f_dbeta + os_ : nullptr, *sdg = bwd ? f_dgate + os_ : nullptr;
     const size_t rows = (size_t)nb * d->T;
@@ -786,8 +820,7 @@ static mxb_status host_gdn_pipeline(mxb_host_ctx* c, const mxb_gdn_desc* d, cons
     MXB_CUDA_TRY(cudaEventRecord(c->d2h_done[sl], c->s_d2h));
   }
   if (bwd) {  // the per-head gradients of the whole batch, once every slice has computed
-    MXB_CUDA_TRY(cudaStreamWaitEvent(c->s_d2h, c->comp_done[0], 0));
-    if (nslices > 1) MXB_CUDA_TRY(cudaStreamWaitEvent(c->s_d2h, c->comp_done[1], 0));
+    // (the download stream has waited for each of them)
     MXB_CUDA_TRY(cudaMemcpyAsync(dbeta, f_dbeta, nfull * 4, D2H, c->s_d2h));
     MXB_CUDA_TRY(cudaMemcpyAsync(dgate, f_dgate, nfull * 4, D2H, c->s_d2h));
   }
