@@ -236,14 +236,14 @@ __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid
   tc::fence_after_sync();
   const int ir = 16 * warp + (lane & 15);  // M=64: row m sits in TMEM lane (m%16) + 32*(m/16)
   if (ok) {
-    // the u image (un-swizzled K-major layout; rows 0-31 and 32-63 are its two contiguous halves) over the v boxes
+    // the u image (column-blocked: columns 0-63 and 64-127 are its two contiguous halves) over the v boxes
     for (int c0 = 0; c0 < 128; c0 += 32) {
       float f[32];
       ld_acc32(taddr, warp, c0, f);
       if (lane < 16) {
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
-          const uint32_t off = tc::kmajor_unit(ir, (c0 >> 3) + x, KD);
+          const uint32_t off = tc::colblk_unit(ir, (c0 >> 3) + x, C);
           sts16(Akq, 8192u + (off >> 13) * 16384u + (off & 8191u), pack8f(&f[8 * x]));
         }
       }
@@ -292,128 +292,207 @@ __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid
 }
 
 // ------------------------------------------------------------ state forward
-// One CTA (256 threads) per (batch, head).  Thread t owns state row kk = t & 127 and the
-// 64 columns of half t >> 7.  The operand tiles are double-buffered (buffer c & 1 for chunk c): the operands of
-// chunk c+2 are requested as soon as the MMA (or epilogue) that last read the buffer for chunk c has finished, so
-// a copy has more than a whole chunk period to land (a chunk takes ~2.5 us, a copy from HBM up to ~1.5 us):
-//   group A  [w;q]      buffer free after MMA1      needed before MMA1
-//   group U  u          free after epilogue 1       needed before epilogue 1
-//   group PK P and k    free after MMA2/MMA3        needed in the shadow of MMA1 (k is scaled in place there)
-// Six groups are outstanding at the top of every chunk, in the order A, U, PK (chunk c), A, U, PK (chunk c+1).
+// One CTA (256 threads) per (batch, head) and NV columns.  Thread t owns state row kk = t & 127 and the
+// columns of half t >> 7.  The operand tiles are buffered (buffer c & 1 for chunk c; k: c % 3) and requested as soon
+// as the MMA (or epilogue) that last read the buffer has finished, a chunk period or more before they are needed:
+//   A  [w;q]   buffer free after w S           needed before w S
+//   U  u       free after v_new                needed before v_new
+//   K  k       free after (r k)^T v_new        needed in the shadow of the chunk before (k is scaled in place there)
+//   P          free after P v_new              needed before P v_new
+//
+// Bound by the chain S -> w S -> v_new -> (r k)^T v_new -> S where the heads are few, by HBM where they fill the GPU.
+// Only what the chain needs stands between its products: q S and the output rows (E(gam) q S + P v_new) are finished in
+// the shadow of the next chunk's w S, the decay factors and the scaled k of the next chunk in the shadow of this one's
+// products, and P v_new is issued behind the state update (16 heads of 128, 24 chunks, NV = 64: 2.3 -> 1.9 us a chunk).  More work moved into the shadow of w S
+// (half of the scaling of k, the u operand into registers) slowed the product down: both need shared memory, 47 -> 50 us.
 //
 // TMA = true: q and k rows arrive as tensor-map boxes (128-byte swizzle) issued by ONE thread and complete on the
 // barrier of their group, like the images: no thread spends issue slots on copies (four cp.async per thread and
-// group cost every thread ~1.6 k and ~1.1 k cycles per chunk, on the critical path between an MMA and its epilogue).
+// group cost every thread ~1.6 k and ~1.1 k cycles per chunk).
 // TMA = false: the same rows by cp.async into the same swizzled positions.
 //
 // NV: columns of the state per CTA.  128 (all of them) where the (batch, head) pairs fill the GPU; 64 otherwise: a
 // chunk's chain of products and epilogues is then half as wide (columns of the state are independent; w, q, k and P are
 // read by both CTAs, the second time from L2).
 template <int NV>
-constexpr int kStateFwdSmem = 2 * 32768 + 256 * NV + 2 * 16384 + 128 * NV + 128 * NV + 2 * 16384 + 2 * 128 * NV + 2 * C * 4 + 128 + 1024;
+constexpr int kStateFwdSmem =
+    2 * 32768 + 256 * NV + 2 * 8192 + 128 * NV + 128 * NV + 3 * 16384 + 2 * 128 * NV + 4 * C * 4 + 128 + 1024;
 
 template <bool TMA, int NV>
-__global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+__global__ void __launch_bounds__(kStateThreads<NV>, 1) gdn_tc_state_fwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
   static_assert(NV == KD || TMA, "the per-thread staging moves whole rows");
   constexpr int NC = NV / 2;                   // columns per thread
-  constexpr int NST = NV == KD ? 1 : 16;       // pieces of a state image in the workspace (rows of eight, NV columns)
   const int col0 = blockIdx.y * NV;
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
   uint8_t* A1 = sm;                 // x2 [128: w rows 0-63, q rows 64-127][128 kk], two swizzled slabs of 64 columns
   uint8_t* Sop = A1 + 2 * 32768;    // [128 kk][NV j]    bf16 copy of the state
-  uint8_t* A2 = Sop + 256 * NV;       // x2 [128: zero rows 0-63, P rows 64-127][64 m]
-  uint8_t* Vn = A2 + 2 * 16384;     // [64 i][NV j]      v_new
+  uint8_t* Pm = Sop + 256 * NV;     // x2 [64 i][64 m]   P
+  uint8_t* Vn = Pm + 2 * 8192;      // [64 i][NV j]      v_new
   uint8_t* Ot = Vn + 128 * NV;      // [64 i][NV j]      output tile on its way out (swizzled slabs of 64 columns)
-  uint8_t* A3 = Ot + 128 * NV;       // x2 [64 i][128 kk] k, then diag(E(gam_last-gam_i)) k  (A = k^T), swizzled slabs
-  uint8_t* Ut = A3 + 2 * 16384;     // x2 [64 i][NV j]   u
+  uint8_t* A3 = Ot + 128 * NV;      // x3 [64 i][128 kk] k, then diag(E(gam_last-gam_i)) k  (A = k^T), swizzled slabs
+  uint8_t* Ut = A3 + 3 * 16384;     // x2 [64 i][NV j]   u
   float* dd = reinterpret_cast<float*>(Ut + 2 * 128 * NV);
-  float* rr = dd + C;
-  // [0] MMA completion; per buffer: [1 + buf] w image and q rows, [3 + buf] u image, [5 + buf] P image and k rows landed
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(rr + C);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 8);
+  float* rr = dd + 2 * C;           // (both: two buffers)
+  // [0] w S and q S, later (r k)^T v_new; [10] P v_new; landed, per buffer: [1..] w image and q rows, [3..] u image,
+  // [5..] k rows, [8..] P image
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(rr + 2 * C);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 11);
 
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int kk = tid & 127, half = tid >> 7, j0 = NC * half;
+  const int kk = tid & 127, half = tid >> 7, j0 = NC * half;  // (of the 256 threads of warps 0-7)
+  const bool lead = tid == 256;  // issues the products and the copies
   const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
-  const uint32_t sA1b = tc::smem_u32(A1), sA2b = tc::smem_u32(A2), sA3b = tc::smem_u32(A3), sUb = tc::smem_u32(Ut);
+  const uint32_t sA1b = tc::smem_u32(A1), sPb = tc::smem_u32(Pm), sA3b = tc::smem_u32(A3), sUb = tc::smem_u32(Ut);
   const uint32_t sOt = tc::smem_u32(Ot);
-  constexpr int kOutThread = 96;  // hands the output tiles to the copy engine (its own bulk-group queue)
 
   auto grow = [&](int c, int i) { return ((size_t)(b * p.T + c * C + i) * p.H + h); };
-  // The workspace tiles (w, u, P) are byte images of the operand layout: one bulk copy each, issued by one
-  // thread, completing on an mbarrier.  The raw q and k rows come by cp.async.
-  // Slab s of A1 (columns 64 s ..): the w slab (rows 0-63), then the q box (rows 64-127).  The issuing threads sit
-  // in warps whose epilogue after the issue point is the short one (tid 64: q rows; tid 32: state update).
-  auto issue_A = [&](int c) {  // [w;q] of chunk c
-    if (c < p.n) {
-      const size_t ci = (size_t)bh * p.n + c;
-      const uint32_t sA1 = sA1b + (c & 1) * 32768;
-      uint64_t* mb = &mbar[1 + (c & 1)];
-      if (tid == 64) {
-        tc::mbar_expect_tx(mb, TMA ? 32768 : 16384);
-        for (int sl = 0; sl < 2; ++sl) {
-          tc::bulk_load(sA1 + sl * 16384, p.w + ci * C * KD + sl * 4096, 8192, mb);
-          if (TMA) tc::tma_load_4d(sA1 + sl * 16384 + 8192, &maps.q, 64 * sl, h, c * C, b, mb);
-        }
-      }
-      if (!TMA) {
-        const int imax = min(C, p.T - c * C);
-        for (int u = tid; u < 64 * 16; u += 256) {
-          const int i = urow16(u), c8 = ucol16(u);
-          const uint32_t off = (uint32_t)(c8 >> 3) * 16384u + 8192u + (uint32_t)i * 128u + (uint32_t)(((c8 & 7) ^ (i & 7)) << 4);
-          tc::cp_async16(sA1 + off, i < imax ? p.q + grow(c, i) * KD + c8 * 8 : p.q, i < imax);
-        }
-      }
+  // The workspace tiles (w, u, P) are byte images of the operand layout: one bulk copy each, completing on an mbarrier.
+  // Slab s of A1 (columns 64 s ..): the w slab (rows 0-63), then the q box (rows 64-127).
+  auto load_A = [&](int c) {  // [w;q] of chunk c
+    if (c >= p.n) return;
+    const size_t ci = (size_t)bh * p.n + c;
+    const uint32_t sA1 = sA1b + (c & 1) * 32768;
+    uint64_t* mb = &mbar[1 + (c & 1)];
+    tc::mbar_expect_tx(mb, TMA ? 32768 : 16384);
+    for (int sl = 0; sl < 2; ++sl) {
+      tc::bulk_load(sA1 + sl * 16384, p.w + ci * C * KD + sl * 4096, 8192, mb);
+      if (TMA) tc::tma_load_4d(sA1 + sl * 16384 + 8192, &maps.q, 64 * sl, h, c * C, b, mb);
     }
-    if (!TMA) tc::cp_async_commit();
   };
-  auto issue_U = [&](int c) {
-    if (c < p.n && tid == 64) {
-      const size_t ci = (size_t)bh * p.n + c;
-      tc::mbar_expect_tx(&mbar[3 + (c & 1)], 128 * NV);
-      for (int g = 0; g < (NST + 1) / 2; ++g)  // this CTA's columns of each group of eight rows
-        tc::bulk_load(sUb + (c & 1) * 128 * NV + g * 16 * NV, p.u + ci * C * KD + g * 8 * KD + 8 * col0, 256 * NV / (NST + (NST & 1)),
-                      &mbar[3 + (c & 1)]);
-    }
-    if (!TMA) tc::cp_async_commit();  // (empty: keeps the group count of the schedule below)
+  auto load_U = [&](int c) {
+    if (c >= p.n) return;
+    uint64_t* mb = &mbar[3 + (c & 1)];
+    tc::mbar_expect_tx(mb, 128 * NV);
+    tc::bulk_load(sUb + (c & 1) * 128 * NV, p.u + ((size_t)bh * p.n + c) * C * KD + C * col0, 128 * NV, mb);
   };
-  auto issue_PK = [&](int c) {
-    if (c < p.n) {
-      const size_t ci = (size_t)bh * p.n + c;
-      const uint32_t sA2 = sA2b + (c & 1) * 16384, sA3 = sA3b + (c & 1) * 16384;
-      uint64_t* mb = &mbar[5 + (c & 1)];
-      if (tid == 32) {
-        tc::mbar_expect_tx(mb, TMA ? 8192 + 16384 : 8192);
-        tc::bulk_load(sA2 + 8192, p.P + ci * C * C, 8192, mb);  // rows 64..127 of the [128][64] tile
-        if (TMA)
-          for (int sl = 0; sl < 2; ++sl) tc::tma_load_4d(sA3 + sl * 8192, &maps.k, 64 * sl, h, c * C, b, mb);
-      }
-      if (!TMA) {
-        const int imax = min(C, p.T - c * C);
-        for (int u = tid; u < 64 * 16; u += 256) {
-          const int i = urow16(u), c8 = ucol16(u);
-          tc::cp_async16(sA3 + tc::sw128_unit(i, c8), i < imax ? p.k + grow(c, i) * KD + c8 * 8 : p.k, i < imax);
-        }
-      }
+  auto load_K = [&](int c) {
+    if (!TMA || c >= p.n) return;
+    uint64_t* mb = &mbar[5 + c % 3];
+    tc::mbar_expect_tx(mb, 16384);
+    for (int sl = 0; sl < 2; ++sl) tc::tma_load_4d(sA3b + (c % 3) * 16384 + sl * 8192, &maps.k, 64 * sl, h, c * C, b, mb);
+  };
+  auto load_P = [&](int c) {
+    if (c >= p.n) return;
+    tc::mbar_expect_tx(&mbar[8 + (c & 1)], 8192);
+    tc::bulk_load(sPb + (c & 1) * 8192, p.P + ((size_t)bh * p.n + c) * C * C, 8192, &mbar[8 + (c & 1)]);
+  };
+  auto store_out = [&](int c) {
+    for (int sl = 0; sl < (TMA ? NV / 64 : 0); ++sl)  // a slab that lies wholly past the true width is not stored at all
+      if (col0 + 64 * sl < p.Dv) tc::tma_store_4d(&maps.o, sOt + sl * 8192, col0 + 64 * sl, h, c * C, b);
+  };
+  // TMA = false: the q and k rows, by the 256 threads (a group per call, empty past the end)
+  auto copy_q = [&](int c) {
+    if (TMA) return;
+    const int imax = c < p.n ? min(C, p.T - c * C) : -1;
+    for (int u = tid; u < 64 * 16 && imax >= 0; u += 256) {
+      const int i = urow16(u), c8 = ucol16(u);
+      const uint32_t off = (uint32_t)(c8 >> 3) * 16384u + 8192u + (uint32_t)i * 128u + (uint32_t)(((c8 & 7) ^ (i & 7)) << 4);
+      tc::cp_async16(sA1b + (c & 1) * 32768 + off, i < imax ? p.q + grow(c, i) * KD + c8 * 8 : p.q, i < imax);
     }
-    if (!TMA) tc::cp_async_commit();
+    tc::cp_async_commit();
+  };
+  auto copy_k = [&](int c) {
+    if (TMA) return;
+    const int imax = c < p.n ? min(C, p.T - c * C) : -1;
+    for (int u = tid; u < 64 * 16 && imax >= 0; u += 256) {
+      const int i = urow16(u), c8 = ucol16(u);
+      tc::cp_async16(sA3b + (c % 3) * 16384 + tc::sw128_unit(i, c8), i < imax ? p.k + grow(c, i) * KD + c8 * 8 : p.k, i < imax);
+    }
+    tc::cp_async_commit();
   };
 
   if (warp == 0) {
     tc::tmem_alloc(tslot, 512);
     tc::tmem_relinquish();
   }
-  if (tid == 0) {
-    for (int m = 0; m < 7; ++m) tc::mbar_init(&mbar[m], 1);
+  if (lead) {
+    for (int m = 0; m < 11; ++m) tc::mbar_init(&mbar[m], 1);
     tc::mbar_fence_init();
+    for (int c = 0; c < 2; ++c) {
+      load_A(c);
+      load_U(c);
+      load_K(c);
+      load_P(c);
+    }
+    load_K(2);
   }
-  __syncthreads();  // barriers initialised before the copies can complete on them
-  for (int c = 0; c < 2; ++c) {
-    issue_A(c);
-    issue_U(c);
-    issue_PK(c);
+  if (warp >= 8) {
+    if (NV == KD) tc::reg_dec<40>();
+    tc::fence_before_sync();
+    __syncthreads();  // barriers initialised, TMEM allocated
+    tc::fence_after_sync();
+    const uint32_t taddr = *tslot;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int c = 0; c < p.n; ++c) {
+      const size_t ci = (size_t)bh * p.n + c;
+      const int buf = c & 1;
+      const uint32_t lph = (c >> 1) & 1;  // phase of the image barriers of this buffer
+      if (lead) {
+        tc::bulk_wait_read<0>();  // v_new and the output tile of the chunk before have left
+        ok = tc::mbar_wait(&mbar[1 + buf], lph);
+      }
+      ok = __syncthreads_and(ok);
+      if (!ok) break;
+      if (lead) {
+        tc::fence_after_sync();
+        // D1 = [w;q] S
+        tc::issue_gemm(taddr, tc::kmajor_sw128_tile(A1 + buf * 32768, 16384), tc::colblk_mnmajor_tile(Sop, KD), 128, NV, KD, false);
+        tc::mma_commit(mbar);
+        if (p.save) {  // the state at chunk start, saved for the backward as the byte image of the operand tile
+          tc::bulk_store(p.hs + ci * KD * KD + KD * col0, tc::smem_u32(Sop), 256 * NV);
+          tc::bulk_commit();
+        }
+        if (c > 0) {
+          ok = tc::mbar_wait(&mbar[10], (c - 1) & 1);
+          if (ok) load_P(c + 1);
+        }
+        ok = ok && tc::mbar_wait(&mbar[8 + buf], lph);
+        ok = ok && tc::mbar_wait(mbar, ph);
+        if (ok) load_A(c + 2);
+        tc::bulk_wait_read<0>();  // the state image has left its tile
+      }
+      ph ^= 1;
+      __syncthreads();
+      if (lead && ok) {
+        tc::fence_after_sync();
+        // D3 = (r k)^T v_new, which the next chunk waits for, then P v_new into rows 64-127 of D2: the tile is the 128 rows
+        // that end with P; what the 64 rows before it hold (other tiles) only reaches rows of D2 that nothing reads
+        tc::issue_gemm(taddr + 256, tc::mnmajor_sw128_tile(A3 + (c % 3) * 16384, 8192), tc::colblk_mnmajor_tile(Vn, C), 128, NV, C, false);
+        tc::mma_commit(mbar);
+        tc::issue_gemm(taddr + 128, tc::kmajor_tile(Pm + (buf - 1) * 8192, C), tc::colblk_mnmajor_tile(Vn, C), 128, NV, C, false);
+        tc::mma_commit(mbar + 10);
+        if (p.save) tc::bulk_store(p.vn + ci * C * KD + C * col0, tc::smem_u32(Vn), 128 * NV);
+        if (c > 0) store_out(c - 1);  // (its tile is complete since the barrier above)
+        tc::bulk_commit();
+        load_U(c + 2);  // u has been consumed by every thread
+        ok = tc::mbar_wait(mbar, ph);
+        if (ok) load_K(c + 3);
+      }
+      ph ^= 1;
+    }
+    if (lead) tc::bulk_wait_read<0>();
+    __syncthreads();  // the output tile is free
+    __syncthreads();  // and full
+    if (lead) {
+      if (ok) {
+        store_out(p.n - 1);
+        tc::bulk_commit();
+      } else {
+        atomicExch(p.status, 2);
+      }
+      tc::bulk_wait_read<0>();  // shared memory must outlive the copies
+    }
+    __syncthreads();
+    return;
   }
+  if (NV == KD) tc::reg_inc<216>();
+  copy_q(0);
+  copy_k(0);
+  copy_q(1);
+  copy_k(1);
+  copy_k(2);
   float S[NC];  // state row kk, columns col0 + j0 .. (zero outside the true Dk x Dv state)
   if (p.h0) {
     const float4* src = reinterpret_cast<const float4*>(p.h0 + ((size_t)bh * p.Dk + kk) * p.Dv + col0 + j0);
@@ -426,80 +505,88 @@ __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __gr
 #pragma unroll
     for (int x = 0; x < NC; ++x) S[x] = 0.f;
   }
-  for (int u = tid; u < 2 * 64 * 8; u += 256)  // the zero rows of both [0;P] tiles
-    sts16(A2 + (u >> 9) * 16384, tc::kmajor_unit((u >> 3) & 63, u & 7, C), zero16());
+  // Decay factors of a chunk, fetched and computed while the tensor core works on the chunk before it; the k rows of a
+  // chunk are scaled by r in place there too, so that the state update contracts them with v_new itself (every thread
+  // scales the 16-byte units it would copy in the cp.async variant: no barrier needed for those).
+  float g_nxt = p.gam[(size_t)bh * p.n * C + (tid & 63)], gl_nxt = p.gam[(size_t)bh * p.n * C + C - 1];
+  auto decay = [&](int c) {
+    if (tid < C) {
+      dd[(c & 1) * C + tid] = exp_nonpos(g_nxt);
+      rr[(c & 1) * C + tid] = exp_nonpos(gl_nxt - g_nxt);
+    }
+  };
+  bool ok = true;
+  auto scale_k = [&](int c) {
+    if (TMA && ok) ok = tc::mbar_wait(&mbar[5 + c % 3], (c / 3) & 1);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int u = tid + 256 * m, i = urow16(u);
+      uint4* unit = reinterpret_cast<uint4*>(A3 + (c % 3) * 16384 + tc::sw128_unit(i, ucol16(u)));
+      *unit = tc::scale_bf16x8(*unit, rr[(c & 1) * C + i]);
+    }
+  };
+  decay(0);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t taddr = *tslot;
+  if (!TMA) tc::cp_async_wait<3>();  // k of chunk 0 (groups q0 k0 q1 k1 k2)
+  scale_k(0);
   uint32_t ph = 0;
-  bool ok = true;
-
-  // in-chunk cumulative log decay of the chunk ahead, fetched one chunk early (its latency would otherwise sit
-  // at the top of every link of the chain)
-  float g_nxt = p.gam[(size_t)bh * p.n * C + (tid & 63)], gl_nxt = p.gam[(size_t)bh * p.n * C + C - 1];
+  float f[NC];  // accumulator row; rows 64-127 keep E(gam_i) (q S) here until P v_new arrives
+  // out = E(gam)(q S) + P v_new of chunk c, rows in the upper half of the threads
+  auto put_out = [&](int c) {
+    if (ok) ok = tc::mbar_wait(&mbar[10], c & 1);
+    tc::fence_after_sync();
+    if (!ok || kk < 64) return;  // (warp-uniform)
+    const int i = kk & 63;
+    float a[NC];
+    ld_accN(taddr + 128 + j0, warp, a);
+    uint4 o[NC / 8];
+#pragma unroll
+    for (int x = 0; x < NC / 8; ++x)
+      o[x] = make_uint4(tc::pack_bf16(f[8 * x] + a[8 * x], f[8 * x + 1] + a[8 * x + 1]),
+                        tc::pack_bf16(f[8 * x + 2] + a[8 * x + 2], f[8 * x + 3] + a[8 * x + 3]),
+                        tc::pack_bf16(f[8 * x + 4] + a[8 * x + 4], f[8 * x + 5] + a[8 * x + 5]),
+                        tc::pack_bf16(f[8 * x + 6] + a[8 * x + 6], f[8 * x + 7] + a[8 * x + 7]));
+    if (TMA) {  // into the swizzled output tile; one thread hands it to the copy engine after the next barrier
+#pragma unroll
+      for (int x = 0; x < NC / 8; ++x) sts16(Ot, tc::sw128_unit(i, NC / 8 * half + x), o[x]);
+    } else if (c * C + i < p.T) {
+      uint4* dst = reinterpret_cast<uint4*>(p.out + grow(c, i) * KD + j0);
+#pragma unroll
+      for (int x = 0; x < NC / 8; ++x) dst[x] = o[x];
+    }
+  };
   for (int c = 0; c < p.n; ++c) {
     const size_t ci = (size_t)bh * p.n + c;
-    const int t0 = c * C, imax = min(C, p.T - t0);
     const int buf = c & 1;
     const uint32_t lph = (c >> 1) & 1;  // phase of the image barriers of this buffer
-    uint8_t* A1c = A1 + buf * 32768;
-    uint8_t* A2c = A2 + buf * 16384;
-    uint8_t* A3c = A3 + buf * 16384;
-    uint8_t* Utc = Ut + buf * 128 * NV;
-    const float glast = gl_nxt, g = g_nxt;
+    const float L = exp_nonpos(gl_nxt);
     if (c + 1 < p.n) {
       g_nxt = p.gam[(ci + 1) * C + (tid & 63)];
       gl_nxt = p.gam[(ci + 1) * C + C - 1];
-    }
-    const float L = exp_nonpos(glast);
-    if (tid < C) {
-      dd[tid] = exp_nonpos(g);
-      rr[tid] = exp_nonpos(glast - g);
     }
 #pragma unroll
     for (int c8 = 0; c8 < NC / 8; ++c8) {  // state as the MMA operand (and saved for the backward)
       const uint4 val = make_uint4(tc::pack_bf16(S[8 * c8], S[8 * c8 + 1]), tc::pack_bf16(S[8 * c8 + 2], S[8 * c8 + 3]),
                                    tc::pack_bf16(S[8 * c8 + 4], S[8 * c8 + 5]), tc::pack_bf16(S[8 * c8 + 6], S[8 * c8 + 7]));
-      sts16(Sop, tc::mnmajor_unit(kk, NC / 8 * half + c8, NV), val);
+      sts16(Sop, tc::colblk_unit(kk, NC / 8 * half + c8, KD), val);
     }
-    if (tid < NST) tc::bulk_wait_read<0>();  // the previous chunk's v_new image has left its tile
-    if (!TMA) tc::cp_async_wait<5>();  // group A of this chunk has landed (q rows; the images on the barrier)
-    if (ok) ok = tc::mbar_wait(&mbar[1 + buf], lph);
+    if (!TMA) tc::cp_async_wait<3>();  // q rows of this chunk (groups since: k of it, q and k of the next, k of the third)
     tc::fence_async_smem();
     tc::fence_before_sync();
     ok = __syncthreads_and(ok);  // the barrier also makes the verdict of the bounded waits uniform, so that all
     if (!ok) break;              // threads leave the loop together
     tc::fence_after_sync();
-    if (tid == 0) {  // D1 = [w;q] S
-      tc::issue_gemm(taddr, tc::kmajor_sw128_tile(A1c, 16384), tc::mnmajor_tile(Sop, NV), 128, NV, KD, false);
-      tc::mma_commit(mbar);
-    }
-    if (p.save && tid < NST) {  // the state at chunk start, saved for the backward as the byte image of the operand tile
-      tc::bulk_store(p.hs + ci * KD * KD + tid * 8 * KD + 8 * col0, tc::smem_u32(Sop) + tid * 16 * NV, 256 * NV / NST);
-      tc::bulk_commit();
-    }
-    if (TMA && tid == kOutThread && c > 0) {  // the previous chunk's output tile (complete since the barrier above)
-      for (int sl = 0; sl < NV / 64; ++sl)  // a slab that lies wholly past the true width is not stored at all
-        if (col0 + 64 * sl < p.Dv) tc::tma_store_4d(&maps.o, sOt + sl * 8192, col0 + 64 * sl, h, t0 - C, b);
-      tc::bulk_commit();
-    }
-    // In the shadow of the MMA: k <- diag(r) k in place, so that the state update contracts it with v_new itself
-    // (every thread scales the 16-byte units it would copy in the cp.async variant: no barrier needed for those)
-    if (!TMA) tc::cp_async_wait<3>();
-    if (ok) ok = tc::mbar_wait(&mbar[5 + buf], lph);  // P image and k rows of this chunk
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int u = tid + 256 * m, i = urow16(u);
-      uint4* unit = reinterpret_cast<uint4*>(A3c + tc::sw128_unit(i, ucol16(u)));
-      *unit = tc::scale_bf16x8(*unit, rr[i]);
-    }
+    // in the shadow of [w;q] S: the output of the chunk before, the decay factors of the chunk after
+    if (c > 0) put_out(c - 1);
+    decay(c + 1);
+    if (ok) ok = tc::mbar_wait(&mbar[3 + buf], lph);  // u image of this chunk
     if (ok) ok = tc::mbar_wait(mbar, ph);
     ph ^= 1;
     tc::fence_after_sync();
-    issue_A(c + 2);
-    if (ok) ok = tc::mbar_wait(&mbar[3 + buf], lph);  // u image of this chunk
-    float f[NC];  // accumulator row; rows 64-127 keep E(gam_i) (q S) here until P v_new arrives
+    copy_q(c + 2);
     if (ok) {
       const int i = kk & 63;
       ld_accN(taddr + j0, warp, f);
@@ -507,85 +594,46 @@ __global__ void __launch_bounds__(256) gdn_tc_state_fwd_kernel(TcP p, const __gr
 #pragma unroll
         for (int x = 0; x < NC / 8; ++x) {
           const int c8 = NC / 8 * half + x;
-          const uint4 uu = *reinterpret_cast<const uint4*>(Utc + tc::kmajor_unit(i, c8, NV));
+          const uint4 uu = *reinterpret_cast<const uint4*>(Ut + buf * 128 * NV + tc::colblk_unit(i, c8, C));
           float e[8];
           tc::unpack_bf16(uu.x, e[0], e[1]); tc::unpack_bf16(uu.y, e[2], e[3]);
           tc::unpack_bf16(uu.z, e[4], e[5]); tc::unpack_bf16(uu.w, e[6], e[7]);
 #pragma unroll
           for (int y = 0; y < 8; ++y) e[y] -= f[8 * x + y];
-          sts16(Vn, tc::mnmajor_unit(i, c8, NV), make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]),
-                                                            tc::pack_bf16(e[4], e[5]), tc::pack_bf16(e[6], e[7])));
+          sts16(Vn, tc::colblk_unit(i, c8, C), make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]),
+                                                          tc::pack_bf16(e[4], e[5]), tc::pack_bf16(e[6], e[7])));
         }
       } else {
-        const float di = dd[i];
+        const float di = dd[buf * C + i];
 #pragma unroll
         for (int jj = 0; jj < NC; ++jj) f[jj] *= di;
       }
     }
-    if (tid < NST) tc::bulk_wait_read<0>();  // the state image has left its tile
-    if (TMA && tid == kOutThread) tc::bulk_wait_read<0>();  // the previous output tile has left its tile
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
-    tc::fence_after_sync();
-    issue_U(c + 2);  // u has been consumed by every thread
-    if (ok && tid == 0) {
-      // D2 = [0;P] v_new          D3 = (r k)^T v_new
-      tc::issue_gemm(taddr + 128, tc::kmajor_tile(A2c, C), tc::mnmajor_tile(Vn, NV), 128, NV, C, false);
-      tc::issue_gemm(taddr + 256, tc::mnmajor_sw128_tile(A3c, 8192), tc::mnmajor_tile(Vn, NV), 128, NV, C, false);
-      tc::mma_commit(mbar);
-    }
-    if (ok && p.save && tid < (NST + 1) / 2) {
-      tc::bulk_store(p.vn + ci * C * KD + tid * 8 * KD + 8 * col0, tc::smem_u32(Vn) + tid * 16 * NV, 256 * NV / (NST + (NST & 1)));
-      tc::bulk_commit();
+    if (c + 1 < p.n) {
+      if (!TMA) tc::cp_async_wait<2>();  // k of the next chunk (groups since: k of the third, q of the third)
+      scale_k(c + 1);
     }
     if (ok) {
       ok = tc::mbar_wait(mbar, ph);
       ph ^= 1;
     }
     tc::fence_after_sync();
-    issue_PK(c + 2);
+    copy_k(c + 3);
     if (ok) {
-      const int i = kk & 63;
       float a[NC];
-      if (kk >= 64) {  // out = E(gam)(q S) + P v_new      (warp-uniform branch)
-        ld_accN(taddr + 128 + j0, warp, a);
-        if (TMA) {     // into the swizzled output tile; one thread hands it to the copy engine after the next barrier
-#pragma unroll
-          for (int x = 0; x < NC / 8; ++x)
-            sts16(Ot, tc::sw128_unit(i, NC / 8 * half + x),
-                  make_uint4(tc::pack_bf16(f[8 * x] + a[8 * x], f[8 * x + 1] + a[8 * x + 1]),
-                             tc::pack_bf16(f[8 * x + 2] + a[8 * x + 2], f[8 * x + 3] + a[8 * x + 3]),
-                             tc::pack_bf16(f[8 * x + 4] + a[8 * x + 4], f[8 * x + 5] + a[8 * x + 5]),
-                             tc::pack_bf16(f[8 * x + 6] + a[8 * x + 6], f[8 * x + 7] + a[8 * x + 7])));
-        } else if (i < imax) {
-          uint4* dst = reinterpret_cast<uint4*>(p.out + grow(c, i) * KD + j0);
-#pragma unroll
-          for (int x = 0; x < NC / 8; ++x)
-            dst[x] = make_uint4(tc::pack_bf16(f[8 * x] + a[8 * x], f[8 * x + 1] + a[8 * x + 1]),
-                                tc::pack_bf16(f[8 * x + 2] + a[8 * x + 2], f[8 * x + 3] + a[8 * x + 3]),
-                                tc::pack_bf16(f[8 * x + 4] + a[8 * x + 4], f[8 * x + 5] + a[8 * x + 5]),
-                                tc::pack_bf16(f[8 * x + 6] + a[8 * x + 6], f[8 * x + 7] + a[8 * x + 7]));
-        }
-      }
       ld_accN(taddr + 256 + j0, warp, a);  // S <- E(gam_last) S + (r k)^T v_new
 #pragma unroll
       for (int jj = 0; jj < NC; ++jj) S[jj] = fmaf(L, S[jj], a[jj]);
     }
     tc::fence_before_sync();
   }
-  if (!TMA) tc::cp_async_wait<0>();
-  if (TMA) {  // the last chunk's output tile
-    tc::fence_async_smem();
-    __syncthreads();
-    if (ok && tid == kOutThread) {
-      for (int sl = 0; sl < NV / 64; ++sl)
-        if (col0 + 64 * sl < p.Dv) tc::tma_store_4d(&maps.o, sOt + sl * 8192, col0 + 64 * sl, h, (p.n - 1) * C, b);
-      tc::bulk_commit();
-    }
-    if (tid == kOutThread) tc::bulk_wait_read<0>();
-  }
-  if (tid < NST) tc::bulk_wait_read<0>();  // shared memory must outlive the copies
+  __syncthreads();  // the output tile is free
+  put_out(p.n - 1);
+  tc::fence_async_smem();
+  __syncthreads();
   if (!ok && tid == 0) atomicExch(p.status, 2);
   if (ok && p.hT && kk < p.Dk) {
     float4* dst = reinterpret_cast<float4*>(p.hT + ((size_t)bh * p.Dk + kk) * p.Dv + col0 + j0);
@@ -719,7 +767,7 @@ mxb_status tc_run_fwd(TcP& p, cudaStream_t st) {
     constexpr int NV = decltype(nv)::value;
     if (MXB_ALLOW_SMEM(kStateFwdSmem<NV>, gdn_tc_state_fwd_kernel<TMA, NV>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_state_fwd_kernel", st,
-               (gdn_tc_state_fwd_kernel<TMA, NV><<<dim3(p.B * p.H, (p.Dv + NV - 1) / NV), 256, kStateFwdSmem<NV>, st>>>(p, maps)));
+               (gdn_tc_state_fwd_kernel<TMA, NV><<<dim3(p.B * p.H, (p.Dv + NV - 1) / NV), kStateThreads<NV>, kStateFwdSmem<NV>, st>>>(p, maps)));
     return MXB_OK;
   };
   if (!tma) s = state(std::false_type{}, std::integral_constant<int, KD>{});

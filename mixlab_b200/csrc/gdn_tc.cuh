@@ -56,21 +56,6 @@ struct alignas(64) RowMaps {
   CUtensorMap k, q, v, dO, o, dq, dk, dv;
 };
 
-// Views of a [64][128] tile for tcgen05 and for 16-byte unit access: written by the copy engine with 128-byte
-// swizzle (SW = true: two 8 KB slabs of 64 columns) or staged un-swizzled in the blocked layout.
-template <bool SW>
-__device__ __forceinline__ tc::Tile in_kmajor(const void* ptr) {
-  return SW ? tc::kmajor_sw128_tile(ptr, 8192) : tc::kmajor_tile(ptr, KD);
-}
-template <bool SW>
-__device__ __forceinline__ tc::Tile in_mnmajor(const void* ptr) {
-  return SW ? tc::mnmajor_sw128_tile(ptr, 8192) : tc::mnmajor_tile(ptr, KD);
-}
-template <bool SW>
-__device__ __forceinline__ uint32_t in_unit(int r, int c8) {
-  return SW ? tc::sw128_unit(r, c8) : tc::kmajor_unit(r, c8, KD);
-}
-
 __device__ __forceinline__ float log_gate_tc(float g, int gate_is_log) {
   return gate_is_log ? fmaxf(g, kLogGateFloor) : __logf(fmaxf(g, kGateFloor));
 }
@@ -114,9 +99,16 @@ __device__ __forceinline__ void for_acc2x32(uint32_t taddr, int warp, int c0, F&
   process(c0 + 32, f);
 }
 // The sequential passes of 128-wide heads take half of the state's columns per CTA where that still puts every CTA on an
-// SM of its own: the chain of a chunk is what counts then, not the bytes (16 heads, 24 chunks: 65 -> 56 us
-// forward).
+// SM of its own: the chain of a chunk is what counts then, not the bytes (forward and backward, us a chunk: 2.55 and 2.4
+// with all columns, 1.9 and 1.8 with half of them).
 inline bool tc_split_columns(const TcP& p) { return p.Dv > 64 && 2 * p.B * p.H <= 148; }
+
+// Threads of a forward state-pass CTA: 256 that hold the state and run the epilogues, and a warp of one issuing thread (on
+// a thread with an epilogue of its own, 70 cycles per product made that thread's warp the one all others waited for: 2.4
+// -> 1.9 us a chunk with NV = 64, 2.8 -> 2.55 with 128).  With 128 columns per CTA that warp is a warpgroup, so that
+// registers can be moved to the others: 8 x 216 + 4 x 40 registers a lane, of 12 x 168 at launch.
+template <int NV>
+constexpr int kStateThreads = NV == KD ? 384 : 288;
 
 // Loads 64 fp32 accumulator columns [0, 64) at taddr of this thread's TMEM lane: both loads in flight, one wait.
 __device__ __forceinline__ void ld_acc64(uint32_t taddr, int warp, float (&f)[64]) {

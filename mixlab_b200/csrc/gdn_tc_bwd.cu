@@ -26,13 +26,18 @@
 
 namespace mxb {
 
-// One CTA (256 threads) per (batch, head); thread t owns row kk = t & 127 of dS and the 64
+// One CTA (256 threads) per (batch, head) and NV columns; thread t owns row kk = t & 127 of dS and the
 // columns of half t >> 7.  Chunks run in reverse.  The operand tiles are double-buffered (buffer c & 1 for
-// chunk c) and requested two chunks ahead, as soon as the MMA batch that last read the buffer has completed:
-//   group A  k, dO, q rows and the P image   free after the first MMA batch
-//   group B  the w image                     free after the second MMA batch
-// q is scaled in place to diag(E(gam)) q one chunk early, in the shadow of the second MMA batch, so that the
-// first batch contracts it with the raw dO tile:  dS <- E(gam_last) dS + (d q)^T dO - w^T dv_new.
+// chunk c) and requested two chunks ahead, as soon as the products that last read the buffer have completed:
+//   group A  k, dO, q rows and the P image   free after k dS
+//   group B  the w image                     free after w^T dv_new
+// q is scaled in place to diag(E(gam)) q, so that it is contracted with the raw dO tile:
+//   dv_new = diag(r) k dS + P^T dO,   dS <- E(gam_last) dS + (d q)^T dO - w^T dv_new.
+//
+// Bound by the chain dS -> k dS -> dv_new -> w^T dv_new -> dS where the heads are few, by HBM where they fill the GPU.
+// P^T dO and (d q)^T dO need no dS: those of chunk c-1 are issued behind w^T dv_new of chunk c and run while dS is
+// updated, and q is scaled in the shadow of the k dS before (16 heads of 128, NV = 64: 2.6 -> 1.8 us a chunk).
+// (An issuing warp of its own, as in the forward pass, was slower here: 1.8 -> 2.1 us.)
 //
 // TMA = true: the k, dO and q rows arrive as tensor-map boxes (128-byte swizzle, two 8 KB slabs of 64 columns per
 // tile) issued by one thread on the barrier of group A; TMA = false: by cp.async into the same swizzled positions
@@ -46,7 +51,6 @@ template <bool TMA, int NV>
 __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
   static_assert(NV == KD || TMA, "the per-thread staging moves whole rows");
   constexpr int NC = NV / 2;                   // columns per thread
-  constexpr int NST = NV == KD ? 1 : 16;       // pieces of a state image in the workspace (rows of eight, NV columns)
   const int col0 = blockIdx.y * NV;
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
@@ -144,22 +148,30 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
 #pragma unroll
     for (int x = 0; x < NC; ++x) dS[x] = 0.f;
   }
-  // in-chunk cumulative log decay: this chunk's, and the next (earlier) one's fetched a chunk early
+  // Decay factors: rr of the chunk ahead and ddn of the one after it, computed in the shadow of w^T dv_new.
   const size_t gbase = (size_t)bh * p.n * C;
-  float g_cur = p.gam[gbase + (size_t)(p.n - 1) * C + (tid & 63)], gl_cur = p.gam[gbase + (size_t)(p.n - 1) * C + C - 1];
-  float g_nxt = 0.f, gl_nxt = 0.f;
-  if (p.n > 1) {
-    g_nxt = p.gam[gbase + (size_t)(p.n - 2) * C + (tid & 63)];
-    gl_nxt = p.gam[gbase + (size_t)(p.n - 2) * C + C - 1];
+  auto gam_at = [&](int c) { return c >= 0 ? p.gam[gbase + (size_t)c * C + (tid & 63)] : 0.f; };
+  auto gam_end = [&](int c) { return c >= 0 ? p.gam[gbase + (size_t)c * C + C - 1] : 0.f; };
+  float gl_cur = gam_end(p.n - 1), g_nxt = gam_at(p.n - 2), gl_nxt = gam_end(p.n - 2);
+  if (tid < C) {
+    const float g = gam_at(p.n - 1);
+    rr[tid] = exp_nonpos(gl_cur - g);
+    ddn[((p.n - 1) & 1) * C + tid] = exp_nonpos(g);
+    ddn[(p.n & 1) * C + tid] = exp_nonpos(g_nxt);
   }
-  if (tid < C) ddn[((p.n - 1) & 1) * C + tid] = exp_nonpos(g_cur);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t taddr = *tslot;
   uint32_t ph = 0;
   bool ok = true;
-  {  // the last chunk's q is scaled here; every later one in the shadow of the previous iteration's second batch
+  // P^T dO and (d q)^T dO of chunk c (accumulators at 128 and at 256 or 384)
+  auto issue_dO = [&](int c) {
+    const tc::Tile dO = tc::mnmajor_sw128_tile(dOop + (c & 1) * 128 * NV, 8192);
+    tc::issue_gemm(taddr + 128, tc::mnmajor_tile(Pt + (c & 1) * 8192, C), dO, 64, NV, C, false);
+    tc::issue_gemm(taddr + 256 + 128 * (c & 1), tc::mnmajor_sw128_tile(Aq + (c & 1) * 16384, 8192), dO, 128, NV, C, false);
+  };
+  {  // the last chunk's q is scaled here; every later one a chunk ahead
     const int c = p.n - 1;
     if (!TMA) tc::cp_async_wait<2>();
     ok = tc::mbar_wait(&mbar[1 + (c & 1)], 0);
@@ -170,42 +182,34 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
     const size_t ci = (size_t)bh * p.n + c;
     const int buf = c & 1;
     const uint32_t lph = ((p.n - 1 - c) >> 1) & 1;  // phase of this buffer's barriers
-    const float glast = gl_cur, g = g_cur;
-    g_cur = g_nxt; gl_cur = gl_nxt;
-    if (c > 1) {
-      g_nxt = p.gam[(ci - 2) * C + (tid & 63)];
-      gl_nxt = p.gam[(ci - 2) * C + C - 1];
-    }
-    const float L = exp_nonpos(glast);
-    if (tid < C) {
-      rr[tid] = exp_nonpos(glast - g);
-      if (c > 0) ddn[(buf ^ 1) * C + tid] = exp_nonpos(g_cur);  // for the next chunk's q
-    }
+    const float L = exp_nonpos(gl_cur);
+    const float g_far = gam_at(c - 2), gl_far = gam_end(c - 2);
 #pragma unroll
     for (int c8 = 0; c8 < NC / 8; ++c8) {  // dS at chunk end: MMA operand + saved for the chunk kernel
       const uint4 val = make_uint4(tc::pack_bf16(dS[8 * c8], dS[8 * c8 + 1]), tc::pack_bf16(dS[8 * c8 + 2], dS[8 * c8 + 3]),
                                    tc::pack_bf16(dS[8 * c8 + 4], dS[8 * c8 + 5]), tc::pack_bf16(dS[8 * c8 + 6], dS[8 * c8 + 7]));
-      sts16(dSop, tc::mnmajor_unit(kk, NC / 8 * half + c8, NV), val);
+      sts16(dSop, tc::colblk_unit(kk, NC / 8 * half + c8, KD), val);
     }
-    if (tid < NST) tc::bulk_wait_read<0>();  // the previous chunk's -dv_new image has left its tile
-    // group A of this chunk was waited for when its q was scaled (previous iteration / prologue)
+    if (tid == 0) tc::bulk_wait_read<0>();  // the previous chunk's -dv_new image has left its tile
     tc::fence_async_smem();
     tc::fence_before_sync();
     ok = __syncthreads_and(ok);  // the barrier also makes the verdict of the bounded waits uniform, so that all
     if (!ok) break;              // threads leave the loop together
     tc::fence_after_sync();
     if (tid == 0) {
-      tc::issue_gemm(taddr, tc::kmajor_sw128_tile(Ak + buf * 16384, 8192), tc::mnmajor_tile(dSop, NV), 64, NV, KD, false);  // k dS
-      tc::issue_gemm(taddr + 128, tc::mnmajor_tile(Pt + buf * 8192, C), tc::mnmajor_sw128_tile(dOop + buf * 128 * NV, 8192), 64, NV,
-                     C, false);                                                                                           // P^T dO
-      tc::issue_gemm(taddr + 256, tc::mnmajor_sw128_tile(Aq + buf * 16384, 8192), tc::mnmajor_sw128_tile(dOop + buf * 128 * NV, 8192),
-                     128, NV, C, false);                                                                                  // (d q)^T dO
+      if (c == p.n - 1) issue_dO(c);
+      tc::issue_gemm(taddr, tc::kmajor_sw128_tile(Ak + buf * 16384, 8192), tc::colblk_mnmajor_tile(dSop, KD), 64, NV, KD, false);  // k dS
       tc::mma_commit(mbar);
-    }
-    if (tid < NST) {  // dS at chunk end, as the operand-tile image
-      tc::bulk_store(p.dhs + ci * KD * KD + tid * 8 * KD + 8 * col0, tc::smem_u32(dSop) + tid * 16 * NV, 256 * NV / NST);
+      // dS at chunk end, as the operand-tile image
+      tc::bulk_store(p.dhs + ci * KD * KD + KD * col0, tc::smem_u32(dSop), 256 * NV);
       tc::bulk_commit();
     }
+    if (c > 0) {  // in the shadow of that product: the next chunk's q (its group was requested a chunk ago)
+      if (!TMA) tc::cp_async_wait<1>();
+      ok = tc::mbar_wait(&mbar[1 + (buf ^ 1)], ((p.n - c) >> 1) & 1);
+      scale_q(c - 1);
+    }
+    if (ok) ok = tc::mbar_wait(&mbar[3 + buf], lph);  // w image of this chunk
     if (ok) ok = tc::mbar_wait(mbar, ph);
     ph ^= 1;
     tc::fence_after_sync();
@@ -224,31 +228,31 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
 #pragma unroll
             for (int y = 0; y < 8; ++y) e[y] = -fmaf(ri, fa[8 * x + y], fb[8 * x + y]);
             const int c8 = NC / 8 * half + (c0 >> 3) + x;
-            sts16(Bd, tc::kmajor_unit(i, c8, NV), make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]),
+            sts16(Bd, tc::colblk_unit(i, c8, C), make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]),
                                                              tc::pack_bf16(e[4], e[5]), tc::pack_bf16(e[6], e[7])));
           }
         }
       }
     }
-    if (tid < NST) tc::bulk_wait_read<0>();  // the dS image has left its tile
-    if (ok) ok = tc::mbar_wait(&mbar[3 + buf], lph);  // w image of this chunk
+    if (tid == 0) tc::bulk_wait_read<0>();  // the dS image has left its tile
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     if (ok && tid == 0) {  // ... - w^T dv_new
-      tc::issue_gemm(taddr + 256, tc::mnmajor_sw128_tile(Aw + buf * 16384, 8192), tc::mnmajor_tile(Bd, NV), 128, NV, C, true);
+      tc::issue_gemm(taddr + 256 + 128 * buf, tc::mnmajor_sw128_tile(Aw + buf * 16384, 8192), tc::colblk_mnmajor_tile(Bd, C), 128, NV, C,
+                     true);
       tc::mma_commit(mbar);
-    }
-    if (ok && tid < (NST + 1) / 2) {  // -dv_new as the operand-tile image
-      tc::bulk_store(p.dvn + ci * C * KD + tid * 8 * KD + 8 * col0, tc::smem_u32(Bd) + tid * 16 * NV, 256 * NV / (NST + (NST & 1)));
+      if (c > 0) issue_dO(c - 1);  // (completes with the next commit)
+      // -dv_new as the operand-tile image
+      tc::bulk_store(p.dvn + ci * C * KD + C * col0, tc::smem_u32(Bd), 128 * NV);
       tc::bulk_commit();
     }
-    if (c > 0) {  // in the shadow of the MMA: the next chunk's q (its group landed a chunk ago)
-      if (!TMA) tc::cp_async_wait<2>();
-      if (ok) ok = tc::mbar_wait(&mbar[1 + (buf ^ 1)], ((p.n - c) >> 1) & 1);
-      scale_q(c - 1);
+    if (tid < C && c > 0) {
+      rr[tid] = exp_nonpos(gl_nxt - g_nxt);
+      ddn[buf * C + tid] = exp_nonpos(g_far);
     }
+    gl_cur = gl_nxt; g_nxt = g_far; gl_nxt = gl_far;
     if (ok) {
       ok = tc::mbar_wait(mbar, ph);
       ph ^= 1;
@@ -257,14 +261,14 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
     issue_B(c - 2);
     if (ok) {
       float a[NC];
-      ld_accN(taddr + 256 + j0, warp, a);
+      ld_accN(taddr + 256 + 128 * buf + j0, warp, a);
 #pragma unroll
       for (int jj = 0; jj < NC; ++jj) dS[jj] = fmaf(L, dS[jj], a[jj]);
     }
     tc::fence_before_sync();
   }
   if (!TMA) tc::cp_async_wait<0>();
-  if (tid < NST) tc::bulk_wait_read<0>();  // shared memory must outlive the copies
+  if (tid == 0) tc::bulk_wait_read<0>();  // shared memory must outlive the copies
   if (!ok && tid == 0) atomicExch(p.status, 3);
   if (ok && p.dh0 && kk < p.Dk) {
     float4* dst = reinterpret_cast<float4*>(p.dh0 + ((size_t)bh * p.Dk + kk) * p.Dv + col0 + j0);
@@ -398,8 +402,8 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   uint32_t ph = 0;
   // ---- batch 1: -e = T^T (-dv_new) (both operands contracted over their rows), dP = dO v_new^T ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tA, tc::mnmajor_tile(Xt, C), tc::mnmajor_tile(Xe, KD), 64, 128, C, false);
-    tc::issue_gemm(tB, tc::kmajor_sw128_tile(XdO, 8192), tc::kmajor_tile(Xvn, KD), 64, 64, KD, false);
+    tc::issue_gemm(tA, tc::mnmajor_tile(Xt, C), tc::colblk_mnmajor_tile(Xe, C), 64, 128, C, false);
+    tc::issue_gemm(tB, tc::kmajor_sw128_tile(XdO, 8192), tc::colblk_kmajor_tile(Xvn, C), 64, 64, KD, false);
     tc::mma_commit(mbar);
   }
   __syncthreads();  // dd, rr visible
@@ -446,8 +450,8 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   tc::fence_after_sync();
   // ---- batch 2: DQ = (d dO) S0^T, z = (-e) S0^T ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tA, tc::kmajor_sw128_tile(XdO, 8192), tc::kmajor_tile(R1, KD), 64, 128, KD, false);
-    tc::issue_gemm(tB, tc::kmajor_sw128_tile(Xe, 8192), tc::kmajor_tile(R1, KD), 64, 128, KD, false);
+    tc::issue_gemm(tA, tc::kmajor_sw128_tile(XdO, 8192), tc::colblk_kmajor_tile(R1, KD), 64, 128, KD, false);
+    tc::issue_gemm(tB, tc::kmajor_sw128_tile(Xe, 8192), tc::colblk_kmajor_tile(R1, KD), 64, 128, KD, false);
     tc::mma_commit(mbar);  // one commit: z overwrites d dO and dS overwrites S0, which DQ reads as well
   }
   uint4 s0u[8];  // this thread's 8 units of S0, kept for <dS, S0> (the buffer is about to be reused)
@@ -478,7 +482,7 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   tc::fence_after_sync();
   // ---- batch 3: v_new dS^T ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tB, tc::kmajor_tile(Xvn, KD), tc::kmajor_tile(R1, KD), 64, 128, KD, false);
+    tc::issue_gemm(tB, tc::colblk_kmajor_tile(Xvn, C), tc::colblk_kmajor_tile(R1, KD), 64, 128, KD, false);
     tc::mma_commit(mbar);
   }
   {  // <dS, S0>

@@ -106,6 +106,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint3
   return false;
 }
 
+// Registers per thread of a warpgroup (every warp of it calls this), given back to or taken from the block's own.
+template <int N>
+__device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // ---- TMEM -> registers: 32 lanes x 32-bit, N consecutive columns; thread l of warp w
 // reads TMEM lane 32*(w%4)+l.  taddr = (lane << 16) | column.
 __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[32]) {

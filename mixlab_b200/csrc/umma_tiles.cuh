@@ -8,6 +8,9 @@
 // the natural row-major layout of an operand whose contraction runs over rows):
 //   byte(k, m) = (m/8)*128 + (k/8)*LBO + (k%8)*16 + (m%8)*2,  SBO = 128, LBO = (MN/8)*128
 //   one MMA K-step advances the start address by 2*LBO bytes.
+// Column-blocked tile X[R rows][cols]: all rows of eight columns, then the next eight columns, so that a range of columns
+// is one contiguous piece of memory (contraction along the columns or, MN-major view, along the rows):
+//   byte(r, c) = (c/8)*R*16 + r*16 + (c%8)*2
 #pragma once
 
 #include "tcgen05.cuh"
@@ -30,6 +33,13 @@ __device__ __forceinline__ Tile kmajor_tile(const void* smem, int kcols) {
 __device__ __forceinline__ Tile mnmajor_tile(const void* smem, int mn) {
   const uint32_t lbo = (uint32_t)(mn / 8) * 128u;
   return Tile{smem_u32(smem), lbo, 128u, 2u * lbo, 1};
+}
+__device__ __forceinline__ Tile colblk_kmajor_tile(const void* smem, int rows) {
+  const uint32_t block = (uint32_t)rows * 16u;
+  return Tile{smem_u32(smem), block, 128u, 2u * block, 0};
+}
+__device__ __forceinline__ Tile colblk_mnmajor_tile(const void* smem, int rows) {
+  return Tile{smem_u32(smem), 128u, (uint32_t)rows * 16u, 256u, 1};
 }
 // Tiles written by TMA with 128-byte swizzle: slabs of [rows][64 bf16] (128-byte rows, 8-row groups
 // 1024 bytes apart), slab s holding columns 64 s .. 64 s + 63; slabs are slab_bytes apart and 1024-byte
@@ -59,6 +69,8 @@ __device__ __forceinline__ Tile skip_k(Tile t, int k0) { t.saddr += (uint32_t)(k
 __device__ __forceinline__ uint32_t kmajor_unit(int r, int c8, int kcols) {
   return (uint32_t)(r >> 3) * (uint32_t)(kcols / 8) * 128u + (uint32_t)c8 * 128u + (uint32_t)(r & 7) * 16u;
 }
+// ... of a column-blocked tile.
+__device__ __forceinline__ uint32_t colblk_unit(int r, int c8, int rows) { return (uint32_t)(c8 * rows + r) * 16u; }
 // Byte offset of the 16-byte unit holding elements (r, 8*c8 .. 8*c8+7) of a 64-row tile written by TMA with
 // 128-byte swizzle (8 KB slabs of 64 columns, 1024-byte aligned): the unit index within a 128-byte row is
 // XORed with the row's position in its 8-row group.
