@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(kStateThreads<NV>, 1) gdn_tc_state_fwd_kernel(
 
   const int tid = threadIdx.x, warp = tid >> 5;
   const int kk = tid & 127, half = tid >> 7, j0 = NC * half;  // (of the 256 threads of warps 0-7)
-  const bool lead = tid == 256;  // issues the products and the copies
+  auto lead = [&] { return warp == 8 && tc::elect_one(); };  // issues the products and the copies
   const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
   const uint32_t sA1b = tc::smem_u32(A1), sPb = tc::smem_u32(Pm), sA3b = tc::smem_u32(A3), sUb = tc::smem_u32(Ut);
   const uint32_t sOt = tc::smem_u32(Ot);
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(kStateThreads<NV>, 1) gdn_tc_state_fwd_kernel(
     tc::tmem_alloc(tslot, 512);
     tc::tmem_relinquish();
   }
-  if (lead) {
+  if (lead()) {
     for (int m = 0; m < 11; ++m) tc::mbar_init(&mbar[m], 1);
     tc::mbar_fence_init();
     for (int c = 0; c < 2; ++c) {
@@ -429,13 +429,13 @@ __global__ void __launch_bounds__(kStateThreads<NV>, 1) gdn_tc_state_fwd_kernel(
       const size_t ci = (size_t)bh * p.n + c;
       const int buf = c & 1;
       const uint32_t lph = (c >> 1) & 1;  // phase of the image barriers of this buffer
-      if (lead) {
+      if (lead()) {
         tc::bulk_wait_read<0>();  // v_new and the output tile of the chunk before have left
         ok = tc::mbar_wait(&mbar[1 + buf], lph);
       }
       ok = __syncthreads_and(ok);
       if (!ok) break;
-      if (lead) {
+      if (lead()) {
         tc::fence_after_sync();
         // D1 = [w;q] S
         tc::issue_gemm(taddr, tc::kmajor_sw128_tile(A1 + buf * 32768, 16384), tc::colblk_mnmajor_tile(Sop, KD), 128, NV, KD, false);
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(kStateThreads<NV>, 1) gdn_tc_state_fwd_kernel(
       }
       ph ^= 1;
       __syncthreads();
-      if (lead && ok) {
+      if (lead() && ok) {
         tc::fence_after_sync();
         // D3 = (r k)^T v_new, which the next chunk waits for, then P v_new into rows 64-127 of D2: the tile is the 128 rows
         // that end with P; what the 64 rows before it hold (other tiles) only reaches rows of D2 that nothing reads
@@ -472,10 +472,10 @@ __global__ void __launch_bounds__(kStateThreads<NV>, 1) gdn_tc_state_fwd_kernel(
       }
       ph ^= 1;
     }
-    if (lead) tc::bulk_wait_read<0>();
+    if (lead()) tc::bulk_wait_read<0>();
     __syncthreads();  // the output tile is free
     __syncthreads();  // and full
-    if (lead) {
+    if (lead()) {
       if (ok) {
         store_out(p.n - 1);
         tc::bulk_commit();
