@@ -49,7 +49,7 @@ struct SsdP {
   float *dphi, *da, *de, *dgam; // [B,NH,T] per-token scalar gradients
   float* dal_part;              // [B,NH] per-batch shares of da_log
   float* cs;                    // [B,NH,n] ChunkScal records
-  bf16 *pb, *pc;                // [B,NH,T,N] per-head partial dB, dC (summed in fp32 by the reduce kernel)
+  bf16 *pb, *pc;                // [B,NH,n] column-blocked [64][128] images: per-head partial dB, dC (summed in fp32 by the reduce kernel)
 };
 
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : (x < -20.f ? expf(x) : log1pf(expf(x))); }
@@ -479,9 +479,12 @@ __global__ void __launch_bounds__(256) m3s_state_pass_kernel(SsdP p, int mode, c
 }
 
 // ------------------------------------------------------------ chunk output
-// A CTA is a chain of dependent steps, so the kernel is sized for FOUR CTAs per SM: 128 TMEM columns and 51 KB of
-// shared memory.  The chunk state H0 lands in the Brot tile once G = Crot Brot^T has been formed (its copy hides
-// behind the mask epilogue), and Crot H0 joins the second MMA batch.
+// A CTA is a chain of dependent steps, so the kernel is sized for FOUR CTAs per SM: 64 TMEM columns (weight-stationary
+// products: every thread has a row and half of the columns of a result) and 51 KB of shared memory.  The chunk state H0
+// lands in the Brot tile once G = Crot Brot^T has been formed (its copy hides behind the mask epilogue), and Crot H0
+// joins the second MMA batch.  Bound by shared memory (the copies, the rotation in place and the operand reads move
+// about 200 KB per chunk): 8 x 4096 x 32 heads 194 us with half of the lanes idle in the epilogues, 185 now; 256 threads
+// per CTA 188.
 constexpr int kOutSmem = 16384 * 2 + 8192 * 2 + sizeof(ChunkScal) + 64 + 1024;
 
 template <bool TMA>
@@ -501,7 +504,7 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
   const int d0 = head * P, g = d0 / (p.D / p.G);
   const size_t ci = ((size_t)b * p.NH + head) * p.n + c;
 
-  if (warp == 0) { tc::tmem_alloc(tslot, 128); tc::tmem_relinquish(); }
+  if (warp == 0) { tc::tmem_alloc(tslot, 64); tc::tmem_relinquish(); }
   // the thread that initialises the barriers also issues the copies, on another warp than the TMEM allocation
   if (tid == 32) {
     for (int m = 0; m < 3; ++m) tc::mbar_init(mbar + m, 1);
@@ -537,7 +540,7 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
   tc::fence_after_sync();
   const uint32_t taddr = *tslot;
   if (tid == 0) {
-    tc::issue_gemm(taddr, in_kmajor<TMA>(Ct, N), in_kmajor<TMA>(Bt, N), 64, Q, N, false);           // G = Crot Brot^T
+    tc::issue_gemm<true>(taddr, in_kmajor<TMA>(Ct, N), in_kmajor<TMA>(Bt, N), 64, Q, N, false);           // G = Crot Brot^T
     tc::mma_commit(mbar);
   }
   if (ok) ok = tc::mbar_wait(mbar, 0);
@@ -552,32 +555,26 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
     issue_state_tile(Ht, p.H0 + ci * (N * P));
     tc::cp_async_commit();
   }
-  const int t = 16 * warp + (lane & 15);
-  const bool own = lane < 16;
+  // weight-stationary products: this thread's row, and the half of the columns it holds of every result
+  const int t = 32 * (warp & 1) + lane, n0 = 32 * (warp >> 1);
   if (ok) {
-    // Lanes 16-31 hold no accumulator rows: they take over columns 32..63 of the row of lane - 16, so all 32
-    // lanes share the mask arithmetic (branch-free, so the exponentials of different columns overlap).
     const float lt = s.Lam[t], gt = s.gam[t];
-    const int hx = lane >> 4;
     float f[32];
-    {
-      float fa[32], fb[32];
-      ld_acc32(taddr, warp, 0, fa);
-      ld_acc32(taddr, warp, 32, fb);
+    ld_acc32(taddr, warp, 0, f);
 #pragma unroll
-      for (int q = 0; q < 32; ++q) {
-        const float up = __shfl_sync(0xffffffffu, fb[q], lane & 15);
-        f[q] = hx ? up : fa[q];
+    for (int x = 0; x < 8; ++x) {  // branch-free, so the exponentials of different columns overlap
+      const float4 l4 = *reinterpret_cast<const float4*>(s.Lam + n0 + 4 * x);
+      const float4 e4 = *reinterpret_cast<const float4*>(s.e + n0 + 4 * x);
+      const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, es[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const int jj = 4 * x + y, sx = n0 + jj;
+        const float mv = __expf(fminf(lt - ls[y], 0.f)) * (sx < t ? es[y] : gt);
+        f[jj] = (sx <= t) ? f[jj] * mv : 0.f;
       }
     }
 #pragma unroll
-    for (int jj = 0; jj < 32; ++jj) {
-      const int sx = 32 * hx + jj;
-      const float mv = __expf(fminf(lt - s.Lam[sx], 0.f)) * (sx < t ? s.e[sx] : gt);
-      f[jj] = (sx <= t) ? f[jj] * mv : 0.f;
-    }
-#pragma unroll
-    for (int x = 0; x < 4; ++x) sts16(Gm, tc::kmajor_unit(t, 4 * hx + x, Q), pack8(&f[8 * x]));
+    for (int x = 0; x < 4; ++x) sts16(Gm, tc::kmajor_unit(t, (n0 >> 3) + x, Q), pack8(&f[8 * x]));
   }
   if (TMA) { if (ok) ok = tc::mbar_wait(mbar + 2, 0); }  // H0
   else tc::cp_async_wait<0>();
@@ -586,25 +583,21 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
   __syncthreads();
   tc::fence_after_sync();
   if (ok && tid == 0) {
-    tc::issue_gemm(taddr, tc::kmajor_tile(Gm, Q), in_mnmajor<TMA>(Xt, P), 64, P, Q, false);  // (G*M) X, over the consumed G
-    tc::issue_gemm(taddr + 64, in_kmajor<TMA>(Ct, N), tc::mnmajor_tile(Ht, P), 64, P, N, false);    // Crot H0
+    tc::issue_gemm<true>(taddr, tc::kmajor_tile(Gm, Q), in_mnmajor<TMA>(Xt, P), 64, P, Q, false);  // (G*M) X, over the consumed G
+    tc::issue_gemm<true>(taddr + 32, in_kmajor<TMA>(Ct, N), tc::mnmajor_tile(Ht, P), 64, P, N, false);    // Crot H0
     tc::mma_commit(mbar);
   }
   if (ok) ok = tc::mbar_wait(mbar, 1);
   tc::fence_after_sync();
   if (ok) {  // y = (G*M) X + exp(Lam) Crot H0, assembled over the x tile (dead) and written out in full rows
     const float de = s.dexp[t];
-    for (int c0 = 0; c0 < P; c0 += 32) {
-      float f[32], f2[32];
-      ld_acc32(taddr, warp, c0, f);
-      ld_acc32(taddr + 64, warp, c0, f2);
-      if (own) {
+    float f[32], f2[32];
+    ld_acc32(taddr, warp, 0, f);
+    ld_acc32(taddr + 32, warp, 0, f2);
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) f[jj] = fmaf(de, f2[jj], f[jj]);
+    for (int jj = 0; jj < 32; ++jj) f[jj] = fmaf(de, f2[jj], f[jj]);
 #pragma unroll
-        for (int x = 0; x < 4; ++x) sts16(Xt, tc::kmajor_unit(t, (c0 >> 3) + x, P), pack8(&f[8 * x]));
-      }
-    }
+    for (int x = 0; x < 4; ++x) sts16(Xt, tc::kmajor_unit(t, (n0 >> 3) + x, P), pack8(&f[8 * x]));
   } else if (tid == 0) {
     atomicExch(p.status, 12);
   }
@@ -618,33 +611,34 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
             *reinterpret_cast<const uint4*>(Xt + 16 * u);
     }
   }
-  if (warp == 0) tc::tmem_dealloc(taddr, 128);
+  if (warp == 0) tc::tmem_dealloc(taddr, 64);
 }
 
 // ------------------------------------------------------------ chunk gradients
-// 256 TMEM columns and < 113 KB of shared memory, so two CTAs share an SM:
-//   phase 1: G [0,64), dY X^T [64,128), Crot H0 [128,192), Brot dH1 [192,256)
-//   phase 2: dx [0,64), dCrot [64,192)           (Brot dH1 still live in [192,256))
-//   phase 3: dBrot [0,128)
-// All accumulators are M=64: row i of every result is in TMEM lane (i%16)+32*(i/16); warps 0-3 take the
-// first half of the columns, warps 4-7 the second.  The G*M tile reuses the x tile once x is dead.
-constexpr int kGradSmem = 16384 * 4 + 8192 * 5 + sizeof(ChunkScal) + (4 * Q + 4 * Q + 8 * Q + 32) * 4 + 64 + 1024;
+// 256 TMEM columns and < 114 KB of shared memory, so two CTAs share an SM.  Every product with M = 64 is issued in the
+// weight-stationary form: all 128 TMEM lanes hold results, so that every thread has a row (t) and a quarter of the
+// columns (16 of 64, 32 of 128), and a result takes half of the TMEM columns:
+//   batch 1: G [0,32), dY X^T [32,64); then Crot H0 [64,96), Brot dH1 [96,128), (e^Lam dY) H0^T [192,256),
+//            (r e x) dH1^T [128,192)
+//   batch 2: dx [0,32), dCrot: += dG Brot [192,256); then dBrot: += dG^T Crot [128,192)
+// The G*M tile reuses the x tile once x is dead.  The column sums of dM*D*w that dLam needs are e_s (or gamma_s on the
+// diagonal) times those of dM*D, which de needs anyway.
+// Bound by the phases of a CTA that follow one another (HBM: 1.5 GB, 0.23 ms).  8 x 4096 x 32 heads: three batches with
+// half of the lanes idle in every epilogue 726 us, this 531 us.
+constexpr int kGradSmem = 16384 * 4 + 8192 * 5 + sizeof(ChunkScal) + (2 * Q + 16 * Q + 32) * 4 + 64 + 1024;
 
+// sum_k tile[r][c0 + k] f[k], 16 columns of a [.][64] tile
 template <bool SW>
-__device__ __forceinline__ float row_dot32_64(const uint8_t* tile, int r, int c0, const float (&f)[32]) {
-  // sum_k tile[r][c0 + k] f[k] for a [.][64] tile: four independent chains
-  uint4 raw[4];
+__device__ __forceinline__ float row_dot16_64(const uint8_t* tile, int r, int c0, const float (&f)[16]) {
+  float acc[2] = {0.f, 0.f};
 #pragma unroll
-  for (int x = 0; x < 4; ++x) raw[x] = *reinterpret_cast<const uint4*>(tile + in_unit<SW>(r, (c0 >> 3) + x, P));
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int x = 0; x < 4; ++x) {
+  for (int x = 0; x < 2; ++x) {
     float e[8];
-    unpack8(raw[x], e);
+    unpack8(*reinterpret_cast<const uint4*>(tile + in_unit<SW>(r, (c0 >> 3) + x, P)), e);
 #pragma unroll
     for (int y = 0; y < 8; ++y) acc[x] = fmaf(e[y], f[8 * x + y], acc[x]);
   }
-  return (acc[0] + acc[1]) + (acc[2] + acc[3]);
+  return acc[0] + acc[1];
 }
 
 template <bool TMA>
@@ -662,24 +656,24 @@ __global__ void __launch_bounds__(256) m3s_chunk_grad_kernel(SsdP p, const __gri
   uint8_t* GMt = Xt;               // [64][64]  G*M  (written after the last read of x)
   uint8_t* dGt = Ys + 8192;        // [64][64]  dG
   ChunkScal& s = *reinterpret_cast<ChunkScal*>(dGt + 8192);
-  float* csw_e = reinterpret_cast<float*>(&s + 1);  // [4][Q] per-warp column sums for de
-  float* csw_l = csw_e + 4 * Q;                     // [4][Q] per-warp column sums for dLam
-  float* part = csw_l + 4 * Q;                      // [2][4][Q]: per half: dLam, de, dgam, dphi row partials
-  float* red = part + 8 * Q;                        // [32]
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(red + 32);  // [0] MMA completion, [1] token tiles, [2] state images
+  float* csw = reinterpret_cast<float*>(&s + 1);    // [2][Q] column sums of dM*D (s < t) over the two halves of the rows
+  float* part = csw + 2 * Q;                        // [4][4][Q]: per column quarter: dLam, de, dgam, dphi row partials
+  float* red = part + 16 * Q;                       // [32]
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(red + 32);  // [0], [3] MMA completion, [1] token tiles, [2] state images
   uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 4);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int c = blockIdx.x, head = blockIdx.y, b = blockIdx.z, t0 = c * Q;
   const int d0 = head * P, g = d0 / (p.D / p.G);
   const size_t ci = ((size_t)b * p.NH + head) * p.n + c;
-  const bool own = lane < 16;
-  const int t = 16 * (warp & 3) + (lane & 15), hc = warp >> 2;
+  // this thread's row and column quarter of every result; tc16 / tc32: its TMEM columns of a [64][64] / [64][128] result
+  const int t = 32 * (warp & 1) + lane, qd = (warp & 2) + (warp >> 2), n16 = 16 * qd, n32 = 32 * qd;
+  const int tc16 = 16 * (warp >> 2), tc32 = 32 * (warp >> 2);
 
   if (warp == 0) { tc::tmem_alloc(tslot, 256); tc::tmem_relinquish(); }
   // the thread that initialises the barriers also issues the copies, on another warp than the TMEM allocation
   if (tid == 32) {
-    for (int m = 0; m < 3; ++m) tc::mbar_init(mbar + m, 1);
+    for (int m = 0; m < 4; ++m) tc::mbar_init(mbar + m, 1);
     tc::mbar_fence_init();
   }
   bool ok = true;
@@ -708,7 +702,6 @@ __global__ void __launch_bounds__(256) m3s_chunk_grad_kernel(SsdP p, const __gri
     issue_state_tile(Dt, p.dH1 + ci * (N * P));
     tc::cp_async_commit();
   }
-  for (int u = tid; u < 8 * Q; u += 256) { csw_e[u] = 0.f; }  // csw_e and csw_l are contiguous
   if (TMA) __syncthreads();  // barriers initialised before anyone waits on them
   if (TMA) ok = tc::mbar_wait(mbar + 1, 0);
   else tc::cp_async_wait<1>();
@@ -725,11 +718,14 @@ __global__ void __launch_bounds__(256) m3s_chunk_grad_kernel(SsdP p, const __gri
   tc::fence_after_sync();
   const uint32_t taddr = *tslot;
   if (tid == 0) {
-    tc::issue_gemm(taddr + 0, in_kmajor<TMA>(Ct, N), in_kmajor<TMA>(Bt, N), 64, Q, N, false);         // G
-    tc::issue_gemm(taddr + 64, in_kmajor<TMA>(Yt, P), in_kmajor<TMA>(Xt, P), 64, Q, P, false);        // dY X^T
-    tc::issue_gemm(taddr + 128, in_kmajor<TMA>(Ct, N), tc::mnmajor_tile(Ht, P), 64, P, N, false);     // Crot H0
-    tc::issue_gemm(taddr + 192, in_kmajor<TMA>(Bt, N), tc::mnmajor_tile(Dt, P), 64, P, N, false);     // Brot dH1
+    tc::issue_gemm<true>(taddr + 0, in_kmajor<TMA>(Ct, N), in_kmajor<TMA>(Bt, N), 64, Q, N, false);      // G
+    tc::issue_gemm<true>(taddr + 32, in_kmajor<TMA>(Yt, P), in_kmajor<TMA>(Xt, P), 64, Q, P, false);     // dY X^T
     tc::mma_commit(mbar);
+    tc::issue_gemm<true>(taddr + 64, in_kmajor<TMA>(Ct, N), tc::mnmajor_tile(Ht, P), 64, P, N, false);   // Crot H0
+    tc::issue_gemm<true>(taddr + 96, in_kmajor<TMA>(Bt, N), tc::mnmajor_tile(Dt, P), 64, P, N, false);   // Brot dH1
+    tc::issue_gemm<true>(taddr + 192, in_kmajor<TMA>(Ys, P), tc::kmajor_tile(Ht, P), 64, N, P, false);   // (e^Lam dY) H0^T
+    tc::issue_gemm<true>(taddr + 128, in_kmajor<TMA>(Xs, P), tc::kmajor_tile(Dt, P), 64, N, P, false);   // (r e x) dH1^T
+    tc::mma_commit(mbar + 3);
   }
   {  // <dH1, H0> while the tensor core works
     float acc = 0.f;
@@ -745,184 +741,144 @@ __global__ void __launch_bounds__(256) m3s_chunk_grad_kernel(SsdP p, const __gri
   }
   if (ok) ok = tc::mbar_wait(mbar, 0);
   tc::fence_after_sync();
+  ok = __all_sync(0xffffffffu, ok);  // warp-uniform: the column sums below shuffle with a full mask
   float dl_own = 0.f, de_own = 0.f, dg_own = 0.f, zsum = 0.f;
   const float lt = s.Lam[t], gt = s.gam[t], et = s.e[t], rt = s.r[t], dxt = s.dexp[t];
+  uint4 gmu[2];  // this thread's 16 elements of G*M, until the x tile is dead
   if (ok) {
-    {  // kappa_t = exp(Lam_t) dY_t . (Crot H0)_t   and   zeta_s = (Brot dH1)_s . x_s   (32 channels per half)
-      const int c0 = 32 * hc;
-      float f[32];
-      ld_acc32(taddr + 128, warp, c0, f);
-      if (own) dl_own += dxt * row_dot32_64<TMA>(Yt, t, c0, f);
-      ld_acc32(taddr + 192, warp, c0, f);
-      if (own) {
-        const float zeta = row_dot32_64<TMA>(Xt, t, c0, f);
-        de_own += rt * zeta;
-        dl_own -= rt * et * zeta;
-        zsum = rt * et * zeta;
-      }
-    }
-  }
-  __syncthreads();  // every read of the x tile is done: G*M may overwrite it
-  if (ok) {
-    {  // G and dY X^T: 32 columns per half.  Lanes 16-31 hold no accumulator rows; they take over columns
-       // 16..31 of the row of lane - 16, so all 32 lanes share the mask arithmetic.
-      const int c0 = 32 * hc, hx = lane >> 4;
-      float fg[16], fd[16];
-      {
-        float fa[32];
-        ld_acc32(taddr + 0, warp, c0, fa);
+    float fg[16], fd[16];
+    ld_acc16(taddr + 0, warp, tc16, fg);
+    ld_acc16(taddr + 32, warp, tc16, fd);
+    float rs = 0.f, dgc = 0.f;
+    float gm[16], dg[16], ce[16];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const float up = __shfl_sync(0xffffffffu, fa[16 + q], lane & 15);
-          fg[q] = hx ? up : fa[q];
-        }
-        ld_acc32(taddr + 64, warp, c0, fa);
+    for (int x = 0; x < 4; ++x) {
+      const float4 l4 = *reinterpret_cast<const float4*>(s.Lam + n16 + 4 * x);
+      const float4 e4 = *reinterpret_cast<const float4*>(s.e + n16 + 4 * x);
+      const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, es[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const float up = __shfl_sync(0xffffffffu, fa[16 + q], lane & 15);
-          fd[q] = hx ? up : fa[q];
-        }
-      }
-      float rs = 0.f, dgc = 0.f;
-      float gm[16], dg[16], ce[16], cl[16];
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const int sx = c0 + 16 * hx + q;
+      for (int y = 0; y < 4; ++y) {
+        const int q = 4 * x + y, sx = n16 + q;
         // branch-free so that the exponentials of different columns overlap
         const bool in = sx <= t;
-        const float Dv = in ? __expf(fminf(lt - s.Lam[sx], 0.f)) : 0.f;
-        const float Mv = Dv * (sx < t ? s.e[sx] : gt);
+        const float Dv = in ? __expf(fminf(lt - ls[y], 0.f)) : 0.f;
+        const float Mv = Dv * (sx < t ? es[y] : gt);
         const float dGM = in ? fd[q] : 0.f;
         const float gv = in ? fg[q] : 0.f;
         gm[q] = gv * Mv;                 // (G*M)_ts
         dg[q] = dGM * Mv;                // dG_ts
         const float dM = dGM * gv;
         const float dw = dM * Dv;
-        const float ml = dM * Mv;
-        rs += ml;
+        rs = fmaf(dM, Mv, rs);
         dgc += (sx == t) ? dw : 0.f;
-        ce[q] = (sx < t) ? dw : 0.f;     // de_s and dLam_s: column sums over the 16 rows of this warp
-        cl[q] = ml;
+        ce[q] = (sx < t) ? dw : 0.f;     // de_s: column sums
       }
-#pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        sts16(GMt, tc::kmajor_unit(t, (c0 >> 3) + 2 * hx + x, Q), pack8(&gm[8 * x]));
-        sts16(dGt, tc::kmajor_unit(t, (c0 >> 3) + 2 * hx + x, Q), pack8(&dg[8 * x]));
-      }
-      colsum16(ce, lane);  // the two 16-lane halves reduce their own 16 columns side by side
-      colsum16(cl, lane);
-      {
-        const int sx = c0 + 16 * hx + (lane & 15);
-        csw_e[(warp & 3) * Q + sx] += ce[0];
-        csw_l[(warp & 3) * Q + sx] -= cl[0];
-      }
-      rs += __shfl_xor_sync(0xffffffffu, rs, 16);
-      dgc += __shfl_xor_sync(0xffffffffu, dgc, 16);
-      dl_own += rs;
-      dg_own += dgc;
     }
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      gmu[x] = pack8(&gm[8 * x]);
+      sts16(dGt, tc::kmajor_unit(t, 2 * qd + x, Q), pack8(&dg[8 * x]));
+    }
+    colsum16(ce, lane);  // lane l: column l & 15 over the 16 rows of its half
+    const float cs16 = ce[0] + __shfl_xor_sync(0xffffffffu, ce[0], 16);
+    if (lane < 16) csw[(warp & 1) * Q + n16 + lane] = cs16;
+    dl_own = rs;
+    dg_own = dgc;
+    ok = tc::mbar_wait(mbar + 3, 0);
+  }
+  tc::fence_after_sync();
+  float bd[16];  // Brot dH1, used again for dx
+  if (ok) {  // kappa_t = exp(Lam_t) dY_t . (Crot H0)_t   and   zeta_s = (Brot dH1)_s . x_s
+    float f[16];
+    ld_acc16(taddr + 64, warp, tc16, f);
+    ld_acc16(taddr + 96, warp, tc16, bd);
+    dl_own = fmaf(dxt, row_dot16_64<TMA>(Yt, t, n16, f), dl_own);
+    const float zeta = row_dot16_64<TMA>(Xt, t, n16, bd);
+    de_own = rt * zeta;
+    zsum = rt * et * zeta;
+    dl_own -= zsum;
   }
   {
-    const float tot = warp_sum(own ? zsum : 0.f);
+    const float tot = warp_sum(zsum);
     if (lane == 0) red[8 + warp] = tot;
+  }
+  __syncthreads();  // every read of the x tile is done: G*M may overwrite it
+  if (ok) {
+#pragma unroll
+    for (int x = 0; x < 2; ++x) sts16(GMt, tc::kmajor_unit(t, 2 * qd + x, Q), gmu[x]);
   }
   tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   if (ok && tid == 0) {
-    tc::issue_gemm(taddr + 0, tc::mnmajor_tile(GMt, Q), in_mnmajor<TMA>(Yt, P), 64, P, Q, false);     // (G*M)^T dY
-    tc::issue_gemm(taddr + 64, in_kmajor<TMA>(Ys, P), tc::kmajor_tile(Ht, P), 64, N, P, false);       // (e^Lam dY) H0^T
-    tc::issue_gemm(taddr + 64, tc::kmajor_tile(dGt, Q), in_mnmajor<TMA>(Bt, N), 64, N, Q, true);      // + dG Brot
+    tc::issue_gemm<true>(taddr + 0, tc::mnmajor_tile(GMt, Q), in_mnmajor<TMA>(Yt, P), 64, P, Q, false);   // (G*M)^T dY
+    tc::issue_gemm<true>(taddr + 192, tc::kmajor_tile(dGt, Q), in_mnmajor<TMA>(Bt, N), 64, N, Q, true);   // + dG Brot
     tc::mma_commit(mbar);
+    tc::issue_gemm<true>(taddr + 128, tc::mnmajor_tile(dGt, Q), in_mnmajor<TMA>(Ct, N), 64, N, Q, true);  // + dG^T Crot
+    tc::mma_commit(mbar + 3);
   }
   if (ok) ok = tc::mbar_wait(mbar, 1);
   tc::fence_after_sync();
+  ok = __all_sync(0xffffffffu, ok);
   float dphi_own = 0.f;
+  const float sn = s.sn[t], cs = s.cs[t];
+  // dCrot / dBrot rows: un-rotate into the per-head partial image, and their share of the angle gradient
+  auto put_rows = [&](uint32_t col, const uint8_t* tile, bf16* image) {
+    float f[32];
+    ld_acc32(taddr + col, warp, tc32, f);
+    uint4* dst = reinterpret_cast<uint4*>(image + ci * (N * Q)) + t;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      float rot[8], o[8];
+      unpack8(*reinterpret_cast<const uint4*>(tile + in_unit<TMA>(t, 4 * qd + x, N)), rot);
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        const float f0 = f[8 * x + k], f1 = f[8 * x + k + 1];
+        o[k] = cs * f0 - sn * f1;
+        o[k + 1] = sn * f0 + cs * f1;
+        dphi_own += rot[k + 1] * f0 - rot[k] * f1;
+      }
+      dst[(4 * qd + x) * Q] = pack8(o);
+    }
+  };
   if (ok) {
     {  // dx_s = (G*M)^T dY + r e (Brot dH1)
-      const int c0 = 32 * hc;
-      float f[32], f2[32];
-      ld_acc32(taddr + 0, warp, c0, f);
-      ld_acc32(taddr + 192, warp, c0, f2);
-      if (own && t0 + t < p.T) {
+      float f[16];
+      ld_acc16(taddr + 0, warp, tc16, f);
+      if (t0 + t < p.T) {
         const float sc = rt * et;
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) f[jj] = fmaf(sc, f2[jj], f[jj]);
-        uint4* dst = reinterpret_cast<uint4*>(p.dx + ((size_t)b * p.T + t0 + t) * p.D + d0 + c0);
+        for (int jj = 0; jj < 16; ++jj) f[jj] = fmaf(sc, bd[jj], f[jj]);
+        uint4* dst = reinterpret_cast<uint4*>(p.dx + ((size_t)b * p.T + t0 + t) * p.D + d0 + n16);
 #pragma unroll
-        for (int x = 0; x < 4; ++x) dst[x] = pack8(&f[8 * x]);
+        for (int x = 0; x < 2; ++x) dst[x] = pack8(&f[8 * x]);
       }
     }
-    // dCrot rows: un-rotate into the per-head partial rows of dC, and their share of the angle gradient
-    const float sn = s.sn[t], cs = s.cs[t];
-    for (int c0 = 64 * hc; c0 < 64 * hc + 64; c0 += 32) {
-      float gc[32];
-      ld_acc32(taddr + 64, warp, c0, gc);
-      if (own && t0 + t < p.T) {
-        bf16* pcr = p.pc + ((((size_t)b * p.NH + head) * p.T) + t0 + t) * N + c0;
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          float cr[8], oc[8];
-          unpack8(*reinterpret_cast<const uint4*>(Ct + in_unit<TMA>(t, (c0 >> 3) + x, N)), cr);
-#pragma unroll
-          for (int k = 0; k < 8; k += 2) {
-            const float c0v = gc[8 * x + k], c1v = gc[8 * x + k + 1];
-            oc[k] = cs * c0v - sn * c1v; oc[k + 1] = sn * c0v + cs * c1v;
-            dphi_own += cr[k + 1] * c0v - cr[k] * c1v;
-          }
-          *reinterpret_cast<uint4*>(pcr + 8 * x) = pack8(oc);
-        }
-      }
-    }
+    put_rows(192, Ct, p.pc);
+    ok = tc::mbar_wait(mbar + 3, 1);
   }
-  tc::fence_before_sync();
-  __syncthreads();  // columns [0,192) are free again
   tc::fence_after_sync();
-  if (ok && tid == 0) {
-    tc::issue_gemm(taddr + 0, in_kmajor<TMA>(Xs, P), tc::kmajor_tile(Dt, P), 64, N, P, false);        // (r e x) dH1^T
-    tc::issue_gemm(taddr + 0, tc::mnmajor_tile(dGt, Q), in_mnmajor<TMA>(Ct, N), 64, N, Q, true);      // + dG^T Crot
-    tc::mma_commit(mbar);
-  }
-  if (ok) ok = tc::mbar_wait(mbar, 0);
-  tc::fence_after_sync();
-  if (ok) {
-    const float sn = s.sn[t], cs = s.cs[t];
-    for (int c0 = 64 * hc; c0 < 64 * hc + 64; c0 += 32) {
-      float gb[32];
-      ld_acc32(taddr + 0, warp, c0, gb);
-      if (own && t0 + t < p.T) {
-        bf16* pbr = p.pb + ((((size_t)b * p.NH + head) * p.T) + t0 + t) * N + c0;
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          float br[8], ob[8];
-          unpack8(*reinterpret_cast<const uint4*>(Bt + in_unit<TMA>(t, (c0 >> 3) + x, N)), br);
-#pragma unroll
-          for (int k = 0; k < 8; k += 2) {
-            const float b0 = gb[8 * x + k], b1 = gb[8 * x + k + 1];
-            ob[k] = cs * b0 - sn * b1; ob[k + 1] = sn * b0 + cs * b1;
-            dphi_own += br[k + 1] * b0 - br[k] * b1;
-          }
-          *reinterpret_cast<uint4*>(pbr + 8 * x) = pack8(ob);
-        }
-      }
-    }
-  }
-  if (own) {
-    part[(hc * 4 + 0) * Q + t] = dl_own;
-    part[(hc * 4 + 1) * Q + t] = de_own;
-    part[(hc * 4 + 2) * Q + t] = dg_own;
-    part[(hc * 4 + 3) * Q + t] = dphi_own;
-  }
+  ok = __all_sync(0xffffffffu, ok);
+  if (ok) put_rows(128, Bt, p.pb);
+  part[(qd * 4 + 0) * Q + t] = dl_own;
+  part[(qd * 4 + 1) * Q + t] = de_own;
+  part[(qd * 4 + 2) * Q + t] = dg_own;
+  part[(qd * 4 + 3) * Q + t] = dphi_own;
   tc::fence_before_sync();
   __syncthreads();
+  auto part_sum = [&](int what, int q) {
+    return (part[what * Q + q] + part[(4 + what) * Q + q]) + (part[(8 + what) * Q + q] + part[(12 + what) * Q + q]);
+  };
   if (tid < 32) {  // dLam -> da: reverse in-chunk cumulative sum (one warp, two rows per lane, fixed order)
     float zs = 0.f, hh = 0.f;
     for (int wv = 0; wv < 8; ++wv) { zs += red[8 + wv]; hh += red[wv]; }
     const float base = zs + s.L * hh;  // d/dLam_end
     const int ra = Q - 1 - 2 * tid, rb = ra - 1;
-    float a = part[0 * Q + ra] + part[4 * Q + ra] + csw_l[ra] + csw_l[Q + ra] + csw_l[2 * Q + ra] + csw_l[3 * Q + ra];
-    float bq = part[0 * Q + rb] + part[4 * Q + rb] + csw_l[rb] + csw_l[Q + rb] + csw_l[2 * Q + rb] + csw_l[3 * Q + rb];
+    auto dlam = [&](int q) {
+      return part_sum(0, q) - (s.e[q] * (csw[q] + csw[Q + q]) + s.gam[q] * part_sum(2, q));
+    };
+    float a = dlam(ra), bq = dlam(rb);
     warp_rcumsum64(a, bq, tid);
     s.Lam[ra] = base + a;  // Lam is dead by now: reuse for da
     s.Lam[rb] = base + bq;
@@ -932,9 +888,9 @@ __global__ void __launch_bounds__(256) m3s_chunk_grad_kernel(SsdP p, const __gri
   if (ok && tid < Q && t0 + tid < p.T) {
     const size_t o = ((size_t)b * p.NH + head) * p.T + t0 + tid;
     p.da[o] = s.Lam[tid];
-    p.de[o] = part[1 * Q + tid] + part[5 * Q + tid] + csw_e[tid] + csw_e[Q + tid] + csw_e[2 * Q + tid] + csw_e[3 * Q + tid];
-    p.dgam[o] = part[2 * Q + tid] + part[6 * Q + tid];
-    p.dphi[o] = part[3 * Q + tid] + part[7 * Q + tid];
+    p.de[o] = part_sum(1, tid) + (csw[tid] + csw[Q + tid]);
+    p.dgam[o] = part_sum(2, tid);
+    p.dphi[o] = part_sum(3, tid);
   }
   if (warp == 0) tc::tmem_dealloc(taddr, 256);
 }
@@ -1013,27 +969,25 @@ __global__ void m3s_dalog_kernel(SsdP p) {
   p.da_log[head] = s;
 }
 
-// dB[b,t,g,:] = sum over the heads of group g of the per-head partial rows (fp32, fixed order).
-// One warp per (b, t, g): a lane owns 4 consecutive states.
+// dB[b,t,g,:] = sum over the heads of group g of the per-head partial images (fp32, fixed order).  A thread owns eight
+// states of a row; consecutive threads hold consecutive rows, which are neighbours in the column-blocked images.
 __global__ void __launch_bounds__(128) m3s_reduce_kernel(const bf16* __restrict__ pb, const bf16* __restrict__ pc,
-                                                         bf16* __restrict__ db, bf16* __restrict__ dc, int T, int G, int NH) {
-  const int lane = threadIdx.x & 31;
-  const int t = blockIdx.x * 4 + (threadIdx.x >> 5), g = blockIdx.y, b = blockIdx.z, per = NH / G;
+                                                         bf16* __restrict__ db, bf16* __restrict__ dc, int T, int G, int NH,
+                                                         int n) {
+  const int c = blockIdx.x >> 4, which = blockIdx.x & 1, r = threadIdx.x & 63, c8 = (blockIdx.x & 14) + (threadIdx.x >> 6);
+  const int g = blockIdx.y, b = blockIdx.z, per = NH / G, t = c * Q + r;
   if (t >= T) return;
-  float sb[4] = {0.f, 0.f, 0.f, 0.f}, sc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int h = g * per; h < (g + 1) * per; ++h) {
-    const size_t pi = (((size_t)b * NH + h) * T + t) * N + 4 * lane;
-    const uint2 vb = __ldg(reinterpret_cast<const uint2*>(pb + pi));
-    const uint2 vc = __ldg(reinterpret_cast<const uint2*>(pc + pi));
-    float a0, a1;
-    tc::unpack_bf16(vb.x, a0, a1); sb[0] += a0; sb[1] += a1;
-    tc::unpack_bf16(vb.y, a0, a1); sb[2] += a0; sb[3] += a1;
-    tc::unpack_bf16(vc.x, a0, a1); sc[0] += a0; sc[1] += a1;
-    tc::unpack_bf16(vc.y, a0, a1); sc[2] += a0; sc[3] += a1;
+  const uint4* src = reinterpret_cast<const uint4*>(which ? pc : pb) +
+                     (((size_t)b * NH + (size_t)g * per) * n + c) * (N / 8 * Q) + c8 * Q + r;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+  for (int h = 0; h < per; ++h) {
+    float e[8];
+    unpack8(__ldg(src + (size_t)h * n * (N / 8 * Q)), e);
+#pragma unroll
+    for (int y = 0; y < 8; ++y) acc[y] += e[y];
   }
-  const size_t gi = (((size_t)b * T + t) * G + g) * N + 4 * lane;
-  *reinterpret_cast<uint2*>(db + gi) = make_uint2(tc::pack_bf16(sb[0], sb[1]), tc::pack_bf16(sb[2], sb[3]));
-  *reinterpret_cast<uint2*>(dc + gi) = make_uint2(tc::pack_bf16(sc[0], sc[1]), tc::pack_bf16(sc[2], sc[3]));
+  *reinterpret_cast<uint4*>((which ? dc : db) + (((size_t)b * T + t) * G + g) * N + 8 * c8) = pack8(acc);
 }
 
 }  // namespace m3s
@@ -1064,8 +1018,8 @@ static size_t carve_ssd(SsdP& p, void* ws, bool bwd) {
     p.de = cv.take<float>(bh * p.T);
     p.dgam = cv.take<float>(bh * p.T);
     p.dal_part = cv.take<float>(bh);
-    p.pb = cv.take<m3s::bf16>(bh * p.T * m3s::N);
-    p.pc = cv.take<m3s::bf16>(bh * p.T * m3s::N);
+    p.pb = cv.take<m3s::bf16>(bh * p.n * m3s::Q * m3s::N);
+    p.pc = cv.take<m3s::bf16>(bh * p.n * m3s::Q * m3s::N);
   }
   return cv.bytes();
 }
@@ -1175,8 +1129,8 @@ mxb_status mamba3_ssd_bwd(const mxb_mamba3_desc* d, const void* x, const float* 
   MXB_LAUNCH("m3s_final_kernel", st, (m3s::m3s_final_kernel<<<dim3(p.NH, p.B), m3s::kScalThreads, 0, st>>>(p)));
   MXB_LAUNCH("m3s_dalog_kernel", st, (m3s::m3s_dalog_kernel<<<(p.NH + 127) / 128, 128, 0, st>>>(p)));
   MXB_LAUNCH("m3s_reduce_kernel", st,
-             (m3s::m3s_reduce_kernel<<<dim3((p.T + 3) / 4, p.G, p.B), 128, 0, st>>>(p.pb, p.pc, static_cast<m3s::bf16*>(db),
-                                                                            static_cast<m3s::bf16*>(dc), p.T, p.G, p.NH)));
+             (m3s::m3s_reduce_kernel<<<dim3(16 * p.n, p.G, p.B), 128, 0, st>>>(p.pb, p.pc, static_cast<m3s::bf16*>(db),
+                                                                            static_cast<m3s::bf16*>(dc), p.T, p.G, p.NH, p.n)));
   return check_launch("mamba3 ssd backward");
 }
 

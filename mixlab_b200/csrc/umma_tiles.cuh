@@ -82,7 +82,8 @@ __device__ __forceinline__ uint32_t mnmajor_unit(int k, int c8, int mn) {
   return (uint32_t)c8 * 128u + (uint32_t)(k >> 3) * (uint32_t)(mn / 8) * 128u + (uint32_t)(k & 7) * 16u;
 }
 
-// D[tmem] (+)= A * B over ktotal contraction elements; one thread issues.
+// D[tmem] (+)= A * B over ktotal contraction elements; one thread issues.  WS: the weight-stationary form.
+template <bool WS = false>
 __device__ __forceinline__ void issue_gemm(uint32_t tmem_d, const Tile& a, const Tile& b, int M, int N, int ktotal,
                                            bool accumulate) {
   const uint32_t idesc = make_idesc_bf16(M, N, a.mn_major, b.mn_major);
@@ -91,9 +92,11 @@ __device__ __forceinline__ void issue_gemm(uint32_t tmem_d, const Tile& a, const
   auto koff = [](const Tile& t, uint32_t ks) {
     return t.slab_ksteps ? (ks / t.slab_ksteps) * t.slab_stride + (ks % t.slab_ksteps) * t.kstep : ks * t.kstep;
   };
-  for (int ks = 0; ks < ktotal / 16; ++ks)
-    mma_ss(tmem_d, da + (uint64_t)(koff(a, ks) >> 4), db + (uint64_t)(koff(b, ks) >> 4), idesc,
-           (accumulate || ks > 0) ? 1u : 0u);
+  for (int ks = 0; ks < ktotal / 16; ++ks) {
+    const uint64_t xa = da + (uint64_t)(koff(a, ks) >> 4), xb = db + (uint64_t)(koff(b, ks) >> 4);
+    if (WS) mma_ws(tmem_d, xa, xb, idesc, (accumulate || ks > 0) ? 1u : 0u);
+    else mma_ss(tmem_d, xa, xb, idesc, (accumulate || ks > 0) ? 1u : 0u);
+  }
 }
 
 // ---- bf16 packing ---------------------------------------------------------
