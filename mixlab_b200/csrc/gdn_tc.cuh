@@ -110,6 +110,13 @@ inline bool tc_split_columns(const TcP& p) { return p.Dv > 64 && 2 * p.B * p.H <
 template <int NV>
 constexpr int kStateThreads = NV == KD ? 384 : 288;
 
+__device__ __forceinline__ void ld_acc16(uint32_t taddr, int warp, int c0, float (&f)[16]) {
+  uint32_t r[16];
+  tc::tmem_ld_32x32b_x16(taddr + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)c0, r);
+  tc::tmem_ld_wait();
+#pragma unroll
+  for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(r[i]);
+}
 // Loads 64 fp32 accumulator columns [0, 64) at taddr of this thread's TMEM lane: both loads in flight, one wait.
 __device__ __forceinline__ void ld_acc64(uint32_t taddr, int warp, float (&f)[64]) {
   uint32_t r0[32], r1[32];

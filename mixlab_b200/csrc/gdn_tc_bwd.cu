@@ -298,12 +298,14 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
 // 256 TMEM columns and 107 KB of shared memory: two CTAs share an SM.  Every buffer is reused as soon as it is dead:
 //   XdO   dO (TMA tile) -> d dO -> z                      Xe   -dv_new image -> -e -> dv = beta e on its way out
 //   Xvn   v_new image -> v (TMA) -> q (TMA) -> dq         R1   S0 image -> dS image -> k (TMA) | dkp -> dk
-// TMEM: [0,128) -e, then DQ until the end; [128,256) the other products one after the other.  All accumulators are
-// M=64: row i sits in TMEM lane (i%16) + 32*(i/16) and is handled by thread (warp i/16, lane i%16); warps 4-7 take
-// the second half of the columns.  Grid = (batch*head, chunk) with batch*head fastest: neighbouring CTAs read
+// TMEM: [0,64) -e, then DQ until the end; [64,128) the other products one after the other, [128,160) k k^T.  Every
+// product is issued in the weight-stationary form, whose M = 64 accumulators fill all 128 lanes: each thread has a row
+// (i) and a quarter of the columns (16 of 64, 32 of 128) in every epilogue.
+// Bound by the six batches that follow one another within a CTA (HBM: 1.77 GB, 0.27 ms at 8 x 4096 x 16 heads): with
+// half of the lanes idle in every epilogue 404 us, this 365 us.  Grid = (batch*head, chunk) with batch*head fastest: neighbouring CTAs read
 // neighbouring heads of the same time steps (one contiguous row of the token tensors between them), and the chunks
 // the reverse state pass wrote last are read first.
-constexpr int kChunkBwdSmem = 3 * 16384 + 32768 + 3 * 8192 + 8 * C * 4 + 16 * 4 + 64 + 64 + 1024;
+constexpr int kChunkBwdSmem = 3 * 16384 + 32768 + 3 * 8192 + 12 * C * 4 + 16 * 4 + 64 + 64 + 1024;
 
 __device__ __forceinline__ void unpack8(uint4 v, float (&e)[8]) {
   tc::unpack_bf16(v.x, e[0], e[1]); tc::unpack_bf16(v.y, e[2], e[3]);
@@ -313,18 +315,6 @@ __device__ __forceinline__ uint4 pack8(const float* e) {
   return make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]), tc::pack_bf16(e[4], e[5]),
                     tc::pack_bf16(e[6], e[7]));
 }
-// M=64 accumulators leave lanes 16-31 of every warp without a row.  Where an epilogue does real arithmetic per
-// element, the owning lane l hands columns 16..31 of its 32-column block to lane l + 16: both then work on 16
-// columns of the same row (16 shuffles buy half of the arithmetic).  h[q] = column c0 + 16 (lane >> 4) + q.
-__device__ __forceinline__ void split_block32(const float (&f)[32], int lane, float (&h)[16]) {
-  const bool upper = (lane >> 4) != 0;
-#pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    const float up = __shfl_sync(0xffffffffu, f[16 + q], lane & 15);
-    h[q] = upper ? up : f[q];
-  }
-}
-
 __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
@@ -341,9 +331,9 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   float* bet = gam + C;
   float* dd = bet + C;
   float* rr = dd + C;
-  float* dgo = rr + C;              // [2][C] per-row dgam / dbeta partials of the two column halves
-  float* dbo = dgo + 2 * C;
-  float* red = dbo + 2 * C;         // [0,8) <dS,S0> per warp, [8,16) sum of k.dkp per warp
+  float* dgo = rr + C;              // [4][C] per-row dgam / dbeta partials of the column quarters
+  float* dbo = dgo + 4 * C;
+  float* red = dbo + 4 * C;         // [0,8) <dS,S0> per warp, [8,16) sum of k.dkp per warp
   // [0] MMA, [6] second MMA barrier of the last batch; loads: [1] -dv_new/T/dO/v_new, [2] S0, [3] dS, [4] k/v, [5] q
   uint64_t* mbar = reinterpret_cast<uint64_t*>(red + 16);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 8);
@@ -353,12 +343,17 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   const size_t ci = (size_t)bh * p.n + c;
   const int imax = min(C, p.T - t0);
   auto row = [&](int i) { return ((size_t)(b * p.T + t0 + i) * p.H + h); };
-  const bool own = lane < 16;
-  const int i = 16 * (warp & 3) + (lane & 15);  // the row this thread owns in every epilogue
-  const int hc = warp >> 2;   // warps 0-3 take the first half of an accumulator's columns, warps 4-7 the second
-  const int cb = 32 * hc;     // this thread's 32 columns of every [64][64] accumulator
-  const int cw = 64 * hc;     // this thread's 64 columns of every [64][128] accumulator
-  const int hx = lane >> 4;   // which 16 columns of a shared 32-column block this lane works on (split_block32)
+  // this thread's row and column quarter of every result; tc16 / tc32: its TMEM columns of a [64][64] / [64][128] result
+  const int i = 32 * (warp & 1) + lane, qd = (warp & 2) + (warp >> 2), n16 = 16 * qd;
+  const int tc16 = 16 * (warp >> 2), tc32 = 32 * (warp >> 2);
+  // sixteen per-row scalars of this thread's columns of a [64][64] result
+  auto row16 = [&](const float* v, float (&e)[16]) {
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float4 q = *reinterpret_cast<const float4*>(v + n16 + 4 * x);
+      e[4 * x] = q.x; e[4 * x + 1] = q.y; e[4 * x + 2] = q.z; e[4 * x + 3] = q.w;
+    }
+  };
 
   // prologue latencies side by side: warp 0 allocates TMEM, one thread of warp 1 initialises the barriers and issues
   // the first copies, warps 2-3 fetch the per-row scalars
@@ -397,13 +392,13 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
     dd[tid] = exp_nonpos(gam[tid]);
     rr[tid] = exp_nonpos(glast - gam[tid]);
   }
-  const uint32_t tA = *tslot, tB = tA + 128;
+  const uint32_t tA = *tslot, tB = tA + 64, tK = tA + 128;
   bool ok = tc::mbar_wait(mbar + 1, 0);
   uint32_t ph = 0;
   // ---- batch 1: -e = T^T (-dv_new) (both operands contracted over their rows), dP = dO v_new^T ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tA, tc::mnmajor_tile(Xt, C), tc::colblk_mnmajor_tile(Xe, C), 64, 128, C, false);
-    tc::issue_gemm(tB, tc::kmajor_sw128_tile(XdO, 8192), tc::colblk_kmajor_tile(Xvn, C), 64, 64, KD, false);
+    tc::issue_gemm<true>(tA, tc::mnmajor_tile(Xt, C), tc::colblk_mnmajor_tile(Xe, C), 64, 128, C, false);
+    tc::issue_gemm<true>(tB, tc::kmajor_sw128_tile(XdO, 8192), tc::colblk_kmajor_tile(Xvn, C), 64, 64, KD, false);
     tc::mma_commit(mbar);
   }
   __syncthreads();  // dd, rr visible
@@ -416,25 +411,23 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   if (ok) {
     // -e goes back over the operand it was computed from (its MMA is complete), in the swizzled layout of a TMA
     // tile: scaled by -beta in place later, the same bytes leave as dv through a tiled store
-    for_acc2x32(tA, warp, cw, [&](int c0, const float (&f)[32]) {
-      if (own) {
+    {
+      float f[32];
+      ld_acc32(tA, warp, tc32, f);
 #pragma unroll
-        for (int x = 0; x < 4; ++x) sts16(Xe, tc::sw128_unit(i, (c0 >> 3) + x), pack8(&f[8 * x]));
-      }
-    });
+      for (int x = 0; x < 4; ++x) sts16(Xe, tc::sw128_unit(i, 4 * qd + x), pack8(&f[8 * x]));
+    }
     {  // dP * Gamma, lower triangle incl. diagonal
-      float f[32], hq[16];
-      ld_acc32(tB, warp, cb, f);
-      split_block32(f, lane, hq);
-      const int j0 = cb + 16 * hx;
+      float hq[16], gj[16];
+      ld_acc16(tB, warp, tc16, hq);
+      row16(gam, gj);
 #pragma unroll
       for (int q = 0; q < 16; ++q) {
-        const int j = j0 + q;
-        const float val = hq[q] * exp_nonpos(gi - gam[j]);  // unconditional: the exponentials overlap
-        hq[q] = (j <= i) ? val : 0.f;
+        const float val = hq[q] * exp_nonpos(gi - gj[q]);  // unconditional: the exponentials overlap
+        hq[q] = (n16 + q <= i) ? val : 0.f;
       }
 #pragma unroll
-      for (int x = 0; x < 2; ++x) sts16(Xpg, tc::kmajor_unit(i, (j0 >> 3) + x, C), pack8(&hq[8 * x]));
+      for (int x = 0; x < 2; ++x) sts16(Xpg, tc::kmajor_unit(i, 2 * qd + x, C), pack8(&hq[8 * x]));
     }
 #pragma unroll
     for (int m = 0; m < 4; ++m) {  // dO <- diag(d) dO in place, so that DQ can take dPG k on top later
@@ -450,8 +443,8 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   tc::fence_after_sync();
   // ---- batch 2: DQ = (d dO) S0^T, z = (-e) S0^T ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tA, tc::kmajor_sw128_tile(XdO, 8192), tc::colblk_kmajor_tile(R1, KD), 64, 128, KD, false);
-    tc::issue_gemm(tB, tc::kmajor_sw128_tile(Xe, 8192), tc::colblk_kmajor_tile(R1, KD), 64, 128, KD, false);
+    tc::issue_gemm<true>(tA, tc::kmajor_sw128_tile(XdO, 8192), tc::colblk_kmajor_tile(R1, KD), 64, 128, KD, false);
+    tc::issue_gemm<true>(tB, tc::kmajor_sw128_tile(Xe, 8192), tc::colblk_kmajor_tile(R1, KD), 64, 128, KD, false);
     tc::mma_commit(mbar);  // one commit: z overwrites d dO and dS overwrites S0, which DQ reads as well
   }
   uint4 s0u[8];  // this thread's 8 units of S0, kept for <dS, S0> (the buffer is about to be reused)
@@ -467,13 +460,11 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
     tc::mbar_expect_tx(mbar + 3, 32768);
     tc::bulk_load(tc::smem_u32(R1), p.dhs + ci * KD * KD, 32768, mbar + 3);
   }
-  if (ok) {
-    for_acc2x32(tB, warp, cw, [&](int c0, const float (&f)[32]) {  // z -> bf16 operand over the dead dO tile (blocked layout)
-      if (own) {
+  if (ok) {  // z -> bf16 operand over the dead dO tile (blocked layout)
+    float f[32];
+    ld_acc32(tB, warp, tc32, f);
 #pragma unroll
-        for (int x = 0; x < 4; ++x) sts16(XdO, tc::kmajor_unit(i, (c0 >> 3) + x, KD), pack8(&f[8 * x]));
-      }
-    });
+    for (int x = 0; x < 4; ++x) sts16(XdO, tc::kmajor_unit(i, 4 * qd + x, KD), pack8(&f[8 * x]));
   }
   if (ok) ok = tc::mbar_wait(mbar + 3, 0);  // dS
   tc::fence_async_smem();
@@ -482,7 +473,7 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   tc::fence_after_sync();
   // ---- batch 3: v_new dS^T ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tB, tc::colblk_kmajor_tile(Xvn, C), tc::colblk_kmajor_tile(R1, KD), 64, 128, KD, false);
+    tc::issue_gemm<true>(tB, tc::colblk_kmajor_tile(Xvn, C), tc::colblk_kmajor_tile(R1, KD), 64, 128, KD, false);
     tc::mma_commit(mbar);
   }
   {  // <dS, S0>
@@ -511,15 +502,13 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
       tc::tma_load_4d(tc::smem_u32(Xvn) + 8192 * sl, &maps.v, 64 * sl, h, t0, b, mbar + 4);
     }
   }
-  if (ok) {
-    for_acc2x32(tB, warp, cw, [&](int c0, float (&f)[32]) {  // dkp = r (v_new dS^T), kept as bf16 where dk will be assembled
-      if (own) {
+  if (ok) {  // dkp = r (v_new dS^T), kept as bf16 where dk will be assembled
+    float f[32];
+    ld_acc32(tB, warp, tc32, f);
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) f[jj] *= ri;
+    for (int jj = 0; jj < 32; ++jj) f[jj] *= ri;
 #pragma unroll
-        for (int x = 0; x < 4; ++x) sts16(Xdk, tc::sw128_unit(i, (c0 >> 3) + x), pack8(&f[8 * x]));
-      }
-    });
+    for (int x = 0; x < 4; ++x) sts16(Xdk, tc::sw128_unit(i, 4 * qd + x), pack8(&f[8 * x]));
   }
   if (ok) ok = tc::mbar_wait(mbar + 4, 0);  // k, v
   tc::fence_before_sync();
@@ -527,9 +516,10 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   tc::fence_after_sync();
   // ---- batch 4: (-e) v^T and z k^T; their column-scaled sum is Y = T^T dT (dT is never formed) ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tB, tc::kmajor_sw128_tile(Xe, 8192), tc::kmajor_sw128_tile(Xvn, 8192), 64, 64, KD, false);
-    tc::issue_gemm(tB + 64, tc::kmajor_tile(XdO, KD), tc::kmajor_sw128_tile(Xk, 8192), 64, 64, KD, false);
+    tc::issue_gemm<true>(tB, tc::kmajor_sw128_tile(Xe, 8192), tc::kmajor_sw128_tile(Xvn, 8192), 64, 64, KD, false);
+    tc::issue_gemm<true>(tB + 32, tc::kmajor_tile(XdO, KD), tc::kmajor_sw128_tile(Xk, 8192), 64, 64, KD, false);
     tc::mma_commit(mbar);
+    tc::issue_gemm<true>(tK, tc::kmajor_sw128_tile(Xk, 8192), tc::kmajor_sw128_tile(Xk, 8192), 64, 64, KD, false);  // k k^T, for batch 5
   }
   float vdot = 0.f, kz = 0.f;  // e_i . v_i and k_i . z_i: the diagonals of the two products of this batch
   if (ok) ok = tc::mbar_wait(mbar, ph);
@@ -537,23 +527,20 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   tc::fence_after_sync();
   ok = __all_sync(0xffffffffu, ok);  // warp-uniform: the epilogues below shuffle with a full mask
   if (ok) {  // Y[i][m] = beta_m ((e_i . v_m) + d_m (z_i . k_m))
-    float f[32], ha[16], hb[16];
-    ld_acc32(tB, warp, cb, f);
-    split_block32(f, lane, ha);
-    ld_acc32(tB + 64, warp, cb, f);
-    split_block32(f, lane, hb);
-    const int j0 = cb + 16 * hx;
+    float ha[16], hb[16], dj[16], bj[16];
+    ld_acc16(tB, warp, tc16, ha);
+    ld_acc16(tB + 32, warp, tc16, hb);
+    row16(dd, dj);
+    row16(bet, bj);
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {  // the lane whose 16 columns contain column i picks the two row dots off the diagonal
-      vdot = (j0 + q == i) ? -ha[q] : vdot;
-      kz = (j0 + q == i) ? hb[q] : kz;
+    for (int q = 0; q < 16; ++q) {  // the thread whose columns contain column i picks the two row dots off the diagonal
+      vdot = (n16 + q == i) ? -ha[q] : vdot;
+      kz = (n16 + q == i) ? hb[q] : kz;
     }
-    vdot += __shfl_xor_sync(0xffffffffu, vdot, 16);  // one of the two lanes of a row found it (the other holds 0);
-    kz += __shfl_xor_sync(0xffffffffu, kz, 16);      // rows whose diagonal lies in the other column half keep 0
 #pragma unroll
-    for (int q = 0; q < 16; ++q) ha[q] = bet[j0 + q] * fmaf(dd[j0 + q], hb[q], -ha[q]);
+    for (int q = 0; q < 16; ++q) ha[q] = bj[q] * fmaf(dj[q], hb[q], -ha[q]);
 #pragma unroll
-    for (int x = 0; x < 2; ++x) sts16(Xy, tc::kmajor_unit(i, (j0 >> 3) + x, C), pack8(&ha[8 * x]));
+    for (int x = 0; x < 2; ++x) sts16(Xy, tc::kmajor_unit(i, 2 * qd + x, C), pack8(&ha[8 * x]));
   }
   tc::fence_async_smem();
   tc::fence_before_sync();
@@ -563,10 +550,9 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
     tc::mbar_expect_tx(mbar + 5, 16384);
     for (int sl = 0; sl < 2; ++sl) tc::tma_load_4d(tc::smem_u32(Xvn) + 8192 * sl, &maps.q, 64 * sl, h, t0, b, mbar + 5);
   }
-  // ---- batch 5: dA = tril(Y T^T, -1) and k k^T ----
+  // ---- batch 5: dA = tril(Y T^T, -1) ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tB, tc::kmajor_tile(Xy, C), tc::kmajor_tile(Xt, C), 64, 64, C, false);
-    tc::issue_gemm(tB + 64, tc::kmajor_sw128_tile(Xk, 8192), tc::kmajor_sw128_tile(Xk, 8192), 64, 64, KD, false);
+    tc::issue_gemm<true>(tB, tc::kmajor_tile(Xy, C), tc::kmajor_tile(Xt, C), 64, 64, C, false);
     tc::mma_commit(mbar);
   }
   if (ok) {  // -e has served as an operand and in the row dots for the last time (barrier above): dv = beta e in place
@@ -583,28 +569,22 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   ok = __all_sync(0xffffffffu, ok);  // warp-uniform: the epilogues below shuffle with a full mask
   float db_own = 0.f, dg_own = 0.f;
   if (ok) {  // Xy <- Mb = beta_i M, M = -dA*Gamma strictly lower, zeros elsewhere
-    float f[32], ha[16], hk[16];
-    ld_acc32(tB, warp, cb, f);
-    split_block32(f, lane, ha);
-    ld_acc32(tB + 64, warp, cb, f);
-    split_block32(f, lane, hk);
-    const int j0 = cb + 16 * hx;
+    float ha[16], hk[16], gj[16];
+    ld_acc16(tB, warp, tc16, ha);
+    ld_acc16(tK, warp, tc16, hk);
+    row16(gam, gj);
     float rs = 0.f;
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
-      const int j = j0 + q;
-      const float mv = -ha[q] * exp_nonpos(gi - gam[j]);  // unconditional: the exponentials overlap
-      const float M = (j < i) ? mv : 0.f;
+      const float mv = -ha[q] * exp_nonpos(gi - gj[q]);  // unconditional: the exponentials overlap
+      const float M = (n16 + q < i) ? mv : 0.f;
       rs = fmaf(M, hk[q], rs);
       ha[q] = bi * M;
     }
 #pragma unroll
-    for (int x = 0; x < 2; ++x) sts16(Xy, tc::kmajor_unit(i, (j0 >> 3) + x, C), pack8(&ha[8 * x]));
-    rs += __shfl_xor_sync(0xffffffffu, rs, 16);
-    if (own) {
-      db_own = vdot + di * kz + rs;
-      dg_own = 2.f * bi * (di * kz + rs);
-    }
+    for (int x = 0; x < 2; ++x) sts16(Xy, tc::kmajor_unit(i, 2 * qd + x, C), pack8(&ha[8 * x]));
+    db_own = vdot + di * kz + rs;
+    dg_own = 2.f * bi * (di * kz + rs);
   }
   if (ok) ok = tc::mbar_wait(mbar + 5, 0);  // q
   tc::fence_async_smem();
@@ -614,11 +594,11 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   // ---- batch 6: dPG^T q + Mb k + Mb^T k (one tile read K-major and MN-major), committed first: the dk epilogue
   //      runs while DQ += dPG k is still on the tensor core ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tB, tc::mnmajor_tile(Xpg, C), tc::mnmajor_sw128_tile(Xvn, 8192), 64, 128, C, false);
-    tc::issue_gemm(tB, tc::kmajor_tile(Xy, C), tc::mnmajor_sw128_tile(Xk, 8192), 64, 128, C, true);
-    tc::issue_gemm(tB, tc::mnmajor_tile(Xy, C), tc::mnmajor_sw128_tile(Xk, 8192), 64, 128, C, true);
+    tc::issue_gemm<true>(tB, tc::mnmajor_tile(Xpg, C), tc::mnmajor_sw128_tile(Xvn, 8192), 64, 128, C, false);
+    tc::issue_gemm<true>(tB, tc::kmajor_tile(Xy, C), tc::mnmajor_sw128_tile(Xk, 8192), 64, 128, C, true);
+    tc::issue_gemm<true>(tB, tc::mnmajor_tile(Xy, C), tc::mnmajor_sw128_tile(Xk, 8192), 64, 128, C, true);
     tc::mma_commit(mbar + 6);
-    tc::issue_gemm(tA, tc::kmajor_tile(Xpg, C), tc::mnmajor_sw128_tile(Xk, 8192), 64, 128, C, true);
+    tc::issue_gemm<true>(tA, tc::kmajor_tile(Xpg, C), tc::mnmajor_sw128_tile(Xk, 8192), 64, 128, C, true);
     tc::mma_commit(mbar);
   }
   if (ok) ok = tc::mbar_wait(mbar + 6, 0);
@@ -626,68 +606,51 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   ok = __all_sync(0xffffffffu, ok);  // warp-uniform: the epilogues below shuffle with a full mask
   float rho = 0.f;
   if (ok) {  // dk = dkp + (dPG^T q + (Mb + Mb^T) k) + beta d z, assembled over dkp (each thread rewrites the units it read)
-    float kd = 0.f;
-    for (int s = 0; s < 2; ++s) {
-      const int c0 = cw + 32 * s;
-      float f[32], g2[16];
-      ld_acc32(tB, warp, c0, f);
-      split_block32(f, lane, g2);
-      float r2[2] = {0.f, 0.f}, k2[2] = {0.f, 0.f};
+    float f[32], r4[4] = {0.f, 0.f, 0.f, 0.f}, k4[4] = {0.f, 0.f, 0.f, 0.f};
+    ld_acc32(tB, warp, tc32, f);
 #pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        const int c8 = (c0 >> 3) + 2 * hx + x;
-        float e[8], z[8], kr[8];
-        unpack8(*reinterpret_cast<const uint4*>(Xdk + tc::sw128_unit(i, c8)), e);
-        unpack8(*reinterpret_cast<const uint4*>(XdO + tc::kmajor_unit(i, c8, KD)), z);
-        unpack8(*reinterpret_cast<const uint4*>(Xk + tc::sw128_unit(i, c8)), kr);
+    for (int x = 0; x < 4; ++x) {
+      const int c8 = 4 * qd + x;
+      float e[8], z[8], kr[8];
+      unpack8(*reinterpret_cast<const uint4*>(Xdk + tc::sw128_unit(i, c8)), e);
+      unpack8(*reinterpret_cast<const uint4*>(XdO + tc::kmajor_unit(i, c8, KD)), z);
+      unpack8(*reinterpret_cast<const uint4*>(Xk + tc::sw128_unit(i, c8)), kr);
 #pragma unroll
-        for (int y = 0; y < 8; ++y) {
-          r2[x] = fmaf(kr[y], e[y], r2[x]);              // k_i . dkp_i
-          const float val = g2[8 * x + y] + e[y] + bd_i * z[y];
-          k2[x] = fmaf(kr[y], val, k2[x]);               // k_i . dk_i
-          g2[8 * x + y] = val;
-        }
-        sts16(Xdk, tc::sw128_unit(i, c8), pack8(&g2[8 * x]));
+      for (int y = 0; y < 8; ++y) {
+        r4[x] = fmaf(kr[y], e[y], r4[x]);              // k_i . dkp_i
+        const float val = f[8 * x + y] + e[y] + bd_i * z[y];
+        k4[x] = fmaf(kr[y], val, k4[x]);               // k_i . dk_i
+        f[8 * x + y] = val;
       }
-      rho += r2[0] + r2[1];
-      kd += k2[0] + k2[1];
+      sts16(Xdk, tc::sw128_unit(i, c8), pack8(&f[8 * x]));
     }
-    rho += __shfl_xor_sync(0xffffffffu, rho, 16);
-    kd += __shfl_xor_sync(0xffffffffu, kd, 16);
-    dg_own -= kd;
+    rho = (r4[0] + r4[1]) + (r4[2] + r4[3]);
+    dg_own -= (k4[0] + k4[1]) + (k4[2] + k4[3]);
   }
   if (ok) ok = tc::mbar_wait(mbar, ph);  // every product has completed
   ph ^= 1;
   tc::fence_after_sync();
   ok = __all_sync(0xffffffffu, ok);  // warp-uniform: the epilogues below shuffle with a full mask
   if (ok) {  // dq, assembled over q (each thread rewrites the units it read)
-    float qd = 0.f;
-    for (int s = 0; s < 2; ++s) {
-      const int c0 = cw + 32 * s;
-      float f[32], hq[16];
-      ld_acc32(tA, warp, c0, f);
-      split_block32(f, lane, hq);
+    float f[32], q4[4] = {0.f, 0.f, 0.f, 0.f};
+    ld_acc32(tA, warp, tc32, f);
 #pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        const int c8 = (c0 >> 3) + 2 * hx + x;
-        float qr[8];
-        unpack8(*reinterpret_cast<const uint4*>(Xvn + tc::sw128_unit(i, c8)), qr);
+    for (int x = 0; x < 4; ++x) {
+      const int c8 = 4 * qd + x;
+      float qr[8];
+      unpack8(*reinterpret_cast<const uint4*>(Xvn + tc::sw128_unit(i, c8)), qr);
 #pragma unroll
-        for (int y = 0; y < 8; ++y) qd = fmaf(qr[y], hq[8 * x + y], qd);
-        sts16(Xvn, tc::sw128_unit(i, c8), pack8(&hq[8 * x]));
-      }
+      for (int y = 0; y < 8; ++y) q4[x] = fmaf(qr[y], f[8 * x + y], q4[x]);
+      sts16(Xvn, tc::sw128_unit(i, c8), pack8(&f[8 * x]));
     }
-    qd += __shfl_xor_sync(0xffffffffu, qd, 16);
-    dg_own += qd;
+    dg_own += (q4[0] + q4[1]) + (q4[2] + q4[3]);
   }
   {
-    const float tot = warp_sum(own ? rho : 0.f);
+    const float tot = warp_sum(rho);
     if (lane == 0) red[8 + warp] = tot;  // summed in a fixed order below (deterministic)
   }
-  if (own) {  // the two column halves hold partial sums of the same row
-    dgo[hc * C + i] = dg_own;
-    dbo[hc * C + i] = db_own;
-  }
+  dgo[qd * C + i] = dg_own;
+  dbo[qd * C + i] = db_own;
   tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
@@ -707,8 +670,8 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
     for (int wv = 0; wv < 8; ++wv) { base += red[wv]; kp += red[8 + wv]; }
     base = L * base + kp;
     const int ra = C - 1 - 2 * tid, rb = ra - 1;
-    float a = dgo[ra] + dgo[C + ra];
-    float bq = dgo[rb] + dgo[C + rb];
+    float a = (dgo[ra] + dgo[C + ra]) + (dgo[2 * C + ra] + dgo[3 * C + ra]);
+    float bq = (dgo[rb] + dgo[C + rb]) + (dgo[2 * C + rb] + dgo[3 * C + rb]);
     warp_rcumsum64(a, bq, tid);
     __syncwarp();  // every lane has read its rows before any lane overwrites them
     dgo[ra] = base + a;
@@ -717,7 +680,7 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   __syncthreads();
   if (!ok && tid == 0) atomicExch(p.status, 4);
   if (ok && tid < imax) {
-    p.dbeta[row(tid)] = dbo[tid] + dbo[C + tid];
+    p.dbeta[row(tid)] = (dbo[tid] + dbo[C + tid]) + (dbo[2 * C + tid] + dbo[3 * C + tid]);
     float dg = dgo[tid];
     const float gin = p.gate[row(tid)];
     if (p.gate_is_log) {
