@@ -225,53 +225,34 @@ __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  // D1[64 x 128] = (T beta) v -> u     (v contracted over its rows)
+  // u = (T beta) v and w = (T beta)(d k), contracted over the rows of v and k; weight-stationary: a thread has a row and
+  // half of the columns of both
   if (ok && tid == 0) {
-    tc::issue_gemm(taddr, tc::kmajor_tile(Tb, C), tc::mnmajor_sw128_tile(Akq + 8192, 16384), 64, KD, C, false);
+    tc::issue_gemm<true>(taddr, tc::kmajor_tile(Tb, C), tc::mnmajor_sw128_tile(Akq + 8192, 16384), 64, KD, C, false);
+    tc::issue_gemm<true>(taddr + 64, tc::kmajor_tile(Tb, C), tc::mnmajor_sw128_tile(Akq, 16384), 64, KD, C, false);
     tc::mma_commit(mbar);
     tc::bulk_store(p.Tm + ci * C * C, tc::smem_u32(Tt), 8192);  // T leaves as the byte image of its operand tile
     tc::bulk_commit();
   }
   if (ok) ok = tc::mbar_wait(mbar, 1);
   tc::fence_after_sync();
-  const int ir = 16 * warp + (lane & 15);  // M=64: row m sits in TMEM lane (m%16) + 32*(m/16)
   if (ok) {
-    // the u image (column-blocked: columns 0-63 and 64-127 are its two contiguous halves) over the v boxes
-    for (int c0 = 0; c0 < 128; c0 += 32) {
+    // the u image (column-blocked: columns 0-63 and 64-127 are its two contiguous halves) over the v boxes, and the w image
+    // in the 128-byte-swizzled layout of a TMA tile (two 8 KB slabs of 64 columns) over the k boxes, so that the state
+    // kernels can put it beside TMA-loaded q rows in one operand
+    const int ir = 32 * (warp & 1) + lane, c8 = 8 * (warp >> 1);
+#pragma unroll
+    for (int c0 = 0; c0 < 64; c0 += 32) {
       float f[32];
       ld_acc32(taddr, warp, c0, f);
-      if (lane < 16) {
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          const uint32_t off = tc::colblk_unit(ir, (c0 >> 3) + x, C);
-          sts16(Akq, 8192u + (off >> 13) * 16384u + (off & 8191u), pack8f(&f[8 * x]));
-        }
+      for (int x = 0; x < 4; ++x) {
+        const uint32_t off = tc::colblk_unit(ir, c8 + (c0 >> 3) + x, C);
+        sts16(Akq, 8192u + (off >> 13) * 16384u + (off & 8191u), pack8f(&f[8 * x]));
       }
-    }
-  }
-  tc::fence_async_smem();
-  tc::fence_before_sync();
-  __syncthreads();  // the accumulator columns have been read: the second product may overwrite them
-  tc::fence_after_sync();
-  // D1[64 x 128] = (T beta)(d k) -> w
-  if (ok && tid == 0) {
-    tc::issue_gemm(taddr, tc::kmajor_tile(Tb, C), tc::mnmajor_sw128_tile(Akq, 16384), 64, KD, C, false);
-    tc::mma_commit(mbar);
-    for (int hf = 0; hf < 2; ++hf) tc::bulk_store(p.u + ci * C * KD + hf * 4096, sAkq + 8192 + hf * 16384, 8192);
-    tc::bulk_commit();
-  }
-  if (ok) ok = tc::mbar_wait(mbar, 0);
-  tc::fence_after_sync();
-  if (ok) {
-    // the w image in the 128-byte-swizzled layout of a TMA tile (two 8 KB slabs of 64 columns), over the k boxes, so
-    // that the state kernels can put it beside TMA-loaded q rows in one operand
-    for (int c0 = 0; c0 < 128; c0 += 32) {
-      float f[32];
-      ld_acc32(taddr, warp, c0, f);
-      if (lane < 16) {
+      ld_acc32(taddr + 64, warp, c0, f);
 #pragma unroll
-        for (int x = 0; x < 4; ++x) sts16(Akq, kq_unit(ir, (c0 >> 3) + x), pack8f(&f[8 * x]));
-      }
+      for (int x = 0; x < 4; ++x) sts16(Akq, kq_unit(ir, c8 + (c0 >> 3) + x), pack8f(&f[8 * x]));
     }
   } else if (tid == 0) {
     atomicExch(p.status, 1);
@@ -281,7 +262,10 @@ __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid
   __syncthreads();
   if (tid == 0) {
     if (ok) {
-      for (int sl = 0; sl < 2; ++sl) tc::bulk_store(p.w + ci * C * KD + sl * 4096, sAkq + sl * 16384, 8192);
+      for (int hf = 0; hf < 2; ++hf) {
+        tc::bulk_store(p.u + ci * C * KD + hf * 4096, sAkq + 8192 + hf * 16384, 8192);
+        tc::bulk_store(p.w + ci * C * KD + hf * 4096, sAkq + hf * 16384, 8192);
+      }
       tc::bulk_commit();
     }
     tc::bulk_wait_read<0>();  // shared memory must outlive the copies

@@ -176,38 +176,34 @@ __global__ void __launch_bounds__(128, 6) gdn_tc_prep_kernel(TcP p, const __grid
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  // w = (T beta)(d k), then u = (T beta) v through the same accumulator columns
-  const int ir = 16 * warp + (lane & 15);  // M=64: row m sits in TMEM lane (m%16) + 32*(m/16)
-  for (int which = 0; which < 2; ++which) {
-    uint8_t* X = which ? Xq : Xk;
-    if (ok && tid == 0) {
-      tc::issue_gemm(taddr, tc::kmajor_tile(Tb, C), tc::mnmajor_sw128_tile(X, kTile), 64, W, C, false);
-      tc::mma_commit(mbar);
-      if (which) tc::bulk_store(p.w + ci * C * W, tc::smem_u32(Xk), kTile);
-      else if (p.save) tc::bulk_store(p.Tm + ci * C * C, tc::smem_u32(Tt), kTile);
-      tc::bulk_commit();
-    }
-    if (ok) ok = tc::mbar_wait(mbar, 1 ^ which);
-    tc::fence_after_sync();
-    if (ok) {
-      for (int c0 = 0; c0 < 64; c0 += 32) {
-        float f[32];
-        ld_acc32(taddr, warp, c0, f);
-        if (lane < 16) {
-#pragma unroll
-          for (int x = 0; x < 4; ++x)  // the w image is swizzled, the u image is not
-            sts16(X, which ? tc::kmajor_unit(ir, (c0 >> 3) + x, W) : sw_unit(ir, (c0 >> 3) + x), pack8(&f[8 * x]));
-        }
-      }
-    }
-    tc::fence_async_smem();
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
+  // w = (T beta)(d k) and u = (T beta) v, weight-stationary: a thread has a row and half of the columns of both
+  if (ok && tid == 0) {
+    tc::issue_gemm<true>(taddr, tc::kmajor_tile(Tb, C), tc::mnmajor_sw128_tile(Xk, kTile), 64, W, C, false);
+    tc::issue_gemm<true>(taddr + 32, tc::kmajor_tile(Tb, C), tc::mnmajor_sw128_tile(Xq, kTile), 64, W, C, false);
+    tc::mma_commit(mbar);
+    if (p.save) tc::bulk_store(p.Tm + ci * C * C, tc::smem_u32(Tt), kTile);
+    tc::bulk_commit();
   }
-  if (!ok && tid == 0) atomicExch(p.status, 1);
+  if (ok) ok = tc::mbar_wait(mbar, 1);
+  tc::fence_after_sync();
+  if (ok) {
+    const int ir = 32 * (warp & 1) + lane, c8 = 4 * (warp >> 1);
+    float f[32];
+    ld_acc32(taddr, warp, 0, f);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) sts16(Xk, sw_unit(ir, c8 + x), pack8(&f[8 * x]));  // the w image is swizzled, the u image is not
+    ld_acc32(taddr + 32, warp, 0, f);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) sts16(Xq, tc::kmajor_unit(ir, c8 + x, W), pack8(&f[8 * x]));
+  } else if (tid == 0) {
+    atomicExch(p.status, 1);
+  }
+  tc::fence_async_smem();
+  tc::fence_before_sync();
+  __syncthreads();
   if (tid == 0) {
     if (ok) {
+      tc::bulk_store(p.w + ci * C * W, tc::smem_u32(Xk), kTile);
       tc::bulk_store(p.u + ci * C * W, tc::smem_u32(Xq), kTile);
       tc::bulk_commit();
     }
@@ -584,13 +580,15 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_state_bwd_kernel(TcP p, const _
 // ---------------------------------------------------------- chunk backward
 // One CTA per chunk, everything that is not the sequential pass (gdn_tc_bwd.cu has the formulas).  Five batches:
 //   1  -e = T^T (-dv_new)          dP = dO v_new^T            -> dPG
-//   2  z = (-e) S0^T               v_new dS^T                 -> dkp = r (.)     <dS, S0> on the side
-//   3  (-e) v^T                    z k^T                      -> Y
-//   4  Y T^T                       k k^T                      -> Mb
-//   5  dPG^T q + (Mb + Mb^T) k     (d dO) S0^T + dPG k        -> dk, dq
-// 128 TMEM columns (two products at a time) and 73 KB: three CTAs per SM.  Buffers: dO -> d dO; -dv_new -> -e -> dv;
-// v_new -> v -> q -> dq; dS -> k; T -> dk; dkp stays in registers.
-constexpr int kChunkSmem = 9 * kTile + 8 * C * 4 + 16 * 4 + 64 + 64;
+//   2  z = (-e) S0^T               v_new dS^T                 -> dkp = r (.)     <dS, S0> on the side; (d dO) S0^T
+//   3  (-e) v^T                    z k^T                      -> Y;  k k^T
+//   4  Y T^T                                                  -> Mb
+//   5  dPG^T q + (Mb + Mb^T) k     DQ += dPG k                -> dk, dq
+// 128 TMEM columns (weight-stationary products take 32 each) and 75 KB: three CTAs per SM.  A thread has a row and a
+// quarter of the columns of every result.  Buffers: dO -> d dO; -dv_new -> -e -> dv; v_new -> v -> q -> dq; dS -> k;
+// T -> dk; Mb -> row partials; dkp stays in registers.
+// 16 x 2048 x 16 heads: 220 us with half of the lanes idle in the epilogues, 184 now (HBM: 1.1 GB, 164 us).
+constexpr int kChunkSmem = 9 * kTile + 4 * C * 4 + 16 * 4 + 64 + 64;
 static_assert(3 * (kChunkSmem + 1024) <= 228 * 1024, "three CTAs per SM");
 
 __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
@@ -608,9 +606,9 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
   float* bet = gam + C;
   float* dd = bet + C;
   float* rr = dd + C;
-  float* dgo = rr + C;            // [2][C] per-row dgam / dbeta partials of the two column halves
-  float* dbo = dgo + 2 * C;
-  float* red = dbo + 2 * C;       // [0,8) <dS,S0> per warp, [8,16) sum of k.dkp per warp
+  float* dgo = reinterpret_cast<float*>(Xy);  // [4][C] per-row dgam / dbeta partials of the column quarters, over Mb
+  float* dbo = dgo + 4 * C;
+  float* red = rr + C;            // [0,8) <dS,S0> per warp, [8,16) sum of k.dkp per warp
   uint64_t* mbar = reinterpret_cast<uint64_t*>(red + 16);  // [0] MMA; loads: [1] first tiles, [2] S0 and dS, [3] k and v, [4] q
   uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 8);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -618,18 +616,14 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
   const size_t ci = (size_t)bh * p.n + c;
   const int imax = min(C, p.T - t0);
   auto row = [&](int i) { return ((size_t)(b * p.T + t0 + i) * p.H + h); };
-  const bool own = lane < 16;
-  const int i = 16 * (warp & 3) + (lane & 15);  // the row this thread works on in every epilogue
-  const int hc = warp >> 2, cb = 32 * hc;       // warps 0-3 take the first 32 columns of an accumulator, warps 4-7 the rest
-  const int hx = lane >> 4, j0 = cb + 16 * hx;  // 16 of them per lane, after the owner has handed half to its twin
-  // a block of 32 accumulator columns, this lane's 16 of them
-  auto block = [&](uint32_t taddr, float (&v)[16]) {
-    float f[32];
-    ld_acc32(taddr, warp, cb, f);
+  // this thread's row and 16 columns of every result
+  const int i = 32 * (warp & 1) + lane, qd = (warp & 2) + (warp >> 2), j0 = 16 * qd;
+  auto block = [&](uint32_t taddr, float (&v)[16]) { ld_acc16(taddr, warp, 16 * (warp >> 2), v); };
+  auto row16 = [&](const float* v, float (&e)[16]) {  // per-row scalars of the same 16 columns
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const float up = __shfl_sync(0xffffffffu, f[16 + q], lane & 15);
-      v[q] = hx ? up : f[q];
+    for (int x = 0; x < 4; ++x) {
+      const float4 q = *reinterpret_cast<const float4*>(v + j0 + 4 * x);
+      e[4 * x] = q.x; e[4 * x + 1] = q.y; e[4 * x + 2] = q.z; e[4 * x + 3] = q.w;
     }
   };
 
@@ -665,14 +659,14 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
     dd[tid] = exp_nonpos(gam[tid]);
     rr[tid] = exp_nonpos(glast - gam[tid]);
   }
-  const uint32_t tA = *tslot, tB = tA + 64;
+  const uint32_t tA = *tslot, tB = tA + 32, tK = tA + 64, tQ = tA + 96;
   uint32_t ph = 0;
   bool ok = (tc::smem_u32(sm) & 1023u) == 0 && tc::mbar_wait(mbar + 1, 0);
   auto wait_mma = [&]() {
     if (ok) ok = tc::mbar_wait(mbar, ph);
     ph ^= 1;
     tc::fence_after_sync();
-    ok = __all_sync(0xffffffffu, ok);  // warp-uniform: the epilogues shuffle with a full mask
+    ok = __all_sync(0xffffffffu, ok);  // warp-uniform: whole warps read the accumulators
   };
   auto publish = [&]() {  // shared-memory writes -> operands of the next batch
     tc::fence_async_smem();
@@ -682,8 +676,8 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
   };
   // ---- batch 1 ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tA, tc::mnmajor_tile(Xt, C), tc::mnmajor_tile(Xe, W), 64, W, C, false);
-    tc::issue_gemm(tB, tc::kmajor_sw128_tile(XdO, kTile), tc::kmajor_tile(Xvn, W), 64, 64, W, false);
+    tc::issue_gemm<true>(tA, tc::mnmajor_tile(Xt, C), tc::mnmajor_tile(Xe, W), 64, W, C, false);
+    tc::issue_gemm<true>(tB, tc::kmajor_sw128_tile(XdO, kTile), tc::kmajor_tile(Xvn, W), 64, 64, W, false);
     tc::mma_commit(mbar);
   }
   __syncthreads();  // dd, rr visible
@@ -695,9 +689,11 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
 #pragma unroll
     for (int x = 0; x < 2; ++x) sts16(Xe, sw_unit(i, (j0 >> 3) + x), pack8(&v[8 * x]));
     block(tB, v);  // dP Gamma, lower triangle incl. diagonal
+    float gj[16];
+    row16(gam, gj);
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
-      const float val = v[q] * exp_nonpos(gi - gam[j0 + q]);  // unconditional: the exponentials overlap
+      const float val = v[q] * exp_nonpos(gi - gj[q]);  // unconditional: the exponentials overlap
       v[q] = (j0 + q <= i) ? val : 0.f;
     }
 #pragma unroll
@@ -708,8 +704,9 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
   publish();
   // ---- batch 2 ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tA, tc::kmajor_sw128_tile(Xe, kTile), tc::kmajor_tile(Xs, W), 64, W, W, false);
-    tc::issue_gemm(tB, tc::kmajor_tile(Xvn, W), tc::kmajor_tile(Xk, W), 64, W, W, false);
+    tc::issue_gemm<true>(tA, tc::kmajor_sw128_tile(Xe, kTile), tc::kmajor_tile(Xs, W), 64, W, W, false);
+    tc::issue_gemm<true>(tB, tc::kmajor_tile(Xvn, W), tc::kmajor_tile(Xk, W), 64, W, W, false);
+    tc::issue_gemm<true>(tQ, tc::kmajor_sw128_tile(XdO, kTile), tc::kmajor_tile(Xs, W), 64, W, W, false);
     tc::mma_commit(mbar);
   }
   {  // <dS, S0>
@@ -749,9 +746,10 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
   publish();
   // ---- batch 3 ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tA, tc::kmajor_sw128_tile(Xe, kTile), tc::kmajor_sw128_tile(Xvn, kTile), 64, 64, W, false);
-    tc::issue_gemm(tB, tc::kmajor_tile(Xz, W), tc::kmajor_sw128_tile(Xk, kTile), 64, 64, W, false);
+    tc::issue_gemm<true>(tA, tc::kmajor_sw128_tile(Xe, kTile), tc::kmajor_sw128_tile(Xvn, kTile), 64, 64, W, false);
+    tc::issue_gemm<true>(tB, tc::kmajor_tile(Xz, W), tc::kmajor_sw128_tile(Xk, kTile), 64, 64, W, false);
     tc::mma_commit(mbar);
+    tc::issue_gemm<true>(tK, tc::kmajor_sw128_tile(Xk, kTile), tc::kmajor_sw128_tile(Xk, kTile), 64, 64, W, false);  // for batch 4
   }
   float vdot = 0.f, kz = 0.f;  // e_i . v_i and k_i . z_i: the diagonals of the two products
   wait_mma();
@@ -764,10 +762,11 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
       vdot = (j0 + q == i) ? -ha[q] : vdot;
       kz = (j0 + q == i) ? hb[q] : kz;
     }
-    vdot += __shfl_xor_sync(0xffffffffu, vdot, 16);
-    kz += __shfl_xor_sync(0xffffffffu, kz, 16);
+    float bj[16], dj[16];
+    row16(bet, bj);
+    row16(dd, dj);
 #pragma unroll
-    for (int q = 0; q < 16; ++q) ha[q] = bet[j0 + q] * fmaf(dd[j0 + q], hb[q], -ha[q]);
+    for (int q = 0; q < 16; ++q) ha[q] = bj[q] * fmaf(dj[q], hb[q], -ha[q]);
 #pragma unroll
     for (int x = 0; x < 2; ++x) sts16(Xy, tc::kmajor_unit(i, (j0 >> 3) + x, C), pack8(&ha[8 * x]));
   }
@@ -778,8 +777,7 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
   }
   // ---- batch 4 ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tA, tc::kmajor_tile(Xy, C), tc::kmajor_tile(Xt, C), 64, 64, C, false);
-    tc::issue_gemm(tB, tc::kmajor_sw128_tile(Xk, kTile), tc::kmajor_sw128_tile(Xk, kTile), 64, 64, W, false);
+    tc::issue_gemm<true>(tA, tc::kmajor_tile(Xy, C), tc::kmajor_tile(Xt, C), 64, 64, C, false);
     tc::mma_commit(mbar);
   }
   if (ok)  // -e has served as an operand for the last time: dv = beta e in place
@@ -790,39 +788,36 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
   wait_mma();
   float db_own = 0.f, dg_own = 0.f;
   if (ok) {  // Xy <- Mb = beta_i M, M = -dA Gamma strictly lower, zeros elsewhere
-    float ha[16], hk[16], rs = 0.f;
+    float ha[16], hk[16], gj[16], rs = 0.f;
     block(tA, ha);
-    block(tB, hk);
+    block(tK, hk);
+    row16(gam, gj);
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
-      const float mv = -ha[q] * exp_nonpos(gi - gam[j0 + q]);
+      const float mv = -ha[q] * exp_nonpos(gi - gj[q]);
       const float M = (j0 + q < i) ? mv : 0.f;
       rs = fmaf(M, hk[q], rs);
       ha[q] = bi * M;
     }
 #pragma unroll
     for (int x = 0; x < 2; ++x) sts16(Xy, tc::kmajor_unit(i, (j0 >> 3) + x, C), pack8(&ha[8 * x]));
-    rs += __shfl_xor_sync(0xffffffffu, rs, 16);
-    if (own) {
-      db_own = vdot + di * kz + rs;
-      dg_own = 2.f * bi * (di * kz + rs);
-    }
+    db_own = vdot + di * kz + rs;
+    dg_own = 2.f * bi * (di * kz + rs);
   }
   if (ok) ok = tc::mbar_wait(mbar + 4, 0);  // q
   publish();
   // ---- batch 5 ----
   if (ok && tid == 0) {
-    tc::issue_gemm(tA, tc::mnmajor_tile(Xpg, C), tc::mnmajor_sw128_tile(Xvn, kTile), 64, W, C, false);
-    tc::issue_gemm(tA, tc::kmajor_tile(Xy, C), tc::mnmajor_sw128_tile(Xk, kTile), 64, W, C, true);
-    tc::issue_gemm(tA, tc::mnmajor_tile(Xy, C), tc::mnmajor_sw128_tile(Xk, kTile), 64, W, C, true);
-    tc::issue_gemm(tB, tc::kmajor_sw128_tile(XdO, kTile), tc::kmajor_tile(Xs, W), 64, W, W, false);
-    tc::issue_gemm(tB, tc::kmajor_tile(Xpg, C), tc::mnmajor_sw128_tile(Xk, kTile), 64, W, C, true);
+    tc::issue_gemm<true>(tA, tc::mnmajor_tile(Xpg, C), tc::mnmajor_sw128_tile(Xvn, kTile), 64, W, C, false);
+    tc::issue_gemm<true>(tA, tc::kmajor_tile(Xy, C), tc::mnmajor_sw128_tile(Xk, kTile), 64, W, C, true);
+    tc::issue_gemm<true>(tA, tc::mnmajor_tile(Xy, C), tc::mnmajor_sw128_tile(Xk, kTile), 64, W, C, true);
+    tc::issue_gemm<true>(tQ, tc::kmajor_tile(Xpg, C), tc::mnmajor_sw128_tile(Xk, kTile), 64, W, C, true);
     tc::mma_commit(mbar);
   }
   wait_mma();
   float rho = 0.f;
   if (ok) {
-    float v[16], kd = 0.f, qd = 0.f;
+    float v[16], kd = 0.f, qdot = 0.f;
     block(tA, v);
 #pragma unroll
     for (int x = 0; x < 2; ++x) {  // dk = dkp + (dPG^T q + (Mb + Mb^T) k) + beta d z, over T
@@ -840,28 +835,24 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
       }
       sts16(Xt, sw_unit(i, c8), pack8(&v[8 * x]));
     }
-    block(tB, v);
+    block(tQ, v);
 #pragma unroll
     for (int x = 0; x < 2; ++x) {  // dq, assembled over q (each thread rewrites the units it read)
       const int c8 = (j0 >> 3) + x;
       float qr[8];
       unpack8(*reinterpret_cast<const uint4*>(Xvn + sw_unit(i, c8)), qr);
 #pragma unroll
-      for (int y = 0; y < 8; ++y) qd = fmaf(qr[y], v[8 * x + y], qd);
+      for (int y = 0; y < 8; ++y) qdot = fmaf(qr[y], v[8 * x + y], qdot);
       sts16(Xvn, sw_unit(i, c8), pack8(&v[8 * x]));
     }
-    rho += __shfl_xor_sync(0xffffffffu, rho, 16);
-    const float s = qd - kd;
-    dg_own += s + __shfl_xor_sync(0xffffffffu, s, 16);
+    dg_own += qdot - kd;
   }
   {
-    const float tot = warp_sum(own ? rho : 0.f);
+    const float tot = warp_sum(rho);
     if (lane == 0) red[8 + warp] = tot;  // summed in a fixed order below
   }
-  if (own) {  // the two column halves hold partial sums of the same row
-    dgo[hc * C + i] = dg_own;
-    dbo[hc * C + i] = db_own;
-  }
+  dgo[qd * C + i] = dg_own;  // (every product that read Mb has completed)
+  dbo[qd * C + i] = db_own;
   publish();
   if (ok && tid == 64) {  // rows past the end of the sequence are clipped
     tc::tma_store_4d(&maps.dq, tc::smem_u32(Xvn), 0, h, t0, b);
@@ -874,8 +865,8 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
     for (int wv = 0; wv < 8; ++wv) { base += red[wv]; kp += red[8 + wv]; }
     base = L * base + kp;
     const int ra = C - 1 - 2 * tid, rb = ra - 1;
-    float a = dgo[ra] + dgo[C + ra];
-    float bq = dgo[rb] + dgo[C + rb];
+    float a = (dgo[ra] + dgo[C + ra]) + (dgo[2 * C + ra] + dgo[3 * C + ra]);
+    float bq = (dgo[rb] + dgo[C + rb]) + (dgo[2 * C + rb] + dgo[3 * C + rb]);
     warp_rcumsum64(a, bq, tid);
     __syncwarp();
     dgo[ra] = base + a;
@@ -884,7 +875,7 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
   __syncthreads();
   if (!ok && tid == 0) atomicExch(p.status, 4);
   if (ok && tid < imax) {
-    p.dbeta[row(tid)] = dbo[tid] + dbo[C + tid];
+    p.dbeta[row(tid)] = (dbo[tid] + dbo[C + tid]) + (dbo[2 * C + tid] + dbo[3 * C + tid]);
     float dg = dgo[tid];
     const float gin = p.gate[row(tid)];
     if (p.gate_is_log) {
