@@ -132,6 +132,7 @@ __device__ __forceinline__ void ld_acc64(uint32_t taddr, int warp, float (&f)[64
 }
 __device__ __forceinline__ void ld_accN(uint32_t taddr, int warp, float (&f)[64]) { ld_acc64(taddr, warp, f); }
 __device__ __forceinline__ void ld_accN(uint32_t taddr, int warp, float (&f)[32]) { ld_acc32(taddr, warp, 0, f); }
+__device__ __forceinline__ void ld_accN(uint32_t taddr, int warp, float (&f)[16]) { ld_acc16(taddr, warp, 0, f); }
 // T = (I - A)^-1 in fp32, in place over the strictly lower triangular [64][LDA] matrix A; 128 threads, `other(t)` is run
 // by threads 64 + t beside the first step.  The four 16 x 16 diagonal blocks by forward substitution (thread = block and
 // column, the column in registers), then pairs of blocks are joined twice, T21 = T22 (A21 T11): 16-wide for both halves

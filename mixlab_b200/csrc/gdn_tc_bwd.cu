@@ -36,7 +36,7 @@ namespace mxb {
 //
 // Bound by the chain dS -> k dS -> dv_new -> w^T dv_new -> dS where the heads are few, by HBM where they fill the GPU.
 // P^T dO and (d q)^T dO need no dS: those of chunk c-1 are issued behind w^T dv_new of chunk c and run while dS is
-// updated, and q is scaled in the shadow of the k dS before (16 heads of 128, NV = 64: 2.6 -> 1.8 us a chunk).
+// updated, and q is scaled in the shadow of the k dS before (16 heads of 128, NV = 64: 2.6 -> 1.7 us a chunk).
 // (An issuing warp of its own, as in the forward pass, was slower here: 1.8 -> 2.1 us.)
 //
 // TMA = true: the k, dO and q rows arrive as tensor-map boxes (128-byte swizzle, two 8 KB slabs of 64 columns per
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
   // P^T dO and (d q)^T dO of chunk c (accumulators at 128 and at 256 or 384)
   auto issue_dO = [&](int c) {
     const tc::Tile dO = tc::mnmajor_sw128_tile(dOop + (c & 1) * 128 * NV, 8192);
-    tc::issue_gemm(taddr + 128, tc::mnmajor_tile(Pt + (c & 1) * 8192, C), dO, 64, NV, C, false);
+    tc::issue_gemm<true>(taddr + 128, tc::mnmajor_tile(Pt + (c & 1) * 8192, C), dO, 64, NV, C, false);
     tc::issue_gemm(taddr + 256 + 128 * (c & 1), tc::mnmajor_sw128_tile(Aq + (c & 1) * 16384, 8192), dO, 128, NV, C, false);
   };
   {  // the last chunk's q is scaled here; every later one a chunk ahead
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
     tc::fence_after_sync();
     if (tid == 0) {
       if (c == p.n - 1) issue_dO(c);
-      tc::issue_gemm(taddr, tc::kmajor_sw128_tile(Ak + buf * 16384, 8192), tc::colblk_mnmajor_tile(dSop, KD), 64, NV, KD, false);  // k dS
+      tc::issue_gemm<true>(taddr, tc::kmajor_sw128_tile(Ak + buf * 16384, 8192), tc::colblk_mnmajor_tile(dSop, KD), 64, NV, KD, false);  // k dS
       tc::mma_commit(mbar);
       // dS at chunk end, as the operand-tile image
       tc::bulk_store(p.dhs + ci * KD * KD + KD * col0, tc::smem_u32(dSop), 256 * NV);
@@ -215,23 +215,20 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
     tc::fence_after_sync();
     issue_A(c - 2);
     if (ok) {
-      const int i = 16 * (warp & 3) + (lane & 15);  // M=64 accumulators: row i in TMEM lane (i%16) + 32*(i/16)
+      // weight-stationary: this thread's row and quarter of the columns (the second half of them in lanes 64-127)
+      constexpr int NQ = NV / 4;
+      const int i = 32 * (warp & 1) + lane, tc0 = NQ * (warp >> 2), c8 = NV / 16 * ((warp >> 1) & 1) + NQ / 8 * (warp >> 2);
       const float ri = rr[i];
-      for (int c0 = 0; c0 < NC; c0 += 32) {
-        float fa[32], fb[32];
-        ld_acc32(taddr + j0, warp, c0, fa);
-        ld_acc32(taddr + 128 + j0, warp, c0, fb);
-        if (lane < 16) {
+      float fa[NQ], fb[NQ];
+      ld_accN(taddr + tc0, warp, fa);
+      ld_accN(taddr + 128 + tc0, warp, fb);
 #pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            float e[8];
+      for (int x = 0; x < NQ / 8; ++x) {
+        float e[8];
 #pragma unroll
-            for (int y = 0; y < 8; ++y) e[y] = -fmaf(ri, fa[8 * x + y], fb[8 * x + y]);
-            const int c8 = NC / 8 * half + (c0 >> 3) + x;
-            sts16(Bd, tc::colblk_unit(i, c8, C), make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]),
-                                                             tc::pack_bf16(e[4], e[5]), tc::pack_bf16(e[6], e[7])));
-          }
-        }
+        for (int y = 0; y < 8; ++y) e[y] = -fmaf(ri, fa[8 * x + y], fb[8 * x + y]);
+        sts16(Bd, tc::colblk_unit(i, c8 + x, C), make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]),
+                                                            tc::pack_bf16(e[4], e[5]), tc::pack_bf16(e[6], e[7])));
       }
     }
     if (tid == 0) tc::bulk_wait_read<0>();  // the dS image has left its tile
