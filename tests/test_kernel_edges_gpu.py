@@ -1,0 +1,147 @@
+"""The kernels' own edges: shapes around tiles, windows, runs and the lines of the dispatch, against the CPU oracle."""
+import ctypes as C
+
+import pytest
+import torch
+
+import mixlab_b200
+from mixlab_b200 import _lib, ops
+from oracle import gdn, inputs
+from tests import test_gdn_block_gpu as blocks
+from tests import test_mamba3_gpu as mamba
+from tests.util import assert_close
+
+pytestmark = pytest.mark.gpu
+F32, BF16 = torch.float32, torch.bfloat16
+TOL = {F32: 1e-4, BF16: 2e-2}
+GRADS = ("dq", "dk", "dv", "dbeta", "dgate", "dh0")
+
+
+def _dev(t):
+    return t.to("cuda").contiguous()
+
+
+def _check_scan(B, T, H, K, V, io, chunk=64, offset=0):
+    """Forward, backward with recompute and backward from the saved forward, with both states, at `offset` elements from
+    an aligned base."""
+    a = inputs.gdn_inputs(B, T, H, K, V, seed=91, io_dtype=io, with_grad_out=True, with_h0=True)
+    f = {n: t.double() for n, t in a.items()}
+    want = gdn.scan_grads(f["q"], f["k"], f["v"], f["beta"], f["g"], f["d_out"], f["d_state"], f["h0"], gate_is_log=True)
+
+    def put(t):
+        if not offset:
+            return _dev(t)
+        flat = torch.empty(t.numel() + offset, dtype=t.dtype, device="cuda")[offset:]
+        return flat.copy_(t.reshape(-1)).view(t.shape)
+
+    args = tuple(put(a[n]) for n in ("q", "k", "v", "beta", "g"))
+    d_out, h0, d_state = put(a["d_out"]), _dev(a["h0"]), _dev(a["d_state"])
+    kw = dict(gate_is_log=True, h0=h0)
+    ref = ops.gated_delta_scan_backward(*args, d_out, chunk, d_final_state=d_state, **kw)
+    ref = {n: ref[n].clone() for n in GRADS}
+    o, s = ops.gated_delta_scan(*args, chunk, return_final_state=True, **kw)
+    saved = ops.gated_delta_scan(*args, chunk, save_for_backward=True, **kw)
+    got = ops.gated_delta_scan_backward(*args, d_out, chunk, d_final_state=d_state, use_saved=True, **kw)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    assert torch.equal(o, saved)
+    assert_close(o, want["out"], TOL[io], "out")
+    assert_close(s, want["state"], TOL[io], "final_state")
+    for n in GRADS:
+        assert torch.equal(got[n], ref[n]), n
+        assert_close(got[n], want[n], TOL[io], n)
+
+
+@pytest.mark.parametrize("shape,chunk,offset", [
+    ((1, 65, 1, 16, 24), 64, 0),       # narrowest column slabs, ragged in columns and steps
+    ((2, 64, 2, 128, 128), 64, 0),     # two K tiles, whole chunks
+    ((3, 63, 4, 96, 40), 64, 0),       # middle slab width, K between the tiles
+    ((8, 66, 8, 64, 64), 64, 0),       # enough heads for the widest slabs
+    ((1, 70, 2, 18, 20), 64, 0),       # rows that no tensor copy can move
+    ((1, 70, 2, 16, 24), 64, 1),       # nor from such a base
+    ((2, 70, 2, 32, 16), 16, 0), ((1, 1, 1, 8, 8), 64, 0),
+])
+def test_float32_scan(shape, chunk, offset):
+    _check_scan(*shape, F32, chunk, offset)
+
+
+@pytest.mark.parametrize("shape", [
+    (1, 1, 1, 128, 128), (1, 64, 2, 128, 96), (2, 129, 3, 96, 72), (1, 193, 2, 64, 128),   # split columns
+    (2, 65, 37, 128, 128),             # the most heads that split
+    (3, 65, 25, 128, 128),             # the fewest that do not
+    (1, 1, 1, 64, 64), (2, 63, 3, 64, 64), (1, 64, 2, 64, 64), (1, 130, 5, 64, 64),        # 64-wide kernels
+])
+def test_tensor_core_scan(shape):
+    _check_scan(*shape, BF16)
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 4, 4), (2, 3, 256, 8), (1, 2, 64, 36), (2, 2, 100, 28), (1, 1, 128, 256),
+                                  (70, 5, 64, 96)])
+@pytest.mark.parametrize("io", [F32, BF16])
+def test_decode_slabs(dims, io):
+    N, H, K, V = dims
+    a = inputs.gdn_decode_inputs(N, H, K, V, 1, seed=92, io_dtype=io)
+    x = {n: a[n][0] for n in ("q", "k", "v", "beta", "g")}
+    o_ref, st_ref = gdn.decode_step(a["state"].double(), x["q"].double(), x["k"].double(), x["v"].double(),
+                                    x["beta"].double(), torch.exp(x["g"].double()))
+    st = _dev(a["state"].clone())
+    o = ops.gated_delta_decode_step(st, *(_dev(x[n]) for n in ("q", "k", "v", "beta", "g")), gate_is_log=True)
+    assert_close(o, o_ref, TOL[io], "out")
+    assert_close(st, st_ref, TOL[F32], "state")
+
+
+@pytest.mark.parametrize("cfg", [(1, 31, 1, 64, 64), (1, 33, 5, 8, 64), (2, 129, 2, 64, 8), (1, 65, 3, 32, 48)])
+@pytest.mark.parametrize("io", [F32, BF16])
+def test_block_stages(cfg, io):
+    """Runs of steps that end inside a sequence, rows narrower than a warp, queries and values of different widths."""
+    blocks.test_block_pre_forward_and_gradients(cfg, io, True)
+    B, T, H, _, V = cfg
+    blocks.test_block_post_forward_and_gradients((B, T, H, V), io)
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 4, 8, 1), (1, 7, 4, 16, 1), (2, 8, 8, 16, 2), (1, 9, 4, 32, 1),
+                                   (1, 24, 4, 64, 1), (1, 17, 2, 256, 1), (1, 15, 4, 6, 1), (1, 41, 3, 128, 1)])
+def test_mamba3_windows(shape):
+    """Windows of eight steps: none full, exactly full, one step over; vector and scalar rows, each lane count."""
+    mamba.test_window_parallel_matches_serial_walk(shape)
+    B, T, D, N, G = shape
+    a = inputs.mamba3_inputs(B, T, D, 1, N, G=G, seed=93, per_head=False)
+    dev, dy = [_dev(a[n]) for n in mamba.ARGS], _dev(a["dy"])
+    kw = dict(flags=_lib.MXB_MAMBA3_WINDOW_PARALLEL)
+    want = {n: t.clone() for n, t in ops.mamba3_selective_scan_backward(*dev, dy, **kw).items()}
+    ops.mamba3_selective_scan(*dev, save_for_backward=True, **kw)
+    got = ops.mamba3_selective_scan_backward(*dev, dy, use_saved=True, **kw)
+    for n in mamba.GRADS:
+        assert torch.equal(got[n], want[n]), n
+
+
+@pytest.mark.parametrize("cfg", [(1, 63, 1, 1), (2, 65, 3, 3), (1, 129, 2, 2)])
+def test_mamba3_chunks(cfg):
+    """Chunks of 64 steps, one short, one over; one head per group."""
+    mamba.test_chunked_tensor_core_kernels(cfg)
+
+
+@pytest.mark.parametrize("B,T,H,arena_mb", [(1, 130, 4, 256), (4, 600, 8, 256), (4, 600, 8, 40), (2, 2100, 8, 256)])
+def test_host_slicing(B, T, H, arena_mb):
+    """Slices of whole sequences and of groups of heads, two to four in flight, and finer ones where the arena is small:
+    the results of the device entry points, bit for bit."""
+    lib = mixlab_b200.lib()
+    a = inputs.gdn_inputs(B, T, H, 128, 128, seed=94, io_dtype=BF16, with_grad_out=True)
+    names = ("q", "k", "v", "beta", "g")
+    dev = [_dev(a[n]) for n in names]
+    want = dict(out=ops.gated_delta_scan(*dev, 64, gate_is_log=True).clone())
+    want.update(ops.gated_delta_scan_backward(*dev, _dev(a["d_out"]), 64, gate_is_log=True))
+    host = {n: a[n].contiguous().pin_memory() for n in names + ("d_out",)}
+    res = {n: torch.empty_like(host[m]).pin_memory() for n, m in
+           (("out", "v"), ("dq", "q"), ("dk", "k"), ("dv", "v"), ("dbeta", "beta"), ("dgate", "g"))}
+    p = lambda t: C.c_void_p(t.data_ptr())
+    ctx = C.c_void_p()
+    assert lib.mxb_host_ctx_create(0, arena_mb << 20, C.byref(ctx)) == 0
+    try:
+        d = mixlab_b200.GdnDesc(B, T, H, 128, 128, 64, mixlab_b200.MXB_BF16, 1, 0)
+        assert lib.mxb_host_gdn(ctx, C.byref(d), *(p(host[n]) for n in names), p(res["out"]), p(host["d_out"]),
+                                *(p(res[n]) for n in ("dq", "dk", "dv", "dbeta", "dgate"))) == 0
+    finally:
+        lib.mxb_host_ctx_destroy(ctx)
+    for n, t in res.items():
+        assert torch.equal(t, want[n].cpu()), n
