@@ -57,18 +57,18 @@ M3_BLOCK_BYTES_PER_TOKEN = lambda D, GN: (13 * D + 10 * GN) * 2
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum, MB per launch at the full workload size) per kernel, from
 # one ncu byte capture of a step.  Keyed by kernel name: when the kernels a step launches are not exactly these, the
 # capture no longer describes the step and roofline.traffic is reported as null instead of a stale number.
-GDN_NCU_TRAFFIC_MB = {   # captured at B=4 (4096 units); at B=8 a little less of the producer -> consumer tiles stays in L2
-    "gdn_tc_prep_kernel": 353.9, "gdn_tc_state_fwd_kernel": 524.6, "gdn_tc_state_bwd_kernel": 464.9,
-    "gdn_tc_chunk_bwd_kernel": 886.5,
+GDN_NCU_TRAFFIC_MB = {   # captured at B=6, T=2048; a larger step keeps a little less of the producer -> consumer tiles in L2
+    "gdn_tc_prep_kernel": 252.4, "gdn_tc_state_fwd_kernel": 378.9, "gdn_tc_state_bwd_kernel": 336.4,
+    "gdn_tc_chunk_bwd_kernel": 658.5,
 }
-GDN_NCU_TRAFFIC_UNITS = 4096     # (batch, head, chunk) units of the captured step
+GDN_NCU_TRAFFIC_UNITS = 3072     # (batch, head, chunk) units of the captured step
 M3_NCU_TRAFFIC_MB = {
     "m3s_scalars_kernel": 12.6, "m3s_chunk_scalars_kernel": 12.6, "m3s_state_pass_kernel": 390.3 + 390.4,
     "m3s_chunk_out_kernel": 566.2, "m3s_chunk_grad_kernel": 1494.2, "m3s_final_kernel": 33.6, "m3s_dalog_kernel": 0.0,
     "m3s_reduce_kernel": 548.0,
 }
 M3_NCU_TRAFFIC_UNITS = 16384
-DECODE_NCU_TRAFFIC_MB = {"gdn_decode_bulk_kernel": 482.8}
+DECODE_NCU_TRAFFIC_MB = {"gdn_decode_kernel": 483.7}
 DECODE_NCU_TRAFFIC_UNITS = 4096  # (sequence, head) tiles of the captured launch
 
 
