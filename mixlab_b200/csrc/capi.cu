@@ -2,6 +2,7 @@
 // context.  Declarations and the reference interfaces they replace are in
 // include/mixlab_b200.h.
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -638,20 +639,21 @@ __global__ void __launch_bounds__(256) head_scatter_kernel(const float* __restri
 // copy when both directions run (the strided row width makes no difference down to 512 bytes): with S slices of 4
 // copies, bytes / (S * 49 GB/s) + S * 44 us, least near S = sqrt(bytes / 2.25 MB).  More slices than that lost at
 // every size (2 x 2048 x 16 heads of 128: 2, 4, 8 slices 2161, 1852, 1980 us; 4 x 1024 x 16: 4, 8, 16 slices 1868,
-// 1855, 2500; 2 x 700 x 16: 2, 4, 8 slices 756, 793, 988; 1 x 200 x 8: 1, 2 slices 156, 181).
+// 1855, 2500; 2 x 700 x 16: 2, 4, 8 slices 756, 793, 988; 1 x 200 x 8: 1, 2 slices 156, 181;
+// 8 x 4096 x 16: 8, 16, 32 slices 13.6, 11.9, 12.7 ms).
 struct HostSlicing {
   int per, nsplit;  // sequences per slice; head groups per sequence (one sequence per slice then)
 };
 static HostSlicing host_slicing(const mxb_gdn_desc* d, size_t es) {
   const double bytes = 2.0 * d->B * d->T * d->H * ((double)d->Dk + d->Dv) * es;
-  int want = 1;
-  while (want < 16 && (want + 1.0) * (want + 1.0) * 2.25e6 <= bytes) ++want;
+  const double best = sqrt(bytes / 2.25e6) < 16.0 ? sqrt(bytes / 2.25e6) : 16.0;
+  const int want = best < 1.0 ? 1 : (int)best;
   HostSlicing h{(d->B + want - 1) / want, 1};
   // Head groups in halves, or in rows of a host page at least: with a quarter of a page per row every slice's copies
   // touch every page again, which some hosts translate slowly (1 x 4096 x 16 heads of 128, two and four groups: 2185
   // and 2014 us on one host, 2350 and 2709 on another).
   const size_t row = (size_t)d->H * (d->Dk < d->Dv ? d->Dk : d->Dv) * es;
-  while (d->B * 2 * h.nsplit <= want && d->H % (2 * h.nsplit) == 0 && (h.nsplit == 1 || row / (2 * h.nsplit) >= 4096))
+  while (h.per == 1 && d->B * 2 * h.nsplit <= 1.1 * best && d->H % (2 * h.nsplit) == 0 && (h.nsplit == 1 || row / (2 * h.nsplit) >= 4096))
     h.nsplit *= 2;
   return h;
 }
