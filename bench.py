@@ -64,8 +64,8 @@ GDN_NCU_TRAFFIC_MB = {   # captured at B=6, T=2048; a larger step keeps a little
 GDN_NCU_TRAFFIC_UNITS = 3072     # (batch, head, chunk) units of the captured step
 M3_NCU_TRAFFIC_MB = {
     "m3s_scalars_kernel": 12.6, "m3s_chunk_scalars_kernel": 12.6, "m3s_state_pass_kernel": 390.3 + 390.4,
-    "m3s_chunk_out_kernel": 566.2, "m3s_chunk_grad_kernel": 1494.2, "m3s_final_kernel": 33.6, "m3s_dalog_kernel": 0.0,
-    "m3s_reduce_kernel": 548.0,
+    "m3s_chunk_out_kernel": 566.2, "m3s_chunk_grad_kernel": 1494.2, "m3s_tail_kernel": 33.6 + 548.0,
+    "m3s_dalog_kernel": 0.0,
 }
 M3_NCU_TRAFFIC_UNITS = 16384
 DECODE_NCU_TRAFFIC_MB = {"gdn_decode_kernel": 483.7}

@@ -19,7 +19,8 @@
 //                           Brot^T diag(r e) X (or Crot^T diag(exp(Lam)) dY) folded into the running state
 //   m3s_chunk_out_kernel    per chunk: Y
 //   m3s_chunk_grad_kernel   per chunk: dx, rotated-row gradients -> dB, dC partials, per-token scalars
-//   m3s_final_kernel        per (b, head): suffix sum of the angle gradient, ddt, dlambda, dtheta, da_log
+//   m3s_tail_kernel         per (b, head): suffix sum of the angle gradient, ddt, dlambda, dtheta, da_log shares; per chunk:
+//                           dB, dC summed over the heads of a group
 #include <cuda.h>
 
 #include <cstring>
@@ -49,7 +50,7 @@ struct SsdP {
   float *dphi, *da, *de, *dgam; // [B,NH,T] per-token scalar gradients
   float* dal_part;              // [B,NH] per-batch shares of da_log
   float* cs;                    // [B,NH,n] ChunkScal records
-  bf16 *pb, *pc;                // [B,NH,n] column-blocked [64][128] images: per-head partial dB, dC (summed in fp32 by the reduce kernel)
+  bf16 *pb, *pc;                // [B,NH,n] column-blocked [64][128] images: per-head partial dB, dC (summed in fp32 by the tail kernel)
 };
 
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : (x < -20.f ? expf(x) : log1pf(expf(x))); }
@@ -897,10 +898,10 @@ __global__ void __launch_bounds__(256) m3s_chunk_grad_kernel(SsdP p, const __gri
 
 
 // ------------------------------------------------------------ final per-token scalars
-__global__ void __launch_bounds__(kScalThreads) m3s_final_kernel(SsdP p) {
+__device__ __forceinline__ void final_scalars(const SsdP& p, int head, int b) {
   __shared__ double wtot[kScalThreads / 32];
   __shared__ float wsum[kScalThreads / 32];
-  const int head = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+  const int tid = threadIdx.x;
   const size_t base = ((size_t)b * p.NH + head) * p.T;
   const float A = -expf(p.a_log[head]);
   const int per = (p.T + kScalThreads - 1) / kScalThreads, lo = tid * per, hi = min(p.T, lo + per);
@@ -961,21 +962,16 @@ __global__ void __launch_bounds__(kScalThreads) m3s_final_kernel(SsdP p) {
     p.dal_part[b * p.NH + head] = A * tot;  // summed over the batch in a fixed order by m3s_dalog_kernel
   }
 }
-__global__ void m3s_dalog_kernel(SsdP p) {
-  const int head = blockIdx.x * blockDim.x + threadIdx.x;
-  if (head >= p.NH) return;
-  float s = 0.f;
-  for (int b = 0; b < p.B; ++b) s += p.dal_part[b * p.NH + head];
-  p.da_log[head] = s;
-}
-
 // dB[b,t,g,:] = sum over the heads of group g of the per-head partial images (fp32, fixed order).  A thread owns eight
 // states of a row; consecutive threads hold consecutive rows, which are neighbours in the column-blocked images.
-__global__ void __launch_bounds__(128) m3s_reduce_kernel(const bf16* __restrict__ pb, const bf16* __restrict__ pc,
-                                                         bf16* __restrict__ db, bf16* __restrict__ dc, int T, int G, int NH,
-                                                         int n) {
-  const int c = blockIdx.x >> 4, which = blockIdx.x & 1, r = threadIdx.x & 63, c8 = (blockIdx.x & 14) + (threadIdx.x >> 6);
-  const int g = blockIdx.y, b = blockIdx.z, per = NH / G, t = c * Q + r;
+__device__ __forceinline__ void reduce_rows(const bf16* __restrict__ pb, const bf16* __restrict__ pc, bf16* __restrict__ db,
+                                            bf16* __restrict__ dc, int T, int G, int NH, int n, int block) {
+  static_assert(kScalThreads == N / 8 * Q, "a block covers one chunk of one gradient");
+  const int which = block & 1, r = threadIdx.x & 63, c8 = threadIdx.x >> 6;
+  int rest = block >> 1;
+  const int c = rest % n;
+  rest /= n;
+  const int g = rest % G, b = rest / G, per = NH / G, t = c * Q + r;
   if (t >= T) return;
   const uint4* src = reinterpret_cast<const uint4*>(which ? pc : pb) +
                      (((size_t)b * NH + (size_t)g * per) * n + c) * (N / 8 * Q) + c8 * Q + r;
@@ -988,6 +984,23 @@ __global__ void __launch_bounds__(128) m3s_reduce_kernel(const bf16* __restrict_
     for (int y = 0; y < 8; ++y) acc[y] += e[y];
   }
   *reinterpret_cast<uint4*>((which ? dc : db) + (((size_t)b * T + t) * G + g) * N + 8 * c8) = pack8(acc);
+}
+
+// Every `stride`-th of the first blocks does the per-token scalars of a (batch, head), the others the row sums: both read
+// what the chunk kernel left.  One block fills an SM's registers, so the former (chains of dependent steps, DRAM idle: 38 us
+// as a kernel of their own at 8 x 4096 x 32 heads) are spread over the first half of the grid, where the streams of the
+// latter (90 us at the copy rate) keep DRAM busy beside them: 115 us together (124 with all of them first).
+__global__ void __launch_bounds__(kScalThreads) m3s_tail_kernel(SsdP p, bf16* __restrict__ db, bf16* __restrict__ dc, int stride) {
+  const int nf = p.B * p.NH, block = blockIdx.x, q = block / stride, rem = block - q * stride;
+  if (rem == 0 && q < nf) final_scalars(p, q % p.NH, q / p.NH);
+  else reduce_rows(p.pb, p.pc, db, dc, p.T, p.G, p.NH, p.n, block - min(nf, q + 1));
+}
+__global__ void m3s_dalog_kernel(SsdP p) {
+  const int head = blockIdx.x * blockDim.x + threadIdx.x;
+  if (head >= p.NH) return;
+  float s = 0.f;
+  for (int b = 0; b < p.B; ++b) s += p.dal_part[b * p.NH + head];
+  p.da_log[head] = s;
 }
 
 }  // namespace m3s
@@ -1126,11 +1139,11 @@ mxb_status mamba3_ssd_bwd(const mxb_mamba3_desc* d, const void* x, const float* 
     if (MXB_ALLOW_SMEM(m3s::kGradSmem, m3s::m3s_chunk_grad_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("m3s_chunk_grad_kernel", st, (m3s::m3s_chunk_grad_kernel<false><<<gc, 256, m3s::kGradSmem, st>>>(p, maps)));
   }
-  MXB_LAUNCH("m3s_final_kernel", st, (m3s::m3s_final_kernel<<<dim3(p.NH, p.B), m3s::kScalThreads, 0, st>>>(p)));
+  const int nf = p.B * p.NH, tail = nf + 2 * p.n * p.G * p.B;
+  MXB_LAUNCH("m3s_tail_kernel", st,
+             (m3s::m3s_tail_kernel<<<tail, m3s::kScalThreads, 0, st>>>(p, static_cast<m3s::bf16*>(db), static_cast<m3s::bf16*>(dc),
+                                                                       tail >= 2 * nf ? tail / (2 * nf) : 1)));
   MXB_LAUNCH("m3s_dalog_kernel", st, (m3s::m3s_dalog_kernel<<<(p.NH + 127) / 128, 128, 0, st>>>(p)));
-  MXB_LAUNCH("m3s_reduce_kernel", st,
-             (m3s::m3s_reduce_kernel<<<dim3(16 * p.n, p.G, p.B), 128, 0, st>>>(p.pb, p.pc, static_cast<m3s::bf16*>(db),
-                                                                            static_cast<m3s::bf16*>(dc), p.T, p.G, p.NH, p.n)));
   return check_launch("mamba3 ssd backward");
 }
 
