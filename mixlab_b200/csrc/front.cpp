@@ -11,6 +11,8 @@
 #include <torch/extension.h>
 
 #include <map>
+#include <memory>
+#include <mutex>
 #include <optional>
 #include <string>
 #include <vector>
@@ -30,7 +32,8 @@ namespace {
   X(mxb_gdn_block_workspace_bytes) X(mxb_gdn_block_pre_fwd) X(mxb_gdn_block_pre_bwd) X(mxb_gdn_block_post_fwd)        \
   X(mxb_gdn_block_post_bwd) X(mxb_mamba3_fwd_workspace_bytes) X(mxb_mamba3_bwd_workspace_bytes) X(mxb_mamba3_fwd)     \
   X(mxb_mamba3_bwd) X(mxb_mamba3_block_workspace_bytes) X(mxb_mamba3_block_conv_fwd) X(mxb_mamba3_block_conv_bwd)     \
-  X(mxb_mamba3_block_bc_fwd) X(mxb_mamba3_block_bc_bwd) X(mxb_mamba3_block_post_fwd) X(mxb_mamba3_block_post_bwd)
+  X(mxb_mamba3_block_bc_fwd) X(mxb_mamba3_block_bc_bwd) X(mxb_mamba3_block_post_fwd) X(mxb_mamba3_block_post_bwd)     \
+  X(mxb_ir_op_workspace_bytes) X(mxb_ir_op_forward)
 struct Abi {
 #define X(name) decltype(&::name) name = nullptr;
   MXB_FUNCTIONS(X)
@@ -90,27 +93,28 @@ struct On {
   c10::cuda::CUDAGuard guard;
   at::Device dev;
   void* stream;
-  explicit On(const Tensor& t)
-      : guard((t.is_cuda() ? (void)0 : not_cuda(), t.device())), dev(t.device()), stream(c10::cuda::getCurrentCUDAStream(dev.index()).stream()) {}
+  explicit On(at::Device d) : guard(d), dev(d), stream(c10::cuda::getCurrentCUDAStream(d.index()).stream()) {}
+  explicit On(const Tensor& t) : On((t.is_cuda() ? (void)0 : not_cuda(), t.device())) {}
 };
 
 template <typename Fn, typename... A>
-void call(const char* what, Fn fn, A... args) {
-  mxb_status s;
-  {
-    py::gil_scoped_release nogil;  // a launch can block while the stream's queue is full
-    s = fn(args...);
-  }
+mxb_status run(Fn fn, A... args) {
+  py::gil_scoped_release nogil;  // a launch can block while the stream's queue is full
+  return fn(args...);
+}
+void raise_unless_ok(mxb_status s, const char* what) {
   if (s != MXB_OK) py::module_::import("mixlab_b200._lib").attr("check")(s, what);  // raises MxbError
 }
+template <typename Fn, typename... A>
+void call(const char* what, Fn fn, A... args) { raise_unless_ok(run(fn, args...), what); }
 
 // ------------------------------------------------------------------ workspace
-// One cached byte buffer per device, grown to the largest size asked for.  `saved` describes the forward call whose
-// intermediates it holds; any other use of the buffer clears it, so that a backward with use_saved=True cannot consume
-// overwritten tiles.  Guarded by the interpreter lock.
+// One cached byte buffer per device and stream, grown to the largest size asked for: launches of one stream run one after
+// the other and can share scratch, those of two streams cannot.  `saved` describes the forward call whose intermediates
+// the buffer holds; any other use of the buffer clears it, so that a backward with use_saved=True cannot consume
+// overwritten tiles.
 struct Token {
   int kind = 0;  // 0: nothing saved
-  void* stream = nullptr;
   int64_t extra[4] = {};
   struct Operand {
     const void* data;
@@ -120,44 +124,98 @@ struct Token {
   };
   std::vector<Operand> operands;
   bool operator==(const Token& o) const {
-    return kind == o.kind && stream == o.stream && std::equal(extra, extra + 4, o.extra) && operands == o.operands;
+    return kind == o.kind && std::equal(extra, extra + 4, o.extra) && operands == o.operands;
   }
 };
 struct Workspace {
+  std::mutex busy;  // held by a Lease
   Tensor buf;
   Token saved;
+  uint64_t used = 0;  // for the choice of the one to give back
 };
-std::map<int, Workspace>& workspaces() {
-  static auto* m = new std::map<int, Workspace>;  // never destroyed: the allocator may be gone by then
-  return *m;
-}
-Tensor workspace(size_t nbytes, int device) {
-  Workspace& w = workspaces()[device];
-  w.saved.kind = 0;
-  if (!w.buf.defined() || static_cast<size_t>(w.buf.numel()) < nbytes) {
-    w.buf = Tensor();
-    w.buf = make({static_cast<int64_t>(nbytes < 256 ? 256 : nbytes)}, at::kByte, at::Device(at::kCUDA, device));
+// At most this many streams of a device keep a buffer; the one unused for longest goes back to the allocator (it was
+// allocated on the stream that used it, so its memory is handed on in that stream's order).
+constexpr size_t kStreamsPerDevice = 8;
+using Workspaces = std::map<std::pair<int, void*>, std::shared_ptr<Workspace>>;
+// The workspace of a stream.  The table is only touched under the interpreter lock.
+std::shared_ptr<Workspace> workspace_of(int device, void* stream) {
+  static auto* all = new Workspaces;  // never destroyed: the allocator may be gone by then
+  static uint64_t clock = 0;
+  auto& w = (*all)[{device, stream}];
+  if (!w) w = std::make_shared<Workspace>();
+  w->used = ++clock;
+  const std::shared_ptr<Workspace> found = w;
+  size_t count = 0;
+  auto oldest = all->end();
+  for (auto i = all->begin(); i != all->end(); ++i) {
+    if (i->first.first != device) continue;
+    ++count;
+    if (i->second.use_count() == 1 && (oldest == all->end() || i->second->used < oldest->second->used)) oldest = i;
   }
-  return w.buf;
+  if (count > kStreamsPerDevice && oldest != all->end()) all->erase(oldest);
+  return found;
 }
-Token token(int kind, void* stream, std::initializer_list<const Tensor*> ts, std::initializer_list<int64_t> extra) {
+// The workspace of the current stream, for one call: from the look at its buffer and token until the launches are
+// enqueued and the new token is set.  The interpreter lock does not cover that span - run() releases it - so the
+// workspace has a lock of its own, which is waited for without the interpreter lock.  Whatever may run Python code
+// (allocating results, raising) stays outside the span.
+class Lease {
+ public:
+  explicit Lease(const On& on) : w_(workspace_of(on.dev.index(), on.stream)), dev_(on.dev) {
+    py::gil_scoped_release nogil;
+    lock_ = std::unique_lock<std::mutex>(w_->busy);
+  }
+  // a buffer of at least nbytes, whatever it held
+  void take(size_t nbytes) {
+    w_->saved.kind = 0;
+    if (!w_->buf.defined() || bytes() < nbytes) {
+      w_->buf = Tensor();
+      w_->buf = make({static_cast<int64_t>(nbytes < 256 ? 256 : nbytes)}, at::kByte, dev_);
+    }
+  }
+  // the buffer of a use_saved backward, which still has to hold what the forward described by `want` left in it
+  void take_saved(const Token& want, size_t nbytes, const char* what) {
+    if (!(w_->saved == want))
+      throw std::runtime_error(std::string(what) + ": use_saved=True needs the immediately preceding save_for_backward forward on "
+                               "the same tensors, stream and device (the cached workspace has been reused since, or never held them)");
+    if (bytes() < nbytes)
+      throw std::runtime_error(std::string(what) + ": the cached workspace was reallocated after the forward saved into it");
+  }
+  void save(Token t) { w_->saved = std::move(t); }
+  void* data() const { return ptr(w_->buf); }
+  size_t bytes() const { return static_cast<size_t>(w_->buf.numel()); }
+  const Tensor& buffer() const { return w_->buf; }
+
+ private:
+  std::shared_ptr<Workspace> w_;  // (released after the lock: the last owner frees it)
+  std::unique_lock<std::mutex> lock_;
+  at::Device dev_;
+};
+// The current stream's buffer itself (its contents are the caller's from then on).
+Tensor workspace(size_t nbytes, int device) {
+  const On on(at::Device(at::kCUDA, device));
+  Lease ws(on);
+  ws.take(nbytes);
+  return ws.buffer();
+}
+Token token(int kind, std::initializer_list<const Tensor*> ts, std::initializer_list<int64_t> extra) {
   Token t;
   t.kind = kind;
-  t.stream = stream;
   std::copy(extra.begin(), extra.end(), t.extra);
   t.operands.reserve(ts.size());
   for (const Tensor* x : ts) t.operands.push_back({x->data_ptr(), x->sizes().vec(), x->scalar_type()});
   return t;
 }
-// The workspace of a use_saved backward, which still has to hold what the forward described by `want` left in it.
-Tensor saved_workspace(const Token& want, size_t nbytes, int device, const char* what) {
-  Workspace& w = workspaces()[device];
-  if (!(w.saved == want))
-    throw std::runtime_error(std::string(what) + ": use_saved=True needs the immediately preceding save_for_backward forward on "
-                             "the same tensors, stream and device (the cached workspace has been reused since, or never held them)");
-  if (static_cast<size_t>(w.buf.numel()) < nbytes)
-    throw std::runtime_error(std::string(what) + ": the cached workspace was reallocated after the forward saved into it");
-  return w.buf;
+// A call that needs scratch and leaves nothing in it.
+template <typename Fn, typename... A>
+void call_with_scratch(const On& on, size_t nbytes, const char* what, Fn fn, A... args) {
+  mxb_status s;
+  {
+    Lease ws(on);
+    ws.take(nbytes);
+    s = run([&] { return fn(args..., ws.data(), ws.bytes(), on.stream); });
+  }
+  raise_unless_ok(s, what);
 }
 
 // ------------------------------------------------------------------ gated delta rule
@@ -176,10 +234,10 @@ void check_gdn(const mxb_gdn_desc& d, const Tensor& q, const Tensor& k, const Te
   check(beta, Shape(kd, 3), F, dev, "beta");
   check(gate, Shape(kd, 3), F, dev, "gate");
 }
-Token gdn_token(const On& on, const mxb_gdn_desc& d, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta,
+Token gdn_token(const mxb_gdn_desc& d, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta,
                 const Tensor& gate) {
   // the flag bits that choose a kernel family choose the layout of what a forward saves
-  return token(1, on.stream, {&q, &k, &v, &beta, &gate},
+  return token(1, {&q, &k, &v, &beta, &gate},
                {d.chunk, d.gate_is_log, d.flags & ~(MXB_GDN_SAVE_FOR_BWD | MXB_GDN_BWD_USE_SAVED)});
 }
 
@@ -192,10 +250,15 @@ py::object gdn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const 
   check(h0, sd, F, on.dev, "h0");
   Tensor out = like(v), hT;
   if (want_final) hT = make(sd, F, on.dev);
-  Tensor ws = workspace(abi.mxb_gdn_fwd_workspace_bytes(&d), on.dev.index());
-  call("mxb_gdn_fwd", abi.mxb_gdn_fwd, &d, ptr(q), ptr(k), ptr(v), ptr<float>(beta), ptr<float>(gate), ptr<float>(h0), ptr(out),
-       want_final ? ptr<float>(hT) : nullptr, ptr(ws), (size_t)ws.numel(), on.stream);
-  if (save) workspaces()[on.dev.index()].saved = gdn_token(on, d, q, k, v, beta, gate);
+  mxb_status s;
+  {
+    Lease ws(on);
+    ws.take(abi.mxb_gdn_fwd_workspace_bytes(&d));
+    s = run(abi.mxb_gdn_fwd, &d, ptr(q), ptr(k), ptr(v), ptr<float>(beta), ptr<float>(gate), ptr<float>(h0), ptr(out),
+            want_final ? ptr<float>(hT) : nullptr, ws.data(), ws.bytes(), on.stream);
+    if (save && s == MXB_OK) ws.save(gdn_token(d, q, k, v, beta, gate));
+  }
+  raise_unless_ok(s, "mxb_gdn_fwd");
   return want_final ? py::object(py::make_tuple(out, hT)) : py::cast(out);
 }
 
@@ -208,15 +271,20 @@ py::dict gdn_backward(const Tensor& q, const Tensor& k, const Tensor& v, const T
   check(d_out, v.sizes(), q.scalar_type(), on.dev, "d_out");
   check(h0, sd, F, on.dev, "h0");
   check(d_final, sd, F, on.dev, "d_final_state");
-  const size_t nws = abi.mxb_gdn_bwd_workspace_bytes(&d);
-  Tensor ws = use_saved ? saved_workspace(gdn_token(on, d, q, k, v, beta, gate), nws, on.dev.index(), "gated_delta_scan_backward")
-                        : workspace(nws, on.dev.index());
   Tensor dq = like(q), dk = like(k), dv = like(v), db = like(beta), dg = like(gate);
   Opt dh0;
   if (h0) dh0 = like(*h0);
-  call("mxb_gdn_bwd", abi.mxb_gdn_bwd, &d, ptr(q), ptr(k), ptr(v), ptr<float>(beta), ptr<float>(gate), ptr<float>(h0), ptr(d_out),
-       ptr<float>(d_final), ptr(dq), ptr(dk), ptr(dv), ptr<float>(db), ptr<float>(dg), ptr<float>(dh0), ptr(ws), (size_t)ws.numel(),
-       on.stream);
+  const size_t nws = abi.mxb_gdn_bwd_workspace_bytes(&d);
+  mxb_status s;
+  {
+    Lease ws(on);
+    if (use_saved) ws.take_saved(gdn_token(d, q, k, v, beta, gate), nws, "gated_delta_scan_backward");
+    else ws.take(nws);
+    s = run(abi.mxb_gdn_bwd, &d, ptr(q), ptr(k), ptr(v), ptr<float>(beta), ptr<float>(gate), ptr<float>(h0), ptr(d_out),
+            ptr<float>(d_final), ptr(dq), ptr(dk), ptr(dv), ptr<float>(db), ptr<float>(dg), ptr<float>(dh0), ws.data(), ws.bytes(),
+            on.stream);
+  }
+  raise_unless_ok(s, "mxb_gdn_bwd");
   py::dict r;
   r["dq"] = dq; r["dk"] = dk; r["dv"] = dv; r["dbeta"] = db; r["dgate"] = dg; r["dh0"] = dh0;
   return r;
@@ -297,11 +365,11 @@ py::dict gdn_block_pre_backward(const Tensor& qp, const Tensor& kp, const Tensor
   check(dgate, x.hd, F, on.dev, "dgate");
   Tensor dqp = like(qp), dkp = like(kp), dvp = like(vp), dcq = like(cq), dck = like(ck), dcv = like(cv), da = like(a), db = like(b),
          dal = like(al), dbias = like(bias);
-  Tensor ws = workspace(abi.mxb_gdn_block_workspace_bytes(&x.d), on.dev.index());
-  call("mxb_gdn_block_pre_bwd", abi.mxb_gdn_block_pre_bwd, &x.d, ptr(qp), ptr(kp), ptr(vp), ptr<float>(cq), ptr<float>(ck), ptr<float>(cv),
-       ptr<float>(a), ptr<float>(b), ptr<float>(al), ptr<float>(bias), ptr(dq), ptr(dk), ptr(dv), ptr<float>(dbeta), ptr<float>(dgate),
-       ptr(dqp), ptr(dkp), ptr(dvp), ptr<float>(dcq), ptr<float>(dck), ptr<float>(dcv), ptr<float>(da), ptr<float>(db), ptr<float>(dal),
-       ptr<float>(dbias), ptr(ws), (size_t)ws.numel(), on.stream);
+  call_with_scratch(on, abi.mxb_gdn_block_workspace_bytes(&x.d), "mxb_gdn_block_pre_bwd", abi.mxb_gdn_block_pre_bwd,
+                    &x.d, ptr(qp), ptr(kp), ptr(vp), ptr<float>(cq), ptr<float>(ck), ptr<float>(cv), ptr<float>(a),
+                    ptr<float>(b), ptr<float>(al), ptr<float>(bias), ptr(dq), ptr(dk), ptr(dv), ptr<float>(dbeta),
+                    ptr<float>(dgate), ptr(dqp), ptr(dkp), ptr(dvp), ptr<float>(dcq), ptr<float>(dck),
+                    ptr<float>(dcv), ptr<float>(da), ptr<float>(db), ptr<float>(dal), ptr<float>(dbias));
   py::dict r;
   r["dq_proj"] = dqp; r["dk_proj"] = dkp; r["dv_proj"] = dvp; r["dconv_q"] = dcq; r["dconv_k"] = dck; r["dconv_v"] = dcv;
   r["da_raw"] = da; r["db_raw"] = db; r["da_log"] = dal; r["ddt_bias"] = dbias;
@@ -328,9 +396,8 @@ py::dict gdn_block_post_backward(const Tensor& o, const Tensor& z, const Tensor&
   const mxb_gdn_desc d = check_block_post(on, o, z, w);
   check(dy, z.sizes(), o.scalar_type(), on.dev, "dy");
   Tensor d_o = like(o), dz = like(z), dw = like(w);
-  Tensor ws = workspace(abi.mxb_gdn_block_workspace_bytes(&d), on.dev.index());
-  call("mxb_gdn_block_post_bwd", abi.mxb_gdn_block_post_bwd, &d, ptr(o), ptr(z), ptr<float>(w), ptr(dy), ptr(d_o), ptr(dz), ptr<float>(dw),
-       ptr(ws), (size_t)ws.numel(), on.stream);
+  call_with_scratch(on, abi.mxb_gdn_block_workspace_bytes(&d), "mxb_gdn_block_post_bwd", abi.mxb_gdn_block_post_bwd,
+                    &d, ptr(o), ptr(z), ptr<float>(w), ptr(dy), ptr(d_o), ptr(dz), ptr<float>(dw));
   py::dict r;
   r["do"] = d_o; r["dz"] = dz; r["do_norm"] = dw;
   return r;
@@ -353,19 +420,24 @@ mxb_mamba3_desc check_mamba3(const On& on, const Tensor& x, const Tensor& dt, co
   check(c, gn, io, on.dev, "c");
   return d;
 }
-Token mamba3_token(const On& on, const mxb_mamba3_desc& d, const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta,
+Token mamba3_token(const mxb_mamba3_desc& d, const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta,
                    const Tensor& a_log, const Tensor& b, const Tensor& c) {
-  return token(2, on.stream, {&x, &dt, &lam, &theta, &a_log, &b, &c}, {d.nheads, d.flags & ~(MXB_MAMBA3_SAVE_FOR_BWD | MXB_MAMBA3_BWD_USE_SAVED)});
+  return token(2, {&x, &dt, &lam, &theta, &a_log, &b, &c}, {d.nheads, d.flags & ~(MXB_MAMBA3_SAVE_FOR_BWD | MXB_MAMBA3_BWD_USE_SAVED)});
 }
 Tensor mamba3_forward(const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta, const Tensor& a_log, const Tensor& b,
                       const Tensor& c, int64_t nheads, int64_t flags, bool save) {
   On on(x);
   const mxb_mamba3_desc d = check_mamba3(on, x, dt, lam, theta, a_log, b, c, nheads, save ? flags | MXB_MAMBA3_SAVE_FOR_BWD : flags);
   Tensor y = like(x);
-  Tensor ws = workspace(abi.mxb_mamba3_fwd_workspace_bytes(&d), on.dev.index());
-  call("mxb_mamba3_fwd", abi.mxb_mamba3_fwd, &d, ptr(x), ptr<float>(dt), ptr<float>(lam), ptr<float>(theta), ptr<float>(a_log), ptr(b), ptr(c),
-       ptr(y), ptr(ws), (size_t)ws.numel(), on.stream);
-  if (save) workspaces()[on.dev.index()].saved = mamba3_token(on, d, x, dt, lam, theta, a_log, b, c);
+  mxb_status s;
+  {
+    Lease ws(on);
+    ws.take(abi.mxb_mamba3_fwd_workspace_bytes(&d));
+    s = run(abi.mxb_mamba3_fwd, &d, ptr(x), ptr<float>(dt), ptr<float>(lam), ptr<float>(theta), ptr<float>(a_log), ptr(b), ptr(c),
+            ptr(y), ws.data(), ws.bytes(), on.stream);
+    if (save && s == MXB_OK) ws.save(mamba3_token(d, x, dt, lam, theta, a_log, b, c));
+  }
+  raise_unless_ok(s, "mxb_mamba3_fwd");
   return y;
 }
 py::dict mamba3_backward(const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta, const Tensor& a_log, const Tensor& b,
@@ -373,13 +445,18 @@ py::dict mamba3_backward(const Tensor& x, const Tensor& dt, const Tensor& lam, c
   On on(x);
   const mxb_mamba3_desc d = check_mamba3(on, x, dt, lam, theta, a_log, b, c, nheads, use_saved ? flags | MXB_MAMBA3_BWD_USE_SAVED : flags);
   check(dy, x.sizes(), x.scalar_type(), on.dev, "dy");
-  const size_t nws = abi.mxb_mamba3_bwd_workspace_bytes(&d);
-  Tensor ws = use_saved ? saved_workspace(mamba3_token(on, d, x, dt, lam, theta, a_log, b, c), nws, on.dev.index(), "mamba3_selective_scan_backward")
-                        : workspace(nws, on.dev.index());
   Tensor dx = like(x), ddt = like(dt), dlam = like(lam), dth = like(theta), dal = like(a_log), db = like(b), dc = like(c);
-  call("mxb_mamba3_bwd", abi.mxb_mamba3_bwd, &d, ptr(x), ptr<float>(dt), ptr<float>(lam), ptr<float>(theta), ptr<float>(a_log), ptr(b), ptr(c),
-       ptr(dy), ptr(dx), ptr<float>(ddt), ptr<float>(dlam), ptr<float>(dth), ptr<float>(dal), ptr(db), ptr(dc), ptr(ws), (size_t)ws.numel(),
-       on.stream);
+  const size_t nws = abi.mxb_mamba3_bwd_workspace_bytes(&d);
+  mxb_status s;
+  {
+    Lease ws(on);
+    if (use_saved) ws.take_saved(mamba3_token(d, x, dt, lam, theta, a_log, b, c), nws, "mamba3_selective_scan_backward");
+    else ws.take(nws);
+    s = run(abi.mxb_mamba3_bwd, &d, ptr(x), ptr<float>(dt), ptr<float>(lam), ptr<float>(theta), ptr<float>(a_log), ptr(b), ptr(c),
+            ptr(dy), ptr(dx), ptr<float>(ddt), ptr<float>(dlam), ptr<float>(dth), ptr<float>(dal), ptr(db), ptr(dc), ws.data(),
+            ws.bytes(), on.stream);
+  }
+  raise_unless_ok(s, "mxb_mamba3_bwd");
   py::dict r;
   r["dx"] = dx; r["ddt"] = ddt; r["dlambda"] = dlam; r["dtheta"] = dth; r["da_log"] = dal; r["db"] = db; r["dc"] = dc;
   return r;
@@ -409,9 +486,9 @@ py::dict mamba3_block_conv_backward(const Tensor& x, const Tensor& w, const Tens
   const mxb_mamba3_desc d = check_conv(on, x, w);
   check(dy, x.sizes(), x.scalar_type(), on.dev, "dy");
   Tensor dx = like(x), dw = like(w);
-  Tensor ws = workspace(abi.mxb_mamba3_block_workspace_bytes(&d), on.dev.index());
-  call("mxb_mamba3_block_conv_bwd", abi.mxb_mamba3_block_conv_bwd, &d, (int32_t)w.size(1), ptr(x), ptr<float>(w), ptr(dy), ptr(dx),
-       ptr<float>(dw), ptr(ws), (size_t)ws.numel(), on.stream);
+  call_with_scratch(on, abi.mxb_mamba3_block_workspace_bytes(&d), "mxb_mamba3_block_conv_bwd",
+                    abi.mxb_mamba3_block_conv_bwd, &d, (int32_t)w.size(1), ptr(x), ptr<float>(w), ptr(dy), ptr(dx),
+                    ptr<float>(dw));
   py::dict r;
   r["dx"] = dx; r["dw"] = dw;
   return r;
@@ -446,10 +523,10 @@ py::dict mamba3_block_bc_backward(const Tensor& bp, const Tensor& cp, const Tens
   check(db, o4, bp.scalar_type(), on.dev, "db");
   check(dc, o4, bp.scalar_type(), on.dev, "dc");
   Tensor dbp = like(bp), dcp = like(cp), dbs = like(bs), dcs = like(cs), dbb = make(Shape(&gn, 1), F, on.dev), dcb = make(Shape(&gn, 1), F, on.dev);
-  Tensor ws = workspace(abi.mxb_mamba3_block_workspace_bytes(&d), on.dev.index());
-  call("mxb_mamba3_block_bc_bwd", abi.mxb_mamba3_block_bc_bwd, &d, (float)eps, ptr(bp), ptr(cp), ptr<float>(bs), ptr<float>(cs), ptr(db),
-       ptr(dc), ptr(dbp), ptr(dcp), ptr<float>(dbs), ptr<float>(dcs), ptr<float>(dbb), ptr<float>(dcb), ptr(ws), (size_t)ws.numel(),
-       on.stream);
+  call_with_scratch(on, abi.mxb_mamba3_block_workspace_bytes(&d), "mxb_mamba3_block_bc_bwd",
+                    abi.mxb_mamba3_block_bc_bwd, &d, (float)eps, ptr(bp), ptr(cp), ptr<float>(bs), ptr<float>(cs),
+                    ptr(db), ptr(dc), ptr(dbp), ptr(dcp), ptr<float>(dbs), ptr<float>(dcs), ptr<float>(dbb),
+                    ptr<float>(dcb));
   py::dict r;
   r["db_proj"] = dbp; r["dc_proj"] = dcp; r["db_scale"] = dbs; r["dc_scale"] = dcs; r["db_bias"] = dbb; r["dc_bias"] = dcb;
   return r;
@@ -474,12 +551,35 @@ py::dict mamba3_block_post_backward(const Tensor& y, const Tensor& z, const Tens
   const mxb_mamba3_desc d = check_post(on, y, z, w);
   check(dout, y.sizes(), y.scalar_type(), on.dev, "dout");
   Tensor dy = like(y), dz = like(z), dw = like(w);
-  Tensor ws = workspace(abi.mxb_mamba3_block_workspace_bytes(&d), on.dev.index());
-  call("mxb_mamba3_block_post_bwd", abi.mxb_mamba3_block_post_bwd, &d, (float)eps, ptr(y), ptr(z), ptr<float>(w), ptr(dout), ptr(dy), ptr(dz),
-       ptr<float>(dw), ptr(ws), (size_t)ws.numel(), on.stream);
+  call_with_scratch(on, abi.mxb_mamba3_block_workspace_bytes(&d), "mxb_mamba3_block_post_bwd",
+                    abi.mxb_mamba3_block_post_bwd, &d, (float)eps, ptr(y), ptr(z), ptr<float>(w), ptr(dout), ptr(dy),
+                    ptr(dz), ptr<float>(dw));
   py::dict r;
   r["dy"] = dy; r["dz"] = dz; r["dpost_norm"] = dw;
   return r;
+}
+
+// ------------------------------------------------------------------ IR op records
+Tensor ir_op_forward(int64_t op_type, const std::vector<Tensor>& inputs, const std::vector<int64_t>& int_params,
+                     const std::vector<int64_t>& out_shape, const std::vector<double>& float_params) {
+  for (const Tensor& t : inputs)
+    if (!t.is_cuda()) not_cuda();
+  for (size_t i = 0; i < inputs.size(); ++i)
+    if (!inputs[i].is_contiguous() || inputs[i].device() != inputs[0].device())
+      throw py::value_error("input " + std::to_string(i) + ": contiguous tensors on one device expected");
+  if (inputs.empty()) throw py::value_error("an op record has inputs");
+  On on(inputs[0]);
+  const int32_t io = io_code(inputs[0]);
+  Tensor out = make(out_shape, inputs[0].scalar_type(), on.dev);
+  std::vector<const void*> in;
+  for (const Tensor& t : inputs) in.push_back(t.data_ptr());
+  void* outs[] = {out.data_ptr()};
+  const std::vector<int32_t> ints(int_params.begin(), int_params.end());
+  const std::vector<float> floats(float_params.begin(), float_params.end());
+  const mxb_ir_op op{(int32_t)op_type, in.data(), (int32_t)in.size(), outs, 1, floats.data(), (int32_t)floats.size(),
+                     ints.data(), (int32_t)ints.size(), io};
+  call_with_scratch(on, abi.mxb_ir_op_workspace_bytes(&op), "mxb_ir_op_forward", abi.mxb_ir_op_forward, &op);
+  return out;
 }
 
 }  // namespace
@@ -487,6 +587,7 @@ py::dict mamba3_block_post_backward(const Tensor& y, const Tensor& z, const Tens
 PYBIND11_MODULE(_front, m) {
   m.def("open", &open_library);
   m.def("workspace", &workspace);
+  m.def("ir_op_forward", &ir_op_forward);
   m.def("gdn_forward", &gdn_forward);
   m.def("gdn_backward", &gdn_backward);
   m.def("gdn_decode", &gdn_decode);

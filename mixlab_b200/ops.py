@@ -41,22 +41,6 @@ def _io(t: torch.Tensor) -> int:
     raise TypeError(f"unsupported dtype {t.dtype} (float32 or bfloat16)")
 
 
-def _ptr(t):
-    if t is None:
-        return None
-    if not t.is_cuda:
-        raise ValueError("mixlab_b200 operators take CUDA tensors only (no CPU fallback)")
-    if not t.is_contiguous():
-        raise ValueError("tensor must be contiguous")
-    return C.c_void_p(t.data_ptr())
-
-
-def _require_cuda(*tensors):
-    for t in tensors:
-        if t is not None and not t.is_cuda:
-            raise ValueError("mixlab_b200 operators take CUDA tensors only (no CPU fallback)")
-
-
 def _check_like(t, shape, dtype, device, name):
     """Raises unless ``t`` (None allowed) is a contiguous CUDA tensor of exactly this shape, dtype and device:
     the C ABI sees only pointers, so a wrong operand would otherwise be read out of bounds or as the wrong type."""
@@ -75,12 +59,9 @@ def _check_like(t, shape, dtype, device, name):
 
 
 def workspace(nbytes: int, device) -> torch.Tensor:
-    """A cached byte buffer of at least ``nbytes`` on ``device`` (torch allocator)."""
+    """The cached byte buffer of the current stream of ``device``, of at least ``nbytes`` (torch allocator).  The operators
+    called on that stream use it too."""
     return _native().workspace(int(nbytes), device.index if device.index is not None else torch.cuda.current_device())
-
-
-def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def gdn_desc(q, v, chunk, gate_is_log, flags=0) -> GdnDesc:
@@ -106,30 +87,17 @@ def ir_op_forward(op_type: int, inputs, int_params, *, out_shape, float_params=(
     """Runs one IR op record the way the reference's interpreter does after resolving its names
     (gpu/ir.cpp:4633-4654, :4837-4853): ``inputs`` in the record's order, IntParams as the Go side emits them
     (arch/ir.go:550-555, :600-602).  Returns the output tensor of ``out_shape`` in the dtype of the first input."""
-    _require_cuda(*inputs)
-    for i, t in enumerate(inputs):
-        if not t.is_contiguous() or t.device != inputs[0].device:
-            raise ValueError(f"input {i}: contiguous tensors on one device expected")
-    l = _lib.lib()
-    with torch.cuda.device(inputs[0].device):
-        out = torch.empty(out_shape, dtype=inputs[0].dtype, device=inputs[0].device)
-        ins = (C.c_void_p * len(inputs))(*[t.data_ptr() for t in inputs])
-        outs = (C.c_void_p * 1)(out.data_ptr())
-        ip = (C.c_int32 * len(int_params))(*[int(v) for v in int_params])
-        fp = (C.c_float * max(len(float_params), 1))(*[float(v) for v in float_params])
-        rec = _lib.IrOp(int(op_type), ins, len(inputs), outs, 1, fp, len(float_params), ip, len(int_params), _io(inputs[0]))
-        nws = l.mxb_ir_op_workspace_bytes(C.byref(rec))
-        ws = workspace(nws, inputs[0].device)
-        _lib.check(l.mxb_ir_op_forward(C.byref(rec), _ptr(ws), ws.numel(), _stream()), "mxb_ir_op_forward")
-    return out
+    return _native().ir_op_forward(int(op_type), list(inputs), [int(v) for v in int_params], list(out_shape),
+                                   [float(v) for v in float_params])
 
 
 def device_status(device=None) -> int:
-    """Blocking read of the device-side error word of the cached workspace (0 = ok)."""
+    """Blocking read of the device-side error word of the current stream's cached workspace (0 = ok)."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else device
     ws = workspace(256, dev)
+    torch.cuda.current_stream(dev).synchronize()
     out = C.c_int32(0)
-    _lib.check(_lib.lib().mxb_gdn_device_status(_ptr(ws), C.byref(out)), "mxb_gdn_device_status")
+    _lib.check(_lib.lib().mxb_gdn_device_status(C.c_void_p(ws.data_ptr()), C.byref(out)), "mxb_gdn_device_status")
     return out.value
 
 
