@@ -7,6 +7,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
 #include <dlfcn.h>
 #include <torch/extension.h>
 
@@ -113,6 +114,10 @@ void call(const char* what, Fn fn, A... args) { raise_unless_ok(run(fn, args...)
 // the other and can share scratch, those of two streams cannot.  `saved` describes the forward call whose intermediates
 // the buffer holds; any other use of the buffer clears it, so that a backward with use_saved=True cannot consume
 // overwritten tiles.
+//
+// A graph keeps the addresses it was captured with.  So a buffer belongs to the capture it was allocated in (its memory
+// then comes from that graph's own pool, which nobody else is given): calls outside that capture take another one, and
+// a captured call never takes one that a later call may outgrow and give back.
 struct Token {
   int kind = 0;  // 0: nothing saved
   int64_t extra[4] = {};
@@ -131,6 +136,7 @@ struct Workspace {
   std::mutex busy;  // held by a Lease
   Tensor buf;
   Token saved;
+  unsigned long long capture = 0;  // the capture `buf` was allocated in, 0: none
   uint64_t used = 0;  // for the choice of the one to give back
 };
 // At most this many streams of a device keep a buffer; the one unused for longest goes back to the allocator (it was
@@ -155,22 +161,32 @@ std::shared_ptr<Workspace> workspace_of(int device, void* stream) {
   if (count > kStreamsPerDevice && oldest != all->end()) all->erase(oldest);
   return found;
 }
+unsigned long long capture_of(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &status, &id) != cudaSuccess) {
+    cudaGetLastError();  // (the legacy stream may not be asked while another one captures; it does not capture itself)
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusActive ? id : 0;
+}
 // The workspace of the current stream, for one call: from the look at its buffer and token until the launches are
 // enqueued and the new token is set.  The interpreter lock does not cover that span - run() releases it - so the
 // workspace has a lock of its own, which is waited for without the interpreter lock.  Whatever may run Python code
 // (allocating results, raising) stays outside the span.
 class Lease {
  public:
-  explicit Lease(const On& on) : w_(workspace_of(on.dev.index(), on.stream)), dev_(on.dev) {
+  explicit Lease(const On& on) : w_(workspace_of(on.dev.index(), on.stream)), dev_(on.dev), capture_(capture_of(on.stream)) {
     py::gil_scoped_release nogil;
     lock_ = std::unique_lock<std::mutex>(w_->busy);
   }
   // a buffer of at least nbytes, whatever it held
   void take(size_t nbytes) {
     w_->saved.kind = 0;
-    if (!w_->buf.defined() || bytes() < nbytes) {
+    if (!w_->buf.defined() || bytes() < nbytes || w_->capture != capture_) {
       w_->buf = Tensor();
       w_->buf = make({static_cast<int64_t>(nbytes < 256 ? 256 : nbytes)}, at::kByte, dev_);
+      w_->capture = capture_;
     }
   }
   // the buffer of a use_saved backward, which still has to hold what the forward described by `want` left in it
@@ -190,6 +206,7 @@ class Lease {
   std::shared_ptr<Workspace> w_;  // (released after the lock: the last owner frees it)
   std::unique_lock<std::mutex> lock_;
   at::Device dev_;
+  unsigned long long capture_;
 };
 // The current stream's buffer itself (its contents are the caller's from then on).
 Tensor workspace(size_t nbytes, int device) {

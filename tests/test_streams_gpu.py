@@ -1,4 +1,4 @@
-"""Calls on several streams and from several threads: the cached scratch of one is not touched by another."""
+"""Calls on several streams, from several threads and in graphs: the cached scratch of one is not touched by another."""
 import threading
 
 import pytest
@@ -94,3 +94,55 @@ def test_streams_beyond_the_kept_ones():
     torch.cuda.synchronize()
     for n, w in zip(("dq", "dk", "dv", "dbeta", "dgate"), want[1:]):
         assert torch.equal(g[n], w), n
+
+
+def _capture(stream, args, d_out):
+    with torch.cuda.stream(stream):
+        _train(args, d_out)  # (code and attributes loaded before the capture)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        res = _train(args, d_out)
+    return graph, res
+
+
+def test_graph_keeps_its_scratch():
+    """A graph captured on a stream that has a buffer already; then a call there that outgrows that buffer, and tensors
+    over the memory it gave back: replays give the same results and leave those tensors alone."""
+    args, d_out = _scan_case(6, 700)
+    want = [t.clone() for t in _train(args, d_out)]
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    graph, res = _capture(stream, args, d_out)
+    big, big_do = _scan_case(7, 2100)
+    with torch.cuda.stream(stream):
+        _train(big, big_do)
+        over = [torch.full((1 << 20,), 7, dtype=torch.uint8, device="cuda") for _ in range(64)]
+        over += [torch.full((8 << 20,), 7, dtype=torch.uint8, device="cuda") for _ in range(32)]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for t in res:
+            t.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        for x, y in zip(res, want):
+            assert torch.equal(x, y)
+    assert all(bool((t == 7).all()) for t in over)
+
+
+def test_graphs_of_one_stream_side_by_side():
+    """Two graphs captured one after the other on the same stream, replayed on two: each has scratch of its own."""
+    cases = [_scan_case(s, 900) for s in (8, 9)]
+    want = [[t.clone() for t in _train(*c)] for c in cases]
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    graphs = [_capture(stream, *c) for c in cases]
+    others = [torch.cuda.Stream() for _ in cases]
+    for _ in range(20):
+        for (graph, _), st in zip(graphs, others):
+            with torch.cuda.stream(st):
+                graph.replay()
+        torch.cuda.synchronize()
+        for (_, res), w in zip(graphs, want):
+            for x, y in zip(res, w):
+                assert torch.equal(x, y)
