@@ -66,6 +66,10 @@ std::string text(Shape s) {
   return r + ")";
 }
 
+at::Device cuda_device(const Tensor& t) {
+  if (!t.is_cuda()) not_cuda();
+  return t.device();
+}
 void check(const Tensor& t, Shape shape, at::ScalarType dtype, at::Device dev, const char* name) {
   if (!t.is_cuda()) not_cuda();
   if (t.sizes() != shape) throw py::value_error(std::string(name) + ": shape " + text(t.sizes()) + ", expected " + text(shape));
@@ -89,13 +93,13 @@ Tensor make(Shape shape, at::ScalarType dtype, at::Device dev) {
 Tensor like(const Tensor& t) { return make(t.sizes(), t.scalar_type(), t.device()); }
 constexpr at::ScalarType F = at::kFloat;
 
-// A call on the device of `t`: that device is current, its current stream is the one to launch on.
+// A call on a device: that device is current, its current stream is the one to launch on.  Made when every operand has
+// been checked: a refused call does not touch the device.
 struct On {
   c10::cuda::CUDAGuard guard;
   at::Device dev;
   void* stream;
   explicit On(at::Device d) : guard(d), dev(d), stream(c10::cuda::getCurrentCUDAStream(d.index()).stream()) {}
-  explicit On(const Tensor& t) : On((t.is_cuda() ? (void)0 : not_cuda(), t.device())) {}
 };
 
 template <typename Fn, typename... A>
@@ -260,11 +264,12 @@ Token gdn_token(const mxb_gdn_desc& d, const Tensor& q, const Tensor& k, const T
 
 py::object gdn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta, const Tensor& gate, int64_t chunk,
                        bool gate_is_log, const Opt& h0, bool want_final, int64_t flags, bool save) {
-  On on(q);
+  const at::Device dev = cuda_device(q);
   const mxb_gdn_desc d = gdn_desc(q, v, chunk, gate_is_log, save ? flags | MXB_GDN_SAVE_FOR_BWD : flags);
   check_gdn(d, q, k, v, beta, gate);
   const int64_t sd[] = {d.B, d.H, d.Dk, d.Dv};
-  check(h0, sd, F, on.dev, "h0");
+  check(h0, sd, F, dev, "h0");
+  const On on(dev);
   Tensor out = like(v), hT;
   if (want_final) hT = make(sd, F, on.dev);
   mxb_status s;
@@ -281,13 +286,14 @@ py::object gdn_forward(const Tensor& q, const Tensor& k, const Tensor& v, const 
 
 py::dict gdn_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta, const Tensor& gate, const Tensor& d_out,
                       int64_t chunk, bool gate_is_log, const Opt& h0, const Opt& d_final, int64_t flags, bool use_saved) {
-  On on(q);
+  const at::Device dev = cuda_device(q);
   const mxb_gdn_desc d = gdn_desc(q, v, chunk, gate_is_log, use_saved ? flags | MXB_GDN_BWD_USE_SAVED : flags);
   check_gdn(d, q, k, v, beta, gate);
   const int64_t sd[] = {d.B, d.H, d.Dk, d.Dv};
-  check(d_out, v.sizes(), q.scalar_type(), on.dev, "d_out");
-  check(h0, sd, F, on.dev, "h0");
-  check(d_final, sd, F, on.dev, "d_final_state");
+  check(d_out, v.sizes(), q.scalar_type(), dev, "d_out");
+  check(h0, sd, F, dev, "h0");
+  check(d_final, sd, F, dev, "d_final_state");
+  const On on(dev);
   Tensor dq = like(q), dk = like(k), dv = like(v), db = like(beta), dg = like(gate);
   Opt dh0;
   if (h0) dh0 = like(*h0);
@@ -309,20 +315,21 @@ py::dict gdn_backward(const Tensor& q, const Tensor& k, const Tensor& v, const T
 
 Tensor gdn_decode(const Tensor& state, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& beta, const Tensor& gate,
                   bool gate_is_log, const Opt& out_, int64_t flags) {
-  On on(state);
+  const at::Device dev = cuda_device(state);
   if (!q.is_cuda()) not_cuda();
   if (state.dim() != 4) throw py::value_error("state must be [N,H,Dk,Dv]");
   const int64_t N = state.size(0), H = state.size(1), K = state.size(2), V = state.size(3);
   const mxb_gdn_desc d{(int32_t)N, 1, (int32_t)H, (int32_t)K, (int32_t)V, 0, io_code(q), gate_is_log ? 1 : 0, (int32_t)flags};
   const auto io = q.scalar_type();
   const int64_t kd[] = {N, H, K}, vd[] = {N, H, V};
-  check(state, state.sizes(), F, on.dev, "state");
-  check(q, kd, io, on.dev, "q");
-  check(k, kd, io, on.dev, "k");
-  check(v, vd, io, on.dev, "v");
-  check(beta, Shape(kd, 2), F, on.dev, "beta");
-  check(gate, Shape(kd, 2), F, on.dev, "gate");
-  check(out_, vd, io, on.dev, "out");
+  check(state, state.sizes(), F, dev, "state");
+  check(q, kd, io, dev, "q");
+  check(k, kd, io, dev, "k");
+  check(v, vd, io, dev, "v");
+  check(beta, Shape(kd, 2), F, dev, "beta");
+  check(gate, Shape(kd, 2), F, dev, "gate");
+  check(out_, vd, io, dev, "out");
+  const On on(dev);
   Tensor out = out_ ? *out_ : like(v);
   call("mxb_gdn_decode_step", abi.mxb_gdn_decode_step, &d, ptr<float>(state), ptr(q), ptr(k), ptr(v), ptr<float>(beta),
        ptr<float>(gate), ptr(out), on.stream);
@@ -334,7 +341,7 @@ struct BlockArgs {
   mxb_gdn_desc d;
   int64_t kd[3], vd[3], hd[3];
 };
-BlockArgs check_block_pre(const On& on, const Tensor& qp, const Tensor& kp, const Tensor& vp, const Tensor& cq, const Tensor& ck,
+BlockArgs check_block_pre(at::Device dev, const Tensor& qp, const Tensor& kp, const Tensor& vp, const Tensor& cq, const Tensor& ck,
                           const Tensor& cv, const Tensor& a, const Tensor& b, const Tensor& al, const Tensor& bias, int64_t H,
                           int64_t Dk, int64_t Dv, bool gate_is_log) {
   if (qp.dim() != 3) throw py::value_error("q_proj must be [B,T,H*Dk]");
@@ -343,23 +350,24 @@ BlockArgs check_block_pre(const On& on, const Tensor& qp, const Tensor& kp, cons
               {B, T, H * Dk}, {B, T, H * Dv}, {B, T, H}};
   const auto io = qp.scalar_type();
   const int64_t wk[] = {4, H * Dk}, wv[] = {4, H * Dv};
-  check(qp, r.kd, io, on.dev, "q_proj");
-  check(kp, r.kd, io, on.dev, "k_proj");
-  check(vp, r.vd, io, on.dev, "v_proj");
-  check(cq, wk, F, on.dev, "conv_q");
-  check(ck, wk, F, on.dev, "conv_k");
-  check(cv, wv, F, on.dev, "conv_v");
-  check(a, r.hd, F, on.dev, "a_raw");
-  check(b, r.hd, F, on.dev, "b_raw");
-  check(al, Shape(&H, 1), F, on.dev, "a_log");
-  check(bias, Shape(&H, 1), F, on.dev, "dt_bias");
+  check(qp, r.kd, io, dev, "q_proj");
+  check(kp, r.kd, io, dev, "k_proj");
+  check(vp, r.vd, io, dev, "v_proj");
+  check(cq, wk, F, dev, "conv_q");
+  check(ck, wk, F, dev, "conv_k");
+  check(cv, wv, F, dev, "conv_v");
+  check(a, r.hd, F, dev, "a_raw");
+  check(b, r.hd, F, dev, "b_raw");
+  check(al, Shape(&H, 1), F, dev, "a_log");
+  check(bias, Shape(&H, 1), F, dev, "dt_bias");
   return r;
 }
 py::tuple gdn_block_pre(const Tensor& qp, const Tensor& kp, const Tensor& vp, const Tensor& cq, const Tensor& ck, const Tensor& cv,
                         const Tensor& a, const Tensor& b, const Tensor& al, const Tensor& bias, int64_t H, int64_t Dk, int64_t Dv,
                         bool gate_is_log) {
-  On on(qp);
-  BlockArgs x = check_block_pre(on, qp, kp, vp, cq, ck, cv, a, b, al, bias, H, Dk, Dv, gate_is_log);
+  const at::Device dev = cuda_device(qp);
+  BlockArgs x = check_block_pre(dev, qp, kp, vp, cq, ck, cv, a, b, al, bias, H, Dk, Dv, gate_is_log);
+  const On on(dev);
   const int64_t k4[] = {x.d.B, x.d.T, H, Dk}, v4[] = {x.d.B, x.d.T, H, Dv};
   const auto io = qp.scalar_type();
   Tensor q = make(k4, io, on.dev), k = make(k4, io, on.dev), v = make(v4, io, on.dev), beta = make(x.hd, F, on.dev), gate = make(x.hd, F, on.dev);
@@ -371,15 +379,16 @@ py::dict gdn_block_pre_backward(const Tensor& qp, const Tensor& kp, const Tensor
                                 const Tensor& cv, const Tensor& a, const Tensor& b, const Tensor& al, const Tensor& bias, int64_t H,
                                 int64_t Dk, int64_t Dv, const Tensor& dq, const Tensor& dk, const Tensor& dv, const Tensor& dbeta,
                                 const Tensor& dgate, bool gate_is_log) {
-  On on(qp);
-  BlockArgs x = check_block_pre(on, qp, kp, vp, cq, ck, cv, a, b, al, bias, H, Dk, Dv, gate_is_log);
+  const at::Device dev = cuda_device(qp);
+  BlockArgs x = check_block_pre(dev, qp, kp, vp, cq, ck, cv, a, b, al, bias, H, Dk, Dv, gate_is_log);
   const int64_t k4[] = {x.d.B, x.d.T, H, Dk}, v4[] = {x.d.B, x.d.T, H, Dv};
   const auto io = qp.scalar_type();
-  check(dq, k4, io, on.dev, "dq");
-  check(dk, k4, io, on.dev, "dk");
-  check(dv, v4, io, on.dev, "dv");
-  check(dbeta, x.hd, F, on.dev, "dbeta");
-  check(dgate, x.hd, F, on.dev, "dgate");
+  check(dq, k4, io, dev, "dq");
+  check(dk, k4, io, dev, "dk");
+  check(dv, v4, io, dev, "dv");
+  check(dbeta, x.hd, F, dev, "dbeta");
+  check(dgate, x.hd, F, dev, "dgate");
+  const On on(dev);
   Tensor dqp = like(qp), dkp = like(kp), dvp = like(vp), dcq = like(cq), dck = like(ck), dcv = like(cv), da = like(a), db = like(b),
          dal = like(al), dbias = like(bias);
   call_with_scratch(on, abi.mxb_gdn_block_workspace_bytes(&x.d), "mxb_gdn_block_pre_bwd", abi.mxb_gdn_block_pre_bwd,
@@ -392,26 +401,28 @@ py::dict gdn_block_pre_backward(const Tensor& qp, const Tensor& kp, const Tensor
   r["da_raw"] = da; r["db_raw"] = db; r["da_log"] = dal; r["ddt_bias"] = dbias;
   return r;
 }
-mxb_gdn_desc check_block_post(const On& on, const Tensor& o, const Tensor& z, const Tensor& w) {
+mxb_gdn_desc check_block_post(at::Device dev, const Tensor& o, const Tensor& z, const Tensor& w) {
   if (o.dim() != 4) throw py::value_error("o must be [B,T,H,Dv]");
   const int64_t B = o.size(0), T = o.size(1), H = o.size(2), Dv = o.size(3), zd[] = {B, T, H * Dv};
   const mxb_gdn_desc d{(int32_t)B, (int32_t)T, (int32_t)H, 8, (int32_t)Dv, 64, io_code(o), 0, 0};
-  check(o, o.sizes(), o.scalar_type(), on.dev, "o");
-  check(z, zd, o.scalar_type(), on.dev, "z");
-  check(w, Shape(&Dv, 1), F, on.dev, "o_norm");
+  check(o, o.sizes(), o.scalar_type(), dev, "o");
+  check(z, zd, o.scalar_type(), dev, "z");
+  check(w, Shape(&Dv, 1), F, dev, "o_norm");
   return d;
 }
 Tensor gdn_block_post(const Tensor& o, const Tensor& z, const Tensor& w) {
-  On on(o);
-  const mxb_gdn_desc d = check_block_post(on, o, z, w);
+  const at::Device dev = cuda_device(o);
+  const mxb_gdn_desc d = check_block_post(dev, o, z, w);
+  const On on(dev);
   Tensor y = like(z);
   call("mxb_gdn_block_post_fwd", abi.mxb_gdn_block_post_fwd, &d, ptr(o), ptr(z), ptr<float>(w), ptr(y), on.stream);
   return y;
 }
 py::dict gdn_block_post_backward(const Tensor& o, const Tensor& z, const Tensor& w, const Tensor& dy) {
-  On on(o);
-  const mxb_gdn_desc d = check_block_post(on, o, z, w);
-  check(dy, z.sizes(), o.scalar_type(), on.dev, "dy");
+  const at::Device dev = cuda_device(o);
+  const mxb_gdn_desc d = check_block_post(dev, o, z, w);
+  check(dy, z.sizes(), o.scalar_type(), dev, "dy");
+  const On on(dev);
   Tensor d_o = like(o), dz = like(z), dw = like(w);
   call_with_scratch(on, abi.mxb_gdn_block_workspace_bytes(&d), "mxb_gdn_block_post_bwd", abi.mxb_gdn_block_post_bwd,
                     &d, ptr(o), ptr(z), ptr<float>(w), ptr(dy), ptr(d_o), ptr(dz), ptr<float>(dw));
@@ -421,20 +432,20 @@ py::dict gdn_block_post_backward(const Tensor& o, const Tensor& z, const Tensor&
 }
 
 // ------------------------------------------------------------------ Mamba-3 scan
-mxb_mamba3_desc check_mamba3(const On& on, const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta,
+mxb_mamba3_desc check_mamba3(at::Device dev, const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta,
                              const Tensor& a_log, const Tensor& b, const Tensor& c, int64_t nheads, int64_t flags) {
   if (x.dim() != 3 || b.dim() != 4) throw py::value_error("x must be [B,T,D] and b, c [B,T,G,N]");
   const int64_t B = x.size(0), T = x.size(1), D = x.size(2), G = b.size(2), N = b.size(3);
   const mxb_mamba3_desc d{(int32_t)B, (int32_t)T, (int32_t)D, (int32_t)N, (int32_t)G, (int32_t)nheads, io_code(x), (int32_t)flags};
   const auto io = x.scalar_type();
   const int64_t per[] = {B, T, nheads > 0 ? nheads : D, N / 2}, al[] = {nheads > 0 ? nheads : D, N}, gn[] = {B, T, G, N};
-  check(x, x.sizes(), io, on.dev, "x");
-  check(dt, Shape(per, 3), F, on.dev, "dt");
-  check(lam, Shape(per, 3), F, on.dev, "lambda");
-  check(theta, Shape(per, nheads > 0 ? 3 : 4), F, on.dev, "theta");
-  check(a_log, Shape(al, nheads > 0 ? 1 : 2), F, on.dev, "a_log");
-  check(b, gn, io, on.dev, "b");
-  check(c, gn, io, on.dev, "c");
+  check(x, x.sizes(), io, dev, "x");
+  check(dt, Shape(per, 3), F, dev, "dt");
+  check(lam, Shape(per, 3), F, dev, "lambda");
+  check(theta, Shape(per, nheads > 0 ? 3 : 4), F, dev, "theta");
+  check(a_log, Shape(al, nheads > 0 ? 1 : 2), F, dev, "a_log");
+  check(b, gn, io, dev, "b");
+  check(c, gn, io, dev, "c");
   return d;
 }
 Token mamba3_token(const mxb_mamba3_desc& d, const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta,
@@ -443,8 +454,9 @@ Token mamba3_token(const mxb_mamba3_desc& d, const Tensor& x, const Tensor& dt, 
 }
 Tensor mamba3_forward(const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta, const Tensor& a_log, const Tensor& b,
                       const Tensor& c, int64_t nheads, int64_t flags, bool save) {
-  On on(x);
-  const mxb_mamba3_desc d = check_mamba3(on, x, dt, lam, theta, a_log, b, c, nheads, save ? flags | MXB_MAMBA3_SAVE_FOR_BWD : flags);
+  const at::Device dev = cuda_device(x);
+  const mxb_mamba3_desc d = check_mamba3(dev, x, dt, lam, theta, a_log, b, c, nheads, save ? flags | MXB_MAMBA3_SAVE_FOR_BWD : flags);
+  const On on(dev);
   Tensor y = like(x);
   mxb_status s;
   {
@@ -459,9 +471,10 @@ Tensor mamba3_forward(const Tensor& x, const Tensor& dt, const Tensor& lam, cons
 }
 py::dict mamba3_backward(const Tensor& x, const Tensor& dt, const Tensor& lam, const Tensor& theta, const Tensor& a_log, const Tensor& b,
                          const Tensor& c, const Tensor& dy, int64_t nheads, int64_t flags, bool use_saved) {
-  On on(x);
-  const mxb_mamba3_desc d = check_mamba3(on, x, dt, lam, theta, a_log, b, c, nheads, use_saved ? flags | MXB_MAMBA3_BWD_USE_SAVED : flags);
-  check(dy, x.sizes(), x.scalar_type(), on.dev, "dy");
+  const at::Device dev = cuda_device(x);
+  const mxb_mamba3_desc d = check_mamba3(dev, x, dt, lam, theta, a_log, b, c, nheads, use_saved ? flags | MXB_MAMBA3_BWD_USE_SAVED : flags);
+  check(dy, x.sizes(), x.scalar_type(), dev, "dy");
+  const On on(dev);
   Tensor dx = like(x), ddt = like(dt), dlam = like(lam), dth = like(theta), dal = like(a_log), db = like(b), dc = like(c);
   const size_t nws = abi.mxb_mamba3_bwd_workspace_bytes(&d);
   mxb_status s;
@@ -484,24 +497,26 @@ mxb_mamba3_desc m3_rows(const Tensor& x) {
   if (x.dim() != 3) throw py::value_error("expected a [B,T,D] tensor");
   return {(int32_t)x.size(0), (int32_t)x.size(1), (int32_t)x.size(2), 8, 1, 0, io_code(x), 0};
 }
-mxb_mamba3_desc check_conv(const On& on, const Tensor& x, const Tensor& w) {
+mxb_mamba3_desc check_conv(at::Device dev, const Tensor& x, const Tensor& w) {
   const mxb_mamba3_desc d = m3_rows(x);
   const int64_t wd[] = {d.D, w.dim() ? w.size(-1) : 0};
-  check(x, x.sizes(), x.scalar_type(), on.dev, "x");
-  check(w, wd, F, on.dev, "w");
+  check(x, x.sizes(), x.scalar_type(), dev, "x");
+  check(w, wd, F, dev, "w");
   return d;
 }
 Tensor mamba3_block_conv(const Tensor& x, const Tensor& w) {
-  On on(x);
-  const mxb_mamba3_desc d = check_conv(on, x, w);
+  const at::Device dev = cuda_device(x);
+  const mxb_mamba3_desc d = check_conv(dev, x, w);
+  const On on(dev);
   Tensor y = like(x);
   call("mxb_mamba3_block_conv_fwd", abi.mxb_mamba3_block_conv_fwd, &d, (int32_t)w.size(1), ptr(x), ptr<float>(w), ptr(y), on.stream);
   return y;
 }
 py::dict mamba3_block_conv_backward(const Tensor& x, const Tensor& w, const Tensor& dy) {
-  On on(x);
-  const mxb_mamba3_desc d = check_conv(on, x, w);
-  check(dy, x.sizes(), x.scalar_type(), on.dev, "dy");
+  const at::Device dev = cuda_device(x);
+  const mxb_mamba3_desc d = check_conv(dev, x, w);
+  check(dy, x.sizes(), x.scalar_type(), dev, "dy");
+  const On on(dev);
   Tensor dx = like(x), dw = like(w);
   call_with_scratch(on, abi.mxb_mamba3_block_workspace_bytes(&d), "mxb_mamba3_block_conv_bwd",
                     abi.mxb_mamba3_block_conv_bwd, &d, (int32_t)w.size(1), ptr(x), ptr<float>(w), ptr(dy), ptr(dx),
@@ -510,23 +525,24 @@ py::dict mamba3_block_conv_backward(const Tensor& x, const Tensor& w, const Tens
   r["dx"] = dx; r["dw"] = dw;
   return r;
 }
-mxb_mamba3_desc check_bc(const On& on, const Tensor& bp, const Tensor& cp, const Tensor& bs, const Tensor& cs, int64_t G, int64_t N) {
+mxb_mamba3_desc check_bc(at::Device dev, const Tensor& bp, const Tensor& cp, const Tensor& bs, const Tensor& cs, int64_t G, int64_t N) {
   if (bp.dim() != 3) throw py::value_error("b_proj must be [B,T,G*N]");
   const int64_t gn[] = {bp.size(0), bp.size(1), G * N};
   const mxb_mamba3_desc d{(int32_t)gn[0], (int32_t)gn[1], 8, (int32_t)N, (int32_t)G, 0, io_code(bp), 0};
-  check(bp, gn, bp.scalar_type(), on.dev, "b_proj");
-  check(cp, gn, bp.scalar_type(), on.dev, "c_proj");
-  check(bs, Shape(&N, 1), F, on.dev, "b_scale");
-  check(cs, Shape(&N, 1), F, on.dev, "c_scale");
+  check(bp, gn, bp.scalar_type(), dev, "b_proj");
+  check(cp, gn, bp.scalar_type(), dev, "c_proj");
+  check(bs, Shape(&N, 1), F, dev, "b_scale");
+  check(cs, Shape(&N, 1), F, dev, "c_scale");
   return d;
 }
 py::tuple mamba3_block_bc(const Tensor& bp, const Tensor& cp, const Tensor& bs, const Tensor& cs, const Tensor& bb, const Tensor& cb,
                           int64_t G, int64_t N, double eps) {
-  On on(bp);
-  const mxb_mamba3_desc d = check_bc(on, bp, cp, bs, cs, G, N);
+  const at::Device dev = cuda_device(bp);
+  const mxb_mamba3_desc d = check_bc(dev, bp, cp, bs, cs, G, N);
   const int64_t gn = G * N, o4[] = {d.B, d.T, G, N};
-  check(bb, Shape(&gn, 1), F, on.dev, "b_bias");
-  check(cb, Shape(&gn, 1), F, on.dev, "c_bias");
+  check(bb, Shape(&gn, 1), F, dev, "b_bias");
+  check(cb, Shape(&gn, 1), F, dev, "c_bias");
+  const On on(dev);
   Tensor b = make(o4, bp.scalar_type(), on.dev), c = make(o4, bp.scalar_type(), on.dev);
   call("mxb_mamba3_block_bc_fwd", abi.mxb_mamba3_block_bc_fwd, &d, (float)eps, ptr(bp), ptr(cp), ptr<float>(bs), ptr<float>(cs),
        ptr<float>(bb), ptr<float>(cb), ptr(b), ptr(c), on.stream);
@@ -534,11 +550,12 @@ py::tuple mamba3_block_bc(const Tensor& bp, const Tensor& cp, const Tensor& bs, 
 }
 py::dict mamba3_block_bc_backward(const Tensor& bp, const Tensor& cp, const Tensor& bs, const Tensor& cs, const Tensor& db,
                                   const Tensor& dc, int64_t G, int64_t N, double eps) {
-  On on(bp);
-  const mxb_mamba3_desc d = check_bc(on, bp, cp, bs, cs, G, N);
+  const at::Device dev = cuda_device(bp);
+  const mxb_mamba3_desc d = check_bc(dev, bp, cp, bs, cs, G, N);
   const int64_t gn = G * N, o4[] = {d.B, d.T, G, N};
-  check(db, o4, bp.scalar_type(), on.dev, "db");
-  check(dc, o4, bp.scalar_type(), on.dev, "dc");
+  check(db, o4, bp.scalar_type(), dev, "db");
+  check(dc, o4, bp.scalar_type(), dev, "dc");
+  const On on(dev);
   Tensor dbp = like(bp), dcp = like(cp), dbs = like(bs), dcs = like(cs), dbb = make(Shape(&gn, 1), F, on.dev), dcb = make(Shape(&gn, 1), F, on.dev);
   call_with_scratch(on, abi.mxb_mamba3_block_workspace_bytes(&d), "mxb_mamba3_block_bc_bwd",
                     abi.mxb_mamba3_block_bc_bwd, &d, (float)eps, ptr(bp), ptr(cp), ptr<float>(bs), ptr<float>(cs),
@@ -548,25 +565,27 @@ py::dict mamba3_block_bc_backward(const Tensor& bp, const Tensor& cp, const Tens
   r["db_proj"] = dbp; r["dc_proj"] = dcp; r["db_scale"] = dbs; r["dc_scale"] = dcs; r["db_bias"] = dbb; r["dc_bias"] = dcb;
   return r;
 }
-mxb_mamba3_desc check_post(const On& on, const Tensor& y, const Tensor& z, const Tensor& w) {
+mxb_mamba3_desc check_post(at::Device dev, const Tensor& y, const Tensor& z, const Tensor& w) {
   const mxb_mamba3_desc d = m3_rows(y);
   const int64_t D = d.D;
-  check(y, y.sizes(), y.scalar_type(), on.dev, "y");
-  check(z, y.sizes(), y.scalar_type(), on.dev, "z");
-  check(w, Shape(&D, 1), F, on.dev, "post_norm");
+  check(y, y.sizes(), y.scalar_type(), dev, "y");
+  check(z, y.sizes(), y.scalar_type(), dev, "z");
+  check(w, Shape(&D, 1), F, dev, "post_norm");
   return d;
 }
 Tensor mamba3_block_post(const Tensor& y, const Tensor& z, const Tensor& w, double eps) {
-  On on(y);
-  const mxb_mamba3_desc d = check_post(on, y, z, w);
+  const at::Device dev = cuda_device(y);
+  const mxb_mamba3_desc d = check_post(dev, y, z, w);
+  const On on(dev);
   Tensor out = like(y);
   call("mxb_mamba3_block_post_fwd", abi.mxb_mamba3_block_post_fwd, &d, (float)eps, ptr(y), ptr(z), ptr<float>(w), ptr(out), on.stream);
   return out;
 }
 py::dict mamba3_block_post_backward(const Tensor& y, const Tensor& z, const Tensor& w, const Tensor& dout, double eps) {
-  On on(y);
-  const mxb_mamba3_desc d = check_post(on, y, z, w);
-  check(dout, y.sizes(), y.scalar_type(), on.dev, "dout");
+  const at::Device dev = cuda_device(y);
+  const mxb_mamba3_desc d = check_post(dev, y, z, w);
+  check(dout, y.sizes(), y.scalar_type(), dev, "dout");
+  const On on(dev);
   Tensor dy = like(y), dz = like(z), dw = like(w);
   call_with_scratch(on, abi.mxb_mamba3_block_workspace_bytes(&d), "mxb_mamba3_block_post_bwd",
                     abi.mxb_mamba3_block_post_bwd, &d, (float)eps, ptr(y), ptr(z), ptr<float>(w), ptr(dout), ptr(dy),
@@ -585,8 +604,9 @@ Tensor ir_op_forward(int64_t op_type, const std::vector<Tensor>& inputs, const s
     if (!inputs[i].is_contiguous() || inputs[i].device() != inputs[0].device())
       throw py::value_error("input " + std::to_string(i) + ": contiguous tensors on one device expected");
   if (inputs.empty()) throw py::value_error("an op record has inputs");
-  On on(inputs[0]);
+  const at::Device dev = cuda_device(inputs[0]);
   const int32_t io = io_code(inputs[0]);
+  const On on(dev);
   Tensor out = make(out_shape, inputs[0].scalar_type(), on.dev);
   std::vector<const void*> in;
   for (const Tensor& t : inputs) in.push_back(t.data_ptr());

@@ -41,23 +41,6 @@ def _io(t: torch.Tensor) -> int:
     raise TypeError(f"unsupported dtype {t.dtype} (float32 or bfloat16)")
 
 
-def _check_like(t, shape, dtype, device, name):
-    """Raises unless ``t`` (None allowed) is a contiguous CUDA tensor of exactly this shape, dtype and device:
-    the C ABI sees only pointers, so a wrong operand would otherwise be read out of bounds or as the wrong type."""
-    if t is None:
-        return
-    if not t.is_cuda:
-        raise ValueError("mixlab_b200 operators take CUDA tensors only (no CPU fallback)")
-    if tuple(t.shape) != tuple(shape):
-        raise ValueError(f"{name}: shape {tuple(t.shape)}, expected {tuple(shape)}")
-    if t.dtype != dtype:
-        raise TypeError(f"{name}: dtype {t.dtype}, expected {dtype}")
-    if t.device != device:
-        raise ValueError(f"{name}: on {t.device}, expected {device}")
-    if not t.is_contiguous():
-        raise ValueError(f"{name}: tensor must be contiguous")
-
-
 def workspace(nbytes: int, device) -> torch.Tensor:
     """The cached byte buffer of the current stream of ``device``, of at least ``nbytes`` (torch allocator).  The operators
     called on that stream use it too."""

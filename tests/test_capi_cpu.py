@@ -121,35 +121,71 @@ def test_chunk_above_64_is_accepted():
     assert lib.mxb_gdn_bwd_workspace_bytes(C.byref(wide)) > 0
 
 
-def test_ops_check_every_operand():
-    """Shape, dtype and device of every operand are checked in Python before the C ABI sees a pointer.  The checks
-    run before the CUDA requirement is looked at only for CUDA tensors, so this uses the helper directly."""
+B, T, H, DK, DV, N, G, D = 2, 6, 4, 8, 16, 8, 2, 24
+F32, BF16 = "float32", "bfloat16"
+_SCAN = {"q": ((B, T, H, DK), BF16), "k": ((B, T, H, DK), BF16), "v": ((B, T, H, DV), BF16), "beta": ((B, T, H), F32),
+         "gate": ((B, T, H), F32)}
+_STATE = ((B, H, DK, DV), F32)
+_PRE = {"q_proj": ((B, T, H * DK), BF16), "k_proj": ((B, T, H * DK), BF16), "v_proj": ((B, T, H * DV), BF16),
+        "conv_q": ((4, H * DK), F32), "conv_k": ((4, H * DK), F32), "conv_v": ((4, H * DV), F32), "a_raw": ((B, T, H), F32),
+        "b_raw": ((B, T, H), F32), "a_log": ((H,), F32), "dt_bias": ((H,), F32)}
+_POST = {"o": ((B, T, H, DV), BF16), "z": ((B, T, H * DV), BF16), "o_norm": ((DV,), F32)}
+_M3 = {"x": ((B, T, D), BF16), "dt": ((B, T, D), F32), "lam": ((B, T, D), F32), "theta": ((B, T, D, N // 2), F32),
+       "a_log": ((D, N), F32), "b": ((B, T, G, N), BF16), "c": ((B, T, G, N), BF16)}
+_M3H = dict(_M3, dt=((B, T, H), F32), lam=((B, T, H), F32), theta=((B, T, H), F32), a_log=((H,), F32))
+_BC = {"b_proj": ((B, T, G * N), BF16), "c_proj": ((B, T, G * N), BF16), "b_scale": ((N,), F32), "c_scale": ((N,), F32)}
+_ROWS = ((B, T, D), BF16)
+_OPERANDS = {  # operator: its tensor operands (shape, dtype), the other arguments
+    "gated_delta_scan": (dict(_SCAN, h0=_STATE), {}),
+    "gated_delta_scan_backward": (dict(_SCAN, d_out=((B, T, H, DV), BF16), h0=_STATE, d_final_state=_STATE), {}),
+    "gated_delta_decode_step": (dict(state=_STATE, q=((B, H, DK), BF16), k=((B, H, DK), BF16), v=((B, H, DV), BF16),
+                                     beta=((B, H), F32), gate=((B, H), F32), out=((B, H, DV), BF16)), {}),
+    "gdn_block_pre": (_PRE, dict(H=H, Dk=DK, Dv=DV)),
+    "gdn_block_pre_backward": (dict(_PRE, dq=((B, T, H, DK), BF16), dk=((B, T, H, DK), BF16), dv=((B, T, H, DV), BF16),
+                                    dbeta=((B, T, H), F32), dgate=((B, T, H), F32)), dict(H=H, Dk=DK, Dv=DV)),
+    "gdn_block_post": (_POST, {}),
+    "gdn_block_post_backward": (dict(_POST, dy=((B, T, H * DV), BF16)), {}),
+    "mamba3_selective_scan": (_M3, {}),
+    "mamba3_selective_scan_backward": (dict(_M3, dy=((B, T, D), BF16)), {}),
+    "mamba3_selective_scan (heads)": (_M3H, dict(nheads=H)),
+    "mamba3_block_conv": (dict(x=_ROWS, w=((D, 4), F32)), {}),
+    "mamba3_block_conv_backward": (dict(x=_ROWS, w=((D, 4), F32), dy=_ROWS), {}),
+    "mamba3_block_bc": (dict(_BC, b_bias=((G * N,), F32), c_bias=((G * N,), F32)), dict(G=G, N=N)),
+    "mamba3_block_bc_backward": (dict(_BC, db=((B, T, G, N), BF16), dc=((B, T, G, N), BF16)), dict(G=G, N=N)),
+    "mamba3_block_post": (dict(y=_ROWS, z=_ROWS, post_norm=((D,), F32)), {}),
+    "mamba3_block_post_backward": (dict(y=_ROWS, z=_ROWS, post_norm=((D,), F32), dout=_ROWS), {}),
+}
+
+
+@pytest.mark.parametrize("op", _OPERANDS)
+def test_ops_check_every_operand(op):
+    """Shape, dtype, device and layout of every operand are checked before the C ABI sees a pointer and before the device
+    is touched: tensors without storage that say they are on a GPU get as far as the checks here."""
     import torch
-    from mixlab_b200 import ops
-    dev = torch.device("cpu")
-    t = torch.zeros(2, 3)
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    specs, rest = _OPERANDS[op]
+    fn = getattr(mixlab_b200.ops, op.split()[0])
 
-    class FakeCuda:
-        """Stands in for a CUDA tensor: only the attributes the checker reads."""
-        def __init__(self, shape, dtype, device="cuda:0", contiguous=True):
-            self.shape, self.dtype, self.device, self._c, self.is_cuda = shape, dtype, device, contiguous, True
+    def refused(name, error, make):
+        args = {n: torch.empty(shape, dtype=getattr(torch, dt), device="cuda:0") for n, (shape, dt) in specs.items()}
+        args[name] = make(*specs[name])
+        with pytest.raises(error) as e:
+            fn(**args, **rest)
+        return str(e.value)
 
-        def is_contiguous(self):
-            return self._c
-
-    good = FakeCuda((2, 3), torch.float32)
-    ops._check_like(good, (2, 3), torch.float32, "cuda:0", "x")
-    ops._check_like(None, (2, 3), torch.float32, "cuda:0", "x")
-    with pytest.raises(ValueError):
-        ops._check_like(t, (2, 3), torch.float32, dev, "x")                              # not a CUDA tensor
-    with pytest.raises(ValueError):
-        ops._check_like(FakeCuda((2, 4), torch.float32), (2, 3), torch.float32, "cuda:0", "x")
-    with pytest.raises(TypeError):
-        ops._check_like(FakeCuda((2, 3), torch.bfloat16), (2, 3), torch.float32, "cuda:0", "x")
-    with pytest.raises(ValueError):
-        ops._check_like(FakeCuda((2, 3), torch.float32, "cuda:1"), (2, 3), torch.float32, "cuda:0", "x")
-    with pytest.raises(ValueError):
-        ops._check_like(FakeCuda((2, 3), torch.float32, contiguous=False), (2, 3), torch.float32, "cuda:0", "x")
+    first = next(iter(specs))
+    with FakeTensorMode():
+        for name, (shape, dt) in specs.items():
+            own, other = getattr(torch, dt), torch.float64 if name == first else torch.float16
+            refused(name, ValueError, lambda s, _: torch.empty(s, dtype=own, device="cpu"))
+            refused(name, ValueError, lambda s, _: torch.empty(*s, 1, dtype=own, device="cuda:0"))
+            refused(name, TypeError, lambda s, _: torch.empty(s, dtype=other, device="cuda:0"))
+            msg = refused(name, ValueError, lambda s, _: torch.empty(*s[:-1], 2 * s[-1], dtype=own, device="cuda:0")[..., ::2])
+            assert "contiguous" in msg, (name, msg)
+            if name != first:  # (the first operand's sizes and device are what the others are held to)
+                refused(name, ValueError, lambda s, _: torch.empty(s[0] + 1, *s[1:], dtype=own, device="cuda:0"))
+                msg = refused(name, ValueError, lambda s, _: torch.empty(s, dtype=own, device="cuda:1"))
+                assert "cuda:1" in msg, (name, msg)
 
 
 def test_ir_op_records_are_validated_like_the_interpreter():
