@@ -722,16 +722,13 @@ bool make_tma_map_f32(CUtensorMap* m, const void* base, int B, int T, int H, int
   return make_tma_map(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, B, T, H, D);
 }
 
-static bool g_tc_use_tma = true;
-void gdn_tc_set_tma(bool on) { g_tc_use_tma = on; }
-
 mxb_status tc_run_fwd(TcP& p, cudaStream_t st) {
   if (is64(p)) return tc64_run_fwd(p, st);
   PrepMaps maps;
   std::memset(&maps, 0, sizeof maps);
   // heads narrower than the tiles exist only through the copy engine (the per-thread staging addresses full rows)
   const bool narrow = p.Dk != KD || p.Dv != KD;
-  const bool tma = g_tc_use_tma && (!p.no_tma || narrow) && make_tma_map_bthd(&maps.k, p.k, p.B, p.T, p.H, p.Dk) &&
+  const bool tma = (!p.no_tma || narrow) && make_tma_map_bthd(&maps.k, p.k, p.B, p.T, p.H, p.Dk) &&
                    make_tma_map_bthd(&maps.q, p.q, p.B, p.T, p.H, p.Dk) && make_tma_map_bthd(&maps.v, p.v, p.B, p.T, p.H, p.Dv) &&
                    make_tma_map_bthd(&maps.o, p.out, p.B, p.T, p.H, p.Dv);
   if (narrow && !tma) return MXB_ERR_UNSUPPORTED;

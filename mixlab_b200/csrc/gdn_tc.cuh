@@ -17,7 +17,6 @@ bool make_tma_map_bthd(CUtensorMap* m, const void* base, int B, int T, int H, in
 namespace tcg {
 constexpr int C = 64;     // chunk
 constexpr int KD = 128;   // Dk = Dv
-constexpr int VS = 64;    // Dv columns per state CTA
 constexpr int LDA = 68;   // fp32 row pitch of the 64x64 solve matrix (16-byte aligned rows)
 using bf16 = __nv_bfloat16;
 
@@ -59,7 +58,6 @@ struct alignas(64) RowMaps {
 __device__ __forceinline__ float log_gate_tc(float g, int gate_is_log) {
   return gate_is_log ? fmaxf(g, kLogGateFloor) : __logf(fmaxf(g, kGateFloor));
 }
-__device__ __forceinline__ uint4 ldg16(const void* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
 __device__ __forceinline__ void sts16(uint8_t* base, uint32_t off, uint4 v) {
   *reinterpret_cast<uint4*>(base + off) = v;
 }
@@ -79,24 +77,6 @@ __device__ __forceinline__ void ld_acc32(uint32_t taddr, int warp, int c0, float
   tc::tmem_ld_wait();
 #pragma unroll
   for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(r[i]);
-}
-// Two blocks of 32 accumulator columns [c0, c0+32), [c0+32, c0+64) of this thread's TMEM lane, the second load in
-// flight while the first block is processed: process(column of the block, values).
-template <typename F>
-__device__ __forceinline__ void for_acc2x32(uint32_t taddr, int warp, int c0, F&& process) {
-  uint32_t r0[32], r1[32];
-  const uint32_t base = taddr + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)c0;
-  tc::tmem_ld_32x32b_x32(base, r0);
-  tc::tmem_ld_wait();
-  tc::tmem_ld_32x32b_x32(base + 32u, r1);
-  float f[32];
-#pragma unroll
-  for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(r0[i]);
-  process(c0, f);
-  tc::tmem_ld_wait();
-#pragma unroll
-  for (int i = 0; i < 32; ++i) f[i] = __uint_as_float(r1[i]);
-  process(c0 + 32, f);
 }
 // The sequential passes of 128-wide heads take half of the state's columns per CTA where that still puts every CTA on an
 // SM of its own: the chain of a chunk is what counts then, not the bytes (forward and backward, us a chunk: 2.55 and 2.4

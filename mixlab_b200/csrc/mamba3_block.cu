@@ -144,16 +144,6 @@ __global__ void __launch_bounds__(128) m3b_conv_bwd_kernel(BlkP p, const IO* __r
 #pragma unroll
   for (int k = 0; k < kMaxK; ++k) store8<float>(dst + (size_t)k * p.D, dw[k]);
 }
-// dw[d][k] = sum over rows of dwp[row][k][d]  (fixed order); one thread per (d, k)
-__global__ void __launch_bounds__(256) m3b_conv_dw_kernel(BlkP p, const float* __restrict__ dwp, int rows,
-                                                          float* __restrict__ dw) {
-  const int i = blockIdx.x * 256 + threadIdx.x;
-  if (i >= p.D * p.K) return;
-  const int d = i / p.K, k = i % p.K;
-  float s = 0.f;
-  for (int r = 0; r < rows; ++r) s += dwp[((size_t)r * kMaxK + k) * p.D + d];
-  dw[i] = s;
-}
 // out[f(j)] = sum over rows of part[row][j] in a fixed order: a CTA owns 32 columns, its 8 warps take every 8th row,
 // then the 8 slices are added in order.  K > 0: columns are [k][d] and the result is stored as [d][K] (k < K only).
 __global__ void __launch_bounds__(256) m3b_colsum_kernel(const float* __restrict__ part, int rows, int n,

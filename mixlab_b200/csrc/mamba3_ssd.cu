@@ -55,7 +55,6 @@ struct SsdP {
 
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : (x < -20.f ? expf(x) : log1pf(expf(x))); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + expf(-x)); }
-__device__ __forceinline__ uint4 ldg16(const void* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
 __device__ __forceinline__ void sts16(uint8_t* base, uint32_t off, uint4 v) { *reinterpret_cast<uint4*>(base + off) = v; }
 __device__ __forceinline__ void unpack8(uint4 v, float (&e)[8]) {
   tc::unpack_bf16(v.x, e[0], e[1]); tc::unpack_bf16(v.y, e[2], e[3]);
@@ -668,7 +667,7 @@ __global__ void __launch_bounds__(256) m3s_chunk_grad_kernel(SsdP p, const __gri
   const int d0 = head * P, g = d0 / (p.D / p.G);
   const size_t ci = ((size_t)b * p.NH + head) * p.n + c;
   // this thread's row and column quarter of every result; tc16 / tc32: its TMEM columns of a [64][64] / [64][128] result
-  const int t = 32 * (warp & 1) + lane, qd = (warp & 2) + (warp >> 2), n16 = 16 * qd, n32 = 32 * qd;
+  const int t = 32 * (warp & 1) + lane, qd = (warp & 2) + (warp >> 2), n16 = 16 * qd;
   const int tc16 = 16 * (warp >> 2), tc32 = 32 * (warp >> 2);
 
   if (warp == 0) { tc::tmem_alloc(tslot, 256); tc::tmem_relinquish(); }

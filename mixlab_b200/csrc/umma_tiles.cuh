@@ -58,13 +58,6 @@ __device__ __forceinline__ Tile mnmajor_sw128_tile(const void* smem, uint32_t sl
   t.swizzle = kSwizzle128;
   return t;
 }
-// Sub-tile starting at row r0 (multiple of 8) of a K-major tile / at column m0 (multiple
-// of 8) of an MN-major tile.
-__device__ __forceinline__ Tile kmajor_rows(Tile t, int r0) { t.saddr += (uint32_t)(r0 / 8) * t.sbo; return t; }
-__device__ __forceinline__ Tile mnmajor_cols(Tile t, int m0) { t.saddr += (uint32_t)(m0 / 8) * 128u; return t; }
-// Skip k0 (multiple of 16) contraction elements.
-__device__ __forceinline__ Tile skip_k(Tile t, int k0) { t.saddr += (uint32_t)(k0 / 16) * t.kstep; return t; }
-
 // Byte offset of the 16-byte unit holding elements (r, 8*c8 .. 8*c8+7) of a K-major tile.
 __device__ __forceinline__ uint32_t kmajor_unit(int r, int c8, int kcols) {
   return (uint32_t)(r >> 3) * (uint32_t)(kcols / 8) * 128u + (uint32_t)c8 * 128u + (uint32_t)(r & 7) * 16u;
