@@ -98,9 +98,9 @@ def test_gdn_saved_forward_and_staging_variants():
     assert all(bool(torch.isfinite(t.float()).all()) for t in (out, g["dq"], g["dk"], g["dv"], g["dbeta"], g["dgate"]))
 
 
-def test_gdn_decode_kernels_agree_and_match_one_step_scan():
-    """256 sequences x 16 heads: the streaming decode kernel and the register kernel give the same step; a
-    one-token scan from the same state gives the same output and state (fp32 I/O; summation orders differ: 1e-5)."""
+def test_gdn_decode_matches_one_step_scan():
+    """256 sequences x 16 heads: a decode step gives the output and state of a one-token scan from the same state (fp32 I/O;
+    summation orders differ: 1e-4).  The flag that once chose a kernel is accepted and changes no bit."""
     N, H, D = 256, 16, 128
     g = torch.Generator(device=DEV).manual_seed(21)
 
@@ -123,7 +123,7 @@ def test_gdn_decode_kernels_agree_and_match_one_step_scan():
     def close(x, y, tol):
         return float((x.double() - y.double()).abs().max()) <= tol * max(1.0, float(y.double().abs().max()))
 
-    assert close(o1, o2, 1e-5) and close(s1, s2, 1e-5)
+    assert torch.equal(o1, o2) and torch.equal(s1, s2)
     assert close(o1, o3[:, 0], 1e-4) and close(s1, s3, 1e-4)
 
 
