@@ -401,6 +401,11 @@ MXB_API mxb_status mxb_selftest_umma(const void* a_img, uint32_t a_bytes, const 
 MXB_API mxb_status mxb_selftest_wait_timeout(void* workspace, size_t workspace_bytes,
                                      uint32_t poll_limit, void* stream);
 
+/* Sines and cosines of n angles (device arrays) as the window-parallel Mamba-3 kernels
+ * form them: exact to 1.2e-7 for angles in [-pi, pi], where those kernels keep theirs. */
+MXB_API mxb_status mxb_selftest_sincos(const float* angles, size_t n, float* sines, float* cosines,
+                                     void* stream);
+
 /* ------------------------------------------------------------------------
  * Host-buffer evaluation, the shape of the reference bridge's
  * mlx_ir_eval_program_named_for_output / _grads_named_for_output

@@ -100,6 +100,7 @@ mxb_status gdn_tc_bwd(const mxb_gdn_desc*, const void*, const void*, const void*
                       float*, float*, float*, void*, cudaStream_t);
 mxb_status umma_selftest(const void*, uint32_t, const void*, uint32_t, const uint32_t*, float*, int*, cudaStream_t);
 mxb_status wait_timeout_selftest(void*, uint32_t, cudaStream_t);
+mxb_status m3w_sincos_selftest(const float*, size_t, float*, float*, cudaStream_t);
 bool gdn_block_supported(const mxb_gdn_desc*);
 size_t gdn_block_workspace_bytes(const mxb_gdn_desc*);
 mxb_status gdn_block_pre_fwd(const mxb_gdn_desc*, const void*, const void*, const void*, const float*, const float*,
@@ -460,6 +461,11 @@ mxb_status mxb_selftest_wait_timeout(void* workspace, size_t workspace_bytes, ui
   if (!workspace || workspace_bytes < 256) return MXB_ERR_WORKSPACE;
   if (!aligned16(workspace)) return MXB_ERR_ALIGNMENT;
   return wait_timeout_selftest(workspace, poll_limit, static_cast<cudaStream_t>(stream));
+}
+
+mxb_status mxb_selftest_sincos(const float* angles, size_t n, float* sines, float* cosines, void* stream) {
+  if (!angles || !sines || !cosines || n == 0) return MXB_ERR_INVALID_ARGUMENT;
+  return m3w_sincos_selftest(angles, n, sines, cosines, static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------- Mamba-3 block stages

@@ -1,12 +1,14 @@
 """Parity of the CUDA Mamba-3 scan (through the C ABI) with the CPU oracle."""
+import ctypes as C
 import json
+import math
 import os
 
 import numpy as np
 import pytest
 import torch
 
-from mixlab_b200 import ops
+from mixlab_b200 import _lib, ops
 from oracle import inputs, mamba3
 from tests.util import assert_close, rel_errs
 
@@ -256,3 +258,24 @@ def test_window_parallel_matches_serial_walk(shape):
     gw = ops.mamba3_selective_scan_backward(*dev, _dev(a["dy"]), flags=_lib.MXB_MAMBA3_WINDOW_PARALLEL)
     for name in GRADS:
         assert_close(gw[name], gs[name].double(), 1e-5, name)
+
+
+@pytest.mark.parametrize("n", [1, 2, 513, 1 << 24])
+def test_sines_and_cosines_of_the_window_kernels(n):
+    """Against double precision.  The bound is that of the method, two roundings of the reduced angle (6e-8) and the last
+    operations of the polynomials (5e-8): 1.2e-7.  NaN and infinity give NaN."""
+    pi = math.pi
+    x = torch.linspace(-pi, pi, n, dtype=torch.float64, device="cuda").float() if n > 513 else torch.empty(n, device="cuda")
+    if n <= 513:  # the ends, the multiples of pi/4 where the reduction changes over, and their neighbours
+        at = torch.tensor([0.0, pi, -pi] + [k * pi / 4 for k in range(-4, 5)], dtype=torch.float64).float()
+        at = torch.cat([at, torch.nextafter(at, at + 1), torch.nextafter(at, at - 1), at * 1e-20, 1e-3 * at])
+        x.copy_(at.repeat(n // at.numel() + 1)[-n:])
+    sn, cs = torch.empty_like(x), torch.empty_like(x)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    assert _lib.lib().mxb_selftest_sincos(p(x), n, p(sn), p(cs), None) == 0
+    assert float((sn.double() - torch.sin(x.double())).abs().max()) <= 1.2e-7
+    assert float((cs.double() - torch.cos(x.double())).abs().max()) <= 1.2e-7
+    bad = torch.tensor([float("nan"), float("inf"), float("-inf")], device="cuda")
+    sn, cs = torch.empty_like(bad), torch.empty_like(bad)
+    assert _lib.lib().mxb_selftest_sincos(p(bad), 3, p(sn), p(cs), None) == 0
+    assert bool(torch.isnan(sn).all()) and bool(torch.isnan(cs).all())
