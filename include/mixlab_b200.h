@@ -247,8 +247,8 @@ enum {
                                       (batch, channel) pair, also where there are too few pairs to fill the GPU */
   MXB_MAMBA3_WINDOW_PARALLEL = 64, /* warp-per-channel kernels: one lane group per (batch, channel, window of 8
                                       steps) with scans over the windows in between, also where the pairs alone
-                                      would fill the GPU (the window form does about twice the arithmetic; by
-                                      default it is taken when 2 B D <= 148 x 64 warps).  The forward then needs
+                                      would fill the GPU (the window form keeps several times the scratch; by
+                                      default it is taken when 2 B D <= 148 x 64 and T > 16).  The forward then needs
                                       the workspace mxb_mamba3_fwd_workspace_bytes reports. */
   MXB_MAMBA3_BWD_USE_SAVED = 8     /* backward: the workspace is the one a forward call with
                                       MXB_MAMBA3_SAVE_FOR_BWD just filled for the same inputs; the forward

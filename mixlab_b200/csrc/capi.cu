@@ -643,10 +643,22 @@ __global__ void __launch_bounds__(256) head_scatter_kernel(const float* __restri
 // Bound by the PCIe link, 64 MB each way in 1.36 ms when both directions run.  Besides that a call takes the first
 // upload and the last download (one slice, which nothing overlaps), one slice's chain of kernels, and about 11 us per
 // copy when both directions run (the strided row width makes no difference down to 512 bytes): with S slices of 4
-// copies, bytes / (S * 49 GB/s) + S * 44 us, least near S = sqrt(bytes / 2.25 MB).  More slices than that lost at
-// every size (2 x 2048 x 16 heads of 128: 2, 4, 8 slices 2161, 1852, 1980 us; 4 x 1024 x 16: 4, 8, 16 slices 1868,
-// 1855, 2500; 2 x 700 x 16: 2, 4, 8 slices 756, 793, 988; 1 x 200 x 8: 1, 2 slices 156, 181;
-// 8 x 4096 x 16: 8, 16, 32 slices 13.6, 11.9, 12.7 ms).
+// copies, bytes / (S * 49 GB/s) + S * 44 us, least near S* = sqrt(bytes / 2.25 MB), and flat around it.  Measured on
+// buffers in use (heads of 128, bf16, forward + backward, us at 1, 2, 4, 8, 16, .. slices):
+//   1 x 200 x 8    S* 0.9    144, 174                      2 x 2048 x 16  S* 5.5   2360, 2088, 1854, 1857, 1941
+//   1 x 700 x 8    S* 1.6    290-310, 303-317, 341         4 x 1024 x 16  S* 5.5   2335, 2040, 2015, 1780, 2400
+//   2 x 700 x 16   S* 3.2    875, 770, 757, 925            1 x 4096 x 16  S* 5.5   2400, 2016, 1940, 1915
+//   4 x 512 x 16   S* 3.9    1216, 1100, 1110, 1156        4 x 2048 x 16  S* 7.7   4584, 3920, 3770, 3338, 3459
+//   8 x 4096 x 16  S* 15.5   17.8, 14.8, 13.6, 13.6, 11.8, 12.7 ms
+// (at 4 x 1024 x 16 another host took 1868 with four slices, 1855 with eight).  The cut goes up to S* whole sequences,
+// then to groups of heads as long as the doubled count is at most 1.1 S*.  In the model doubling S pays up to 2 S = 1.41 S*;
+// between the two lie 2 x 700 x 16 and 1 x 700 x 8, where it gained and lost a few percent, and the coarser cut leaves
+// more of the arena.
+//
+// Pinned pages that the copy engines meet for the first time are slow whatever the cut: medians over 20 fresh sets of
+// buffers, us against buffers in use: 2 x 2048 x 16 2167 against 1862, 1 x 2048 x 16 2333 against 1089, 4 x 1024 x 8
+// 2447 against 1131, 2 x 700 x 16 2254 against 803 (cuts of 16 slices with per-thread staging: 2408, 2301, 2566, 2075).
+// A new context costs nothing.
 struct HostSlicing {
   int per, nsplit;  // sequences per slice; head groups per sequence (one sequence per slice then)
 };

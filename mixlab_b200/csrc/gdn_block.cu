@@ -275,7 +275,8 @@ __global__ void __launch_bounds__(256) gdn_block_gate_fwd_kernel(BlockP p, const
 // Same map as the forward.  A run recomputes the convolution of its steps and of the three steps after it (their ds
 // feeds dx of the run) and emits dx three steps behind.  Bound: HBM (nine tensors) and, close behind, issue: about
 // 17 instructions per element with packed arithmetic (40 and half of the lanes idle at 64 channels before: 760 us for
-// 16 x 2048 x 16 heads of 64 bf16 channels).
+// 16 x 2048 x 16 heads of 64 bf16 channels, 189 now).  Two CTAs per SM leave a thread 128 registers, which its weights,
+// weight gradients, seven inputs and seven ds of four channels exceed: the compiler spills about 180 bytes of them.
 template <typename IO, int LPR>
 __global__ void __launch_bounds__(256, 2) gdn_block_pre_bwd_kernel(BlockP p, PreArgs<IO> a, int run, int first) {
   extern __shared__ __align__(16) uint8_t pre_smem[];

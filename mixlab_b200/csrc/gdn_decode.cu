@@ -13,8 +13,9 @@
 // (a row of the slab is one 128-byte line, a warp reads four rows with 128-bit loads), thread group rg = tid / 8
 // owns rows rg, rg + 16, ... and keeps its ROWS float4 pieces of the state in registers between load and store.
 // Many small CTAs keep more loads in flight than a pipeline over shared memory did (64 KB tiles, one persistent CTA per
-// SM, bulk copies): 256 sequences x 16 heads of 128 x 128 take 80 us instead of 93.7 (6.8 TB/s read + written), one
-// sequence 1.9 us instead of 4.5.  Bound: HBM, and the latency of one load -> sum -> store chain for the small calls.
+// SM, bulk copies): a step of 256 sequences x 16 heads of 128 x 128 takes 84 us instead of 95 (6.5 TB/s read + written),
+// one sequence 4.1 us beside other steps instead of 17 (most of that was host work).  Bound: HBM, and the launch and the
+// latency of one load -> sum -> store chain for the small calls.
 #include "common.cuh"
 
 namespace mxb {

@@ -54,7 +54,7 @@ struct GdnP {
   void *dq, *dk, *dv;
   float *dbeta, *dgate, *dh0;
   // workspace, all fp32, indexed by ci = (b*H+h)*n + chunk
-  int* status;  // 256-byte header, always zero on this path
+  int* status;  // 256-byte header: 5 when a bounded wait gave up
   float *gam;   // [C]
   float *Tm;    // [C,C]  (written when the forward saves for the backward)
   float *w;     // [C,K]
@@ -1311,7 +1311,7 @@ __global__ void __launch_bounds__(256) gdn_recurrent_fwd_kernel(GdnP p) {
 static size_t carve(GdnP& p, void* ws, bool bwd) {
   Carver cv(ws);
   const size_t nc = (size_t)p.B * p.H * p.n, C = p.C, K = p.K, V = p.V;
-  p.status = cv.take<int>(64);  // device status header (always zero on this path)
+  p.status = cv.take<int>(64);
   p.gam = cv.take<float>(nc * C);
   p.Tm = cv.take<float>(nc * C * C);
   p.w = cv.take<float>(nc * C * K);

@@ -10,11 +10,11 @@
 // the triangular inverse, all decay factors, the recurrent state and every
 // reduction stay in fp32.
 //
-//   gdn_tc_prep_kernel       one CTA per chunk (three per SM): [k;q] k^T (M=128), fp32 solve,
-//                            (T beta) v and (T beta E(gam)) k (M=64, N=128 each) -> u, w, P, T
-//   gdn_tc_state_fwd_kernel  one CTA per (batch, head), sequential over chunks, fp32 state in
-//                            registers (thread = state row, 64 columns), operands two chunks ahead:
-//                            [w;q] S (M=128) -> v_new, then [0;P] v_new and (r k)^T v_new
+//   gdn_tc_prep_kernel       one CTA per chunk (four per SM): [k;q] k^T (M=128), fp32 solve,
+//                            (T beta) v and (T beta) (E(gam) k) (M=64, N=128 each) -> u, w, P, T
+//   gdn_tc_state_fwd_kernel  one CTA per (batch, head) and 128 or 64 columns of the state, sequential over
+//                            chunks, fp32 state in registers (thread = state row, half of the columns), operands
+//                            two chunks ahead: [w;q] S (M=128) -> v_new, then (r k)^T v_new and P v_new
 #include <cuda.h>
 
 #include <cstring>
@@ -25,12 +25,12 @@ namespace mxb {
 
 // ------------------------------------------------------------------ prep
 // u = T (v beta) and w = T (k beta E(gam)) are evaluated as (T diag(beta)) v and
-// (T diag(beta E(gam))) k: the scaling goes into two column-scaled bf16 copies of T written
-// straight from the solve's registers, so k, q and v are staged raw.
+// (T diag(beta)) (diag(E(gam)) k): one column-scaled bf16 copy of T serves both, k, q and v are staged raw
+// and k is scaled in place while T is formed.
 //
 // A CTA is a chain of dependent steps (copy -> MMA -> epilogue -> solve -> MMA -> epilogue -> stores) that leaves
-// the SM idle most of the time, so the kernel is sized for FOUR CTAs per SM: 128 TMEM columns (u and w go through
-// the same columns one after the other) and 51 KB of shared memory, every region reused as soon as it is dead:
+// the SM idle most of the time, so the kernel is sized for FOUR CTAs per SM: 128 TMEM columns (u and w side by side,
+// 64 each, once the product before has been read) and 51 KB of shared memory, every region reused as soon as it is dead:
 //   [k;q] (32 KB, two slabs of 64 columns: k box then q box)  ->  v lands in the q boxes once q k^T is done
 //                                                              ->  k scaled to diag(d) k in place during the solve
 //                                                              ->  u image over v, w image over k

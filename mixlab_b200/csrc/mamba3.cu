@@ -17,8 +17,9 @@
 // without a state pair at the sizes the reference runs (d_state 16).  The cumulative angle is kept wrapped
 // to [-pi, pi] so fp32 keeps its resolution over thousands of steps.
 //
-// Short problems (few batch x channel pairs) would leave most of the GPU idle behind T-long walks: they run
-// window-parallel (mamba3_windows.cu), with about twice the arithmetic.
+// Problems of few batch x channel pairs would leave most of the GPU idle behind T-long walks: they run
+// window-parallel (mamba3_windows.cu), which forms the decays, sines and cosines of a step in two passes (three with the
+// backward's) and needs several times the scratch.
 //
 // Two parameter layouts share the kernels through index helpers: the
 // reference's per-channel one, and a head-broadcast one where dt, lambda, theta
@@ -420,7 +421,15 @@ static int m3_channel_warps(const M3P& p) {
 }
 
 // Window-parallel channel kernels: where the (batch, channel) pairs alone leave half of the GPU's warp slots empty,
-// unless a flag asks for one of the two forms.
+// unless a flag asks for one of the two forms.  The line bounds scratch and is not where the times cross.  Scratch, bytes
+// per channel and step, forward / backward: windows 20 / 50 at N 16, 104 / 456 at N 128; serial walk 0 / 10, 0 / 176.  The
+// windows are the faster form on both sides of the line but for sequences of a few windows and the forward of N 256.
+// Float32, forward / backward, serial walk against windows, us:
+//   N 16, T 512   2BD  3,584   1203 / 2706 against  112 /  249       N 16, T 17    2BD 14,336     47 /  116 against   89 /  181
+//                      8,960   1220 / 3036 against  232 /  572       N 16, T 64        14,336    159 /  378 against  118 /  245
+//                     14,336   1180 / 3068 against  357 /  894                         57,344    311 / 1037 against  394 /  914
+//                     57,344   2351 / 8399 against 1330 / 3408       N 64, T 256        8,192    633 / 2649 against  480 / 1424
+//   N 256, T 256       8,192   1841 / 12303 against 2594 / 10306                       24,576   1243 / 5548 against 1388 / 4161
 static bool m3_use_windows(const mxb_mamba3_desc* d) {
   if (d->flags & MXB_MAMBA3_SERIAL_WALK) return false;
   if ((d->T + kM3WinSteps - 1) / kM3WinSteps > 65535) return false;  // windows are a grid axis
