@@ -54,21 +54,22 @@ M3_FLOPS_PER_TOKEN = 5.50e6
 GDN_BLOCK_BYTES_PER_TOKEN_HEAD = 23 * 128 * 2 + 10 * 4
 # Mamba-3 block stages, fwd+bwd, bf16: conv 2 + 3, post 3 + 5 tensors of D channels; B/C norm 4 + 6 tensors of G*N
 M3_BLOCK_BYTES_PER_TOKEN = lambda D, GN: (13 * D + 10 * GN) * 2
-# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum, MB per launch at the full workload size) per kernel, from
-# one ncu byte capture of a step.  Keyed by kernel name: when the kernels a step launches are not exactly these, the
-# capture no longer describes the step and roofline.traffic is reported as null instead of a stale number.
-GDN_NCU_TRAFFIC_MB = {   # captured at B=6, T=2048; a larger step keeps a little less of the producer -> consumer tiles in L2
-    "gdn_tc_prep_kernel": 252.4, "gdn_tc_state_fwd_kernel": 378.9, "gdn_tc_state_bwd_kernel": 336.4,
-    "gdn_tc_chunk_bwd_kernel": 658.5,
+# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum, MB a step) per kernel, from one ncu byte capture of a step at
+# the workload's own size, caches as the step leaves them (profiles/launches_and_traffic.md).  Keyed by kernel name: when
+# the kernels a step launches are not exactly these, roofline.traffic is reported as null.  A kernel that is changed under
+# its old name, or takes over another's work, needs a new capture all the same.
+GDN_NCU_TRAFFIC_MB = {
+    "gdn_tc_prep_kernel": 781.4, "gdn_tc_state_fwd_kernel": 1141.1, "gdn_tc_state_bwd_kernel": 994.7,
+    "gdn_tc_chunk_bwd_kernel": 1812.2,
 }
-GDN_NCU_TRAFFIC_UNITS = 3072     # (batch, head, chunk) units of the captured step
+GDN_NCU_TRAFFIC_UNITS = 8192     # (batch, head, chunk) units of the captured step
 M3_NCU_TRAFFIC_MB = {
-    "m3s_scalars_kernel": 12.6, "m3s_chunk_scalars_kernel": 12.6, "m3s_state_pass_kernel": 390.3 + 390.4,
-    "m3s_chunk_out_kernel": 566.2, "m3s_chunk_grad_kernel": 1494.2, "m3s_tail_kernel": 33.6 + 548.0,
+    "m3s_scalars_kernel": 13.1, "m3s_chunk_scalars_kernel": 1.5, "m3s_state_pass_kernel": 841.3,
+    "m3s_chunk_out_kernel": 614.2, "m3s_chunk_grad_kernel": 1551.3, "m3s_tail_kernel": 643.9,
     "m3s_dalog_kernel": 0.0,
 }
 M3_NCU_TRAFFIC_UNITS = 16384
-DECODE_NCU_TRAFFIC_MB = {"gdn_decode_kernel": 483.7}
+DECODE_NCU_TRAFFIC_MB = {"gdn_decode_kernel": 535.3}
 DECODE_NCU_TRAFFIC_UNITS = 4096  # (sequence, head) tiles of the captured launch
 
 
