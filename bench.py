@@ -398,7 +398,7 @@ def build_mamba3_ref_shape(cx, batch):
                 alg_bytes=B * T * per_token, alg_flops=0.0, traffic=lambda kernels: None,
                 traffic_note="no byte capture for this workload (7 MB of tensors: it lives in L2)",
                 cfg={"workload": "mamba3_ref_shape", **w, "io": "f32", "layout": "per-channel dt/lambda/theta/a_log (the reference's)",
-                     "l2": "the whole problem fits L2; the step is bound by the T-long serial walk, not by HBM"})
+                     "l2": "the whole problem fits L2; the step is bound by the arithmetic and the launches of the window walks, not by HBM"})
 
 
 BUILDERS = {"mamba3_ref_shape": build_mamba3_ref_shape, "gdn_train": build_gdn_train, "gdn_decode": build_gdn_decode, "gdn_block": build_gdn_block,
