@@ -491,22 +491,36 @@ __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(GdnP p, const __grid_c
   }
   if (KP == 64) load_v(0);
   if (c == 0 && bh == 0 && tid >= 64 && tid < 128) p.status[tid - 64] = 0;
-  if (tid >= 32 && tid < 64) {  // inclusive cumulative sum of the log gate, two elements per lane
+  if (tid >= 32 && tid < 64) {
+    // Inclusive cumulative sum of the log gate, one step after the other: neighbouring sums then differ by a gate and ONE
+    // rounding, and it is differences of near sums that E(gam_i - gam_j) is large for.  (The rounding of these sums is the
+    // error of the whole scan.  Summed by a tree across the lanes it was 1.7 times as large; the chain of 64 additions runs
+    // beside the copies of k and q.)
     const int i0 = 2 * lane, i1 = i0 + 1;
-    const float g0 = i0 < imax ? log_gate(p.gate[row(i0)], p.gate_is_log) : 0.f;
-    const float g1 = i1 < imax ? log_gate(p.gate[row(i1)], p.gate_is_log) : 0.f;
     const float b0 = i0 < imax ? p.beta[row(i0)] : 0.f, b1 = i1 < imax ? p.beta[row(i1)] : 0.f;
-    float s = g0 + g1;
+    gam[i0] = i0 < imax ? log_gate(p.gate[row(i0)], p.gate_is_log) : 0.f;
+    gam[i1] = i1 < imax ? log_gate(p.gate[row(i1)], p.gate_is_log) : 0.f;
+    __syncwarp();
+    if (lane == 0) {
+      float4 g[R / 4];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float t = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= o) s += t;
+      for (int x = 0; x < R / 4; ++x) g[x] = *reinterpret_cast<const float4*>(gam + 4 * x);
+      float s = 0.f;
+#pragma unroll
+      for (int x = 0; x < R / 4; ++x) {
+        g[x].x = s += g[x].x;
+        g[x].y = s += g[x].y;
+        g[x].z = s += g[x].z;
+        g[x].w = s += g[x].w;
+        *reinterpret_cast<float4*>(gam + 4 * x) = g[x];
+      }
     }
-    gam[i0] = s - g1; gam[i1] = s;
+    __syncwarp();
+    const float c0 = gam[i0], c1 = gam[i1];
     bet[i0] = b0; bet[i1] = b1;
-    dd[i0] = exp_nonpos_precise(s - g1); dd[i1] = exp_nonpos_precise(s);
-    if (i0 < C) p.gam[ci * C + i0] = s - g1;
-    if (i1 < C) p.gam[ci * C + i1] = s;
+    dd[i0] = exp_nonpos_precise(c0); dd[i1] = exp_nonpos_precise(c1);
+    if (i0 < C) p.gam[ci * C + i0] = c0;
+    if (i1 < C) p.gam[ci * C + i1] = c1;
   }
   __syncthreads();
   bool ok = !tma || tc::mbar_wait(bar, 0);

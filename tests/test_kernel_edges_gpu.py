@@ -65,6 +65,28 @@ def test_float32_scan(shape, chunk, offset):
     _check_scan(*shape, F32, chunk, offset)
 
 
+@pytest.mark.parametrize("T,chunk", [(64, 64), (50, 64), (33, 33), (16, 16), (1, 64)])
+def test_float32_decay_matrix(T, chunk):
+    """Unit vectors for keys, their sum for every query, unit vectors for values, beta 1: the output of a chunk is
+    exp(G_i - G_j), G the float32 sums of the log gates taken one after the other (sums in another order are 1e-5 away).
+    What is left is expf: 2 ulp, and an ulp for the additions of zeros."""
+    B, H = 2, 8
+    eye = torch.eye(T, 64).expand(B, H, T, 64).transpose(1, 2)
+    q = torch.ones(B, T, H, 64)
+    gate = -torch.nn.functional.softplus(torch.randn(B, T, H, generator=torch.Generator().manual_seed(95)))
+    out = ops.gated_delta_scan(_dev(q), _dev(eye), _dev(eye), _dev(torch.ones(B, T, H)), _dev(gate), chunk, gate_is_log=True)
+    sums, acc = [], torch.zeros(B, H)
+    for t in range(T):
+        acc = acc + gate[:, t]
+        sums.append(acc)
+    G = torch.stack(sums, 1)                                     # [B,T,H]
+    diff = G[:, :, None] - G[:, None]                            # float32, [B,T,T,H]
+    assert float(diff.min()) > -80
+    want = torch.exp(diff.double()) * torch.tril(torch.ones(T, T))[None, :, :, None].double()
+    got = out.double().cpu()[..., :T].permute(0, 1, 3, 2)
+    assert float((got - want).abs().div(want.clamp_min(1e-30)).max()) <= 3 * 2 ** -23
+
+
 @pytest.mark.parametrize("shape", [
     (1, 1, 1, 128, 128), (1, 64, 2, 128, 96), (2, 129, 3, 96, 72), (1, 193, 2, 64, 128),   # split columns
     (2, 65, 37, 128, 128),             # the most heads that split
