@@ -998,12 +998,15 @@ __global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p, const __g
 //   Y = e (v beta)^T + z (k beta E(gam))^T             M = -tril(Y T^T, -1) Gamma,  Mb = beta_i M
 //   dk = r (v_new dS^T) + dPG^T q + (Mb + Mb^T) k + beta E(gam) z            dv = beta e
 //   dbeta = e.v + E(gam) (k.z) + sum_j M_ij (k_i.k_j)
-//   dgam_i = q_i.dq_i - k_i.dk_i + 2 beta_i (E(gam_i) (k_i.z_i) + sum_j M_ij (k_i.k_j)),
+//   dgam_i = q_i.(E(gam) dO S0^T)_i - k_i.(r v_new dS^T)_i + beta_i E(gam_i) (k_i.z_i)
+//            + the row sums minus the column sums of (dP P) and of (Mb k k^T), below the diagonal,
 //   dgam_last += L <dS,S0> + sum_i r_i k_i.(v_new dS^T)_i
-// (the row and column sums over Gamma of the P and A terms are the parts of q.dq and k.dk that come from dPG and Mb).
+// (The row and column sums are the parts of q.dq and k.dk that come from dPG and Mb, so q.dq - k.dk + 2 (..) needs no sums.
+// But it cancels what it need not form: the diagonal of dP P and twice the A terms.  Its dgate was 1.5 to 2.4 times as far
+// from a float64 scan, with nothing gained in time.)
 // Three 64 x 64 matrices live in shared memory, every wide operand is streamed; e and z make a round trip through the
-// workspace (L2).  105 KB: two CTAs per SM.
-constexpr int kChunkF32Smem = (simt::kStageFloats + 3 * simt::R * simt::LD + 9 * simt::R + 16) * 4;
+// workspace (L2).  106 KB: two CTAs per SM.
+constexpr int kChunkF32Smem = (simt::kStageFloats + 3 * simt::R * simt::LD + 10 * simt::R + 16) * 4;
 static_assert(2 * (kChunkF32Smem + 1024) <= 228 * 1024, "two CTAs per SM");
 
 template <typename IO, int NGK>
@@ -1023,7 +1026,8 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_bwd_kernel(GdnP p) {
   float* dbe = rs + R;   // dbeta
   float* dg = dbe + R;   // dgam
   float* rho = dg + R;   // k_i . dkp_i
-  float* red = rho + R;  // [8]
+  float* pw = rho + R;   // row sums minus column sums of dP P
+  float* red = pw + R;   // [8]
   const int C = p.C, K = p.K, V = p.V;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31, warp = tid >> 5;
   const int c = blockIdx.x, bh = blockIdx.y, b = bh / p.H, h = bh % p.H, t0 = c * C;
@@ -1102,18 +1106,45 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_bwd_kernel(GdnP p) {
       if (tx == 0) dbe[4 * ty + r] = vd[r];
     }
   }
-  // ---- dP Gamma ----
+  // Column sums of a 64 x 64 result held as rows ty + 16 r, columns tx + 16 x, each thread's four rows added already: the
+  // two rows of a warp, then the warps in order, by the first 64 threads.  In the streaming buffers, which are free.
+  auto col_sums = [&](const float (&v)[4]) {
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const float s = v[x] + __shfl_xor_sync(0xffffffffu, v[x], 16);
+      if (lane < 16) stage[warp * R + tx + 16 * x] = s;
+    }
+    __syncthreads();
+    float s = 0.f;
+    if (tid < R)
+      for (int w = 0; w < 8; ++w) s += stage[w * R + tid];
+    return s;
+  };
+  // ---- dP Gamma, and the sums of dP P ----
   {
     f2 acc[4][4];
     clear(acc);
     stream_nt(acc, stage, V, ldo, ldvn);
+    const float* P = p.P + ci * C * C;
+    float cs[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 4; ++r) {
+      const int i = ty + 16 * r;
+      float sum = 0.f;
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
-        const int i = ty + 16 * r, j = tx + 16 * x;
-        X1[i * LD + j] = (i >= j) ? sum2(acc[r][x]) * exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
+        const int j = tx + 16 * x;
+        const float dP = sum2(acc[r][x]);
+        X1[i * LD + j] = (i >= j) ? dP * exp_nonpos_precise(gam[i] - gam[j]) : 0.f;
+        const float w = (i > j && i < C) ? dP * P[i * C + j] : 0.f;
+        sum += w;
+        cs[x] += w;
       }
+      sum = row_sum(sum);
+      if (tx == 0) pw[i] = sum;
+    }
+    const float col = col_sums(cs);
+    if (tid < R) pw[tid] -= col;
   }
   // ---- dq = E(gam) dO S0^T + dPG k ----
   {
@@ -1125,22 +1156,20 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_bwd_kernel(GdnP p) {
       const f2 s = pack2(dd[4 * ty + r], dd[4 * ty + r]);
 #pragma unroll
       for (int x = 0; x < 2 * NGK; ++x) acc[r][x] = mul2(acc[r][x], s);
+      float qd = 0.f;
+#pragma unroll
+      for (int g = 0; g < NGK; ++g) qd = dot4(acc4<NGK>(acc, r, g), ldq(4 * ty + r, 64 * g + 4 * tx), qd);
+      qd = row_sum(qd);
+      if (tx == 0) dg[4 * ty + r] = qd;
     }
     stream_nn<NGK, 1>(acc, stage, R, X1, NoA{}, ldk);
     IO* dq = static_cast<IO*>(p.dq);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int i = 4 * ty + r;
-      float qd = 0.f;
 #pragma unroll
-      for (int g = 0; g < NGK; ++g) {
-        const int j = 64 * g + 4 * tx;
-        const float4 x = acc4<NGK>(acc, r, g);
-        qd = dot4(x, ldq(i, j), qd);
-        if (i < imax) st4(dq + row(i) * K, j, K, p.vecK, x);
-      }
-      qd = row_sum(qd);
-      if (tx == 0) dg[i] = qd;
+      for (int g = 0; g < NGK; ++g)
+        if (i < imax) st4(dq + row(i) * K, 64 * g + 4 * tx, K, p.vecK, acc4<NGK>(acc, r, g));
     }
   }
   // ---- z = -e S0^T, k.z ----
@@ -1162,7 +1191,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_bwd_kernel(GdnP p) {
       kz = row_sum(kz);
       if (tx == 0) {
         dbe[i] += dd[i] * kz;
-        dg[i] += 2.f * bd[i] * kz;
+        dg[i] += bd[i] * kz;
       }
     }
     __syncthreads();  // e and z are complete
@@ -1183,6 +1212,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_bwd_kernel(GdnP p) {
     clear(acc);
     tile_nt(acc, X2, LD, Tm, LD, R);
     __syncthreads();  // Y has been read
+    float cs[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int i = ty + 16 * r;
@@ -1191,8 +1221,9 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_bwd_kernel(GdnP p) {
       for (int x = 0; x < 4; ++x) {
         const int j = tx + 16 * x;
         if (i > j) {
-          const float M = -sum2(acc[r][x]) * exp_nonpos_precise(gam[i] - gam[j]);
-          sum = fmaf(M, sum2(kk[r][x]), sum);
+          const float M = -sum2(acc[r][x]) * exp_nonpos_precise(gam[i] - gam[j]), w = M * sum2(kk[r][x]);
+          sum += w;
+          cs[x] = fmaf(bet[i], w, cs[x]);
           X2[i * LD + j] = bet[i] * M;
           X2[j * LD + i] = bet[i] * M;
         } else if (i == j) {
@@ -1202,6 +1233,8 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_bwd_kernel(GdnP p) {
       sum = row_sum(sum);
       if (tx == 0) rs[i] = sum;
     }
+    const float col = col_sums(cs);
+    if (tid < R) pw[tid] -= col;
   }
   // ---- dk ----
   {
@@ -1228,19 +1261,16 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_bwd_kernel(GdnP p) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int i = 4 * ty + r;
-      float kd = 0.f;
 #pragma unroll
       for (int g = 0; g < NGK; ++g) {
         const int j = 64 * g + 4 * tx;
         const float4 a = acc4<NGK>(acc, r, g), zz = ldz(i, j);
         const float4 x = make_float4(fmaf(bd[i], zz.x, a.x), fmaf(bd[i], zz.y, a.y), fmaf(bd[i], zz.z, a.z), fmaf(bd[i], zz.w, a.w));
-        kd = dot4(x, ldk(i, j), kd);
         if (i < imax) st4(dk + row(i) * K, j, K, p.vecK, x);
       }
-      kd = row_sum(kd);
       if (tx == 0) {
         dbe[i] += rs[i];
-        dg[i] += 2.f * bet[i] * rs[i] - kd;
+        dg[i] += pw[i] + bet[i] * rs[i] - rho[i];
       }
     }
   }

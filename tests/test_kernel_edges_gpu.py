@@ -87,6 +87,28 @@ def test_float32_decay_matrix(T, chunk):
     assert float((got - want).abs().div(want.clamp_min(1e-30)).max()) <= 3 * 2 ** -23
 
 
+@pytest.mark.parametrize("log_gate", [True, False])
+@pytest.mark.parametrize("shape", [(2, 256, 4, 64, 64), (1, 300, 2, 128, 256), (2, 513, 3, 96, 200), (2, 70, 2, 16, 24)])
+def test_float32_scan_loses_no_more_than_plain_float32(shape, log_gate):
+    """Every result is as close to the float64 oracle as the same formulas in plain float32 are (a quarter more for sums in
+    another order)."""
+    a = inputs.gdn_inputs(*shape, seed=5, io_dtype=F32, with_grad_out=True, with_h0=True)
+    gate = a["g"] if log_gate else torch.exp(a["g"])
+
+    def oracle(dtype):
+        f = {n: t.to(dtype) for n, t in a.items()}
+        return gdn.scan_grads(f["q"], f["k"], f["v"], f["beta"], gate.to(dtype), f["d_out"], f["d_state"], f["h0"],
+                              gate_is_log=log_gate, chunk_size=64)
+
+    want, plain = oracle(torch.float64), oracle(F32)
+    args, kw = tuple(_dev(t) for t in (a["q"], a["k"], a["v"], a["beta"], gate)), dict(gate_is_log=log_gate, h0=_dev(a["h0"]))
+    got = ops.gated_delta_scan_backward(*args, _dev(a["d_out"]), 64, d_final_state=_dev(a["d_state"]), **kw)
+    got["out"], got["state"] = ops.gated_delta_scan(*args, 64, return_final_state=True, **kw)
+    off = lambda x, w: float((x.double().cpu() - w).norm() / w.norm())
+    for n in GRADS + ("out", "state"):
+        assert off(got[n], want[n]) <= 1.25 * off(plain[n], want[n]), n
+
+
 @pytest.mark.parametrize("shape", [
     (1, 1, 1, 128, 128), (1, 64, 2, 128, 96), (2, 129, 3, 96, 72), (1, 193, 2, 64, 128),   # split columns
     (2, 65, 37, 128, 128),             # the most heads that split
