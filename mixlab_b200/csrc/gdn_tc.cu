@@ -47,10 +47,6 @@ static_assert(4 * (kPrepSmem + 1024) <= 228 * 1024, "four CTAs per SM");
 
 using PrepMaps = RowMaps;
 
-__device__ __forceinline__ uint4 pack8f(const float* e) {
-  return make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]), tc::pack_bf16(e[4], e[5]),
-                    tc::pack_bf16(e[6], e[7]));
-}
 
 template <bool TMA>
 __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid_constant__ PrepMaps maps) {
@@ -248,11 +244,11 @@ __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
         const uint32_t off = tc::colblk_unit(ir, c8 + (c0 >> 3) + x, C);
-        sts16(Akq, 8192u + (off >> 13) * 16384u + (off & 8191u), pack8f(&f[8 * x]));
+        sts16(Akq, 8192u + (off >> 13) * 16384u + (off & 8191u), pack8(&f[8 * x]));
       }
       ld_acc32(taddr + 64, warp, c0, f);
 #pragma unroll
-      for (int x = 0; x < 4; ++x) sts16(Akq, kq_unit(ir, c8 + (c0 >> 3) + x), pack8f(&f[8 * x]));
+      for (int x = 0; x < 4; ++x) sts16(Akq, kq_unit(ir, c8 + (c0 >> 3) + x), pack8(&f[8 * x]));
     }
   } else if (tid == 0) {
     atomicExch(p.status, 1);

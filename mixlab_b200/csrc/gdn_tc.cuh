@@ -19,6 +19,8 @@ constexpr int C = 64;     // chunk
 constexpr int KD = 128;   // Dk = Dv
 constexpr int LDA = 68;   // fp32 row pitch of the 64x64 solve matrix (16-byte aligned rows)
 using bf16 = __nv_bfloat16;
+using tc::pack8;
+using tc::unpack8;
 
 struct TcP {
   int B, T, H, n, gate_is_log, save, no_tma;

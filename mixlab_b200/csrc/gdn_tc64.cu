@@ -24,13 +24,6 @@ namespace g64 {
 constexpr int W = 64;          // width of every tile
 constexpr int kTile = 8192;    // bytes of a [64][64] bf16 tile
 
-__device__ __forceinline__ uint4 pack8(const float* e) {
-  return make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]), tc::pack_bf16(e[4], e[5]), tc::pack_bf16(e[6], e[7]));
-}
-__device__ __forceinline__ void unpack8(uint4 v, float (&e)[8]) {
-  tc::unpack_bf16(v.x, e[0], e[1]); tc::unpack_bf16(v.y, e[2], e[3]);
-  tc::unpack_bf16(v.z, e[4], e[5]); tc::unpack_bf16(v.w, e[6], e[7]);
-}
 // byte offset of unit (r, c8) of a swizzled tile (one slab)
 __device__ __forceinline__ uint32_t sw_unit(int r, int c8) { return (uint32_t)r * 128u + (uint32_t)((c8 ^ (r & 7)) << 4); }
 

@@ -304,14 +304,6 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
 // the reverse state pass wrote last are read first.
 constexpr int kChunkBwdSmem = 3 * 16384 + 32768 + 3 * 8192 + 12 * C * 4 + 16 * 4 + 64 + 64 + 1024;
 
-__device__ __forceinline__ void unpack8(uint4 v, float (&e)[8]) {
-  tc::unpack_bf16(v.x, e[0], e[1]); tc::unpack_bf16(v.y, e[2], e[3]);
-  tc::unpack_bf16(v.z, e[4], e[5]); tc::unpack_bf16(v.w, e[6], e[7]);
-}
-__device__ __forceinline__ uint4 pack8(const float* e) {
-  return make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]), tc::pack_bf16(e[4], e[5]),
-                    tc::pack_bf16(e[6], e[7]));
-}
 __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);

@@ -35,6 +35,8 @@ constexpr int Q = 64;    // chunk
 constexpr int P = 64;    // head dim
 constexpr int N = 128;   // d_state
 using bf16 = __nv_bfloat16;
+using tc::pack8;
+using tc::unpack8;
 
 struct SsdP {
   int B, T, D, G, NH, n;   // n = chunks
@@ -56,14 +58,6 @@ struct SsdP {
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : (x < -20.f ? expf(x) : log1pf(expf(x))); }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + expf(-x)); }
 __device__ __forceinline__ void sts16(uint8_t* base, uint32_t off, uint4 v) { *reinterpret_cast<uint4*>(base + off) = v; }
-__device__ __forceinline__ void unpack8(uint4 v, float (&e)[8]) {
-  tc::unpack_bf16(v.x, e[0], e[1]); tc::unpack_bf16(v.y, e[2], e[3]);
-  tc::unpack_bf16(v.z, e[4], e[5]); tc::unpack_bf16(v.w, e[6], e[7]);
-}
-__device__ __forceinline__ uint4 pack8(const float* e) {
-  return make_uint4(tc::pack_bf16(e[0], e[1]), tc::pack_bf16(e[2], e[3]), tc::pack_bf16(e[4], e[5]),
-                    tc::pack_bf16(e[6], e[7]));
-}
 __device__ __forceinline__ void ld_acc32(uint32_t taddr, int warp, int c0, float (&f)[32]) {
   uint32_t r[32];
   tc::tmem_ld_32x32b_x32(taddr + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)c0, r);

@@ -102,6 +102,13 @@ __device__ __forceinline__ void unpack_bf16(uint32_t w, float& lo, float& hi) {
   lo = __low2float(v);
   hi = __high2float(v);
 }
+__device__ __forceinline__ uint4 pack8(const float* e) {
+  return make_uint4(pack_bf16(e[0], e[1]), pack_bf16(e[2], e[3]), pack_bf16(e[4], e[5]), pack_bf16(e[6], e[7]));
+}
+__device__ __forceinline__ void unpack8(uint4 v, float (&e)[8]) {
+  unpack_bf16(v.x, e[0], e[1]); unpack_bf16(v.y, e[2], e[3]);
+  unpack_bf16(v.z, e[4], e[5]); unpack_bf16(v.w, e[6], e[7]);
+}
 __device__ __forceinline__ uint4 scale_bf16x8(uint4 v, float s) {
   float a, b;
   uint4 r;
