@@ -59,13 +59,18 @@ void trace_begin(const char* name, cudaStream_t st) {
 void trace_end(cudaStream_t st) {
   if (!g_open_e0) return;
   cudaEvent_t e = nullptr;
+  bool kept = false;
   if (cudaEventCreate(&e) == cudaSuccess) {
     cudaEventRecord(e, st);
-    std::lock_guard<std::mutex> lk(g_trace_mu);
-    g_trace.push_back({g_open_name, g_open_e0, e});
-  } else {
-    cudaEventDestroy(g_open_e0);
+    try {  // (a record that finds no memory is dropped: no exception may leave the library)
+      std::lock_guard<std::mutex> lk(g_trace_mu);
+      g_trace.push_back({g_open_name, g_open_e0, e});
+      kept = true;
+    } catch (...) {
+      cudaEventDestroy(e);
+    }
   }
+  if (!kept) cudaEventDestroy(g_open_e0);
   g_open_e0 = nullptr;
 }
 static void trace_clear() {
@@ -172,7 +177,7 @@ void mxb_trace_enable(int on) {
   g_trace_on.store(on != 0);
 }
 
-size_t mxb_trace_summary(char* buf, size_t cap) {
+size_t mxb_trace_summary(char* buf, size_t cap) try {
   // one line per kernel name: "<name> <launches> <total_ms>\n"; waits for the recorded events.
   std::lock_guard<std::mutex> lk(g_trace_mu);
   std::vector<std::string> names;
@@ -200,6 +205,9 @@ size_t mxb_trace_summary(char* buf, size_t cap) {
     buf[n] = 0;
   }
   return out.size();
+} catch (...) {  // out of host memory
+  if (buf && cap > 0) buf[0] = 0;
+  return 0;
 }
 
 size_t mxb_gdn_fwd_workspace_bytes(const mxb_gdn_desc* d) {
@@ -755,14 +763,6 @@ static mxb_status host_gdn_pipeline(mxb_host_ctx* c, const mxb_gdn_desc* d, cons
   const int per = cut.per, nsplit = cut.nsplit, Hs = d->H / nsplit;
   // per-sequence element counts of a slice's tensors
   const size_t sk = (size_t)d->T * Hs * d->Dk, sv = (size_t)d->T * Hs * d->Dv;
-  struct Slice { int b0, nb, h0, hs; };
-  std::vector<Slice> slices;
-  if (nsplit > 1) {
-    for (int b0 = 0; b0 < d->B; ++b0)
-      for (int g = 0; g < nsplit; ++g) slices.push_back({b0, 1, g * Hs, Hs});
-  } else {
-    for (int b0 = 0; b0 < d->B; b0 += per) slices.push_back({b0, b0 + per <= d->B ? per : d->B - b0, 0, d->H});
-  }
   auto hp = [](const void* base, size_t off) { return static_cast<const char*>(base) + off; };
   auto hpw = [](void* base, size_t off) { return static_cast<char*>(base) + off; };
   const cudaMemcpyKind H2D = cudaMemcpyHostToDevice, D2H = cudaMemcpyDeviceToHost;
@@ -782,7 +782,9 @@ static mxb_status host_gdn_pipeline(mxb_host_ctx* c, const mxb_gdn_desc* d, cons
   MXB_CUDA_TRY(cudaEventRecord(c->bg_up, c->s_h2d));
   for (int bi = 0; bi < nslices; ++bi) {
     const int sl = bi % nslots;
-    const int b0 = slices[bi].b0, nb = slices[bi].nb, h0 = slices[bi].h0, hs = slices[bi].hs;
+    // sequences b0 .. b0 + nb - 1, heads h0 .. h0 + hs - 1
+    const int b0 = nsplit > 1 ? bi / nsplit : bi * per, nb = b0 + per <= d->B ? per : d->B - b0;
+    const int h0 = bi % nsplit * Hs, hs = Hs;
     const size_t ck = sk * nb * es, cvb = sv * nb * es;   // bytes of this slice (contiguous slices only)
     // element offsets of the slice's first row in the full tensors
     const size_t ok_ = ((size_t)b0 * d->T * d->H + h0) * d->Dk * es, ov_ = ((size_t)b0 * d->T * d->H + h0) * d->Dv * es;
