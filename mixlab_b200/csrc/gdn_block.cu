@@ -186,10 +186,10 @@ struct PreMap {
 };
 
 // ------------------------------------------------------------------ pre: forward
-// grid (head blocks, time tiles, streams x B)
+// grid (head blocks, time tiles, streams x B from z0 on)
 template <typename IO, int LPR>
-__global__ void __launch_bounds__(256) gdn_block_pre_fwd_kernel(BlockP p, PreArgs<IO> a, int run, int first) {
-  const int which = first + blockIdx.z / p.B, b = blockIdx.z % p.B;
+__global__ void __launch_bounds__(256) gdn_block_pre_fwd_kernel(BlockP p, PreArgs<IO> a, int run, int first, int z0) {
+  const int which = first + (z0 + blockIdx.z) / p.B, b = (z0 + blockIdx.z) % p.B;
   const int D = which == 2 ? p.Dv : p.Dk, C = p.H * D;
   const PreMap m = PreMap::make<LPR>(p.H, D, run);
   const IO* x = a.x[which] + (size_t)b * p.T * C + m.ch;
@@ -278,10 +278,10 @@ __global__ void __launch_bounds__(256) gdn_block_gate_fwd_kernel(BlockP p, const
 // 16 x 2048 x 16 heads of 64 bf16 channels, 189 now).  Two CTAs per SM leave a thread 128 registers, which its weights,
 // weight gradients, seven inputs and seven ds of four channels exceed: the compiler spills about 180 bytes of them.
 template <typename IO, int LPR>
-__global__ void __launch_bounds__(256, 2) gdn_block_pre_bwd_kernel(BlockP p, PreArgs<IO> a, int run, int first) {
+__global__ void __launch_bounds__(256, 2) gdn_block_pre_bwd_kernel(BlockP p, PreArgs<IO> a, int run, int first, int z0) {
   extern __shared__ __align__(16) uint8_t pre_smem[];
   __shared__ float red[kPreRuns][4][256];
-  const int which = first + blockIdx.z / p.B, b = blockIdx.z % p.B;
+  const int which = first + (z0 + blockIdx.z) / p.B, b = (z0 + blockIdx.z) % p.B;
   const int D = which == 2 ? p.Dv : p.Dk, C = p.H * D;
   const PreMap m = PreMap::make<LPR>(p.H, D, run);
   const IO* x = a.x[which] + (size_t)b * p.T * C + m.ch;
@@ -667,9 +667,13 @@ static int blk_lanes(int D, int per) {
   return l;
 }
 // Steps per run: 32 (a halo of three steps is recomputed per run in the backward) while that still gives two CTAs per
-// SM, shorter runs for smaller problems, where the length of the chain is what counts.
+// SM, shorter runs for smaller problems, where the length of the chain is what counts.  Longer ones where the tiles of a
+// sequence would not fit a grid axis.
 static int blk_run(const mxb_gdn_desc* d) {
   const int hk = 64 / blk_lanes(d->Dk, 4);
+  int longest = 32;
+  while (d->T / (4 * longest) >= 65535) longest *= 2;
+  if (longest > 32) return longest;
   for (int run = 32; run > 4; run /= 2)
     if ((size_t)3 * d->B * ((d->H + hk - 1) / hk) * ((d->T + 4 * run - 1) / (4 * run)) >= 2 * 148) return run;
   return 4;
@@ -708,13 +712,20 @@ static void with_lanes(int lanes, F&& call) {
     default: call(std::integral_constant<int, 32>{}); break;
   }
 }
-// The convolution kernels over q, k (streams 0, 1) and v (2): one launch where the lane counts agree, two otherwise.
+// The convolution kernels over q, k (streams 0, 1) and v (2): one launch where the lane counts agree, two otherwise, and
+// more where the sequences of all streams do not fit a grid axis.
+constexpr int kGridZ = 65535;
 template <typename F>
 static void blk_streams(const mxb_gdn_desc* d, F&& launch) {
   const int lk = blk_lanes(d->Dk, 4), lv = blk_lanes(d->Dv, 4), nt = blk_tiles(d);
-  auto grid = [&](int lanes, int streams) { return dim3((d->H + 64 / lanes - 1) / (64 / lanes), nt, streams * d->B); };
-  launch(lk, grid(lk, lk == lv ? 3 : 2), 0);
-  if (lk != lv) launch(lv, grid(lv, 1), 2);
+  auto over = [&](int lanes, int streams, int first) {
+    for (int z0 = 0; z0 < streams * d->B; z0 += kGridZ) {
+      const int nz = streams * d->B - z0 < kGridZ ? streams * d->B - z0 : kGridZ;
+      launch(lanes, dim3((d->H + 64 / lanes - 1) / (64 / lanes), nt, nz), first, z0);
+    }
+  };
+  over(lk, lk == lv ? 3 : 2, 0);
+  if (lk != lv) over(lv, 1, 2);
 }
 
 template <typename IO>
@@ -728,11 +739,11 @@ static mxb_status blk_pre_fwd(const mxb_gdn_desc* d, const void* qp, const void*
   a.w[0] = cq; a.w[1] = ck; a.w[2] = cv;
   a.y[0] = static_cast<IO*>(q); a.y[1] = static_cast<IO*>(k); a.y[2] = static_cast<IO*>(v);
   const int run = blk_run(d);
-  blk_streams(d, [&](int lanes, dim3 grid, int first) {
+  blk_streams(d, [&](int lanes, dim3 grid, int first, int z0) {
     with_lanes(lanes, [&](auto lpr) {
       constexpr int LPR = decltype(lpr)::value;
       if constexpr (LPR >= 4)
-        MXB_LAUNCH("gdn_block_pre_fwd_kernel", st, (blk::gdn_block_pre_fwd_kernel<IO, LPR><<<grid, 256, 0, st>>>(p, a, run, first)));
+        MXB_LAUNCH("gdn_block_pre_fwd_kernel", st, (blk::gdn_block_pre_fwd_kernel<IO, LPR><<<grid, 256, 0, st>>>(p, a, run, first, z0)));
     });
   });
   const size_t n = (size_t)d->B * d->T * d->H;
@@ -768,15 +779,15 @@ static mxb_status blk_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void*
   float* base = reinterpret_cast<float*>(static_cast<char*>(ws) + 256);
   a.dwp[0] = base; a.dwp[1] = base + rows * 4 * Ck; a.dwp[2] = base + rows * 8 * Ck;
   mxb_status s = MXB_OK;
-  blk_streams(d, [&](int lanes, dim3 grid, int first) {
+  blk_streams(d, [&](int lanes, dim3 grid, int first, int z0) {
     with_lanes(lanes, [&](auto lpr) {
       constexpr int LPR = decltype(lpr)::value;
-      if constexpr (LPR >= 4)
-        s = MXB_ALLOW_SMEM(blk::PreRing<IO>::kBytes, blk::gdn_block_pre_bwd_kernel<IO, LPR>);
-      if constexpr (LPR >= 4)
+      if constexpr (LPR >= 4) {
+        if (s == MXB_OK) s = MXB_ALLOW_SMEM(blk::PreRing<IO>::kBytes, blk::gdn_block_pre_bwd_kernel<IO, LPR>);
         if (s == MXB_OK)
           MXB_LAUNCH("gdn_block_pre_bwd_kernel", st,
-                     (blk::gdn_block_pre_bwd_kernel<IO, LPR><<<grid, 256, blk::PreRing<IO>::kBytes, st>>>(p, a, run, first)));
+                     (blk::gdn_block_pre_bwd_kernel<IO, LPR><<<grid, 256, blk::PreRing<IO>::kBytes, st>>>(p, a, run, first, z0)));
+      }
     });
   });
   if (s != MXB_OK) return s;

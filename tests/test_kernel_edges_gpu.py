@@ -143,6 +143,39 @@ def test_block_stages(cfg, io):
     blocks.test_block_post_forward_and_gradients((B, T, H, V), io)
 
 
+@pytest.mark.parametrize("B,T,H,K,V", [(21846, 2, 1, 8, 8), (65535, 1, 1, 8, 16), (70000, 1, 1, 8, 8), (1, 65535 * 128 + 1, 1, 8, 8)])
+def test_block_stages_beyond_a_grid_axis(B, T, H, K, V):
+    """More sequences than a grid axis holds for three streams, and a sequence of more tiles: the same bits as those
+    sequences (or that piece of the sequence) alone; the gradients of the weights against sums over the pieces."""
+    g = torch.Generator(device="cuda").manual_seed(96)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    seq = [rn(B, T, H * K).to(BF16), rn(B, T, H * K).to(BF16), rn(B, T, H * V).to(BF16)]
+    conv, gates, head = [0.4 * rn(4, H * K), 0.4 * rn(4, H * K), 0.4 * rn(4, H * V)], [rn(B, T, H), rn(B, T, H)], [rn(H), rn(H)]
+    grads = [rn(B, T, H, K).to(BF16), rn(B, T, H, K).to(BF16), rn(B, T, H, V).to(BF16), rn(B, T, H), rn(B, T, H)]
+    args = lambda cut: [cut(t) for t in seq] + conv + [cut(t) for t in gates] + head + [H, K, V]
+    whole = ops.gdn_block_pre(*args(lambda t: t), gate_is_log=True)
+    back = ops.gdn_block_pre_backward(*args(lambda t: t), *grads, gate_is_log=True)
+    if B > 1:
+        pieces = [lambda t: t[:100].contiguous(), lambda t: t[B - 100:].contiguous(), lambda t: t[B // 2:B // 2 + 100].contiguous()]
+        mid = slice(None)
+    else:  # the first steps of a piece lack the steps before it, the last ones the gradients behind it
+        pieces = [lambda t: t[:, T - 200:].contiguous(), lambda t: t[:, T // 2:T // 2 + 200].contiguous()]
+        mid = slice(3, -3)
+    for cut in pieces:
+        part = ops.gdn_block_pre(*args(cut), gate_is_log=True)
+        for x, y in zip(whole, part):
+            assert torch.equal(cut(x)[:, mid], y[:, mid])
+        pb = ops.gdn_block_pre_backward(*args(cut), *(cut(t) for t in grads), gate_is_log=True)
+        for n in ("dq_proj", "dk_proj", "dv_proj", "da_raw", "db_raw"):
+            assert torch.equal(cut(back[n])[:, mid], pb[n][:, mid]), n
+    assert all(bool(torch.isfinite(back[n]).all()) for n in ("dconv_q", "dconv_k", "dconv_v"))
+    if B > 1:  # halves of the batch add up
+        halves = [ops.gdn_block_pre_backward(*args(c), *(c(t) for t in grads), gate_is_log=True)
+                  for c in (lambda t: t[:B // 2].contiguous(), lambda t: t[B // 2:].contiguous())]
+        for n in ("dconv_q", "dconv_k", "dconv_v", "da_log", "ddt_bias"):
+            assert_close(back[n], halves[0][n].double() + halves[1][n].double(), 1e-4, n)
+
+
 @pytest.mark.parametrize("shape", [(1, 2, 4, 8, 1), (1, 7, 4, 16, 1), (2, 8, 8, 16, 2), (1, 9, 4, 32, 1),
                                    (1, 24, 4, 64, 1), (1, 17, 2, 256, 1), (1, 15, 4, 6, 1), (1, 41, 3, 128, 1)])
 def test_mamba3_windows(shape):
