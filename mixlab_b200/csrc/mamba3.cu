@@ -432,7 +432,6 @@ static int m3_channel_warps(const M3P& p) {
 //   N 256, T 256       8,192   1841 / 12303 against 2594 / 10306                       24,576   1243 / 5548 against 1388 / 4161
 static bool m3_use_windows(const mxb_mamba3_desc* d) {
   if (d->flags & MXB_MAMBA3_SERIAL_WALK) return false;
-  if ((d->T + kM3WinSteps - 1) / kM3WinSteps > 65535) return false;  // windows are a grid axis
   if (d->flags & MXB_MAMBA3_WINDOW_PARALLEL) return true;
   return (size_t)d->B * d->D * 2 <= (size_t)148 * 64 && d->T > kM3Window;
 }

@@ -23,6 +23,7 @@ struct M3P {
   float* hd;           // head-broadcast layout only: per-channel ddt, dlam, dtheta, 3 x [B,T,D]
   float* dal_part;     // per-batch (window-parallel: per batch and window) da_log: [.,D,N], or [.,D] head-broadcast
   // window-parallel kernels (mamba3_windows.cu)
+  int w0;              // first window of a launch
   int vec;             // rows of b, c, theta can be read two state pairs at a time
   float *dtv, *lamv;   // softplus(dt), sigmoid(lambda) in the layout of dt, lambda
   float* dtsum;        // [B,nW,D] sum of dt over the window

@@ -111,7 +111,7 @@ struct Walker {
   float* rows;  // [kRows][2 (even, odd)][NP]
   __device__ Walker(const M3P& p_, float* rows_)
       : p(p_), ix(p_), lane(threadIdx.x & 31), sl(lane % LPC), wc((threadIdx.x >> 5) * CPW + lane / LPC),
-        d(blockIdx.x * ((blockDim.x >> 5) * CPW) + wc), b(blockIdx.z), w(blockIdx.y), ts(w * W), base(lane / LPC * LPC),
+        d(blockIdx.x * ((blockDim.x >> 5) * CPW) + wc), b(blockIdx.z), w(p_.w0 + blockIdx.y), ts(w * W), base(lane / LPC * LPC),
         row0((size_t)b * p_.T + ts), rows(rows_) {}
   __device__ bool act(int r) const { return sl * PR + r < p.Kp; }
   __device__ bool in(int s) const { return ts + s < p.T; }
@@ -808,14 +808,17 @@ M3WinShape m3w_shape(const M3P& p) {
 
 struct M3WGrid {
   M3WinShape shape;
-  dim3 walk;
   int threads;
 };
 static M3WGrid m3w_grid(const M3P& p) {
-  M3WGrid g{m3w_shape(p), {}, 0};
-  g.threads = 32 * g.shape.warps;
-  g.walk = dim3((p.D + g.shape.warps * (32 / g.shape.lanes) - 1) / (g.shape.warps * (32 / g.shape.lanes)), p.nW, p.B);
-  return g;
+  const M3WinShape s = m3w_shape(p);
+  return {s, 32 * s.warps};
+}
+// A walk over every window: launch(parameters, grid), once per 65535 windows (a grid axis).
+template <typename F>
+static void m3w_walk(const M3P& p, const M3WGrid& g, F&& launch) {
+  const int channels = g.shape.warps * (32 / g.shape.lanes);
+  for (M3P q = p; q.w0 < p.nW; q.w0 += 65535) launch(q, dim3((p.D + channels - 1) / channels, std::min(65535, p.nW - q.w0), p.B));
 }
 static dim3 chain_grid(const M3P& p, int chains, int kinds) { return dim3((chains + 31) / 32, p.B, kinds); }
 
@@ -824,7 +827,9 @@ static mxb_status launch_local(const M3P& p, const M3WGrid& g, cudaStream_t st) 
   constexpr int per_thread = DH ? W * 2 * PR * 8 : 0, rows = kRowBytes<IO, PR, LPC>;
   const int sm = per_thread * g.threads + rows;
   if (MXB_ALLOW_SMEM(per_thread * (PR == 4 ? 128 : 256) + rows, m3w_local_kernel<IO, PR, LPC, FWD, DH>) != MXB_OK) return MXB_ERR_CUDA;
-  MXB_LAUNCH("m3w_local_kernel", st, (m3w_local_kernel<IO, PR, LPC, FWD, DH><<<g.walk, g.threads, sm, st>>>(p)));
+  m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
+    MXB_LAUNCH("m3w_local_kernel", st, (m3w_local_kernel<IO, PR, LPC, FWD, DH><<<grid, g.threads, sm, st>>>(q)));
+  });
   return MXB_OK;
 }
 template <typename IO, int PR, int LPC>
@@ -832,12 +837,16 @@ static mxb_status launch_grad(const M3P& p, const M3WGrid& g, cudaStream_t st) {
   constexpr int per_warp = 32 * GradSmem<PR, LPC>::kThread + GradSmem<PR, LPC>::kWarp, rows = kRowBytes<IO, PR, LPC>;
   if (MXB_ALLOW_SMEM((PR == 4 ? 4 : 8) * per_warp + rows, m3w_grad_kernel<IO, PR, LPC>) != MXB_OK) return MXB_ERR_CUDA;
   const int sm = g.shape.warps * per_warp + rows;
-  MXB_LAUNCH("m3w_grad_kernel", st, (m3w_grad_kernel<IO, PR, LPC><<<g.walk, g.threads, sm, st>>>(p)));
+  m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
+    MXB_LAUNCH("m3w_grad_kernel", st, (m3w_grad_kernel<IO, PR, LPC><<<grid, g.threads, sm, st>>>(q)));
+  });
   return MXB_OK;
 }
 template <typename IO>
 static mxb_status prepare(const M3P& p, const M3WGrid& g, cudaStream_t st) {
-  M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_prepare_kernel", st, (m3w_prepare_kernel<IO, PRV, LPCV><<<g.walk, g.threads, 0, st>>>(p))));
+  m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
+    M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_prepare_kernel", st, (m3w_prepare_kernel<IO, PRV, LPCV><<<grid, g.threads, 0, st>>>(q))));
+  });
   MXB_LAUNCH("m3w_phase_scan_kernel", st, (m3w_phase_scan_kernel<<<chain_grid(p, p.D * p.Kp, 1), 32 * kSegs, 0, st>>>(p)));
   return check_launch("mamba3 window preparation");
 }
@@ -850,7 +859,9 @@ static mxb_status forward(const M3P& p, cudaStream_t st) {
   M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_local<IO, PRV, LPCV, true, false>(p, g, st)));
   if (s != MXB_OK) return s;
   MXB_LAUNCH("m3w_linear_scan_kernel", st, (m3w_linear_scan_kernel<<<chain_grid(p, p.D * p.N, 1), 32 * kSegs, 0, st>>>(p, 0)));
-  M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_out_kernel", st, (m3w_out_kernel<IO, PRV, LPCV><<<g.walk, g.threads, kRowBytes<IO, PRV, LPCV>, st>>>(p))));
+  m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
+    M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_out_kernel", st, (m3w_out_kernel<IO, PRV, LPCV><<<grid, g.threads, kRowBytes<IO, PRV, LPCV>, st>>>(q))));
+  });
   return check_launch("mamba3 window-parallel forward");
 }
 // have_states: angles and states at the window starts (and dtv, lamv) are those a forward on the same inputs left.
@@ -871,7 +882,9 @@ static mxb_status backward(const M3P& p, bool have_states, cudaStream_t st) {
   M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_grad<IO, PRV, LPCV>(p, g, st)));
   if (s != MXB_OK) return s;
   MXB_LAUNCH("m3w_angle_scan_kernel", st, (m3w_angle_scan_kernel<<<chain_grid(p, p.D * p.Kp, 1), 32 * kSegs, 0, st>>>(p)));
-  M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_fix_kernel", st, (m3w_fix_kernel<IO, PRV, LPCV><<<g.walk, g.threads, 0, st>>>(p))));
+  m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
+    M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_fix_kernel", st, (m3w_fix_kernel<IO, PRV, LPCV><<<grid, g.threads, 0, st>>>(q))));
+  });
   return check_launch("mamba3 window-parallel backward");
 }
 

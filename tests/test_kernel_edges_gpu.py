@@ -192,6 +192,24 @@ def test_mamba3_windows(shape):
         assert torch.equal(got[n], want[n]), n
 
 
+def test_mamba3_windows_beyond_a_grid_axis():
+    """More windows than a grid axis holds, against the serial walk.  Angles turn in the last thousand steps only: over half a
+    million the two forms would round them apart.  da_log adds 5e5 terms, in the serial walk one after the other in
+    float32 (a random walk of 4e-5, more where they lean one way): 1e-3."""
+    B, T, D, N, G = 1, 65535 * 8 + 9, 4, 4, 1
+    a = inputs.mamba3_inputs(B, T, D, 1, N, G=G, seed=97, per_head=False)
+    a["theta"][:, :T - 1000] = 0
+    dev, dy = [_dev(a[n]) for n in mamba.ARGS], _dev(a["dy"])
+    serial, default = dict(flags=_lib.MXB_MAMBA3_SERIAL_WALK), {}
+    n0 = mixlab_b200.lib().mxb_launch_count()
+    y = ops.mamba3_selective_scan(*dev, **default)
+    assert mixlab_b200.lib().mxb_launch_count() - n0 > 1      # the windows, not the walk of one launch
+    assert_close(y, ops.mamba3_selective_scan(*dev, **serial).double(), 1e-5, "y")
+    got, want = (ops.mamba3_selective_scan_backward(*dev, dy, **kw) for kw in (default, serial))
+    for n in mamba.GRADS:
+        assert_close(got[n], want[n].double(), 1e-3 if n == "da_log" else 1e-4, n)
+
+
 @pytest.mark.parametrize("cfg", [(1, 63, 1, 1), (2, 65, 3, 3), (1, 129, 2, 2)])
 def test_mamba3_chunks(cfg):
     """Chunks of 64 steps, one short, one over; one head per group."""
