@@ -55,7 +55,7 @@ GDN_BLOCK_BYTES_PER_TOKEN_HEAD = 23 * 128 * 2 + 10 * 4
 # Mamba-3 block stages, fwd+bwd, bf16: conv 2 + 3, post 3 + 5 tensors of D channels; B/C norm 4 + 6 tensors of G*N
 M3_BLOCK_BYTES_PER_TOKEN = lambda D, GN: (13 * D + 10 * GN) * 2
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum, MB a step) per kernel, from one ncu byte capture of a step at
-# the workload's own size, caches as the step leaves them (profiles/launches_and_traffic.md).  Keyed by kernel name: when
+# the workload's own size, caches as the step leaves them.  Keyed by kernel name: when
 # the kernels a step launches are not exactly these, roofline.traffic is reported as null.  A kernel that is changed under
 # its old name, or takes over another's work, needs a new capture all the same.
 GDN_NCU_TRAFFIC_MB = {

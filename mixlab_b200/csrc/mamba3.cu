@@ -595,7 +595,9 @@ mxb_status mamba3_bwd(const mxb_mamba3_desc* d, const void* x, const float* dt, 
   }
   // warp-per-channel kernels: checkpoints (no y), reverse pass, fixed-order sums of the partials
   if (windows) {
-    s = m3w_backward(p, f32, (d->flags & MXB_MAMBA3_BWD_USE_SAVED) != 0, st);
+    // Only a forward that ran as windows has left their states: heads of 8 channels take the CTA-per-head kernel forward.
+    const bool head_fwd = !(d->flags & MXB_MAMBA3_CHANNEL_KERNELS) && mamba3_head_supported(d);
+    s = m3w_backward(p, f32, (d->flags & MXB_MAMBA3_BWD_USE_SAVED) && !head_fwd, st);
   } else {
     s = f32 ? m3_fwd_serial<float>(p, st) : m3_fwd_serial<__nv_bfloat16>(p, st);
     if (s != MXB_OK) return s;

@@ -260,6 +260,21 @@ def test_window_parallel_matches_serial_walk(shape):
         assert_close(gw[name], gs[name].double(), 1e-5, name)
 
 
+@pytest.mark.parametrize("P,N", [(8, 64), (8, 128), (16, 64), (64, 64), (8, 16)])
+@pytest.mark.parametrize("io", [torch.float32, torch.bfloat16])
+def test_saved_forward_of_every_head_width(P, N, io):
+    """A backward from the saved forward gives the bits of one with its own recompute, whichever families the forward and the
+    backward of a head width belong to: the workspace held something else before."""
+    a = inputs.mamba3_inputs(1, 130, 2, P, N, G=1, seed=23, io_dtype=io, per_head=True)
+    dev, dy, kw = [_dev(a[k]) for k in ARGS], _dev(a["dy"]), dict(nheads=2)
+    want = {n: t.clone() for n, t in ops.mamba3_selective_scan_backward(*dev, dy, **kw).items()}
+    ops.workspace(1 << 24, torch.device(DEV)).fill_(0xA5)
+    ops.mamba3_selective_scan(*dev, save_for_backward=True, **kw)
+    got = ops.mamba3_selective_scan_backward(*dev, dy, use_saved=True, **kw)
+    for n in GRADS:
+        assert torch.equal(got[n], want[n]), n
+
+
 @pytest.mark.parametrize("n", [1, 2, 513, 1 << 24])
 def test_sines_and_cosines_of_the_window_kernels(n):
     """Against double precision.  The bound is that of the method, two roundings of the reduced angle (6e-8) and the last
