@@ -768,8 +768,11 @@ mxb_status gdn_tc_fwd(const mxb_gdn_desc* d, const void* q, const void* k, const
 mxb_status gdn_tc_bwd(const mxb_gdn_desc* d, const void* q, const void* k, const void* v, const float* beta,
                       const float* gate, const float* h0, const void* dO, const float* dhT, void* dq, void* dk,
                       void* dv, float* dbeta, float* dgate, float* dh0, void* ws, cudaStream_t st) {
-  if (d->flags & MXB_GDN_BWD_FP32_KERNELS)
-    return gdn_simt_bwd(d, q, k, v, beta, gate, h0, dO, dhT, dq, dk, dv, dbeta, dgate, dh0, ws, st);
+  if (d->flags & MXB_GDN_BWD_FP32_KERNELS) {  // what a forward saved is in these kernels' layout: the others recompute
+    mxb_gdn_desc own = *d;
+    own.flags &= ~MXB_GDN_BWD_USE_SAVED;
+    return gdn_simt_bwd(&own, q, k, v, beta, gate, h0, dO, dhT, dq, dk, dv, dbeta, dgate, dh0, ws, st);
+  }
   TcP p = make_tc(d);
   p.q = static_cast<const bf16*>(q); p.k = static_cast<const bf16*>(k); p.v = static_cast<const bf16*>(v);
   p.beta = beta; p.gate = gate; p.h0 = h0;

@@ -308,6 +308,20 @@ def test_backward_from_saved_forward(case):
         assert torch.equal(got[name], ref[name]), name
 
 
+@pytest.mark.parametrize("io,flags", [(torch.bfloat16, 0), (torch.float32, 64)])
+@pytest.mark.parametrize("K", [64, 128])
+def test_float32_backward_behind_a_saved_tensor_core_forward(K, io, flags):
+    """MXB_GDN_BWD_FP32_KERNELS after a forward that saved in the tensor-core kernels' layout: recomputed, the same bits as
+    without the saved forward."""
+    a = inputs.gdn_inputs(2, 130, 2, K, K, seed=33, io_dtype=io, with_grad_out=True)
+    args, kw = tuple(_dev(a[n]) for n in ("q", "k", "v", "beta", "g")), dict(gate_is_log=True, flags=flags | 2)
+    want = {n: t.clone() for n, t in ops.gated_delta_scan_backward(*args, _dev(a["d_out"]), 64, **kw).items() if t is not None}
+    ops.gated_delta_scan(*args, 64, save_for_backward=True, **kw)
+    got = ops.gated_delta_scan_backward(*args, _dev(a["d_out"]), 64, use_saved=True, **kw)
+    for n, t in want.items():
+        assert torch.equal(got[n], t), n
+
+
 @pytest.mark.parametrize("dims", [(40, 16, 128, 128, torch.bfloat16), (10, 3, 64, 128, torch.float32),
                                   (150, 4, 128, 128, torch.float32)])
 def test_decode_steps_on_many_states(dims):
