@@ -11,6 +11,7 @@
 #include <dlfcn.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -461,7 +462,9 @@ Tensor mamba3_forward(const Tensor& x, const Tensor& dt, const Tensor& lam, cons
   mxb_status s;
   {
     Lease ws(on);
-    ws.take(abi.mxb_mamba3_fwd_workspace_bytes(&d));
+    // (a forward that saves nothing needs little or no scratch, but the backward that may follow finds its buffer here)
+    const size_t fwd = abi.mxb_mamba3_fwd_workspace_bytes(&d), bwd = save ? abi.mxb_mamba3_bwd_workspace_bytes(&d) : 0;
+    ws.take(std::max(fwd, bwd));
     s = run(abi.mxb_mamba3_fwd, &d, ptr(x), ptr<float>(dt), ptr<float>(lam), ptr<float>(theta), ptr<float>(a_log), ptr(b), ptr(c),
             ptr(y), ws.data(), ws.bytes(), on.stream);
     if (save && s == MXB_OK) ws.save(mamba3_token(d, x, dt, lam, theta, a_log, b, c));

@@ -4,7 +4,7 @@ import threading
 import pytest
 import torch
 
-from mixlab_b200 import ops
+from mixlab_b200 import _lib, ops
 from oracle import inputs
 
 pytestmark = pytest.mark.gpu
@@ -94,6 +94,24 @@ def test_streams_beyond_the_kept_ones():
     torch.cuda.synchronize()
     for n, w in zip(("dq", "dk", "dv", "dbeta", "dgate"), want[1:]):
         assert torch.equal(g[n], w), n
+
+
+@pytest.mark.parametrize("flags,nheads", [(_lib.MXB_MAMBA3_SERIAL_WALK, 0), (_lib.MXB_MAMBA3_WINDOW_PARALLEL, 0),
+                                          (_lib.MXB_MAMBA3_RECURRENT_KERNELS, 2), (0, 2)])
+def test_saved_mamba3_forward_on_a_new_stream(flags, nheads):
+    """A stream whose buffer nobody has used: the backward of a saving forward finds room, also where that kernel family
+    saves nothing and recomputes."""
+    a = inputs.mamba3_inputs(1, 130, 2, 64, 128, G=1, seed=24, io_dtype=torch.bfloat16, per_head=nheads > 0)
+    args = [a[n].cuda().contiguous() for n in ("x", "dt_raw", "lambda_raw", "theta", "a_log", "b", "c")]
+    dy, kw = a["dy"].cuda().contiguous(), dict(flags=flags, nheads=nheads)
+    want = {n: t.clone() for n, t in ops.mamba3_selective_scan_backward(*args, dy, **kw).items()}
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream(priority=-1)):
+        ops.mamba3_selective_scan(*args, save_for_backward=True, **kw)
+        got = ops.mamba3_selective_scan_backward(*args, dy, use_saved=True, **kw)
+    torch.cuda.synchronize()
+    for n, t in want.items():
+        assert torch.equal(got[n], t), n
 
 
 def _capture(stream, args, d_out):
