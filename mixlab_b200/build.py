@@ -19,7 +19,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libmixlab_b200.so")
 FRONT = os.path.join(PKG, "_front.so")
-SOURCES = ["capi.cu", "dp_grad.cu", "gdn_block.cu", "gdn_decode.cu", "gdn_f32io.cu", "gdn_simt.cu", "gdn_static_scratch.cu", "gdn_tc.cu", "gdn_tc64.cu", "gdn_tc_bwd.cu", "mamba3.cu", "mamba3_block.cu", "mamba3_head.cu", "mamba3_ssd.cu", "mamba3_windows.cu", "umma_selftest.cu"]
+SOURCES = ["capi.cu", "dp_grad.cu", "gdn_block.cu", "gdn_chain.cu", "gdn_decode.cu", "gdn_f32io.cu", "gdn_simt.cu", "gdn_static_scratch.cu", "gdn_tc.cu", "gdn_tc64.cu", "gdn_tc_bwd.cu", "mamba3.cu", "mamba3_block.cu", "mamba3_head.cu", "mamba3_ssd.cu", "mamba3_windows.cu", "umma_selftest.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "--std=c++17",
     "--extended-lambda", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",

@@ -681,6 +681,8 @@ size_t gdn_tc_workspace_bytes(const mxb_gdn_desc* d, bool bwd) {
 
 mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st);
 mxb_status tc64_run_fwd(TcP& p, cudaStream_t st);
+int chain_columns(const TcP& p, bool whole);
+mxb_status chain_fwd(const TcP& p, const RowMaps& maps, int nv, cudaStream_t st);
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -700,19 +702,26 @@ static EncodeTiledFn encode_tiled_fn() {
 // [B,T,H,D] bf16 as a 4-d tensor (D, H, T, B) with boxes of 64 columns x 64 time steps, 128-byte swizzle
 // (D a multiple of 8: rows are 16-byte multiples; columns past D and rows past T are zero-filled by the copy engine
 // on loads and clipped on stores); float32 tensors: boxes of 32 columns.  Shared with the other kernels.
-static bool make_tma_map(CUtensorMap* m, CUtensorMapDataType type, int size, const void* base, int B, int T, int H, int D) {
+static bool make_tma_map(CUtensorMap* m, CUtensorMapDataType type, int size, const void* base, int B, int T, int H, int D, int cols = 0) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn || (reinterpret_cast<uintptr_t>(base) & 15) || D * size % 16 || D <= 0) return false;
   const cuuint64_t row = (cuuint64_t)D * size;
   const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)H, (cuuint64_t)T, (cuuint64_t)B};
   const cuuint64_t strides[3] = {row, H * row, T * (H * row)};
-  const cuuint32_t box[4] = {128u / size, 1, 64, 1}, estr[4] = {1, 1, 1, 1};
+  const cuuint32_t box[4] = {cols ? (cuuint32_t)cols : 128u / size, 1, 64, 1}, estr[4] = {1, 1, 1, 1};
+  const CUtensorMapSwizzle swizzle = box[0] * size == 128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                                     : box[0] * size == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                           : CU_TENSOR_MAP_SWIZZLE_32B;
   return fn(m, type, 4, const_cast<void*>(base), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 bool make_tma_map_bthd(CUtensorMap* m, const void* base, int B, int T, int H, int D) {
   return make_tma_map(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, B, T, H, D);
+}
+// Boxes of 16, 32 or 64 columns, swizzled over their own width.
+bool make_tma_map_cols(CUtensorMap* m, const void* base, int B, int T, int H, int D, int cols) {
+  return make_tma_map(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, B, T, H, D, cols);
 }
 bool make_tma_map_f32(CUtensorMap* m, const void* base, int B, int T, int H, int D) {
   return make_tma_map(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, B, T, H, D);
@@ -747,6 +756,7 @@ mxb_status tc_run_fwd(TcP& p, cudaStream_t st) {
                (gdn_tc_state_fwd_kernel<TMA, NV><<<dim3(p.B * p.H, (p.Dv + NV - 1) / NV), kStateThreads<NV>, kStateFwdSmem<NV>, st>>>(p, maps)));
     return MXB_OK;
   };
+  if (tma && chain_columns(p, p.save)) return chain_fwd(p, maps, chain_columns(p, p.save), st);
   if (!tma) s = state(std::false_type{}, std::integral_constant<int, KD>{});
   else if (tc_split_columns(p)) s = state(std::true_type{}, std::integral_constant<int, 64>{});
   else s = state(std::true_type{}, std::integral_constant<int, KD>{});

@@ -886,6 +886,9 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
 }  // namespace g64
 
 // ------------------------------------------------------------------ host
+int chain_columns(const TcP& p, bool whole);
+mxb_status chain_fwd(const TcP& p, const RowMaps& maps, int nv, cudaStream_t st);
+mxb_status chain_bwd(const TcP& p, const RowMaps& maps, int nv, cudaStream_t st);
 mxb_status tc64_run_fwd(TcP& p, cudaStream_t st) {
   RowMaps maps;
   std::memset(&maps, 0, sizeof maps);
@@ -897,6 +900,7 @@ mxb_status tc64_run_fwd(TcP& p, cudaStream_t st) {
     return MXB_ERR_CUDA;
   MXB_LAUNCH("gdn_tc_prep_kernel", st,
              (g64::gdn_tc_prep_kernel<<<dim3(p.n, p.B * p.H), 128, g64::kPrepSmem, st>>>(p, maps)));
+  if (const int nv = chain_columns(p, p.save)) return chain_fwd(p, maps, nv, st);
   MXB_LAUNCH("gdn_tc_state_fwd_kernel", st,
              (g64::gdn_tc_state_fwd_kernel<<<p.B * p.H, 256, g64::kStateFwdSmem, st>>>(p, maps)));
   return check_launch("gdn_tc64 forward");
@@ -913,8 +917,13 @@ mxb_status tc64_run_bwd(const TcP& p, cudaStream_t st) {
   if (MXB_ALLOW_SMEM(g64::kStateBwdSmem, g64::gdn_tc_state_bwd_kernel) != MXB_OK ||
       MXB_ALLOW_SMEM(g64::kChunkSmem, g64::gdn_tc_chunk_bwd_kernel) != MXB_OK)
     return MXB_ERR_CUDA;
-  MXB_LAUNCH("gdn_tc_state_bwd_kernel", st,
-             (g64::gdn_tc_state_bwd_kernel<<<p.B * p.H, 256, g64::kStateBwdSmem, st>>>(p, maps)));
+  if (const int nv = chain_columns(p, true)) {
+    const mxb_status s = chain_bwd(p, maps, nv, st);
+    if (s != MXB_OK) return s;
+  } else {
+    MXB_LAUNCH("gdn_tc_state_bwd_kernel", st,
+               (g64::gdn_tc_state_bwd_kernel<<<p.B * p.H, 256, g64::kStateBwdSmem, st>>>(p, maps)));
+  }
   MXB_LAUNCH("gdn_tc_chunk_bwd_kernel", st,
              (g64::gdn_tc_chunk_bwd_kernel<<<dim3(p.B * p.H, p.n), 256, g64::kChunkSmem, st>>>(p, maps)));
   return check_launch("gdn_tc64 backward");

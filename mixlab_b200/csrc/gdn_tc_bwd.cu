@@ -688,6 +688,8 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
 // ------------------------------------------------------------------ host
 mxb_status tc_run_fwd(TcP& p, cudaStream_t st);
 mxb_status tc64_run_bwd(const TcP& p, cudaStream_t st);
+int chain_columns(const TcP& p, bool whole);
+mxb_status chain_bwd(const TcP& p, const RowMaps& maps, int nv, cudaStream_t st);
 
 // Forward recompute (saving per-chunk states and v_new), reverse state pass, per-chunk pass.
 mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st) {
@@ -719,7 +721,8 @@ mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st) {
                (gdn_tc_state_bwd_kernel<TMA, NV><<<dim3(p.B * p.H, (p.Dv + NV - 1) / NV), 256, kStateBwdSmem<NV>, st>>>(p, maps)));
     return MXB_OK;
   };
-  if (!tma) s = state(std::false_type{}, std::integral_constant<int, KD>{});
+  if (tma && chain_columns(p, true)) s = chain_bwd(p, maps, chain_columns(p, true), st);
+  else if (!tma) s = state(std::false_type{}, std::integral_constant<int, KD>{});
   else if (tc_split_columns(p)) s = state(std::true_type{}, std::integral_constant<int, 64>{});
   else s = state(std::true_type{}, std::integral_constant<int, KD>{});
   if (s != MXB_OK) return s;

@@ -240,3 +240,33 @@ def test_host_slicing(B, T, H, arena_mb):
         lib.mxb_host_ctx_destroy(ctx)
     for n, t in res.items():
         assert torch.equal(t, want[n].cpu()), n
+
+
+@pytest.mark.parametrize("T,K,V,batches", [
+    (150, 128, 128, (2, 8, 18)),   # of 4 heads: 16 and 32 columns of the state per CTA, the tcgen05 pass of 64 columns
+    (64, 128, 72, (3, 9)),         # one whole chunk, columns past the values' width
+    (449, 72, 128, (1, 9)),        # more chunks than buffers, rows past the keys' width
+    (130, 64, 64, (9, 18)),        # heads of 64 columns: 16 and 32 columns per CTA
+])
+def test_gdn_state_passes_agree_bit_for_bit(T, K, V, batches):
+    """Sequences of a batch that fills the GPU (tcgen05 state passes) and the first few of them alone (mma.sync passes of
+    16 and 32 columns): the same roundings and the same order of sums, so the same bits.  The oracle pins either route."""
+    a = inputs.gdn_inputs(40, T, 4, K, V, seed=17, io_dtype=BF16, with_grad_out=True, with_h0=True)
+    d = {n: _dev(t) for n, t in a.items()}
+
+    def run(nb):
+        x = {n: t[:nb] for n, t in d.items()}
+        args = tuple(x[n] for n in ("q", "k", "v", "beta", "g"))
+        kw = dict(gate_is_log=True, h0=x["h0"])
+        o, s = ops.gated_delta_scan(*args, 64, return_final_state=True, **kw)
+        saved = ops.gated_delta_scan(*args, 64, save_for_backward=True, **kw)
+        g = ops.gated_delta_scan_backward(*args, x["d_out"], 64, d_final_state=x["d_state"], use_saved=True, **kw)
+        torch.cuda.synchronize()
+        assert ops.device_status() == 0 and torch.equal(o, saved)
+        return dict(out=o, state=s, **g)
+
+    whole = run(40)
+    for nb in batches:
+        part = run(nb)
+        for n in whole:
+            assert torch.equal(whole[n][:nb], part[n]), (nb, n)
