@@ -45,10 +45,10 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Sums of 16 columns over the 16 lanes of each half of a warp: v[c] is this lane's value for column c.  Recursive halving,
-// 15 shuffles instead of 16 x 4.  On return lane l holds in v[0] the sum of column l & 15 over its half.
+// Sums of 8 columns over the 32 lanes of a warp: v[c] is this lane's value for column c.  Recursive halving, 9 shuffles
+// instead of 40.  On return lane l holds in v[0] the sum of column l & 7.
 template <int M, int N>
-__device__ __forceinline__ void colsum16_step(float (&v)[16], int lane) {
+__device__ __forceinline__ void colsum8_step(float (&v)[8], int lane) {
   const bool up = (lane & M) != 0;
 #pragma unroll
   for (int k = 0; k < N; ++k) {
@@ -57,11 +57,12 @@ __device__ __forceinline__ void colsum16_step(float (&v)[16], int lane) {
     v[k] = keep + __shfl_xor_sync(0xffffffffu, send, M);
   }
 }
-__device__ __forceinline__ void colsum16(float (&v)[16], int lane) {
-  colsum16_step<8, 8>(v, lane);
-  colsum16_step<4, 4>(v, lane);
-  colsum16_step<2, 2>(v, lane);
-  colsum16_step<1, 1>(v, lane);
+__device__ __forceinline__ void colsum8(float (&v)[8], int lane) {
+  colsum8_step<4, 4>(v, lane);
+  colsum8_step<2, 2>(v, lane);
+  colsum8_step<1, 1>(v, lane);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 8);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);
 }
 
 // Reverse inclusive cumulative sum over 64 values by one warp, two per lane: call with a = x[63 - 2 lane],

@@ -18,14 +18,17 @@
 //   m3s_state_pass_kernel   per (b, head), sequential over the chunks, forward or reverse: the chunk contribution
 //                           Brot^T diag(r e) X (or Crot^T diag(exp(Lam)) dY) folded into the running state
 //   m3s_chunk_out_kernel    per chunk: Y
-//   m3s_chunk_grad_kernel   per chunk: dx, rotated-row gradients -> dB, dC partials, per-token scalars
+//   m3s_chunk_grad_kernel   per chunk and up to 16 heads of a group: dx, dB, dC summed over these heads, per-token scalars
 //   m3s_tail_kernel         per (b, head): suffix sum of the angle gradient, ddt, dlambda, dtheta, da_log shares; per chunk:
-//                           dB, dC summed over the heads of a group
+//                           dB, dC summed over the CTAs of a group
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "common.cuh"
+#include "packed.cuh"
 #include "umma_tiles.cuh"
 
 namespace mxb {
@@ -40,6 +43,7 @@ using tc::unpack8;
 
 struct SsdP {
   int B, T, D, G, NH, n;   // n = chunks
+  int splits, hp;          // CTAs of the chunk-gradient kernel per group of heads, heads of each (the last one may have fewer)
   int no_tma;              // stage operands with cp.async even where tensor maps can be made
   const bf16 *x, *b, *c, *dy;
   const float *dt_raw, *lam_raw, *theta, *a_log;
@@ -52,7 +56,7 @@ struct SsdP {
   float *dphi, *da, *de, *dgam; // [B,NH,T] per-token scalar gradients
   float* dal_part;              // [B,NH] per-batch shares of da_log
   float* cs;                    // [B,NH,n] ChunkScal records
-  bf16 *pb, *pc;                // [B,NH,n] column-blocked [64][128] images: per-head partial dB, dC (summed in fp32 by the tail kernel)
+  bf16 *pb, *pc;                // [B,G*splits,n] column-blocked [64][128] images: partial dB, dC (summed in fp32 by the tail kernel)
 };
 
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : (x < -20.f ? expf(x) : log1pf(expf(x))); }
@@ -72,6 +76,22 @@ __device__ __forceinline__ void ld_acc16(uint32_t taddr, int warp, int c0, float
   tc::tmem_ld_wait();
 #pragma unroll
   for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ float ex2(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+// Two packed bf16 as two floats and back.
+__device__ __forceinline__ f2 widen2(uint32_t w) { return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+__device__ __forceinline__ uint32_t narrow2(f2 v) {
+  const float2 t = unpack2(v);
+  return tc::pack_bf16(t.x, t.y);
+}
+__device__ __forceinline__ f2 neg2(f2 v) { return v ^ 0x8000000080000000ull; }
+__device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(mbar)) : "memory");
 }
 
 // Per-chunk scalars: computed once per (batch, head, chunk) by m3s_chunk_scalars_kernel into a workspace record
@@ -160,6 +180,15 @@ __device__ __forceinline__ void issue_x_tile(uint8_t* dst, const bf16* src, cons
     tc::cp_async16(sd + 16 * u, ok ? src + ((size_t)b * p.T + t0 + t) * p.D + d0 + c8 * 8 : src, ok);
   }
 }
+// Rows of a token tensor ([B,T,heads,64] or a 64-column slab of [B,T,G,128]) into a swizzled slab, by threads tid of nt;
+// src: the row of step t0.
+__device__ __forceinline__ void stage_slab(uint32_t dst, const bf16* src, int T, size_t stride, int t0, int tid, int nt) {
+  for (int u = tid; u < Q * 8; u += nt) {
+    const int t = u >> 3, c8 = u & 7;
+    const bool ok = t0 + t < T;
+    tc::cp_async16(dst + (uint32_t)t * 128u + (uint32_t)((c8 ^ (t & 7)) << 4), ok ? src + (size_t)t * stride + c8 * 8 : src, ok);
+  }
+}
 // [128 n][64 p] bf16 state saved by the state pass as the byte image of the blocked tile
 __device__ __forceinline__ void issue_state_tile(uint8_t* dst, const bf16* src) {
   const uint32_t sd = tc::smem_u32(dst);
@@ -181,15 +210,6 @@ __device__ __forceinline__ void rotate_tile(uint8_t* tile, const float* sn, cons
     *reinterpret_cast<uint4*>(tile + 16 * u) = pack8(e);
   }
 }
-// dst = diag(rowscale) src for [64][64] tiles (dst may be src).
-__device__ __forceinline__ void scale_x_tile(uint8_t* dst, const uint8_t* src, const float* rowscale) {
-  for (int u = threadIdx.x; u < Q * 8; u += blockDim.x) {
-    const int t = ((u >> 6) << 3) | (u & 7);
-    *reinterpret_cast<uint4*>(dst + 16 * u) =
-        tc::scale_bf16x8(*reinterpret_cast<const uint4*>(src + 16 * u), rowscale[t]);
-  }
-}
-
 // ---- the same fix-ups and views for tiles that the copy engine wrote with 128-byte swizzle (SW = true) ----
 template <bool SW>
 __device__ __forceinline__ uint32_t in_unit(int t, int c8, int W) {
@@ -234,41 +254,44 @@ __device__ __forceinline__ void rotate_in_tile(uint8_t* tile, const float* sn, c
     for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(tile + 16 * (w0 + q * nt)) = raw[q];
   }
 }
-template <bool SW>
-__device__ __forceinline__ void scale_in_tile(uint8_t* dst, const uint8_t* src, const float* rowscale) {
-  if (!SW) { scale_x_tile(dst, src, rowscale); return; }
-  for (int w = threadIdx.x; w < Q * 8; w += blockDim.x)
-    *reinterpret_cast<uint4*>(dst + 16 * w) =
-        tc::scale_bf16x8(*reinterpret_cast<const uint4*>(src + 16 * w), rowscale[w >> 3]);
-}
 struct ChunkMaps {
   CUtensorMap b, c;   // [B,T,G,128] viewed as (N, G, T, B), boxes of 64 columns x 64 steps, 128-byte swizzle
-  CUtensorMap x, dy;  // [B,T,heads,64] viewed as (P, heads, T, B)
+  CUtensorMap x, dy, dx;  // [B,T,heads,64] viewed as (P, heads, T, B)
 };
 
 // Threads of the two per-(batch, head) scalar kernels: they are chains of dependent fp64 operations behind strided
 // loads, so many short chains (4 steps per thread at T = 4096) hide the latencies that few long ones expose.
 constexpr int kScalThreads = 1024;
-// Inclusive prefix sum of one double per thread over a kScalThreads-thread CTA (warp scans + the warp totals, a fixed
-// order); wtot is kScalThreads / 32 doubles of shared memory.  Also returns the CTA total.
-__device__ __forceinline__ double cta_scan(double v, double* wtot, double& total) {
+// Inclusive prefix sums of M doubles per thread over a kScalThreads-thread CTA (warp scans + the warp totals, a fixed order);
+// wtot is M x kScalThreads / 32 doubles of shared memory.  Also returns the CTA totals.
+template <int M>
+__device__ __forceinline__ void cta_scan(double (&v)[M], double* wtot, double (&total)[M]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const double t = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += t;
-  }
-  if (lane == 31) wtot[warp] = v;
-  __syncthreads();
-  double off = 0.0, tot = 0.0;
 #pragma unroll
-  for (int w = 0; w < kScalThreads / 32; ++w) {
-    const double x = wtot[w];
-    if (w < warp) off += x;
-    tot += x;
+    for (int m = 0; m < M; ++m) {
+      const double t = __shfl_up_sync(0xffffffffu, v[m], o);
+      if (lane >= o) v[m] += t;
+    }
   }
-  total = tot;
-  return v + off;
+  if (lane == 31) {
+#pragma unroll
+    for (int m = 0; m < M; ++m) wtot[m * (kScalThreads / 32) + warp] = v[m];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    double off = 0.0, tot = 0.0;
+#pragma unroll
+    for (int w = 0; w < kScalThreads / 32; ++w) {
+      const double x = wtot[m * (kScalThreads / 32) + w];
+      if (w < warp) off += x;
+      tot += x;
+    }
+    total[m] = tot;
+    v[m] += off;
+  }
 }
 
 // ------------------------------------------------------------ per-(b,head) scalars
@@ -302,8 +325,9 @@ __global__ void __launch_bounds__(kScalThreads) m3s_scalars_kernel(SsdP p) {
       }
     }
   }
-  double total;
-  double phi = cta_scan(acc, wtot, total) - acc;  // angle at the start of this thread's steps
+  double incl[1] = {acc}, total[1];
+  cta_scan(incl, wtot, total);
+  double phi = incl[0] - acc;  // angle at the start of this thread's steps
   const double two_pi = 6.283185307179586476925, inv_two_pi = 1.0 / two_pi;
   for (int t0 = lo; t0 < hi; t0 += kScalBatch) {
     float dtv[kScalBatch], th[kScalBatch];
@@ -328,148 +352,172 @@ __global__ void __launch_bounds__(kScalThreads) m3s_scalars_kernel(SsdP p) {
 // state in registers (thread = state row n and 32 of its 64 fp32 columns):
 //   mode 0: H0_c = H;  H = L_c H + Brot_c^T diag(r e) X_c          (states at chunk start, for y and the backward)
 //   mode 1: dH1_c = dH; dH = L_c dH + Crot_c^T diag(exp(Lam)) dY_c  (state gradients at chunk end)
-// The chunk contribution is one M=128 tcgen05 tile that never leaves the SM; the operands of the next chunks are
-// in flight in a ring of kPassStages buffers (a chunk takes ~1.5 us here and a copy up to ~2 us, so with two
-// buffers every chunk waited ~0.9 k cycles for its tiles) while the current one is rotated, multiplied and folded
-// in.  The saved state leaves as the byte image of the [128][64] operand tile (one bulk copy per chunk).
-constexpr int kPassStages = 3;
-constexpr int kPassStoreThread = 64;   // issues the state-image stores (its own bulk-group queue)
-constexpr int kPassSmem = kPassStages * (16384 + 8192) + kPassStages * sizeof(ChunkScal) + 2 * 16384 + 64 + 1024;
+// The rotation goes to the narrow operand, which is scaled anyway: with J^T(e, o) = (o, -e) on every pair of states
+//   Brot^T diag(r e) X = B^T diag(r e cos) X + J^T-rows of (B^T diag(r e sin) X)
+// so a chunk contributes one product of 128 columns, B^T [cosine image | sine image], whose second half is exchanged
+// between the two states of a pair (neighbouring lanes).  It never leaves the SM.  The saved state goes from registers to the
+// byte image of the [128][64] operand tile (eight rows of a unit column are one 128-byte line).
+//
+// Only the update of the state is sequential, so everything before it runs ahead: a warp issues the copies, two warps scale
+// landed tiles to their two images, a warp issues the products into two accumulators by turns, eight warps hold the state,
+// fold in an accumulator and store the state (one sequence of 32 heads x 64 chunks: 49 us, 8 sequences 93; chunk by chunk in
+// one group of warps, with B rotated in place, 84 and 104).  Every hand-over is an mbarrier with a bounded wait; a warp whose wait has run out stops waiting and working but goes through its loop.
+constexpr int kPassThreads = 32 * 12;
+template <int NS>
+constexpr int kPassSmem = NS * (16384 + 16384) + (NS + 2) * (int)sizeof(ChunkScal) + (4 * NS + 12) * 8 + 16 + 1024;
 
 struct PassMaps {
   CUtensorMap r;  // b or c: [B,T,G,128] viewed as (N, G, T, B), boxes of 64 columns x 64 steps, 128-byte swizzle
   CUtensorMap x;  // x or dy: [B,T,heads,64] viewed as (P, heads, T, B)
 };
 
-// TMA = true: the three operand boxes of a chunk and its scalar record arrive by the copy engine on one mbarrier
-// per buffer (tiles in the 128-byte-swizzled layout); TMA = false: cp.async staging into the un-swizzled layout.
-template <bool TMA>
-__global__ void __launch_bounds__(256) m3s_state_pass_kernel(SsdP p, int mode, const __grid_constant__ PassMaps maps) {
+// TMA = true: the three operand boxes of a chunk arrive by the copy engine; TMA = false: cp.async staging into the same
+// swizzled positions.  NS: stages in flight; three where two CTAs share an SM.
+template <bool TMA, int NS>
+__global__ void __launch_bounds__(kPassThreads, NS == 3 ? 2 : 1) m3s_state_pass_kernel(SsdP p, int mode, const __grid_constant__ PassMaps maps) {
+  constexpr int NC = NS + 2;         // scalar records: the decay is read behind the product
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
-  uint8_t* Himg = sm + kPassStages * (16384 + 8192);  // 2 x [128 n][64 p] bf16 images of the state on their way out
-  uint8_t* scal = Himg + 2 * 16384;
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(scal + kPassStages * sizeof(ChunkScal));  // [0] MMA, [1 + stage] stage full
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 1 + kPassStages);
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int nrow = tid & 127, half = tid >> 7;  // thread = state row n, 32 of its 64 columns
-  const int head = blockIdx.x, b = blockIdx.y;
+  uint8_t* Rt = sm;                  // xNS [64 s][128 n] B or C rows
+  uint8_t* Xt = Rt + NS * 16384;     // xNS [64 s][64 p] x or dy, then its cosine image; the sine image
+  ChunkScal* scal = reinterpret_cast<ChunkScal*>(Xt + NS * 16384);
+  uint64_t* full = reinterpret_cast<uint64_t*>(scal + NC);  // xNS: tiles landed
+  uint64_t* ready = full + NS;       // xNS: images written
+  uint64_t* freed = ready + NS;      // xNS: product done
+  uint64_t* accfull = freed + NS;    // x2: product done
+  uint64_t* accfree = accfull + 2;   // x2: accumulator read
+  uint64_t* cfree = accfree + 2;       // xNC: scalar record read
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(cfree + NC);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int head = blockIdx.x, b = blockIdx.y, n = p.n;
   const int d0 = head * P, g = d0 / (p.D / p.G);
-  const size_t cbase = ((size_t)b * p.NH + head) * p.n;
-  auto Rt = [&](int buf) { return sm + buf * 16384; };             // [64 s][128 n] B or C rows, rotated in place
-  auto Xt = [&](int buf) { return sm + kPassStages * 16384 + buf * 8192; };  // [64 s][64 p]  x or dy, scaled in place
-  auto Sc = [&](int buf) -> ChunkScal& { return *reinterpret_cast<ChunkScal*>(scal + buf * sizeof(ChunkScal)); };
-  auto chunk_at = [&](int it) { return mode == 0 ? it : p.n - 1 - it; };
-  auto issue = [&](int it) {
-    if (it < p.n) {
-      const int c = chunk_at(it), buf = it % kPassStages;
-      if (TMA) {
-        // two threads of two other warps than the one that issues the MMAs share the copies; the barrier's single
-        // arrival is the expect_tx, so the phase cannot complete before every byte announced there has landed
-        if (tid == 32) {
-          tc::mbar_expect_tx(&mbar[1 + buf], 16384 + 8192 + (uint32_t)sizeof(ChunkScal));
-          tc::tma_load_4d(tc::smem_u32(Rt(buf)), &maps.r, 0, g, c * Q, b, &mbar[1 + buf]);
-          tc::tma_load_4d(tc::smem_u32(Rt(buf)) + 8192, &maps.r, 64, g, c * Q, b, &mbar[1 + buf]);
-        }
-        if (tid == 96) {
-          tc::tma_load_4d(tc::smem_u32(Xt(buf)), &maps.x, 0, head, c * Q, b, &mbar[1 + buf]);
-          tc::bulk_load(tc::smem_u32(&Sc(buf)), p.cs + (cbase + c) * (sizeof(ChunkScal) / 4), (uint32_t)sizeof(ChunkScal),
-                        &mbar[1 + buf]);
-        }
-      } else {
-        issue_rows_tile(Rt(buf), mode == 0 ? p.b : p.c, p, b, g, c * Q);
-        issue_x_tile(Xt(buf), mode == 0 ? p.x : p.dy, p, b, d0, c * Q);
-        issue_chunk_scalars(p, cbase + c, Sc(buf));
-      }
-    }
-    if (!TMA) tc::cp_async_commit();
-  };
-  // rows of the landed tiles: rotate B/C pairs, scale x/dy (16-byte units; a unit never straddles a pair)
-  auto fix_tiles = [&](int buf) {
-    const ChunkScal& s = Sc(buf);
-    const float* rowscale = mode == 0 ? s.re : s.dexp;
-    if (TMA) {  // swizzled slabs of [64 rows][128 bytes]: unit w of a slab belongs to row w / 8
-      rotate_in_tile<true>(Rt(buf), s.sn, s.cs);
-      {  // both units of this thread: loads first, then the stores
-        const uint4 a = *reinterpret_cast<const uint4*>(Xt(buf) + 16 * tid);
-        const uint4 c2 = *reinterpret_cast<const uint4*>(Xt(buf) + 16 * (tid + 256));
-        const float ra = rowscale[tid >> 3], rc = rowscale[(tid + 256) >> 3];
-        *reinterpret_cast<uint4*>(Xt(buf) + 16 * tid) = tc::scale_bf16x8(a, ra);
-        *reinterpret_cast<uint4*>(Xt(buf) + 16 * (tid + 256)) = tc::scale_bf16x8(c2, rc);
-      }
-    } else {
-      rotate_tile(Rt(buf), s.sn, s.cs);
-      scale_x_tile(Xt(buf), Xt(buf), rowscale);
-    }
-  };
-  if (warp == 0) { tc::tmem_alloc(tslot, 64); tc::tmem_relinquish(); }
-  if (tid == 0) {
-    for (int m = 0; m < 1 + kPassStages; ++m) tc::mbar_init(&mbar[m], 1);
+  const size_t cbase = ((size_t)b * p.NH + head) * n;
+  auto chunk_at = [&](int it) { return mode == 0 ? it : n - 1 - it; };
+  if (warp == 0) { tc::tmem_alloc(tslot, 256); tc::tmem_relinquish(); }
+  if (tid == 32) {
+    for (int s = 0; s < NS; ++s) { tc::mbar_init(full + s, TMA ? 1 : 33); tc::mbar_init(ready + s, 2); tc::mbar_init(freed + s, 1); }
+    for (int s = 0; s < 2; ++s) { tc::mbar_init(accfull + s, 1); tc::mbar_init(accfree + s, 8); }
+    for (int s = 0; s < NC; ++s) tc::mbar_init(cfree + s, 8);
     tc::mbar_fence_init();
   }
-  __syncthreads();  // barriers initialised before the copies can complete on them
-  for (int it = 0; it < kPassStages; ++it) issue(it);
-  float H[32];
-#pragma unroll
-  for (int x = 0; x < 32; ++x) H[x] = 0.f;
-  bool ok = true;
-  if (TMA) ok = tc::mbar_wait(&mbar[1], 0);
-  else tc::cp_async_wait<kPassStages - 1>();  // operands of the first chunk
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t taddr = *tslot;
-  bf16* out = mode == 0 ? p.H0 : p.dH1;
-  uint32_t ph = 0;
-  fix_tiles(0);
-  for (int it = 0; it < p.n; ++it) {
-    const int c = chunk_at(it), buf = it % kPassStages, nbuf = (it + 1) % kPassStages;
-    const float L = Sc(buf).L;
-    uint8_t* Hi = Himg + (it & 1) * 16384;  // the image written two chunks ago has left this tile (checked below)
+  bool ok = true;
+  auto wait = [&](uint64_t* m, int parity) { if (ok) ok = tc::mbar_wait(m, (uint32_t)parity & 1u); };
+  auto arrive = [&](uint64_t* m) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(m);
+  };
+  if (warp == 8) {          // ---- copies
+    int issued = 0;
+    for (int it = 0; it < n; ++it) {
+      const int s = it % NS, c = chunk_at(it);
+      if (it >= NS) wait(freed + s, it / NS - 1);
+      if (it >= NC) wait(cfree + it % NC, it / NC - 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      ++issued;
+      if (lane == 0) {
+        tc::mbar_expect_tx(full + s, (TMA ? 16384 + 8192 : 0) + (uint32_t)sizeof(ChunkScal));
+        if (TMA) {
+          tc::tma_load_4d(tc::smem_u32(Rt + s * 16384), &maps.r, 0, g, c * Q, b, full + s);
+          tc::tma_load_4d(tc::smem_u32(Rt + s * 16384) + 8192, &maps.r, 64, g, c * Q, b, full + s);
+          tc::tma_load_4d(tc::smem_u32(Xt + s * 16384), &maps.x, 0, head, c * Q, b, full + s);
+        }
+        tc::bulk_load(tc::smem_u32(scal + it % NC), p.cs + (cbase + c) * (sizeof(ChunkScal) / 4), (uint32_t)sizeof(ChunkScal), full + s);
+      }
+      if (!TMA) {
+        const size_t row = (size_t)b * p.T + c * Q;
+        const bf16* rsrc = (mode == 0 ? p.b : p.c) + (row * p.G + g) * N;
+        for (int sl = 0; sl < 2; ++sl)
+          stage_slab(tc::smem_u32(Rt + s * 16384) + 8192 * sl, rsrc + 64 * sl, p.T, (size_t)p.G * N, c * Q, lane, 32);
+        stage_slab(tc::smem_u32(Xt + s * 16384), (mode == 0 ? p.x : p.dy) + row * p.D + d0, p.T, p.D, c * Q, lane, 32);
+        tc::cp_async_wait_all();
+        tc::fence_async_smem();
+        mbar_arrive(full + s);
+      }
+    }
+    for (int q = max(0, issued - NS); q < issued; ++q) tc::mbar_wait(full + q % NS, (q / NS) & 1);  // (outlive the copies)
+  } else if (warp == 9) {   // ---- products
+    if (tc::elect_one()) {
+      for (int it = 0; it < n; ++it) {
+        const int s = it % NS, a = it & 1;
+        wait(ready + s, it / NS);
+        if (it > 1) wait(accfree + a, (it >> 1) - 1);
+        if (!ok) break;
+        tc::fence_after_sync();
+        // [128 n x 2 64 p], contracted over the rows
+        tc::issue_gemm(taddr + 128 * a, tc::mnmajor_sw128_tile(Rt + s * 16384, 8192), tc::mnmajor_sw128_tile(Xt + s * 16384, 8192), 128, 2 * P, Q, false);
+        tc::mma_commit(accfull + a);
+        tc::mma_commit(freed + s);
+      }
+    }
+    __syncwarp();
+  } else if (warp >= 10) {  // ---- images of x or dy: a row per thread, four units at a time, loads first
+    const int r = tid - 320;
+    for (int it = 0; it < n; ++it) {
+      const int st = it % NS;
+      wait(full + st, it / NS);
+      const ChunkScal& s = scal[it % NC];
+      const float f = mode == 0 ? s.re[r] : s.dexp[r];
+      const f2 c2 = dup2(f * s.cs[r]), s2 = dup2(f * s.sn[r]);
+      uint8_t* X = Xt + st * 16384 + 128 * r;
 #pragma unroll
-    for (int x = 0; x < 4; ++x) sts16(Hi, tc::kmajor_unit(nrow, 4 * half + x, P), pack8(&H[8 * x]));
-    tc::fence_async_smem();
-    tc::fence_before_sync();
-    // tiles of this chunk rotated and scaled (during the previous chunk's MMA), image staged
-    ok = __syncthreads_and(ok);  // the barrier also makes the verdict of the bounded waits uniform, so that all
-    if (!ok) break;              // threads leave the loop together
-    tc::fence_after_sync();
-    if (tid == 0) {  // [128 n x 64 p] = R^T X, both contracted over their rows
-      if (TMA)
-        tc::issue_gemm(taddr, tc::mnmajor_sw128_tile(Rt(buf), 8192), tc::mnmajor_sw128_tile(Xt(buf), 8192), 128, P, Q, false);
-      else
-        tc::issue_gemm(taddr, tc::mnmajor_tile(Rt(buf), N), tc::mnmajor_tile(Xt(buf), P), 128, P, Q, false);
-      tc::mma_commit(mbar);
-    }
-    if (tid == kPassStoreThread) {  // the state image leaves from another warp than the one issuing the MMAs
-      tc::bulk_store(out + (cbase + c) * (N * P), tc::smem_u32(Hi), 16384);
-      tc::bulk_commit();
-      tc::bulk_wait_read<1>();  // all but the copy just issued have been read out of shared memory
-    }
-    if (it + 1 < p.n) {  // while the tensor core works: the next chunk's tiles
-      if (TMA) { if (ok) ok = tc::mbar_wait(&mbar[1 + nbuf], ((it + 1) / kPassStages) & 1); }
-      else tc::cp_async_wait<kPassStages - 2>();
-      __syncthreads();
-      fix_tiles(nbuf);
-    }
-    if (ok) ok = tc::mbar_wait(mbar, ph);
-    ph ^= 1;
-    tc::fence_after_sync();
-    issue(it + kPassStages);  // this buffer is free: the MMA has read the tiles, every thread has read L
-    if (ok) {
-      float f[32];
-      ld_acc32(taddr, warp, 32 * half, f);
+      for (int w0 = 0; w0 < 8; w0 += 4) {
+        uint4 x[4];
 #pragma unroll
-      for (int jj = 0; jj < 32; ++jj) H[jj] = fmaf(L, H[jj], f[jj]);
+        for (int q = 0; q < 4; ++q) x[q] = *reinterpret_cast<const uint4*>(X + (((w0 + q) ^ (r & 7)) << 4));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const f2 v[4] = {widen2(x[q].x), widen2(x[q].y), widen2(x[q].z), widen2(x[q].w)};
+          uint8_t* dst = X + (((w0 + q) ^ (r & 7)) << 4);
+          *reinterpret_cast<uint4*>(dst) =
+              make_uint4(narrow2(mul2(v[0], c2)), narrow2(mul2(v[1], c2)), narrow2(mul2(v[2], c2)), narrow2(mul2(v[3], c2)));
+          *reinterpret_cast<uint4*>(dst + 8192) =
+              make_uint4(narrow2(mul2(v[0], s2)), narrow2(mul2(v[1], s2)), narrow2(mul2(v[2], s2)), narrow2(mul2(v[3], s2)));
+        }
+      }
+      tc::fence_async_smem();
+      arrive(ready + st);
     }
-    tc::fence_before_sync();
+  } else if (warp < 8) {    // ---- the state: thread = state row and 32 of its 64 columns
+    const int nrow = tid & 127, half = tid >> 7;
+    const float sign = nrow & 1 ? -1.f : 1.f;
+    float H[32];
+#pragma unroll
+    for (int x = 0; x < 32; ++x) H[x] = 0.f;
+    uint4* out = reinterpret_cast<uint4*>((mode == 0 ? p.H0 : p.dH1) + cbase * (N * P)) + (tc::kmajor_unit(nrow, 4 * half, P) >> 4);
+    for (int it = 0; it < n; ++it) {
+      const int a = it & 1;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) out[(size_t)chunk_at(it) * (N * P / 8) + 8 * x] = pack8(&H[8 * x]);
+      wait(accfull + a, it >> 1);
+      tc::fence_after_sync();
+      ok = __all_sync(0xffffffffu, ok);
+      const float L = scal[it % NC].L;
+      if (ok) {
+#pragma unroll
+        for (int c0 = 0; c0 < 32; c0 += 16) {
+          float f[16], o[16];
+          ld_acc16(taddr + 128 * a + P, warp, 32 * half + c0, o);
+          ld_acc16(taddr + 128 * a, warp, 32 * half + c0, f);
+#pragma unroll
+          for (int jj = 0; jj < 16; ++jj) {
+            f[jj] = fmaf(sign, __shfl_xor_sync(0xffffffffu, o[jj], 1), f[jj]);
+            H[c0 + jj] = fmaf(L, H[c0 + jj], f[jj]);
+          }
+        }
+      }
+      tc::fence_before_sync();
+      arrive(accfree + a);
+      arrive(cfree + it % NC);
+    }
   }
-  if (!TMA) tc::cp_async_wait<0>();
-  if (tid == kPassStoreThread) tc::bulk_wait_read<0>();  // shared memory must outlive the copies
-  if (!ok && tid == 0) atomicExch(p.status, 11);
-  tc::fence_before_sync();
+  if (!ok && lane == 0) atomicExch(p.status, 11);
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(taddr, 64);
+  if (warp == 0) tc::tmem_dealloc(taddr, 256);
 }
 
 // ------------------------------------------------------------ chunk output
@@ -609,306 +657,533 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
 }
 
 // ------------------------------------------------------------ chunk gradients
-// 256 TMEM columns and < 114 KB of shared memory, so two CTAs share an SM.  Every product with M = 64 is issued in the
-// weight-stationary form: all 128 TMEM lanes hold results, so that every thread has a row (t) and a quarter of the
-// columns (16 of 64, 32 of 128), and a result takes half of the TMEM columns:
-//   batch 1: G [0,32), dY X^T [32,64); then Crot H0 [64,96), Brot dH1 [96,128), (e^Lam dY) H0^T [192,256),
-//            (r e x) dH1^T [128,192)
-//   batch 2: dx [0,32), dCrot: += dG Brot [192,256); then dBrot: += dG^T Crot [128,192)
-// The G*M tile reuses the x tile once x is dead.  The column sums of dM*D*w that dLam needs are e_s (or gamma_s on the
-// diagonal) times those of dM*D, which de needs anyway.
-// Bound by the phases of a CTA that follow one another (HBM: 1.5 GB, 0.23 ms).  8 x 4096 x 32 heads: three batches with
-// half of the lanes idle in every epilogue 726 us, this 531 us.
-constexpr int kGradSmem = 16384 * 4 + 8192 * 5 + sizeof(ChunkScal) + (2 * Q + 16 * Q + 32) * 4 + 64 + 1024;
+// One CTA per chunk and up to kGradHeads heads of a group.  The heads of a group share B and C and differ by one angle per
+// step, so nothing is rotated: with J(e, o) = (-o, e) on every pair of states and delta = phi_t - phi_s
+//     Crot_t . Brot_s = cos(delta) (C B^T)_ts + sin(delta) (C (J B)^T)_ts
+//     (Crot H0)_t     = cos(phi_t) (C H0)_t + sin(phi_t) (CJ H0)_t,   CJ = J^T C
+// the two 64 x 64 products stay in registers for all heads, and what the heads add to dB and dC is summed before it meets
+// B and C: over the 64 x 64 products in registers (W1, W2), over the chunk states in tensor memory,
+//     dC = W1 B + W2 (J B) + Z1 + J Z2,   Z1 = sum_h (cos e^Lam dY) H0^T,  Z2 = sum_h (sin e^Lam dY) H0^T
+//     dB = W1^T C + W2^T CJ + Y1 + J Y2,  Y1 = sum_h (cos r e x) dH1^T,     Y2 = sum_h (sin r e x) dH1^T
+//     W1_ts = sum_h cos(delta) dG_ts,  W2_ts = sum_h sin(delta) dG_ts,      dG = (dY X^T) * M
+// so one partial image of dB and dC leaves per CTA instead of one per head.
+//
+// One CTA per SM: 16 warps with a row t and 8 of 64 columns of every product, one warp that issues the copies, one that
+// issues the products (an elected thread of a warp of its own: 33 cycles an instruction, 60 behind a test of the thread's
+// index), one that finishes the per-step scalars and one that stores dx; everything is handed over by mbarriers.
+// Products of a head: dP = dY X^T, U = {C, CJ} H0, V = {B, JB} dH1 (asked for a head ahead), Z and Y, then dX = (G*M)^T dY.
+// 8 x 4096 x 32 heads: 338 us + 60 for the row sums behind it, 1.0 GB (0.15 ms); a CTA per head and chunk that rotated B and C
+// took 527 + 118 with 1.5 + 0.6 GB.  A head takes 5.0 k cycles, most of it the arithmetic of the 64 x 64 products (1.3 k), of U
+// and V (0.9 k) and of the scaled images (0.6 k) at half of the issue slots; pairs of columns in packed registers (7.8 k without).
+// TMEM: Z [0,128), Y [128,256), U [256,320), V [320,384), dP [384,416), dX [416,448); at the start C B^T and C (J B)^T in
+// the last two, at the end the products with W1 and W2 in U and V.
+constexpr int kGradWarps = 16;
+constexpr int kGradThreads = 32 * (kGradWarps + 4);
+constexpr int kGradStage = 2 * 8192 + 2 * 16384;  // x, dY, H0, dH1 of a head
+constexpr int kGradPart = (8 * 4 * Q + 4 * Q + 32) * 4;
+constexpr int kGradSmem = 4 * 16384 + 2 * kGradStage + 4 * 8192 + 8192 + 8192 + kGradPart + 4 * (int)sizeof(ChunkScal) + 24 * 8 + 16 + 1024;
+static_assert(kGradSmem <= 227 * 1024, "one CTA per SM");
+constexpr int kGradPitch = N + 4;  // floats per row of the sums on their way out (over the stages)
+static_assert(2 * Q * kGradPitch * 4 <= 2 * kGradStage, "two tiles of row sums fit into the stages");
 
-// sum_k tile[r][c0 + k] f[k], 16 columns of a [.][64] tile
-template <bool SW>
-__device__ __forceinline__ float row_dot16_64(const uint8_t* tile, int r, int c0, const float (&f)[16]) {
-  float acc[2] = {0.f, 0.f};
+// 8 columns of a result as four pairs.
+__device__ __forceinline__ void ld_pairs(uint32_t taddr, int warp, f2 (&f)[4]) {
+  uint32_t r[8];
+  tc::tmem_ld_32x32b_x8(taddr + ((uint32_t)(32 * (warp & 3)) << 16), r);
 #pragma unroll
-  for (int x = 0; x < 2; ++x) {
-    float e[8];
-    unpack8(*reinterpret_cast<const uint4*>(tile + in_unit<SW>(r, (c0 >> 3) + x, P)), e);
-#pragma unroll
-    for (int y = 0; y < 8; ++y) acc[x] = fmaf(e[y], f[8 * x + y], acc[x]);
-  }
-  return acc[0] + acc[1];
+  for (int i = 0; i < 4; ++i) f[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
 }
-
 template <bool TMA>
-__global__ void __launch_bounds__(256) m3s_chunk_grad_kernel(SsdP p, const __grid_constant__ ChunkMaps maps) {
+__global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p, const __grid_constant__ ChunkMaps maps) {
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
-  uint8_t* Bt = sm;                // [64][128] Brot
-  uint8_t* Ct = Bt + 16384;        // [64][128] Crot
-  uint8_t* Ht = Ct + 16384;        // [128][64] H0
-  uint8_t* Dt = Ht + 16384;        // [128][64] dH1
-  uint8_t* Xt = Dt + 16384;        // [64][64]  x
-  uint8_t* Yt = Xt + 8192;         // [64][64]  dY
-  uint8_t* Xs = Yt + 8192;         // [64][64]  r e x
-  uint8_t* Ys = Xs + 8192;         // [64][64]  exp(Lam) dY
-  uint8_t* GMt = Xt;               // [64][64]  G*M  (written after the last read of x)
-  uint8_t* dGt = Ys + 8192;        // [64][64]  dG
-  ChunkScal& s = *reinterpret_cast<ChunkScal*>(dGt + 8192);
-  float* csw = reinterpret_cast<float*>(&s + 1);    // [2][Q] column sums of dM*D (s < t) over the two halves of the rows
-  float* part = csw + 2 * Q;                        // [4][4][Q]: per column quarter: dLam, de, dgam, dphi row partials
-  float* red = part + 16 * Q;                       // [32]
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(red + 32);  // [0], [3] MMA completion, [1] token tiles, [2] state images
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 4);
+  uint8_t* Bt = sm;                    // [64][128] B, J B, C, CJ (swizzled slabs)
+  uint8_t* Jt = Bt + 16384;
+  uint8_t* Ct = Jt + 16384;
+  uint8_t* Kt = Ct + 16384;
+  uint8_t* Yc = Kt + 16384;            // [64][64] cos e^Lam dY, then sin e^Lam dY, cos r e x, sin r e x (swizzled like their sources)
+  uint8_t* Xc = Yc + 2 * 8192;
+  uint8_t* GMt = Xc + 2 * 8192;        // [64][64] G*M
+  uint8_t* Dx = GMt + 8192;            // [64][64] dx on its way out (swizzled)
+  uint8_t* St = Dx + 8192;             // two stages: x, dY (swizzled), H0, dH1 (images)
+  ChunkScal* scal = reinterpret_cast<ChunkScal*>(St + 2 * kGradStage);  // x4: the scalars of a head (read longer than its tiles)
+  float* part = reinterpret_cast<float*>(scal + 4);  // [8 column groups][4][Q]: dLam, de, dgam, dphi row partials
+  float* csw = part + 8 * 4 * Q;       // [2][2][Q] column sums over the two halves of the rows: of dM*D (s < t), of dG dG/ddelta
+  float* red = csw + 4 * Q;            // [16] <dH1, H0> per warp
+  uint64_t* full = reinterpret_cast<uint64_t*>(red + 32);  // x2: a head's operands landed
+  uint64_t* freed = full + 2;          // x2: and are no longer needed
+  uint64_t* tiles = freed + 2;         // B, C landed
+  uint64_t* images = tiles + 1;        // the scaled images of a head are written (first: J B and CJ; last: W1 and W2)
+  uint64_t* gready = images + 1;       // G*M is written
+  uint64_t* uvfree = gready + 1;       // dP, U, V are read
+  uint64_t* pready = uvfree + 1;       // row partials are written
+  uint64_t* pfree = pready + 1;
+  uint64_t* xready = pfree + 1;        // dx is written
+  uint64_t* xfree = xready + 1;
+  uint64_t* m1 = xfree + 1;            // products: dP, U, V
+  uint64_t* m2 = m1 + 1;               // products: Z, Y, dX
+  uint64_t* m0 = m2 + 1;               // products of the start
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(m0 + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int c = blockIdx.x, head = blockIdx.y, b = blockIdx.z, t0 = c * Q;
-  const int d0 = head * P, g = d0 / (p.D / p.G);
-  const size_t ci = ((size_t)b * p.NH + head) * p.n + c;
-  // this thread's row and column quarter of every result; tc16 / tc32: its TMEM columns of a [64][64] / [64][128] result
-  const int t = 32 * (warp & 1) + lane, qd = (warp & 2) + (warp >> 2), n16 = 16 * qd;
-  const int tc16 = 16 * (warp >> 2), tc32 = 32 * (warp >> 2);
+  const int c = blockIdx.x, b = blockIdx.z, t0 = c * Q;
+  const int per = p.NH / p.G, g = blockIdx.y / p.splits, sp = blockIdx.y % p.splits;
+  const int h0 = g * per + sp * p.hp, nh = min(p.hp, g * per + per - h0);  // this CTA's heads
+  auto unit_of = [&](int head) { return ((size_t)b * p.NH + head) * p.n + c; };
 
-  if (warp == 0) { tc::tmem_alloc(tslot, 256); tc::tmem_relinquish(); }
-  // the thread that initialises the barriers also issues the copies, on another warp than the TMEM allocation
+  if (warp == 0) { tc::tmem_alloc(tslot, 512); tc::tmem_relinquish(); }
   if (tid == 32) {
-    for (int m = 0; m < 4; ++m) tc::mbar_init(mbar + m, 1);
+    for (int s = 0; s < 2; ++s) {
+      tc::mbar_init(full + s, TMA ? 1 : 33); tc::mbar_init(freed + s, kGradWarps + 1);
+    }
+    tc::mbar_init(tiles, TMA ? 1 : 32);
+    tc::mbar_init(images, kGradWarps); tc::mbar_init(gready, kGradWarps); tc::mbar_init(uvfree, kGradWarps);
+    tc::mbar_init(pready, kGradWarps); tc::mbar_init(pfree, 1); tc::mbar_init(xready, kGradWarps); tc::mbar_init(xfree, 1);
+    tc::mbar_init(m0, 1); tc::mbar_init(m1, 1); tc::mbar_init(m2, 1);
     tc::mbar_fence_init();
   }
-  bool ok = true;
-  if (TMA) {  // every operand by the copy engine: token tiles on one barrier, the state images on another
-    if (tid == 32) {
-      tc::mbar_expect_tx(mbar + 1, 2 * 16384 + 2 * 8192 + (uint32_t)sizeof(ChunkScal));
-      for (int sl = 0; sl < 2; ++sl) {
-        tc::tma_load_4d(tc::smem_u32(Bt) + 8192 * sl, &maps.b, 64 * sl, g, t0, b, mbar + 1);
-        tc::tma_load_4d(tc::smem_u32(Ct) + 8192 * sl, &maps.c, 64 * sl, g, t0, b, mbar + 1);
-      }
-      tc::tma_load_4d(tc::smem_u32(Xt), &maps.x, 0, head, t0, b, mbar + 1);
-      tc::tma_load_4d(tc::smem_u32(Yt), &maps.dy, 0, head, t0, b, mbar + 1);
-      tc::bulk_load(tc::smem_u32(&s), p.cs + ci * (sizeof(ChunkScal) / 4), (uint32_t)sizeof(ChunkScal), mbar + 1);
-      tc::mbar_expect_tx(mbar + 2, 2 * 16384);
-      tc::bulk_load(tc::smem_u32(Ht), p.H0 + ci * (N * P), 16384, mbar + 2);
-      tc::bulk_load(tc::smem_u32(Dt), p.dH1 + ci * (N * P), 16384, mbar + 2);
-    }
-  } else {
-    issue_rows_tile(Bt, p.b, p, b, g, t0);
-    issue_rows_tile(Ct, p.c, p, b, g, t0);
-    issue_x_tile(Xt, p.x, p, b, d0, t0);
-    issue_x_tile(Yt, p.dy, p, b, d0, t0);
-    issue_chunk_scalars(p, ci, s);
-    tc::cp_async_commit();
-    issue_state_tile(Ht, p.H0 + ci * (N * P));
-    issue_state_tile(Dt, p.dH1 + ci * (N * P));
-    tc::cp_async_commit();
-  }
-  if (TMA) __syncthreads();  // barriers initialised before anyone waits on them
-  if (TMA) ok = tc::mbar_wait(mbar + 1, 0);
-  else tc::cp_async_wait<1>();
-  __syncthreads();
-  rotate_in_tile<TMA>(Bt, s.sn, s.cs);
-  rotate_in_tile<TMA>(Ct, s.sn, s.cs);
-  scale_in_tile<TMA>(Xs, Xt, s.re);
-  scale_in_tile<TMA>(Ys, Yt, s.dexp);
-  if (TMA) { if (ok) ok = tc::mbar_wait(mbar + 2, 0); }
-  else tc::cp_async_wait<0>();
-  tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t taddr = *tslot;
-  if (tid == 0) {
-    tc::issue_gemm<true>(taddr + 0, in_kmajor<TMA>(Ct, N), in_kmajor<TMA>(Bt, N), 64, Q, N, false);      // G
-    tc::issue_gemm<true>(taddr + 32, in_kmajor<TMA>(Yt, P), in_kmajor<TMA>(Xt, P), 64, Q, P, false);     // dY X^T
-    tc::mma_commit(mbar);
-    tc::issue_gemm<true>(taddr + 64, in_kmajor<TMA>(Ct, N), tc::mnmajor_tile(Ht, P), 64, P, N, false);   // Crot H0
-    tc::issue_gemm<true>(taddr + 96, in_kmajor<TMA>(Bt, N), tc::mnmajor_tile(Dt, P), 64, P, N, false);   // Brot dH1
-    tc::issue_gemm<true>(taddr + 192, in_kmajor<TMA>(Ys, P), tc::kmajor_tile(Ht, P), 64, N, P, false);   // (e^Lam dY) H0^T
-    tc::issue_gemm<true>(taddr + 128, in_kmajor<TMA>(Xs, P), tc::kmajor_tile(Dt, P), 64, N, P, false);   // (r e x) dH1^T
-    tc::mma_commit(mbar + 3);
-  }
-  {  // <dH1, H0> while the tensor core works
-    float acc = 0.f;
-    for (int u = tid; u < N * 8; u += 256) {
-      float a[8], d[8];
-      unpack8(*reinterpret_cast<const uint4*>(Ht + u * 16), a);
-      unpack8(*reinterpret_cast<const uint4*>(Dt + u * 16), d);
-#pragma unroll
-      for (int y = 0; y < 8; ++y) acc = fmaf(a[y], d[y], acc);
-    }
-    acc = warp_sum(acc);
-    if (lane == 0) red[warp] = acc;
-  }
-  if (ok) ok = tc::mbar_wait(mbar, 0);
-  tc::fence_after_sync();
-  ok = __all_sync(0xffffffffu, ok);  // warp-uniform: the column sums below shuffle with a full mask
-  float dl_own = 0.f, de_own = 0.f, dg_own = 0.f, zsum = 0.f;
-  const float lt = s.Lam[t], gt = s.gam[t], et = s.e[t], rt = s.r[t], dxt = s.dexp[t];
-  uint4 gmu[2];  // this thread's 16 elements of G*M, until the x tile is dead
-  if (ok) {
-    float fg[16], fd[16];
-    ld_acc16(taddr + 0, warp, tc16, fg);
-    ld_acc16(taddr + 32, warp, tc16, fd);
-    float rs = 0.f, dgc = 0.f;
-    float gm[16], dg[16], ce[16];
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      const float4 l4 = *reinterpret_cast<const float4*>(s.Lam + n16 + 4 * x);
-      const float4 e4 = *reinterpret_cast<const float4*>(s.e + n16 + 4 * x);
-      const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, es[4] = {e4.x, e4.y, e4.z, e4.w};
-#pragma unroll
-      for (int y = 0; y < 4; ++y) {
-        const int q = 4 * x + y, sx = n16 + q;
-        // branch-free so that the exponentials of different columns overlap
-        const bool in = sx <= t;
-        const float Dv = in ? __expf(fminf(lt - ls[y], 0.f)) : 0.f;
-        const float Mv = Dv * (sx < t ? es[y] : gt);
-        const float dGM = in ? fd[q] : 0.f;
-        const float gv = in ? fg[q] : 0.f;
-        gm[q] = gv * Mv;                 // (G*M)_ts
-        dg[q] = dGM * Mv;                // dG_ts
-        const float dM = dGM * gv;
-        const float dw = dM * Dv;
-        rs = fmaf(dM, Mv, rs);
-        dgc += (sx == t) ? dw : 0.f;
-        ce[q] = (sx < t) ? dw : 0.f;     // de_s: column sums
-      }
-    }
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-      gmu[x] = pack8(&gm[8 * x]);
-      sts16(dGt, tc::kmajor_unit(t, 2 * qd + x, Q), pack8(&dg[8 * x]));
-    }
-    colsum16(ce, lane);  // lane l: column l & 15 over the 16 rows of its half
-    const float cs16 = ce[0] + __shfl_xor_sync(0xffffffffu, ce[0], 16);
-    if (lane < 16) csw[(warp & 1) * Q + n16 + lane] = cs16;
-    dl_own = rs;
-    dg_own = dgc;
-    ok = tc::mbar_wait(mbar + 3, 0);
-  }
-  tc::fence_after_sync();
-  float bd[16];  // Brot dH1, used again for dx
-  if (ok) {  // kappa_t = exp(Lam_t) dY_t . (Crot H0)_t   and   zeta_s = (Brot dH1)_s . x_s
-    float f[16];
-    ld_acc16(taddr + 64, warp, tc16, f);
-    ld_acc16(taddr + 96, warp, tc16, bd);
-    dl_own = fmaf(dxt, row_dot16_64<TMA>(Yt, t, n16, f), dl_own);
-    const float zeta = row_dot16_64<TMA>(Xt, t, n16, bd);
-    de_own = rt * zeta;
-    zsum = rt * et * zeta;
-    dl_own -= zsum;
-  }
-  {
-    const float tot = warp_sum(zsum);
-    if (lane == 0) red[8 + warp] = tot;
-  }
-  __syncthreads();  // every read of the x tile is done: G*M may overwrite it
-  if (ok) {
-#pragma unroll
-    for (int x = 0; x < 2; ++x) sts16(GMt, tc::kmajor_unit(t, 2 * qd + x, Q), gmu[x]);
-  }
-  tc::fence_async_smem();
-  tc::fence_before_sync();
-  __syncthreads();
-  tc::fence_after_sync();
-  if (ok && tid == 0) {
-    tc::issue_gemm<true>(taddr + 0, tc::mnmajor_tile(GMt, Q), in_mnmajor<TMA>(Yt, P), 64, P, Q, false);   // (G*M)^T dY
-    tc::issue_gemm<true>(taddr + 192, tc::kmajor_tile(dGt, Q), in_mnmajor<TMA>(Bt, N), 64, N, Q, true);   // + dG Brot
-    tc::mma_commit(mbar);
-    tc::issue_gemm<true>(taddr + 128, tc::mnmajor_tile(dGt, Q), in_mnmajor<TMA>(Ct, N), 64, N, Q, true);  // + dG^T Crot
-    tc::mma_commit(mbar + 3);
-  }
-  if (ok) ok = tc::mbar_wait(mbar, 1);
-  tc::fence_after_sync();
-  ok = __all_sync(0xffffffffu, ok);
-  float dphi_own = 0.f;
-  const float sn = s.sn[t], cs = s.cs[t];
-  // dCrot / dBrot rows: un-rotate into the per-head partial image, and their share of the angle gradient
-  auto put_rows = [&](uint32_t col, const uint8_t* tile, bf16* image) {
-    float f[32];
-    ld_acc32(taddr + col, warp, tc32, f);
-    uint4* dst = reinterpret_cast<uint4*>(image + ci * (N * Q)) + t;
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      float rot[8], o[8];
-      unpack8(*reinterpret_cast<const uint4*>(tile + in_unit<TMA>(t, 4 * qd + x, N)), rot);
-#pragma unroll
-      for (int k = 0; k < 8; k += 2) {
-        const float f0 = f[8 * x + k], f1 = f[8 * x + k + 1];
-        o[k] = cs * f0 - sn * f1;
-        o[k + 1] = sn * f0 + cs * f1;
-        dphi_own += rot[k + 1] * f0 - rot[k] * f1;
-      }
-      dst[(4 * qd + x) * Q] = pack8(o);
-    }
+  bool ok = true;
+  auto wait = [&](uint64_t* m, int parity) { if (ok) ok = tc::mbar_wait(m, (uint32_t)parity & 1u); };
+  auto arrive = [&](uint64_t* m) {  // of a whole warp
+    __syncwarp();
+    if (lane == 0) mbar_arrive(m);
   };
-  if (ok) {
-    {  // dx_s = (G*M)^T dY + r e (Brot dH1)
-      float f[16];
-      ld_acc16(taddr + 0, warp, tc16, f);
-      if (t0 + t < p.T) {
-        const float sc = rt * et;
-#pragma unroll
-        for (int jj = 0; jj < 16; ++jj) f[jj] = fmaf(sc, bd[jj], f[jj]);
-        uint4* dst = reinterpret_cast<uint4*>(p.dx + ((size_t)b * p.T + t0 + t) * p.D + d0 + n16);
-#pragma unroll
-        for (int x = 0; x < 2; ++x) dst[x] = pack8(&f[8 * x]);
+  constexpr uint32_t tZ = 0, tY = 128, tU = 256, tV = 320, tP = 384, tX = 416;
+
+  if (warp == kGradWarps) {  // ---- copies
+    tc::reg_dec<40>();
+    if (TMA) {
+      if (lane == 0) {
+        tc::mbar_expect_tx(tiles, 2 * 16384);
+        for (int sl = 0; sl < 2; ++sl) {
+          tc::tma_load_4d(tc::smem_u32(Bt) + 8192 * sl, &maps.b, 64 * sl, g, t0, b, tiles);
+          tc::tma_load_4d(tc::smem_u32(Ct) + 8192 * sl, &maps.c, 64 * sl, g, t0, b, tiles);
+        }
+      }
+    } else {
+      const size_t row = ((size_t)b * p.T + t0) * p.G + g;
+      for (int sl = 0; sl < 2; ++sl) {
+        stage_slab(tc::smem_u32(Bt) + 8192 * sl, p.b + row * N + 64 * sl, p.T, (size_t)p.G * N, t0, lane, 32);
+        stage_slab(tc::smem_u32(Ct) + 8192 * sl, p.c + row * N + 64 * sl, p.T, (size_t)p.G * N, t0, lane, 32);
+      }
+      tc::cp_async_wait_all();
+      tc::fence_async_smem();
+      mbar_arrive(tiles);
+    }
+    int issued = 0;
+    for (int h = 0; h < nh; ++h) {
+      const int s = h & 1, head = h0 + h;
+      if (h > 1) wait(freed + s, (h >> 1) - 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      uint8_t* S = St + s * kGradStage;
+      if (lane == 0) {
+        tc::mbar_expect_tx(full + s, (uint32_t)kGradStage + (uint32_t)sizeof(ChunkScal) - (TMA ? 0u : 16384u));
+        if (TMA) {
+          tc::tma_load_4d(tc::smem_u32(S), &maps.x, 0, head, t0, b, full + s);
+          tc::tma_load_4d(tc::smem_u32(S) + 8192, &maps.dy, 0, head, t0, b, full + s);
+        }
+        tc::bulk_load(tc::smem_u32(S) + 16384, p.H0 + unit_of(head) * (N * P), 16384, full + s);
+        tc::bulk_load(tc::smem_u32(S) + 32768, p.dH1 + unit_of(head) * (N * P), 16384, full + s);
+        tc::bulk_load(tc::smem_u32(scal + (h & 3)), p.cs + unit_of(head) * (sizeof(ChunkScal) / 4), (uint32_t)sizeof(ChunkScal), full + s);
+      }
+      ++issued;
+      if (!TMA) {
+        const size_t row = (size_t)b * p.T + t0;
+        stage_slab(tc::smem_u32(S), p.x + row * p.D + head * P, p.T, p.D, t0, lane, 32);
+        stage_slab(tc::smem_u32(S) + 8192, p.dy + row * p.D + head * P, p.T, p.D, t0, lane, 32);
+        tc::cp_async_wait_all();
+        tc::fence_async_smem();
+        mbar_arrive(full + s);
       }
     }
-    put_rows(192, Ct, p.pc);
-    ok = tc::mbar_wait(mbar + 3, 1);
+    for (int q = max(0, issued - 2); q < issued; ++q) tc::mbar_wait(full + (q & 1), (q >> 1) & 1);  // (outlive the copies)
+  } else if (warp == kGradWarps + 1) {  // ---- products
+    tc::reg_dec<40>();
+    if (tc::elect_one()) {
+      wait(images, 0);
+      tc::fence_after_sync();
+      if (ok) {
+        tc::issue_gemm<true>(taddr + tP, tc::kmajor_sw128_tile(Ct, 8192), tc::kmajor_sw128_tile(Bt, 8192), 64, Q, N, false);
+        tc::issue_gemm<true>(taddr + tX, tc::kmajor_sw128_tile(Kt, 8192), tc::kmajor_sw128_tile(Bt, 8192), 64, Q, N, false);
+        tc::mma_commit(m0);
+      }
+      for (int h = 0; h < nh && ok; ++h) {
+        const int s = h & 1;
+        uint8_t* S = St + s * kGradStage;
+        wait(full + s, h >> 1);
+        wait(uvfree, h);  // (once more at the start: the first products have been read)
+        tc::fence_after_sync();
+        if (!ok) break;
+        const tc::Tile X = tc::kmajor_sw128_tile(S, 8192), Y = tc::kmajor_sw128_tile(S + 8192, 8192);
+        const tc::Tile H = tc::mnmajor_tile(S + 16384, P), D = tc::mnmajor_tile(S + 32768, P);
+        tc::issue_gemm<true>(taddr + tP, Y, X, 64, Q, P, false);
+        tc::issue_gemm<true>(taddr + tU, tc::kmajor_sw128_tile(Ct, 8192), H, 64, P, N, false);
+        tc::issue_gemm<true>(taddr + tU + 32, tc::kmajor_sw128_tile(Kt, 8192), H, 64, P, N, false);
+        tc::issue_gemm<true>(taddr + tV, tc::kmajor_sw128_tile(Bt, 8192), D, 64, P, N, false);
+        tc::issue_gemm<true>(taddr + tV + 32, tc::kmajor_sw128_tile(Jt, 8192), D, 64, P, N, false);
+        tc::mma_commit(m1);
+        wait(images, h + 1);
+        tc::fence_after_sync();
+        if (!ok) break;
+        tc::issue_gemm(taddr + tZ, tc::kmajor_sw128_tile(Yc, 8192), tc::kmajor_tile(S + 16384, P), 128, N, P, h > 0);
+        tc::issue_gemm(taddr + tY, tc::kmajor_sw128_tile(Xc, 8192), tc::kmajor_tile(S + 32768, P), 128, N, P, h > 0);
+        wait(gready, h);
+        tc::fence_after_sync();
+        if (!ok) break;
+        tc::issue_gemm<true>(taddr + tX, tc::mnmajor_tile(GMt, Q), tc::mnmajor_sw128_tile(S + 8192, 8192), 64, P, Q, false);
+        tc::mma_commit(m2);
+        tc::mma_commit(freed + s);
+      }
+      wait(images, nh + 1);
+      wait(uvfree, nh);
+      tc::fence_after_sync();
+      if (ok) {  // W1, W2 (images over the scaled ones)
+        tc::issue_gemm<true>(taddr + tU, tc::kmajor_tile(Yc, Q), tc::mnmajor_sw128_tile(Bt, 8192), 64, N, Q, false);
+        tc::issue_gemm<true>(taddr + tU, tc::kmajor_tile(Yc + 8192, Q), tc::mnmajor_sw128_tile(Jt, 8192), 64, N, Q, true);
+        tc::issue_gemm<true>(taddr + tV, tc::mnmajor_tile(Yc, Q), tc::mnmajor_sw128_tile(Ct, 8192), 64, N, Q, false);
+        tc::issue_gemm<true>(taddr + tV, tc::mnmajor_tile(Yc + 8192, Q), tc::mnmajor_sw128_tile(Kt, 8192), 64, N, Q, true);
+        tc::mma_commit(m1);
+      }
+    }
+    __syncwarp();
+  } else if (warp == kGradWarps + 2) {  // ---- per-step scalars
+    tc::reg_dec<40>();
+    for (int h = 0; h < nh; ++h) {
+      const ChunkScal& s = scal[h & 3];
+      wait(pready, h);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      auto part_sum = [&](int what, int q) {
+        float v[8];
+#pragma unroll
+        for (int x = 0; x < 8; ++x) v[x] = part[(4 * x + what) * Q + q];
+        return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+      };
+      const int ra = Q - 1 - 2 * lane, rb = ra - 1;
+      const float zra = part_sum(1, ra), zrb = part_sum(1, rb);            // r_s zeta_s
+      const float cea = csw[ra] + csw[Q + ra], ceb = csw[rb] + csw[Q + rb];
+      const float dga = part_sum(2, ra), dgb = part_sum(2, rb);
+      const float dpa = part_sum(3, ra) - (csw[2 * Q + ra] + csw[3 * Q + ra]);
+      const float dpb = part_sum(3, rb) - (csw[2 * Q + rb] + csw[3 * Q + rb]);
+      const float dla = part_sum(0, ra), dlb = part_sum(0, rb);
+      const float hw = lane < kGradWarps ? red[lane] : 0.f;
+      const float ea = s.e[ra], eb = s.e[rb], ga = s.gam[ra], gb = s.gam[rb], L = s.L;
+      arrive(pfree);
+      const float hh = warp_sum(hw), zs = warp_sum(fmaf(ea, zra, eb * zrb));
+      const float base = zs + L * hh;  // d/dLam_end
+      // dLam -> da: reverse in-chunk cumulative sum
+      float a = dla - ea * zra - (ea * cea + ga * dga);
+      float bq = dlb - eb * zrb - (eb * ceb + gb * dgb);
+      warp_rcumsum64(a, bq, lane);
+      const size_t o = ((size_t)b * p.NH + h0 + h) * p.T + t0;
+      if (t0 + ra < p.T) { p.da[o + ra] = base + a; p.de[o + ra] = zra + cea; p.dgam[o + ra] = dga; p.dphi[o + ra] = dpa; }
+      if (t0 + rb < p.T) { p.da[o + rb] = base + bq; p.de[o + rb] = zrb + ceb; p.dgam[o + rb] = dgb; p.dphi[o + rb] = dpb; }
+    }
+  } else if (warp == kGradWarps + 3) {  // ---- dx
+    tc::reg_dec<40>();
+    for (int h = 0; h < nh; ++h) {
+      wait(xready, h);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      if (TMA) {
+        if (lane == 0) {
+          tc::tma_store_4d(&maps.dx, tc::smem_u32(Dx), 0, h0 + h, t0, b);
+          tc::bulk_commit();
+          tc::bulk_wait_read<0>();
+        }
+      } else {
+        for (int u = lane; u < Q * 8; u += 32) {
+          const int t = u >> 3, c8 = u & 7;
+          if (t0 + t < p.T)
+            *reinterpret_cast<uint4*>(p.dx + ((size_t)b * p.T + t0 + t) * p.D + (h0 + h) * P + 8 * c8) =
+                *reinterpret_cast<const uint4*>(Dx + t * 128 + ((c8 ^ (t & 7)) << 4));
+        }
+      }
+      arrive(xfree);
+    }
+  } else if (warp < kGradWarps) {  // ---- rows and columns
+    tc::reg_inc<104>();  // (16 x 104 + 4 x 40 registers a lane, of 20 x 96 at launch)
+    // this thread's row, its 8 of 64 columns of a result and their first TMEM column
+    const int t = 32 * (warp & 1) + lane, tc8 = 8 * (warp >> 2), n8 = 32 * ((warp >> 1) & 1) + tc8, slot = 4 * ((warp >> 1) & 1) + (warp >> 2);
+    wait(tiles, 0);
+    for (int u = tid; u < Q * 16; u += 32 * kGradWarps) {  // J B = (-o, e), CJ = (o, -e) of every pair
+      const uint4 vb = *reinterpret_cast<const uint4*>(Bt + 16 * u), vc = *reinterpret_cast<const uint4*>(Ct + 16 * u);
+      auto sw = [](uint32_t x, uint32_t sign) { return __byte_perm(x, x, 0x1032) ^ sign; };
+      *reinterpret_cast<uint4*>(Jt + 16 * u) = make_uint4(sw(vb.x, 0x8000u), sw(vb.y, 0x8000u), sw(vb.z, 0x8000u), sw(vb.w, 0x8000u));
+      *reinterpret_cast<uint4*>(Kt + 16 * u) =
+          make_uint4(sw(vc.x, 0x80000000u), sw(vc.y, 0x80000000u), sw(vc.z, 0x80000000u), sw(vc.w, 0x80000000u));
+    }
+    tc::fence_async_smem();
+    arrive(images);
+    wait(m0, 0);
+    tc::fence_after_sync();
+    f2 g1[4] = {}, g2[4] = {}, w1[4] = {}, w2[4] = {};  // C B^T, C (J B)^T; the sums over the heads
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok) {
+      ld_pairs(taddr + tP + tc8, warp, g1);
+      ld_pairs(taddr + tX + tc8, warp, g2);
+      tc::tmem_ld_wait();
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {  // (causal part only)
+        const float2 a = unpack2(g1[x]), d = unpack2(g2[x]);
+        const bool in0 = n8 + 2 * x <= t, in1 = n8 + 2 * x + 1 <= t;
+        g1[x] = pack2(in0 ? a.x : 0.f, in1 ? a.y : 0.f);
+        g2[x] = pack2(in0 ? d.x : 0.f, in1 ? d.y : 0.f);
+      }
+    }
+    tc::fence_before_sync();
+    arrive(uvfree);
+    const bool above = n8 > t - lane + 31;               // the warp's rows lie wholly above these columns
+    const bool diagonal = (n8 >> 5) == (warp & 1);        // its rows and columns may meet
+    const uint32_t tunit = (uint32_t)t * 128u + (uint32_t)(((n8 >> 3) ^ (t & 7)) << 4);  // this thread's 16 bytes of a swizzled tile
+    for (int h = 0; h < nh; ++h) {
+      uint8_t* S = St + (h & 1) * kGradStage;
+      const ChunkScal& s = scal[h & 3];
+      wait(full + (h & 1), h >> 1);
+      wait(uvfree, h);  // (nobody reads the images of the head before any more)
+      {  // scaled images: one unit of x and of dY per thread (unit u lies in row u / 8)
+        const int r = tid >> 3;
+        const float sn = s.sn[r], cs = s.cs[r], xd = s.dexp[r], xr = s.re[r];
+        auto put = [&](const uint8_t* src, uint8_t* dst, float sc, float ss) {
+          const uint4 x = *reinterpret_cast<const uint4*>(src + 16 * tid);
+          const f2 v[4] = {widen2(x.x), widen2(x.y), widen2(x.z), widen2(x.w)}, c2 = dup2(sc), s2 = dup2(ss);
+          *reinterpret_cast<uint4*>(dst + 16 * tid) =
+              make_uint4(narrow2(mul2(v[0], c2)), narrow2(mul2(v[1], c2)), narrow2(mul2(v[2], c2)), narrow2(mul2(v[3], c2)));
+          *reinterpret_cast<uint4*>(dst + 8192 + 16 * tid) =
+              make_uint4(narrow2(mul2(v[0], s2)), narrow2(mul2(v[1], s2)), narrow2(mul2(v[2], s2)), narrow2(mul2(v[3], s2)));
+        };
+        put(S + 8192, Yc, xd * cs, xd * sn);
+        put(S, Xc, xr * cs, xr * sn);
+      }
+      tc::fence_async_smem();
+      arrive(images);
+      f2 hh = 0;  // <dH1, H0>: by the warps that have nothing below the diagonal in the product to come
+      if (above) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int u = 16 * (32 * (warp >> 2) + lane + 128 * q);
+          const uint4 a = *reinterpret_cast<const uint4*>(S + 16384 + u), d = *reinterpret_cast<const uint4*>(S + 32768 + u);
+          fma2(hh, widen2(a.x), widen2(d.x));
+          fma2(hh, widen2(a.y), widen2(d.y));
+          fma2(hh, widen2(a.z), widen2(d.z));
+          fma2(hh, widen2(a.w), widen2(d.w));
+        }
+      }
+      wait(m1, h);
+      tc::fence_after_sync();
+      ok = __all_sync(0xffffffffu, ok);
+      const float lt = s.Lam[t], gt = s.gam[t], ct = s.cs[t], st = s.sn[t];
+      float dg = 0.f;
+      f2 dl = 0, dphi = 0, dpm = 0;   // (dphi: sums of what is added and of what is taken away)
+      float ce[8] = {}, cq[8] = {};
+      if (ok) {
+        uint32_t gm[4] = {};
+        if (!above) {
+          f2 fd[4];
+          ld_pairs(taddr + tP + tc8, warp, fd);
+          tc::tmem_ld_wait();
+          const f2 lt2 = dup2(lt), ct2 = dup2(ct), st2 = dup2(st), nct2 = dup2(-ct), one = dup2(-1.f), log2e = dup2(1.4426950408889634f);
+          const int k = t - n8;
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            const ulonglong2 l4 = *reinterpret_cast<const ulonglong2*>(s.Lam + n8 + 4 * x), e4 = *reinterpret_cast<const ulonglong2*>(s.e + n8 + 4 * x);
+            const ulonglong2 c4 = *reinterpret_cast<const ulonglong2*>(s.cs + n8 + 4 * x), s4 = *reinterpret_cast<const ulonglong2*>(s.sn + n8 + 4 * x);
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+              const int z = 2 * x + y, q = 2 * z;
+              const f2 cc = y ? c4.y : c4.x, ss = y ? s4.y : s4.x;
+              const float2 arg = unpack2(mul2(mad2(y ? l4.y : l4.x, one, lt2), log2e)), es = unpack2(y ? e4.y : e4.x), pd = unpack2(fd[z]);
+              // selects, no branches: the exponentials of different columns overlap
+              const f2 D = pack2(q <= k ? ex2(arg.x) : 0.f, q + 1 <= k ? ex2(arg.y) : 0.f);
+              const f2 M = mul2(D, pack2(q < k ? es.x : gt, q + 1 < k ? es.y : gt));
+              const f2 dP = pack2(q <= k ? pd.x : 0.f, q + 1 <= k ? pd.y : 0.f);
+              const f2 cd = mad2(ct2, cc, mul2(st2, ss)), sd = mad2(st2, cc, mul2(nct2, ss));
+              const f2 gv = mad2(cd, g1[z], mul2(sd, g2[z])), gd = mad2(mul2(sd, g1[z]), one, mul2(cd, g2[z]));  // G, dG/ddelta
+              const f2 dG = mul2(dP, M), dM = mul2(dP, gv), dw = mul2(dM, D), qq = mul2(dG, gd);
+              gm[z] = narrow2(mul2(gv, M));
+              fma2(dl, dM, M);
+              dphi = add2(dphi, qq);            // row sums minus column sums
+              fma2(w1[z], dG, cd);
+              fma2(w2[z], dG, sd);
+              const float2 q2 = unpack2(qq), w = unpack2(dw);
+              cq[q] = q2.x; cq[q + 1] = q2.y;
+              ce[q] = w.x; ce[q + 1] = w.y;     // de_s: column sums, without the diagonal
+            }
+          }
+          if (diagonal) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              dg = q == k ? ce[q] : dg;
+              ce[q] = q < k ? ce[q] : 0.f;
+            }
+          }
+        }
+        sts16(GMt, tc::kmajor_unit(t, n8 >> 3, Q), make_uint4(gm[0], gm[1], gm[2], gm[3]));
+      }
+      tc::fence_async_smem();
+      arrive(gready);
+      // U, V: kappa_t = e^Lam dY_t . (Crot H0)_t, zeta_s = x_s . (Brot dH1)_s and their derivatives by the angle.  The latter
+      // are summed over all later steps, where what a state adds to its readers and takes from its writers cancels: both
+      // sides take the rounded images that the states were made of.
+      f2 v[4] = {}, de = 0;
+      wait(images, h + 1);  // (written by other threads)
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) {
+        f2 fa[4], fb[4];
+        auto word = [](const uint4& u, int i) { return i == 0 ? u.x : i == 1 ? u.y : i == 2 ? u.z : u.w; };
+        ld_pairs(taddr + tU + tc8, warp, fa);
+        ld_pairs(taddr + tU + 32 + tc8, warp, fb);
+        uint4 ic = *reinterpret_cast<const uint4*>(Yc + tunit), is = *reinterpret_cast<const uint4*>(Yc + 8192 + tunit);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int z = 0; z < 4; ++z) {
+          const f2 a = widen2(word(ic, z)), e = widen2(word(is, z));
+          fma2(dl, a, fa[z]);
+          fma2(dl, e, fb[z]);
+          fma2(dphi, a, fb[z]);
+          fma2(dpm, e, fa[z]);
+        }
+        ld_pairs(taddr + tV + tc8, warp, fa);
+        ld_pairs(taddr + tV + 32 + tc8, warp, fb);
+        ic = *reinterpret_cast<const uint4*>(Xc + tunit);
+        is = *reinterpret_cast<const uint4*>(Xc + 8192 + tunit);
+        const uint4 ix = *reinterpret_cast<const uint4*>(S + tunit);
+        const f2 ct2 = dup2(ct), nst2 = dup2(-st);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int z = 0; z < 4; ++z) {
+          fma2(dpm, widen2(word(ic, z)), fb[z]);
+          fma2(dpm, widen2(word(is, z)), fa[z]);
+          v[z] = mad2(ct2, fa[z], mul2(nst2, fb[z]));   // Brot = cos B - sin (J B)
+          fma2(de, widen2(word(ix, z)), v[z]);
+        }
+      }
+      tc::fence_before_sync();
+      arrive(uvfree);
+      colsum8(ce, lane);
+      colsum8(cq, lane);
+      const float acc = above ? warp_sum(sum2(hh)) : 0.f;
+      if (h > 0) wait(pfree, h - 1);
+      if (lane < 8) {
+        csw[(warp & 1) * Q + n8 + lane] = ce[0];
+        csw[(2 + (warp & 1)) * Q + n8 + lane] = cq[0];
+      }
+      part[(4 * slot + 0) * Q + t] = sum2(dl);
+      part[(4 * slot + 1) * Q + t] = s.r[t] * sum2(de);
+      part[(4 * slot + 2) * Q + t] = dg;
+      part[(4 * slot + 3) * Q + t] = sum2(dphi) - sum2(dpm);
+      if (lane == 0) red[warp] = acc;
+      arrive(pready);
+      const float ret = s.re[t];
+      wait(m2, h);
+      tc::fence_after_sync();
+      if (h > 0) wait(xfree, h - 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) {  // dx_s = (G*M)^T dY + r e (Brot dH1)
+        f2 f[4];
+        ld_pairs(taddr + tX + tc8, warp, f);
+        tc::tmem_ld_wait();
+        const f2 r2 = dup2(ret);
+        *reinterpret_cast<uint4*>(Dx + tunit) = make_uint4(narrow2(mad2(r2, v[0], f[0])), narrow2(mad2(r2, v[1], f[1])),
+                                                           narrow2(mad2(r2, v[2], f[2])), narrow2(mad2(r2, v[3], f[3])));
+      }
+      tc::fence_before_sync();
+      tc::fence_async_smem();
+      arrive(xready);
+      arrive(freed + (h & 1));
+    }
+    // the sums over the heads
+    wait(uvfree, nh);
+    sts16(Yc, tc::kmajor_unit(t, n8 >> 3, Q), make_uint4(narrow2(w1[0]), narrow2(w1[1]), narrow2(w1[2]), narrow2(w1[3])));
+    sts16(Yc + 8192, tc::kmajor_unit(t, n8 >> 3, Q), make_uint4(narrow2(w2[0]), narrow2(w2[1]), narrow2(w2[2]), narrow2(w2[3])));
+    tc::fence_async_smem();
+    tc::fence_before_sync();
+    arrive(images);
+    // while they meet B and C: the sums over the chunk states, put together over the stages
+    float* Sum = reinterpret_cast<float*>(St);  // [2][64][kGradPitch]: dC, dB
+    auto rows_sync = [] { asm volatile("bar.sync 1, 512;" ::: "memory"); };
+    rows_sync();
+    const int zr = 32 * (warp & 1) + lane, zc = 32 * (warp >> 2);  // row and 32 columns of Z1, Y1 (warps 0, 1 of four) or Z2, Y2
+    for (int pass = 0; pass < 2; ++pass) {
+      if (ok && ((warp >> 1) & 1) == 1 - pass) {
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {
+          float f[32];
+          ld_acc32(taddr + (which ? tY : tZ), warp, zc, f);
+          float4* dst = reinterpret_cast<float4*>(Sum + (which * Q + zr) * kGradPitch + zc);
+#pragma unroll
+          for (int x = 0; x < 8; ++x) {
+            if (pass == 0) {  // J of the sine part
+              dst[x] = make_float4(-f[4 * x + 1], f[4 * x], -f[4 * x + 3], f[4 * x + 2]);
+            } else {
+              const float4 o = dst[x];
+              dst[x] = make_float4(o.x + f[4 * x], o.y + f[4 * x + 1], o.z + f[4 * x + 2], o.w + f[4 * x + 3]);
+            }
+          }
+        }
+      }
+      rows_sync();
+    }
+    wait(m1, nh);
+    tc::fence_after_sync();
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok) {
+      const int c16 = 64 * ((warp >> 1) & 1) + 16 * (warp >> 2);
+      const size_t ui = ((size_t)b * p.G * p.splits + blockIdx.y) * p.n + c;
+#pragma unroll
+      for (int which = 0; which < 2; ++which) {
+        float f[16];
+        ld_acc16(taddr + (which ? tV : tU), warp, 16 * (warp >> 2), f);
+        const float4* src = reinterpret_cast<const float4*>(Sum + (which * Q + t) * kGradPitch + c16);
+        uint4* dst = reinterpret_cast<uint4*>((which ? p.pb : p.pc) + ui * (N * Q)) + t;
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const float4 o = src[x];
+          f[4 * x] += o.x; f[4 * x + 1] += o.y; f[4 * x + 2] += o.z; f[4 * x + 3] += o.w;
+        }
+        dst[(c16 >> 3) * Q] = pack8(f);
+        dst[((c16 >> 3) + 1) * Q] = pack8(f + 8);
+      }
+    }
+    tc::fence_before_sync();
   }
-  tc::fence_after_sync();
-  ok = __all_sync(0xffffffffu, ok);
-  if (ok) put_rows(128, Bt, p.pb);
-  part[(qd * 4 + 0) * Q + t] = dl_own;
-  part[(qd * 4 + 1) * Q + t] = de_own;
-  part[(qd * 4 + 2) * Q + t] = dg_own;
-  part[(qd * 4 + 3) * Q + t] = dphi_own;
-  tc::fence_before_sync();
+  if (!ok && lane == 0) atomicExch(p.status, 13);
   __syncthreads();
-  auto part_sum = [&](int what, int q) {
-    return (part[what * Q + q] + part[(4 + what) * Q + q]) + (part[(8 + what) * Q + q] + part[(12 + what) * Q + q]);
-  };
-  if (tid < 32) {  // dLam -> da: reverse in-chunk cumulative sum (one warp, two rows per lane, fixed order)
-    float zs = 0.f, hh = 0.f;
-    for (int wv = 0; wv < 8; ++wv) { zs += red[8 + wv]; hh += red[wv]; }
-    const float base = zs + s.L * hh;  // d/dLam_end
-    const int ra = Q - 1 - 2 * tid, rb = ra - 1;
-    auto dlam = [&](int q) {
-      return part_sum(0, q) - (s.e[q] * (csw[q] + csw[Q + q]) + s.gam[q] * part_sum(2, q));
-    };
-    float a = dlam(ra), bq = dlam(rb);
-    warp_rcumsum64(a, bq, tid);
-    s.Lam[ra] = base + a;  // Lam is dead by now: reuse for da
-    s.Lam[rb] = base + bq;
-  }
-  __syncthreads();
-  if (!ok && tid == 0) atomicExch(p.status, 13);
-  if (ok && tid < Q && t0 + tid < p.T) {
-    const size_t o = ((size_t)b * p.NH + head) * p.T + t0 + tid;
-    p.da[o] = s.Lam[tid];
-    p.de[o] = part_sum(1, tid) + (csw[tid] + csw[Q + tid]);
-    p.dgam[o] = part_sum(2, tid);
-    p.dphi[o] = part_sum(3, tid);
-  }
-  if (warp == 0) tc::tmem_dealloc(taddr, 256);
+  if (warp == 0) tc::tmem_dealloc(taddr, 512);
 }
 
 
 // ------------------------------------------------------------ final per-token scalars
 __device__ __forceinline__ void final_scalars(const SsdP& p, int head, int b) {
-  __shared__ double wtot[kScalThreads / 32];
+  __shared__ double wtot[2 * kScalThreads / 32];
   __shared__ float wsum[kScalThreads / 32];
   const int tid = threadIdx.x;
   const size_t base = ((size_t)b * p.NH + head) * p.T;
   const float A = -expf(p.a_log[head]);
   const int per = (p.T + kScalThreads - 1) / kScalThreads, lo = tid * per, hi = min(p.T, lo + per);
-  double acc = 0.0;
+  double acc = 0.0, mag = 0.0;
   for (int t0 = lo; t0 < hi; t0 += kScalBatch) {
     float v[kScalBatch];
 #pragma unroll
     for (int x = 0; x < kScalBatch; ++x) v[x] = t0 + x < hi ? p.dphi[base + t0 + x] : 0.f;
 #pragma unroll
-    for (int x = 0; x < kScalBatch; ++x) acc += (double)v[x];
+    for (int x = 0; x < kScalBatch; ++x) {
+      acc += (double)v[x];
+      mag += (double)fabsf(v[x]);
+    }
   }
-  double total;
-  const double incl = cta_scan(acc, wtot, total);
-  double suf = total - incl;  // sum over the threads after this one (exclusive suffix; exact enough in fp64)
+  double incl[2] = {acc, mag}, total[2];
+  cta_scan(incl, wtot, total);
+  double suf = total[0] - incl[0], msuf = total[1] - incl[1];  // sums over the threads after this one (exclusive suffixes; exact enough in fp64)
+  // The outputs depend on differences of angles only, so the terms add up to zero over a sequence.  What they do add up to
+  // is the error of the rounded states; it is taken out where the terms are, in proportion to their size.  The error of a
+  // suffix sum then grows from both ends of the sequence instead of over all of it: dtheta of 2000 steps 0.87 -> 0.5 %.
+  const double share = total[1] > 0.0 ? total[0] / total[1] : 0.0;
   float dal = 0.f;
   // backwards over this thread's steps, kFinalBatch at a time with the loads of a batch ahead of its stores
   constexpr int kFinalBatch = 4;
@@ -934,7 +1209,8 @@ __device__ __forceinline__ void final_scalars(const SsdP& p, int head, int b) {
       const int t = t1 - x;
       if (t >= lo) {
         suf += (double)dph[x];
-        const float dinc = (float)suf;
+        msuf += (double)fabsf(dph[x]);
+        const float dinc = (float)(suf - share * msuf);
         const size_t r = ((size_t)b * p.T + t) * p.NH + head;
         const float dt = dtv[x], lam = lamv[x];
         const float dgam = dgv[x] + dev[x], dnxt = dnv[x], da = dav[x];
@@ -955,19 +1231,19 @@ __device__ __forceinline__ void final_scalars(const SsdP& p, int head, int b) {
     p.dal_part[b * p.NH + head] = A * tot;  // summed over the batch in a fixed order by m3s_dalog_kernel
   }
 }
-// dB[b,t,g,:] = sum over the heads of group g of the per-head partial images (fp32, fixed order).  A thread owns eight
+// dB[b,t,g,:] = sum over the partial images of group g (fp32, fixed order).  A thread owns eight
 // states of a row; consecutive threads hold consecutive rows, which are neighbours in the column-blocked images.
 __device__ __forceinline__ void reduce_rows(const bf16* __restrict__ pb, const bf16* __restrict__ pc, bf16* __restrict__ db,
-                                            bf16* __restrict__ dc, int T, int G, int NH, int n, int block) {
+                                            bf16* __restrict__ dc, int T, int G, int per, int n, int block) {
   static_assert(kScalThreads == N / 8 * Q, "a block covers one chunk of one gradient");
   const int which = block & 1, r = threadIdx.x & 63, c8 = threadIdx.x >> 6;
   int rest = block >> 1;
   const int c = rest % n;
   rest /= n;
-  const int g = rest % G, b = rest / G, per = NH / G, t = c * Q + r;
+  const int g = rest % G, b = rest / G, t = c * Q + r;
   if (t >= T) return;
   const uint4* src = reinterpret_cast<const uint4*>(which ? pc : pb) +
-                     (((size_t)b * NH + (size_t)g * per) * n + c) * (N / 8 * Q) + c8 * Q + r;
+                     (((size_t)b * G + g) * per * n + c) * (N / 8 * Q) + c8 * Q + r;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 8
   for (int h = 0; h < per; ++h) {
@@ -986,7 +1262,7 @@ __device__ __forceinline__ void reduce_rows(const bf16* __restrict__ pb, const b
 __global__ void __launch_bounds__(kScalThreads) m3s_tail_kernel(SsdP p, bf16* __restrict__ db, bf16* __restrict__ dc, int stride) {
   const int nf = p.B * p.NH, block = blockIdx.x, q = block / stride, rem = block - q * stride;
   if (rem == 0 && q < nf) final_scalars(p, q % p.NH, q / p.NH);
-  else reduce_rows(p.pb, p.pc, db, dc, p.T, p.G, p.NH, p.n, block - min(nf, q + 1));
+  else reduce_rows(p.pb, p.pc, db, dc, p.T, p.G, p.splits, p.n, block - min(nf, q + 1));
 }
 __global__ void m3s_dalog_kernel(SsdP p) {
   const int head = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1024,8 +1300,9 @@ static size_t carve_ssd(SsdP& p, void* ws, bool bwd) {
     p.de = cv.take<float>(bh * p.T);
     p.dgam = cv.take<float>(bh * p.T);
     p.dal_part = cv.take<float>(bh);
-    p.pb = cv.take<m3s::bf16>(bh * p.n * m3s::Q * m3s::N);
-    p.pc = cv.take<m3s::bf16>(bh * p.n * m3s::Q * m3s::N);
+    const size_t images = (size_t)p.B * p.G * p.splits * p.n * m3s::Q * m3s::N;
+    p.pb = cv.take<m3s::bf16>(images);
+    p.pc = cv.take<m3s::bf16>(images);
   }
   return cv.bytes();
 }
@@ -1034,6 +1311,14 @@ static SsdP make_ssd(const mxb_mamba3_desc* d) {
   SsdP p{};
   p.B = d->B; p.T = d->T; p.D = d->D; p.G = d->G; p.NH = d->nheads;
   p.n = (d->T + m3s::Q - 1) / m3s::Q;
+  const int per = p.NH / p.G;
+  // Heads per CTA of the chunk-gradient kernel: a CTA costs 7 us and 2.7 us a head, one runs per SM.  Not by the batch, so
+  // that a sequence gives the same bits alone (the partial sums are rounded).  us with 16 / 8 / 4 / 2 heads, chunks x heads of
+  // a sequence: 2048 (8 sequences) 361 / 406 / 676 / -; 512 (8) 105 / 117 / 129 / 174, (2) 54 / 34 / 41 / 54;
+  // 256 (8) 56 / 64 / 76 / 93, (1) 53 / 33 / 23 / 17; 32 (1) - / 32 / 22 / 17.
+  const int u = p.n * p.NH;
+  p.hp = std::min(per, u >= 1024 ? 16 : u >= 512 ? 8 : u >= 256 ? 4 : 2);
+  p.splits = (per + p.hp - 1) / p.hp;
   p.no_tma = (d->flags & MXB_MAMBA3_NO_TMA) ? 1 : 0;
   return p;
 }
@@ -1053,7 +1338,8 @@ static bool ssd_chunk_maps(const SsdP& p, m3s::ChunkMaps& maps) {
   if (p.no_tma) return false;
   bool ok = make_tma_map_bthd(&maps.b, p.b, p.B, p.T, p.G, m3s::N) && make_tma_map_bthd(&maps.c, p.c, p.B, p.T, p.G, m3s::N) &&
             make_tma_map_bthd(&maps.x, p.x, p.B, p.T, p.NH, m3s::P);
-  if (ok && p.dy) ok = make_tma_map_bthd(&maps.dy, p.dy, p.B, p.T, p.NH, m3s::P);
+  if (ok && p.dy)
+    ok = make_tma_map_bthd(&maps.dy, p.dy, p.B, p.T, p.NH, m3s::P) && make_tma_map_bthd(&maps.dx, p.dx, p.B, p.T, p.NH, m3s::P);
   return ok;
 }
 
@@ -1064,15 +1350,20 @@ static mxb_status ssd_state_pass(SsdP& p, int mode, cudaStream_t st) {
   std::memset(&maps, 0, sizeof maps);
   const bool tma = !p.no_tma && make_tma_map_bthd(&maps.r, mode == 0 ? p.b : p.c, p.B, p.T, p.G, m3s::N) &&
                    make_tma_map_bthd(&maps.x, mode == 0 ? p.x : p.dy, p.B, p.T, p.NH, m3s::P);
-  if (tma) {
-    if (MXB_ALLOW_SMEM(m3s::kPassSmem, m3s::m3s_state_pass_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
+  auto launch = [&](auto tma_v, auto ns) {
+    constexpr bool TMA = decltype(tma_v)::value;
+    constexpr int NS = decltype(ns)::value;
+    if (MXB_ALLOW_SMEM(m3s::kPassSmem<NS>, m3s::m3s_state_pass_kernel<TMA, NS>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("m3s_state_pass_kernel", st,
-               (m3s::m3s_state_pass_kernel<true><<<dim3(p.NH, p.B), 256, m3s::kPassSmem, st>>>(p, mode, maps)));
-  } else {
-    if (MXB_ALLOW_SMEM(m3s::kPassSmem, m3s::m3s_state_pass_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
-    MXB_LAUNCH("m3s_state_pass_kernel", st,
-               (m3s::m3s_state_pass_kernel<false><<<dim3(p.NH, p.B), 256, m3s::kPassSmem, st>>>(p, mode, maps)));
-  }
+               (m3s::m3s_state_pass_kernel<TMA, NS><<<dim3(p.NH, p.B), m3s::kPassThreads, m3s::kPassSmem<NS>, st>>>(p, mode, maps)));
+    return MXB_OK;
+  };
+  const std::integral_constant<int, 3> three;
+  const std::integral_constant<int, 6> six;
+  const bool alone = p.NH * p.B <= 148;  // every CTA has an SM of its own
+  const mxb_status s = tma ? (alone ? launch(std::true_type{}, six) : launch(std::true_type{}, three))
+                           : (alone ? launch(std::false_type{}, six) : launch(std::false_type{}, three));
+  if (s != MXB_OK) return s;
   return check_launch("m3s_state_pass_kernel");
 }
 
@@ -1121,16 +1412,16 @@ mxb_status mamba3_ssd_bwd(const mxb_mamba3_desc* d, const void* x, const float* 
     mxb_status s = ssd_forward(p, st);
     if (s != MXB_OK) return s;
   }
-  const dim3 gc(p.n, p.NH, p.B);
+  const dim3 gg(p.n, p.G * p.splits, p.B);
   mxb_status ps = ssd_state_pass(p, 1, st);
   if (ps != MXB_OK) return ps;
   m3s::ChunkMaps maps;
   if (ssd_chunk_maps(p, maps)) {
     if (MXB_ALLOW_SMEM(m3s::kGradSmem, m3s::m3s_chunk_grad_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
-    MXB_LAUNCH("m3s_chunk_grad_kernel", st, (m3s::m3s_chunk_grad_kernel<true><<<gc, 256, m3s::kGradSmem, st>>>(p, maps)));
+    MXB_LAUNCH("m3s_chunk_grad_kernel", st, (m3s::m3s_chunk_grad_kernel<true><<<gg, m3s::kGradThreads, m3s::kGradSmem, st>>>(p, maps)));
   } else {
     if (MXB_ALLOW_SMEM(m3s::kGradSmem, m3s::m3s_chunk_grad_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
-    MXB_LAUNCH("m3s_chunk_grad_kernel", st, (m3s::m3s_chunk_grad_kernel<false><<<gc, 256, m3s::kGradSmem, st>>>(p, maps)));
+    MXB_LAUNCH("m3s_chunk_grad_kernel", st, (m3s::m3s_chunk_grad_kernel<false><<<gg, m3s::kGradThreads, m3s::kGradSmem, st>>>(p, maps)));
   }
   const int nf = p.B * p.NH, tail = nf + 2 * p.n * p.G * p.B;
   MXB_LAUNCH("m3s_tail_kernel", st,

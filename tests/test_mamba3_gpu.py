@@ -294,3 +294,23 @@ def test_sines_and_cosines_of_the_window_kernels(n):
     sn, cs = torch.empty_like(bad), torch.empty_like(bad)
     assert _lib.lib().mxb_selftest_sincos(p(bad), 3, p(sn), p(cs), None) == 0
     assert bool(torch.isnan(sn).all()) and bool(torch.isnan(cs).all())
+
+
+@pytest.mark.parametrize("B,T,NH,G", [(2, 130, 3, 1), (1, 700, 24, 2), (1, 1100, 32, 2), (1, 2800, 24, 1), (160, 65, 1, 1)])
+def test_chunked_kernels_by_heads_per_cta(B, T, NH, G):
+    """2, 4, 8 and 16 heads per CTA of the chunk-gradient kernel, the last CTA of a group with fewer, groups with their own B
+    and C, more (batch, head) pairs than SMs: against the recurrent kernels, which share nothing with them (bf16 tensors)."""
+    from mixlab_b200 import _lib
+    m = inputs.mamba3_inputs(B, T, NH, 64, 128, G=G, seed=40 + NH, io_dtype=torch.bfloat16, per_head=True)
+    dev = [m[k].cuda().contiguous() for k in ("x", "dt_raw", "lambda_raw", "theta", "a_log", "b", "c")]
+    dy = m["dy"].cuda().contiguous()
+    y = ops.mamba3_selective_scan(*dev, nheads=NH, save_for_backward=True)
+    got = ops.mamba3_selective_scan_backward(*dev, dy, nheads=NH, use_saved=True)
+    assert ops.device_status() == 0
+    flags = _lib.MXB_MAMBA3_RECURRENT_KERNELS
+    y_r = ops.mamba3_selective_scan(*dev, nheads=NH, flags=flags)
+    want = ops.mamba3_selective_scan_backward(*dev, dy, nheads=NH, flags=flags)
+    torch.cuda.synchronize()
+    assert_close(y, y_r.double().cpu(), 2e-2, "y")
+    for n in want:
+        assert_close(got[n], want[n].double().cpu(), 2e-2, n)
