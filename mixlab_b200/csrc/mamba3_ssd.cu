@@ -17,7 +17,7 @@
 //   m3s_chunk_scalars_kernel per chunk: decay sums, trapezoid weights, rotation sines/cosines (one record)
 //   m3s_state_pass_kernel   per (b, head), sequential over the chunks, forward or reverse: the chunk contribution
 //                           Brot^T diag(r e) X (or Crot^T diag(exp(Lam)) dY) folded into the running state
-//   m3s_chunk_out_kernel    per chunk and some heads of a group: Y
+//   m3s_chunk_out_kernel    per chunk: Y
 //   m3s_chunk_grad_kernel   per chunk and up to 16 heads of a group: dx, dB, dC summed over these heads, per-token scalars
 //   m3s_tail_kernel         per (b, head): suffix sum of the angle gradient, ddt, dlambda, dtheta, da_log shares; per chunk:
 //                           dB, dC summed over the CTAs of a group
@@ -43,7 +43,6 @@ using tc::unpack8;
 
 struct SsdP {
   int B, T, D, G, NH, n;   // n = chunks
-  int hpo;                 // heads per CTA of the output kernel
   int splits, hp;          // CTAs of the chunk-gradient kernel per group of heads, heads of each (the last one may have fewer)
   int no_tma;              // stage operands with cp.async even where tensor maps can be made
   const bf16 *x, *b, *c, *dy;
@@ -154,6 +153,33 @@ __global__ void __launch_bounds__(64) m3s_chunk_scalars_kernel(SsdP p) {
   uint4* dst = reinterpret_cast<uint4*>(p.cs + ci * (sizeof(ChunkScal) / 4));
   for (int u = tid; u < kScalUnits; u += 64) dst[u] = reinterpret_cast<const uint4*>(&s)[u];
 }
+// cp.async of the record of chunk ci into shared memory (part of the caller's current cp.async group)
+__device__ __forceinline__ void issue_chunk_scalars(const SsdP& p, size_t ci, ChunkScal& s) {
+  const uint32_t sd = tc::smem_u32(&s);
+  const float* src = p.cs + ci * (sizeof(ChunkScal) / 4);
+  for (int u = threadIdx.x; u < kScalUnits; u += blockDim.x) tc::cp_async16(sd + 16 * u, src + 4 * u);
+}
+
+// ---- asynchronous staging: raw cp.async copies into the blocked layout, then in-place fix-ups ----
+// With t = 8 (u / 128) + u % 8 and c8 = (u / 8) % 16 the unit of a [64][128] tile sits at byte 16 u, and
+// likewise for [.][64] tiles with t = 8 (u / 64) + u % 8, c8 = (u / 8) % 8: eight consecutive lanes fill one
+// 128-byte row group (no bank conflicts) and read 64-byte pieces of a row.
+__device__ __forceinline__ void issue_rows_tile(uint8_t* dst, const bf16* src, const SsdP& p, int b, int g, int t0) {
+  const uint32_t sd = tc::smem_u32(dst);
+  for (int u = threadIdx.x; u < Q * 16; u += blockDim.x) {
+    const int t = ((u >> 7) << 3) | (u & 7), c8 = (u >> 3) & 15;
+    const bool ok = t0 + t < p.T;
+    tc::cp_async16(sd + 16 * u, ok ? src + (((size_t)b * p.T + t0 + t) * p.G + g) * N + c8 * 8 : src, ok);
+  }
+}
+__device__ __forceinline__ void issue_x_tile(uint8_t* dst, const bf16* src, const SsdP& p, int b, int d0, int t0) {
+  const uint32_t sd = tc::smem_u32(dst);
+  for (int u = threadIdx.x; u < Q * 8; u += blockDim.x) {
+    const int t = ((u >> 6) << 3) | (u & 7), c8 = (u >> 3) & 7;
+    const bool ok = t0 + t < p.T;
+    tc::cp_async16(sd + 16 * u, ok ? src + ((size_t)b * p.T + t0 + t) * p.D + d0 + c8 * 8 : src, ok);
+  }
+}
 // Rows of a token tensor ([B,T,heads,64] or a 64-column slab of [B,T,G,128]) into a swizzled slab, by threads tid of nt;
 // src: the row of step t0.
 __device__ __forceinline__ void stage_slab(uint32_t dst, const bf16* src, int T, size_t stride, int t0, int tid, int nt) {
@@ -163,9 +189,74 @@ __device__ __forceinline__ void stage_slab(uint32_t dst, const bf16* src, int T,
     tc::cp_async16(dst + (uint32_t)t * 128u + (uint32_t)((c8 ^ (t & 7)) << 4), ok ? src + (size_t)t * stride + c8 * 8 : src, ok);
   }
 }
+// [128 n][64 p] bf16 state saved by the state pass as the byte image of the blocked tile
+__device__ __forceinline__ void issue_state_tile(uint8_t* dst, const bf16* src) {
+  const uint32_t sd = tc::smem_u32(dst);
+  for (int u = threadIdx.x; u < N * 8; u += blockDim.x) tc::cp_async16(sd + 16 * u, src + 8 * u);
+}
+// Rotates the (even, odd) pairs of every row of a landed [64][128] tile in place.
+__device__ __forceinline__ void rotate_tile(uint8_t* tile, const float* sn, const float* cs) {
+  for (int u = threadIdx.x; u < Q * 16; u += blockDim.x) {
+    const int t = ((u >> 7) << 3) | (u & 7);
+    float e[8];
+    unpack8(*reinterpret_cast<const uint4*>(tile + 16 * u), e);
+    const float s_ = sn[t], c_ = cs[t];
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      const float ev = e[k], od = e[k + 1];
+      e[k] = c_ * ev + s_ * od;
+      e[k + 1] = -s_ * ev + c_ * od;
+    }
+    *reinterpret_cast<uint4*>(tile + 16 * u) = pack8(e);
+  }
+}
+// ---- the same fix-ups and views for tiles that the copy engine wrote with 128-byte swizzle (SW = true) ----
+template <bool SW>
+__device__ __forceinline__ uint32_t in_unit(int t, int c8, int W) {
+  return SW ? tc::sw128_unit(t, c8) : tc::kmajor_unit(t, c8, W);
+}
+template <bool SW>
+__device__ __forceinline__ tc::Tile in_kmajor(const void* ptr, int W) {
+  return SW ? tc::kmajor_sw128_tile(ptr, 8192) : tc::kmajor_tile(ptr, W);
+}
+template <bool SW>
+__device__ __forceinline__ tc::Tile in_mnmajor(const void* ptr, int W) {
+  return SW ? tc::mnmajor_sw128_tile(ptr, 8192) : tc::mnmajor_tile(ptr, W);
+}
+template <bool SW>
+__device__ __forceinline__ void rotate_in_tile(uint8_t* tile, const float* sn, const float* cs) {
+  if (!SW) { rotate_tile(tile, sn, cs); return; }
+  // four units per pass, all loads before the first store (a store in between would pin the order of the
+  // loads that follow it); unit w of a slab belongs to row w / 8
+  const int nt = blockDim.x;
+  for (int w0 = threadIdx.x; w0 < Q * 16; w0 += 4 * nt) {
+    uint4 raw[4];
+    float sv[4], cv[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int w = w0 + q * nt, t = (w >> 3) & 63;
+      raw[q] = *reinterpret_cast<const uint4*>(tile + 16 * w);
+      sv[q] = sn[t]; cv[q] = cs[t];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float e[8];
+      unpack8(raw[q], e);
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        const float ev = e[k], od = e[k + 1];
+        e[k] = cv[q] * ev + sv[q] * od;
+        e[k + 1] = -sv[q] * ev + cv[q] * od;
+      }
+      raw[q] = pack8(e);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(tile + 16 * (w0 + q * nt)) = raw[q];
+  }
+}
 struct ChunkMaps {
   CUtensorMap b, c;   // [B,T,G,128] viewed as (N, G, T, B), boxes of 64 columns x 64 steps, 128-byte swizzle
-  CUtensorMap x, dy, dx, y;  // [B,T,heads,64] viewed as (P, heads, T, B)
+  CUtensorMap x, dy, dx;  // [B,T,heads,64] viewed as (P, heads, T, B)
 };
 
 // Threads of the two per-(batch, head) scalar kernels: they are chains of dependent fp64 operations behind strided
@@ -429,271 +520,140 @@ __global__ void __launch_bounds__(kPassThreads, NS == 3 ? 2 : 1) m3s_state_pass_
   if (warp == 0) tc::tmem_dealloc(taddr, 256);
 }
 
-// 8 columns of a result as four pairs.
-__device__ __forceinline__ void ld_pairs(uint32_t taddr, int warp, f2 (&f)[4]) {
-  uint32_t r[8];
-  tc::tmem_ld_32x32b_x8(taddr + ((uint32_t)(32 * (warp & 3)) << 16), r);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) f[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-}
-// J^T of the pairs of unit u of a swizzled tile: (e, o) -> (o, -e).
-__device__ __forceinline__ void put_jt(const uint8_t* src, uint8_t* dst, int u) {
-  const uint4 v = *reinterpret_cast<const uint4*>(src + 16 * u);
-  auto sw = [](uint32_t x) { return __byte_perm(x, x, 0x1032) ^ 0x80000000u; };
-  *reinterpret_cast<uint4*>(dst + 16 * u) = make_uint4(sw(v.x), sw(v.y), sw(v.z), sw(v.w));
-}
-// Columns n8 .. n8 + 7 of row t: zero where they lie above the diagonal.
-__device__ __forceinline__ void causal(f2 (&g1)[4], f2 (&g2)[4], int t, int n8) {
-#pragma unroll
-  for (int x = 0; x < 4; ++x) {
-    const float2 a = unpack2(g1[x]), d = unpack2(g2[x]);
-    const bool in0 = n8 + 2 * x <= t, in1 = n8 + 2 * x + 1 <= t;
-    g1[x] = pack2(in0 ? a.x : 0.f, in1 ? a.y : 0.f);
-    g2[x] = pack2(in0 ? d.x : 0.f, in1 ? d.y : 0.f);
-  }
-}
 // ------------------------------------------------------------ chunk output
-// One CTA per chunk and up to hpo heads of a group, in the manner of the chunk-gradient kernel below: nothing is rotated, the
-// heads share C B^T and C (J B)^T (in registers), and a head adds
-//     y_t = sum_s (G * M)_ts x_s + e^Lam (cos (C H0)_t + sin (CJ H0)_t),   G_ts = cos(delta) (C B^T)_ts + sin(delta) (C (J B)^T)_ts
-// Sixteen warps with a row t and 8 of 64 columns, a warp each for the copies (kOutStages heads ahead), the products and the
-// stores of y.  The warps mask the products of a head while the tensor core works on the head before, whose y they finish
-// then: two of everything between them.  TMEM: U of the two heads [0,128), (G*M) X [128,192), the first products [192,256).
-// 8 x 4096 x 32 heads: 124 us (0.56 GB, 86 us; the rest is the masks, half of the issue slots); one CTA per head and chunk that
-// rotated B and C took 184.
-constexpr int kOutWarps = 16;
-constexpr int kOutThreads = 32 * (kOutWarps + 4);
-constexpr int kOutStages = 4;
-constexpr int kOutStage = 8192 + 16384;  // x, H0 of a head
-constexpr int kOutSmem = 3 * 16384 + kOutStages * (kOutStage + (int)sizeof(ChunkScal)) + 4 * 8192 + (2 * kOutStages + 14) * 8 + 16 + 1024;
-static_assert(kOutSmem <= 227 * 1024, "one CTA per SM");
+// A CTA is a chain of dependent steps, so the kernel is sized for FOUR CTAs per SM: 64 TMEM columns (weight-stationary
+// products: every thread has a row and half of the columns of a result) and 51 KB of shared memory.  The chunk state H0
+// lands in the Brot tile once G = Crot Brot^T has been formed (its copy hides behind the mask epilogue), and Crot H0
+// joins the second MMA batch.  Bound by shared memory (the copies, the rotation in place and the operand reads move
+// about 200 KB per chunk): 8 x 4096 x 32 heads 194 us with half of the lanes idle in the epilogues, 185 now; 256 threads
+// per CTA 188.
+constexpr int kOutSmem = 16384 * 2 + 8192 * 2 + sizeof(ChunkScal) + 64 + 1024;
 
 template <bool TMA>
-__global__ void __launch_bounds__(kOutThreads, 1) m3s_chunk_out_kernel(SsdP p, const __grid_constant__ ChunkMaps maps) {
+__global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __grid_constant__ ChunkMaps maps) {
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
-  uint8_t* Bt = sm;                    // [64][128] B, C, CJ (swizzled slabs)
-  uint8_t* Ct = Bt + 16384;
-  uint8_t* Kt = Ct + 16384;
-  uint8_t* GMt = Kt + 16384;           // x2 [64][64] G*M
-  uint8_t* Yt = GMt + 2 * 8192;        // x2 [64][64] y on its way out (swizzled)
-  uint8_t* St = Yt + 2 * 8192;         // stages: x (swizzled), H0 (image)
-  ChunkScal* scal = reinterpret_cast<ChunkScal*>(St + kOutStages * kOutStage);
-  uint64_t* full = reinterpret_cast<uint64_t*>(scal + kOutStages);  // a head's operands landed
-  uint64_t* freed = full + kOutStages;  // and are no longer needed
-  uint64_t* tiles = freed + kOutStages; // B, C landed
-  uint64_t* images = tiles + 1;         // CJ written
-  uint64_t* m0 = images + 1;            // first products done
-  uint64_t* gready = m0 + 1;            // x2: G*M written (and, a head ago, U and (G*M) X of that buffer read)
-  uint64_t* done = gready + 2;          // x2: products of a head done
-  uint64_t* yready = done + 2;          // x2: y written
-  uint64_t* yfree = yready + 2;         // x2: and gone
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(yfree + 2);
-
+  uint8_t* Bt = sm;               // [64][128] Brot, then [128][64] H0
+  uint8_t* Ct = Bt + 16384;       // [64][128] Crot
+  uint8_t* Ht = Bt;
+  uint8_t* Xt = Ct + 16384;       // [64][64]  x
+  uint8_t* Gm = Xt + 8192;        // [64][64]  (Crot Brot^T) * M
+  ChunkScal& s = *reinterpret_cast<ChunkScal*>(Gm + 8192);
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(&s + 1);  // [0] MMA completion, [1] token tiles landed, [2] H0 landed
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(mbar + 3);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int c = blockIdx.x, b = blockIdx.z, t0 = c * Q;
-  const int per = p.NH / p.G, splits = gridDim.y / p.G, g = blockIdx.y / splits, sp = blockIdx.y % splits;
-  const int h0 = g * per + sp * p.hpo, nh = min(p.hpo, g * per + per - h0);  // this CTA's heads
-  auto unit_of = [&](int head) { return ((size_t)b * p.NH + head) * p.n + c; };
+  const int c = blockIdx.x, head = blockIdx.y, b = blockIdx.z, t0 = c * Q;
+  const int d0 = head * P, g = d0 / (p.D / p.G);
+  const size_t ci = ((size_t)b * p.NH + head) * p.n + c;
 
-  if (warp == 0) { tc::tmem_alloc(tslot, 256); tc::tmem_relinquish(); }
+  if (warp == 0) { tc::tmem_alloc(tslot, 64); tc::tmem_relinquish(); }
+  // the thread that initialises the barriers also issues the copies, on another warp than the TMEM allocation
   if (tid == 32) {
-    for (int s = 0; s < kOutStages; ++s) { tc::mbar_init(full + s, TMA ? 1 : 33); tc::mbar_init(freed + s, kOutWarps + 1); }
-    tc::mbar_init(tiles, TMA ? 1 : 32); tc::mbar_init(images, kOutWarps); tc::mbar_init(m0, 1);
-    for (int s = 0; s < 2; ++s) { tc::mbar_init(gready + s, kOutWarps); tc::mbar_init(done + s, 1); tc::mbar_init(yready + s, kOutWarps); tc::mbar_init(yfree + s, 1); }
+    for (int m = 0; m < 3; ++m) tc::mbar_init(mbar + m, 1);
     tc::mbar_fence_init();
   }
+  bool ok = true;
+  if (TMA) {  // every operand by the copy engine
+    if (tid == 32) {
+      tc::mbar_expect_tx(mbar + 1, 2 * 16384 + 8192 + (uint32_t)sizeof(ChunkScal));
+      for (int sl = 0; sl < 2; ++sl) {
+        tc::tma_load_4d(tc::smem_u32(Bt) + 8192 * sl, &maps.b, 64 * sl, g, t0, b, mbar + 1);
+        tc::tma_load_4d(tc::smem_u32(Ct) + 8192 * sl, &maps.c, 64 * sl, g, t0, b, mbar + 1);
+      }
+      tc::tma_load_4d(tc::smem_u32(Xt), &maps.x, 0, head, t0, b, mbar + 1);
+      tc::bulk_load(tc::smem_u32(&s), p.cs + ci * (sizeof(ChunkScal) / 4), (uint32_t)sizeof(ChunkScal), mbar + 1);
+    }
+    __syncthreads();  // barriers initialised before anyone waits on them
+    ok = tc::mbar_wait(mbar + 1, 0);
+  } else {
+    issue_rows_tile(Bt, p.b, p, b, g, t0);
+    issue_rows_tile(Ct, p.c, p, b, g, t0);
+    issue_x_tile(Xt, p.x, p, b, d0, t0);
+    issue_chunk_scalars(p, ci, s);
+    tc::cp_async_commit();
+    tc::cp_async_wait<0>();
+  }
+  __syncthreads();
+  rotate_in_tile<TMA>(Bt, s.sn, s.cs);
+  rotate_in_tile<TMA>(Ct, s.sn, s.cs);
+  tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t taddr = *tslot;
-  bool ok = true;
-  auto wait = [&](uint64_t* m, int parity) { if (ok) ok = tc::mbar_wait(m, (uint32_t)parity & 1u); };
-  auto arrive = [&](uint64_t* m) {  // of a whole warp
-    __syncwarp();
-    if (lane == 0) mbar_arrive(m);
-  };
-  constexpr uint32_t tU = 0, tG = 128, t1 = 192, t2 = 224;
-
-  if (warp == kOutWarps) {  // ---- copies
-    if (TMA) {
-      if (lane == 0) {
-        tc::mbar_expect_tx(tiles, 2 * 16384);
-        for (int sl = 0; sl < 2; ++sl) {
-          tc::tma_load_4d(tc::smem_u32(Bt) + 8192 * sl, &maps.b, 64 * sl, g, t0, b, tiles);
-          tc::tma_load_4d(tc::smem_u32(Ct) + 8192 * sl, &maps.c, 64 * sl, g, t0, b, tiles);
-        }
-      }
-    } else {
-      const size_t row = ((size_t)b * p.T + t0) * p.G + g;
-      for (int sl = 0; sl < 2; ++sl) {
-        stage_slab(tc::smem_u32(Bt) + 8192 * sl, p.b + row * N + 64 * sl, p.T, (size_t)p.G * N, t0, lane, 32);
-        stage_slab(tc::smem_u32(Ct) + 8192 * sl, p.c + row * N + 64 * sl, p.T, (size_t)p.G * N, t0, lane, 32);
-      }
-      tc::cp_async_wait_all();
-      tc::fence_async_smem();
-      mbar_arrive(tiles);
-    }
-    int issued = 0;
-    for (int h = 0; h < nh; ++h) {
-      const int s = h % kOutStages, head = h0 + h;
-      if (h >= kOutStages) wait(freed + s, h / kOutStages - 1);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      ++issued;
-      uint8_t* S = St + s * kOutStage;
-      if (lane == 0) {
-        tc::mbar_expect_tx(full + s, 16384 + (TMA ? 8192 : 0) + (uint32_t)sizeof(ChunkScal));
-        if (TMA) tc::tma_load_4d(tc::smem_u32(S), &maps.x, 0, head, t0, b, full + s);
-        tc::bulk_load(tc::smem_u32(S) + 8192, p.H0 + unit_of(head) * (N * P), 16384, full + s);
-        tc::bulk_load(tc::smem_u32(scal + s), p.cs + unit_of(head) * (sizeof(ChunkScal) / 4), (uint32_t)sizeof(ChunkScal), full + s);
-      }
-      if (!TMA) {
-        stage_slab(tc::smem_u32(S), p.x + ((size_t)b * p.T + t0) * p.D + head * P, p.T, p.D, t0, lane, 32);
-        tc::cp_async_wait_all();
-        tc::fence_async_smem();
-        mbar_arrive(full + s);
-      }
-    }
-    for (int q = max(0, issued - kOutStages); q < issued; ++q) tc::mbar_wait(full + q % kOutStages, (q / kOutStages) & 1);  // (outlive the copies)
-  } else if (warp == kOutWarps + 1) {  // ---- products
-    if (tc::elect_one()) {
-      wait(images, 0);
-      tc::fence_after_sync();
-      if (ok) {
-        tc::issue_gemm<true>(taddr + t1, tc::kmajor_sw128_tile(Ct, 8192), tc::kmajor_sw128_tile(Bt, 8192), 64, Q, N, false);
-        tc::issue_gemm<true>(taddr + t2, tc::kmajor_sw128_tile(Kt, 8192), tc::kmajor_sw128_tile(Bt, 8192), 64, Q, N, false);
-        tc::mma_commit(m0);
-      }
-      for (int h = 0; h < nh && ok; ++h) {
-        const int s = h % kOutStages, a = h & 1;
-        uint8_t* S = St + s * kOutStage;
-        wait(full + s, h / kOutStages);
-        wait(gready + a, h >> 1);
-        tc::fence_after_sync();
-        if (!ok) break;
-        const tc::Tile H = tc::mnmajor_tile(S + 8192, P);
-        tc::issue_gemm<true>(taddr + tU + 64 * a, tc::kmajor_sw128_tile(Ct, 8192), H, 64, P, N, false);
-        tc::issue_gemm<true>(taddr + tU + 64 * a + 32, tc::kmajor_sw128_tile(Kt, 8192), H, 64, P, N, false);
-        tc::issue_gemm<true>(taddr + tG + 32 * a, tc::kmajor_tile(GMt + 8192 * a, Q), tc::mnmajor_sw128_tile(S, 8192), 64, P, Q, false);
-        tc::mma_commit(done + a);
-        tc::mma_commit(freed + s);
-      }
-    }
-    __syncwarp();
-  } else if (warp == kOutWarps + 2) {  // ---- y
-    for (int h = 0; h < nh; ++h) {
-      const int a = h & 1;
-      wait(yready + a, h >> 1);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      if (TMA) {
-        if (lane == 0) {
-          tc::tma_store_4d(&maps.y, tc::smem_u32(Yt + 8192 * a), 0, h0 + h, t0, b);
-          tc::bulk_commit();
-          tc::bulk_wait_read<0>();
-        }
-      } else {
-        for (int u = lane; u < Q * 8; u += 32) {
-          const int t = u >> 3, c8 = u & 7;
-          if (t0 + t < p.T)
-            *reinterpret_cast<uint4*>(p.y + ((size_t)b * p.T + t0 + t) * p.D + (h0 + h) * P + 8 * c8) =
-                *reinterpret_cast<const uint4*>(Yt + 8192 * a + t * 128 + ((c8 ^ (t & 7)) << 4));
-        }
-      }
-      arrive(yfree + a);
-    }
-  } else if (warp < kOutWarps) {  // ---- rows and columns
-    // this thread's row, its 8 of 64 columns of a result and their first TMEM column
-    const int t = 32 * (warp & 1) + lane, tc8 = 8 * (warp >> 2), n8 = 32 * ((warp >> 1) & 1) + tc8;
-    wait(tiles, 0);
-    for (int u = tid; u < Q * 16; u += 32 * kOutWarps) put_jt(Ct, Kt, u);
-    tc::fence_async_smem();
-    arrive(images);
-    wait(m0, 0);
-    tc::fence_after_sync();
-    f2 g1[4] = {}, g2[4] = {};  // C B^T, C (J B)^T
-    ok = __all_sync(0xffffffffu, ok);
-    if (ok) {
-      ld_pairs(taddr + t1 + tc8, warp, g1);
-      ld_pairs(taddr + t2 + tc8, warp, g2);
-      tc::tmem_ld_wait();
-      causal(g1, g2, t, n8);
-    }
-    const uint32_t tunit = (uint32_t)t * 128u + (uint32_t)(((n8 >> 3) ^ (t & 7)) << 4);  // this thread's 16 bytes of a swizzled tile
-    const bool above = n8 > t - lane + 31;               // the warp's rows lie wholly above these columns
-    float ec[2], es[2];  // e^Lam cos, e^Lam sin of a head and the head before
-    auto mask = [&](int h, const int a) {  // a: h & 1
-      const ChunkScal& s = scal[h % kOutStages];
-      wait(full + h % kOutStages, h / kOutStages);
-      uint32_t gm[4] = {};
-      if (ok && !above) {
-        const float lt = s.Lam[t], gt = s.gam[t], ct = s.cs[t], st = s.sn[t];
-        const f2 lt2 = dup2(lt), ct2 = dup2(ct), st2 = dup2(st), nct2 = dup2(-ct), one = dup2(-1.f), log2e = dup2(1.4426950408889634f);
-        const int k = t - n8;
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          const ulonglong2 l4 = *reinterpret_cast<const ulonglong2*>(s.Lam + n8 + 4 * x), e4 = *reinterpret_cast<const ulonglong2*>(s.e + n8 + 4 * x);
-          const ulonglong2 c4 = *reinterpret_cast<const ulonglong2*>(s.cs + n8 + 4 * x), s4 = *reinterpret_cast<const ulonglong2*>(s.sn + n8 + 4 * x);
-#pragma unroll
-          for (int y = 0; y < 2; ++y) {
-            const int z = 2 * x + y, q = 2 * z;
-            const f2 cc = y ? c4.y : c4.x, ss = y ? s4.y : s4.x;
-            const float2 arg = unpack2(mul2(mad2(y ? l4.y : l4.x, one, lt2), log2e)), w = unpack2(y ? e4.y : e4.x);
-            // selects, no branches: the exponentials of different columns overlap
-            const f2 M = mul2(pack2(q <= k ? ex2(arg.x) : 0.f, q + 1 <= k ? ex2(arg.y) : 0.f), pack2(q < k ? w.x : gt, q + 1 < k ? w.y : gt));
-            const f2 cd = mad2(ct2, cc, mul2(st2, ss)), sd = mad2(st2, cc, mul2(nct2, ss));
-            gm[z] = narrow2(mul2(mad2(cd, g1[z], mul2(sd, g2[z])), M));
-          }
-        }
-      }
-      if (ok) {
-        const float d = s.dexp[t];
-        ec[a] = d * s.cs[t];
-        es[a] = d * s.sn[t];
-      }
-      // (the products that read this buffer two heads ago are done: their y has been made)
-      sts16(GMt + 8192 * a, tc::kmajor_unit(t, n8 >> 3, Q), make_uint4(gm[0], gm[1], gm[2], gm[3]));
-      tc::fence_async_smem();
-      tc::fence_before_sync();
-      arrive(gready + a);
-      arrive(freed + h % kOutStages);
-    };
-    auto finish = [&](int h, const int a) {
-      wait(done + a, h >> 1);
-      tc::fence_after_sync();
-      if (h > 1) wait(yfree + a, (h >> 1) - 1);
-      ok = __all_sync(0xffffffffu, ok);
-      if (ok) {
-        f2 f[4], u1[4], u2[4];
-        ld_pairs(taddr + tG + 32 * a + tc8, warp, f);
-        ld_pairs(taddr + tU + 64 * a + tc8, warp, u1);
-        ld_pairs(taddr + tU + 64 * a + 32 + tc8, warp, u2);
-        tc::tmem_ld_wait();
-        const f2 c2 = dup2(ec[a]), s2 = dup2(es[a]);
-        uint32_t o[4];
-#pragma unroll
-        for (int z = 0; z < 4; ++z) o[z] = narrow2(mad2(c2, u1[z], mad2(s2, u2[z], f[z])));
-        *reinterpret_cast<uint4*>(Yt + 8192 * a + tunit) = make_uint4(o[0], o[1], o[2], o[3]);
-      }
-      tc::fence_async_smem();
-      arrive(yready + a);
-    };
-    for (int h = 0; h < nh; h += 2) {  // (in pairs, so that the indices of two-entry arrays are known)
-      mask(h, 0);
-      if (h > 0) finish(h - 1, 1);
-      if (h + 1 < nh) {
-        mask(h + 1, 1);
-        finish(h, 0);
-      }
-    }
-    if (nh & 1) finish(nh - 1, 0);
-    else finish(nh - 1, 1);
-    tc::fence_before_sync();
+  if (tid == 0) {
+    tc::issue_gemm<true>(taddr, in_kmajor<TMA>(Ct, N), in_kmajor<TMA>(Bt, N), 64, Q, N, false);           // G = Crot Brot^T
+    tc::mma_commit(mbar);
   }
-  if (!ok && lane == 0) atomicExch(p.status, 12);
+  if (ok) ok = tc::mbar_wait(mbar, 0);
+  tc::fence_after_sync();
+  // Brot is dead: the chunk state takes its place while the mask is applied
+  if (TMA) {
+    if (tid == 32) {
+      tc::mbar_expect_tx(mbar + 2, 16384);
+      tc::bulk_load(tc::smem_u32(Ht), p.H0 + ci * (N * P), 16384, mbar + 2);
+    }
+  } else {
+    issue_state_tile(Ht, p.H0 + ci * (N * P));
+    tc::cp_async_commit();
+  }
+  // weight-stationary products: this thread's row, and the half of the columns it holds of every result
+  const int t = 32 * (warp & 1) + lane, n0 = 32 * (warp >> 1);
+  if (ok) {
+    const float lt = s.Lam[t], gt = s.gam[t];
+    float f[32];
+    ld_acc32(taddr, warp, 0, f);
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {  // branch-free, so the exponentials of different columns overlap
+      const float4 l4 = *reinterpret_cast<const float4*>(s.Lam + n0 + 4 * x);
+      const float4 e4 = *reinterpret_cast<const float4*>(s.e + n0 + 4 * x);
+      const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, es[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const int jj = 4 * x + y, sx = n0 + jj;
+        const float mv = __expf(fminf(lt - ls[y], 0.f)) * (sx < t ? es[y] : gt);
+        f[jj] = (sx <= t) ? f[jj] * mv : 0.f;
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) sts16(Gm, tc::kmajor_unit(t, (n0 >> 3) + x, Q), pack8(&f[8 * x]));
+  }
+  if (TMA) { if (ok) ok = tc::mbar_wait(mbar + 2, 0); }  // H0
+  else tc::cp_async_wait<0>();
+  tc::fence_async_smem();
+  tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(taddr, 256);
+  tc::fence_after_sync();
+  if (ok && tid == 0) {
+    tc::issue_gemm<true>(taddr, tc::kmajor_tile(Gm, Q), in_mnmajor<TMA>(Xt, P), 64, P, Q, false);  // (G*M) X, over the consumed G
+    tc::issue_gemm<true>(taddr + 32, in_kmajor<TMA>(Ct, N), tc::mnmajor_tile(Ht, P), 64, P, N, false);    // Crot H0
+    tc::mma_commit(mbar);
+  }
+  if (ok) ok = tc::mbar_wait(mbar, 1);
+  tc::fence_after_sync();
+  if (ok) {  // y = (G*M) X + exp(Lam) Crot H0, assembled over the x tile (dead) and written out in full rows
+    const float de = s.dexp[t];
+    float f[32], f2[32];
+    ld_acc32(taddr, warp, 0, f);
+    ld_acc32(taddr + 32, warp, 0, f2);
+#pragma unroll
+    for (int jj = 0; jj < 32; ++jj) f[jj] = fmaf(de, f2[jj], f[jj]);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) sts16(Xt, tc::kmajor_unit(t, (n0 >> 3) + x, P), pack8(&f[8 * x]));
+  } else if (tid == 0) {
+    atomicExch(p.status, 12);
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (ok) {
+    for (int u = tid; u < Q * 8; u += 128) {  // 64-byte row pieces, conflict-free shared-memory reads
+      const int r = ((u >> 6) << 3) | (u & 7), c8 = (u >> 3) & 7;
+      if (t0 + r < p.T)
+        *reinterpret_cast<uint4*>(p.y + ((size_t)b * p.T + t0 + r) * p.D + d0 + c8 * 8) =
+            *reinterpret_cast<const uint4*>(Xt + 16 * u);
+    }
+  }
+  if (warp == 0) tc::tmem_dealloc(taddr, 64);
 }
 
 // ------------------------------------------------------------ chunk gradients
@@ -726,6 +686,13 @@ static_assert(kGradSmem <= 227 * 1024, "one CTA per SM");
 constexpr int kGradPitch = N + 4;  // floats per row of the sums on their way out (over the stages)
 static_assert(2 * Q * kGradPitch * 4 <= 2 * kGradStage, "two tiles of row sums fit into the stages");
 
+// 8 columns of a result as four pairs.
+__device__ __forceinline__ void ld_pairs(uint32_t taddr, int warp, f2 (&f)[4]) {
+  uint32_t r[8];
+  tc::tmem_ld_32x32b_x8(taddr + ((uint32_t)(32 * (warp & 3)) << 16), r);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+}
 template <bool TMA>
 __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p, const __grid_constant__ ChunkMaps maps) {
   extern __shared__ uint8_t raw[];
@@ -945,10 +912,11 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
     const int t = 32 * (warp & 1) + lane, tc8 = 8 * (warp >> 2), n8 = 32 * ((warp >> 1) & 1) + tc8, slot = 4 * ((warp >> 1) & 1) + (warp >> 2);
     wait(tiles, 0);
     for (int u = tid; u < Q * 16; u += 32 * kGradWarps) {  // J B = (-o, e), CJ = (o, -e) of every pair
-      const uint4 v = *reinterpret_cast<const uint4*>(Bt + 16 * u);
-      auto sw = [](uint32_t x) { return __byte_perm(x, x, 0x1032) ^ 0x8000u; };
-      *reinterpret_cast<uint4*>(Jt + 16 * u) = make_uint4(sw(v.x), sw(v.y), sw(v.z), sw(v.w));
-      put_jt(Ct, Kt, u);
+      const uint4 vb = *reinterpret_cast<const uint4*>(Bt + 16 * u), vc = *reinterpret_cast<const uint4*>(Ct + 16 * u);
+      auto sw = [](uint32_t x, uint32_t sign) { return __byte_perm(x, x, 0x1032) ^ sign; };
+      *reinterpret_cast<uint4*>(Jt + 16 * u) = make_uint4(sw(vb.x, 0x8000u), sw(vb.y, 0x8000u), sw(vb.z, 0x8000u), sw(vb.w, 0x8000u));
+      *reinterpret_cast<uint4*>(Kt + 16 * u) =
+          make_uint4(sw(vc.x, 0x80000000u), sw(vc.y, 0x80000000u), sw(vc.z, 0x80000000u), sw(vc.w, 0x80000000u));
     }
     tc::fence_async_smem();
     arrive(images);
@@ -960,7 +928,13 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       ld_pairs(taddr + tP + tc8, warp, g1);
       ld_pairs(taddr + tX + tc8, warp, g2);
       tc::tmem_ld_wait();
-      causal(g1, g2, t, n8);
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {  // (causal part only)
+        const float2 a = unpack2(g1[x]), d = unpack2(g2[x]);
+        const bool in0 = n8 + 2 * x <= t, in1 = n8 + 2 * x + 1 <= t;
+        g1[x] = pack2(in0 ? a.x : 0.f, in1 ? a.y : 0.f);
+        g2[x] = pack2(in0 ? d.x : 0.f, in1 ? d.y : 0.f);
+      }
     }
     tc::fence_before_sync();
     arrive(uvfree);
@@ -1364,7 +1338,6 @@ static bool ssd_chunk_maps(const SsdP& p, m3s::ChunkMaps& maps) {
   if (p.no_tma) return false;
   bool ok = make_tma_map_bthd(&maps.b, p.b, p.B, p.T, p.G, m3s::N) && make_tma_map_bthd(&maps.c, p.c, p.B, p.T, p.G, m3s::N) &&
             make_tma_map_bthd(&maps.x, p.x, p.B, p.T, p.NH, m3s::P);
-  if (ok && p.y) ok = make_tma_map_bthd(&maps.y, p.y, p.B, p.T, p.NH, m3s::P);
   if (ok && p.dy)
     ok = make_tma_map_bthd(&maps.dy, p.dy, p.B, p.T, p.NH, m3s::P) && make_tma_map_bthd(&maps.dx, p.dx, p.B, p.T, p.NH, m3s::P);
   return ok;
@@ -1402,23 +1375,12 @@ static mxb_status ssd_forward(SsdP& p, cudaStream_t st) {
   if (ps != MXB_OK) return ps;
   if (p.y) {
     m3s::ChunkMaps maps;
-    // Heads per CTA: the fewest waves' time of CTAs that cost 4 us and 0.9 us a head, one per SM (a head's result does not
-    // depend on it).
-    const int per = p.NH / p.G;
-    float best = 0.f;
-    for (int hp = 1; hp < 2 * per; hp *= 2) {
-      const int h = std::min(hp, per);
-      const long ctas = (long)p.n * p.G * ((per + h - 1) / h) * p.B;
-      const float us = (float)((ctas + 147) / 148) * (4.f + 0.9f * (float)h);
-      if (hp == 1 || us < best) { best = us; p.hpo = h; }
-    }
-    const dim3 go(p.n, p.G * ((per + p.hpo - 1) / p.hpo), p.B);
     if (ssd_chunk_maps(p, maps)) {
       if (MXB_ALLOW_SMEM(m3s::kOutSmem, m3s::m3s_chunk_out_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
-      MXB_LAUNCH("m3s_chunk_out_kernel", st, (m3s::m3s_chunk_out_kernel<true><<<go, m3s::kOutThreads, m3s::kOutSmem, st>>>(p, maps)));
+      MXB_LAUNCH("m3s_chunk_out_kernel", st, (m3s::m3s_chunk_out_kernel<true><<<gc, 128, m3s::kOutSmem, st>>>(p, maps)));
     } else {
       if (MXB_ALLOW_SMEM(m3s::kOutSmem, m3s::m3s_chunk_out_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
-      MXB_LAUNCH("m3s_chunk_out_kernel", st, (m3s::m3s_chunk_out_kernel<false><<<go, m3s::kOutThreads, m3s::kOutSmem, st>>>(p, maps)));
+      MXB_LAUNCH("m3s_chunk_out_kernel", st, (m3s::m3s_chunk_out_kernel<false><<<gc, 128, m3s::kOutSmem, st>>>(p, maps)));
     }
   }
   return check_launch("mamba3 ssd forward");
