@@ -19,7 +19,7 @@
 //                           Brot^T diag(r e) X (or Crot^T diag(exp(Lam)) dY) folded into the running state
 //   m3s_chunk_out_kernel    per chunk: Y
 //   m3s_chunk_grad_kernel   per chunk and up to 16 heads of a group: dx, dB, dC summed over these heads, per-token scalars
-//   m3s_tail_kernel         per (b, head): suffix sum of the angle gradient, ddt, dlambda, dtheta, da_log shares; per chunk:
+//   m3s_tail_kernel         per (b, head): ddt, dlambda, dtheta, da_log shares; per chunk:
 //                           dB, dC summed over the CTAs of a group
 #include <cuda.h>
 
@@ -28,6 +28,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "mma_sync.cuh"
 #include "packed.cuh"
 #include "umma_tiles.cuh"
 
@@ -53,7 +54,7 @@ struct SsdP {
   // workspace
   float *dt, *lam, *phi;        // [B,NH,T]
   bf16 *H0, *dH1;               // [B,NH,n,N,P] state at chunk start / state gradient at chunk end
-  float *dphi, *da, *de, *dgam; // [B,NH,T] per-token scalar gradients
+  float *dphi, *da, *de, *dgam; // [B,NH,T] per-token scalar gradients (dphi: of the angle increment of a step)
   float* dal_part;              // [B,NH] per-batch shares of da_log
   float* cs;                    // [B,NH,n] ChunkScal records
   bf16 *pb, *pc;                // [B,G*splits,n] column-blocked [64][128] images: partial dB, dC (summed in fp32 by the tail kernel)
@@ -204,8 +205,8 @@ __device__ __forceinline__ void rotate_tile(uint8_t* tile, const float* sn, cons
 #pragma unroll
     for (int k = 0; k < 8; k += 2) {
       const float ev = e[k], od = e[k + 1];
-      e[k] = c_ * ev + s_ * od;
-      e[k + 1] = -s_ * ev + c_ * od;
+      e[k] = fmaf(c_, ev, s_ * od);
+      e[k + 1] = fmaf(c_, od, -(s_ * ev));
     }
     *reinterpret_cast<uint4*>(tile + 16 * u) = pack8(e);
   }
@@ -224,34 +225,30 @@ __device__ __forceinline__ tc::Tile in_mnmajor(const void* ptr, int W) {
   return SW ? tc::mnmajor_sw128_tile(ptr, 8192) : tc::mnmajor_tile(ptr, W);
 }
 template <bool SW>
-__device__ __forceinline__ void rotate_in_tile(uint8_t* tile, const float* sn, const float* cs) {
+__device__ __forceinline__ void rotate_in_tile(uint8_t* tile, const float* sn, const float* cs, int tid, int nt) {
   if (!SW) { rotate_tile(tile, sn, cs); return; }
   // four units per pass, all loads before the first store (a store in between would pin the order of the
   // loads that follow it); unit w of a slab belongs to row w / 8
-  const int nt = blockDim.x;
-  for (int w0 = threadIdx.x; w0 < Q * 16; w0 += 4 * nt) {
+  for (int w0 = tid; w0 < Q * 16; w0 += 4 * nt) {
     uint4 raw[4];
     float sv[4], cv[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int w = w0 + q * nt, t = (w >> 3) & 63;
+      const int w = min(w0 + q * nt, Q * 16 - 1), t = (w >> 3) & 63;
       raw[q] = *reinterpret_cast<const uint4*>(tile + 16 * w);
       sv[q] = sn[t]; cv[q] = cs[t];
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      float e[8];
-      unpack8(raw[q], e);
-#pragma unroll
-      for (int k = 0; k < 8; k += 2) {
-        const float ev = e[k], od = e[k + 1];
-        e[k] = cv[q] * ev + sv[q] * od;
-        e[k + 1] = -sv[q] * ev + cv[q] * od;
-      }
-      raw[q] = pack8(e);
+      auto rot = [&](uint32_t w) {
+        const float2 v = unpack2(widen2(w));
+        return tc::pack_bf16(fmaf(cv[q], v.x, sv[q] * v.y), fmaf(cv[q], v.y, -(sv[q] * v.x)));
+      };
+      raw[q] = make_uint4(rot(raw[q].x), rot(raw[q].y), rot(raw[q].z), rot(raw[q].w));
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(tile + 16 * (w0 + q * nt)) = raw[q];
+    for (int q = 0; q < 4; ++q)
+      if (w0 + q * nt < Q * 16) *reinterpret_cast<uint4*>(tile + 16 * (w0 + q * nt)) = raw[q];
   }
 }
 struct ChunkMaps {
@@ -262,36 +259,23 @@ struct ChunkMaps {
 // Threads of the two per-(batch, head) scalar kernels: they are chains of dependent fp64 operations behind strided
 // loads, so many short chains (4 steps per thread at T = 4096) hide the latencies that few long ones expose.
 constexpr int kScalThreads = 1024;
-// Inclusive prefix sums of M doubles per thread over a kScalThreads-thread CTA (warp scans + the warp totals, a fixed order);
-// wtot is M x kScalThreads / 32 doubles of shared memory.  Also returns the CTA totals.
-template <int M>
-__device__ __forceinline__ void cta_scan(double (&v)[M], double* wtot, double (&total)[M]) {
+// Inclusive prefix sum of one double per thread over a kScalThreads-thread CTA (warp scans + the warp totals, a fixed
+// order); wtot is kScalThreads / 32 doubles of shared memory.
+__device__ __forceinline__ double cta_scan(double v, double* wtot) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const double t = __shfl_up_sync(0xffffffffu, v[m], o);
-      if (lane >= o) v[m] += t;
-    }
+    const double t = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += t;
   }
-  if (lane == 31) {
-#pragma unroll
-    for (int m = 0; m < M; ++m) wtot[m * (kScalThreads / 32) + warp] = v[m];
-  }
+  if (lane == 31) wtot[warp] = v;
   __syncthreads();
+  double off = 0.0;
 #pragma unroll
-  for (int m = 0; m < M; ++m) {
-    double off = 0.0, tot = 0.0;
-#pragma unroll
-    for (int w = 0; w < kScalThreads / 32; ++w) {
-      const double x = wtot[m * (kScalThreads / 32) + w];
-      if (w < warp) off += x;
-      tot += x;
-    }
-    total[m] = tot;
-    v[m] += off;
+  for (int w = 0; w < kScalThreads / 32; ++w) {
+    if (w < warp) off += wtot[w];
   }
+  return v + off;
 }
 
 // ------------------------------------------------------------ per-(b,head) scalars
@@ -325,9 +309,7 @@ __global__ void __launch_bounds__(kScalThreads) m3s_scalars_kernel(SsdP p) {
       }
     }
   }
-  double incl[1] = {acc}, total[1];
-  cta_scan(incl, wtot, total);
-  double phi = incl[0] - acc;  // angle at the start of this thread's steps
+  double phi = cta_scan(acc, wtot) - acc;  // angle at the start of this thread's steps
   const double two_pi = 6.283185307179586476925, inv_two_pi = 1.0 / two_pi;
   for (int t0 = lo; t0 < hi; t0 += kScalBatch) {
     float dtv[kScalBatch], th[kScalBatch];
@@ -352,19 +334,20 @@ __global__ void __launch_bounds__(kScalThreads) m3s_scalars_kernel(SsdP p) {
 // state in registers (thread = state row n and 32 of its 64 fp32 columns):
 //   mode 0: H0_c = H;  H = L_c H + Brot_c^T diag(r e) X_c          (states at chunk start, for y and the backward)
 //   mode 1: dH1_c = dH; dH = L_c dH + Crot_c^T diag(exp(Lam)) dY_c  (state gradients at chunk end)
-// The rotation goes to the narrow operand, which is scaled anyway: with J^T(e, o) = (o, -e) on every pair of states
-//   Brot^T diag(r e) X = B^T diag(r e cos) X + J^T-rows of (B^T diag(r e sin) X)
-// so a chunk contributes one product of 128 columns, B^T [cosine image | sine image], whose second half is exchanged
-// between the two states of a pair (neighbouring lanes).  It never leaves the SM.  The saved state goes from registers to the
-// byte image of the [128][64] operand tile (eight rows of a unit column are one 128-byte line).
+// The chunk contribution is one M=128 tcgen05 tile that never leaves the SM.  The saved state goes from registers to the byte
+// image of the [128][64] operand tile (eight rows of a unit column are one 128-byte line).
 //
-// Only the update of the state is sequential, so everything before it runs ahead: a warp issues the copies, two warps scale
-// landed tiles to their two images, a warp issues the products into two accumulators by turns, eight warps hold the state,
-// fold in an accumulator and store the state (one sequence of 32 heads x 64 chunks: 49 us, 8 sequences 93; chunk by chunk in
-// one group of warps, with B rotated in place, 84 and 104).  Every hand-over is an mbarrier with a bounded wait; a warp whose wait has run out stops waiting and working but goes through its loop.
-constexpr int kPassThreads = 32 * 12;
+// Only the update of the state is sequential, so everything before it runs ahead: a warp issues the copies, four warps rotate
+// and scale landed tiles in place, a warp issues the products into two accumulators by turns, eight warps hold the state,
+// fold in an accumulator and store the state (one sequence of 32 heads x 64 chunks: 57 us a pass, chunk by chunk in one group
+// of warps 84; 8 sequences 104, where it is the arithmetic of the rotation that counts, 107).  Every hand-over is an mbarrier with a bounded wait; a warp whose wait has run out stops waiting and working but goes through its loop.
+// NS stages in flight: three and four warps that prepare tiles where two CTAs share an SM, six and eight where one has it.
 template <int NS>
-constexpr int kPassSmem = NS * (16384 + 16384) + (NS + 2) * (int)sizeof(ChunkScal) + (4 * NS + 12) * 8 + 16 + 1024;
+constexpr int kPassPrep = NS == 3 ? 4 : 8;
+template <int NS>
+constexpr int kPassThreads = 32 * (10 + kPassPrep<NS>);
+template <int NS>
+constexpr int kPassSmem = NS * (16384 + 8192) + (NS + 2) * (int)sizeof(ChunkScal) + (4 * NS + 12) * 8 + 16 + 1024;
 
 struct PassMaps {
   CUtensorMap r;  // b or c: [B,T,G,128] viewed as (N, G, T, B), boxes of 64 columns x 64 steps, 128-byte swizzle
@@ -372,17 +355,17 @@ struct PassMaps {
 };
 
 // TMA = true: the three operand boxes of a chunk arrive by the copy engine; TMA = false: cp.async staging into the same
-// swizzled positions.  NS: stages in flight; three where two CTAs share an SM.
+// swizzled positions.
 template <bool TMA, int NS>
-__global__ void __launch_bounds__(kPassThreads, NS == 3 ? 2 : 1) m3s_state_pass_kernel(SsdP p, int mode, const __grid_constant__ PassMaps maps) {
+__global__ void __launch_bounds__(kPassThreads<NS>, NS == 3 ? 2 : 1) m3s_state_pass_kernel(SsdP p, int mode, const __grid_constant__ PassMaps maps) {
   constexpr int NC = NS + 2;         // scalar records: the decay is read behind the product
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
-  uint8_t* Rt = sm;                  // xNS [64 s][128 n] B or C rows
-  uint8_t* Xt = Rt + NS * 16384;     // xNS [64 s][64 p] x or dy, then its cosine image; the sine image
-  ChunkScal* scal = reinterpret_cast<ChunkScal*>(Xt + NS * 16384);
+  uint8_t* Rt = sm;                  // xNS [64 s][128 n] B or C rows, rotated in place
+  uint8_t* Xt = Rt + NS * 16384;     // xNS [64 s][64 p] x or dy, scaled in place
+  ChunkScal* scal = reinterpret_cast<ChunkScal*>(Xt + NS * 8192);
   uint64_t* full = reinterpret_cast<uint64_t*>(scal + NC);  // xNS: tiles landed
-  uint64_t* ready = full + NS;       // xNS: images written
+  uint64_t* ready = full + NS;       // xNS: tiles rotated and scaled
   uint64_t* freed = ready + NS;      // xNS: product done
   uint64_t* accfull = freed + NS;    // x2: product done
   uint64_t* accfree = accfull + 2;   // x2: accumulator read
@@ -393,9 +376,9 @@ __global__ void __launch_bounds__(kPassThreads, NS == 3 ? 2 : 1) m3s_state_pass_
   const int d0 = head * P, g = d0 / (p.D / p.G);
   const size_t cbase = ((size_t)b * p.NH + head) * n;
   auto chunk_at = [&](int it) { return mode == 0 ? it : n - 1 - it; };
-  if (warp == 0) { tc::tmem_alloc(tslot, 256); tc::tmem_relinquish(); }
+  if (warp == 0) { tc::tmem_alloc(tslot, 128); tc::tmem_relinquish(); }
   if (tid == 32) {
-    for (int s = 0; s < NS; ++s) { tc::mbar_init(full + s, TMA ? 1 : 33); tc::mbar_init(ready + s, 2); tc::mbar_init(freed + s, 1); }
+    for (int s = 0; s < NS; ++s) { tc::mbar_init(full + s, TMA ? 1 : 33); tc::mbar_init(ready + s, kPassPrep<NS>); tc::mbar_init(freed + s, 1); }
     for (int s = 0; s < 2; ++s) { tc::mbar_init(accfull + s, 1); tc::mbar_init(accfree + s, 8); }
     for (int s = 0; s < NC; ++s) tc::mbar_init(cfree + s, 8);
     tc::mbar_fence_init();
@@ -424,7 +407,7 @@ __global__ void __launch_bounds__(kPassThreads, NS == 3 ? 2 : 1) m3s_state_pass_
         if (TMA) {
           tc::tma_load_4d(tc::smem_u32(Rt + s * 16384), &maps.r, 0, g, c * Q, b, full + s);
           tc::tma_load_4d(tc::smem_u32(Rt + s * 16384) + 8192, &maps.r, 64, g, c * Q, b, full + s);
-          tc::tma_load_4d(tc::smem_u32(Xt + s * 16384), &maps.x, 0, head, c * Q, b, full + s);
+          tc::tma_load_4d(tc::smem_u32(Xt + s * 8192), &maps.x, 0, head, c * Q, b, full + s);
         }
         tc::bulk_load(tc::smem_u32(scal + it % NC), p.cs + (cbase + c) * (sizeof(ChunkScal) / 4), (uint32_t)sizeof(ChunkScal), full + s);
       }
@@ -433,7 +416,7 @@ __global__ void __launch_bounds__(kPassThreads, NS == 3 ? 2 : 1) m3s_state_pass_
         const bf16* rsrc = (mode == 0 ? p.b : p.c) + (row * p.G + g) * N;
         for (int sl = 0; sl < 2; ++sl)
           stage_slab(tc::smem_u32(Rt + s * 16384) + 8192 * sl, rsrc + 64 * sl, p.T, (size_t)p.G * N, c * Q, lane, 32);
-        stage_slab(tc::smem_u32(Xt + s * 16384), (mode == 0 ? p.x : p.dy) + row * p.D + d0, p.T, p.D, c * Q, lane, 32);
+        stage_slab(tc::smem_u32(Xt + s * 8192), (mode == 0 ? p.x : p.dy) + row * p.D + d0, p.T, p.D, c * Q, lane, 32);
         tc::cp_async_wait_all();
         tc::fence_async_smem();
         mbar_arrive(full + s);
@@ -448,43 +431,30 @@ __global__ void __launch_bounds__(kPassThreads, NS == 3 ? 2 : 1) m3s_state_pass_
         if (it > 1) wait(accfree + a, (it >> 1) - 1);
         if (!ok) break;
         tc::fence_after_sync();
-        // [128 n x 2 64 p], contracted over the rows
-        tc::issue_gemm(taddr + 128 * a, tc::mnmajor_sw128_tile(Rt + s * 16384, 8192), tc::mnmajor_sw128_tile(Xt + s * 16384, 8192), 128, 2 * P, Q, false);
+        // [128 n x 64 p] = R^T X, both contracted over their rows
+        tc::issue_gemm(taddr + 64 * a, tc::mnmajor_sw128_tile(Rt + s * 16384, 8192), tc::mnmajor_sw128_tile(Xt + s * 8192, 8192), 128, P, Q, false);
         tc::mma_commit(accfull + a);
         tc::mma_commit(freed + s);
       }
     }
     __syncwarp();
-  } else if (warp >= 10) {  // ---- images of x or dy: a row per thread, four units at a time, loads first
-    const int r = tid - 320;
+  } else if (warp >= 10) {  // ---- rows rotated, x or dy scaled
+    const int u0 = tid - 320;
     for (int it = 0; it < n; ++it) {
       const int st = it % NS;
       wait(full + st, it / NS);
       const ChunkScal& s = scal[it % NC];
-      const float f = mode == 0 ? s.re[r] : s.dexp[r];
-      const f2 c2 = dup2(f * s.cs[r]), s2 = dup2(f * s.sn[r]);
-      uint8_t* X = Xt + st * 16384 + 128 * r;
-#pragma unroll
-      for (int w0 = 0; w0 < 8; w0 += 4) {
-        uint4 x[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) x[q] = *reinterpret_cast<const uint4*>(X + (((w0 + q) ^ (r & 7)) << 4));
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const f2 v[4] = {widen2(x[q].x), widen2(x[q].y), widen2(x[q].z), widen2(x[q].w)};
-          uint8_t* dst = X + (((w0 + q) ^ (r & 7)) << 4);
-          *reinterpret_cast<uint4*>(dst) =
-              make_uint4(narrow2(mul2(v[0], c2)), narrow2(mul2(v[1], c2)), narrow2(mul2(v[2], c2)), narrow2(mul2(v[3], c2)));
-          *reinterpret_cast<uint4*>(dst + 8192) =
-              make_uint4(narrow2(mul2(v[0], s2)), narrow2(mul2(v[1], s2)), narrow2(mul2(v[2], s2)), narrow2(mul2(v[3], s2)));
-        }
+      rotate_in_tile<true>(Rt + st * 16384, s.sn, s.cs, u0, 32 * kPassPrep<NS>);
+      const float* rowscale = mode == 0 ? s.re : s.dexp;
+      for (int u = u0; u < Q * 8; u += 32 * kPassPrep<NS>) {  // unit u lies in row u / 8
+        uint4* unit = reinterpret_cast<uint4*>(Xt + st * 8192 + 16 * u);
+        *unit = tc::scale_bf16x8(*unit, rowscale[u >> 3]);
       }
       tc::fence_async_smem();
       arrive(ready + st);
     }
   } else if (warp < 8) {    // ---- the state: thread = state row and 32 of its 64 columns
     const int nrow = tid & 127, half = tid >> 7;
-    const float sign = nrow & 1 ? -1.f : 1.f;
     float H[32];
 #pragma unroll
     for (int x = 0; x < 32; ++x) H[x] = 0.f;
@@ -498,17 +468,10 @@ __global__ void __launch_bounds__(kPassThreads, NS == 3 ? 2 : 1) m3s_state_pass_
       ok = __all_sync(0xffffffffu, ok);
       const float L = scal[it % NC].L;
       if (ok) {
+        float f[32];
+        ld_acc32(taddr + 64 * a, warp, 32 * half, f);
 #pragma unroll
-        for (int c0 = 0; c0 < 32; c0 += 16) {
-          float f[16], o[16];
-          ld_acc16(taddr + 128 * a + P, warp, 32 * half + c0, o);
-          ld_acc16(taddr + 128 * a, warp, 32 * half + c0, f);
-#pragma unroll
-          for (int jj = 0; jj < 16; ++jj) {
-            f[jj] = fmaf(sign, __shfl_xor_sync(0xffffffffu, o[jj], 1), f[jj]);
-            H[c0 + jj] = fmaf(L, H[c0 + jj], f[jj]);
-          }
-        }
+        for (int jj = 0; jj < 32; ++jj) H[jj] = fmaf(L, H[jj], f[jj]);
       }
       tc::fence_before_sync();
       arrive(accfree + a);
@@ -517,7 +480,7 @@ __global__ void __launch_bounds__(kPassThreads, NS == 3 ? 2 : 1) m3s_state_pass_
   }
   if (!ok && lane == 0) atomicExch(p.status, 11);
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(taddr, 256);
+  if (warp == 0) tc::tmem_dealloc(taddr, 128);
 }
 
 // ------------------------------------------------------------ chunk output
@@ -574,8 +537,8 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
     tc::cp_async_wait<0>();
   }
   __syncthreads();
-  rotate_in_tile<TMA>(Bt, s.sn, s.cs);
-  rotate_in_tile<TMA>(Ct, s.sn, s.cs);
+  rotate_in_tile<TMA>(Bt, s.sn, s.cs, tid, 128);
+  rotate_in_tile<TMA>(Ct, s.sn, s.cs, tid, 128);
   tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
@@ -672,7 +635,7 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
 // issues the products (an elected thread of a warp of its own: 33 cycles an instruction, 60 behind a test of the thread's
 // index), one that finishes the per-step scalars and one that stores dx; everything is handed over by mbarriers.
 // Products of a head: dP = dY X^T, U = {C, CJ} H0, V = {B, JB} dH1 (asked for a head ahead), Z and Y, then dX = (G*M)^T dY.
-// 8 x 4096 x 32 heads: 338 us + 60 for the row sums behind it, 1.0 GB (0.15 ms); a CTA per head and chunk that rotated B and C
+// 8 x 4096 x 32 heads: 349 us + 54 for the row sums behind it, 1.0 GB (0.15 ms); a CTA per head and chunk that rotated B and C
 // took 527 + 118 with 1.5 + 0.6 GB.  A head takes 5.0 k cycles, most of it the arithmetic of the 64 x 64 products (1.3 k), of U
 // and V (0.9 k) and of the scaled images (0.6 k) at half of the issue slots; pairs of columns in packed registers (7.8 k without).
 // TMEM: Z [0,128), Y [128,256), U [256,320), V [320,384), dP [384,416), dX [416,448); at the start C B^T and C (J B)^T in
@@ -680,7 +643,7 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
 constexpr int kGradWarps = 16;
 constexpr int kGradThreads = 32 * (kGradWarps + 4);
 constexpr int kGradStage = 2 * 8192 + 2 * 16384;  // x, dY, H0, dH1 of a head
-constexpr int kGradPart = (8 * 4 * Q + 4 * Q + 32) * 4;
+constexpr int kGradPart = (8 * 4 * Q + 5 * Q + 32) * 4;
 constexpr int kGradSmem = 4 * 16384 + 2 * kGradStage + 4 * 8192 + 8192 + 8192 + kGradPart + 4 * (int)sizeof(ChunkScal) + 24 * 8 + 16 + 1024;
 static_assert(kGradSmem <= 227 * 1024, "one CTA per SM");
 constexpr int kGradPitch = N + 4;  // floats per row of the sums on their way out (over the stages)
@@ -707,9 +670,10 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
   uint8_t* Dx = GMt + 8192;            // [64][64] dx on its way out (swizzled)
   uint8_t* St = Dx + 8192;             // two stages: x, dY (swizzled), H0, dH1 (images)
   ChunkScal* scal = reinterpret_cast<ChunkScal*>(St + 2 * kGradStage);  // x4: the scalars of a head (read longer than its tiles)
-  float* part = reinterpret_cast<float*>(scal + 4);  // [8 column groups][4][Q]: dLam, de, dgam, dphi row partials
+  float* part = reinterpret_cast<float*>(scal + 4);  // [8 column groups][4][Q]: dLam, de, dphi (negative: by the states read), dphi row partials
   float* csw = part + 8 * 4 * Q;       // [2][2][Q] column sums over the two halves of the rows: of dM*D (s < t), of dG dG/ddelta
-  float* red = csw + 4 * Q;            // [16] <dH1, H0> per warp
+  float* dgs = csw + 4 * Q;            // [Q] dgam
+  float* red = dgs + Q;                // [16] <dH1, H0>, [16] <dH1, J H0> per warp
   uint64_t* full = reinterpret_cast<uint64_t*>(red + 32);  // x2: a head's operands landed
   uint64_t* freed = full + 2;          // x2: and are no longer needed
   uint64_t* tiles = freed + 2;         // B, C landed
@@ -867,19 +831,25 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       const int ra = Q - 1 - 2 * lane, rb = ra - 1;
       const float zra = part_sum(1, ra), zrb = part_sum(1, rb);            // r_s zeta_s
       const float cea = csw[ra] + csw[Q + ra], ceb = csw[rb] + csw[Q + rb];
-      const float dga = part_sum(2, ra), dgb = part_sum(2, rb);
-      const float dpa = part_sum(3, ra) - (csw[2 * Q + ra] + csw[3 * Q + ra]);
-      const float dpb = part_sum(3, rb) - (csw[2 * Q + rb] + csw[3 * Q + rb]);
+      const float dga = dgs[ra], dgb = dgs[rb], bsa = part_sum(2, ra), bsb = part_sum(2, rb);
+      float dpa = part_sum(3, ra) - bsa - (csw[2 * Q + ra] + csw[3 * Q + ra]);
+      float dpb = part_sum(3, rb) - bsb - (csw[2 * Q + rb] + csw[3 * Q + rb]);
       const float dla = part_sum(0, ra), dlb = part_sum(0, rb);
-      const float hw = lane < kGradWarps ? red[lane] : 0.f;
+      const float hw = red[lane];
       const float ea = s.e[ra], eb = s.e[rb], ga = s.gam[ra], gb = s.gam[rb], L = s.L;
       arrive(pfree);
-      const float hh = warp_sum(hw), zs = warp_sum(fmaf(ea, zra, eb * zrb));
+      const float hh = warp_sum(lane < kGradWarps ? hw : 0.f), later = warp_sum((lane < kGradWarps ? 0.f : L * hw) + (bsa + bsb));
+      const float zs = warp_sum(fmaf(ea, zra, eb * zrb));
       const float base = zs + L * hh;  // d/dLam_end
       // dLam -> da: reverse in-chunk cumulative sum
       float a = dla - ea * zra - (ea * cea + ga * dga);
       float bq = dlb - eb * zrb - (eb * ceb + gb * dgb);
       warp_rcumsum64(a, bq, lane);
+      // and dphi -> the sum over this and all later steps, which is what theta and dt get: later steps enter through the states
+      // at the end of the chunk (summed up step by step, the error of the rounded states grew with the length of the sequence)
+      warp_rcumsum64(dpa, dpb, lane);
+      dpa += later;
+      dpb += later;
       const size_t o = ((size_t)b * p.NH + h0 + h) * p.T + t0;
       if (t0 + ra < p.T) { p.da[o + ra] = base + a; p.de[o + ra] = zra + cea; p.dgam[o + ra] = dga; p.dphi[o + ra] = dpa; }
       if (t0 + rb < p.T) { p.da[o + rb] = base + bq; p.de[o + rb] = zrb + ceb; p.dgam[o + rb] = dgb; p.dphi[o + rb] = dpb; }
@@ -962,16 +932,27 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       }
       tc::fence_async_smem();
       arrive(images);
-      f2 hh = 0;  // <dH1, H0>: by the warps that have nothing below the diagonal in the product to come
+      float hh = 0.f, jj = 0.f;  // <dH1, H0> and <dH1, J H0>
+      // By the warps that have nothing below the diagonal in the product to come: blocks of 16 state rows of dH1 times the same rows of H0 (mma.sync), whose diagonals and their neighbours are the row products that are wanted.
       if (above) {
+        const uint32_t sh = tc::smem_u32(S + 16384), sd = sh + 16384;
+        float d1[4] = {}, d2[4] = {};
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int u = 16 * (32 * (warp >> 2) + lane + 128 * q);
-          const uint4 a = *reinterpret_cast<const uint4*>(S + 16384 + u), d = *reinterpret_cast<const uint4*>(S + 32768 + u);
-          fma2(hh, widen2(a.x), widen2(d.x));
-          fma2(hh, widen2(a.y), widen2(d.y));
-          fma2(hh, widen2(a.z), widen2(d.z));
-          fma2(hh, widen2(a.w), widen2(d.w));
+        for (int blk = 0; blk < 2; ++blk)
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks) {
+            const uint32_t u = tc::kmajor_unit(32 * (warp >> 2) + 16 * blk + (lane & 15), 2 * ks + (lane >> 4), P);
+            uint32_t a[4], o[4];
+            ms::ldsm(a, sd + u);
+            ms::ldsm(o, sh + u);
+            ms::mma(d1, a, o[0], o[2]);  // rows 0-7 of H0: wanted in rows 0-7 of the block
+            ms::mma(d2, a, o[1], o[3]);  // rows 8-15
+          }
+        // (sums over both blocks) this lane has row lane / 4 and columns 2 (lane % 4), + 1
+        if ((lane >> 3) == (lane & 3)) {
+          const bool odd = (lane >> 2) & 1;
+          hh = odd ? d1[1] + d2[3] : d1[0] + d2[2];
+          jj = odd ? d1[0] + d2[2] : -(d1[1] + d2[3]);
         }
       }
       wait(m1, h);
@@ -979,7 +960,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       ok = __all_sync(0xffffffffu, ok);
       const float lt = s.Lam[t], gt = s.gam[t], ct = s.cs[t], st = s.sn[t];
       float dg = 0.f;
-      f2 dl = 0, dphi = 0, dpm = 0;   // (dphi: sums of what is added and of what is taken away)
+      f2 dl = 0, dphi = 0, dpm = 0, dpb = 0;   // (dphi: sums of what is added and of what is taken away)
       float ce[8] = {}, cq[8] = {};
       if (ok) {
         uint32_t gm[4] = {};
@@ -1027,9 +1008,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       }
       tc::fence_async_smem();
       arrive(gready);
-      // U, V: kappa_t = e^Lam dY_t . (Crot H0)_t, zeta_s = x_s . (Brot dH1)_s and their derivatives by the angle.  The latter
-      // are summed over all later steps, where what a state adds to its readers and takes from its writers cancels: both
-      // sides take the rounded images that the states were made of.
+      // U, V: kappa_t = e^Lam dY_t . (Crot H0)_t, zeta_s = x_s . (Brot dH1)_s and their derivatives by the angle
       f2 v[4] = {}, de = 0;
       wait(images, h + 1);  // (written by other threads)
       ok = __all_sync(0xffffffffu, ok);
@@ -1057,8 +1036,8 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
         tc::tmem_ld_wait();
 #pragma unroll
         for (int z = 0; z < 4; ++z) {
-          fma2(dpm, widen2(word(ic, z)), fb[z]);
-          fma2(dpm, widen2(word(is, z)), fa[z]);
+          fma2(dpb, widen2(word(ic, z)), fb[z]);
+          fma2(dpb, widen2(word(is, z)), fa[z]);
           v[z] = mad2(ct2, fa[z], mul2(nst2, fb[z]));   // Brot = cos B - sin (J B)
           fma2(de, widen2(word(ix, z)), v[z]);
         }
@@ -1067,7 +1046,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       arrive(uvfree);
       colsum8(ce, lane);
       colsum8(cq, lane);
-      const float acc = above ? warp_sum(sum2(hh)) : 0.f;
+      const float acc = above ? warp_sum(hh) : 0.f, accj = above ? warp_sum(jj) : 0.f;
       if (h > 0) wait(pfree, h - 1);
       if (lane < 8) {
         csw[(warp & 1) * Q + n8 + lane] = ce[0];
@@ -1075,9 +1054,13 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       }
       part[(4 * slot + 0) * Q + t] = sum2(dl);
       part[(4 * slot + 1) * Q + t] = s.r[t] * sum2(de);
-      part[(4 * slot + 2) * Q + t] = dg;
+      part[(4 * slot + 2) * Q + t] = sum2(dpb);
+      if ((t >> 3) == (n8 >> 3)) dgs[t] = dg;
       part[(4 * slot + 3) * Q + t] = sum2(dphi) - sum2(dpm);
-      if (lane == 0) red[warp] = acc;
+      if (lane == 0) {
+        red[warp] = acc;
+        red[kGradWarps + warp] = accj;
+      }
       arrive(pready);
       const float ret = s.re[t];
       wait(m2, h);
@@ -1160,30 +1143,11 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
 
 // ------------------------------------------------------------ final per-token scalars
 __device__ __forceinline__ void final_scalars(const SsdP& p, int head, int b) {
-  __shared__ double wtot[2 * kScalThreads / 32];
   __shared__ float wsum[kScalThreads / 32];
   const int tid = threadIdx.x;
   const size_t base = ((size_t)b * p.NH + head) * p.T;
   const float A = -expf(p.a_log[head]);
   const int per = (p.T + kScalThreads - 1) / kScalThreads, lo = tid * per, hi = min(p.T, lo + per);
-  double acc = 0.0, mag = 0.0;
-  for (int t0 = lo; t0 < hi; t0 += kScalBatch) {
-    float v[kScalBatch];
-#pragma unroll
-    for (int x = 0; x < kScalBatch; ++x) v[x] = t0 + x < hi ? p.dphi[base + t0 + x] : 0.f;
-#pragma unroll
-    for (int x = 0; x < kScalBatch; ++x) {
-      acc += (double)v[x];
-      mag += (double)fabsf(v[x]);
-    }
-  }
-  double incl[2] = {acc, mag}, total[2];
-  cta_scan(incl, wtot, total);
-  double suf = total[0] - incl[0], msuf = total[1] - incl[1];  // sums over the threads after this one (exclusive suffixes; exact enough in fp64)
-  // The outputs depend on differences of angles only, so the terms add up to zero over a sequence.  What they do add up to
-  // is the error of the rounded states; it is taken out where the terms are, in proportion to their size.  The error of a
-  // suffix sum then grows from both ends of the sequence instead of over all of it: dtheta of 2000 steps 0.87 -> 0.5 %.
-  const double share = total[1] > 0.0 ? total[0] / total[1] : 0.0;
   float dal = 0.f;
   // backwards over this thread's steps, kFinalBatch at a time with the loads of a batch ahead of its stores
   constexpr int kFinalBatch = 4;
@@ -1208,9 +1172,7 @@ __device__ __forceinline__ void final_scalars(const SsdP& p, int head, int b) {
     for (int x = 0; x < kFinalBatch; ++x) {
       const int t = t1 - x;
       if (t >= lo) {
-        suf += (double)dph[x];
-        msuf += (double)fabsf(dph[x]);
-        const float dinc = (float)(suf - share * msuf);
+        const float dinc = dph[x];
         const size_t r = ((size_t)b * p.T + t) * p.NH + head;
         const float dt = dtv[x], lam = lamv[x];
         const float dgam = dgv[x] + dev[x], dnxt = dnv[x], da = dav[x];
@@ -1355,7 +1317,7 @@ static mxb_status ssd_state_pass(SsdP& p, int mode, cudaStream_t st) {
     constexpr int NS = decltype(ns)::value;
     if (MXB_ALLOW_SMEM(m3s::kPassSmem<NS>, m3s::m3s_state_pass_kernel<TMA, NS>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("m3s_state_pass_kernel", st,
-               (m3s::m3s_state_pass_kernel<TMA, NS><<<dim3(p.NH, p.B), m3s::kPassThreads, m3s::kPassSmem<NS>, st>>>(p, mode, maps)));
+               (m3s::m3s_state_pass_kernel<TMA, NS><<<dim3(p.NH, p.B), m3s::kPassThreads<NS>, m3s::kPassSmem<NS>, st>>>(p, mode, maps)));
     return MXB_OK;
   };
   const std::integral_constant<int, 3> three;
