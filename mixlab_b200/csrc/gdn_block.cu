@@ -189,6 +189,7 @@ struct PreMap {
 // grid (head blocks, time tiles, streams x B from z0 on)
 template <typename IO, int LPR>
 __global__ void __launch_bounds__(256) gdn_block_pre_fwd_kernel(BlockP p, PreArgs<IO> a, int run, int first, int z0) {
+  begin_dependent();
   const int which = first + (z0 + blockIdx.z) / p.B, b = (z0 + blockIdx.z) % p.B;
   const int D = which == 2 ? p.Dv : p.Dk, C = p.H * D;
   const PreMap m = PreMap::make<LPR>(p.H, D, run);
@@ -262,6 +263,7 @@ __global__ void __launch_bounds__(256) gdn_block_gate_fwd_kernel(BlockP p, const
                                                                  const float* __restrict__ a_log,
                                                                  const float* __restrict__ dt_bias,
                                                                  float* __restrict__ beta, float* __restrict__ gate) {
+  begin_dependent();
   const size_t n = (size_t)p.B * p.T * p.H;
   for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
     const int h = (int)(i % p.H);
@@ -279,6 +281,7 @@ __global__ void __launch_bounds__(256) gdn_block_gate_fwd_kernel(BlockP p, const
 // weight gradients, seven inputs and seven ds of four channels exceed: the compiler spills about 180 bytes of them.
 template <typename IO, int LPR>
 __global__ void __launch_bounds__(256, 2) gdn_block_pre_bwd_kernel(BlockP p, PreArgs<IO> a, int run, int first, int z0) {
+  begin_dependent();
   extern __shared__ __align__(16) uint8_t pre_smem[];
   __shared__ float red[kPreRuns][4][256];
   const int which = first + (z0 + blockIdx.z) / p.B, b = (z0 + blockIdx.z) % p.B;
@@ -450,6 +453,7 @@ struct ColSums {
   int rows[5], n[5], first[6], count;
 };
 __global__ void __launch_bounds__(256) gdn_block_colsum_kernel(ColSums c) {
+  begin_dependent();
   __shared__ float red[8][32];
   int g = 0;
   while (g + 1 < c.count && (int)blockIdx.x >= c.first[g + 1]) ++g;
@@ -480,6 +484,7 @@ __global__ void __launch_bounds__(256) gdn_block_gate_bwd_kernel(BlockP p, const
                                                                  const float* __restrict__ dgate,
                                                                  float* __restrict__ da_raw, float* __restrict__ db_raw,
                                                                  float* __restrict__ da_log, float* __restrict__ ddt_bias) {
+  begin_dependent();
   __shared__ float red[2][8];
   const int h = blockIdx.x, tid = threadIdx.x;
   const float A = expf(a_log[h]), bias = dt_bias[h];
@@ -521,6 +526,7 @@ __global__ void __launch_bounds__(256) gdn_block_gate_bwd_flat_kernel(BlockP p, 
                                                                       float* __restrict__ da_raw,
                                                                       float* __restrict__ db_raw,
                                                                       float* __restrict__ part) {
+  begin_dependent();
   __shared__ float red[2][256];
   const int tid = threadIdx.x, h = tid % p.H;
   const float A = expf(a_log[h]), bias = dt_bias[h];
@@ -563,6 +569,7 @@ template <typename IO, int LPR>
 __global__ void __launch_bounds__(128) gdn_block_post_fwd_kernel(BlockP p, const IO* __restrict__ o,
                                                                  const IO* __restrict__ z,
                                                                  const float* __restrict__ wn, IO* __restrict__ y) {
+  begin_dependent();
   constexpr int kRows = 128 / LPR;  // rows of a CTA
   const int D = p.Dv, l = threadIdx.x % LPR;
   const bool act = l * 8 < D;
@@ -600,6 +607,7 @@ __global__ void __launch_bounds__(128) gdn_block_post_bwd_kernel(BlockP p, const
                                                                  const float* __restrict__ wn,
                                                                  const IO* __restrict__ dy, IO* __restrict__ d_o,
                                                                  IO* __restrict__ dz, float* __restrict__ dwp) {
+  begin_dependent();
   constexpr int kRows = 128 / LPR;
   __shared__ float red[kRows][8 * LPR];
   const int D = p.Dv, l = threadIdx.x % LPR;
@@ -743,13 +751,13 @@ static mxb_status blk_pre_fwd(const mxb_gdn_desc* d, const void* qp, const void*
     with_lanes(lanes, [&](auto lpr) {
       constexpr int LPR = decltype(lpr)::value;
       if constexpr (LPR >= 4)
-        MXB_LAUNCH("gdn_block_pre_fwd_kernel", st, (blk::gdn_block_pre_fwd_kernel<IO, LPR><<<grid, 256, 0, st>>>(p, a, run, first, z0)));
+        MXB_LAUNCH("gdn_block_pre_fwd_kernel", st, (launch_kernel(blk::gdn_block_pre_fwd_kernel<IO, LPR>, grid, 256, 0, st, p, a, run, first, z0)));
     });
   });
   const size_t n = (size_t)d->B * d->T * d->H;
   const int gb = (int)((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8);
   MXB_LAUNCH("gdn_block_gate_fwd_kernel", st,
-             (blk::gdn_block_gate_fwd_kernel<<<gb, 256, 0, st>>>(p, a_raw, b_raw, a_log, dt_bias, beta, gate)));
+             (launch_kernel(blk::gdn_block_gate_fwd_kernel, gb, 256, 0, st, p, a_raw, b_raw, a_log, dt_bias, beta, gate)));
   return check_launch("gdn_block_pre_fwd");
 }
 mxb_status gdn_block_pre_fwd(const mxb_gdn_desc* d, const void* qp, const void* kp, const void* vp, const float* cq,
@@ -786,7 +794,7 @@ static mxb_status blk_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void*
         if (s == MXB_OK) s = MXB_ALLOW_SMEM(blk::PreRing<IO>::kBytes, blk::gdn_block_pre_bwd_kernel<IO, LPR>);
         if (s == MXB_OK)
           MXB_LAUNCH("gdn_block_pre_bwd_kernel", st,
-                     (blk::gdn_block_pre_bwd_kernel<IO, LPR><<<grid, 256, blk::PreRing<IO>::kBytes, st>>>(p, a, run, first, z0)));
+                     (launch_kernel(blk::gdn_block_pre_bwd_kernel<IO, LPR>, grid, 256, blk::PreRing<IO>::kBytes, st, p, a, run, first, z0)));
       }
     });
   });
@@ -804,16 +812,16 @@ static mxb_status blk_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void*
     const int gc = blk_gate_ctas(d);
     float* gpart = base + rows * 4 * (2 * Ck + Cv);
     MXB_LAUNCH("gdn_block_gate_bwd_flat_kernel", st,
-               (blk::gdn_block_gate_bwd_flat_kernel<<<gc, 256, 0, st>>>(p, a_raw, b_raw, a_log, dt_bias, dbeta, dgate,
+               (launch_kernel(blk::gdn_block_gate_bwd_flat_kernel, gc, 256, 0, st, p, a_raw, b_raw, a_log, dt_bias, dbeta, dgate,
                                                                        da_raw, db_raw, gpart)));
     sum(gpart, gc, d->H, da_log);
     sum(gpart + (size_t)gc * d->H, gc, d->H, ddt_bias);
   } else {
     MXB_LAUNCH("gdn_block_gate_bwd_kernel", st,
-               (blk::gdn_block_gate_bwd_kernel<<<d->H, 256, 0, st>>>(p, a_raw, b_raw, a_log, dt_bias, dbeta, dgate,
+               (launch_kernel(blk::gdn_block_gate_bwd_kernel, d->H, 256, 0, st, p, a_raw, b_raw, a_log, dt_bias, dbeta, dgate,
                                                                       da_raw, db_raw, da_log, ddt_bias)));
   }
-  MXB_LAUNCH("gdn_block_colsum_kernel", st, (blk::gdn_block_colsum_kernel<<<c.first[c.count], 256, 0, st>>>(c)));
+  MXB_LAUNCH("gdn_block_colsum_kernel", st, (launch_kernel(blk::gdn_block_colsum_kernel, c.first[c.count], 256, 0, st, c)));
   return check_launch("gdn_block_pre_bwd");
 }
 mxb_status gdn_block_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void* kp, const void* vp, const float* cq,
@@ -840,8 +848,7 @@ static mxb_status blk_post(const mxb_gdn_desc* d, const void* o, const void* z, 
       constexpr int LPR = decltype(lpr)::value;
       if constexpr (LPR <= 16)
         MXB_LAUNCH("gdn_block_post_fwd_kernel", st,
-                   (blk::gdn_block_post_fwd_kernel<IO, LPR><<<ctas, 128, 0, st>>>(
-                       p, static_cast<const IO*>(o), static_cast<const IO*>(z), wn, static_cast<IO*>(y))));
+                   (launch_kernel(blk::gdn_block_post_fwd_kernel<IO, LPR>, ctas, 128, 0, st, p, static_cast<const IO*>(o), static_cast<const IO*>(z), wn, static_cast<IO*>(y))));
     });
     return check_launch("gdn_block_post_fwd");
   }
@@ -850,13 +857,12 @@ static mxb_status blk_post(const mxb_gdn_desc* d, const void* o, const void* z, 
     constexpr int LPR = decltype(lpr)::value;
     if constexpr (LPR <= 16)
       MXB_LAUNCH("gdn_block_post_bwd_kernel", st,
-                 (blk::gdn_block_post_bwd_kernel<IO, LPR><<<ctas, 128, 0, st>>>(
-                     p, static_cast<const IO*>(o), static_cast<const IO*>(z), wn, static_cast<const IO*>(dy),
+                 (launch_kernel(blk::gdn_block_post_bwd_kernel<IO, LPR>, ctas, 128, 0, st, p, static_cast<const IO*>(o), static_cast<const IO*>(z), wn, static_cast<const IO*>(dy),
                      static_cast<IO*>(d_o), static_cast<IO*>(dz), part)));
   });
   blk::ColSums c{};
   c.part[0] = part; c.out[0] = dwn; c.rows[0] = ctas; c.n[0] = d->Dv; c.count = 1; c.first[1] = (d->Dv + 31) / 32;
-  MXB_LAUNCH("gdn_block_colsum_kernel", st, (blk::gdn_block_colsum_kernel<<<c.first[1], 256, 0, st>>>(c)));
+  MXB_LAUNCH("gdn_block_colsum_kernel", st, (launch_kernel(blk::gdn_block_colsum_kernel, c.first[1], 256, 0, st, c)));
   return check_launch("gdn_block_post_bwd");
 }
 mxb_status gdn_block_post(const mxb_gdn_desc* d, const void* o, const void* z, const float* wn, void* y, const void* dy,

@@ -110,6 +110,7 @@ constexpr int kFwdSmem = NS * (3 * W * 128 + NV * 128 + 8192) + NB * (W * NV * 2
 
 template <int W, int NV, int NS, int NB>
 __global__ void __launch_bounds__(kThreads, 1) gdn_chain_fwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+  begin_dependent();
   using L = Layout<W, NV, NS, NB>;
   constexpr int MT = NV / 16, KS = W / 16, NT = W / 32;  // 16-column blocks; steps of a contraction over W; row groups of S per warp
   extern __shared__ uint8_t raw[];
@@ -443,6 +444,7 @@ constexpr int kBwdSmem = NS * (3 * W * 128 + NV * 128 + 8192) + NB * (W * NV * 2
 
 template <int W, int NV, int NS, int NB>
 __global__ void __launch_bounds__(kThreads, 1) gdn_chain_bwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+  begin_dependent();
   using L = Layout<W, NV, NS, NB>;
   constexpr int MT = NV / 16, KS = W / 16, NT = W / 32;
   constexpr int kX = 64 * NV * 4, kY = W * NV * 4;  // dO^T P and dO^T (d q), fp32 fragments
@@ -769,12 +771,12 @@ static mxb_status chain_launch(const TcP& p, const RowMaps& maps, int width, cud
     constexpr int smem = chain::kBwdSmem<W, NV, NS, NB>;
     static_assert(smem <= 227 * 1024, "");
     if (MXB_ALLOW_SMEM(smem, chain::gdn_chain_bwd_kernel<W, NV, NS, NB>) != MXB_OK) return MXB_ERR_CUDA;
-    MXB_LAUNCH("gdn_chain_bwd_kernel", st, (chain::gdn_chain_bwd_kernel<W, NV, NS, NB><<<grid, chain::kThreads, smem, st>>>(p, maps)));
+    MXB_LAUNCH("gdn_chain_bwd_kernel", st, (launch_kernel(chain::gdn_chain_bwd_kernel<W, NV, NS, NB>, grid, chain::kThreads, smem, st, p, maps)));
   } else {
     constexpr int smem = chain::kFwdSmem<W, NV, NS, NB>;
     static_assert(smem <= 227 * 1024, "");
     if (MXB_ALLOW_SMEM(smem, chain::gdn_chain_fwd_kernel<W, NV, NS, NB>) != MXB_OK) return MXB_ERR_CUDA;
-    MXB_LAUNCH("gdn_chain_fwd_kernel", st, (chain::gdn_chain_fwd_kernel<W, NV, NS, NB><<<grid, chain::kThreads, smem, st>>>(p, maps)));
+    MXB_LAUNCH("gdn_chain_fwd_kernel", st, (launch_kernel(chain::gdn_chain_fwd_kernel<W, NV, NS, NB>, grid, chain::kThreads, smem, st, p, maps)));
   }
   return check_launch("gdn_chain kernels");
 }

@@ -26,6 +26,7 @@ gdn_decode_kernel(float* __restrict__ state, const IO* __restrict__ q, const IO*
                   const IO* __restrict__ v, const float* __restrict__ beta,
                   const float* __restrict__ gate, IO* __restrict__ out, int Dk, int Dv,
                   int gate_is_log) {
+  begin_dependent();
   __shared__ float s_k[16 * ROWS], s_q[16 * ROWS];
   __shared__ __align__(16) float4 s_red[4][2][8];
   __shared__ float s_qk[4];
@@ -124,11 +125,11 @@ static mxb_status launch_decode(const mxb_gdn_desc* d, float* state, const void*
   auto V = static_cast<const IO*>(v);
   auto O = static_cast<IO*>(out);
   if (d->Dk <= 64)
-    MXB_LAUNCH("gdn_decode_kernel", st, (gdn_decode_kernel<IO, 4><<<grid, 128, 0, st>>>(state, Q, K, V, beta, gate, O, d->Dk, d->Dv, d->gate_is_log)));
+    MXB_LAUNCH("gdn_decode_kernel", st, (launch_kernel(gdn_decode_kernel<IO, 4>, grid, 128, 0, st, state, Q, K, V, beta, gate, O, d->Dk, d->Dv, d->gate_is_log)));
   else if (d->Dk <= 128)
-    MXB_LAUNCH("gdn_decode_kernel", st, (gdn_decode_kernel<IO, 8><<<grid, 128, 0, st>>>(state, Q, K, V, beta, gate, O, d->Dk, d->Dv, d->gate_is_log)));
+    MXB_LAUNCH("gdn_decode_kernel", st, (launch_kernel(gdn_decode_kernel<IO, 8>, grid, 128, 0, st, state, Q, K, V, beta, gate, O, d->Dk, d->Dv, d->gate_is_log)));
   else
-    MXB_LAUNCH("gdn_decode_kernel", st, (gdn_decode_kernel<IO, 16><<<grid, 128, 0, st>>>(state, Q, K, V, beta, gate, O, d->Dk, d->Dv, d->gate_is_log)));
+    MXB_LAUNCH("gdn_decode_kernel", st, (launch_kernel(gdn_decode_kernel<IO, 16>, grid, 128, 0, st, state, Q, K, V, beta, gate, O, d->Dk, d->Dv, d->gate_is_log)));
   return check_launch("gdn_decode_kernel");
 }
 

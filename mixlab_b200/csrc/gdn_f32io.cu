@@ -38,6 +38,7 @@ struct Segs {
 };
 
 __global__ void __launch_bounds__(kThreads) narrow_kernel(Segs sg) {
+  begin_dependent();
   const int s = blockIdx.y;
   const float4* src = static_cast<const float4*>(sg.src[s]);
   uint4* dst = static_cast<uint4*>(sg.dst[s]);
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(kThreads) narrow_kernel(Segs sg) {
 }
 
 __global__ void __launch_bounds__(kThreads) widen_kernel(Segs sg) {
+  begin_dependent();
   const int s = blockIdx.y;
   const uint4* src = static_cast<const uint4*>(sg.src[s]);
   float4* dst = static_cast<float4*>(sg.dst[s]);
@@ -104,8 +106,8 @@ static Stage carve(const mxb_gdn_desc* d, void* ws, bool bwd, bool inner_bwd) {
 static mxb_status run(bool narrow, const Segs& sg, int nseg, cudaStream_t st) {
   if (nseg == 0) return MXB_OK;
   const dim3 grid(kCtasPerSeg, nseg);
-  if (narrow) MXB_LAUNCH("gdn_f32io_narrow_kernel", st, (narrow_kernel<<<grid, kThreads, 0, st>>>(sg)));
-  else MXB_LAUNCH("gdn_f32io_widen_kernel", st, (widen_kernel<<<grid, kThreads, 0, st>>>(sg)));
+  if (narrow) MXB_LAUNCH("gdn_f32io_narrow_kernel", st, (launch_kernel(narrow_kernel, grid, kThreads, 0, st, sg)));
+  else MXB_LAUNCH("gdn_f32io_widen_kernel", st, (launch_kernel(widen_kernel, grid, kThreads, 0, st, sg)));
   return check_launch(narrow ? "gdn_f32io_narrow_kernel" : "gdn_f32io_widen_kernel");
 }
 

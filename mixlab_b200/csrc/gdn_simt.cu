@@ -438,6 +438,7 @@ __device__ __forceinline__ void prep_product(f2 (&acc)[4][2 * NG], const float* 
 
 template <typename IO, int KP>
 __global__ void __launch_bounds__(256, 2) gdn_prep_kernel(GdnP p, const __grid_constant__ SlabMaps maps) {
+  begin_dependent();
   using namespace simt;
   extern __shared__ float smem_raw[];
   float* Ks = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(smem_raw) + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u));
@@ -730,6 +731,7 @@ __device__ __forceinline__ float slab_sum(const float* part, int rows, int row, 
 // v_new = u - w S;  o = E(gam) (q S) + P v_new;  S <- E(gam_last) S + (k r)^T v_new
 template <typename IO, int W, int KP>
 __global__ void __launch_bounds__(256, 1) gdn_state_fwd_kernel(GdnP p, const __grid_constant__ SlabMaps maps) {
+  begin_dependent();
   using namespace simt;
   constexpr int LK = KP + 4, SP = 32 / W, SPK = 2048 / (W * KP), PITCH = SlabMap<W, 16>::PITCH;
   extern __shared__ float smem_raw[];
@@ -855,6 +857,7 @@ __global__ void __launch_bounds__(256, 1) gdn_state_fwd_kernel(GdnP p, const __g
 // dv_new = P^T dO + r (k dS);  dS <- E(gam_last) dS + (q E(gam))^T dO - w^T dv_new, chunks in reverse.
 template <typename IO, int W, int KP>
 __global__ void __launch_bounds__(256, 1) gdn_state_bwd_kernel(GdnP p, const __grid_constant__ SlabMaps maps) {
+  begin_dependent();
   using namespace simt;
   constexpr int LK = KP + 4, SP = 32 / W, SPK = 2048 / (W * KP), PITCH = SlabMap<W, 16>::PITCH;
   extern __shared__ float smem_raw[];
@@ -1011,6 +1014,7 @@ static_assert(2 * (kChunkF32Smem + 1024) <= 228 * 1024, "two CTAs per SM");
 
 template <typename IO, int NGK>
 __global__ void __launch_bounds__(256, 2) gdn_chunk_bwd_kernel(GdnP p) {
+  begin_dependent();
   using namespace simt;
   extern __shared__ __align__(16) float smem[];
   float* stage = smem;
@@ -1303,6 +1307,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_bwd_kernel(GdnP p) {
 // --------------------------------------------------- token-by-token forward
 template <typename IO>
 __global__ void __launch_bounds__(256) gdn_recurrent_fwd_kernel(GdnP p) {
+  begin_dependent();
   extern __shared__ float smem[];
   const int K = p.K, V = p.V;
   float* S = smem;           // [K][33]
@@ -1413,7 +1418,7 @@ static mxb_status run_prep(GdnP p, cudaStream_t st) {
   p.vtma = sizeof(IO) == 4 && p.C == simt::R && make_tma_map_f32(&maps.P, p.v, p.B, p.T, p.H, p.V);
   constexpr int sm = PrepF32<KP>::smem;
   if (MXB_ALLOW_SMEM(sm, gdn_prep_kernel<IO, KP>) != MXB_OK) return MXB_ERR_CUDA;
-  MXB_LAUNCH("gdn_prep_kernel", st, (gdn_prep_kernel<IO, KP><<<dim3(p.n, p.B * p.H), 256, sm, st>>>(p, maps)));
+  MXB_LAUNCH("gdn_prep_kernel", st, (launch_kernel(gdn_prep_kernel<IO, KP>, dim3(p.n, p.B * p.H), 256, sm, st, p, maps)));
   return check_launch("gdn_prep_kernel");
 }
 
@@ -1436,12 +1441,12 @@ static mxb_status run_state(GdnP p, bool bwd, cudaStream_t st) {
   if (bwd) {
     constexpr int sm = state_bwd_smem<W, KP>();
     if (MXB_ALLOW_SMEM(sm, gdn_state_bwd_kernel<IO, W, KP>) != MXB_OK) return MXB_ERR_CUDA;
-    MXB_LAUNCH("gdn_state_bwd_kernel", st, (gdn_state_bwd_kernel<IO, W, KP><<<grid, 256, sm, st>>>(p, maps)));
+    MXB_LAUNCH("gdn_state_bwd_kernel", st, (launch_kernel(gdn_state_bwd_kernel<IO, W, KP>, grid, 256, sm, st, p, maps)));
     return check_launch("gdn_state_bwd_kernel");
   }
   constexpr int sm = state_fwd_smem<W, KP>();
   if (MXB_ALLOW_SMEM(sm, gdn_state_fwd_kernel<IO, W, KP>) != MXB_OK) return MXB_ERR_CUDA;
-  MXB_LAUNCH("gdn_state_fwd_kernel", st, (gdn_state_fwd_kernel<IO, W, KP><<<grid, 256, sm, st>>>(p, maps)));
+  MXB_LAUNCH("gdn_state_fwd_kernel", st, (launch_kernel(gdn_state_fwd_kernel<IO, W, KP>, grid, 256, sm, st, p, maps)));
   return check_launch("gdn_state_fwd_kernel");
 }
 template <typename IO>
@@ -1457,7 +1462,7 @@ template <typename IO, int NGK>
 static mxb_status run_chunk_bwd(const GdnP& p, cudaStream_t st) {
   if (MXB_ALLOW_SMEM(kChunkF32Smem, gdn_chunk_bwd_kernel<IO, NGK>) != MXB_OK) return MXB_ERR_CUDA;
   MXB_LAUNCH("gdn_chunk_bwd_kernel", st,
-             (gdn_chunk_bwd_kernel<IO, NGK><<<dim3(p.n, p.B * p.H), 256, kChunkF32Smem, st>>>(p)));
+             (launch_kernel(gdn_chunk_bwd_kernel<IO, NGK>, dim3(p.n, p.B * p.H), 256, kChunkF32Smem, st, p)));
   return check_launch("gdn_chunk_bwd_kernel");
 }
 
@@ -1468,7 +1473,7 @@ static mxb_status run_fwd(GdnP& p, bool chunked, cudaStream_t st) {
     dim3 gslab((V + 31) / 32, p.B * p.H);
     size_t sm = sizeof(float) * (K * 33 + 2 * K + 512);
     if (MXB_ALLOW_SMEM((int)sm, gdn_recurrent_fwd_kernel<IO>) != MXB_OK) return MXB_ERR_CUDA;
-    MXB_LAUNCH("gdn_recurrent_fwd_kernel", st, (gdn_recurrent_fwd_kernel<IO><<<gslab, 256, sm, st>>>(p)));
+    MXB_LAUNCH("gdn_recurrent_fwd_kernel", st, (launch_kernel(gdn_recurrent_fwd_kernel<IO>, gslab, 256, sm, st, p)));
     return check_launch("gdn_recurrent_fwd_kernel");
   }
   p.vecK = vec_ok<IO>(K, {p.q, p.k, p.dq, p.dk});

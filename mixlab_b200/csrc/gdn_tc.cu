@@ -50,6 +50,7 @@ using PrepMaps = RowMaps;
 
 template <bool TMA>
 __global__ void __launch_bounds__(128, 4) gdn_tc_prep_kernel(TcP p, const __grid_constant__ PrepMaps maps) {
+  begin_dependent();
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
   uint8_t* Akq = sm;                    // slab s at 16384 s: k box [64][64], then q box [64][64] (later v, u / w images)
@@ -300,6 +301,7 @@ constexpr int kStateFwdSmem =
 
 template <bool TMA, int NV>
 __global__ void __launch_bounds__(kStateThreads<NV>, 1) gdn_tc_state_fwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+  begin_dependent();
   static_assert(NV == KD || TMA, "the per-thread staging moves whole rows");
   constexpr int NC = NV / 2;                   // columns per thread
   const int col0 = blockIdx.y * NV;
@@ -740,11 +742,11 @@ mxb_status tc_run_fwd(TcP& p, cudaStream_t st) {
   if (tma) {
     if (MXB_ALLOW_SMEM(kPrepSmem, gdn_tc_prep_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_prep_kernel", st,
-               (gdn_tc_prep_kernel<true><<<dim3(p.n, p.B * p.H), 128, kPrepSmem, st>>>(p, maps)));
+               (launch_kernel(gdn_tc_prep_kernel<true>, dim3(p.n, p.B * p.H), 128, kPrepSmem, st, p, maps)));
   } else {
     if (MXB_ALLOW_SMEM(kPrepSmem, gdn_tc_prep_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_prep_kernel", st,
-               (gdn_tc_prep_kernel<false><<<dim3(p.n, p.B * p.H), 128, kPrepSmem, st>>>(p, maps)));
+               (launch_kernel(gdn_tc_prep_kernel<false>, dim3(p.n, p.B * p.H), 128, kPrepSmem, st, p, maps)));
   }
   mxb_status s = check_launch("gdn_tc_prep_kernel");
   if (s != MXB_OK) return s;
@@ -753,7 +755,7 @@ mxb_status tc_run_fwd(TcP& p, cudaStream_t st) {
     constexpr int NV = decltype(nv)::value;
     if (MXB_ALLOW_SMEM(kStateFwdSmem<NV>, gdn_tc_state_fwd_kernel<TMA, NV>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_state_fwd_kernel", st,
-               (gdn_tc_state_fwd_kernel<TMA, NV><<<dim3(p.B * p.H, (p.Dv + NV - 1) / NV), kStateThreads<NV>, kStateFwdSmem<NV>, st>>>(p, maps)));
+               (launch_kernel(gdn_tc_state_fwd_kernel<TMA, NV>, dim3(p.B * p.H, (p.Dv + NV - 1) / NV), kStateThreads<NV>, kStateFwdSmem<NV>, st, p, maps)));
     return MXB_OK;
   };
   if (tma && chain_columns(p, p.save)) return chain_fwd(p, maps, chain_columns(p, p.save), st);

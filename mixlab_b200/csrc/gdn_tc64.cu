@@ -43,6 +43,7 @@ constexpr int kPrepSmem = 2 * kTile + C * LDA * 4 + 3 * C * 4 + 64 + 1024;
 static_assert(6 * (kPrepSmem + 1024) <= 228 * 1024, "six CTAs per SM");
 
 __global__ void __launch_bounds__(128, 6) gdn_tc_prep_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+  begin_dependent();
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
   uint8_t* Xk = sm;             // k, then d k, then the w image
@@ -216,6 +217,7 @@ constexpr int kStateFwdSmem = 2 * 2 * kTile + kTile + 2 * 2 * kTile + kTile + kT
 static_assert(2 * (kStateFwdSmem + 1024) <= 228 * 1024, "two CTAs per SM");
 
 __global__ void __launch_bounds__(256, 2) gdn_tc_state_fwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+  begin_dependent();
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
   uint8_t* A1 = sm;                   // x2 [128][64]: w rows, then q rows (swizzled)
@@ -410,6 +412,7 @@ constexpr int kStateBwdSmem = 3 * kTile + 4 * kTile + 2 * kTile + 2 * kTile + kT
 static_assert(2 * (kStateBwdSmem + 1024) <= 228 * 1024, "two CTAs per SM");
 
 __global__ void __launch_bounds__(256, 2) gdn_tc_state_bwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+  begin_dependent();
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
   uint8_t* Ak = sm;                   // x2 k (swizzled); the tile behind the second buffer (dSop) is read beside it
@@ -585,6 +588,7 @@ constexpr int kChunkSmem = 9 * kTile + 4 * C * 4 + 16 * 4 + 64 + 64;
 static_assert(3 * (kChunkSmem + 1024) <= 228 * 1024, "three CTAs per SM");
 
 __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+  begin_dependent();
   extern __shared__ __align__(1024) uint8_t sm[];
   uint8_t* XdO = sm;              // swizzled
   uint8_t* Xz = XdO + kTile;      // un-swizzled
@@ -899,10 +903,10 @@ mxb_status tc64_run_fwd(TcP& p, cudaStream_t st) {
       MXB_ALLOW_SMEM(g64::kStateFwdSmem, g64::gdn_tc_state_fwd_kernel) != MXB_OK)
     return MXB_ERR_CUDA;
   MXB_LAUNCH("gdn_tc_prep_kernel", st,
-             (g64::gdn_tc_prep_kernel<<<dim3(p.n, p.B * p.H), 128, g64::kPrepSmem, st>>>(p, maps)));
+             (launch_kernel(g64::gdn_tc_prep_kernel, dim3(p.n, p.B * p.H), 128, g64::kPrepSmem, st, p, maps)));
   if (const int nv = chain_columns(p, p.save)) return chain_fwd(p, maps, nv, st);
   MXB_LAUNCH("gdn_tc_state_fwd_kernel", st,
-             (g64::gdn_tc_state_fwd_kernel<<<p.B * p.H, 256, g64::kStateFwdSmem, st>>>(p, maps)));
+             (launch_kernel(g64::gdn_tc_state_fwd_kernel, p.B * p.H, 256, g64::kStateFwdSmem, st, p, maps)));
   return check_launch("gdn_tc64 forward");
 }
 // After a forward that saved its intermediates: reverse state pass, per-chunk pass.
@@ -922,10 +926,10 @@ mxb_status tc64_run_bwd(const TcP& p, cudaStream_t st) {
     if (s != MXB_OK) return s;
   } else {
     MXB_LAUNCH("gdn_tc_state_bwd_kernel", st,
-               (g64::gdn_tc_state_bwd_kernel<<<p.B * p.H, 256, g64::kStateBwdSmem, st>>>(p, maps)));
+               (launch_kernel(g64::gdn_tc_state_bwd_kernel, p.B * p.H, 256, g64::kStateBwdSmem, st, p, maps)));
   }
   MXB_LAUNCH("gdn_tc_chunk_bwd_kernel", st,
-             (g64::gdn_tc_chunk_bwd_kernel<<<dim3(p.B * p.H, p.n), 256, g64::kChunkSmem, st>>>(p, maps)));
+             (launch_kernel(g64::gdn_tc_chunk_bwd_kernel, dim3(p.B * p.H, p.n), 256, g64::kChunkSmem, st, p, maps)));
   return check_launch("gdn_tc64 backward");
 }
 

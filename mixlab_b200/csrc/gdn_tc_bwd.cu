@@ -49,6 +49,7 @@ constexpr int kStateBwdSmem =
 
 template <bool TMA, int NV>
 __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+  begin_dependent();
   static_assert(NV == KD || TMA, "the per-thread staging moves whole rows");
   constexpr int NC = NV / 2;                   // columns per thread
   const int col0 = blockIdx.y * NV;
@@ -305,6 +306,7 @@ __global__ void __launch_bounds__(256) gdn_tc_state_bwd_kernel(TcP p, const __gr
 constexpr int kChunkBwdSmem = 3 * 16384 + 32768 + 3 * 8192 + 12 * C * 4 + 16 * 4 + 64 + 64 + 1024;
 
 __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const __grid_constant__ RowMaps maps) {
+  begin_dependent();
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
   uint8_t* XdO = sm;                // [64][128] dO (swizzled TMA tile), d dO in place, then z (blocked layout)
@@ -718,7 +720,7 @@ mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st) {
     constexpr int NV = decltype(nv)::value;
     if (MXB_ALLOW_SMEM(kStateBwdSmem<NV>, gdn_tc_state_bwd_kernel<TMA, NV>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("gdn_tc_state_bwd_kernel", st,
-               (gdn_tc_state_bwd_kernel<TMA, NV><<<dim3(p.B * p.H, (p.Dv + NV - 1) / NV), 256, kStateBwdSmem<NV>, st>>>(p, maps)));
+               (launch_kernel(gdn_tc_state_bwd_kernel<TMA, NV>, dim3(p.B * p.H, (p.Dv + NV - 1) / NV), 256, kStateBwdSmem<NV>, st, p, maps)));
     return MXB_OK;
   };
   if (tma && chain_columns(p, true)) s = chain_bwd(p, maps, chain_columns(p, true), st);
@@ -741,7 +743,7 @@ mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st) {
     return MXB_ERR_UNSUPPORTED;
   if (MXB_ALLOW_SMEM(kChunkBwdSmem, gdn_tc_chunk_bwd_kernel) != MXB_OK) return MXB_ERR_CUDA;
   MXB_LAUNCH("gdn_tc_chunk_bwd_kernel", st,
-             (gdn_tc_chunk_bwd_kernel<<<dim3(p.B * p.H, p.n), 256, kChunkBwdSmem, st>>>(p, maps)));
+             (launch_kernel(gdn_tc_chunk_bwd_kernel, dim3(p.B * p.H, p.n), 256, kChunkBwdSmem, st, p, maps)));
   return check_launch("gdn_tc_chunk_bwd_kernel");
 }
 

@@ -43,6 +43,7 @@ namespace mxb {
 // Also the checkpoint pass of the backward (y == nullptr, ck_h != nullptr).
 template <typename IO, int PR, int LPC>
 __global__ void __launch_bounds__(256) mamba3_fwd_kernel(M3P p) {
+  begin_dependent();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int CPW = 32 / LPC;  // channels per warp
   const int sl = lane % LPC, d_raw = (blockIdx.x * 8 + warp) * CPW + lane / LPC;
@@ -117,6 +118,7 @@ __global__ void __launch_bounds__(256) mamba3_fwd_kernel(M3P p) {
 // sum.
 template <typename IO, int PR, int LPC>
 __global__ void __launch_bounds__(256) mamba3_bwd_kernel(M3P p) {
+  begin_dependent();
   extern __shared__ float smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int CPW = 32 / LPC;  // channels per warp
@@ -313,6 +315,7 @@ __global__ void __launch_bounds__(256) mamba3_bwd_kernel(M3P p) {
 template <typename IO>
 __global__ void __launch_bounds__(256) m3_bc_sum_kernel(const float* __restrict__ pb, const float* __restrict__ pc,
                                                         IO* __restrict__ db, IO* __restrict__ dc, size_t rows, int S, int N) {
+  begin_dependent();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < rows * N; i += (size_t)gridDim.x * blockDim.x) {
     const size_t r = i / N;
     const int n = (int)(i - r * N);
@@ -330,6 +333,7 @@ __global__ void __launch_bounds__(256) m3_bc_sum_kernel(const float* __restrict_
 __global__ void __launch_bounds__(256) m3_head_sum_kernel(const float* __restrict__ hd, float* __restrict__ ddt,
                                                           float* __restrict__ dlam, float* __restrict__ dtheta,
                                                           size_t rows, int D, int NH) {
+  begin_dependent();
   const int cph = D / NH;
   const size_t btd = rows * D;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < rows * NH; i += (size_t)gridDim.x * blockDim.x) {
@@ -353,6 +357,7 @@ __global__ void __launch_bounds__(256) m3_head_sum_kernel(const float* __restric
 constexpr int kDalogSlices = 16;
 __global__ void __launch_bounds__(32 * kDalogSlices) m3_dalog_sum_kernel(const float* __restrict__ part, float* __restrict__ out,
                                                                          int rows, int D, int N, int NH) {
+  begin_dependent();
   __shared__ float red[kDalogSlices][32];
   const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
   const int cph = NH > 0 ? D / NH : 1, outs = NH > 0 ? NH : D * N, total = rows * cph;
@@ -518,7 +523,7 @@ static mxb_status m3_fwd_serial(const M3P& p, cudaStream_t st) {
   const int per_cta = 8 * (32 / p.LPC);  // channels per 256-thread CTA
   const dim3 grid((p.D + per_cta - 1) / per_cta, p.B);
   M3_PR_DISPATCH(p, MXB_LAUNCH("mamba3_fwd_kernel", st,
-                               (mamba3_fwd_kernel<IO, PRV, LPCV><<<grid, 256, 0, st>>>(p))));
+                               (launch_kernel(mamba3_fwd_kernel<IO, PRV, LPCV>, grid, 256, 0, st, p))));
   return check_launch("mamba3_fwd_kernel");
 }
 
@@ -531,7 +536,7 @@ static mxb_status m3_bwd_launch(const M3P& p, cudaStream_t st) {
     if (e != cudaSuccess) { set_last_cuda_error((int)e); return MXB_ERR_CUDA; }
   }
   const dim3 grid(p.D / p.CW, p.B);
-  MXB_LAUNCH("mamba3_bwd_kernel", st, (mamba3_bwd_kernel<IO, PR, LPC><<<grid, 32 * warps, sm, st>>>(p)));
+  MXB_LAUNCH("mamba3_bwd_kernel", st, (launch_kernel(mamba3_bwd_kernel<IO, PR, LPC>, grid, 32 * warps, sm, st, p)));
   return check_launch("mamba3_bwd_kernel");
 }
 template <typename IO>
@@ -607,18 +612,16 @@ mxb_status mamba3_bwd(const mxb_mamba3_desc* d, const void* x, const float* dt, 
   const size_t rows = (size_t)p.B * p.T * p.G;
   const int grid = (int)std::min<size_t>((rows * p.N + 255) / 256, 148 * 8);
   if (f32)
-    MXB_LAUNCH("m3_bc_sum_kernel", st, (m3_bc_sum_kernel<float><<<grid, 256, 0, st>>>(
-        p.pb32, p.pc32, static_cast<float*>(db), static_cast<float*>(dc), rows, p.S, p.N)));
+    MXB_LAUNCH("m3_bc_sum_kernel", st, (launch_kernel(m3_bc_sum_kernel<float>, grid, 256, 0, st, p.pb32, p.pc32, static_cast<float*>(db), static_cast<float*>(dc), rows, p.S, p.N)));
   else
-    MXB_LAUNCH("m3_bc_sum_kernel", st, (m3_bc_sum_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(
-        p.pb32, p.pc32, static_cast<__nv_bfloat16*>(db), static_cast<__nv_bfloat16*>(dc), rows, p.S, p.N)));
+    MXB_LAUNCH("m3_bc_sum_kernel", st, (launch_kernel(m3_bc_sum_kernel<__nv_bfloat16>, grid, 256, 0, st, p.pb32, p.pc32, static_cast<__nv_bfloat16*>(db), static_cast<__nv_bfloat16*>(dc), rows, p.S, p.N)));
   if (p.NH > 0) {
     const size_t bt = (size_t)p.B * p.T;
     const int gh = (int)std::min<size_t>((bt * p.NH + 255) / 256, 148 * 8);
-    MXB_LAUNCH("m3_head_sum_kernel", st, (m3_head_sum_kernel<<<gh, 256, 0, st>>>(p.hd, ddt, dlam, dtheta, bt, p.D, p.NH)));
+    MXB_LAUNCH("m3_head_sum_kernel", st, (launch_kernel(m3_head_sum_kernel, gh, 256, 0, st, p.hd, ddt, dlam, dtheta, bt, p.D, p.NH)));
   }
   const int nal = p.NH > 0 ? p.NH : p.D * p.N;
-  MXB_LAUNCH("m3_dalog_sum_kernel", st, (m3_dalog_sum_kernel<<<(nal + 31) / 32, 32 * kDalogSlices, 0, st>>>(p.dal_part, da_log, windows ? p.B * p.nW : p.B, p.D, p.N, p.NH)));
+  MXB_LAUNCH("m3_dalog_sum_kernel", st, (launch_kernel(m3_dalog_sum_kernel, (nal + 31) / 32, 32 * kDalogSlices, 0, st, p.dal_part, da_log, windows ? p.B * p.nW : p.B, p.D, p.N, p.NH)));
   return check_launch("mamba3 channel backward sums");
 }
 

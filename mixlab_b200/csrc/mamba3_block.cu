@@ -56,6 +56,7 @@ __device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.f, 1.f
 template <typename IO>
 __global__ void __launch_bounds__(128) m3b_conv_fwd_kernel(BlkP p, const IO* __restrict__ x, const float* __restrict__ w,
                                                            IO* __restrict__ y) {
+  begin_dependent();
   const int cg = blockIdx.x * 128 + threadIdx.x, ch = cg * 8;
   if (ch >= p.D) return;
   const int t0 = blockIdx.y * kRun, b = blockIdx.z;
@@ -90,6 +91,7 @@ template <typename IO>
 __global__ void __launch_bounds__(128) m3b_conv_bwd_kernel(BlkP p, const IO* __restrict__ x, const float* __restrict__ w,
                                                            const IO* __restrict__ dy, IO* __restrict__ dx,
                                                            float* __restrict__ dwp) {
+  begin_dependent();
   const int cg = blockIdx.x * 128 + threadIdx.x, ch = cg * 8;
   if (ch >= p.D) return;
   const int t0 = blockIdx.y * kRun, b = blockIdx.z;
@@ -148,6 +150,7 @@ __global__ void __launch_bounds__(128) m3b_conv_bwd_kernel(BlkP p, const IO* __r
 // then the 8 slices are added in order.  K > 0: columns are [k][d] and the result is stored as [d][K] (k < K only).
 __global__ void __launch_bounds__(256) m3b_colsum_kernel(const float* __restrict__ part, int rows, int n,
                                                          float* __restrict__ out, int D, int K) {
+  begin_dependent();
   __shared__ float red[8][32];
   const int j = blockIdx.x * 32 + (threadIdx.x & 31), slice = threadIdx.x >> 5;
   float s = 0.f;
@@ -192,6 +195,7 @@ struct BcArgs {
 };
 template <typename IO>
 __global__ void __launch_bounds__(128) m3b_bc_fwd_kernel(BlkP p, BcArgs<IO> a) {
+  begin_dependent();
   const int which = blockIdx.z, g = blockIdx.y, lane16 = threadIdx.x & 15, grp = threadIdx.x >> 4;
   const bool act = lane16 * 8 < p.N;
   float sc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, bi[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -213,6 +217,7 @@ __global__ void __launch_bounds__(128) m3b_bc_fwd_kernel(BlkP p, BcArgs<IO> a) {
 }
 template <typename IO>
 __global__ void __launch_bounds__(128) m3b_bc_bwd_kernel(BlkP p, BcArgs<IO> a) {
+  begin_dependent();
   __shared__ float red[8][2][128];
   const int which = blockIdx.z, g = blockIdx.y, lane16 = threadIdx.x & 15, grp = threadIdx.x >> 4;
   const bool act = lane16 * 8 < p.N;
@@ -258,6 +263,7 @@ __global__ void __launch_bounds__(128) m3b_bc_bwd_kernel(BlkP p, BcArgs<IO> a) {
 // from the column sums tab[g][kind][c] over the CTAs: dbias[g][c] = tab[g][1][c], dscale[c] = sum over g of tab[g][0][c]
 __global__ void __launch_bounds__(128) m3b_bc_final_kernel(BlkP p, const float* __restrict__ tab,
                                                            float* __restrict__ dscale, float* __restrict__ dbias) {
+  begin_dependent();
   const int c = threadIdx.x;
   if (c >= p.N) return;
   float s = 0.f;
@@ -283,6 +289,7 @@ __device__ __forceinline__ float cta_sum(float v, float* red) {
 template <typename IO>
 __global__ void __launch_bounds__(256) m3b_post_fwd_kernel(BlkP p, const IO* __restrict__ y, const IO* __restrict__ z,
                                                            const float* __restrict__ wn, IO* __restrict__ out) {
+  begin_dependent();
   __shared__ float red[8];
   const int ch = threadIdx.x * 8;
   const bool act = ch < p.D;
@@ -308,6 +315,7 @@ __global__ void __launch_bounds__(256) m3b_post_bwd_kernel(BlkP p, const IO* __r
                                                            const float* __restrict__ wn, const IO* __restrict__ dout,
                                                            IO* __restrict__ dy, IO* __restrict__ dz,
                                                            float* __restrict__ dwp) {
+  begin_dependent();
   __shared__ float red[8];
   const int ch = threadIdx.x * 8;
   const bool act = ch < p.D;
@@ -384,15 +392,15 @@ static mxb_status m3b_conv(const mxb_mamba3_desc* d, int K, const void* x, const
   const dim3 grid((d->D / 8 + 127) / 128, m3b_runs(d), d->B);
   if (!dy) {
     MXB_LAUNCH("m3b_conv_fwd_kernel", st,
-               (m3b::m3b_conv_fwd_kernel<IO><<<grid, 128, 0, st>>>(p, static_cast<const IO*>(x), w, static_cast<IO*>(y))));
+               (launch_kernel(m3b::m3b_conv_fwd_kernel<IO>, grid, 128, 0, st, p, static_cast<const IO*>(x), w, static_cast<IO*>(y))));
     return check_launch("m3b_conv_fwd");
   }
   float* part = reinterpret_cast<float*>(static_cast<char*>(ws) + 256);
   MXB_LAUNCH("m3b_conv_bwd_kernel", st,
-             (m3b::m3b_conv_bwd_kernel<IO><<<grid, 128, 0, st>>>(p, static_cast<const IO*>(x), w, static_cast<const IO*>(dy),
+             (launch_kernel(m3b::m3b_conv_bwd_kernel<IO>, grid, 128, 0, st, p, static_cast<const IO*>(x), w, static_cast<const IO*>(dy),
                                                                  static_cast<IO*>(dx), part)));
   const int rows = d->B * m3b_runs(d), n = m3b::kMaxK * d->D;
-  MXB_LAUNCH("m3b_colsum_kernel", st, (m3b::m3b_colsum_kernel<<<(n + 31) / 32, 256, 0, st>>>(part, rows, n, dw, d->D, K)));
+  MXB_LAUNCH("m3b_colsum_kernel", st, (launch_kernel(m3b::m3b_colsum_kernel, (n + 31) / 32, 256, 0, st, part, rows, n, dw, d->D, K)));
   return check_launch("m3b_conv_bwd");
 }
 mxb_status mamba3_block_conv(const mxb_mamba3_desc* d, int K, const void* x, const float* w, void* y, const void* dy,
@@ -413,7 +421,7 @@ static mxb_status m3b_bc(const mxb_mamba3_desc* d, float eps, const void* bp, co
   const int ctas = m3b_bc_ctas(d);
   if (!db) {
     a.y[0] = static_cast<IO*>(b); a.y[1] = static_cast<IO*>(c);
-    MXB_LAUNCH("m3b_bc_fwd_kernel", st, (m3b::m3b_bc_fwd_kernel<IO><<<dim3(ctas, d->G, 2), 128, 0, st>>>(p, a)));
+    MXB_LAUNCH("m3b_bc_fwd_kernel", st, (launch_kernel(m3b::m3b_bc_fwd_kernel<IO>, dim3(ctas, d->G, 2), 128, 0, st, p, a)));
     return check_launch("m3b_bc_fwd");
   }
   a.dy[0] = static_cast<const IO*>(db); a.dy[1] = static_cast<const IO*>(dc);
@@ -421,15 +429,15 @@ static mxb_status m3b_bc(const mxb_mamba3_desc* d, float eps, const void* bp, co
   float* base = reinterpret_cast<float*>(static_cast<char*>(ws) + 256);
   const size_t per = (size_t)ctas * d->G * 2 * d->N;
   a.part[0] = base; a.part[1] = base + per;
-  MXB_LAUNCH("m3b_bc_bwd_kernel", st, (m3b::m3b_bc_bwd_kernel<IO><<<dim3(ctas, d->G, 2), 128, 0, st>>>(p, a)));
+  MXB_LAUNCH("m3b_bc_bwd_kernel", st, (launch_kernel(m3b::m3b_bc_bwd_kernel<IO>, dim3(ctas, d->G, 2), 128, 0, st, p, a)));
   const int n = d->G * 2 * d->N;
   float* tab = base + 2 * per;  // [2][G][2][N]
   float* outs[2][2] = {{dbs, dbb}, {dcs, dcb}};
   for (int w = 0; w < 2; ++w) {
     MXB_LAUNCH("m3b_colsum_kernel", st,
-               (m3b::m3b_colsum_kernel<<<(n + 31) / 32, 256, 0, st>>>(a.part[w], ctas, n, tab + (size_t)w * n, n, 0)));
+               (launch_kernel(m3b::m3b_colsum_kernel, (n + 31) / 32, 256, 0, st, a.part[w], ctas, n, tab + (size_t)w * n, n, 0)));
     MXB_LAUNCH("m3b_bc_final_kernel", st,
-               (m3b::m3b_bc_final_kernel<<<1, 128, 0, st>>>(p, tab + (size_t)w * n, outs[w][0], outs[w][1])));
+               (launch_kernel(m3b::m3b_bc_final_kernel, 1, 128, 0, st, p, tab + (size_t)w * n, outs[w][0], outs[w][1])));
   }
   return check_launch("m3b_bc_bwd");
 }
@@ -449,17 +457,17 @@ static mxb_status m3b_post(const mxb_mamba3_desc* d, float eps, const void* y, c
   const int ctas = m3b_post_ctas(d);
   if (!dout) {
     MXB_LAUNCH("m3b_post_fwd_kernel", st,
-               (m3b::m3b_post_fwd_kernel<IO><<<ctas, 256, 0, st>>>(p, static_cast<const IO*>(y), static_cast<const IO*>(z),
+               (launch_kernel(m3b::m3b_post_fwd_kernel<IO>, ctas, 256, 0, st, p, static_cast<const IO*>(y), static_cast<const IO*>(z),
                                                                    wn, static_cast<IO*>(out))));
     return check_launch("m3b_post_fwd");
   }
   float* part = reinterpret_cast<float*>(static_cast<char*>(ws) + 256);
   MXB_LAUNCH("m3b_post_bwd_kernel", st,
-             (m3b::m3b_post_bwd_kernel<IO><<<ctas, 256, 0, st>>>(p, static_cast<const IO*>(y), static_cast<const IO*>(z), wn,
+             (launch_kernel(m3b::m3b_post_bwd_kernel<IO>, ctas, 256, 0, st, p, static_cast<const IO*>(y), static_cast<const IO*>(z), wn,
                                                                  static_cast<const IO*>(dout), static_cast<IO*>(dy),
                                                                  static_cast<IO*>(dz), part)));
   MXB_LAUNCH("m3b_colsum_kernel", st,
-             (m3b::m3b_colsum_kernel<<<(d->D + 31) / 32, 256, 0, st>>>(part, ctas, d->D, dwn, d->D, 0)));
+             (launch_kernel(m3b::m3b_colsum_kernel, (d->D + 31) / 32, 256, 0, st, part, ctas, d->D, dwn, d->D, 0)));
   return check_launch("m3b_post_bwd");
 }
 mxb_status mamba3_block_post(const mxb_mamba3_desc* d, float eps, const void* y, const void* z, const float* wn, void* out,

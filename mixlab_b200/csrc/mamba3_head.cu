@@ -78,6 +78,7 @@ __device__ __forceinline__ int reduced_channel(int lane) {
 
 template <typename IO, int SPL, int CPW>
 __global__ void __launch_bounds__(256) mamba3_head_fwd_kernel(M3H p) {
+  begin_dependent();
   constexpr int NW = 8;            // warps
   const int N = SPL * 32, P = CPW * NW;
   __shared__ __align__(16) float s_brot[(kHB + 1) * SPL * 32];  // row 0 = last step of the previous block
@@ -216,6 +217,7 @@ struct M3HB {
 
 template <typename IO, int SPW>
 __global__ void __launch_bounds__(256) mamba3_head_bwd_kernel(M3HB q) {
+  begin_dependent();
   // SPW states per warp (N = 8 SPW); a warp holds all CH = 16 channels of the CTA for its states:
   // lane = (channel group cg, state st), CPT channels per thread.
   constexpr int CH = 16, W = kHB, CG = 32 / SPW, CPT = CH / CG, N = 8 * SPW;
@@ -435,6 +437,7 @@ __global__ void __launch_bounds__(256) mamba3_head_bwd_kernel(M3HB q) {
 __global__ void __launch_bounds__(256) m3h_head_sum_kernel(const float* __restrict__ hpart, float* __restrict__ dtheta,
                                                            float* __restrict__ ddt, float* __restrict__ dlam, size_t rows,
                                                            int nslice, int NH) {
+  begin_dependent();
   const int per = nslice / NH;
   const size_t plane = rows * nslice;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < rows * NH; i += (size_t)gridDim.x * blockDim.x) {
@@ -456,6 +459,7 @@ __global__ void __launch_bounds__(256) m3h_head_sum_kernel(const float* __restri
 // da_log [NH] = the per-warp shares over the batch, the CTAs of the head and their warps, in that order.
 __global__ void __launch_bounds__(128) m3h_dalog_sum_kernel(const float* __restrict__ part, float* __restrict__ da_log, int B,
                                                             int nslice, int NH) {
+  begin_dependent();
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= NH) return;
   const int per = nslice / NH;
@@ -477,7 +481,7 @@ bool mamba3_head_supported(const mxb_mamba3_desc* d) {
 
 template <typename IO, int SPL, int CPW>
 static mxb_status m3h_launch(const M3H& p, cudaStream_t st) {
-  MXB_LAUNCH("mamba3_head_fwd_kernel", st, (mamba3_head_fwd_kernel<IO, SPL, CPW><<<dim3(p.NH, p.B), 256, 0, st>>>(p)));
+  MXB_LAUNCH("mamba3_head_fwd_kernel", st, (launch_kernel(mamba3_head_fwd_kernel<IO, SPL, CPW>, dim3(p.NH, p.B), 256, 0, st, p)));
   return check_launch("mamba3_head_fwd_kernel");
 }
 template <typename IO, int SPL>
@@ -509,6 +513,7 @@ template <typename IO>
 __global__ void __launch_bounds__(128) m3h_reduce_kernel(const float* __restrict__ pb, const float* __restrict__ pc,
                                                          IO* __restrict__ db, IO* __restrict__ dc, int T, int N, int G,
                                                          int nchunks) {
+  begin_dependent();
   const int t = blockIdx.x, g = blockIdx.y, b = blockIdx.z, per = nchunks / G;
   for (int n = threadIdx.x; n < N; n += blockDim.x) {
     float sb = 0.f, sc = 0.f;
@@ -529,20 +534,20 @@ static mxb_status m3hb_launch(const M3HB& q, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(mamba3_head_bwd_kernel<IO, SPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) { set_last_cuda_error((int)e); return MXB_ERR_CUDA; }
   MXB_LAUNCH("mamba3_head_bwd_kernel", st,
-             (mamba3_head_bwd_kernel<IO, SPW><<<dim3(q.f.D / 16, q.f.B), 256, sm, st>>>(q)));
+             (launch_kernel(mamba3_head_bwd_kernel<IO, SPW>, dim3(q.f.D / 16, q.f.B), 256, sm, st, q)));
   mxb_status s = check_launch("mamba3_head_bwd_kernel");
   if (s != MXB_OK) return s;
   const int nchunks = q.f.D / 16;
   MXB_LAUNCH("m3h_reduce_kernel", st,
-             (m3h_reduce_kernel<IO><<<dim3(q.f.T, q.f.G, q.f.B), 128, 0, st>>>(q.pb, q.pc, static_cast<IO*>(q.db),
+             (launch_kernel(m3h_reduce_kernel<IO>, dim3(q.f.T, q.f.G, q.f.B), 128, 0, st, q.pb, q.pc, static_cast<IO*>(q.db),
                                                                             static_cast<IO*>(q.dc), q.f.T, q.f.N,
                                                                             q.f.G, nchunks)));
   const size_t rows = (size_t)q.f.B * q.f.T;
   const int hb = (int)((rows * q.f.NH + 255) / 256 < 1184 ? (rows * q.f.NH + 255) / 256 : 1184);
   MXB_LAUNCH("m3h_head_sum_kernel", st,
-             (m3h_head_sum_kernel<<<hb, 256, 0, st>>>(q.hpart, q.dtheta, q.ddt, q.dlam, rows, nchunks, q.f.NH)));
+             (launch_kernel(m3h_head_sum_kernel, hb, 256, 0, st, q.hpart, q.dtheta, q.ddt, q.dlam, rows, nchunks, q.f.NH)));
   MXB_LAUNCH("m3h_dalog_sum_kernel", st,
-             (m3h_dalog_sum_kernel<<<(q.f.NH + 127) / 128, 128, 0, st>>>(q.dalpart, q.da_log, q.f.B, nchunks, q.f.NH)));
+             (launch_kernel(m3h_dalog_sum_kernel, (q.f.NH + 127) / 128, 128, 0, st, q.dalpart, q.da_log, q.f.B, nchunks, q.f.NH)));
   return check_launch("m3h_reduce_kernel");
 }
 

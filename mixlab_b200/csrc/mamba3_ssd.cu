@@ -111,6 +111,7 @@ static_assert(sizeof(ChunkScal) % 16 == 0, "record moves in 16-byte units");
 constexpr int kScalUnits = sizeof(ChunkScal) / 16;
 
 __global__ void __launch_bounds__(64) m3s_chunk_scalars_kernel(SsdP p) {
+  begin_dependent();
   __shared__ __align__(16) ChunkScal s;
   __shared__ float sdt[Q];
   const int tid = threadIdx.x, c = blockIdx.x, head = blockIdx.y, b = blockIdx.z, t0 = c * Q;
@@ -281,6 +282,7 @@ __device__ __forceinline__ double cta_scan(double v, double* wtot) {
 // ------------------------------------------------------------ per-(b,head) scalars
 constexpr int kScalBatch = 4;
 __global__ void __launch_bounds__(kScalThreads) m3s_scalars_kernel(SsdP p) {
+  begin_dependent();
   __shared__ double wtot[kScalThreads / 32];
   const int head = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const size_t base = ((size_t)b * p.NH + head) * p.T;
@@ -358,6 +360,7 @@ struct PassMaps {
 // swizzled positions.
 template <bool TMA, int NS>
 __global__ void __launch_bounds__(kPassThreads<NS>, NS == 3 ? 2 : 1) m3s_state_pass_kernel(SsdP p, int mode, const __grid_constant__ PassMaps maps) {
+  begin_dependent();
   constexpr int NC = NS + 2;         // scalar records: the decay is read behind the product
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
@@ -494,6 +497,7 @@ constexpr int kOutSmem = 16384 * 2 + 8192 * 2 + sizeof(ChunkScal) + 64 + 1024;
 
 template <bool TMA>
 __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __grid_constant__ ChunkMaps maps) {
+  begin_dependent();
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
   uint8_t* Bt = sm;               // [64][128] Brot, then [128][64] H0
@@ -658,6 +662,7 @@ __device__ __forceinline__ void ld_pairs(uint32_t taddr, int warp, f2 (&f)[4]) {
 }
 template <bool TMA>
 __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p, const __grid_constant__ ChunkMaps maps) {
+  begin_dependent();
   extern __shared__ uint8_t raw[];
   uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
   uint8_t* Bt = sm;                    // [64][128] B, J B, C, CJ (swizzled slabs)
@@ -933,7 +938,8 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       tc::fence_async_smem();
       arrive(images);
       float hh = 0.f, jj = 0.f;  // <dH1, H0> and <dH1, J H0>
-      // By the warps that have nothing below the diagonal in the product to come: blocks of 16 state rows of dH1 times the same rows of H0 (mma.sync), whose diagonals and their neighbours are the row products that are wanted.
+      // By the warps that have nothing below the diagonal in the product to come: blocks of 16 state rows of dH1 times the
+      // same rows of H0 (mma.sync), whose diagonals and their neighbours are the row products that are wanted.
       if (above) {
         const uint32_t sh = tc::smem_u32(S + 16384), sd = sh + 16384;
         float d1[4] = {}, d2[4] = {};
@@ -1222,11 +1228,13 @@ __device__ __forceinline__ void reduce_rows(const bf16* __restrict__ pb, const b
 // as a kernel of their own at 8 x 4096 x 32 heads) are spread over the first half of the grid, where the streams of the
 // latter (90 us at the copy rate) keep DRAM busy beside them: 115 us together (124 with all of them first).
 __global__ void __launch_bounds__(kScalThreads) m3s_tail_kernel(SsdP p, bf16* __restrict__ db, bf16* __restrict__ dc, int stride) {
+  begin_dependent();
   const int nf = p.B * p.NH, block = blockIdx.x, q = block / stride, rem = block - q * stride;
   if (rem == 0 && q < nf) final_scalars(p, q % p.NH, q / p.NH);
   else reduce_rows(p.pb, p.pc, db, dc, p.T, p.G, p.splits, p.n, block - min(nf, q + 1));
 }
 __global__ void m3s_dalog_kernel(SsdP p) {
+  begin_dependent();
   const int head = blockIdx.x * blockDim.x + threadIdx.x;
   if (head >= p.NH) return;
   float s = 0.f;
@@ -1317,7 +1325,7 @@ static mxb_status ssd_state_pass(SsdP& p, int mode, cudaStream_t st) {
     constexpr int NS = decltype(ns)::value;
     if (MXB_ALLOW_SMEM(m3s::kPassSmem<NS>, m3s::m3s_state_pass_kernel<TMA, NS>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("m3s_state_pass_kernel", st,
-               (m3s::m3s_state_pass_kernel<TMA, NS><<<dim3(p.NH, p.B), m3s::kPassThreads<NS>, m3s::kPassSmem<NS>, st>>>(p, mode, maps)));
+               (launch_kernel(m3s::m3s_state_pass_kernel<TMA, NS>, dim3(p.NH, p.B), m3s::kPassThreads<NS>, m3s::kPassSmem<NS>, st, p, mode, maps)));
     return MXB_OK;
   };
   const std::integral_constant<int, 3> three;
@@ -1331,18 +1339,18 @@ static mxb_status ssd_state_pass(SsdP& p, int mode, cudaStream_t st) {
 
 static mxb_status ssd_forward(SsdP& p, cudaStream_t st) {
   const dim3 gc(p.n, p.NH, p.B);
-  MXB_LAUNCH("m3s_scalars_kernel", st, (m3s::m3s_scalars_kernel<<<dim3(p.NH, p.B), m3s::kScalThreads, 0, st>>>(p)));
-  MXB_LAUNCH("m3s_chunk_scalars_kernel", st, (m3s::m3s_chunk_scalars_kernel<<<gc, 64, 0, st>>>(p)));
+  MXB_LAUNCH("m3s_scalars_kernel", st, (launch_kernel(m3s::m3s_scalars_kernel, dim3(p.NH, p.B), m3s::kScalThreads, 0, st, p)));
+  MXB_LAUNCH("m3s_chunk_scalars_kernel", st, (launch_kernel(m3s::m3s_chunk_scalars_kernel, gc, 64, 0, st, p)));
   mxb_status ps = ssd_state_pass(p, 0, st);
   if (ps != MXB_OK) return ps;
   if (p.y) {
     m3s::ChunkMaps maps;
     if (ssd_chunk_maps(p, maps)) {
       if (MXB_ALLOW_SMEM(m3s::kOutSmem, m3s::m3s_chunk_out_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
-      MXB_LAUNCH("m3s_chunk_out_kernel", st, (m3s::m3s_chunk_out_kernel<true><<<gc, 128, m3s::kOutSmem, st>>>(p, maps)));
+      MXB_LAUNCH("m3s_chunk_out_kernel", st, (launch_kernel(m3s::m3s_chunk_out_kernel<true>, gc, 128, m3s::kOutSmem, st, p, maps)));
     } else {
       if (MXB_ALLOW_SMEM(m3s::kOutSmem, m3s::m3s_chunk_out_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
-      MXB_LAUNCH("m3s_chunk_out_kernel", st, (m3s::m3s_chunk_out_kernel<false><<<gc, 128, m3s::kOutSmem, st>>>(p, maps)));
+      MXB_LAUNCH("m3s_chunk_out_kernel", st, (launch_kernel(m3s::m3s_chunk_out_kernel<false>, gc, 128, m3s::kOutSmem, st, p, maps)));
     }
   }
   return check_launch("mamba3 ssd forward");
@@ -1380,16 +1388,16 @@ mxb_status mamba3_ssd_bwd(const mxb_mamba3_desc* d, const void* x, const float* 
   m3s::ChunkMaps maps;
   if (ssd_chunk_maps(p, maps)) {
     if (MXB_ALLOW_SMEM(m3s::kGradSmem, m3s::m3s_chunk_grad_kernel<true>) != MXB_OK) return MXB_ERR_CUDA;
-    MXB_LAUNCH("m3s_chunk_grad_kernel", st, (m3s::m3s_chunk_grad_kernel<true><<<gg, m3s::kGradThreads, m3s::kGradSmem, st>>>(p, maps)));
+    MXB_LAUNCH("m3s_chunk_grad_kernel", st, (launch_kernel(m3s::m3s_chunk_grad_kernel<true>, gg, m3s::kGradThreads, m3s::kGradSmem, st, p, maps)));
   } else {
     if (MXB_ALLOW_SMEM(m3s::kGradSmem, m3s::m3s_chunk_grad_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
-    MXB_LAUNCH("m3s_chunk_grad_kernel", st, (m3s::m3s_chunk_grad_kernel<false><<<gg, m3s::kGradThreads, m3s::kGradSmem, st>>>(p, maps)));
+    MXB_LAUNCH("m3s_chunk_grad_kernel", st, (launch_kernel(m3s::m3s_chunk_grad_kernel<false>, gg, m3s::kGradThreads, m3s::kGradSmem, st, p, maps)));
   }
   const int nf = p.B * p.NH, tail = nf + 2 * p.n * p.G * p.B;
   MXB_LAUNCH("m3s_tail_kernel", st,
-             (m3s::m3s_tail_kernel<<<tail, m3s::kScalThreads, 0, st>>>(p, static_cast<m3s::bf16*>(db), static_cast<m3s::bf16*>(dc),
+             (launch_kernel(m3s::m3s_tail_kernel, tail, m3s::kScalThreads, 0, st, p, static_cast<m3s::bf16*>(db), static_cast<m3s::bf16*>(dc),
                                                                        tail >= 2 * nf ? tail / (2 * nf) : 1)));
-  MXB_LAUNCH("m3s_dalog_kernel", st, (m3s::m3s_dalog_kernel<<<(p.NH + 127) / 128, 128, 0, st>>>(p)));
+  MXB_LAUNCH("m3s_dalog_kernel", st, (launch_kernel(m3s::m3s_dalog_kernel, (p.NH + 127) / 128, 128, 0, st, p)));
   return check_launch("mamba3 ssd backward");
 }
 

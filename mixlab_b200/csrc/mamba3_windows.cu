@@ -72,6 +72,7 @@ __device__ __forceinline__ f2 wrap2(f2 x) {
 }
 __global__ void __launch_bounds__(256) m3w_sincos_kernel(const float* __restrict__ x, size_t n, float* __restrict__ sn,
                                                          float* __restrict__ cs) {
+  begin_dependent();
   for (size_t i = 2 * (blockIdx.x * (size_t)blockDim.x + threadIdx.x); i < n; i += 2 * (size_t)gridDim.x * blockDim.x) {
     const bool two = i + 1 < n;
     f2 s, c;
@@ -228,6 +229,7 @@ constexpr int kRowBytes = (2 * W + 1) * 2 * PR * LPC * 4;
 // ------------------------------------------------------------------ prepare
 template <typename IO, int PR, int LPC>
 __global__ void __launch_bounds__(256) m3w_prepare_kernel(M3P p) {
+  begin_dependent();
   using K = Walker<IO, PR, LPC>;
   const K k(p, nullptr);
   f2 th[W][K::UN], ph[K::UN];
@@ -330,10 +332,13 @@ __device__ __forceinline__ void scan_chain(const M3P& p, int chains) {
     }
   }
 }
-__global__ void __launch_bounds__(32 * kSegs) m3w_phase_scan_kernel(M3P p) { scan_chain<kPhase>(p, p.D * p.Kp); }
-__global__ void __launch_bounds__(32 * kSegs) m3w_angle_scan_kernel(M3P p) { scan_chain<kAngle>(p, p.D * p.Kp); }
+__global__ void __launch_bounds__(32 * kSegs) m3w_phase_scan_kernel(M3P p) {
+  begin_dependent(); scan_chain<kPhase>(p, p.D * p.Kp); }
+__global__ void __launch_bounds__(32 * kSegs) m3w_angle_scan_kernel(M3P p) {
+  begin_dependent(); scan_chain<kAngle>(p, p.D * p.Kp); }
 // blockIdx.z: 0 the states, 1 dh (first: the one to start with)
 __global__ void __launch_bounds__(32 * kSegs) m3w_linear_scan_kernel(M3P p, int first) {
+  begin_dependent();
   if (first + (int)blockIdx.z == 0) scan_chain<kState>(p, p.D * p.N);
   else scan_chain<kDh>(p, p.D * p.N);
 }
@@ -345,6 +350,7 @@ __global__ void __launch_bounds__(32 * kSegs) m3w_linear_scan_kernel(M3P p, int 
 // decay of a step wait in shared memory for the way back.
 template <typename IO, int PR, int LPC, bool FWD, bool DH>
 __global__ void __launch_bounds__(256) m3w_local_kernel(M3P p) {
+  begin_dependent();
   using K = Walker<IO, PR, LPC>;
   constexpr int UN = K::UN;
   extern __shared__ f2 hist[];  // [W][2 PR][threads], then the rows
@@ -436,6 +442,7 @@ __global__ void __launch_bounds__(256) m3w_local_kernel(M3P p) {
 // ------------------------------------------------------------ forward walk
 template <typename IO, int PR, int LPC>
 __global__ void __launch_bounds__(256) m3w_out_kernel(M3P p) {
+  begin_dependent();
   using K = Walker<IO, PR, LPC>;
   constexpr int UN = K::UN;
   extern __shared__ f2 hist[];
@@ -526,6 +533,7 @@ struct GradSmem {  // bytes per thread, per warp and fixed
 // grid (D / channels of a CTA, windows, B)
 template <typename IO, int PR, int LPC>
 __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
+  begin_dependent();
   using K = Walker<IO, PR, LPC>;
   constexpr int UN = K::UN, CPW = K::CPW, KEEP = 4 * PR / CPW > 0 ? 4 * PR / CPW : 1, NR = 2 * K::NP;
   static_assert(4 * PR >= CPW, "a lane keeps at least one sum");
@@ -727,6 +735,7 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
 // (the walks used only the sums inside their own window).
 template <typename IO, int PR, int LPC>
 __global__ void __launch_bounds__(256) m3w_fix_kernel(M3P p) {
+  begin_dependent();
   using K = Walker<IO, PR, LPC>;
   constexpr int UN = K::UN;
   const K k(p, nullptr);
@@ -828,7 +837,7 @@ static mxb_status launch_local(const M3P& p, const M3WGrid& g, cudaStream_t st) 
   const int sm = per_thread * g.threads + rows;
   if (MXB_ALLOW_SMEM(per_thread * (PR == 4 ? 128 : 256) + rows, m3w_local_kernel<IO, PR, LPC, FWD, DH>) != MXB_OK) return MXB_ERR_CUDA;
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
-    MXB_LAUNCH("m3w_local_kernel", st, (m3w_local_kernel<IO, PR, LPC, FWD, DH><<<grid, g.threads, sm, st>>>(q)));
+    MXB_LAUNCH("m3w_local_kernel", st, (launch_kernel(m3w_local_kernel<IO, PR, LPC, FWD, DH>, grid, g.threads, sm, st, q)));
   });
   return MXB_OK;
 }
@@ -838,16 +847,16 @@ static mxb_status launch_grad(const M3P& p, const M3WGrid& g, cudaStream_t st) {
   if (MXB_ALLOW_SMEM((PR == 4 ? 4 : 8) * per_warp + rows, m3w_grad_kernel<IO, PR, LPC>) != MXB_OK) return MXB_ERR_CUDA;
   const int sm = g.shape.warps * per_warp + rows;
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
-    MXB_LAUNCH("m3w_grad_kernel", st, (m3w_grad_kernel<IO, PR, LPC><<<grid, g.threads, sm, st>>>(q)));
+    MXB_LAUNCH("m3w_grad_kernel", st, (launch_kernel(m3w_grad_kernel<IO, PR, LPC>, grid, g.threads, sm, st, q)));
   });
   return MXB_OK;
 }
 template <typename IO>
 static mxb_status prepare(const M3P& p, const M3WGrid& g, cudaStream_t st) {
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
-    M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_prepare_kernel", st, (m3w_prepare_kernel<IO, PRV, LPCV><<<grid, g.threads, 0, st>>>(q))));
+    M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_prepare_kernel", st, (launch_kernel(m3w_prepare_kernel<IO, PRV, LPCV>, grid, g.threads, 0, st, q))));
   });
-  MXB_LAUNCH("m3w_phase_scan_kernel", st, (m3w_phase_scan_kernel<<<chain_grid(p, p.D * p.Kp, 1), 32 * kSegs, 0, st>>>(p)));
+  MXB_LAUNCH("m3w_phase_scan_kernel", st, (launch_kernel(m3w_phase_scan_kernel, chain_grid(p, p.D * p.Kp, 1), 32 * kSegs, 0, st, p)));
   return check_launch("mamba3 window preparation");
 }
 
@@ -858,9 +867,9 @@ static mxb_status forward(const M3P& p, cudaStream_t st) {
   if (s != MXB_OK) return s;
   M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_local<IO, PRV, LPCV, true, false>(p, g, st)));
   if (s != MXB_OK) return s;
-  MXB_LAUNCH("m3w_linear_scan_kernel", st, (m3w_linear_scan_kernel<<<chain_grid(p, p.D * p.N, 1), 32 * kSegs, 0, st>>>(p, 0)));
+  MXB_LAUNCH("m3w_linear_scan_kernel", st, (launch_kernel(m3w_linear_scan_kernel, chain_grid(p, p.D * p.N, 1), 32 * kSegs, 0, st, p, 0)));
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
-    M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_out_kernel", st, (m3w_out_kernel<IO, PRV, LPCV><<<grid, g.threads, kRowBytes<IO, PRV, LPCV>, st>>>(q))));
+    M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_out_kernel", st, (launch_kernel(m3w_out_kernel<IO, PRV, LPCV>, grid, g.threads, kRowBytes<IO, PRV, LPCV>, st, q))));
   });
   return check_launch("mamba3 window-parallel forward");
 }
@@ -878,19 +887,19 @@ static mxb_status backward(const M3P& p, bool have_states, cudaStream_t st) {
   if (s != MXB_OK) return s;
   const int first = have_states ? 1 : 0;
   MXB_LAUNCH("m3w_linear_scan_kernel", st,
-             (m3w_linear_scan_kernel<<<chain_grid(p, p.D * p.N, 2 - first), 32 * kSegs, 0, st>>>(p, first)));
+             (launch_kernel(m3w_linear_scan_kernel, chain_grid(p, p.D * p.N, 2 - first), 32 * kSegs, 0, st, p, first)));
   M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_grad<IO, PRV, LPCV>(p, g, st)));
   if (s != MXB_OK) return s;
-  MXB_LAUNCH("m3w_angle_scan_kernel", st, (m3w_angle_scan_kernel<<<chain_grid(p, p.D * p.Kp, 1), 32 * kSegs, 0, st>>>(p)));
+  MXB_LAUNCH("m3w_angle_scan_kernel", st, (launch_kernel(m3w_angle_scan_kernel, chain_grid(p, p.D * p.Kp, 1), 32 * kSegs, 0, st, p)));
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
-    M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_fix_kernel", st, (m3w_fix_kernel<IO, PRV, LPCV><<<grid, g.threads, 0, st>>>(q))));
+    M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_fix_kernel", st, (launch_kernel(m3w_fix_kernel<IO, PRV, LPCV>, grid, g.threads, 0, st, q))));
   });
   return check_launch("mamba3 window-parallel backward");
 }
 
 mxb_status m3w_sincos_selftest(const float* x, size_t n, float* sn, float* cs, cudaStream_t st) {
   const int grid = (int)std::min<size_t>((n + 511) / 512, 148 * 8);
-  MXB_LAUNCH("m3w_sincos_kernel", st, (m3w_sincos_kernel<<<grid, 256, 0, st>>>(x, n, sn, cs)));
+  MXB_LAUNCH("m3w_sincos_kernel", st, (launch_kernel(m3w_sincos_kernel, grid, 256, 0, st, x, n, sn, cs)));
   return check_launch("m3w_sincos_kernel");
 }
 mxb_status m3w_forward(const M3P& p, bool f32, cudaStream_t st) {
