@@ -19,8 +19,7 @@
 //                           Brot^T diag(r e) X (or Crot^T diag(exp(Lam)) dY) folded into the running state
 //   m3s_chunk_out_kernel    per chunk: Y
 //   m3s_chunk_grad_kernel   per chunk and up to 16 heads of a group: dx, dB, dC summed over these heads, per-token scalars
-//   m3s_tail_kernel         per (b, head): ddt, dlambda, dtheta, da_log shares; per chunk:
-//                           dB, dC summed over the CTAs of a group
+//   m3s_tail_kernel         per chunk: ddt, dlambda, dtheta, da_log shares; dB, dC summed over the CTAs of a group
 #include <cuda.h>
 
 #include <algorithm>
@@ -55,7 +54,7 @@ struct SsdP {
   float *dt, *lam, *phi;        // [B,NH,T]
   bf16 *H0, *dH1;               // [B,NH,n,N,P] state at chunk start / state gradient at chunk end
   float *dphi, *da, *de, *dgam; // [B,NH,T] per-token scalar gradients (dphi: of the angle increment of a step)
-  float* dal_part;              // [B,NH] per-batch shares of da_log
+  float* dal_part;              // [B,n,NH] shares of da_log
   float* cs;                    // [B,NH,n] ChunkScal records
   bf16 *pb, *pc;                // [B,G*splits,n] column-blocked [64][128] images: partial dB, dC (summed in fp32 by the tail kernel)
 };
@@ -1148,64 +1147,63 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
 
 
 // ------------------------------------------------------------ final per-token scalars
-__device__ __forceinline__ void final_scalars(const SsdP& p, int head, int b) {
-  __shared__ float wsum[kScalThreads / 32];
+constexpr int kTailThreads = 512;
+constexpr int kTailHeads = 32;   // heads of a scalar block
+
+// ddt, dlambda, dtheta of the steps of a chunk and up to 32 heads, and their share of da_log.  The workspace has the steps of
+// a head in a row, the caller's tensors the heads of a step: the latter go through shared memory, so that both sides move whole
+// lines (a block per (batch, head) that walked the sequence read and wrote 4 bytes of every 32: 38 us at 8 x 4096 x 32 heads).
+__device__ __forceinline__ void final_scalars(const SsdP& p, int block) {
+  __shared__ float th[Q][kTailHeads + 1], dr[Q][kTailHeads + 1], dl[Q][kTailHeads + 1];  // theta -> dtheta, dt_raw -> ddt, dlambda
+  __shared__ float wsum[2 * kTailHeads];
+  const int groups = (p.NH + kTailHeads - 1) / kTailHeads, hg = block % groups, c = (block / groups) % p.n, b = block / groups / p.n;
+  const int h0 = hg * kTailHeads, nh = min(kTailHeads, p.NH - h0), t0 = c * Q, nt = min(Q, p.T - t0);
   const int tid = threadIdx.x;
-  const size_t base = ((size_t)b * p.NH + head) * p.T;
-  const float A = -expf(p.a_log[head]);
-  const int per = (p.T + kScalThreads - 1) / kScalThreads, lo = tid * per, hi = min(p.T, lo + per);
-  float dal = 0.f;
-  // backwards over this thread's steps, kFinalBatch at a time with the loads of a batch ahead of its stores
-  constexpr int kFinalBatch = 4;
-  for (int t1 = hi - 1; t1 >= lo; t1 -= kFinalBatch) {
-    float dph[kFinalBatch], dtv[kFinalBatch], lamv[kFinalBatch], thv[kFinalBatch], dgv[kFinalBatch], dev[kFinalBatch],
-        dnv[kFinalBatch], dav[kFinalBatch], drw[kFinalBatch];
-#pragma unroll
-    for (int x = 0; x < kFinalBatch; ++x) {
-      const int t = max(t1 - x, lo);
-      const size_t r = ((size_t)b * p.T + t) * p.NH + head;
-      dph[x] = p.dphi[base + t];
-      dtv[x] = p.dt[base + t];
-      lamv[x] = p.lam[base + t];
-      thv[x] = __ldg(p.theta + r);
-      drw[x] = __ldg(p.dt_raw + r);
-      dgv[x] = p.dgam[base + t];
-      dev[x] = p.de[base + t];
-      dnv[x] = t > 0 ? p.de[base + t - 1] : 0.f;
-      dav[x] = p.da[base + t];
-    }
-#pragma unroll
-    for (int x = 0; x < kFinalBatch; ++x) {
-      const int t = t1 - x;
-      if (t >= lo) {
-        const float dinc = dph[x];
-        const size_t r = ((size_t)b * p.T + t) * p.NH + head;
-        const float dt = dtv[x], lam = lamv[x];
-        const float dgam = dgv[x] + dev[x], dnxt = dnv[x], da = dav[x];
-        const float ddelta = A * da + lam * dgam + (1.f - lam) * dnxt + thv[x] * dinc;
-        p.ddt[r] = ddelta * sigmoid_f(drw[x]);
-        p.dlam[r] = dt * (dgam - dnxt) * lam * (1.f - lam);
-        p.dtheta[r] = dt * dinc;
-        dal = fmaf(dt, da, dal);
-      }
-    }
+  const size_t row0 = ((size_t)b * p.T + t0) * p.NH + h0;
+  for (int u = tid; u < Q * kTailHeads; u += kTailThreads) {
+    const int t = u / kTailHeads, h = u % kTailHeads;
+    const bool in = t < nt && h < nh;
+    th[t][h] = in ? __ldg(p.theta + row0 + (size_t)t * p.NH + h) : 0.f;
+    dr[t][h] = in ? __ldg(p.dt_raw + row0 + (size_t)t * p.NH + h) : 0.f;
   }
-  dal = warp_sum(dal);
-  if ((tid & 31) == 0) wsum[tid >> 5] = dal;
   __syncthreads();
-  if (tid == 0) {
-    float tot = 0.f;
-    for (int i = 0; i < kScalThreads / 32; ++i) tot += wsum[i];
-    p.dal_part[b * p.NH + head] = A * tot;  // summed over the batch in a fixed order by m3s_dalog_kernel
+#pragma unroll
+  for (int u = tid; u < Q * kTailHeads; u += kTailThreads) {
+    const int h = u / Q, t = u % Q;
+    float dal = 0.f;
+    if (t < nt && h < nh) {
+      const size_t o = ((size_t)b * p.NH + h0 + h) * p.T + t0 + t;
+      const float A = -expf(p.a_log[h0 + h]);
+      const float dt = p.dt[o], lam = p.lam[o], da = p.da[o], dinc = p.dphi[o];
+      const float dgam = p.dgam[o] + p.de[o], dnxt = t0 + t > 0 ? p.de[o - 1] : 0.f;
+      const float ddelta = A * da + lam * dgam + (1.f - lam) * dnxt + th[t][h] * dinc;
+      dr[t][h] = ddelta * sigmoid_f(dr[t][h]);
+      dl[t][h] = dt * (dgam - dnxt) * lam * (1.f - lam);
+      th[t][h] = dt * dinc;
+      dal = A * dt * da;
+    }
+    dal = warp_sum(dal);  // (a warp has 32 steps of one head)
+    if ((tid & 31) == 0) wsum[u >> 5] = dal;
   }
+  __syncthreads();
+  for (int u = tid; u < Q * kTailHeads; u += kTailThreads) {
+    const int t = u / kTailHeads, h = u % kTailHeads;
+    if (t < nt && h < nh) {
+      const size_t r = row0 + (size_t)t * p.NH + h;
+      p.ddt[r] = dr[t][h];
+      p.dlam[r] = dl[t][h];
+      p.dtheta[r] = th[t][h];
+    }
+  }
+  if (tid < nh) p.dal_part[((size_t)b * p.n + c) * p.NH + h0 + tid] = wsum[2 * tid] + wsum[2 * tid + 1];
 }
 // dB[b,t,g,:] = sum over the partial images of group g (fp32, fixed order).  A thread owns eight
 // states of a row; consecutive threads hold consecutive rows, which are neighbours in the column-blocked images.
 __device__ __forceinline__ void reduce_rows(const bf16* __restrict__ pb, const bf16* __restrict__ pc, bf16* __restrict__ db,
                                             bf16* __restrict__ dc, int T, int G, int per, int n, int block) {
-  static_assert(kScalThreads == N / 8 * Q, "a block covers one chunk of one gradient");
-  const int which = block & 1, r = threadIdx.x & 63, c8 = threadIdx.x >> 6;
-  int rest = block >> 1;
+  static_assert(2 * kTailThreads == N / 8 * Q, "a block covers half of the states of a chunk and one gradient");
+  const int which = (block >> 1) & 1, r = threadIdx.x & 63, c8 = (threadIdx.x >> 6) + 8 * (block & 1);
+  int rest = block >> 2;
   const int c = rest % n;
   rest /= n;
   const int g = rest % G, b = rest / G, t = c * Q + r;
@@ -1213,7 +1211,7 @@ __device__ __forceinline__ void reduce_rows(const bf16* __restrict__ pb, const b
   const uint4* src = reinterpret_cast<const uint4*>(which ? pc : pb) +
                      (((size_t)b * G + g) * per * n + c) * (N / 8 * Q) + c8 * Q + r;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
+#pragma unroll 4
   for (int h = 0; h < per; ++h) {
     float e[8];
     unpack8(__ldg(src + (size_t)h * n * (N / 8 * Q)), e);
@@ -1223,23 +1221,23 @@ __device__ __forceinline__ void reduce_rows(const bf16* __restrict__ pb, const b
   *reinterpret_cast<uint4*>((which ? dc : db) + (((size_t)b * T + t) * G + g) * N + 8 * c8) = pack8(acc);
 }
 
-// Every `stride`-th of the first blocks does the per-token scalars of a (batch, head), the others the row sums: both read
-// what the chunk kernel left.  One block fills an SM's registers, so the former (chains of dependent steps, DRAM idle: 38 us
-// as a kernel of their own at 8 x 4096 x 32 heads) are spread over the first half of the grid, where the streams of the
-// latter (90 us at the copy rate) keep DRAM busy beside them: 115 us together (124 with all of them first).
-__global__ void __launch_bounds__(kScalThreads) m3s_tail_kernel(SsdP p, bf16* __restrict__ db, bf16* __restrict__ dc, int stride) {
+// The first nf blocks do the per-token scalars, the others the row sums: both read what the chunk kernel left.
+__global__ void __launch_bounds__(kTailThreads, 3) m3s_tail_kernel(SsdP p, bf16* __restrict__ db, bf16* __restrict__ dc, int nf) {
   begin_dependent();
-  const int nf = p.B * p.NH, block = blockIdx.x, q = block / stride, rem = block - q * stride;
-  if (rem == 0 && q < nf) final_scalars(p, q % p.NH, q / p.NH);
-  else reduce_rows(p.pb, p.pc, db, dc, p.T, p.G, p.splits, p.n, block - min(nf, q + 1));
+  const int block = blockIdx.x;
+  if (block < nf) final_scalars(p, block);
+  else reduce_rows(p.pb, p.pc, db, dc, p.T, p.G, p.splits, p.n, block - nf);
 }
-__global__ void m3s_dalog_kernel(SsdP p) {
+// A warp per head; the lanes' shares and their sum in a fixed order.
+__global__ void __launch_bounds__(128) m3s_dalog_kernel(SsdP p) {
   begin_dependent();
-  const int head = blockIdx.x * blockDim.x + threadIdx.x;
+  const int head = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (head >= p.NH) return;
   float s = 0.f;
-  for (int b = 0; b < p.B; ++b) s += p.dal_part[b * p.NH + head];
-  p.da_log[head] = s;
+#pragma unroll 4
+  for (int u = lane; u < p.B * p.n; u += 32) s += p.dal_part[(size_t)u * p.NH + head];
+  s = warp_sum(s);
+  if (lane == 0) p.da_log[head] = s;
 }
 
 }  // namespace m3s
@@ -1269,7 +1267,7 @@ static size_t carve_ssd(SsdP& p, void* ws, bool bwd) {
     p.da = cv.take<float>(bh * p.T);
     p.de = cv.take<float>(bh * p.T);
     p.dgam = cv.take<float>(bh * p.T);
-    p.dal_part = cv.take<float>(bh);
+    p.dal_part = cv.take<float>(bh * p.n);
     const size_t images = (size_t)p.B * p.G * p.splits * p.n * m3s::Q * m3s::N;
     p.pb = cv.take<m3s::bf16>(images);
     p.pc = cv.take<m3s::bf16>(images);
@@ -1393,11 +1391,10 @@ mxb_status mamba3_ssd_bwd(const mxb_mamba3_desc* d, const void* x, const float* 
     if (MXB_ALLOW_SMEM(m3s::kGradSmem, m3s::m3s_chunk_grad_kernel<false>) != MXB_OK) return MXB_ERR_CUDA;
     MXB_LAUNCH("m3s_chunk_grad_kernel", st, (launch_kernel(m3s::m3s_chunk_grad_kernel<false>, gg, m3s::kGradThreads, m3s::kGradSmem, st, p, maps)));
   }
-  const int nf = p.B * p.NH, tail = nf + 2 * p.n * p.G * p.B;
+  const int nf = p.B * p.n * ((p.NH + m3s::kTailHeads - 1) / m3s::kTailHeads), tail = nf + 4 * p.n * p.G * p.B;
   MXB_LAUNCH("m3s_tail_kernel", st,
-             (launch_kernel(m3s::m3s_tail_kernel, tail, m3s::kScalThreads, 0, st, p, static_cast<m3s::bf16*>(db), static_cast<m3s::bf16*>(dc),
-                                                                       tail >= 2 * nf ? tail / (2 * nf) : 1)));
-  MXB_LAUNCH("m3s_dalog_kernel", st, (launch_kernel(m3s::m3s_dalog_kernel, (p.NH + 127) / 128, 128, 0, st, p)));
+             (launch_kernel(m3s::m3s_tail_kernel, tail, m3s::kTailThreads, 0, st, p, static_cast<m3s::bf16*>(db), static_cast<m3s::bf16*>(dc), nf)));
+  MXB_LAUNCH("m3s_dalog_kernel", st, (launch_kernel(m3s::m3s_dalog_kernel, (p.NH + 3) / 4, 128, 0, st, p)));
   return check_launch("mamba3 ssd backward");
 }
 
