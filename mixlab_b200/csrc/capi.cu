@@ -99,10 +99,10 @@ mxb_status gdn_f32io_bwd(const mxb_gdn_desc*, const void*, const void*, const vo
                          cudaStream_t);
 size_t gdn_tc_workspace_bytes(const mxb_gdn_desc*, bool bwd);
 mxb_status gdn_tc_fwd(const mxb_gdn_desc*, const void*, const void*, const void*, const float*,
-                      const float*, const float*, void*, float*, void*, cudaStream_t);
+                      const float*, const float*, void*, float* out32, float*, void*, cudaStream_t);
 mxb_status gdn_tc_bwd(const mxb_gdn_desc*, const void*, const void*, const void*, const float*,
-                      const float*, const float*, const void*, const float*, void*, void*, void*,
-                      float*, float*, float*, void*, cudaStream_t);
+                      const float*, const float*, const void*, const float*, void*, void*, void*, float* dq32,
+                      float* dk32, float* dv32, float*, float*, float*, void*, cudaStream_t);
 mxb_status umma_selftest(const void*, uint32_t, const void*, uint32_t, const uint32_t*, float*, int*, cudaStream_t);
 mxb_status wait_timeout_selftest(void*, uint32_t, cudaStream_t);
 mxb_status m3w_sincos_selftest(const float*, size_t, float*, float*, cudaStream_t);
@@ -240,7 +240,7 @@ mxb_status mxb_gdn_fwd(const mxb_gdn_desc* d, const void* q, const void* k, cons
     if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out) || !aligned16(h0) || !aligned16(hT))
       return MXB_ERR_ALIGNMENT;
     if (f32io) return gdn_f32io_fwd(d, q, k, v, beta, gate, h0, out, hT, workspace, st);
-    return gdn_tc_fwd(d, q, k, v, beta, gate, h0, out, hT, workspace, st);
+    return gdn_tc_fwd(d, q, k, v, beta, gate, h0, out, nullptr, hT, workspace, st);
   }
   if (!gdn_simt_supported(d)) return MXB_ERR_UNSUPPORTED;
   return gdn_simt_fwd(d, q, k, v, beta, gate, h0, out, hT, workspace, st);
@@ -265,7 +265,8 @@ mxb_status mxb_gdn_bwd(const mxb_gdn_desc* d, const void* q, const void* k, cons
       return MXB_ERR_ALIGNMENT;
     if (f32io)
       return gdn_f32io_bwd(d, q, k, v, beta, gate, h0, d_out, d_hT, dq, dk, dv, dbeta, dgate, dh0, workspace, st);
-    return gdn_tc_bwd(d, q, k, v, beta, gate, h0, d_out, d_hT, dq, dk, dv, dbeta, dgate, dh0, workspace, st);
+    return gdn_tc_bwd(d, q, k, v, beta, gate, h0, d_out, d_hT, dq, dk, dv, nullptr, nullptr, nullptr, dbeta, dgate, dh0,
+                      workspace, st);
   }
   if (!gdn_simt_supported(d)) return MXB_ERR_UNSUPPORTED;
   return gdn_simt_bwd(d, q, k, v, beta, gate, h0, d_out, d_hT, dq, dk, dv, dbeta, dgate, dh0, workspace, st);

@@ -427,8 +427,11 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chain_fwd_kernel(TcP p, const
         for (int u = lane; u < 16 * (NV / 8); u += 32) {
           const int i = r0 + u / (NV / 8), c8 = u % (NV / 8);
           const uint4 val = *reinterpret_cast<const uint4*>(Ot + slab64(i, c8));
-          if (c * C + i < p.T && col0 + 8 * c8 < p.Dv)
-            *reinterpret_cast<uint4*>(p.out + ((size_t)(b * p.T + c * C + i) * p.H + h) * p.Dv + col0 + 8 * c8) = val;
+          if (c * C + i < p.T && col0 + 8 * c8 < p.Dv) {
+            const size_t o = ((size_t)(b * p.T + c * C + i) * p.H + h) * p.Dv + col0 + 8 * c8;
+            if (p.out32) put_wide(p.out32 + o, val);
+            else *reinterpret_cast<uint4*>(p.out + o) = val;
+          }
         }
       }
       __syncwarp();

@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kStateThreads<NV>, 1) gdn_tc_state_fwd_kernel(
     tc::bulk_load(sPb + (c & 1) * 8192, p.P + ((size_t)bh * p.n + c) * C * C, 8192, &mbar[8 + (c & 1)]);
   };
   auto store_out = [&](int c) {
-    for (int sl = 0; sl < (TMA ? NV / 64 : 0); ++sl)  // a slab that lies wholly past the true width is not stored at all
+    for (int sl = 0; sl < (TMA && !p.out32 ? NV / 64 : 0); ++sl)  // a slab that lies wholly past the true width is not stored at all
       if (col0 + 64 * sl < p.Dv) tc::tma_store_4d(&maps.o, sOt + sl * 8192, col0 + 64 * sl, h, c * C, b);
   };
   // TMA = false: the q and k rows, by the 256 threads (a group per call, empty past the end)
@@ -531,7 +531,14 @@ __global__ void __launch_bounds__(kStateThreads<NV>, 1) gdn_tc_state_fwd_kernel(
                         tc::pack_bf16(f[8 * x + 2] + a[8 * x + 2], f[8 * x + 3] + a[8 * x + 3]),
                         tc::pack_bf16(f[8 * x + 4] + a[8 * x + 4], f[8 * x + 5] + a[8 * x + 5]),
                         tc::pack_bf16(f[8 * x + 6] + a[8 * x + 6], f[8 * x + 7] + a[8 * x + 7]));
-    if (TMA) {  // into the swizzled output tile; one thread hands it to the copy engine after the next barrier
+    if (p.out32) {
+      if (c * C + i < p.T) {
+        float* dst = p.out32 + grow(c, i) * p.Dv + col0 + j0;
+#pragma unroll
+        for (int x = 0; x < NC / 8; ++x)
+          if (col0 + j0 + 8 * x < p.Dv) put_wide(dst + 8 * x, o[x]);
+      }
+    } else if (TMA) {  // into the swizzled output tile; one thread hands it to the copy engine after the next barrier
 #pragma unroll
       for (int x = 0; x < NC / 8; ++x) sts16(Ot, tc::sw128_unit(i, NC / 8 * half + x), o[x]);
     } else if (c * C + i < p.T) {
@@ -767,8 +774,9 @@ mxb_status tc_run_fwd(TcP& p, cudaStream_t st) {
 }
 
 mxb_status gdn_tc_fwd(const mxb_gdn_desc* d, const void* q, const void* k, const void* v, const float* beta,
-                      const float* gate, const float* h0, void* out, float* hT, void* ws, cudaStream_t st) {
+                      const float* gate, const float* h0, void* out, float* out32, float* hT, void* ws, cudaStream_t st) {
   TcP p = make_tc(d);
+  p.out32 = out32;
   p.q = static_cast<const bf16*>(q); p.k = static_cast<const bf16*>(k); p.v = static_cast<const bf16*>(v);
   p.beta = beta; p.gate = gate; p.h0 = h0; p.out = static_cast<bf16*>(out); p.hT = hT;
   p.save = (d->flags & MXB_GDN_SAVE_FOR_BWD) ? 1 : 0;
@@ -779,7 +787,8 @@ mxb_status gdn_tc_fwd(const mxb_gdn_desc* d, const void* q, const void* k, const
 
 mxb_status gdn_tc_bwd(const mxb_gdn_desc* d, const void* q, const void* k, const void* v, const float* beta,
                       const float* gate, const float* h0, const void* dO, const float* dhT, void* dq, void* dk,
-                      void* dv, float* dbeta, float* dgate, float* dh0, void* ws, cudaStream_t st) {
+                      void* dv, float* dq32, float* dk32, float* dv32, float* dbeta, float* dgate, float* dh0, void* ws,
+                      cudaStream_t st) {
   if (d->flags & MXB_GDN_BWD_FP32_KERNELS) {  // what a forward saved is in these kernels' layout: the others recompute
     mxb_gdn_desc own = *d;
     own.flags &= ~MXB_GDN_BWD_USE_SAVED;
@@ -790,6 +799,7 @@ mxb_status gdn_tc_bwd(const mxb_gdn_desc* d, const void* q, const void* k, const
   p.beta = beta; p.gate = gate; p.h0 = h0;
   p.dO = static_cast<const bf16*>(dO); p.dhT_in = dhT;
   p.dq = static_cast<bf16*>(dq); p.dk = static_cast<bf16*>(dk); p.dv = static_cast<bf16*>(dv);
+  p.dq32 = dq32; p.dk32 = dk32; p.dv32 = dv32;
   p.dbeta = dbeta; p.dgate = dgate; p.dh0 = dh0;
   p.no_tma = (d->flags & MXB_GDN_NO_TMA) ? 1 : 0;
   carve_tc(p, ws, true);

@@ -34,6 +34,8 @@ struct TcP {
   const bf16* dO;
   const float* dhT_in;
   bf16 *dq, *dk, *dv;
+  // float32 tensors on these kernels: the results go there, rounded to bf16 all the same, and the bf16 tensors above are scratch
+  float *out32, *dq32, *dk32, *dv32;
   float *dbeta, *dgate, *dh0;
   int* status;   // device word: nonzero when a bounded wait gave up
   // workspace, indexed by ci = (b*H+h)*n + chunk
@@ -70,6 +72,21 @@ __device__ __forceinline__ int urow16(int u) { return ((u >> 7) << 3) | (u & 7);
 __device__ __forceinline__ int ucol16(int u) { return (u >> 3) & 15; }
 __device__ __forceinline__ int urow8(int u) { return ((u >> 6) << 3) | (u & 7); }
 __device__ __forceinline__ int ucol8(int u) { return (u >> 3) & 7; }
+// Eight bf16 as floats (a bf16 is the upper half of the float with the same value).
+__device__ __forceinline__ void put_wide(float* dst, uint4 v) {
+  reinterpret_cast<float4*>(dst)[0] = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u),
+                                                  __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+  reinterpret_cast<float4*>(dst)[1] = make_float4(__uint_as_float(v.z << 16), __uint_as_float(v.z & 0xffff0000u),
+                                                  __uint_as_float(v.w << 16), __uint_as_float(v.w & 0xffff0000u));
+}
+// A finished tile in the layout of a TMA box as rows of a float32 tensor [B,T,H,D], by 256 threads; row0: its first row.
+__device__ __forceinline__ void put_wide_tile(float* dst, const uint8_t* tile, size_t row0, int H, int D, int imax) {
+  const int w8 = D / 8;
+  for (int u = threadIdx.x; u < imax * w8; u += 256) {
+    const int i = u / w8, c8 = u % w8;
+    put_wide(dst + (row0 + (size_t)i * H) * D + 8 * c8, *reinterpret_cast<const uint4*>(tile + tc::sw128_unit(i, c8)));
+  }
+}
 __device__ __forceinline__ uint4 zero16() { return make_uint4(0u, 0u, 0u, 0u); }
 
 // Loads 32 fp32 accumulator columns [c0, c0+32) of this thread's TMEM lane.

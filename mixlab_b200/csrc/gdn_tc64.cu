@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_state_fwd_kernel(TcP p, const _
         tc::bulk_commit();
       }
     }
-    if (tid == 96 && c > 0) {  // the previous chunk's output tile (complete since the barrier above)
+    if (tid == 96 && c > 0 && !p.out32) {  // the previous chunk's output tile (complete since the barrier above)
       tc::tma_store_4d(&maps.o, tc::smem_u32(Ot), 0, h, t0 - C, b);
       tc::bulk_commit();
     }
@@ -379,7 +379,10 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_state_fwd_kernel(TcP p, const _
 #pragma unroll
         for (int jj = 0; jj < 32; ++jj) a[jj] += f[jj];
 #pragma unroll
-        for (int x = 0; x < 4; ++x) sts16(Ot, sw_unit(i, 4 * half + x), pack8(&a[8 * x]));
+        for (int x = 0; x < 4; ++x) {
+          if (!p.out32) sts16(Ot, sw_unit(i, 4 * half + x), pack8(&a[8 * x]));
+          else if (t0 + i < p.T) put_wide(p.out32 + ((size_t)(b * p.T + t0 + i) * p.H + h) * W + j0 + 8 * x, pack8(&a[8 * x]));
+        }
       } else {      // S <- E(gam_last) S + (k r)^T v_new
 #pragma unroll
         for (int jj = 0; jj < 32; ++jj) S[jj] = fmaf(L, S[jj], a[jj]);
@@ -389,7 +392,7 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_state_fwd_kernel(TcP p, const _
   }
   tc::fence_async_smem();
   __syncthreads();
-  if (ok && tid == 96) {  // the last chunk's output tile
+  if (ok && tid == 96 && !p.out32) {  // the last chunk's output tile
     tc::tma_store_4d(&maps.o, tc::smem_u32(Ot), 0, h, (p.n - 1) * C, b);
     tc::bulk_commit();
   }
@@ -851,7 +854,12 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
   dgo[qd * C + i] = dg_own;  // (every product that read Mb has completed)
   dbo[qd * C + i] = db_own;
   publish();
-  if (ok && tid == 64) {  // rows past the end of the sequence are clipped
+  if (ok && p.dq32) {
+    const size_t row0 = (size_t)(b * p.T + t0) * p.H + h;
+    put_wide_tile(p.dq32, Xvn, row0, p.H, W, imax);
+    put_wide_tile(p.dk32, Xt, row0, p.H, W, imax);
+    put_wide_tile(p.dv32, Xe, row0, p.H, W, imax);
+  } else if (ok && tid == 64) {  // rows past the end of the sequence are clipped
     tc::tma_store_4d(&maps.dq, tc::smem_u32(Xvn), 0, h, t0, b);
     tc::tma_store_4d(&maps.dk, tc::smem_u32(Xt), 0, h, t0, b);
     tc::tma_store_4d(&maps.dv, tc::smem_u32(Xe), 0, h, t0, b);

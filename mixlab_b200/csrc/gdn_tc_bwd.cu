@@ -645,7 +645,12 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
   tc::fence_async_smem();
   tc::fence_before_sync();
   __syncthreads();
-  if (ok && tid == 64) {  // dq, dk and dv leave by tiled stores (rows past the end of the sequence are clipped)
+  if (ok && p.dq32) {
+    const size_t row0 = (size_t)(b * p.T + t0) * p.H + h;
+    put_wide_tile(p.dq32, Xvn, row0, p.H, p.Dk, imax);
+    put_wide_tile(p.dk32, Xdk, row0, p.H, p.Dk, imax);
+    put_wide_tile(p.dv32, Xe, row0, p.H, p.Dv, imax);
+  } else if (ok && tid == 64) {  // dq, dk and dv leave by tiled stores (rows past the end of the sequence are clipped)
     for (int sl = 0; sl < 2; ++sl) {  // a slab that lies wholly past the true width is not stored at all
       if (64 * sl < p.Dk) {
         tc::tma_store_4d(&maps.dq, tc::smem_u32(Xvn) + 8192 * sl, 64 * sl, h, t0, b);

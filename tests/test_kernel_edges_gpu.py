@@ -270,3 +270,28 @@ def test_gdn_state_passes_agree_bit_for_bit(T, K, V, batches):
         part = run(nb)
         for n in whole:
             assert torch.equal(whole[n][:nb], part[n]), (nb, n)
+
+
+@pytest.mark.parametrize("B,T,K,V", [
+    (2, 150, 128, 128), (9, 65, 128, 72), (18, 130, 72, 128), (40, 70, 128, 128),   # state passes of 16, 32, 64, 128 columns
+    (2, 100, 64, 64), (18, 64, 64, 64), (40, 66, 64, 64), (40, 66, 96, 88),         # heads of 64 columns; widths between
+])
+def test_float32_results_of_the_tensor_core_kernels(B, T, K, V):
+    """Float32 tensors through the tensor-core kernels: every state pass and chunk kernel writes its rounded results as
+    float32 itself, so they are the bf16 entry's results, widened (gradients from a saved and from a recomputed forward)."""
+    a = inputs.gdn_inputs(B, T, 4, K, V, seed=23, io_dtype=BF16, with_grad_out=True)
+    low = [_dev(a[n]) for n in ("q", "k", "v", "beta", "g")]
+    wide = [t.float() for t in low]
+    d_low = _dev(a["d_out"])
+    kw, flag = dict(gate_is_log=True), _lib.MXB_GDN_F32_IO_BF16_OPERANDS
+    want_o = ops.gated_delta_scan(*low, 64, **kw)
+    want = ops.gated_delta_scan_backward(*low, d_low, 64, **kw)
+    o = ops.gated_delta_scan(*wide, 64, flags=flag, save_for_backward=True, **kw)
+    saved = ops.gated_delta_scan_backward(*wide, d_low.float(), 64, flags=flag, use_saved=True, **kw)
+    again = ops.gated_delta_scan_backward(*wide, d_low.float(), 64, flags=flag, **kw)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    assert o.dtype == F32 and torch.equal(o, want_o.float())
+    for n in ("dq", "dk", "dv", "dbeta", "dgate"):
+        assert torch.equal(saved[n], want[n].float()), n
+        assert torch.equal(again[n], want[n].float()), n
