@@ -99,7 +99,7 @@ __device__ __forceinline__ void ld_acc32(uint32_t taddr, int warp, int c0, float
 }
 // The sequential passes of 128-wide heads take half of the state's columns per CTA where that still puts every CTA on an
 // SM of its own: the chain of a chunk is what counts then, not the bytes (forward and backward, us a chunk: 2.55 and 2.4
-// with all columns, 1.9 and 1.8 with half of them).
+// with all columns, 1.9 and 1.8 with half of them).  Fewer heads yet: gdn_chain.cu.
 inline bool tc_split_columns(const TcP& p) { return p.Dv > 64 && 2 * p.B * p.H <= 148; }
 
 // Threads of a forward state-pass CTA: 256 that hold the state and run the epilogues, and a warp of one issuing thread (on
