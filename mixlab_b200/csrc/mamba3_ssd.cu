@@ -13,8 +13,8 @@
 // hand-derived adjoint of these two lines (checked against float64 autograd of the recurrence
 // before it was written); its sequential part is the mirrored scan dH0 = L dH1 + Dc.
 //
-//   m3s_scalars_kernel      per (b, head): dt, lambda, wrapped cumulative angle (fp64 prefix sum)
-//   m3s_chunk_scalars_kernel per chunk: decay sums, trapezoid weights, rotation sines/cosines (one record)
+//   m3s_scalars_kernel      per chunk: dt, lambda, the chunk's share of the angle (fp64)
+//   m3s_chunk_scalars_kernel per chunk: decay sums, trapezoid weights, sines/cosines of the cumulative angle (one record)
 //   m3s_state_pass_kernel   per (b, head), sequential over the chunks, forward or reverse: the chunk contribution
 //                           Brot^T diag(r e) X (or Crot^T diag(exp(Lam)) dY) folded into the running state
 //   m3s_chunk_out_kernel    per chunk: Y
@@ -51,7 +51,7 @@ struct SsdP {
   float *ddt, *dlam, *dtheta, *da_log;
   int* status;
   // workspace
-  float *dt, *lam, *phi;        // [B,NH,T]
+  float *dt, *lam, *theta_t;    // [B,NH,T]
   bf16 *H0, *dH1;               // [B,NH,n,N,P] state at chunk start / state gradient at chunk end
   float *dphi, *da, *de, *dgam; // [B,NH,T] per-token scalar gradients (dphi: of the angle increment of a step)
   float* dal_part;              // [B,n,NH] shares of da_log
@@ -109,10 +109,11 @@ struct ChunkScal {
 static_assert(sizeof(ChunkScal) % 16 == 0, "record moves in 16-byte units");
 constexpr int kScalUnits = sizeof(ChunkScal) / 16;
 
-__global__ void __launch_bounds__(64) m3s_chunk_scalars_kernel(SsdP p) {
+__global__ void __launch_bounds__(64) m3s_chunk_scalars_kernel(SsdP p, const double* share) {
   begin_dependent();
   __shared__ __align__(16) ChunkScal s;
   __shared__ float sdt[Q];
+  __shared__ double wsum[4];
   const int tid = threadIdx.x, c = blockIdx.x, head = blockIdx.y, b = blockIdx.z, t0 = c * Q;
   const size_t base = ((size_t)b * p.NH + head) * p.T;
   const size_t ci = ((size_t)b * p.NH + head) * p.n + c;
@@ -125,8 +126,26 @@ __global__ void __launch_bounds__(64) m3s_chunk_scalars_kernel(SsdP p) {
     sdt[tid] = dt;
     s.gam[tid] = lam * dt;
     s.e[tid] = lam * dt + nxt;
+    // cumulative rotation angle in fp64: the shares of the chunks in front, then the steps of this one
+    double before = 0.0, phi = ok ? (double)dt * (double)p.theta_t[base + t] : 0.0;
+    for (int x = tid; x < c; x += Q) before += share[((size_t)b * p.n + x) * p.NH + head];
+    const int lane = tid & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double up = __shfl_up_sync(0xffffffffu, phi, o);
+      if (lane >= o) phi += up;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (lane == 31) {
+      wsum[tid >> 5] = before;
+      wsum[2 + (tid >> 5)] = phi;
+    }
+    __syncthreads();
+    phi += wsum[0] + wsum[1] + (tid >= 32 ? wsum[2] : 0.0);
+    const double two_pi = 6.283185307179586476925, inv_two_pi = 1.0 / two_pi;
     float sn = 0.f, cs = 1.f;
-    if (ok) sincosf(p.phi[base + t], &sn, &cs);
+    if (ok) sincosf((float)(phi - two_pi * rint(phi * inv_two_pi)), &sn, &cs);  // wrapped to [-pi, pi]
     s.sn[tid] = sn; s.cs[tid] = cs;
   }
   __syncthreads();
@@ -256,78 +275,48 @@ struct ChunkMaps {
   CUtensorMap x, dy, dx;  // [B,T,heads,64] viewed as (P, heads, T, B)
 };
 
-// Threads of the two per-(batch, head) scalar kernels: they are chains of dependent fp64 operations behind strided
-// loads, so many short chains (4 steps per thread at T = 4096) hide the latencies that few long ones expose.
-constexpr int kScalThreads = 1024;
-// Inclusive prefix sum of one double per thread over a kScalThreads-thread CTA (warp scans + the warp totals, a fixed
-// order); wtot is kScalThreads / 32 doubles of shared memory.
-__device__ __forceinline__ double cta_scan(double v, double* wtot) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const double t = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += t;
-  }
-  if (lane == 31) wtot[warp] = v;
-  __syncthreads();
-  double off = 0.0;
-#pragma unroll
-  for (int w = 0; w < kScalThreads / 32; ++w) {
-    if (w < warp) off += wtot[w];
-  }
-  return v + off;
-}
+// ------------------------------------------------------------ per-token scalars
+constexpr int kScalThreads = 256;
+constexpr int kScalHeads = 8;    // heads of a block: 32 bytes of a step, so that a small call still spreads over SMs
 
-// ------------------------------------------------------------ per-(b,head) scalars
-constexpr int kScalBatch = 4;
-__global__ void __launch_bounds__(kScalThreads) m3s_scalars_kernel(SsdP p) {
+// dt, lambda and theta of a chunk's steps and up to 8 heads, from the caller's [B,T,heads] to rows of [B,heads,T] through shared
+// memory (whole sectors on both sides), and the chunk's share of the rotation angle, in fp64, into `share` [B,n,heads].
+__global__ void __launch_bounds__(kScalThreads) m3s_scalars_kernel(SsdP p, double* share) {
   begin_dependent();
-  __shared__ double wtot[kScalThreads / 32];
-  const int head = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
-  const size_t base = ((size_t)b * p.NH + head) * p.T;
-  const int per = (p.T + kScalThreads - 1) / kScalThreads, lo = tid * per, hi = min(p.T, lo + per);
-  if (head == 0 && b == 0 && tid < 64) p.status[tid] = 0;  // (the kernels behind this one raise it)
-  // Batches of kScalBatch steps: all loads of a batch are issued before its first store (a store in between would
-  // pin the order, since the compiler cannot prove the arrays distinct, and every step would pay a full memory latency).
-  double acc = 0.0;
-  for (int t0 = lo; t0 < hi; t0 += kScalBatch) {
-    float draw[kScalBatch], lraw[kScalBatch], th[kScalBatch];
+  __shared__ float dr[Q][kScalHeads + 1], lr[Q][kScalHeads + 1], th[Q][kScalHeads + 1];
+  __shared__ double wsum[2 * kScalHeads];
+  const int c = blockIdx.y, b = blockIdx.z, h0 = blockIdx.x * kScalHeads, nh = min(kScalHeads, p.NH - h0), t0 = c * Q, nt = min(Q, p.T - t0);
+  const int tid = threadIdx.x;
+  if (blockIdx.x == 0 && c == 0 && b == 0 && tid < 64) p.status[tid] = 0;  // (the kernels behind this one raise it)
+  const size_t row0 = ((size_t)b * p.T + t0) * p.NH + h0;
 #pragma unroll
-    for (int x = 0; x < kScalBatch; ++x) {
-      const int t = min(t0 + x, hi - 1);
-      const size_t r = ((size_t)b * p.T + t) * p.NH + head;
-      draw[x] = __ldg(p.dt_raw + r);
-      lraw[x] = __ldg(p.lam_raw + r);
-      th[x] = __ldg(p.theta + r);
-    }
-#pragma unroll
-    for (int x = 0; x < kScalBatch; ++x) {
-      if (t0 + x < hi) {
-        const float dt = softplus_f(draw[x]);
-        p.dt[base + t0 + x] = dt;
-        p.lam[base + t0 + x] = sigmoid_f(lraw[x]);
-        acc += (double)dt * (double)th[x];
-      }
-    }
+  for (int x = 0; x < Q * kScalHeads / kScalThreads; ++x) {
+    const int u = tid + x * kScalThreads, t = u / kScalHeads, h = u % kScalHeads;
+    const bool in = t < nt && h < nh;
+    const size_t r = in ? row0 + (size_t)t * p.NH + h : row0;
+    dr[t][h] = __ldg(p.dt_raw + r);
+    lr[t][h] = __ldg(p.lam_raw + r);
+    th[t][h] = __ldg(p.theta + r);
   }
-  double phi = cta_scan(acc, wtot) - acc;  // angle at the start of this thread's steps
-  const double two_pi = 6.283185307179586476925, inv_two_pi = 1.0 / two_pi;
-  for (int t0 = lo; t0 < hi; t0 += kScalBatch) {
-    float dtv[kScalBatch], th[kScalBatch];
+  __syncthreads();
 #pragma unroll
-    for (int x = 0; x < kScalBatch; ++x) {
-      const int t = min(t0 + x, hi - 1);
-      dtv[x] = p.dt[base + t];
-      th[x] = __ldg(p.theta + ((size_t)b * p.T + t) * p.NH + head);
+  for (int x = 0; x < Q * kScalHeads / kScalThreads; ++x) {
+    const int u = tid + x * kScalThreads, h = u / Q, t = u % Q;
+    double inc = 0.0;
+    if (t < nt && h < nh) {
+      const size_t o = ((size_t)b * p.NH + h0 + h) * p.T + t0 + t;
+      const float dt = softplus_f(dr[t][h]), theta = th[t][h];
+      p.dt[o] = dt;
+      p.lam[o] = sigmoid_f(lr[t][h]);
+      p.theta_t[o] = theta;
+      inc = (double)dt * (double)theta;
     }
 #pragma unroll
-    for (int x = 0; x < kScalBatch; ++x) {
-      if (t0 + x < hi) {
-        phi += (double)dtv[x] * (double)th[x];
-        p.phi[base + t0 + x] = (float)(phi - two_pi * rint(phi * inv_two_pi));  // wrapped to [-pi, pi]
-      }
-    }
+    for (int o = 16; o > 0; o >>= 1) inc += __shfl_xor_sync(0xffffffffu, inc, o);  // (a warp has 32 steps of one head)
+    if ((tid & 31) == 0) wsum[u >> 5] = inc;
   }
+  __syncthreads();
+  if (tid < nh) share[((size_t)b * p.n + c) * p.NH + h0 + tid] = wsum[2 * tid] + wsum[2 * tid + 1];
 }
 
 // ------------------------------------------------------------ state pass
@@ -1258,7 +1247,7 @@ static size_t carve_ssd(SsdP& p, void* ws, bool bwd) {
   p.status = cv.take<int>(64);
   p.dt = cv.take<float>(bh * p.T);
   p.lam = cv.take<float>(bh * p.T);
-  p.phi = cv.take<float>(bh * p.T);
+  p.theta_t = cv.take<float>(bh * p.T);
   p.cs = cv.take<float>(bh * p.n * (sizeof(m3s::ChunkScal) / 4));
   p.H0 = cv.take<m3s::bf16>(nst);
   if (bwd) {
@@ -1337,8 +1326,11 @@ static mxb_status ssd_state_pass(SsdP& p, int mode, cudaStream_t st) {
 
 static mxb_status ssd_forward(SsdP& p, cudaStream_t st) {
   const dim3 gc(p.n, p.NH, p.B);
-  MXB_LAUNCH("m3s_scalars_kernel", st, (launch_kernel(m3s::m3s_scalars_kernel, dim3(p.NH, p.B), m3s::kScalThreads, 0, st, p)));
-  MXB_LAUNCH("m3s_chunk_scalars_kernel", st, (launch_kernel(m3s::m3s_chunk_scalars_kernel, gc, 64, 0, st, p)));
+  // (the chunks' shares of the angle lie where the state pass writes the chunk states afterwards)
+  double* share = reinterpret_cast<double*>(p.H0);
+  MXB_LAUNCH("m3s_scalars_kernel", st,
+             (launch_kernel(m3s::m3s_scalars_kernel, dim3((p.NH + m3s::kScalHeads - 1) / m3s::kScalHeads, p.n, p.B), m3s::kScalThreads, 0, st, p, share)));
+  MXB_LAUNCH("m3s_chunk_scalars_kernel", st, (launch_kernel(m3s::m3s_chunk_scalars_kernel, gc, 64, 0, st, p, static_cast<const double*>(share))));
   mxb_status ps = ssd_state_pass(p, 0, st);
   if (ps != MXB_OK) return ps;
   if (p.y) {
