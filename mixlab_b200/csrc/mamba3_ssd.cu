@@ -245,29 +245,32 @@ __device__ __forceinline__ tc::Tile in_mnmajor(const void* ptr, int W) {
 }
 template <bool SW>
 __device__ __forceinline__ void rotate_in_tile(uint8_t* tile, const float* sn, const float* cs, int tid, int nt) {
-  if (!SW) { rotate_tile(tile, sn, cs); return; }
-  // four units per pass, all loads before the first store (a store in between would pin the order of the
-  // loads that follow it); unit w of a slab belongs to row w / 8
-  for (int w0 = tid; w0 < Q * 16; w0 += 4 * nt) {
-    uint4 raw[4];
-    float sv[4], cv[4];
+  if constexpr (!SW) {
+    rotate_tile(tile, sn, cs);
+  } else {
+    // four units per pass, all loads before the first store (a store in between would pin the order of the
+    // loads that follow it); unit w of a slab belongs to row w / 8
+    for (int w0 = tid; w0 < Q * 16; w0 += 4 * nt) {
+      uint4 raw[4];
+      float sv[4], cv[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int w = min(w0 + q * nt, Q * 16 - 1), t = (w >> 3) & 63;
-      raw[q] = *reinterpret_cast<const uint4*>(tile + 16 * w);
-      sv[q] = sn[t]; cv[q] = cs[t];
+      for (int q = 0; q < 4; ++q) {
+        const int w = min(w0 + q * nt, Q * 16 - 1), t = (w >> 3) & 63;
+        raw[q] = *reinterpret_cast<const uint4*>(tile + 16 * w);
+        sv[q] = sn[t]; cv[q] = cs[t];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        auto rot = [&](uint32_t w) {
+          const float2 v = unpack2(widen2(w));
+          return tc::pack_bf16(fmaf(cv[q], v.x, sv[q] * v.y), fmaf(cv[q], v.y, -(sv[q] * v.x)));
+        };
+        raw[q] = make_uint4(rot(raw[q].x), rot(raw[q].y), rot(raw[q].z), rot(raw[q].w));
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (w0 + q * nt < Q * 16) *reinterpret_cast<uint4*>(tile + 16 * (w0 + q * nt)) = raw[q];
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      auto rot = [&](uint32_t w) {
-        const float2 v = unpack2(widen2(w));
-        return tc::pack_bf16(fmaf(cv[q], v.x, sv[q] * v.y), fmaf(cv[q], v.y, -(sv[q] * v.x)));
-      };
-      raw[q] = make_uint4(rot(raw[q].x), rot(raw[q].y), rot(raw[q].z), rot(raw[q].w));
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (w0 + q * nt < Q * 16) *reinterpret_cast<uint4*>(tile + 16 * (w0 + q * nt)) = raw[q];
   }
 }
 struct ChunkMaps {
