@@ -288,9 +288,11 @@ __global__ void __launch_bounds__(kScalThreads) m3s_scalars_kernel(SsdP p, doubl
   begin_dependent();
   __shared__ float dr[Q][kScalHeads + 1], lr[Q][kScalHeads + 1], th[Q][kScalHeads + 1];
   __shared__ double wsum[2 * kScalHeads];
-  const int c = blockIdx.y, b = blockIdx.z, h0 = blockIdx.x * kScalHeads, nh = min(kScalHeads, p.NH - h0), t0 = c * Q, nt = min(Q, p.T - t0);
+  // (chunks and groups of heads share the x axis: the others end at 65,535)
+  const int groups = (p.NH + kScalHeads - 1) / kScalHeads, c = blockIdx.x / groups, b = blockIdx.y;
+  const int h0 = blockIdx.x % groups * kScalHeads, nh = min(kScalHeads, p.NH - h0), t0 = c * Q, nt = min(Q, p.T - t0);
   const int tid = threadIdx.x;
-  if (blockIdx.x == 0 && c == 0 && b == 0 && tid < 64) p.status[tid] = 0;  // (the kernels behind this one raise it)
+  if (blockIdx.x == 0 && b == 0 && tid < 64) p.status[tid] = 0;  // (the kernels behind this one raise it)
   const size_t row0 = ((size_t)b * p.T + t0) * p.NH + h0;
 #pragma unroll
   for (int x = 0; x < Q * kScalHeads / kScalThreads; ++x) {
@@ -1332,7 +1334,7 @@ static mxb_status ssd_forward(SsdP& p, cudaStream_t st) {
   // (the chunks' shares of the angle lie where the state pass writes the chunk states afterwards)
   double* share = reinterpret_cast<double*>(p.H0);
   MXB_LAUNCH("m3s_scalars_kernel", st,
-             (launch_kernel(m3s::m3s_scalars_kernel, dim3((p.NH + m3s::kScalHeads - 1) / m3s::kScalHeads, p.n, p.B), m3s::kScalThreads, 0, st, p, share)));
+             (launch_kernel(m3s::m3s_scalars_kernel, dim3(p.n * ((p.NH + m3s::kScalHeads - 1) / m3s::kScalHeads), p.B), m3s::kScalThreads, 0, st, p, share)));
   MXB_LAUNCH("m3s_chunk_scalars_kernel", st, (launch_kernel(m3s::m3s_chunk_scalars_kernel, gc, 64, 0, st, p, static_cast<const double*>(share))));
   mxb_status ps = ssd_state_pass(p, 0, st);
   if (ps != MXB_OK) return ps;

@@ -216,6 +216,31 @@ def test_mamba3_chunks(cfg):
     mamba.test_chunked_tensor_core_kernels(cfg)
 
 
+def test_mamba3_chunks_beyond_a_grid_axis():
+    """More chunks than the 65,535 blocks of a grid's y axis, against the recurrent kernels on the last 2048 steps alone: over
+    the last thousand the states before that piece have decayed (exp(-80) and less), and only differences of angles count."""
+    T, P, N, piece, tail = 65535 * 64 + 65, 64, 128, 2048, 1000
+    g = torch.Generator(device="cuda").manual_seed(98)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    # (the pieces of a sequence this long that matter are its last steps: 64 k random steps, repeated)
+    wide = lambda w: rn(1, 1 << 16, w).to(BF16).repeat(1, T // (1 << 16) + 1, 1)[:, :T].contiguous()
+    x, dy, b, c = wide(P), wide(P), wide(N).view(1, T, 1, N), wide(N).view(1, T, 1, N)
+    dt, lam, theta, a_log = rn(1, T, 1) * 0.5 - 2, rn(1, T, 1), rn(1, T, 1), torch.zeros(1, device="cuda")
+    y = ops.mamba3_selective_scan(x, dt, lam, theta, a_log, b, c, nheads=1, save_for_backward=True)
+    got = ops.mamba3_selective_scan_backward(x, dt, lam, theta, a_log, b, c, dy, nheads=1, use_saved=True)
+    assert ops.device_status() == 0
+    end = lambda t: t[:, T - piece:].contiguous()
+    part = (end(x), end(dt), end(lam), end(theta), a_log, end(b), end(c))
+    kw = dict(nheads=1, flags=_lib.MXB_MAMBA3_RECURRENT_KERNELS)
+    y_r = ops.mamba3_selective_scan(*part, **kw)
+    want = ops.mamba3_selective_scan_backward(*part, end(dy), **kw)
+    assert_close(y[:, -tail:], y_r[:, -tail:].double(), 2e-2, "y")
+    for n in mamba.GRADS:
+        if n != "da_log":  # (a sum over all steps)
+            assert_close(got[n][:, -tail:], want[n][:, -tail:].double(), 2e-2, n)
+    assert bool(torch.isfinite(got["da_log"]).all())
+
+
 @pytest.mark.parametrize("B,T,H,arena_mb", [(1, 130, 4, 256), (4, 600, 8, 256), (4, 600, 8, 40), (2, 2100, 8, 256)])
 def test_host_slicing(B, T, H, arena_mb):
     """Slices of whole sequences and of groups of heads, two to four in flight, and finer ones where the arena is small:
