@@ -14,6 +14,7 @@
 // before it was written); its sequential part is the mirrored scan dH0 = L dH1 + Dc.
 //
 //   m3s_scalars_kernel      per chunk: dt, lambda, the chunk's share of the angle (fp64)
+//   m3s_angle_prefix_kernel (long sequences) the shares to the sums over the chunks in front
 //   m3s_chunk_scalars_kernel per chunk: decay sums, trapezoid weights, sines/cosines of the cumulative angle (one record)
 //   m3s_state_pass_kernel   per (b, head), sequential over the chunks, forward or reverse: the chunk contribution
 //                           Brot^T diag(r e) X (or Crot^T diag(exp(Lam)) dY) folded into the running state
@@ -109,6 +110,8 @@ struct ChunkScal {
 static_assert(sizeof(ChunkScal) % 16 == 0, "record moves in 16-byte units");
 constexpr int kScalUnits = sizeof(ChunkScal) / 16;
 
+// PREFIX: share has the sum over the chunks in front (m3s_angle_prefix_kernel) instead of the chunk's own.
+template <bool PREFIX>
 __global__ void __launch_bounds__(64) m3s_chunk_scalars_kernel(SsdP p, const double* share) {
   begin_dependent();
   __shared__ __align__(16) ChunkScal s;
@@ -128,7 +131,11 @@ __global__ void __launch_bounds__(64) m3s_chunk_scalars_kernel(SsdP p, const dou
     s.e[tid] = lam * dt + nxt;
     // cumulative rotation angle in fp64: the shares of the chunks in front, then the steps of this one
     double before = 0.0, phi = ok ? (double)dt * (double)p.theta_t[base + t] : 0.0;
-    for (int x = tid; x < c; x += Q) before += share[((size_t)b * p.n + x) * p.NH + head];
+    if (PREFIX) {
+      if (tid == 0) before = share[((size_t)b * p.n + c) * p.NH + head];
+    } else {
+      for (int x = tid; x < c; x += Q) before += share[((size_t)b * p.n + x) * p.NH + head];
+    }
     const int lane = tid & 31;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -322,6 +329,37 @@ __global__ void __launch_bounds__(kScalThreads) m3s_scalars_kernel(SsdP p, doubl
   }
   __syncthreads();
   if (tid < nh) share[((size_t)b * p.n + c) * p.NH + h0 + tid] = wsum[2 * tid] + wsum[2 * tid + 1];
+}
+
+// The chunks' shares of the angle to the sums of the shares in front of them, in place: a thread adds a segment of the chunks of
+// one head, the segments are scanned in shared memory, and the thread goes through its segment again.  Eight heads a block, so
+// that a row of shares is read by whole sectors.
+constexpr int kPrefixSegs = 128;
+__global__ void __launch_bounds__(kScalHeads * kPrefixSegs) m3s_angle_prefix_kernel(SsdP p, double* share) {
+  begin_dependent();
+  __shared__ double sums[kPrefixSegs][kScalHeads];
+  const int seg = threadIdx.x / kScalHeads, hl = threadIdx.x % kScalHeads, head = blockIdx.x * kScalHeads + hl;
+  const int len = (p.n + kPrefixSegs - 1) / kPrefixSegs, c0 = min(seg * len, p.n), c1 = head < p.NH ? min(c0 + len, p.n) : c0;
+  double* col = share + (size_t)blockIdx.y * p.n * p.NH + head;
+  double sum = 0.0;
+#pragma unroll 8
+  for (int c = c0; c < c1; ++c) sum += col[(size_t)c * p.NH];
+  sums[seg][hl] = sum;
+  __syncthreads();
+#pragma unroll
+  for (int o = 1; o < kPrefixSegs; o <<= 1) {
+    const double up = seg >= o ? sums[seg - o][hl] : 0.0;
+    __syncthreads();
+    sums[seg][hl] += up;
+    __syncthreads();
+  }
+  double before = seg > 0 ? sums[seg - 1][hl] : 0.0;
+#pragma unroll 8
+  for (int c = c0; c < c1; ++c) {
+    const double own = col[(size_t)c * p.NH];
+    col[(size_t)c * p.NH] = before;
+    before += own;
+  }
 }
 
 // ------------------------------------------------------------ state pass
@@ -1335,7 +1373,19 @@ static mxb_status ssd_forward(SsdP& p, cudaStream_t st) {
   double* share = reinterpret_cast<double*>(p.H0);
   MXB_LAUNCH("m3s_scalars_kernel", st,
              (launch_kernel(m3s::m3s_scalars_kernel, dim3(p.n * ((p.NH + m3s::kScalHeads - 1) / m3s::kScalHeads), p.B), m3s::kScalThreads, 0, st, p, share)));
-  MXB_LAUNCH("m3s_chunk_scalars_kernel", st, (launch_kernel(m3s::m3s_chunk_scalars_kernel, gc, 64, 0, st, p, static_cast<const double*>(share))));
+  const double* angles = share;
+  // A block of the next kernel adds the shares of all chunks in front of its own: fine for short sequences, but it grows with the
+  // square of their number.  Sums by a launch of their own from chunks^2 x heads of 2 M on (not by the batch: a sequence gives the
+  // same bits alone).  Forward, us, without / with it, chunks x heads: 64 x 32 84 / 86, 128 x 32 161 / 162, 256 x 8 228 / 231,
+  // 256 x 32 309 / 306 (4 sequences 599 / 587), 512 x 8 450 / 452, 1024 x 8 890 / 886, 512 x 32 607 / 596, 2048 x 32 2594 / 2364.
+  if ((long long)p.n * p.n * p.NH >= 1 << 21) {
+    MXB_LAUNCH("m3s_angle_prefix_kernel", st,
+               (launch_kernel(m3s::m3s_angle_prefix_kernel, dim3((p.NH + m3s::kScalHeads - 1) / m3s::kScalHeads, p.B),
+                              m3s::kScalHeads * m3s::kPrefixSegs, 0, st, p, share)));
+    MXB_LAUNCH("m3s_chunk_scalars_kernel", st, (launch_kernel(m3s::m3s_chunk_scalars_kernel<true>, gc, 64, 0, st, p, angles)));
+  } else {
+    MXB_LAUNCH("m3s_chunk_scalars_kernel", st, (launch_kernel(m3s::m3s_chunk_scalars_kernel<false>, gc, 64, 0, st, p, angles)));
+  }
   mxb_status ps = ssd_state_pass(p, 0, st);
   if (ps != MXB_OK) return ps;
   if (p.y) {

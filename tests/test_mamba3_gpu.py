@@ -314,3 +314,35 @@ def test_chunked_kernels_by_heads_per_cta(B, T, NH, G):
     assert_close(y, y_r.double().cpu(), 2e-2, "y")
     for n in want:
         assert_close(got[n], want[n].double().cpu(), 2e-2, n)
+
+
+@pytest.mark.parametrize("B,chunks,NH", [(1, 256, 32), (2, 419, 12), (1, 1449, 1)])
+def test_chunked_kernels_of_long_sequences(B, chunks, NH):
+    """Sequences whose chunks get the sums of the angle in front of them from a launch of their own (work that grows with the
+    length, not with its square): against the recurrent kernels, and the first heads alone, which are below that line unless
+    there is one head: angles that agree in float64 but for the order of a sum, so results within one bf16 rounding, 2^-8."""
+    T = 64 * chunks - 17
+    m = inputs.mamba3_inputs(B, T, NH, 64, 128, G=1, seed=70 + NH, io_dtype=torch.bfloat16, per_head=True)
+    dev = {k: _dev(m[k]) for k in ARGS + ("dy",)}
+
+    def run(h, flags=0):
+        cut = {k: t if k in ("b", "c") else t[..., :64 * h] if k in ("x", "dy") else t[..., :h] for k, t in dev.items()}
+        cut = {k: t.contiguous() for k, t in cut.items()}
+        args = tuple(cut[k] for k in ARGS)
+        n0 = _lib.lib().mxb_launch_count()
+        y = ops.mamba3_selective_scan(*args, nheads=h, flags=flags)
+        launches = _lib.lib().mxb_launch_count() - n0
+        return y, ops.mamba3_selective_scan_backward(*args, cut["dy"], nheads=h, flags=flags), launches
+
+    y, got, launches = run(NH)
+    y_r, want, _ = run(NH, _lib.MXB_MAMBA3_RECURRENT_KERNELS)
+    assert_close(y, y_r.double(), 2e-2, "y")
+    for n in GRADS:
+        assert_close(got[n], want[n].double(), 2e-2, n)
+    few = NH // 4
+    if few:
+        y_f, part, fewer = run(few)
+        assert launches == fewer + 1  # (the launch that adds the angles)
+        assert_close(y[..., :64 * few], y_f.double(), 2.0 ** -8, "y")
+        for n in ("dx", "ddt", "dlambda", "dtheta"):
+            assert_close(got[n][..., :part[n].shape[-1]], part[n].double(), 2.0 ** -8, n)
