@@ -670,9 +670,11 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
 // issues the products (an elected thread of a warp of its own: 33 cycles an instruction, 60 behind a test of the thread's
 // index), one that finishes the per-step scalars and one that stores dx; everything is handed over by mbarriers.
 // Products of a head: dP = dY X^T, U = {C, CJ} H0, V = {B, JB} dH1 (asked for a head ahead), Z and Y, then dX = (G*M)^T dY.
-// 8 x 4096 x 32 heads: 349 us + 54 for the row sums behind it, 1.0 GB (0.15 ms); a CTA per head and chunk that rotated B and C
-// took 527 + 118 with 1.5 + 0.6 GB.  A head takes 5.0 k cycles, most of it the arithmetic of the 64 x 64 products (1.3 k), of U
-// and V (0.9 k) and of the scaled images (0.6 k) at half of the issue slots; pairs of columns in packed registers (7.8 k without).
+// 8 x 4096 x 32 heads: 335 us + 29 for the row sums behind it, 1.0 GB (0.15 ms); a CTA per head and chunk that rotated B and C
+// took 527 + 118 with 1.5 + 0.6 GB.  Bound by instruction issue: most of a head is the arithmetic of the 64 x 64 products, of U
+// and V and of the scaled images at half of the issue slots; pairs of columns in packed registers (7.8 k cycles a head without,
+// 5.0 k with them, 4.7 k since U and V meet x and dY as they landed instead of two images each: also the closer result, the
+// images are rounded to bf16: dtheta 8.1e-4 -> 7.0e-4 from float64, ddt 5.9e-4 -> 5.4e-4).
 // TMEM: Z [0,128), Y [128,256), U [256,320), V [320,384), dP [384,416), dX [416,448); at the start C B^T and C (J B)^T in
 // the last two, at the end the products with W1 and W2 in U and V.
 constexpr int kGradWarps = 16;
@@ -951,7 +953,6 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       uint8_t* S = St + (h & 1) * kGradStage;
       const ChunkScal& s = scal[h & 3];
       wait(full + (h & 1), h >> 1);
-      wait(uvfree, h);  // (nobody reads the images of the head before any more)
       {  // scaled images: one unit of x and of dY per thread (unit u lies in row u / 8)
         const int r = tid >> 3;
         const float sn = s.sn[r], cs = s.cs[r], xd = s.dexp[r], xr = s.re[r];
@@ -997,7 +998,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       ok = __all_sync(0xffffffffu, ok);
       const float lt = s.Lam[t], gt = s.gam[t], ct = s.cs[t], st = s.sn[t];
       float dg = 0.f;
-      f2 dl = 0, dphi = 0, dpm = 0, dpb = 0;   // (dphi: sums of what is added and of what is taken away)
+      f2 dl = 0, dphi = 0, pya = 0, pyb = 0, pxa = 0;  // row sums; of dY with C H0 and CJ H0, of x with B dH1 (and (J B) dH1)
       float ce[8] = {}, cq[8] = {};
       if (ok) {
         uint32_t gm[4] = {};
@@ -1045,38 +1046,33 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       }
       tc::fence_async_smem();
       arrive(gready);
-      // U, V: kappa_t = e^Lam dY_t . (Crot H0)_t, zeta_s = x_s . (Brot dH1)_s and their derivatives by the angle
-      f2 v[4] = {}, de = 0;
-      wait(images, h + 1);  // (written by other threads)
-      ok = __all_sync(0xffffffffu, ok);
+      // U, V: kappa_t = e^Lam dY_t . (Crot H0)_t, zeta_s = x_s . (Brot dH1)_s and their derivatives by the angle.  dY and x as they
+      // landed: the factors of a row are applied to its sums.
+      f2 v[4] = {}, pxb = 0;
       if (ok) {
         f2 fa[4], fb[4];
         auto word = [](const uint4& u, int i) { return i == 0 ? u.x : i == 1 ? u.y : i == 2 ? u.z : u.w; };
         ld_pairs(taddr + tU + tc8, warp, fa);
         ld_pairs(taddr + tU + 32 + tc8, warp, fb);
-        uint4 ic = *reinterpret_cast<const uint4*>(Yc + tunit), is = *reinterpret_cast<const uint4*>(Yc + 8192 + tunit);
+        const uint4 iy = *reinterpret_cast<const uint4*>(S + 8192 + tunit);
         tc::tmem_ld_wait();
 #pragma unroll
         for (int z = 0; z < 4; ++z) {
-          const f2 a = widen2(word(ic, z)), e = widen2(word(is, z));
-          fma2(dl, a, fa[z]);
-          fma2(dl, e, fb[z]);
-          fma2(dphi, a, fb[z]);
-          fma2(dpm, e, fa[z]);
+          const f2 y = widen2(word(iy, z));
+          fma2(pya, y, fa[z]);
+          fma2(pyb, y, fb[z]);
         }
         ld_pairs(taddr + tV + tc8, warp, fa);
         ld_pairs(taddr + tV + 32 + tc8, warp, fb);
-        ic = *reinterpret_cast<const uint4*>(Xc + tunit);
-        is = *reinterpret_cast<const uint4*>(Xc + 8192 + tunit);
         const uint4 ix = *reinterpret_cast<const uint4*>(S + tunit);
         const f2 ct2 = dup2(ct), nst2 = dup2(-st);
         tc::tmem_ld_wait();
 #pragma unroll
         for (int z = 0; z < 4; ++z) {
-          fma2(dpb, widen2(word(ic, z)), fb[z]);
-          fma2(dpb, widen2(word(is, z)), fa[z]);
+          const f2 xz = widen2(word(ix, z));
+          fma2(pxa, xz, fa[z]);
+          fma2(pxb, xz, fb[z]);
           v[z] = mad2(ct2, fa[z], mul2(nst2, fb[z]));   // Brot = cos B - sin (J B)
-          fma2(de, widen2(word(ix, z)), v[z]);
         }
       }
       tc::fence_before_sync();
@@ -1089,17 +1085,17 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
         csw[(warp & 1) * Q + n8 + lane] = ce[0];
         csw[(2 + (warp & 1)) * Q + n8 + lane] = cq[0];
       }
-      part[(4 * slot + 0) * Q + t] = sum2(dl);
-      part[(4 * slot + 1) * Q + t] = s.r[t] * sum2(de);
-      part[(4 * slot + 2) * Q + t] = sum2(dpb);
+      const float ret = s.re[t], det = s.dexp[t], ya = sum2(pya), yb = sum2(pyb), xa = sum2(pxa), xb = sum2(pxb);
+      part[(4 * slot + 0) * Q + t] = fmaf(det, fmaf(ct, ya, st * yb), sum2(dl));
+      part[(4 * slot + 1) * Q + t] = s.r[t] * fmaf(ct, xa, -(st * xb));
+      part[(4 * slot + 2) * Q + t] = ret * fmaf(ct, xb, st * xa);
       if ((t >> 3) == (n8 >> 3)) dgs[t] = dg;
-      part[(4 * slot + 3) * Q + t] = sum2(dphi) - sum2(dpm);
+      part[(4 * slot + 3) * Q + t] = fmaf(det, fmaf(ct, yb, -(st * ya)), sum2(dphi));
       if (lane == 0) {
         red[warp] = acc;
         red[kGradWarps + warp] = accj;
       }
       arrive(pready);
-      const float ret = s.re[t];
       wait(m2, h);
       tc::fence_after_sync();
       if (h > 0) wait(xfree, h - 1);
@@ -1118,7 +1114,6 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       arrive(freed + (h & 1));
     }
     // the sums over the heads
-    wait(uvfree, nh);
     sts16(Yc, tc::kmajor_unit(t, n8 >> 3, Q), make_uint4(narrow2(w1[0]), narrow2(w1[1]), narrow2(w1[2]), narrow2(w1[3])));
     sts16(Yc + 8192, tc::kmajor_unit(t, n8 >> 3, Q), make_uint4(narrow2(w2[0]), narrow2(w2[1]), narrow2(w2[2]), narrow2(w2[3])));
     tc::fence_async_smem();

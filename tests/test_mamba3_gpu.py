@@ -346,3 +346,39 @@ def test_chunked_kernels_of_long_sequences(B, chunks, NH):
         assert_close(y[..., :64 * few], y_f.double(), 2.0 ** -8, "y")
         for n in ("dx", "ddt", "dlambda", "dtheta"):
             assert_close(got[n][..., :part[n].shape[-1]], part[n].double(), 2.0 ** -8, n)
+
+
+def _two_chunks(side):
+    """Two chunks of which the states between them are one outer product of signs, times a factor that the rounding to bf16
+    changes as a whole: x has one value (side "dy", which then has its values in the second chunk), or dy has (side "x")."""
+    T, t = 128, 100
+    m = inputs.mamba3_inputs(1, T, 1, 64, 128, G=1, seed=77, io_dtype=torch.bfloat16, per_head=True)
+    m["a_log"].fill_(math.log(0.05))
+    one, signs, many = ("x", "b", "dy") if side == "dy" else ("dy", "c", "x")
+    m[signs] = torch.where(m[signs] < 0, -1.0, 1.0).to(torch.bfloat16)
+    m[one].zero_()
+    if side == "dy":
+        m["x"][:, 10, 0], m["dy"][:, :64], m["theta"][:, :64] = 1, 0, 0
+    else:  # whole turns up to the step of dy, so that c is not rotated there
+        m["dy"][:, t, 0], m["x"][:, 64:], m["theta"][:, 65:] = 1, 0, 0
+        dt = torch.nn.functional.softplus(m["dt_raw"].double())
+        m["theta"][:, 64] = (-(dt[:, :64] * m["theta"][:, :64].double()).sum(1) / dt[:, 64]).float()
+    full = inputs.mamba3_expand_per_head(m)
+    _, want = mamba3.scan_vjp(*(full[k].double() for k in ARGS), m["dy"].double())
+    want = dict(ddt=want["ddt"].sum(-1), dlambda=want["dlambda"].sum(-1), dtheta=want["dtheta"].sum((-1, -2)))
+    got = ops.mamba3_selective_scan_backward(*(_dev(m[k]) for k in ARGS), _dev(m["dy"]), nheads=1)
+    rows = slice(64, 128) if side == "dy" else slice(0, 64)
+    return {n: (got[n].double().cpu().reshape(T)[rows], want[n].reshape(T)[rows]) for n in want}
+
+
+@pytest.mark.parametrize("side,names", [("dy", ("ddt", "dtheta")), ("x", ("ddt", "dlambda", "dtheta"))])
+def test_row_sums_of_the_chunked_backward_are_float32(side, names):
+    """The gradients of dt, lambda and theta meet dY and x with the chunk states as the tensors came, not as operands rounded to
+    bf16 again: but for a common factor (the rounding of the state, at most 2^-8), they are off by float32 sums of 128
+    states, 64 columns and 64 steps only, 256 x 6e-8 = 1.5e-5."""
+    r = _two_chunks(side)
+    for n in names:
+        got, want = r[n]
+        a = float((got * want).sum() / (want * want).sum())
+        assert abs(a - 1) <= 2.0 ** -8, (n, a)
+        assert float((got - a * want).norm() / want.norm()) <= 1.5e-5, n
