@@ -40,7 +40,8 @@ __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
 
-__device__ __forceinline__ float warp_sum(float v) {
+template <typename F>
+__device__ __forceinline__ F warp_sum(F v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
@@ -68,11 +69,12 @@ __device__ __forceinline__ void colsum8(float (&v)[8], int lane) {
 
 // Reverse inclusive cumulative sum over 64 values by one warp, two per lane: call with a = x[63 - 2 lane],
 // b = x[62 - 2 lane]; returns in a, b the sums x[63] + ... + x[63 - 2 lane] and ... + x[62 - 2 lane].  A fixed order.
-__device__ __forceinline__ void warp_rcumsum64(float& a, float& b, int lane) {
-  float v = a + b;
+template <typename F>
+__device__ __forceinline__ void warp_rcumsum64(F& a, F& b, int lane) {
+  F v = a + b;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const float t = __shfl_up_sync(0xffffffffu, v, o);
+    const F t = __shfl_up_sync(0xffffffffu, v, o);
     if (lane >= o) v += t;
   }
   a = v - b;

@@ -870,13 +870,15 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       const float zra = part_sum(1, ra), zrb = part_sum(1, rb);            // r_s zeta_s
       const float cea = csw[ra] + csw[Q + ra], ceb = csw[rb] + csw[Q + rb];
       const float dga = dgs[ra], dgb = dgs[rb], bsa = part_sum(2, ra), bsb = part_sum(2, rb);
-      float dpa = part_sum(3, ra) - bsa - (csw[2 * Q + ra] + csw[3 * Q + ra]);
-      float dpb = part_sum(3, rb) - bsb - (csw[2 * Q + rb] + csw[3 * Q + rb]);
+      // (the angle in double precision: steps whose gradient is small stand behind sums over large ones that cancel)
+      double dpa = (double)part_sum(3, ra) - bsa - (csw[2 * Q + ra] + csw[3 * Q + ra]);
+      double dpb = (double)part_sum(3, rb) - bsb - (csw[2 * Q + rb] + csw[3 * Q + rb]);
       const float dla = part_sum(0, ra), dlb = part_sum(0, rb);
       const float hw = red[lane];
       const float ea = s.e[ra], eb = s.e[rb], ga = s.gam[ra], gb = s.gam[rb], L = s.L;
       arrive(pfree);
-      const float hh = warp_sum(lane < kGradWarps ? hw : 0.f), later = warp_sum((lane < kGradWarps ? 0.f : L * hw) + (bsa + bsb));
+      const float hh = warp_sum(lane < kGradWarps ? hw : 0.f);
+      const double later = warp_sum((lane < kGradWarps ? 0.0 : (double)L * hw) + ((double)bsa + bsb));
       const float zs = warp_sum(fmaf(ea, zra, eb * zrb));
       const float base = zs + L * hh;  // d/dLam_end
       // dLam -> da: reverse in-chunk cumulative sum
@@ -889,8 +891,8 @@ __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p,
       dpa += later;
       dpb += later;
       const size_t o = ((size_t)b * p.NH + h0 + h) * p.T + t0;
-      if (t0 + ra < p.T) { p.da[o + ra] = base + a; p.de[o + ra] = zra + cea; p.dgam[o + ra] = dga; p.dphi[o + ra] = dpa; }
-      if (t0 + rb < p.T) { p.da[o + rb] = base + bq; p.de[o + rb] = zrb + ceb; p.dgam[o + rb] = dgb; p.dphi[o + rb] = dpb; }
+      if (t0 + ra < p.T) { p.da[o + ra] = base + a; p.de[o + ra] = zra + cea; p.dgam[o + ra] = dga; p.dphi[o + ra] = (float)dpa; }
+      if (t0 + rb < p.T) { p.da[o + rb] = base + bq; p.de[o + rb] = zrb + ceb; p.dgam[o + rb] = dgb; p.dphi[o + rb] = (float)dpb; }
     }
   } else if (warp == kGradWarps + 3) {  // ---- dx
     tc::reg_dec<40>();

@@ -348,9 +348,10 @@ def test_chunked_kernels_of_long_sequences(B, chunks, NH):
             assert_close(got[n][..., :part[n].shape[-1]], part[n].double(), 2.0 ** -8, n)
 
 
-def _two_chunks(side):
+def _two_chunks(side, quiet=0):
     """Two chunks of which the states between them are one outer product of signs, times a factor that the rounding to bf16
-    changes as a whole: x has one value (side "dy", which then has its values in the second chunk), or dy has (side "x")."""
+    changes as a whole: x has one value (side "dy", which then has its values in the second chunk), or dy has (side "x").
+    quiet: the first steps whose x is 2^-12 of the others'."""
     T, t = 128, 100
     m = inputs.mamba3_inputs(1, T, 1, 64, 128, G=1, seed=77, io_dtype=torch.bfloat16, per_head=True)
     m["a_log"].fill_(math.log(0.05))
@@ -361,6 +362,7 @@ def _two_chunks(side):
         m["x"][:, 10, 0], m["dy"][:, :64], m["theta"][:, :64] = 1, 0, 0
     else:  # whole turns up to the step of dy, so that c is not rotated there
         m["dy"][:, t, 0], m["x"][:, 64:], m["theta"][:, 65:] = 1, 0, 0
+        m["x"][:, :quiet] *= 2.0 ** -12
         dt = torch.nn.functional.softplus(m["dt_raw"].double())
         m["theta"][:, 64] = (-(dt[:, :64] * m["theta"][:, :64].double()).sum(1) / dt[:, 64]).float()
     full = inputs.mamba3_expand_per_head(m)
@@ -382,3 +384,14 @@ def test_row_sums_of_the_chunked_backward_are_float32(side, names):
         a = float((got * want).sum() / (want * want).sum())
         assert abs(a - 1) <= 2.0 ** -8, (n, a)
         assert float((got - a * want).norm() / want.norm()) <= 1.5e-5, n
+
+
+def test_angle_gradients_of_quiet_steps():
+    """dtheta of a step is a sum over the steps before it as the difference of the sums over all steps and over the later ones.
+    Where the first steps are 2^-12 of the later ones, sums in float32 leave 6e-8 x 2^12 x sqrt(64) = 2e-3 of theirs; the steps'
+    own float32 sums of 128 states and 64 columns, 1.2e-5, are what may remain (a common factor aside, as above)."""
+    got, want = _two_chunks("x", quiet=12)["dtheta"]
+    got, want = got[1:12], want[1:12]
+    a = float((got * want).sum() / (want * want).sum())
+    assert abs(a - 1) <= 2.0 ** -8
+    assert float((got - a * want).norm() / want.norm()) <= 1.2e-5
