@@ -13,8 +13,10 @@
 //             out^T   = E(gam) (S^T q^T) + v_new^T P^T
 //   backward  dv_new^T = r (dS^T k^T) + dO^T P     dS^T <- E(gam_last) dS^T + dO^T (d q) - dv_new^T w
 // The mathematics, the workspace tiles, the roundings and the order of every sum are those of gdn_tc.cu, gdn_tc_bwd.cu and
-// gdn_tc64.cu, and mma.sync adds the 16 products of a step as tcgen05.mma does: results are equal bit for bit, so a
-// sequence gives the same bits alone and in a batch that takes the other kernels.
+// gdn_tc64.cu, and mma.sync adds the 16 products of a step as tcgen05.mma does: finite results are equal bit for bit, so a
+// sequence gives the same bits alone and in a batch that takes the other kernels.  An infinity or NaN spreads differently: the
+// products with the zero half of P are skipped here and made there, so there it reaches all rows of its chunk (0 x NaN), here
+// the rows that use it and those of its block of 16.
 //
 // Twelve warps.  Chain warps 0-3, one per scheduler: a quarter of the chunk's rows in the first product, a quarter of the
 // state's rows (kept in registers, fp32) in the second; between the two they exchange v_new and S through shared memory as
@@ -34,14 +36,10 @@
 #include "mma_sync.cuh"
 
 namespace mxb {
-bool make_tma_map_cols(CUtensorMap* m, const void* base, int B, int T, int H, int D, int cols);
-
 namespace chain {
 constexpr int kThreads = 384;
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(mbar)) : "memory");
-}
+using tc::mbar_arrive;
 using ms::ldsm;
 using ms::ldsm_t;
 using ms::mma;
@@ -760,7 +758,6 @@ __global__ void __launch_bounds__(kThreads, 1) gdn_chain_bwd_kernel(TcP p, const
 //   128 wide   1 sequence 62 + 58, 43 + 43, 54 + 51     2 sequences 63 + 60, -, 54 + 52
 //   64 wide    1 sequence 64 + 56, 32 + 33, 40 + 39     4 sequences 64 + 56, -, 42 + 42
 // With 64 columns (twice the sequences) the rate of mma.sync tells: 93 + 80 against 63 + 60, and 66 + 58 against 65 + 57.
-// whole: the images of the state are wanted at their full width (saving forward, backward).
 int chain_columns(const TcP& p, bool whole) {
   const int W = p.Dk == 64 && p.Dv == 64 ? 64 : 128, width = whole ? W : p.Dv;
   for (int nv = 16; nv <= 32; nv *= 2)
@@ -783,7 +780,6 @@ static mxb_status chain_launch(const TcP& p, const RowMaps& maps, int width, cud
   }
   return check_launch("gdn_chain kernels");
 }
-// Forward and backward state pass, nv columns per CTA; maps.k, maps.q as the other kernels use them.
 mxb_status chain_fwd(const TcP& p, const RowMaps& maps, int nv, cudaStream_t st) {
   const bool w64 = p.Dk == 64 && p.Dv == 64;
   const int width = p.save ? (w64 ? 64 : 128) : p.Dv;

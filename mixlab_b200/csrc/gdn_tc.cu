@@ -690,8 +690,6 @@ size_t gdn_tc_workspace_bytes(const mxb_gdn_desc* d, bool bwd) {
 
 mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st);
 mxb_status tc64_run_fwd(TcP& p, cudaStream_t st);
-int chain_columns(const TcP& p, bool whole);
-mxb_status chain_fwd(const TcP& p, const RowMaps& maps, int nv, cudaStream_t st);
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -728,7 +726,6 @@ static bool make_tma_map(CUtensorMap* m, CUtensorMapDataType type, int size, con
 bool make_tma_map_bthd(CUtensorMap* m, const void* base, int B, int T, int H, int D) {
   return make_tma_map(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, B, T, H, D);
 }
-// Boxes of 16, 32 or 64 columns, swizzled over their own width.
 bool make_tma_map_cols(CUtensorMap* m, const void* base, int B, int T, int H, int D, int cols) {
   return make_tma_map(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, B, T, H, D, cols);
 }

@@ -13,6 +13,8 @@ namespace mxb {
 
 // [B,T,H,D] bf16 -> tensor map over (D, H, T, B) with 64 x 64 boxes and 128-byte swizzle; false if it cannot be made.
 bool make_tma_map_bthd(CUtensorMap* m, const void* base, int B, int T, int H, int D);
+// The same with boxes of 16 or 32 columns, swizzled over their own width.
+bool make_tma_map_cols(CUtensorMap* m, const void* base, int B, int T, int H, int D, int cols);
 
 namespace tcg {
 constexpr int C = 64;     // chunk
@@ -231,5 +233,12 @@ __device__ __forceinline__ void load_inverse_images(const float* Am, const float
 }
 }  // namespace tcg
 using namespace tcg;
+
+// State passes on mma.sync (gdn_chain.cu).  chain_columns: columns of the state per CTA, 0 where the tcgen05 passes are the better
+// ones; whole: the images of the state are wanted at their full width (saving forward, backward).  Then the passes, nv columns per
+// CTA; maps.k, maps.q as the other kernels use them.
+int chain_columns(const TcP& p, bool whole);
+mxb_status chain_fwd(const TcP& p, const RowMaps& maps, int nv, cudaStream_t st);
+mxb_status chain_bwd(const TcP& p, const RowMaps& maps, int nv, cudaStream_t st);
 
 }  // namespace mxb

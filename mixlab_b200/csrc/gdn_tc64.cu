@@ -898,9 +898,6 @@ __global__ void __launch_bounds__(256, 3) gdn_tc_chunk_bwd_kernel(TcP p, const _
 }  // namespace g64
 
 // ------------------------------------------------------------------ host
-int chain_columns(const TcP& p, bool whole);
-mxb_status chain_fwd(const TcP& p, const RowMaps& maps, int nv, cudaStream_t st);
-mxb_status chain_bwd(const TcP& p, const RowMaps& maps, int nv, cudaStream_t st);
 mxb_status tc64_run_fwd(TcP& p, cudaStream_t st) {
   RowMaps maps;
   std::memset(&maps, 0, sizeof maps);

@@ -695,8 +695,6 @@ __global__ void __launch_bounds__(256, 2) gdn_tc_chunk_bwd_kernel(TcP p, const _
 // ------------------------------------------------------------------ host
 mxb_status tc_run_fwd(TcP& p, cudaStream_t st);
 mxb_status tc64_run_bwd(const TcP& p, cudaStream_t st);
-int chain_columns(const TcP& p, bool whole);
-mxb_status chain_bwd(const TcP& p, const RowMaps& maps, int nv, cudaStream_t st);
 
 // Forward recompute (saving per-chunk states and v_new), reverse state pass, per-chunk pass.
 mxb_status tc_run_bwd(TcP& p, bool recompute, cudaStream_t st) {

@@ -39,6 +39,7 @@ constexpr int Q = 64;    // chunk
 constexpr int P = 64;    // head dim
 constexpr int N = 128;   // d_state
 using bf16 = __nv_bfloat16;
+using tc::mbar_arrive;
 using tc::pack8;
 using tc::unpack8;
 
@@ -91,9 +92,6 @@ __device__ __forceinline__ uint32_t narrow2(f2 v) {
   return tc::pack_bf16(t.x, t.y);
 }
 __device__ __forceinline__ f2 neg2(f2 v) { return v ^ 0x8000000080000000ull; }
-__device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(mbar)) : "memory");
-}
 
 // Per-chunk scalars: computed once per (batch, head, chunk) by m3s_chunk_scalars_kernel into a workspace record
 // and fetched by every chunk kernel with its operand tiles (the record is a whole number of 16-byte units).
@@ -375,6 +373,8 @@ __global__ void __launch_bounds__(kScalHeads * kPrefixSegs) m3s_angle_prefix_ker
 // fold in an accumulator and store the state (one sequence of 32 heads x 64 chunks: 57 us a pass, chunk by chunk in one group
 // of warps 84; 8 sequences 104, where it is the arithmetic of the rotation that counts, 107).  Every hand-over is an mbarrier with a bounded wait; a warp whose wait has run out stops waiting and working but goes through its loop.
 // NS stages in flight: three and four warps that prepare tiles where two CTAs share an SM, six and eight where one has it.
+// With three, 448 threads and 72 registers, 20 bytes are spilled and 28 read back; reading the accumulator in halves avoids that
+// and takes longer (8 sequences 105 us a pass, 108 without spills).
 template <int NS>
 constexpr int kPassPrep = NS == 3 ? 4 : 8;
 template <int NS>
