@@ -291,10 +291,11 @@ struct NoA { __device__ float4 operator()(int, int) const { return make_float4(0
 
 // ------------------------------------------------------------ state passes
 // The sequential passes: one chunk after the other, so the time of a chunk is what counts.  A CTA owns W columns of
-// the state (columns are independent), W as small as still fits the CTAs on the SMs at once.  What bounds a chunk is
-// the shared-memory bandwidth of the products, so every thread computes 4 x 4 outputs (eight loaded values per sixteen
-// multiply-adds) over a part of the contraction, and the parts (32 / W of them for 128 rows) are added through shared
-// memory in a fixed order.  One output per thread and 16-column slabs, operands by one cp.async per 16 bytes:
+// the state (columns are independent), W as small as still fits the CTAs on the SMs at once.  What bounds a chunk are
+// the shared-memory reads of the products and the eight warps an SM that hide them (40 to 43 % of that pipe, 28 to 31 %
+// of the issue slots), so every thread computes 4 x 4 outputs (eight loaded values per sixteen multiply-adds) over a part
+// of the contraction, and the parts (32 / W of them for 128 rows) are added through shared memory in a fixed order.  One
+// output per thread and 16-column slabs, operands by one cp.async per 16 bytes:
 // 8.2 us a chunk at Dk = 64 (6.6 k of 16.4 k cycles went into issuing the copies; one bulk copy per row still took
 // its warp 2.2 k); now a tile is two or four tensor copies issued by one thread as soon as the tile it replaces has
 // been read.

@@ -664,7 +664,8 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
 //     dC = W1 B + W2 (J B) + Z1 + J Z2,   Z1 = sum_h (cos e^Lam dY) H0^T,  Z2 = sum_h (sin e^Lam dY) H0^T
 //     dB = W1^T C + W2^T CJ + Y1 + J Y2,  Y1 = sum_h (cos r e x) dH1^T,     Y2 = sum_h (sin r e x) dH1^T
 //     W1_ts = sum_h cos(delta) dG_ts,  W2_ts = sum_h sin(delta) dG_ts,      dG = (dY X^T) * M
-// so one partial image of dB and dC leaves per CTA instead of one per head.
+// so one partial image of dB and dC leaves per CTA instead of one per head.  W1 and W2 are operands of products, so they are
+// rounded to bf16, once, after the sum over the heads.
 //
 // One CTA per SM: 16 warps with a row t and 8 of 64 columns of every product, one warp that issues the copies, one that
 // issues the products (an elected thread of a warp of its own: 33 cycles an instruction, 60 behind a test of the thread's
