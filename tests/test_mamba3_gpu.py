@@ -397,6 +397,9 @@ def test_angle_gradients_of_quiet_steps():
     assert float((got - a * want).norm() / want.norm()) <= 1.2e-5
 
 
+SCALAR_BOUNDS = {"ddt": 1.5e-3, "dlambda": 1.5e-3, "dtheta": 2.2e-3, "da_log": 6e-3}
+
+
 @pytest.mark.parametrize("T,NH,seed", [(1000, 3, 7), (1500, 2, 6), (2100, 2, 5)])
 def test_scalar_gradients_of_long_sequences(T, NH, seed):
     """The per-token gradients do not drift with the length: against float64.  Their terms carry the rounding of the chunk states
@@ -409,6 +412,19 @@ def test_scalar_gradients_of_long_sequences(T, NH, seed):
     want = dict(ddt=want["ddt"].reshape(1, T, NH, 64).sum(-1), dlambda=want["dlambda"].reshape(1, T, NH, 64).sum(-1),
                 dtheta=want["dtheta"].reshape(1, T, NH, 64, 64).sum((-1, -2)), da_log=want["da_log"].reshape(NH, 64, 128).sum((-1, -2)))
     got = ops.mamba3_selective_scan_backward(*(_dev(a[k]) for k in ARGS), _dev(a["dy"]), nheads=NH)
-    for n, bound in (("ddt", 1.5e-3), ("dlambda", 1.5e-3), ("dtheta", 2.2e-3), ("da_log", 6e-3)):
+    for n, bound in SCALAR_BOUNDS.items():
+        e2, _ = rel_errs(got[n], want[n])
+        assert e2 <= bound, (n, e2)
+
+
+@pytest.mark.parametrize("B,T,NH,G", [(1, 700, 24, 2), (1, 1100, 32, 2), (1, 2800, 24, 1)])
+def test_scalar_gradients_by_heads_per_cta(B, T, NH, G):
+    """The same bounds with 4, 8 and 16 heads per CTA of the chunk-gradient kernel, against the recurrent kernels, whose
+    float32 recurrence on the same bf16 tensors is within 1e-4 of float64."""
+    a = inputs.mamba3_inputs(B, T, NH, 64, 128, G=G, seed=60 + NH, io_dtype=torch.bfloat16, per_head=True)
+    args, dy = tuple(_dev(a[k]) for k in ARGS), _dev(a["dy"])
+    got = ops.mamba3_selective_scan_backward(*args, dy, nheads=NH)
+    want = ops.mamba3_selective_scan_backward(*args, dy, nheads=NH, flags=_lib.MXB_MAMBA3_RECURRENT_KERNELS)
+    for n, bound in SCALAR_BOUNDS.items():
         e2, _ = rel_errs(got[n], want[n])
         assert e2 <= bound, (n, e2)
