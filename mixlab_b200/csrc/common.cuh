@@ -81,6 +81,30 @@ __device__ __forceinline__ void warp_rcumsum64(F& a, F& b, int lane) {
   b = v;
 }
 
+// Sum over `rows` rows of one column (part: its first element) in a fixed order, by a CTA of kSumThreads that owns 16 columns: 64
+// slices of threads take every 64th row (eight loads in flight each), the slices are added pairwise across a warp and then by a
+// warp per column; warp w < 16 gets the sum of column w.  Latency of the loads is all there is:
+// 1184 rows of 448 columns 17.7 us with 8 slices and 32 columns a CTA, 3.8 now.
+constexpr int kSumCols = 16, kSumSlices = 64, kSumThreads = kSumCols * kSumSlices;
+__device__ __forceinline__ float col_sum(const float* __restrict__ part, size_t rows, size_t pitch, bool in) {
+  __shared__ float red[kSumSlices / 2][kSumCols + 1];
+  const int col = threadIdx.x % kSumCols, slice = threadIdx.x / kSumCols, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float s = 0.f;
+  if (in) {
+    for (size_t r0 = slice; r0 < rows; r0 += 8 * kSumSlices) {
+      float v[8];
+#pragma unroll
+      for (int x = 0; x < 8; ++x) v[x] = r0 + x * kSumSlices < rows ? __ldg(part + (r0 + x * kSumSlices) * pitch) : 0.f;
+#pragma unroll
+      for (int x = 0; x < 8; ++x) s += v[x];
+    }
+  }
+  s += __shfl_xor_sync(0xffffffffu, s, kSumCols);
+  if (lane < kSumCols) red[warp][col] = s;
+  __syncthreads();
+  return warp_sum(warp < kSumCols ? red[lane][warp] : 0.f);  // warps 0 .. 15: the sum of column `warp`
+}
+
 // First statement of a kernel that launch_kernel() starts: nothing is read or written before the kernels in front of it in the
 // stream are done and their writes visible.
 __device__ __forceinline__ void begin_dependent() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

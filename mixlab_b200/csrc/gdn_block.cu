@@ -444,35 +444,19 @@ __global__ void __launch_bounds__(256, 2) gdn_block_pre_bwd_kernel(BlockP p, Pre
   }
 }
 
-// out[j] = sum over rows of part[row][j] in a fixed order: a CTA owns 32 columns, its 8 warps take every 8th row
-// (coalesced 128-byte reads, 8 loads in flight per column), then the 8 slices are added in order.  Up to five matrices
-// per launch, segment s starting at block first[s].
+// out[j] = sum over rows of part[row][j] in a fixed order.  Up to five matrices per launch, segment s starting at block first[s].
 struct ColSums {
   const float* part[5];
   float* out[5];
   int rows[5], n[5], first[6], count;
 };
-__global__ void __launch_bounds__(256) gdn_block_colsum_kernel(ColSums c) {
+__global__ void __launch_bounds__(kSumThreads) gdn_block_colsum_kernel(ColSums c) {
   begin_dependent();
-  __shared__ float red[8][32];
   int g = 0;
   while (g + 1 < c.count && (int)blockIdx.x >= c.first[g + 1]) ++g;
-  const int n = c.n[g], rows = c.rows[g];
-  const int j = (blockIdx.x - c.first[g]) * 32 + (threadIdx.x & 31), slice = threadIdx.x >> 5;
-  const float* part = c.part[g];
-  float s = 0.f;
-  if (j < n) {
-#pragma unroll 8
-    for (int r = slice; r < rows; r += 8) s += part[(size_t)r * n + j];
-  }
-  red[slice][threadIdx.x & 31] = s;
-  __syncthreads();
-  if (threadIdx.x < 32 && j < n) {
-    float t = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) t += red[k][threadIdx.x];
-    c.out[g][j] = t;
-  }
+  const int n = c.n[g], j0 = (blockIdx.x - c.first[g]) * kSumCols, mine = j0 + threadIdx.x % kSumCols, j = j0 + (threadIdx.x >> 5);
+  const float t = col_sum(c.part[g] + mine, c.rows[g], n, mine < n);
+  if (threadIdx.x < 32 * kSumCols && (threadIdx.x & 31) == 0 && j < n) c.out[g][j] = t;
 }
 
 // gate / beta backward: one CTA per head walks all (b, t); the two per-head sums (A_log, dt_bias) in a fixed order
@@ -802,7 +786,7 @@ static mxb_status blk_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void*
   blk::ColSums c{};
   auto sum = [&](const float* part, int nrows, int n, float* out) {
     c.part[c.count] = part; c.out[c.count] = out; c.rows[c.count] = nrows; c.n[c.count] = n;
-    c.first[c.count + 1] = c.first[c.count] + (n + 31) / 32;
+    c.first[c.count + 1] = c.first[c.count] + (n + kSumCols - 1) / kSumCols;
     ++c.count;
   };
   sum(a.dwp[0], (int)rows, (int)(4 * Ck), dcq);
@@ -821,7 +805,7 @@ static mxb_status blk_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void*
                (launch_kernel(blk::gdn_block_gate_bwd_kernel, d->H, 256, 0, st, p, a_raw, b_raw, a_log, dt_bias, dbeta, dgate,
                                                                       da_raw, db_raw, da_log, ddt_bias)));
   }
-  MXB_LAUNCH("gdn_block_colsum_kernel", st, (launch_kernel(blk::gdn_block_colsum_kernel, c.first[c.count], 256, 0, st, c)));
+  MXB_LAUNCH("gdn_block_colsum_kernel", st, (launch_kernel(blk::gdn_block_colsum_kernel, c.first[c.count], kSumThreads, 0, st, c)));
   return check_launch("gdn_block_pre_bwd");
 }
 mxb_status gdn_block_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void* kp, const void* vp, const float* cq,
@@ -861,8 +845,8 @@ static mxb_status blk_post(const mxb_gdn_desc* d, const void* o, const void* z, 
                      static_cast<IO*>(d_o), static_cast<IO*>(dz), part)));
   });
   blk::ColSums c{};
-  c.part[0] = part; c.out[0] = dwn; c.rows[0] = ctas; c.n[0] = d->Dv; c.count = 1; c.first[1] = (d->Dv + 31) / 32;
-  MXB_LAUNCH("gdn_block_colsum_kernel", st, (launch_kernel(blk::gdn_block_colsum_kernel, c.first[1], 256, 0, st, c)));
+  c.part[0] = part; c.out[0] = dwn; c.rows[0] = ctas; c.n[0] = d->Dv; c.count = 1; c.first[1] = (d->Dv + kSumCols - 1) / kSumCols;
+  MXB_LAUNCH("gdn_block_colsum_kernel", st, (launch_kernel(blk::gdn_block_colsum_kernel, c.first[1], kSumThreads, 0, st, c)));
   return check_launch("gdn_block_post_bwd");
 }
 mxb_status gdn_block_post(const mxb_gdn_desc* d, const void* o, const void* z, const float* wn, void* y, const void* dy,

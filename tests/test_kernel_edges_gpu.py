@@ -320,3 +320,19 @@ def test_float32_results_of_the_tensor_core_kernels(B, T, K, V):
     for n in ("dq", "dk", "dv", "dbeta", "dgate"):
         assert torch.equal(saved[n], want[n].float()), n
         assert torch.equal(again[n], want[n].float()), n
+
+
+@pytest.mark.parametrize("io", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("cfg", [(1, 4801, 448), (2, 9, 512), (1, 7, 520), (1, 1, 8)])
+def test_block_post_rows_on_both_sides_of_a_warp(cfg, io):
+    """Rows of up to 512 channels belong to a warp, wider ones to a CTA; more partial rows than one round of the column sums."""
+    from test_mamba3_block_gpu import test_post_forward_and_gradients
+    test_post_forward_and_gradients(cfg, io)
+
+
+@pytest.mark.parametrize("io", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("cfg", [(1, 65, 2, 8), (2, 129, 3, 24), (1, 33, 1, 32), (1, 70, 2, 40), (3, 1700, 1, 16), (1, 17, 4, 104)])
+def test_block_bc_rows_of_every_lane_group(cfg, io):
+    """2, 4, 8 and 16 lanes a row, whole and partly filled, with ragged numbers of rows."""
+    from test_mamba3_block_gpu import test_bc_norm_forward_and_gradients
+    test_bc_norm_forward_and_gradients(cfg, io)
