@@ -485,7 +485,6 @@ static size_t carve_m3(M3P& p, void* ws, bool io_f32, size_t partial_floats = 0,
   p.dal_part = cv.take<float>(p.NH > 0 ? parts * p.D : parts * p.D * p.N);
   if (windows) {
     p.dhk = cv.take<float>((size_t)p.B * p.nW * p.D * p.N);
-    p.upk = cv.take<float>((size_t)p.B * p.nW * p.D * p.N);
     p.ang = cv.take<float>((size_t)p.B * p.nW * p.D * p.Kp);
   }
   return cv.bytes();

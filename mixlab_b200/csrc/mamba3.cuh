@@ -27,7 +27,7 @@ struct M3P {
   int vec;             // rows of b, c, theta can be read two state pairs at a time
   float *dtv, *lamv;   // softplus(dt), sigmoid(lambda) in the layout of dt, lambda
   float* dtsum;        // [B,nW,D] sum of dt over the window
-  float *dhk, *upk;    // [B,nW,D,N]: dh entering the window from later steps; `up` of the window's first step
+  float* dhk;          // [B,nW,D,N]: dh entering the window from later steps
   float* ang;          // [B,nW,D,Kp]: angle-gradient sum of the window, then of all later windows
 };
 

@@ -6,7 +6,8 @@
 //   prepare   softplus(dt), sigmoid(lambda) of every (step, channel), window sums of dt theta and dt
 //   scan      angle at each window start
 //   local     walks from a zero state (forward) and from a zero dh (reverse; backward only)
-//   scan      H <- exp(A sum dt) H + local: state at each window start; the same for dh, in reverse
+//   scan      H <- exp(A sum dt) H + local: state at each window start; the same for dh, in reverse (what enters a window is
+//             also what the trapezoid's look-back sends to the window's last step: exp(A dt) up of the step behind)
 //   walk      forward: the true walk writes y;  backward: replay into shared memory, then the true reverse walk with
 //             window-local angle-gradient sums
 //   scan, fix reverse scan of those sums; the later windows' sums are added to ddt and dtheta
@@ -20,6 +21,7 @@
 //
 // Every sum has a fixed order: the same inputs give the same bits.
 #include <algorithm>
+#include <type_traits>
 
 #include "mamba3.cuh"
 #include "packed.cuh"
@@ -261,93 +263,91 @@ __global__ void __launch_bounds__(256) m3w_prepare_kernel(M3P p) {
 }
 
 // -------------------------------------------------------------------- scans
-// 32 chains x 16 segments of windows per CTA: every segment is folded, the folds of the earlier segments give what
-// enters it, and the segment is walked again to write.  Loads in batches ahead of the stores.
+// 16 chains x 32 segments of PER windows per CTA: a segment is loaded once and folded, the folds of the earlier segments give
+// what enters it, and the registers are walked again to write (longer sequences in rounds of 32 PER windows).  Latency and, with
+// a decay, its exponentials bound it.  4096 x 448 channels of 16 states, us: one linear scan / both 20.5 / 51 with every value
+// loaded twice and two or three exponentials, 19.5 / 33 now.
 //   kPhase  ck_phi: window sums -> wrapped angle at each window start
 //   kState  ck_h: local end states -> state at each window start
-//   kDh     dhk: local dh -> dh entering each window from later steps; upk: local -> true `up` of its first step
+//   kDh     dhk: local dh -> dh entering each window from later steps
 //   kAngle  ang: window sums -> sum over all later windows
 enum { kPhase, kState, kDh, kAngle };
-constexpr int kSegs = 16, kBatch = 8;
-template <int MODE>
+constexpr int kChains = 16, kSegs = 32, kScanThreads = kChains * kSegs;
+template <int MODE, int PER>
 __device__ __forceinline__ void scan_chain(const M3P& p, int chains) {
-  __shared__ float s_add[kSegs][32], s_dt[kSegs][32];
-  const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5, b = blockIdx.y;
-  const int i = blockIdx.x * 32 + lane;
+  __shared__ float s_add[kSegs][kChains], s_dec[kSegs][kChains];
+  constexpr bool linear = MODE == kState || MODE == kDh, back = MODE == kDh || MODE == kAngle;
+  const int lane = threadIdx.x % kChains, seg = threadIdx.x / kChains, b = blockIdx.y, i = blockIdx.x * kChains + lane;
   const bool in = i < chains;
-  const bool linear = MODE == kState || MODE == kDh;
-  const int per = (p.nW + kSegs - 1) / kSegs, lo = min(p.nW, seg * per), hi = min(p.nW, lo + per);
   float* buf = MODE == kPhase ? p.ck_phi : MODE == kState ? p.ck_h : MODE == kDh ? p.dhk : p.ang;
   const int d = linear ? i / p.N : 0;
-  const M3Idx ix(p);
-  const float A = linear && in ? -expf(p.a_log[ix.alog(d, i % p.N)]) : 0.f;
-  auto win = [&](int x) { return MODE == kDh || MODE == kAngle ? p.nW - 1 - x : x; };  // x-th window in walking order
-  auto at = [&](int w) { return ((size_t)b * p.nW + w) * chains + i; };
-  float run = 0.f, dts = 0.f;
-  for (int x0 = lo; x0 < hi; x0 += kBatch) {
-    float loc[kBatch], dec[kBatch];
+  const float A = linear && in ? -expf(p.a_log[M3Idx(p).alog(d, i % p.N)]) : 0.f;
+  auto win = [&](int x) { return (size_t)b * p.nW + (back ? p.nW - 1 - x : x); };  // x-th window in walking order
+  auto fold = [](float dec, float run, float add) {
+    return linear ? fmaf(dec, run, add) : MODE == kPhase ? m3_wrap(run + add) : run + add;
+  };
+  float carry = 0.f;
+  for (int x0 = 0; x0 < p.nW; x0 += kSegs * PER) {
+    const int lo = x0 + seg * PER;
+    float loc[PER], dec[PER];
 #pragma unroll
-    for (int x = 0; x < kBatch; ++x) {
-      const bool ok = in && x0 + x < hi;
-      loc[x] = ok ? buf[at(win(x0 + x))] : 0.f;
-      dec[x] = ok && linear ? p.dtsum[((size_t)b * p.nW + win(x0 + x)) * p.D + d] : 0.f;
+    for (int x = 0; x < PER; ++x) {
+      const bool ok = in && lo + x < p.nW;
+      loc[x] = ok ? buf[win(lo + x) * chains + i] : 0.f;
+      dec[x] = ok && linear ? p.dtsum[win(lo + x) * p.D + d] : 0.f;
     }
+    float run = 0.f, dts = 0.f;
 #pragma unroll
-    for (int x = 0; x < kBatch; ++x) {
-      if (linear) run = fmaf(expf(A * dec[x]), run, loc[x]);
-      else run = MODE == kPhase ? m3_wrap(run + loc[x]) : run + loc[x];
+    for (int x = 0; x < PER; ++x) {
       dts += dec[x];
+      if (linear) dec[x] = expf(A * dec[x]);
+      run = fold(dec[x], run, loc[x]);
     }
-  }
-  s_add[seg][lane] = run;
-  s_dt[seg][lane] = dts;
-  __syncthreads();
-  run = 0.f;
-  for (int s = 0; s < seg; ++s) {
-    if (linear) run = fmaf(expf(A * s_dt[s][lane]), run, s_add[s][lane]);
-    else run = MODE == kPhase ? m3_wrap(run + s_add[s][lane]) : run + s_add[s][lane];
-  }
-  for (int x0 = lo; x0 < hi; x0 += kBatch) {
-    float loc[kBatch], dec[kBatch], up[kBatch], dt0[kBatch];
-#pragma unroll
-    for (int x = 0; x < kBatch; ++x) {
-      const bool ok = in && x0 + x < hi;
-      const int w = win(x0 + x);
-      loc[x] = ok ? buf[at(w)] : 0.f;
-      dec[x] = ok && linear ? p.dtsum[((size_t)b * p.nW + w) * p.D + d] : 0.f;
-      if (MODE == kDh) {
-        up[x] = ok ? p.upk[at(w)] : 0.f;
-        dt0[x] = ok ? p.dtv[ix.chan((size_t)b * p.T + (size_t)w * W, d)] : 0.f;
+    s_add[seg][lane] = run;
+    if (linear) s_dec[seg][lane] = expf(A * dts);
+    __syncthreads();
+    run = carry;
+    for (int s = 0; s < kSegs; ++s) {
+      if (s == seg) {
+        carry = run;
+        if (x0 + kSegs * PER >= p.nW) break;  // (the last round)
       }
+      run = fold(linear ? s_dec[s][lane] : 0.f, run, s_add[s][lane]);
     }
+    const float through = run;
+    run = carry;
+    carry = through;
 #pragma unroll
-    for (int x = 0; x < kBatch; ++x) {
-      if (in && x0 + x < hi) {
-        const int w = win(x0 + x);
-        buf[at(w)] = run;
-        if (MODE == kDh) p.upk[at(w)] = fmaf(expf(A * (dec[x] - dt0[x])), run, up[x]);
-      }
-      if (linear) run = fmaf(expf(A * dec[x]), run, loc[x]);
-      else run = MODE == kPhase ? m3_wrap(run + loc[x]) : run + loc[x];
+    for (int x = 0; x < PER; ++x) {
+      if (in && lo + x < p.nW) buf[win(lo + x) * chains + i] = run;
+      run = fold(dec[x], run, loc[x]);
     }
+    __syncthreads();
   }
 }
-__global__ void __launch_bounds__(32 * kSegs) m3w_phase_scan_kernel(M3P p) {
-  begin_dependent(); scan_chain<kPhase>(p, p.D * p.Kp); }
-__global__ void __launch_bounds__(32 * kSegs) m3w_angle_scan_kernel(M3P p) {
-  begin_dependent(); scan_chain<kAngle>(p, p.D * p.Kp); }
-// blockIdx.z: 0 the states, 1 dh (first: the one to start with)
-__global__ void __launch_bounds__(32 * kSegs) m3w_linear_scan_kernel(M3P p, int first) {
+template <int PER>
+__global__ void __launch_bounds__(kScanThreads) m3w_phase_scan_kernel(M3P p) {
   begin_dependent();
-  if (first + (int)blockIdx.z == 0) scan_chain<kState>(p, p.D * p.N);
-  else scan_chain<kDh>(p, p.D * p.N);
+  scan_chain<kPhase, PER>(p, p.D * p.Kp);
+}
+template <int PER>
+__global__ void __launch_bounds__(kScanThreads) m3w_angle_scan_kernel(M3P p) {
+  begin_dependent();
+  scan_chain<kAngle, PER>(p, p.D * p.Kp);
+}
+// blockIdx.z: 0 the states, 1 dh (first: the one to start with)
+template <int PER>
+__global__ void __launch_bounds__(kScanThreads) m3w_linear_scan_kernel(M3P p, int first) {
+  begin_dependent();
+  if (first + (int)blockIdx.z == 0) scan_chain<kState, PER>(p, p.D * p.N);
+  else scan_chain<kDh, PER>(p, p.D * p.N);
 }
 
 // -------------------------------------------------------------- local walks
 // Forward from a zero state (leaves the end state in ck_h) and, with DH, back with dh alone:
 //   up_t = dh_t + dy_t Crot_t,  dh_{t-1} = alpha_t up_t
-// (leaves the dh that leaves the window at its start in dhk and the up of its first step in upk).  Sine, cosine and
-// decay of a step wait in shared memory for the way back.
+// (leaves the dh that leaves the window at its start in dhk).  Sine, cosine and decay of a step wait in shared memory for the
+// way back.
 template <typename IO, int PR, int LPC, bool FWD, bool DH>
 __global__ void __launch_bounds__(256) m3w_local_kernel(M3P p) {
   begin_dependent();
@@ -415,9 +415,9 @@ __global__ void __launch_bounds__(256) m3w_local_kernel(M3P p) {
     for (int u = 0; u < UN; ++u) k.put_states(p.ck_h + k.wrow() * p.N, u, h[2 * u], h[2 * u + 1]);
   }
   if (DH) {
-    f2 dh[PR], up[PR];
+    f2 dh[PR];
 #pragma unroll
-    for (int r = 0; r < PR; ++r) dh[r] = up[r] = 0ull;
+    for (int r = 0; r < PR; ++r) dh[r] = 0ull;
 #pragma unroll
     for (int s = W - 1; s >= 0; --s) {
       const f2 dy = dup2(k.of(dys, s));
@@ -425,17 +425,12 @@ __global__ void __launch_bounds__(256) m3w_local_kernel(M3P p) {
       for (int u = 0; u < UN; ++u) {
         f2 c0, c1;
         k.rot_c(s, u, slot(s, PR + 2 * u), slot(s, PR + 2 * u + 1), c0, c1);
-        up[2 * u] = mad2(dy, c0, dh[2 * u]);
-        up[2 * u + 1] = mad2(dy, c1, dh[2 * u + 1]);
-        dh[2 * u] = mul2(slot(s, 2 * u), up[2 * u]);
-        dh[2 * u + 1] = mul2(slot(s, 2 * u + 1), up[2 * u + 1]);
+        dh[2 * u] = mul2(slot(s, 2 * u), mad2(dy, c0, dh[2 * u]));
+        dh[2 * u + 1] = mul2(slot(s, 2 * u + 1), mad2(dy, c1, dh[2 * u + 1]));
       }
     }
 #pragma unroll
-    for (int u = 0; u < UN; ++u) {
-      k.put_states(p.dhk + k.wrow() * p.N, u, dh[2 * u], dh[2 * u + 1]);
-      k.put_states(p.upk + k.wrow() * p.N, u, up[2 * u], up[2 * u + 1]);
-    }
+    for (int u = 0; u < UN; ++u) k.put_states(p.dhk + k.wrow() * p.N, u, dh[2 * u], dh[2 * u + 1]);
   }
 }
 
@@ -555,19 +550,13 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
   k.own(dys, [&](int s) { return to_f32(DY[(k.row0 + s) * p.D + k.d]); });
   const float px0 = k.ts > 0 ? to_f32(X[(k.row0 - 1) * p.D + k.d]) : 0.f;
   const bool more = k.in(W);  // a window follows: its first step sends something back to this one's last
-  float dt_e = 0.f, bf_e = 0.f;
-  if (more) {
-    dt_e = p.dtv[k.chan(W)];
-    bf_e = (1.f - p.lamv[k.chan(W)]) * dt_e;
-  }
+  const float bf_e = more ? (1.f - p.lamv[k.chan(W)]) * p.dtv[k.chan(W)] : 0.f;
   k.stage(true);
 #pragma unroll
   for (int u = 0; u < UN; ++u) {
     phi[u] = k.two(p.ck_phi + k.wrow() * p.Kp, u);
     k.states(p.ck_h + k.wrow() * p.N, u, h[2 * u], h[2 * u + 1]);
     k.states(p.dhk + k.wrow() * p.N, u, dh[2 * u], dh[2 * u + 1]);
-    pgb[2 * u] = pgb[2 * u + 1] = 0ull;
-    if (more) k.states(p.upk + (k.wrow() + p.D) * p.N, u, pgb[2 * u], pgb[2 * u + 1]);
   }
   k.rates(A);
   __syncthreads();
@@ -604,7 +593,7 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
       slot(s, 2 * PR + 2 * u + 1) = cs;
     }
   }
-  // ---- what the first step of the next window sends back (pgb holds its `up`) ----
+  // ---- what the first step of the next window sends back: its decayed `up` is the dh that enters here ----
   f2 dal[PR], carry[UN];
   f2 pend = 0ull;  // contribution of step t+1 to dx_t (lane partial)
 #pragma unroll
@@ -613,12 +602,10 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
 #pragma unroll
     for (int y = 0; y < 2; ++y) {
       const int r = 2 * u + y;
+      const f2 v = mul2(dup2(bf_e), dh[r]);
       dal[r] = 0ull;
-      if (more) {
-        const f2 v = mul2(pgb[r], mul2(dup2(bf_e), exp2p(A[r], dt_e)));
-        pend = mad2(pb[r], v, pend);
-        pgb[r] = mul2(dup2(px), v);
-      }
+      pend = mad2(pb[r], v, pend);
+      pgb[r] = mul2(dup2(px), v);
     }
   }
   // ---- reverse: pb = rotated b of the step, q = that of the step before ----
@@ -829,7 +816,14 @@ static void m3w_walk(const M3P& p, const M3WGrid& g, F&& launch) {
   const int channels = g.shape.warps * (32 / g.shape.lanes);
   for (M3P q = p; q.w0 < p.nW; q.w0 += 65535) launch(q, dim3((p.D + channels - 1) / channels, std::min(65535, p.nW - q.w0), p.B));
 }
-static dim3 chain_grid(const M3P& p, int chains, int kinds) { return dim3((chains + 31) / 32, p.B, kinds); }
+static dim3 chain_grid(const M3P& p, int chains, int kinds) { return dim3((chains + kChains - 1) / kChains, p.B, kinds); }
+// Windows of a segment: as many as a sequence fills, up to 16 (registers).
+template <typename F>
+static void by_segment(const M3P& p, F&& f) {
+  if (p.nW <= 4 * kSegs) f(std::integral_constant<int, 4>{});
+  else if (p.nW <= 8 * kSegs) f(std::integral_constant<int, 8>{});
+  else f(std::integral_constant<int, 16>{});
+}
 
 template <typename IO, int PR, int LPC, bool FWD, bool DH>
 static mxb_status launch_local(const M3P& p, const M3WGrid& g, cudaStream_t st) {
@@ -856,8 +850,18 @@ static mxb_status prepare(const M3P& p, const M3WGrid& g, cudaStream_t st) {
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
     M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_prepare_kernel", st, (launch_kernel(m3w_prepare_kernel<IO, PRV, LPCV>, grid, g.threads, 0, st, q))));
   });
-  MXB_LAUNCH("m3w_phase_scan_kernel", st, (launch_kernel(m3w_phase_scan_kernel, chain_grid(p, p.D * p.Kp, 1), 32 * kSegs, 0, st, p)));
+  by_segment(p, [&](auto per) {
+    MXB_LAUNCH("m3w_phase_scan_kernel", st,
+               (launch_kernel(m3w_phase_scan_kernel<decltype(per)::value>, chain_grid(p, p.D * p.Kp, 1), kScanThreads, 0, st, p)));
+  });
   return check_launch("mamba3 window preparation");
+}
+
+static void linear_scan(const M3P& p, int first, int kinds, cudaStream_t st) {
+  by_segment(p, [&](auto per) {
+    MXB_LAUNCH("m3w_linear_scan_kernel", st,
+               (launch_kernel(m3w_linear_scan_kernel<decltype(per)::value>, chain_grid(p, p.D * p.N, kinds), kScanThreads, 0, st, p, first)));
+  });
 }
 
 template <typename IO>
@@ -867,7 +871,7 @@ static mxb_status forward(const M3P& p, cudaStream_t st) {
   if (s != MXB_OK) return s;
   M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_local<IO, PRV, LPCV, true, false>(p, g, st)));
   if (s != MXB_OK) return s;
-  MXB_LAUNCH("m3w_linear_scan_kernel", st, (launch_kernel(m3w_linear_scan_kernel, chain_grid(p, p.D * p.N, 1), 32 * kSegs, 0, st, p, 0)));
+  linear_scan(p, 0, 1, st);
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
     M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_out_kernel", st, (launch_kernel(m3w_out_kernel<IO, PRV, LPCV>, grid, g.threads, kRowBytes<IO, PRV, LPCV>, st, q))));
   });
@@ -886,11 +890,13 @@ static mxb_status backward(const M3P& p, bool have_states, cudaStream_t st) {
   }
   if (s != MXB_OK) return s;
   const int first = have_states ? 1 : 0;
-  MXB_LAUNCH("m3w_linear_scan_kernel", st,
-             (launch_kernel(m3w_linear_scan_kernel, chain_grid(p, p.D * p.N, 2 - first), 32 * kSegs, 0, st, p, first)));
+  linear_scan(p, first, 2 - first, st);
   M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_grad<IO, PRV, LPCV>(p, g, st)));
   if (s != MXB_OK) return s;
-  MXB_LAUNCH("m3w_angle_scan_kernel", st, (launch_kernel(m3w_angle_scan_kernel, chain_grid(p, p.D * p.Kp, 1), 32 * kSegs, 0, st, p)));
+  by_segment(p, [&](auto per) {
+    MXB_LAUNCH("m3w_angle_scan_kernel", st,
+               (launch_kernel(m3w_angle_scan_kernel<decltype(per)::value>, chain_grid(p, p.D * p.Kp, 1), kScanThreads, 0, st, p)));
+  });
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
     M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_fix_kernel", st, (launch_kernel(m3w_fix_kernel<IO, PRV, LPCV>, grid, g.threads, 0, st, q))));
   });
