@@ -54,8 +54,8 @@ __device__ __forceinline__ float group_sum(float v) {
 
 struct M3Idx {
   int D, N, G, NH, Kp, cpg, cph;
-  __device__ M3Idx(const M3P& p)
-      : D(p.D), N(p.N), G(p.G), NH(p.NH), Kp(p.Kp), cpg(p.D / p.G), cph(p.NH > 0 ? p.D / p.NH : 1) {}
+  __device__ explicit M3Idx(const M3P& p) : M3Idx(p, p.NH) {}
+  __device__ M3Idx(const M3P& p, int nh) : D(p.D), N(p.N), G(p.G), NH(nh), Kp(p.Kp), cpg(p.D / p.G), cph(nh > 0 ? p.D / nh : 1) {}
   __device__ size_t chan(size_t row, int d) const { return NH > 0 ? row * NH + d / cph : row * D + d; }
   __device__ size_t theta(size_t row, int d, int kp) const {
     return NH > 0 ? row * NH + d / cph : (row * D + d) * Kp + kp;

@@ -17,7 +17,7 @@
 // pairs per lane go through packed arithmetic; a pass keeps sine, cosine and decay in shared memory for its reverse
 // half; rows of dB, dC are added over the channels of a warp by halving exchanges and over the warps once per window.
 // Scans run 16 segments of windows side by side.  2 x 1024 x 128 channels of 16 states, forward + backward:
-// 310 -> 93 us of kernels; 4096 x 448 channels: 1.79 -> 0.59 ms.
+// 70 us a call; 4096 x 448 channels: 0.42 ms.
 //
 // Every sum has a fixed order: the same inputs give the same bits.
 #include <algorithm>
@@ -89,10 +89,18 @@ __global__ void __launch_bounds__(256) m3w_sincos_kernel(const float* __restrict
   }
 }
 __device__ __forceinline__ f2 neg2(f2 v) { return v ^ 0x8000000080000000ull; }
-__device__ __forceinline__ f2 exp2p(f2 a, float dt) {  // exp(dt a), both halves
-  const float2 t = unpack2(a);
-  return pack2(expf(dt * t.x), expf(dt * t.y));
+__device__ __forceinline__ float ex2(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
+// exp(-r dt) of two states, r their decay rates times log2 e.  (expf spends instructions on a range that decays do not have; what
+// ex2 is further off, 2 % of the outputs' distance from float64, is less than the angles at the window starts have gained.)
+__device__ __forceinline__ f2 decay2(f2 r, f2 dt) {
+  const float2 x = unpack2(mul2(r, dt));
+  return pack2(ex2(-x.x), ex2(-x.y));
+}
+constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 
 // One walker: the lanes of one channel in one window.  A lane owns PR state pairs kp = sl PR + r in units of two; a
 // packed value holds the same quantity of both pairs of a unit, even and odd states apart, so that the rotations are
@@ -100,7 +108,8 @@ __device__ __forceinline__ f2 exp2p(f2 a, float dt) {  // exp(dt a), both halves
 // scalars by the lane that owns the step (handed round by shuffles), theta into registers, the rows of b and c into
 // shared memory, where all channels of the CTA read them.  Steps past the end of the sequence read as zeros, which
 // leaves state and gradients untouched; only their results are not stored.
-template <typename IO, int PR, int LPC>
+// PLAIN: per-channel parameters and rows that can be read two pairs at a time, known when compiled.
+template <typename IO, int PR, int LPC, bool PLAIN>
 struct Walker {
   static constexpr int CPW = 32 / LPC;             // channels per warp
   static constexpr int OWN = (W + LPC - 1) / LPC;  // steps whose scalars a lane holds
@@ -109,11 +118,12 @@ struct Walker {
   static constexpr int kRows = 2 * W + 1;          // rows in shared memory: b of ts-1 .. ts+W-1, then c of ts ..
   const M3P& p;
   const M3Idx ix;
+  const bool vec, per_head;
   const int lane, sl, wc, d, b, w, ts, base;
   const size_t row0;
   float* rows;  // [kRows][2 (even, odd)][NP]
   __device__ Walker(const M3P& p_, float* rows_)
-      : p(p_), ix(p_), lane(threadIdx.x & 31), sl(lane % LPC), wc((threadIdx.x >> 5) * CPW + lane / LPC),
+      : p(p_), ix(p_, PLAIN ? 0 : p_.NH), vec(PLAIN || p_.vec), per_head(!PLAIN && p_.NH > 0), lane(threadIdx.x & 31), sl(lane % LPC), wc((threadIdx.x >> 5) * CPW + lane / LPC),
         d(blockIdx.x * ((blockDim.x >> 5) * CPW) + wc), b(blockIdx.z), w(p_.w0 + blockIdx.y), ts(w * W), base(lane / LPC * LPC),
         row0((size_t)b * p_.T + ts), rows(rows_) {}
   __device__ bool act(int r) const { return sl * PR + r < p.Kp; }
@@ -158,7 +168,7 @@ struct Walker {
   // one value per pair, from a row of Kp
   __device__ f2 two(const float* s, int u) const {
     s += sl * PR + 2 * u;
-    if (p.vec) {
+    if (vec) {
       if (!act(2 * u)) return 0ull;
       const float2 x = *reinterpret_cast<const float2*>(s);
       return pack2(x.x, x.y);
@@ -168,7 +178,7 @@ struct Walker {
   __device__ void put_two(float* s, int u, f2 v) const {
     const float2 x = unpack2(v);
     s += sl * PR + 2 * u;
-    if (p.vec) {
+    if (vec) {
       if (act(2 * u)) *reinterpret_cast<float2*>(s) = x;
       return;
     }
@@ -176,17 +186,17 @@ struct Walker {
     if (act(2 * u + 1)) s[1] = x.y;
   }
   __device__ void thetas(f2 (&th)[W][UN]) const {
-    const size_t stride = p.NH > 0 ? p.NH : (size_t)p.D * p.Kp;
+    const size_t stride = per_head ? p.NH : (size_t)p.D * p.Kp;
     const float* src = p.theta + ix.theta(row0, d, 0);
 #pragma unroll
     for (int s = 0; s < W; ++s)
 #pragma unroll
-      for (int u = 0; u < UN; ++u) th[s][u] = !in(s) ? 0ull : p.NH > 0 ? dup2(src[s * stride]) : two(src + s * stride, u);
+      for (int u = 0; u < UN; ++u) th[s][u] = !in(s) ? 0ull : per_head ? dup2(src[s * stride]) : two(src + s * stride, u);
   }
   // a row of N states: even (v0) and odd (v1) states of a unit
   __device__ void states(const float* s, int u, f2& v0, f2& v1) const {
     s += 2 * (sl * PR + 2 * u);
-    if (p.vec) {
+    if (vec) {
       const float4 x = act(2 * u) ? *reinterpret_cast<const float4*>(s) : make_float4(0.f, 0.f, 0.f, 0.f);
       v0 = pack2(x.x, x.z);
       v1 = pack2(x.y, x.w);
@@ -198,19 +208,19 @@ struct Walker {
   __device__ void put_states(float* s, int u, f2 v0, f2 v1) const {
     const float2 x = unpack2(v0), y = unpack2(v1);
     s += 2 * (sl * PR + 2 * u);
-    if (p.vec) {
+    if (vec) {
       if (act(2 * u)) *reinterpret_cast<float4*>(s) = make_float4(x.x, y.x, x.y, y.y);
       return;
     }
     if (act(2 * u)) { s[0] = x.x; s[1] = y.x; }
     if (act(2 * u + 1)) { s[2] = x.y; s[3] = y.y; }
   }
-  __device__ void rates(f2 (&A)[PR]) const {  // A[2 u]: even states of unit u, A[2 u + 1]: odd
+  __device__ void rates(f2 (&A)[PR]) const {  // decay rates times log2 e; A[2 u]: even states of unit u, A[2 u + 1]: odd
 #pragma unroll
     for (int u = 0; u < UN; ++u) {
       float a[4];
 #pragma unroll
-      for (int x = 0; x < 4; ++x) a[x] = act(2 * u + x / 2) ? -expf(p.a_log[ix.alog(d, 2 * (sl * PR + 2 * u) + x)]) : 0.f;
+      for (int x = 0; x < 4; ++x) a[x] = act(2 * u + x / 2) ? kLog2e * expf(p.a_log[ix.alog(d, 2 * (sl * PR + 2 * u) + x)]) : 0.f;
       A[2 * u] = pack2(a[0], a[2]);
       A[2 * u + 1] = pack2(a[1], a[3]);
     }
@@ -225,18 +235,18 @@ struct Walker {
     }
   }
 };
-template <typename IO, int PR, int LPC>
+template <int PR, int LPC>
 constexpr int kRowBytes = (2 * W + 1) * 2 * PR * LPC * 4;
 
 // ------------------------------------------------------------------ prepare
-template <typename IO, int PR, int LPC>
-__global__ void __launch_bounds__(256) m3w_prepare_kernel(M3P p) {
+template <typename IO, int PR, int LPC, bool PLAIN>
+__global__ void __launch_bounds__(256, 7) m3w_prepare_kernel(M3P p) {
   begin_dependent();
-  using K = Walker<IO, PR, LPC>;
+  using K = Walker<IO, PR, LPC, PLAIN>;
   const K k(p, nullptr);
   f2 th[W][K::UN], ph[K::UN];
   k.thetas(th);
-  const bool store = p.NH == 0 || k.d % k.ix.cph == 0;
+  const bool store = !k.per_head || k.d % k.ix.cph == 0;
   float dts[K::OWN];
   k.own(dts, [&](int s) {
     const size_t i = k.chan(s);
@@ -267,36 +277,58 @@ __global__ void __launch_bounds__(256) m3w_prepare_kernel(M3P p) {
 // what enters it, and the registers are walked again to write (longer sequences in rounds of 32 PER windows).  Latency and, with
 // a decay, its exponentials bound it.  4096 x 448 channels of 16 states, us: one linear scan / both 20.5 / 51 with every value
 // loaded twice and two or three exponentials, 19.5 / 33 now.
-//   kPhase  ck_phi: window sums -> wrapped angle at each window start
+//   kPhase  ck_phi: window sums -> wrapped angle at each window start, summed in 32-bit turns, which wrap by themselves and round
+//           nothing: the rounding of float sums, wrapped one by one, was a good part of the distance of every result from
+//           float64 (y 3.19e-7, dtheta 9.5e-7 over six
+//           problems of 257 to 1200 steps; 2.82e-7 and 7.9e-7 now)
 //   kState  ck_h: local end states -> state at each window start
 //   kDh     dhk: local dh -> dh entering each window from later steps
 //   kAngle  ang: window sums -> sum over all later windows
 enum { kPhase, kState, kDh, kAngle };
+// An angle in units of 2^-32 of a turn: the rounded product, and what its rounding left.
+__device__ __forceinline__ uint32_t turns(float x) {
+  x = m3_wrap(x);
+  const float p = x * 683565248.f, e = fmaf(x, 27.5764316f, fmaf(x, 683565248.f, -p));
+  return (uint32_t)__float2int_rn(p) + (uint32_t)__float2int_rn(e);
+}
 constexpr int kChains = 16, kSegs = 32, kScanThreads = kChains * kSegs;
 template <int MODE, int PER>
 __device__ __forceinline__ void scan_chain(const M3P& p, int chains) {
-  __shared__ float s_add[kSegs][kChains], s_dec[kSegs][kChains];
   constexpr bool linear = MODE == kState || MODE == kDh, back = MODE == kDh || MODE == kAngle;
+  using Sum = std::conditional_t<MODE == kPhase, uint32_t, float>;
+  __shared__ Sum s_add[kSegs][kChains];
+  __shared__ float s_dec[kSegs][kChains];
   const int lane = threadIdx.x % kChains, seg = threadIdx.x / kChains, b = blockIdx.y, i = blockIdx.x * kChains + lane;
   const bool in = i < chains;
   float* buf = MODE == kPhase ? p.ck_phi : MODE == kState ? p.ck_h : MODE == kDh ? p.dhk : p.ang;
   const int d = linear ? i / p.N : 0;
   const float A = linear && in ? -expf(p.a_log[M3Idx(p).alog(d, i % p.N)]) : 0.f;
   auto win = [&](int x) { return (size_t)b * p.nW + (back ? p.nW - 1 - x : x); };  // x-th window in walking order
-  auto fold = [](float dec, float run, float add) {
-    return linear ? fmaf(dec, run, add) : MODE == kPhase ? m3_wrap(run + add) : run + add;
+  auto value = [](float x) -> Sum {
+    if constexpr (MODE == kPhase) return turns(x);
+    else return x;
   };
-  float carry = 0.f;
+  auto result = [](Sum run) -> float {
+    if constexpr (MODE == kPhase) return (float)(int)run * 1.4629180792671596e-9f;  // 2 pi / 2^32
+    else return run;
+  };
+  auto fold = [](float dec, Sum run, Sum add) -> Sum {
+    if constexpr (linear) return fmaf(dec, run, add);
+    else return run + add;
+  };
+  Sum carry = 0;
   for (int x0 = 0; x0 < p.nW; x0 += kSegs * PER) {
     const int lo = x0 + seg * PER;
-    float loc[PER], dec[PER];
+    Sum loc[PER];
+    float dec[PER];
 #pragma unroll
     for (int x = 0; x < PER; ++x) {
       const bool ok = in && lo + x < p.nW;
-      loc[x] = ok ? buf[win(lo + x) * chains + i] : 0.f;
+      loc[x] = value(ok ? buf[win(lo + x) * chains + i] : 0.f);
       dec[x] = ok && linear ? p.dtsum[win(lo + x) * p.D + d] : 0.f;
     }
-    float run = 0.f, dts = 0.f;
+    Sum run = 0;
+    float dts = 0.f;
 #pragma unroll
     for (int x = 0; x < PER; ++x) {
       dts += dec[x];
@@ -314,12 +346,12 @@ __device__ __forceinline__ void scan_chain(const M3P& p, int chains) {
       }
       run = fold(linear ? s_dec[s][lane] : 0.f, run, s_add[s][lane]);
     }
-    const float through = run;
+    const Sum through = run;
     run = carry;
     carry = through;
 #pragma unroll
     for (int x = 0; x < PER; ++x) {
-      if (in && lo + x < p.nW) buf[win(lo + x) * chains + i] = run;
+      if (in && lo + x < p.nW) buf[win(lo + x) * chains + i] = result(run);
       run = fold(dec[x], run, loc[x]);
     }
     __syncthreads();
@@ -348,16 +380,16 @@ __global__ void __launch_bounds__(kScanThreads) m3w_linear_scan_kernel(M3P p, in
 //   up_t = dh_t + dy_t Crot_t,  dh_{t-1} = alpha_t up_t
 // (leaves the dh that leaves the window at its start in dhk).  Sine, cosine and decay of a step wait in shared memory for the
 // way back.
-template <typename IO, int PR, int LPC, bool FWD, bool DH>
+template <typename IO, int PR, int LPC, bool PLAIN, bool FWD, bool DH>
 __global__ void __launch_bounds__(256) m3w_local_kernel(M3P p) {
   begin_dependent();
-  using K = Walker<IO, PR, LPC>;
+  using K = Walker<IO, PR, LPC, PLAIN>;
   constexpr int UN = K::UN;
   extern __shared__ f2 hist[];  // [W][2 PR][threads], then the rows
   const K k(p, reinterpret_cast<float*>(hist + (DH ? W * 2 * PR * blockDim.x : 0)));
   auto slot = [&](int s, int x) -> f2& { return hist[(s * (2 * PR) + x) * blockDim.x + threadIdx.x]; };
   const IO *X = static_cast<const IO*>(p.x), *DY = static_cast<const IO*>(p.dy);
-  f2 th[W][UN], A[PR], phi[UN];
+  f2 th[W][UN], phi[UN], A[PR];
   k.thetas(th);
   float dts[K::OWN], lams[K::OWN], xs[K::OWN], dys[K::OWN], px = 0.f;
   k.own(dts, [&](int s) { return p.dtv[k.chan(s)]; });
@@ -393,7 +425,7 @@ __global__ void __launch_bounds__(256) m3w_local_kernel(M3P p) {
       f2 sn, cs;
       phi[u] = wrap2(mad2(dup2(dt), th[s][u], phi[u]));
       sincos2(phi[u], sn, cs);
-      const f2 al0 = exp2p(A[2 * u], dt), al1 = exp2p(A[2 * u + 1], dt);
+      const f2 al0 = decay2(A[2 * u], dup2(dt)), al1 = decay2(A[2 * u + 1], dup2(dt));
       if (DH) {
         slot(s, 2 * u) = al0;
         slot(s, 2 * u + 1) = al1;
@@ -435,16 +467,16 @@ __global__ void __launch_bounds__(256) m3w_local_kernel(M3P p) {
 }
 
 // ------------------------------------------------------------ forward walk
-template <typename IO, int PR, int LPC>
+template <typename IO, int PR, int LPC, bool PLAIN>
 __global__ void __launch_bounds__(256) m3w_out_kernel(M3P p) {
   begin_dependent();
-  using K = Walker<IO, PR, LPC>;
+  using K = Walker<IO, PR, LPC, PLAIN>;
   constexpr int UN = K::UN;
   extern __shared__ f2 hist[];
   const K k(p, reinterpret_cast<float*>(hist));
   const IO* X = static_cast<const IO*>(p.x);
   IO* Y = static_cast<IO*>(p.y);
-  f2 th[W][UN], A[PR], h[PR], phi[UN], pb[PR];
+  f2 th[W][UN], h[PR], phi[UN], pb[PR], A[PR];
   k.thetas(th);
   float dts[K::OWN], lams[K::OWN], xs[K::OWN];
   k.own(dts, [&](int s) { return p.dtv[k.chan(s)]; });
@@ -474,8 +506,8 @@ __global__ void __launch_bounds__(256) m3w_out_kernel(M3P p) {
       sincos2(phi[u], sn, cs);
       k.rot_b(s, u, sn, cs, b0, b1);
       k.rot_c(s, u, sn, cs, c0, c1);
-      h[2 * u] = mad2(exp2p(A[2 * u], dt), mad2(bx, pb[2 * u], h[2 * u]), mul2(gx, b0));
-      h[2 * u + 1] = mad2(exp2p(A[2 * u + 1], dt), mad2(bx, pb[2 * u + 1], h[2 * u + 1]), mul2(gx, b1));
+      h[2 * u] = mad2(decay2(A[2 * u], dup2(dt)), mad2(bx, pb[2 * u], h[2 * u]), mul2(gx, b0));
+      h[2 * u + 1] = mad2(decay2(A[2 * u + 1], dup2(dt)), mad2(bx, pb[2 * u + 1], h[2 * u + 1]), mul2(gx, b1));
       part = mad2(h[2 * u], c0, part);
       part = mad2(h[2 * u + 1], c1, part);
       pb[2 * u] = b0;
@@ -522,26 +554,32 @@ __device__ __forceinline__ float sum_lanes4(float a, float b, float c, float d, 
 }
 
 template <int PR, int LPC>
-struct GradSmem {  // bytes per thread, per warp and fixed
-  static constexpr int kThread = W * 3 * PR * 8, kWarp = W * 2 * 2 * PR * LPC * 4 + W * (32 / LPC) * 5 * 4;
+struct GradSmem {  // bytes per thread and per warp
+  static constexpr int kThread = W * 2 * PR * 8, kWarp = W * 2 * 2 * PR * LPC * 4 + W * (32 / LPC) * 5 * 4;
 };
-// grid (D / channels of a CTA, windows, B)
-template <typename IO, int PR, int LPC>
-__global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
+// grid (D / channels of a CTA, windows, B).  What a step needs of its channel waits in shared memory, one read for all lanes (four
+// shuffles and the products of three scalars a step and pass before), and its results take the place; the decay is computed again
+// on the way back.  That makes room for three CTAs of seven warps an SM (two before): 4096 x 448 channels of 16 states 190 us ->
+// 161.
+template <typename IO, int PR, int LPC, bool PLAIN>
+__global__ void __maxnreg__(PR == 2 ? 96 : 168) m3w_grad_kernel(M3P p) {
   begin_dependent();
-  using K = Walker<IO, PR, LPC>;
+  using K = Walker<IO, PR, LPC, PLAIN>;
   constexpr int UN = K::UN, CPW = K::CPW, KEEP = 4 * PR / CPW > 0 ? 4 * PR / CPW : 1, NR = 2 * K::NP;
   static_assert(4 * PR >= CPW, "a lane keeps at least one sum");
-  extern __shared__ f2 hist[];  // [W][3 PR][threads]: h after the step, decay, sine / cosine
+  extern __shared__ f2 hist[];  // [W][2 PR][threads]: h after the step, sine / cosine
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5;
-  float* red = reinterpret_cast<float*>(hist + (size_t)W * 3 * PR * blockDim.x);  // [W][warps][2 (dB, dC)][NR]
-  float* fin = red + (size_t)W * warps * 2 * NR;                                  // [W][channels][4]
-  float* fin5 = fin + W * warps * CPW * 4;                                        // [W][channels]
+  float* red = reinterpret_cast<float*>(hist + (size_t)W * 2 * PR * blockDim.x);  // [W][warps][2 (dB, dC)][NR]
+  // per (step, channel): dt, lambda dt x, (1 - lambda) dt x of the step before, dy, then b.up, q.v, the rest of d/d dt, dx of the
+  // later step; and (1 - lambda) dt, then the angle's gradient
+  float4* fin = reinterpret_cast<float4*>(red + (size_t)W * warps * 2 * NR);
+  float* fin5 = reinterpret_cast<float*>(fin + W * warps * CPW);
   const K k(p, fin5 + W * warps * CPW);
-  auto slot = [&](int s, int x) -> f2& { return hist[(s * (3 * PR) + x) * blockDim.x + threadIdx.x]; };
+  auto slot = [&](int s, int x) -> f2& { return hist[(s * (2 * PR) + x) * blockDim.x + threadIdx.x]; };
   const IO *X = static_cast<const IO*>(p.x), *DY = static_cast<const IO*>(p.dy);
-  const bool per_head = p.NH > 0;
-  f2 th[W][UN], A[PR], h[PR], pb[PR], phi[UN], dh[PR], pgb[PR];
+  const bool per_head = k.per_head;
+  auto at = [&](int s) { return s * warps * CPW + k.wc; };
+  f2 th[W][UN], h[PR], pb[PR], phi[UN], dh[PR], pgb[PR], A[PR];
   k.thetas(th);
   float dts[K::OWN], lams[K::OWN], xs[K::OWN], dys[K::OWN];
   k.own(dts, [&](int s) { return p.dtv[k.chan(s)]; });
@@ -549,6 +587,19 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
   k.own(xs, [&](int s) { return to_f32(X[(k.row0 + s) * p.D + k.d]); });
   k.own(dys, [&](int s) { return to_f32(DY[(k.row0 + s) * p.D + k.d]); });
   const float px0 = k.ts > 0 ? to_f32(X[(k.row0 - 1) * p.D + k.d]) : 0.f;
+  float xps[K::OWN];  // x of the step before
+#pragma unroll
+  for (int o = 0; o < K::OWN; ++o) {
+    const int s = k.sl + LPC * o;
+    const float xp = __shfl_sync(0xffffffffu, o > 0 && k.sl == LPC - 1 ? xs[o > 0 ? o - 1 : 0] : xs[o], (k.sl == 0 ? k.base + LPC - 1 : k.lane - 1));
+    xps[o] = s == 0 ? px0 : xp;
+    if (s < W) {
+      const float bf = (1.f - lams[o]) * dts[o];
+      fin[at(s)] = make_float4(dts[o], lams[o] * dts[o] * xs[o], bf * xps[o], dys[o]);
+      fin5[at(s)] = bf;
+    }
+  }
+  const float px = k.of(xs, W - 1);
   const bool more = k.in(W);  // a window follows: its first step sends something back to this one's last
   const float bf_e = more ? (1.f - p.lamv[k.chan(W)]) * p.dtv[k.chan(W)] : 0.f;
   k.stage(true);
@@ -567,30 +618,26 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
     hs[r] = h[r];
     pbs[r] = pb[r];
   }
-  // ---- replay, keeping state, decay, sine and cosine of every step ----
-  float px = px0;
+  // ---- replay, keeping state, sine and cosine of every step ----
 #pragma unroll
   for (int s = 0; s < W; ++s) {
-    const float dt = k.of(dts, s), lam = k.of(lams, s), x = k.of(xs, s);
-    const f2 gx = dup2(lam * dt * x), bx = dup2((1.f - lam) * dt * px);
-    px = x;
+    const float4 f = fin[at(s)];
+    const f2 dt = dup2(f.x), gx = dup2(f.y), bx = dup2(f.z);
 #pragma unroll
     for (int u = 0; u < UN; ++u) {
       f2 sn, cs, b0, b1;
-      phi[u] = wrap2(mad2(dup2(dt), th[s][u], phi[u]));
+      phi[u] = wrap2(mad2(dt, th[s][u], phi[u]));
       sincos2(phi[u], sn, cs);
       k.rot_b(s, u, sn, cs, b0, b1);
-      const f2 al0 = exp2p(A[2 * u], dt), al1 = exp2p(A[2 * u + 1], dt);
+      const f2 al0 = decay2(A[2 * u], dt), al1 = decay2(A[2 * u + 1], dt);
       h[2 * u] = mad2(al0, mad2(bx, pb[2 * u], h[2 * u]), mul2(gx, b0));
       h[2 * u + 1] = mad2(al1, mad2(bx, pb[2 * u + 1], h[2 * u + 1]), mul2(gx, b1));
       pb[2 * u] = b0;
       pb[2 * u + 1] = b1;
       slot(s, 2 * u) = h[2 * u];
       slot(s, 2 * u + 1) = h[2 * u + 1];
-      slot(s, PR + 2 * u) = al0;
-      slot(s, PR + 2 * u + 1) = al1;
-      slot(s, 2 * PR + 2 * u) = sn;
-      slot(s, 2 * PR + 2 * u + 1) = cs;
+      slot(s, PR + 2 * u) = sn;
+      slot(s, PR + 2 * u + 1) = cs;
     }
   }
   // ---- what the first step of the next window sends back: its decayed `up` is the dh that enters here ----
@@ -611,17 +658,16 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
   // ---- reverse: pb = rotated b of the step, q = that of the step before ----
 #pragma unroll
   for (int s = W - 1; s >= 0; --s) {
-    const float dt = k.of(dts, s), lam = k.of(lams, s), x = k.of(xs, s), dy = k.of(dys, s);
-    const float xprev = s > 0 ? k.of(xs, s > 0 ? s - 1 : 0) : px0;
-    const float bf = (1.f - lam) * dt;
-    const f2 dy2 = dup2(dy), gx = dup2(lam * dt * x), bx = dup2(bf * xprev), dt2 = dup2(dt);
-    f2 s_bu = 0ull, s_qv = 0ull, s_a = 0ull, s_ca = 0ull;
+    const float4 f = fin[at(s)];
+    const float bf = fin5[at(s)];
+    const f2 dt2 = dup2(f.x), gx = dup2(f.y), bx = dup2(f.z), dy2 = dup2(f.w);
+    f2 s_bu = 0ull, s_qv = 0ull, s_a = 0ull, s_w = 0ull, s_ca = 0ull;  // (s_w: times -log2 e)
     float rows[4 * PR];  // this lane's values of dB (first half) and dC of the step
 #pragma unroll
     for (int u = 0; u < UN; ++u) {
-      const f2 sn = slot(s, 2 * PR + 2 * u), cs = slot(s, 2 * PR + 2 * u + 1), nsn = neg2(sn);
+      const f2 sn = slot(s, PR + 2 * u), cs = slot(s, PR + 2 * u + 1), nsn = neg2(sn);
       f2 q[2], c[2], gb[2], gc[2];
-      if (s > 0) k.rot_b(s - 1, u, slot(s - 1, 2 * PR + 2 * u), slot(s - 1, 2 * PR + 2 * u + 1), q[0], q[1]);
+      if (s > 0) k.rot_b(s - 1, u, slot(s - 1, PR + 2 * u), slot(s - 1, PR + 2 * u + 1), q[0], q[1]);
       else { q[0] = pbs[2 * u]; q[1] = pbs[2 * u + 1]; }
       k.rot_c(s, u, sn, cs, c[0], c[1]);
 #pragma unroll
@@ -629,13 +675,13 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
         const int r = 2 * u + y;
         const f2 hb = s > 0 ? slot(s - 1, r) : hs[r];
         const f2 up = mad2(dy2, c[y], dh[r]);
-        const f2 v = mul2(slot(s, PR + r), up);
+        const f2 v = mul2(decay2(A[r], dt2), up);
         s_bu = mad2(pb[r], up, s_bu);
         s_qv = mad2(q[y], v, s_qv);
         gb[y] = mad2(gx, up, pgb[r]);
         gc[y] = mul2(dy2, slot(s, r));
         const f2 wv = mul2(A[r], mul2(v, mad2(bx, q[y], hb)));
-        s_a = add2(s_a, wv);
+        s_w = add2(s_w, wv);
         dal[r] = mad2(dt2, wv, dal[r]);
         pgb[r] = mul2(bx, v);
         dh[r] = v;
@@ -656,11 +702,13 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
       if (per_head) s_ca = add2(s_ca, carry[u]);
       else if (k.in(s)) k.put_two(p.dtheta + ((k.row0 + s) * p.D + k.d) * p.Kp, u, mul2(carry[u], dt2));
     }
+    s_a = mad2(dup2(-kLn2), s_w, s_a);
     const float v = sum_lanes4<LPC>(sum2(s_bu), sum2(s_qv), sum2(s_a), sum2(pend), k.sl);
-    if (k.sl < 4) fin[(s * warps * CPW + k.wc) * 4 + k.sl] = v;
+    __syncwarp();
+    if (k.sl < 4) reinterpret_cast<float*>(fin + at(s))[k.sl] = v;
     if (per_head) {
       const float t = group_sum<LPC>(sum2(s_ca));
-      if (k.sl == 0) fin5[s * warps * CPW + k.wc] = t;
+      if (k.sl == 0) fin5[at(s)] = t;
     }
     pend = mul2(dup2(bf), s_qv);
     const int first = sum_channels<4 * PR, CPW, LPC>(rows, k.lane / LPC);
@@ -673,7 +721,9 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
   }
 #pragma unroll
   for (int u = 0; u < UN; ++u) k.put_two(p.ang + k.wrow() * p.Kp, u, carry[u]);
-  // da_log: d/d a_log = d/dA * A  (A = -exp(a_log)); the closed form above already carries A
+  // da_log: d/d a_log = d/dA * A  (A = -exp(a_log)); the closed form above already carries A (times -log2 e)
+#pragma unroll
+  for (int r = 0; r < PR; ++r) dal[r] = mul2(dup2(-kLn2), dal[r]);
   if (per_head) {
     f2 sum = 0ull;
 #pragma unroll
@@ -688,10 +738,9 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
 #pragma unroll
   for (int o = 0; o < K::OWN; ++o) {  // the lane that owns a step finishes its scalars: dx, ddt, dlambda
     const int s = k.sl + LPC * o;
-    const float xp = __shfl_sync(0xffffffffu, o > 0 && k.sl == LPC - 1 ? xs[o > 0 ? o - 1 : 0] : xs[o], (k.sl == 0 ? k.base + LPC - 1 : k.lane - 1));
     if (s < W && k.in(s)) {
-      const float4 f = *reinterpret_cast<const float4*>(fin + (s * warps * CPW + k.wc) * 4);  // b.up, q.v, rest, dx of later step
-      const float dt = dts[o], lam = lams[o], x = xs[o], xprev = s == 0 ? px0 : xp;
+      const float4 f = fin[at(s)];  // b.up, q.v, rest, dx of later step
+      const float dt = dts[o], lam = lams[o], x = xs[o], xprev = xps[o];
       const size_t i = (k.row0 + s) * p.D + k.d, ci = k.chan(s);
       static_cast<IO*>(p.dx)[i] = from_f32<IO>(fmaf(lam * dt, f.x, f.w));
       const float dsp = (f.z + (1.f - lam) * xprev * f.y + lam * x * f.x) * m3_sigmoid(p.dt[ci]);
@@ -700,7 +749,7 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
         const size_t btd = (size_t)p.B * p.T * p.D;
         p.hd[i] = dsp;
         p.hd[btd + i] = dlam;
-        p.hd[2 * btd + i] = fin5[s * warps * CPW + k.wc] * dt;
+        p.hd[2 * btd + i] = fin5[at(s)] * dt;
       } else {
         p.ddt[ci] = dsp;
         p.dlam[ci] = dlam;
@@ -720,14 +769,14 @@ __global__ void __launch_bounds__(256) m3w_grad_kernel(M3P p) {
 
 // The angle gradient reaches every earlier step: the later windows' sums are added to ddt and dtheta of each step
 // (the walks used only the sums inside their own window).
-template <typename IO, int PR, int LPC>
+template <typename IO, int PR, int LPC, bool PLAIN>
 __global__ void __launch_bounds__(256) m3w_fix_kernel(M3P p) {
   begin_dependent();
-  using K = Walker<IO, PR, LPC>;
+  using K = Walker<IO, PR, LPC, PLAIN>;
   constexpr int UN = K::UN;
   const K k(p, nullptr);
   if (k.w == p.nW - 1) return;  // nothing comes after the last window (every other one is whole)
-  const bool per_head = p.NH > 0;
+  const bool per_head = k.per_head;
   const size_t stride = (size_t)p.D * p.Kp;
   float* dst = p.dtheta + (k.row0 * p.D + k.d) * p.Kp;
   f2 off[UN], th[W][UN], dth[W][UN];
@@ -793,13 +842,19 @@ M3WinShape m3w_shape(const M3P& p) {
   return s;
 }
 
-#define M3W_DISPATCH(lanes, Kp, call)                                       \
-  do {                                                                      \
-    if ((Kp) > 64) { constexpr int PRV = 4, LPCV = 32; call; }              \
-    else if ((lanes) == 4) { constexpr int PRV = 2, LPCV = 4; call; }       \
-    else if ((lanes) == 8) { constexpr int PRV = 2, LPCV = 8; call; }       \
-    else if ((lanes) == 16) { constexpr int PRV = 2, LPCV = 16; call; }     \
-    else { constexpr int PRV = 2, LPCV = 32; call; }                        \
+#define M3W_DISPATCH(lanes, p, call)                                                                      \
+  do {                                                                                                    \
+    const bool plain = (p).vec && (p).NH == 0;                                                            \
+    if ((p).Kp > 64) { constexpr int PRV = 4, LPCV = 32; constexpr bool PL = false; call; }               \
+    else if ((lanes) == 4) {                                                                              \
+      constexpr int PRV = 2, LPCV = 4;                                                                    \
+      if (plain) { constexpr bool PL = true; call; } else { constexpr bool PL = false; call; }            \
+    } else if ((lanes) == 8) {                                                                            \
+      constexpr int PRV = 2, LPCV = 8;                                                                    \
+      if (plain) { constexpr bool PL = true; call; } else { constexpr bool PL = false; call; }            \
+    }                                                                                                     \
+    else if ((lanes) == 16) { constexpr int PRV = 2, LPCV = 16; constexpr bool PL = false; call; }        \
+    else { constexpr int PRV = 2, LPCV = 32; constexpr bool PL = false; call; }                           \
   } while (0)
 
 struct M3WGrid {
@@ -825,30 +880,30 @@ static void by_segment(const M3P& p, F&& f) {
   else f(std::integral_constant<int, 16>{});
 }
 
-template <typename IO, int PR, int LPC, bool FWD, bool DH>
+template <typename IO, int PR, int LPC, bool PLAIN, bool FWD, bool DH>
 static mxb_status launch_local(const M3P& p, const M3WGrid& g, cudaStream_t st) {
-  constexpr int per_thread = DH ? W * 2 * PR * 8 : 0, rows = kRowBytes<IO, PR, LPC>;
+  constexpr int per_thread = DH ? W * 2 * PR * 8 : 0, rows = kRowBytes<PR, LPC>;
   const int sm = per_thread * g.threads + rows;
-  if (MXB_ALLOW_SMEM(per_thread * (PR == 4 ? 128 : 256) + rows, m3w_local_kernel<IO, PR, LPC, FWD, DH>) != MXB_OK) return MXB_ERR_CUDA;
+  if (MXB_ALLOW_SMEM(per_thread * (PR == 4 ? 128 : 256) + rows, m3w_local_kernel<IO, PR, LPC, PLAIN, FWD, DH>) != MXB_OK) return MXB_ERR_CUDA;
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
-    MXB_LAUNCH("m3w_local_kernel", st, (launch_kernel(m3w_local_kernel<IO, PR, LPC, FWD, DH>, grid, g.threads, sm, st, q)));
+    MXB_LAUNCH("m3w_local_kernel", st, (launch_kernel(m3w_local_kernel<IO, PR, LPC, PLAIN, FWD, DH>, grid, g.threads, sm, st, q)));
   });
   return MXB_OK;
 }
-template <typename IO, int PR, int LPC>
+template <typename IO, int PR, int LPC, bool PLAIN>
 static mxb_status launch_grad(const M3P& p, const M3WGrid& g, cudaStream_t st) {
-  constexpr int per_warp = 32 * GradSmem<PR, LPC>::kThread + GradSmem<PR, LPC>::kWarp, rows = kRowBytes<IO, PR, LPC>;
-  if (MXB_ALLOW_SMEM((PR == 4 ? 4 : 8) * per_warp + rows, m3w_grad_kernel<IO, PR, LPC>) != MXB_OK) return MXB_ERR_CUDA;
+  constexpr int per_warp = 32 * GradSmem<PR, LPC>::kThread + GradSmem<PR, LPC>::kWarp, rows = kRowBytes<PR, LPC>;
+  if (MXB_ALLOW_SMEM((PR == 4 ? 4 : 8) * per_warp + rows, m3w_grad_kernel<IO, PR, LPC, PLAIN>) != MXB_OK) return MXB_ERR_CUDA;
   const int sm = g.shape.warps * per_warp + rows;
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
-    MXB_LAUNCH("m3w_grad_kernel", st, (launch_kernel(m3w_grad_kernel<IO, PR, LPC>, grid, g.threads, sm, st, q)));
+    MXB_LAUNCH("m3w_grad_kernel", st, (launch_kernel(m3w_grad_kernel<IO, PR, LPC, PLAIN>, grid, g.threads, sm, st, q)));
   });
   return MXB_OK;
 }
 template <typename IO>
 static mxb_status prepare(const M3P& p, const M3WGrid& g, cudaStream_t st) {
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
-    M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_prepare_kernel", st, (launch_kernel(m3w_prepare_kernel<IO, PRV, LPCV>, grid, g.threads, 0, st, q))));
+    M3W_DISPATCH(g.shape.lanes, p, MXB_LAUNCH("m3w_prepare_kernel", st, (launch_kernel(m3w_prepare_kernel<IO, PRV, LPCV, PL>, grid, g.threads, 0, st, q))));
   });
   by_segment(p, [&](auto per) {
     MXB_LAUNCH("m3w_phase_scan_kernel", st,
@@ -869,11 +924,11 @@ static mxb_status forward(const M3P& p, cudaStream_t st) {
   const M3WGrid g = m3w_grid(p);
   mxb_status s = prepare<IO>(p, g, st);
   if (s != MXB_OK) return s;
-  M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_local<IO, PRV, LPCV, true, false>(p, g, st)));
+  M3W_DISPATCH(g.shape.lanes, p, (s = launch_local<IO, PRV, LPCV, PL, true, false>(p, g, st)));
   if (s != MXB_OK) return s;
   linear_scan(p, 0, 1, st);
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
-    M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_out_kernel", st, (launch_kernel(m3w_out_kernel<IO, PRV, LPCV>, grid, g.threads, kRowBytes<IO, PRV, LPCV>, st, q))));
+    M3W_DISPATCH(g.shape.lanes, p, MXB_LAUNCH("m3w_out_kernel", st, (launch_kernel(m3w_out_kernel<IO, PRV, LPCV, PL>, grid, g.threads, kRowBytes<PRV, LPCV>, st, q))));
   });
   return check_launch("mamba3 window-parallel forward");
 }
@@ -883,22 +938,22 @@ static mxb_status backward(const M3P& p, bool have_states, cudaStream_t st) {
   const M3WGrid g = m3w_grid(p);
   mxb_status s = MXB_OK;
   if (have_states) {
-    M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_local<IO, PRV, LPCV, false, true>(p, g, st)));
+    M3W_DISPATCH(g.shape.lanes, p, (s = launch_local<IO, PRV, LPCV, PL, false, true>(p, g, st)));
   } else {
     s = prepare<IO>(p, g, st);
-    if (s == MXB_OK) M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_local<IO, PRV, LPCV, true, true>(p, g, st)));
+    if (s == MXB_OK) M3W_DISPATCH(g.shape.lanes, p, (s = launch_local<IO, PRV, LPCV, PL, true, true>(p, g, st)));
   }
   if (s != MXB_OK) return s;
   const int first = have_states ? 1 : 0;
   linear_scan(p, first, 2 - first, st);
-  M3W_DISPATCH(g.shape.lanes, p.Kp, (s = launch_grad<IO, PRV, LPCV>(p, g, st)));
+  M3W_DISPATCH(g.shape.lanes, p, (s = launch_grad<IO, PRV, LPCV, PL>(p, g, st)));
   if (s != MXB_OK) return s;
   by_segment(p, [&](auto per) {
     MXB_LAUNCH("m3w_angle_scan_kernel", st,
                (launch_kernel(m3w_angle_scan_kernel<decltype(per)::value>, chain_grid(p, p.D * p.Kp, 1), kScanThreads, 0, st, p)));
   });
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
-    M3W_DISPATCH(g.shape.lanes, p.Kp, MXB_LAUNCH("m3w_fix_kernel", st, (launch_kernel(m3w_fix_kernel<IO, PRV, LPCV>, grid, g.threads, 0, st, q))));
+    M3W_DISPATCH(g.shape.lanes, p, MXB_LAUNCH("m3w_fix_kernel", st, (launch_kernel(m3w_fix_kernel<IO, PRV, LPCV, PL>, grid, g.threads, 0, st, q))));
   });
   return check_launch("mamba3 window-parallel backward");
 }
