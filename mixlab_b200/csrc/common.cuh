@@ -81,28 +81,51 @@ __device__ __forceinline__ void warp_rcumsum64(F& a, F& b, int lane) {
   b = v;
 }
 
-// Sum over `rows` rows of one column (part: its first element) in a fixed order, by a CTA of kSumThreads that owns 16 columns: 64
-// slices of threads take every 64th row (eight loads in flight each), the slices are added pairwise across a warp and then by a
-// warp per column; warp w < 16 gets the sum of column w.  Latency of the loads is all there is:
-// 1184 rows of 448 columns 17.7 us with 8 slices and 32 columns a CTA, 3.8 now.
-constexpr int kSumCols = 16, kSumSlices = 64, kSumThreads = kSumCols * kSumSlices;
-__device__ __forceinline__ float col_sum(const float* __restrict__ part, size_t rows, size_t pitch, bool in) {
-  __shared__ float red[kSumSlices / 2][kSumCols + 1];
-  const int col = threadIdx.x % kSumCols, slice = threadIdx.x / kSumCols, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// Sums over `rows` rows of 16 (TALL) or 32 columns in a fixed order; part: the calling thread's column, put(c, sum) is called once
+// for each column c of the CTA.  TALL: 1024 threads, 64 slices of them take every 64th row, the slices are added pairwise across a
+// warp and then by a warp per column; otherwise 256 threads and 8 slices.  Eight loads in flight a thread.  Few columns want the
+// first (1184 rows of 448 columns 17.7 us with 8 slices, 3.8 with 64: it is the latency of the loads), columns enough to fill the
+// GPU the second (256 rows of 12,320 columns 6.0 with 8, 12.3 with 64): col_sum_tall().
+template <bool TALL>
+constexpr int kSumCols = TALL ? 16 : 32;
+template <bool TALL>
+constexpr int kSumThreads = TALL ? 1024 : 256;
+inline bool col_sum_tall(size_t columns) { return columns <= 16 * 2 * 148; }
+template <bool TALL, typename F>
+__device__ __forceinline__ void col_sum(const float* __restrict__ part, size_t rows, size_t pitch, bool in, F&& put) {
+  constexpr int COLS = kSumCols<TALL>, SLICES = kSumThreads<TALL> / COLS;
+  __shared__ float red[32][COLS + 1];
+  const int col = threadIdx.x % COLS, slice = threadIdx.x / COLS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float s = 0.f;
   if (in) {
-    for (size_t r0 = slice; r0 < rows; r0 += 8 * kSumSlices) {
+    const float* src = part + slice * pitch;
+    const size_t step = SLICES * pitch;
+    int left = ((int)rows - slice + SLICES - 1) / SLICES;
+    for (; left >= 8; left -= 8, src += 8 * step) {
       float v[8];
 #pragma unroll
-      for (int x = 0; x < 8; ++x) v[x] = r0 + x * kSumSlices < rows ? __ldg(part + (r0 + x * kSumSlices) * pitch) : 0.f;
+      for (int x = 0; x < 8; ++x) v[x] = __ldg(src + x * step);
 #pragma unroll
       for (int x = 0; x < 8; ++x) s += v[x];
     }
+    float v[7];
+#pragma unroll
+    for (int x = 0; x < 7; ++x) v[x] = x < left ? __ldg(src + x * step) : 0.f;
+#pragma unroll
+    for (int x = 0; x < 7; ++x) s += v[x];
   }
-  s += __shfl_xor_sync(0xffffffffu, s, kSumCols);
-  if (lane < kSumCols) red[warp][col] = s;
+  if (TALL) s += __shfl_xor_sync(0xffffffffu, s, COLS & 31);  // two slices a warp
+  if (lane < COLS) red[warp][col] = s;
   __syncthreads();
-  return warp_sum(warp < kSumCols ? red[lane][warp] : 0.f);  // warps 0 .. 15: the sum of column `warp`
+  if constexpr (TALL) {
+    const float t = warp_sum(warp < COLS ? red[lane][warp] : 0.f);
+    if (lane == 0 && warp < COLS) put(warp, t);
+  } else if (warp == 0) {
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < SLICES; ++k) t += red[k][lane];
+    put(lane, t);
+  }
 }
 
 // First statement of a kernel that launch_kernel() starts: nothing is read or written before the kernels in front of it in the

@@ -450,13 +450,16 @@ struct ColSums {
   float* out[5];
   int rows[5], n[5], first[6], count;
 };
-__global__ void __launch_bounds__(kSumThreads) gdn_block_colsum_kernel(ColSums c) {
+template <bool TALL>
+__global__ void __launch_bounds__(kSumThreads<TALL>) gdn_block_colsum_kernel(ColSums c) {
   begin_dependent();
   int g = 0;
   while (g + 1 < c.count && (int)blockIdx.x >= c.first[g + 1]) ++g;
-  const int n = c.n[g], j0 = (blockIdx.x - c.first[g]) * kSumCols, mine = j0 + threadIdx.x % kSumCols, j = j0 + (threadIdx.x >> 5);
-  const float t = col_sum(c.part[g] + mine, c.rows[g], n, mine < n);
-  if (threadIdx.x < 32 * kSumCols && (threadIdx.x & 31) == 0 && j < n) c.out[g][j] = t;
+  const int n = c.n[g], j0 = (blockIdx.x - c.first[g]) * kSumCols<TALL>, mine = j0 + threadIdx.x % kSumCols<TALL>;
+  float* out = c.out[g];
+  col_sum<TALL>(c.part[g] + mine, c.rows[g], n, mine < n, [&](int x, float t) {
+    if (j0 + x < n) out[j0 + x] = t;
+  });
 }
 
 // gate / beta backward: one CTA per head walks all (b, t); the two per-head sums (A_log, dt_bias) in a fixed order
@@ -753,6 +756,20 @@ mxb_status gdn_block_pre_fwd(const mxb_gdn_desc* d, const void* qp, const void* 
              : blk_pre_fwd<blk::bf16>(d, qp, kp, vp, cq, ck, cv, a_raw, b_raw, a_log, dt_bias, q, k, v, beta, gate, st);
 }
 
+static void blk_colsum(blk::ColSums& c, cudaStream_t st) {
+  size_t columns = 0;
+  for (int i = 0; i < c.count; ++i) columns += c.n[i];
+  auto launch = [&](auto tall) {
+    constexpr bool TALL = decltype(tall)::value;
+    for (int i = 0; i < c.count; ++i) c.first[i + 1] = c.first[i] + (c.n[i] + kSumCols<TALL> - 1) / kSumCols<TALL>;
+    MXB_LAUNCH("gdn_block_colsum_kernel", st,
+               (launch_kernel(blk::gdn_block_colsum_kernel<TALL>, c.first[c.count], kSumThreads<TALL>, 0, st, c)));
+  };
+  if (col_sum_tall(columns)) launch(std::true_type{});
+  else launch(std::false_type{});
+}
+
+
 template <typename IO>
 static mxb_status blk_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void* kp, const void* vp, const float* cq,
                               const float* ck, const float* cv, const float* a_raw, const float* b_raw,
@@ -786,7 +803,6 @@ static mxb_status blk_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void*
   blk::ColSums c{};
   auto sum = [&](const float* part, int nrows, int n, float* out) {
     c.part[c.count] = part; c.out[c.count] = out; c.rows[c.count] = nrows; c.n[c.count] = n;
-    c.first[c.count + 1] = c.first[c.count] + (n + kSumCols - 1) / kSumCols;
     ++c.count;
   };
   sum(a.dwp[0], (int)rows, (int)(4 * Ck), dcq);
@@ -805,7 +821,7 @@ static mxb_status blk_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void*
                (launch_kernel(blk::gdn_block_gate_bwd_kernel, d->H, 256, 0, st, p, a_raw, b_raw, a_log, dt_bias, dbeta, dgate,
                                                                       da_raw, db_raw, da_log, ddt_bias)));
   }
-  MXB_LAUNCH("gdn_block_colsum_kernel", st, (launch_kernel(blk::gdn_block_colsum_kernel, c.first[c.count], kSumThreads, 0, st, c)));
+  blk_colsum(c, st);
   return check_launch("gdn_block_pre_bwd");
 }
 mxb_status gdn_block_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void* kp, const void* vp, const float* cq,
@@ -845,8 +861,8 @@ static mxb_status blk_post(const mxb_gdn_desc* d, const void* o, const void* z, 
                      static_cast<IO*>(d_o), static_cast<IO*>(dz), part)));
   });
   blk::ColSums c{};
-  c.part[0] = part; c.out[0] = dwn; c.rows[0] = ctas; c.n[0] = d->Dv; c.count = 1; c.first[1] = (d->Dv + kSumCols - 1) / kSumCols;
-  MXB_LAUNCH("gdn_block_colsum_kernel", st, (launch_kernel(blk::gdn_block_colsum_kernel, c.first[1], kSumThreads, 0, st, c)));
+  c.part[0] = part; c.out[0] = dwn; c.rows[0] = ctas; c.n[0] = d->Dv; c.count = 1;
+  blk_colsum(c, st);
   return check_launch("gdn_block_post_bwd");
 }
 mxb_status gdn_block_post(const mxb_gdn_desc* d, const void* o, const void* z, const float* wn, void* y, const void* dy,

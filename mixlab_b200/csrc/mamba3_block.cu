@@ -162,17 +162,17 @@ __global__ void __launch_bounds__(128) m3b_conv_bwd_kernel(BlkP p, const IO* __r
   for (int k = 0; k < kMaxK; ++k) store_n<float, C>(dst + (size_t)k * p.D, dw[k]);
 }
 // Column sums of partial rows.  K > 0: columns are [k][d] and the result is stored as [d][K] (k < K only).
-__global__ void __launch_bounds__(kSumThreads) m3b_colsum_kernel(const float* __restrict__ part, int rows, int n,
-                                                                           float* __restrict__ out, int D, int K) {
+template <bool TALL>
+__global__ void __launch_bounds__(kSumThreads<TALL>) m3b_colsum_kernel(const float* __restrict__ part, int rows, int n,
+                                                                       float* __restrict__ out, int D, int K) {
   begin_dependent();
-  const int j0 = blockIdx.x * kSumCols, mine = j0 + threadIdx.x % kSumCols;
-  const float t = col_sum(part + mine, rows, n, mine < n);
-  const int j = j0 + (threadIdx.x >> 5);
-  if (threadIdx.x < 32 * kSumCols && (threadIdx.x & 31) == 0 && j < n) {
-    const int k = j / D, d = j % D;
+  const int j0 = blockIdx.x * kSumCols<TALL>, mine = j0 + threadIdx.x % kSumCols<TALL>;
+  col_sum<TALL>(part + mine, rows, n, mine < n, [&](int c, float t) {
+    const int j = j0 + c, k = j / D, d = j % D;
+    if (j >= n) return;
     if (K == 0) out[j] = t;
     else if (k < K) out[(size_t)d * K + k] = t;
-  }
+  });
 }
 
 // sum over the LN lanes of a group; the mask names only the caller's group (the lane groups of a warp may run different numbers
@@ -272,16 +272,16 @@ __global__ void __launch_bounds__(128) m3b_bc_bwd_kernel(BlkP p, BcArgs<IO> a) {
 // The sums of the partial rows of b and c in one launch.  grid (ceil(N/16), G + 1, 2): dbias of group y, or (y == G) dscale,
 // which is the sum over the groups too.
 template <typename IO>
-__global__ void __launch_bounds__(kSumThreads) m3b_bc_sum_kernel(BlkP p, BcArgs<IO> a, int ctas) {
+__global__ void __launch_bounds__(kSumThreads<true>) m3b_bc_sum_kernel(BlkP p, BcArgs<IO> a, int ctas) {
   begin_dependent();
-  const int which = blockIdx.z, g = blockIdx.y, c0 = blockIdx.x * kSumCols, mine = c0 + threadIdx.x % kSumCols;
+  const int which = blockIdx.z, g = blockIdx.y, c0 = blockIdx.x * kSumCols<true>, mine = c0 + threadIdx.x % kSumCols<true>;
   const bool scale = g == p.G;
   const size_t row = 2 * (size_t)p.N;
   const float* part = a.part[which] + (scale ? 0 : g * row + p.N) + mine;
-  const float t = col_sum(part, scale ? (size_t)ctas * p.G : ctas, scale ? row : p.G * row, mine < p.N);
-  const int c = c0 + (threadIdx.x >> 5);
-  if (threadIdx.x < 32 * kSumCols && (threadIdx.x & 31) == 0 && c < p.N)
-    (scale ? a.dscale[which] : a.dbias[which] + g * p.N)[c] = t;
+  float* out = scale ? a.dscale[which] : a.dbias[which] + g * p.N;
+  col_sum<true>(part, scale ? (size_t)ctas * p.G : ctas, scale ? row : p.G * row, mine < p.N, [&](int c, float t) {
+    if (c0 + c < p.N) out[c0 + c] = t;
+  });
 }
 
 // ------------------------------------------------------------------ post: RMSNorm over D x SiLU gate
@@ -518,6 +518,16 @@ size_t mamba3_block_workspace_bytes(const mxb_mamba3_desc* d) {
   return m + 256;
 }
 
+static void m3b_colsum(const float* part, int rows, int n, float* out, int D, int K, cudaStream_t st) {
+  auto launch = [&](auto tall) {
+    constexpr bool TALL = decltype(tall)::value;
+    MXB_LAUNCH("m3b_colsum_kernel", st,
+               (launch_kernel(m3b::m3b_colsum_kernel<TALL>, (n + kSumCols<TALL> - 1) / kSumCols<TALL>, kSumThreads<TALL>, 0, st, part, rows, n, out, D, K)));
+  };
+  if (col_sum_tall(n)) launch(std::true_type{});
+  else launch(std::false_type{});
+}
+
 template <typename IO>
 static mxb_status m3b_conv(const mxb_mamba3_desc* d, int K, const void* x, const float* w, void* y, const void* dy,
                            void* dx, float* dw, void* ws, cudaStream_t st) {
@@ -533,7 +543,7 @@ static mxb_status m3b_conv(const mxb_mamba3_desc* d, int K, const void* x, const
              (launch_kernel(m3b::m3b_conv_bwd_kernel<IO>, grid, 128, 0, st, p, static_cast<const IO*>(x), w, static_cast<const IO*>(dy),
                                                                  static_cast<IO*>(dx), part)));
   const int rows = d->B * m3b_runs(d), n = m3b::kMaxK * d->D;
-  MXB_LAUNCH("m3b_colsum_kernel", st, (launch_kernel(m3b::m3b_colsum_kernel, (n + kSumCols - 1) / kSumCols, kSumThreads, 0, st, part, rows, n, dw, d->D, K)));
+  m3b_colsum(part, rows, n, dw, d->D, K, st);
   return check_launch("m3b_conv_bwd");
 }
 mxb_status mamba3_block_conv(const mxb_mamba3_desc* d, int K, const void* x, const float* w, void* y, const void* dy,
@@ -578,8 +588,8 @@ static mxb_status m3b_bc(const mxb_mamba3_desc* d, float eps, const void* bp, co
     MXB_LAUNCH("m3b_bc_bwd_kernel", st, (launch_kernel(m3b::m3b_bc_bwd_kernel<IO, decltype(ln)::value>, grid, 128, 0, st, p, a)));
   });
   MXB_LAUNCH("m3b_bc_sum_kernel", st,
-             (launch_kernel(m3b::m3b_bc_sum_kernel<IO>, dim3((d->N + kSumCols - 1) / kSumCols, d->G + 1, 2),
-                            kSumThreads, 0, st, p, a, ctas)));
+             (launch_kernel(m3b::m3b_bc_sum_kernel<IO>, dim3((d->N + kSumCols<true> - 1) / kSumCols<true>, d->G + 1, 2),
+                            kSumThreads<true>, 0, st, p, a, ctas)));
   return check_launch("m3b_bc_bwd");
 }
 mxb_status mamba3_block_bc(const mxb_mamba3_desc* d, float eps, const void* bp, const void* cp, const float* bs,
@@ -608,9 +618,7 @@ static mxb_status m3b_post(const mxb_mamba3_desc* d, float eps, const void* y, c
   MXB_LAUNCH("m3b_post_bwd_kernel", st,
              (launch_kernel(narrow ? m3b::m3b_post_bwd_warp_kernel<IO> : m3b::m3b_post_bwd_kernel<IO>, ctas, 256, 0, st, p, yv, zv, wn,
                             static_cast<const IO*>(dout), static_cast<IO*>(dy), static_cast<IO*>(dz), part)));
-  MXB_LAUNCH("m3b_colsum_kernel", st,
-             (launch_kernel(m3b::m3b_colsum_kernel, (d->D + kSumCols - 1) / kSumCols, kSumThreads, 0, st, part,
-                            ctas, d->D, dwn, d->D, 0)));
+  m3b_colsum(part, ctas, d->D, dwn, d->D, 0, st);
   return check_launch("m3b_post_bwd");
 }
 mxb_status mamba3_block_post(const mxb_mamba3_desc* d, float eps, const void* y, const void* z, const float* wn, void* out,
