@@ -277,8 +277,9 @@ __global__ void __launch_bounds__(256) gdn_block_gate_fwd_kernel(BlockP p, const
 // Same map as the forward.  A run recomputes the convolution of its steps and of the three steps after it (their ds
 // feeds dx of the run) and emits dx three steps behind.  Bound: HBM (nine tensors) and, close behind, issue: about
 // 17 instructions per element with packed arithmetic (40 and half of the lanes idle at 64 channels before: 760 us for
-// 16 x 2048 x 16 heads of 64 bf16 channels, 189 now).  Two CTAs per SM leave a thread 128 registers, which its weights,
-// weight gradients, seven inputs and seven ds of four channels exceed: the compiler spills about 180 bytes of them.
+// 16 x 2048 x 16 heads of 64 bf16 channels, 182 now).  Two CTAs per SM leave a thread 128 registers for its weights, weight
+// gradients, seven inputs and seven ds of four channels, so little else may live across the row sums: two products with the
+// derivative of SiLU instead of SiLU, derivative and dy (180 bytes spilled: 198 us; 24 now).
 template <typename IO, int LPR>
 __global__ void __launch_bounds__(256, 2) gdn_block_pre_bwd_kernel(BlockP p, PreArgs<IO> a, int run, int first, int z0) {
   begin_dependent();
@@ -359,7 +360,7 @@ __global__ void __launch_bounds__(256, 2) gdn_block_pre_bwd_kernel(BlockP p, Pre
     }
     issue(k + ring.kStages - 1);
     // one sigmoid per element gives SiLU and its derivative; rows past T have zero dy, hence zero ds
-    f2 sv[4][2], dsl[4][2];
+    f2 sv[4][2];  // SiLU times its derivative (g: the same of dy): what a row sum away becomes ds
     float ss[4], dot[4];
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
@@ -371,10 +372,11 @@ __global__ void __launch_bounds__(256, 2) gdn_block_pre_bwd_kernel(BlockP p, Pre
         fma2(acc, w[2][c], xx[s + 1][c]);
         fma2(acc, w[3][c], xx[s][c]);
         const f2 sg = sigmoid_pair<IO>(acc);
-        sv[s][c] = mul2(acc, sg);
-        dsl[s][c] = mad2(sv[s][c], mad2(sg, dup2(-1.f), dup2(1.f)), sg);  // sg (1 + acc (1 - sg))
-        fma2(sq, sv[s][c], sv[s][c]);
-        fma2(sg_dot, sv[s][c], g[s][c]);
+        const f2 si = mul2(acc, sg), dsl = mad2(si, mad2(sg, dup2(-1.f), dup2(1.f)), sg);  // dsl = sg (1 + acc (1 - sg))
+        fma2(sq, si, si);
+        fma2(sg_dot, si, g[s][c]);
+        sv[s][c] = mul2(si, dsl);
+        g[s][c] = mul2(g[s][c], dsl);
       }
       ss[s] = sum2(sq);
       dot[s] = sum2(sg_dot);
@@ -386,13 +388,14 @@ __global__ void __launch_bounds__(256, 2) gdn_block_pre_bwd_kernel(BlockP p, Pre
       for (int s = 0; s < 4; ++s) {
         const f2 f0 = dup2(of_step(fa, s)), f1 = dup2(of_step(fb, s));
 #pragma unroll
-        for (int c = 0; c < 2; ++c) g[s][c] = mad2(f1, sv[s][c], mul2(f0, g[s][c]));
+        for (int c = 0; c < 2; ++c) dd[3 + s][c] = mad2(f1, sv[s][c], mul2(f0, g[s][c]));
       }
+    } else {
+#pragma unroll
+      for (int s = 0; s < 4; ++s)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) dd[3 + s][c] = g[s][c];
     }
-#pragma unroll
-    for (int s = 0; s < 4; ++s)
-#pragma unroll
-      for (int c = 0; c < 2; ++c) dd[3 + s][c] = mul2(g[s][c], dsl[s][c]);
     if (!halo) {
 #pragma unroll
       for (int s = 0; s < 4; ++s)
