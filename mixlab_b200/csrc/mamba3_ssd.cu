@@ -19,6 +19,7 @@
 //   m3s_state_pass_kernel   per (b, head), sequential over the chunks, forward or reverse: the chunk contribution
 //                           Brot^T diag(r e) X (or Crot^T diag(exp(Lam)) dY) folded into the running state
 //   m3s_chunk_out_kernel    per chunk: Y
+//   m3s_scan_out_kernel     the forward state pass and Y in one kernel, where the (batch, head) pairs fill the GPU
 //   m3s_chunk_grad_kernel   per chunk and up to 16 heads of a group: dx, dB, dC summed over these heads, per-token scalars
 //   m3s_tail_kernel         per chunk: ddt, dlambda, dtheta, da_log shares; dB, dC summed over the CTAs of a group
 #include <cuda.h>
@@ -80,6 +81,13 @@ __device__ __forceinline__ void ld_acc16(uint32_t taddr, int warp, int c0, float
   for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(r[i]);
 }
 
+// 8 columns of a result as four pairs.
+__device__ __forceinline__ void ld_pairs(uint32_t taddr, int warp, f2 (&f)[4]) {
+  uint32_t r[8];
+  tc::tmem_ld_32x32b_x8(taddr + ((uint32_t)(32 * (warp & 3)) << 16), r);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+}
 __device__ __forceinline__ float ex2(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -248,36 +256,70 @@ template <bool SW>
 __device__ __forceinline__ tc::Tile in_mnmajor(const void* ptr, int W) {
   return SW ? tc::mnmajor_sw128_tile(ptr, 8192) : tc::mnmajor_tile(ptr, W);
 }
+// A thread keeps to one row (rows of eight lanes start in eight different banks through the swizzle), so a row's sine and cosine
+// are read once; two pairs of states share a packed register, even and odd states apart.  nt threads, a multiple of 64.
 template <bool SW>
 __device__ __forceinline__ void rotate_in_tile(uint8_t* tile, const float* sn, const float* cs, int tid, int nt) {
   if constexpr (!SW) {
     rotate_tile(tile, sn, cs);
   } else {
-    // four units per pass, all loads before the first store (a store in between would pin the order of the
-    // loads that follow it); unit w of a slab belongs to row w / 8
-    for (int w0 = tid; w0 < Q * 16; w0 += 4 * nt) {
+    const int t = tid & 63, per = 1024 / nt, c0 = (tid >> 6) * per;
+    const f2 c2 = dup2(cs[t]), s2 = dup2(sn[t]), n2 = dup2(-sn[t]);
+    auto rot = [&](uint32_t& a, uint32_t& b) {
+      const f2 e = pack2(__uint_as_float(a << 16), __uint_as_float(b << 16));
+      const f2 o = pack2(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u));
+      const float2 x = unpack2(mad2(c2, e, mul2(s2, o))), y = unpack2(mad2(c2, o, mul2(n2, e)));
+      a = tc::pack_bf16(x.x, y.x);
+      b = tc::pack_bf16(x.y, y.y);
+    };
+#pragma unroll
+    for (int q0 = 0; q0 < per; q0 += 4) {  // four units, all loads before the first store
       uint4 raw[4];
-      float sv[4], cv[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) raw[q] = *reinterpret_cast<const uint4*>(tile + tc::sw128_unit(t, c0 + q0 + q));
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int w = min(w0 + q * nt, Q * 16 - 1), t = (w >> 3) & 63;
-        raw[q] = *reinterpret_cast<const uint4*>(tile + 16 * w);
-        sv[q] = sn[t]; cv[q] = cs[t];
+        rot(raw[q].x, raw[q].y);
+        rot(raw[q].z, raw[q].w);
+        *reinterpret_cast<uint4*>(tile + tc::sw128_unit(t, c0 + q0 + q)) = raw[q];
       }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        auto rot = [&](uint32_t w) {
-          const float2 v = unpack2(widen2(w));
-          return tc::pack_bf16(fmaf(cv[q], v.x, sv[q] * v.y), fmaf(cv[q], v.y, -(sv[q] * v.x)));
-        };
-        raw[q] = make_uint4(rot(raw[q].x), rot(raw[q].y), rot(raw[q].z), rot(raw[q].w));
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (w0 + q * nt < Q * 16) *reinterpret_cast<uint4*>(tile + 16 * (w0 + q * nt)) = raw[q];
     }
   }
 }
+// Rows of a [64][64] tile (swizzled) times a factor each, bf16 again; src and dst may be the same.
+__device__ __forceinline__ void scale_rows(uint8_t* dst, const uint8_t* src, const float* factor, int tid, int nt) {
+  const int t = tid & 63, per = 512 / nt, c0 = (tid >> 6) * per;
+  const f2 f = dup2(factor[t]);
+#pragma unroll
+  for (int q = 0; q < per; ++q) {
+    const uint32_t at = tc::sw128_unit(t, c0 + q);
+    const uint4 x = *reinterpret_cast<const uint4*>(src + at);
+    *reinterpret_cast<uint4*>(dst + at) = make_uint4(narrow2(mul2(widen2(x.x), f)), narrow2(mul2(widen2(x.y), f)),
+                                                     narrow2(mul2(widen2(x.z), f)), narrow2(mul2(widen2(x.w), f)));
+  }
+}
+// G*M of row t and the 32 columns from n0 on: M_ts = exp(Lam_t - Lam_s) e_s below the diagonal, gam_t on it.
+__device__ __forceinline__ void mask_row(float (&g)[32], const ChunkScal& s, int t, int n0) {
+  const float gt = s.gam[t];
+  const f2 lt = dup2(s.Lam[t]), minus = dup2(-1.f), log2e = dup2(1.4426950408889634f);
+  const int k = t - n0;
+#pragma unroll
+  for (int x = 0; x < 8; ++x) {  // branch-free, so the exponentials of different columns overlap
+    const ulonglong2 l4 = *reinterpret_cast<const ulonglong2*>(s.Lam + n0 + 4 * x);
+    const float4 e4 = *reinterpret_cast<const float4*>(s.e + n0 + 4 * x);
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      const int q = 4 * x + 2 * y;
+      const float2 d = unpack2(mad2(y ? l4.y : l4.x, minus, lt));
+      const float2 a = unpack2(mul2(pack2(fminf(d.x, 0.f), fminf(d.y, 0.f)), log2e));
+      const f2 w = pack2(q < k ? (y ? e4.z : e4.x) : gt, q + 1 < k ? (y ? e4.w : e4.y) : gt);
+      const float2 r = unpack2(mul2(pack2(g[q], g[q + 1]), mul2(pack2(ex2(a.x), ex2(a.y)), w)));
+      g[q] = q <= k ? r.x : 0.f;
+      g[q + 1] = q + 1 <= k ? r.y : 0.f;
+    }
+  }
+}
+
 struct ChunkMaps {
   CUtensorMap b, c;   // [B,T,G,128] viewed as (N, G, T, B), boxes of 64 columns x 64 steps, 128-byte swizzle
   CUtensorMap x, dy, dx;  // [B,T,heads,64] viewed as (P, heads, T, B)
@@ -371,10 +413,8 @@ __global__ void __launch_bounds__(kScalHeads * kPrefixSegs) m3s_angle_prefix_ker
 // Only the update of the state is sequential, so everything before it runs ahead: a warp issues the copies, four warps rotate
 // and scale landed tiles in place, a warp issues the products into two accumulators by turns, eight warps hold the state,
 // fold in an accumulator and store the state (one sequence of 32 heads x 64 chunks: 57 us a pass, chunk by chunk in one group
-// of warps 84; 8 sequences 104, where it is the arithmetic of the rotation that counts, 107).  Every hand-over is an mbarrier with a bounded wait; a warp whose wait has run out stops waiting and working but goes through its loop.
+// of warps 84; 8 sequences 101, where it is the arithmetic of the rotation that counts, 107 before a thread kept to a row).  Every hand-over is an mbarrier with a bounded wait; a warp whose wait has run out stops waiting and working but goes through its loop.
 // NS stages in flight: three and four warps that prepare tiles where two CTAs share an SM, six and eight where one has it.
-// With three, 448 threads and 72 registers, 20 bytes are spilled and 28 read back; reading the accumulator in halves avoids that
-// and takes longer (8 sequences 105 us a pass, 108 without spills).
 template <int NS>
 constexpr int kPassPrep = NS == 3 ? 4 : 8;
 template <int NS>
@@ -479,33 +519,32 @@ __global__ void __launch_bounds__(kPassThreads<NS>, NS == 3 ? 2 : 1) m3s_state_p
       wait(full + st, it / NS);
       const ChunkScal& s = scal[it % NC];
       rotate_in_tile<true>(Rt + st * 16384, s.sn, s.cs, u0, 32 * kPassPrep<NS>);
-      const float* rowscale = mode == 0 ? s.re : s.dexp;
-      for (int u = u0; u < Q * 8; u += 32 * kPassPrep<NS>) {  // unit u lies in row u / 8
-        uint4* unit = reinterpret_cast<uint4*>(Xt + st * 8192 + 16 * u);
-        *unit = tc::scale_bf16x8(*unit, rowscale[u >> 3]);
-      }
+      scale_rows(Xt + st * 8192, Xt + st * 8192, mode == 0 ? s.re : s.dexp, u0, 32 * kPassPrep<NS>);
       tc::fence_async_smem();
       arrive(ready + st);
     }
   } else if (warp < 8) {    // ---- the state: thread = state row and 32 of its 64 columns
     const int nrow = tid & 127, half = tid >> 7;
-    float H[32];
+    f2 H[16];
 #pragma unroll
-    for (int x = 0; x < 32; ++x) H[x] = 0.f;
+    for (int x = 0; x < 16; ++x) H[x] = 0ull;
     uint4* out = reinterpret_cast<uint4*>((mode == 0 ? p.H0 : p.dH1) + cbase * (N * P)) + (tc::kmajor_unit(nrow, 4 * half, P) >> 4);
     for (int it = 0; it < n; ++it) {
       const int a = it & 1;
 #pragma unroll
-      for (int x = 0; x < 4; ++x) out[(size_t)chunk_at(it) * (N * P / 8) + 8 * x] = pack8(&H[8 * x]);
+      for (int x = 0; x < 4; ++x) out[(size_t)chunk_at(it) * (N * P / 8) + 8 * x] =
+          make_uint4(narrow2(H[4 * x]), narrow2(H[4 * x + 1]), narrow2(H[4 * x + 2]), narrow2(H[4 * x + 3]));
       wait(accfull + a, it >> 1);
       tc::fence_after_sync();
       ok = __all_sync(0xffffffffu, ok);
-      const float L = scal[it % NC].L;
+      const f2 L = dup2(scal[it % NC].L);
       if (ok) {
-        float f[32];
-        ld_acc32(taddr + 64 * a, warp, 32 * half, f);
+        f2 f[16];
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) H[jj] = fmaf(L, H[jj], f[jj]);
+        for (int q = 0; q < 4; ++q) ld_pairs(taddr + 64 * a + 32 * half + 8 * q, warp, *reinterpret_cast<f2(*)[4]>(f + 4 * q));
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int x = 0; x < 16; ++x) H[x] = mad2(L, H[x], f[x]);
       }
       tc::fence_before_sync();
       arrive(accfree + a);
@@ -598,21 +637,9 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
   // weight-stationary products: this thread's row, and the half of the columns it holds of every result
   const int t = 32 * (warp & 1) + lane, n0 = 32 * (warp >> 1);
   if (ok) {
-    const float lt = s.Lam[t], gt = s.gam[t];
     float f[32];
     ld_acc32(taddr, warp, 0, f);
-#pragma unroll
-    for (int x = 0; x < 8; ++x) {  // branch-free, so the exponentials of different columns overlap
-      const float4 l4 = *reinterpret_cast<const float4*>(s.Lam + n0 + 4 * x);
-      const float4 e4 = *reinterpret_cast<const float4*>(s.e + n0 + 4 * x);
-      const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, es[4] = {e4.x, e4.y, e4.z, e4.w};
-#pragma unroll
-      for (int y = 0; y < 4; ++y) {
-        const int jj = 4 * x + y, sx = n0 + jj;
-        const float mv = __expf(fminf(lt - ls[y], 0.f)) * (sx < t ? es[y] : gt);
-        f[jj] = (sx <= t) ? f[jj] * mv : 0.f;
-      }
-    }
+    mask_row(f, s, t, n0);
 #pragma unroll
     for (int x = 0; x < 4; ++x) sts16(Gm, tc::kmajor_unit(t, (n0 >> 3) + x, Q), pack8(&f[8 * x]));
   }
@@ -654,6 +681,259 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
   if (warp == 0) tc::tmem_dealloc(taddr, 64);
 }
 
+// ------------------------------------------------------------ states and output in one pass
+// The forward state pass with the chunk output behind it: one CTA per (batch, head) walks the chunks, and what the output of a
+// chunk needs (the rotated rows of B, x and the state in front of the chunk) is on the SM already, so B and x are read and B is
+// rotated once and the state is not read back.  The same products, roundings and order of sums as m3s_state_pass_kernel and
+// m3s_chunk_out_kernel: the same bits.
+//
+// 512 threads and 110 KB, two CTAs per SM.  Warps 0-3 hold the state (thread = row, 64 columns) and write its image, which the
+// product with Crot reads and, for a backward, a bulk store keeps; warps 4-7 mask G and put y together; warps 8-11 rotate B and
+// C and scale x; the last four issue copies, state products, output products and stores.  Hand-overs are mbarriers with bounded
+// waits.  A wait cannot miss its phase: a stage is loaded again only when y and the scalars of its chunk are through, so what
+// is counted per stage stays within two chunks, and of every other barrier the next phase needs its waiters to have passed.
+// G*M takes the place of Brot, y that of x.
+// TMEM: the state's contribution [0, 64) and [64, 128) by turns, G [128, 160), Crot H0 [160, 192), (G*M) X [192, 224).
+// Bound by instruction issue (50 % of the slots; rotation, masks and the state's update), with 69 + 16 KB a chunk through shared
+// memory beside it: 8 x 4096 x 32 heads 222 us where the two kernels take 102 + 184 (without keeping the states 200).
+constexpr int kScanThreads = 512;
+constexpr int kScanStage = 2 * 16384 + 8192;
+constexpr int kScanSmem = 2 * kScanStage + 8192 + 16384 + 2 * (int)sizeof(ChunkScal) + 21 * 8 + 16 + 1024;
+static_assert(2 * (kScanSmem + 1024) <= 228 * 1024, "two CTAs per SM");
+
+struct ScanMaps {
+  CUtensorMap b, c;  // as in ChunkMaps
+  CUtensorMap x, y;
+};
+
+__global__ void __launch_bounds__(kScanThreads, 2) m3s_scan_out_kernel(SsdP p, int save, const __grid_constant__ ScanMaps maps) {
+  begin_dependent();
+  extern __shared__ uint8_t raw[];
+  uint8_t* sm = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
+  uint8_t* Xs = sm + 2 * kScanStage;   // [64][64] r e x (swizzled like x); a stage: B, C, x
+  uint8_t* Ht = Xs + 8192;             // [128][64] state in front of the chunk, operand image
+  ChunkScal* scal = reinterpret_cast<ChunkScal*>(Ht + 16384);  // x2
+  uint64_t* full = reinterpret_cast<uint64_t*>(scal + 2);      // x2: a chunk's operands landed
+  uint64_t* sfree = full + 2;          // x2: y has left, the scalars are read
+  uint64_t* accfull = sfree + 2;       // x2: product of the state (Brot and r e x are no longer needed)
+  uint64_t* accfree = accfull + 2;     // x2: accumulator read
+  uint64_t* readyb = accfree + 2;      // x2: Brot and r e x written
+  uint64_t* readyc = readyb + 2;       // x2: Crot written
+  uint64_t* yready = readyc + 2;       // x2: y written
+  uint64_t* xsfree = yready + 2;       // r e x read
+  uint64_t* hready = xsfree + 1;       // image of the state written
+  uint64_t* hfree = hready + 1;        // ... and read, by the product and the store
+  uint64_t* gfull = hfree + 1;         // G
+  uint64_t* gmready = gfull + 1;       // G*M written
+  uint64_t* yfull = gmready + 1;       // both products of y
+  uint64_t* yfree = yfull + 1;         // ... and read
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(yfree + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int head = blockIdx.x, b = blockIdx.y, n = p.n;
+  const int g = head * P / (p.D / p.G);
+  const size_t cbase = ((size_t)b * p.NH + head) * n;
+  constexpr uint32_t tG = 128, tH = 160, tY = 192;
+  if (warp == 0) { tc::tmem_alloc(tslot, 256); tc::tmem_relinquish(); }
+  if (tid == 32) {
+    for (int s = 0; s < 2; ++s) {
+      tc::mbar_init(full + s, 1); tc::mbar_init(sfree + s, 5);
+      tc::mbar_init(accfull + s, 1); tc::mbar_init(accfree + s, 4);
+      tc::mbar_init(readyb + s, 4); tc::mbar_init(readyc + s, 4); tc::mbar_init(yready + s, 4);
+    }
+    tc::mbar_init(xsfree, 1); tc::mbar_init(hready, 4); tc::mbar_init(hfree, 2);
+    tc::mbar_init(gfull, 1); tc::mbar_init(gmready, 4); tc::mbar_init(yfull, 1); tc::mbar_init(yfree, 4);
+    tc::mbar_fence_init();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t taddr = *tslot;
+  bool ok = true;
+  auto wait = [&](uint64_t* m, int parity) { if (ok) ok = tc::mbar_wait(m, (uint32_t)parity & 1u); };
+  auto arrive = [&](uint64_t* m) {  // of a whole warp
+    __syncwarp();
+    if (lane == 0) mbar_arrive(m);
+  };
+  auto stage = [&](int it) { return sm + (it & 1) * kScanStage; };
+  auto fresh = [](tc::Tile t) {  // keeps the descriptors of a product from being held in registers from chunk to chunk
+    asm volatile("" : "+r"(t.saddr));
+    return t;
+  };
+
+  if (warp < 4) {  // ---- the state: thread = row, all 64 columns
+    tc::reg_inc<104>();
+    f2 H[P / 2];
+#pragma unroll
+    for (int x = 0; x < P / 2; ++x) H[x] = 0ull;
+    for (int it = 0; it < n; ++it) {
+      const int a = it & 1;
+      if (it > 0) wait(hfree, it - 1);
+#pragma unroll
+      for (int x = 0; x < P / 8; ++x)
+        sts16(Ht, tc::kmajor_unit(tid, x, P), make_uint4(narrow2(H[4 * x]), narrow2(H[4 * x + 1]), narrow2(H[4 * x + 2]), narrow2(H[4 * x + 3])));
+      tc::fence_async_smem();
+      arrive(hready);
+      wait(full + a, it >> 1);
+      wait(accfull + a, it >> 1);
+      tc::fence_after_sync();
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) {
+        const f2 L = dup2(scal[a].L);
+#pragma unroll
+        for (int q = 0; q < P; q += 8) {
+          f2 f[4];
+          ld_pairs(taddr + 64 * a + q, warp, f);
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int x = 0; x < 4; ++x) H[q / 2 + x] = mad2(L, H[q / 2 + x], f[x]);
+        }
+      }
+      tc::fence_before_sync();
+      arrive(accfree + a);
+      arrive(sfree + a);
+    }
+  } else if (warp < 8) {  // ---- G*M and y: this thread's row and the half of the columns that it holds of every result
+    tc::reg_inc<72>();
+    const int t = 32 * (warp & 1) + lane, n0 = 32 * ((warp >> 1) & 1);
+    for (int it = 0; it < n; ++it) {
+      const ChunkScal& s = scal[it & 1];
+      uint8_t* S = stage(it);
+      wait(full + (it & 1), it >> 1);
+      wait(accfull + (it & 1), it >> 1);  // (Brot makes room)
+      wait(gfull, it);
+      tc::fence_after_sync();
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) {
+        float f[32];
+        ld_acc32(taddr + tG, warp, 0, f);
+        mask_row(f, s, t, n0);
+#pragma unroll
+        for (int x = 0; x < 4; ++x) sts16(S, tc::kmajor_unit(t, (n0 >> 3) + x, Q), pack8(&f[8 * x]));
+      }
+      tc::fence_before_sync();
+      tc::fence_async_smem();
+      arrive(gmready);
+      wait(yfull, it);
+      tc::fence_after_sync();
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) {  // y = (G*M) X + exp(Lam) Crot H0
+        const float de = s.dexp[t];
+#pragma unroll
+        for (int q = 0; q < 32; q += 16) {
+          float f[16], h[16];
+          ld_acc16(taddr + tY, warp, q, f);
+          ld_acc16(taddr + tH, warp, q, h);
+#pragma unroll
+          for (int x = 0; x < 16; ++x) f[x] = fmaf(de, h[x], f[x]);
+          sts16(S + 32768, tc::sw128_unit(t, (n0 + q) >> 3), pack8(f));
+          sts16(S + 32768, tc::sw128_unit(t, ((n0 + q) >> 3) + 1), pack8(f + 8));
+        }
+      }
+      tc::fence_before_sync();
+      arrive(yfree);
+      tc::fence_async_smem();
+      arrive(yready + (it & 1));
+    }
+  } else if (warp < 12) {  // ---- rows rotated, x scaled
+    tc::reg_dec<48>();
+    const int u0 = tid - 256;
+    for (int it = 0; it < n; ++it) {
+      const ChunkScal& s = scal[it & 1];
+      uint8_t* S = stage(it);
+      wait(full + (it & 1), it >> 1);
+      rotate_in_tile<true>(S, s.sn, s.cs, u0, 128);
+      if (it > 0) wait(xsfree, it - 1);
+      scale_rows(Xs, S + 32768, s.re, u0, 128);
+      tc::fence_async_smem();
+      arrive(readyb + (it & 1));
+      rotate_in_tile<true>(S + 16384, s.sn, s.cs, u0, 128);
+      tc::fence_async_smem();
+      arrive(readyc + (it & 1));
+    }
+  } else {
+    tc::reg_dec<32>();
+    if (warp == 12) {  // ---- copies
+      if (lane == 0) {
+        int issued = 0;
+        for (int it = 0; it < n; ++it) {
+          const int s = it & 1;
+          uint8_t* S = stage(it);
+          if (it > 1) wait(sfree + s, (it >> 1) - 1);
+          if (!ok) break;
+          ++issued;
+          tc::mbar_expect_tx(full + s, (uint32_t)kScanStage + (uint32_t)sizeof(ChunkScal));
+          for (int sl = 0; sl < 2; ++sl) tc::tma_load_4d(tc::smem_u32(S) + 8192 * sl, &maps.b, 64 * sl, g, it * Q, b, full + s);
+          tc::tma_load_4d(tc::smem_u32(S) + 32768, &maps.x, 0, head, it * Q, b, full + s);
+          tc::bulk_load(tc::smem_u32(scal + s), p.cs + (cbase + it) * (sizeof(ChunkScal) / 4), (uint32_t)sizeof(ChunkScal), full + s);
+          for (int sl = 0; sl < 2; ++sl) tc::tma_load_4d(tc::smem_u32(S) + 16384 + 8192 * sl, &maps.c, 64 * sl, g, it * Q, b, full + s);
+        }
+        for (int q = max(0, issued - 2); q < issued; ++q) tc::mbar_wait(full + (q & 1), (q >> 1) & 1);  // (outlive the copies)
+      }
+    } else if (warp == 13) {  // ---- products of the state
+      if (tc::elect_one()) {
+        for (int it = 0; it < n; ++it) {
+          const int a = it & 1;
+          wait(readyb + a, it >> 1);
+          if (it > 1) wait(accfree + a, (it >> 1) - 1);
+          if (!ok) break;
+          tc::fence_after_sync();
+          // [128 n x 64 p] = Brot^T diag(r e) X, both contracted over their rows
+          tc::issue_gemm(taddr + 64 * a, fresh(tc::mnmajor_sw128_tile(stage(it), 8192)), fresh(tc::mnmajor_sw128_tile(Xs, 8192)), 128, P, Q, false);
+          tc::mma_commit(accfull + a);
+          tc::mma_commit(xsfree);
+        }
+      }
+    } else if (warp == 14) {  // ---- products of the output
+      if (tc::elect_one()) {
+        for (int it = 0; it < n; ++it) {
+          wait(readyb + (it & 1), it >> 1);
+          wait(readyc + (it & 1), it >> 1);
+          if (!ok) break;
+          tc::fence_after_sync();
+          tc::issue_gemm<true>(taddr + tG, fresh(tc::kmajor_sw128_tile(stage(it) + 16384, 8192)), fresh(tc::kmajor_sw128_tile(stage(it), 8192)), 64, Q, N, false);  // G = Crot Brot^T
+          tc::mma_commit(gfull);
+          wait(hready, it);
+          if (it > 0) wait(yfree, it - 1);
+          if (!ok) break;
+          tc::fence_after_sync();
+          tc::issue_gemm<true>(taddr + tH, fresh(tc::kmajor_sw128_tile(stage(it) + 16384, 8192)), fresh(tc::mnmajor_tile(Ht, P)), 64, P, N, false);         // Crot H0
+          tc::mma_commit(hfree);
+          wait(gmready, it);
+          if (!ok) break;
+          tc::fence_after_sync();
+          tc::issue_gemm<true>(taddr + tY, fresh(tc::kmajor_tile(stage(it), Q)), fresh(tc::mnmajor_sw128_tile(stage(it) + 32768, 8192)), 64, P, Q, false);  // (G*M) X
+          tc::mma_commit(yfull);
+        }
+      }
+    } else {  // ---- stores
+      if (lane == 0) {
+        for (int it = 0; it < n; ++it) {
+          uint8_t* S = stage(it);
+          wait(hready, it);
+          if (!ok) break;
+          if (save) {
+            tc::bulk_store(p.H0 + (cbase + it) * (N * P), tc::smem_u32(Ht), 16384);
+            tc::bulk_commit();
+            tc::bulk_wait_read<0>();
+          }
+          mbar_arrive(hfree);
+          wait(yready + (it & 1), it >> 1);
+          if (!ok) break;
+          tc::tma_store_4d(&maps.y, tc::smem_u32(S) + 32768, 0, head, it * Q, b);
+          tc::bulk_commit();
+          tc::bulk_wait_read<0>();
+          mbar_arrive(sfree + (it & 1));
+        }
+      }
+    }
+    __syncwarp();
+    ok = __all_sync(0xffffffffu, ok);
+  }
+  if (!ok && lane == 0) atomicExch(p.status, 14);
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(taddr, 256);
+}
+
 // ------------------------------------------------------------ chunk gradients
 // One CTA per chunk and up to kGradHeads heads of a group.  The heads of a group share B and C and differ by one angle per
 // step, so nothing is rotated: with J(e, o) = (-o, e) on every pair of states and delta = phi_t - phi_s
@@ -687,13 +967,6 @@ static_assert(kGradSmem <= 227 * 1024, "one CTA per SM");
 constexpr int kGradPitch = N + 4;  // floats per row of the sums on their way out (over the stages)
 static_assert(2 * Q * kGradPitch * 4 <= 2 * kGradStage, "two tiles of row sums fit into the stages");
 
-// 8 columns of a result as four pairs.
-__device__ __forceinline__ void ld_pairs(uint32_t taddr, int warp, f2 (&f)[4]) {
-  uint32_t r[8];
-  tc::tmem_ld_32x32b_x8(taddr + ((uint32_t)(32 * (warp & 3)) << 16), r);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) f[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-}
 template <bool TMA>
 __global__ void __launch_bounds__(kGradThreads, 1) m3s_chunk_grad_kernel(SsdP p, const __grid_constant__ ChunkMaps maps) {
   begin_dependent();
@@ -1365,7 +1638,18 @@ static mxb_status ssd_state_pass(SsdP& p, int mode, cudaStream_t st) {
   return check_launch("m3s_state_pass_kernel");
 }
 
-static mxb_status ssd_forward(SsdP& p, cudaStream_t st) {
+// States and output by one kernel where the CTAs of the state pass would share SMs; false where a tensor map cannot be made.  Of
+// fewer (batch, head) pairs the chain of chunks is what counts, and the output kernel spreads over all SMs.  Forward, us, two
+// kernels / one: 1 x 4096 x 32 heads 76 / 140, 4 x 4096 x 32 147 / 164, 5 x 2000 x 32 114 / 115 (108 without keeping the states),
+// 6 x 2000 x 32 126 / 119, 8 x 1024 x 32 81 / 68, 8 x 4096 x 32 286 / 238 (215).  The bits are the same.
+static bool ssd_scan_maps(const SsdP& p, m3s::ScanMaps& maps) {
+  std::memset(&maps, 0, sizeof maps);
+  return !p.no_tma && make_tma_map_bthd(&maps.b, p.b, p.B, p.T, p.G, m3s::N) && make_tma_map_bthd(&maps.c, p.c, p.B, p.T, p.G, m3s::N) &&
+         make_tma_map_bthd(&maps.x, p.x, p.B, p.T, p.NH, m3s::P) && make_tma_map_bthd(&maps.y, p.y, p.B, p.T, p.NH, m3s::P);
+}
+
+// save: the states at the chunk starts are kept for a backward.
+static mxb_status ssd_forward(SsdP& p, bool save, cudaStream_t st) {
   const dim3 gc(p.n, p.NH, p.B);
   // (the chunks' shares of the angle lie where the state pass writes the chunk states afterwards)
   double* share = reinterpret_cast<double*>(p.H0);
@@ -1383,6 +1667,13 @@ static mxb_status ssd_forward(SsdP& p, cudaStream_t st) {
     MXB_LAUNCH("m3s_chunk_scalars_kernel", st, (launch_kernel(m3s::m3s_chunk_scalars_kernel<true>, gc, 64, 0, st, p, angles)));
   } else {
     MXB_LAUNCH("m3s_chunk_scalars_kernel", st, (launch_kernel(m3s::m3s_chunk_scalars_kernel<false>, gc, 64, 0, st, p, angles)));
+  }
+  m3s::ScanMaps scan;
+  if (p.y && p.NH * p.B > 148 && ssd_scan_maps(p, scan)) {
+    if (MXB_ALLOW_SMEM(m3s::kScanSmem, m3s::m3s_scan_out_kernel) != MXB_OK) return MXB_ERR_CUDA;
+    MXB_LAUNCH("m3s_scan_out_kernel", st,
+               (launch_kernel(m3s::m3s_scan_out_kernel, dim3(p.NH, p.B), m3s::kScanThreads, m3s::kScanSmem, st, p, save ? 1 : 0, scan)));
+    return check_launch("mamba3 ssd forward");
   }
   mxb_status ps = ssd_state_pass(p, 0, st);
   if (ps != MXB_OK) return ps;
@@ -1406,7 +1697,7 @@ mxb_status mamba3_ssd_fwd(const mxb_mamba3_desc* d, const void* x, const float* 
   p.x = static_cast<const m3s::bf16*>(x); p.b = static_cast<const m3s::bf16*>(b); p.c = static_cast<const m3s::bf16*>(c);
   p.dt_raw = dt; p.lam_raw = lam; p.theta = theta; p.a_log = a_log; p.y = static_cast<m3s::bf16*>(y);
   carve_ssd(p, ws, false);
-  return ssd_forward(p, st);
+  return ssd_forward(p, (d->flags & MXB_MAMBA3_SAVE_FOR_BWD) != 0, st);
 }
 
 mxb_status mamba3_ssd_bwd(const mxb_mamba3_desc* d, const void* x, const float* dt, const float* lam,
@@ -1422,7 +1713,7 @@ mxb_status mamba3_ssd_bwd(const mxb_mamba3_desc* d, const void* x, const float* 
   p.y = nullptr;  // the forward recompute stops at the chunk states
   // with saved intermediates dt, lambda, phi, the chunk decays and H0 are still in place
   if (!(d->flags & MXB_MAMBA3_BWD_USE_SAVED)) {
-    mxb_status s = ssd_forward(p, st);
+    mxb_status s = ssd_forward(p, true, st);
     if (s != MXB_OK) return s;
   }
   const dim3 gg(p.n, p.G * p.splits, p.B);

@@ -336,3 +336,24 @@ def test_block_bc_rows_of_every_lane_group(cfg, io):
     """2, 4, 8 and 16 lanes a row, whole and partly filled, with ragged numbers of rows."""
     from test_mamba3_block_gpu import test_bc_norm_forward_and_gradients
     test_bc_norm_forward_and_gradients(cfg, io)
+
+
+@pytest.mark.parametrize("T", [1, 64, 65, 130, 257])
+@pytest.mark.parametrize("G", [1, 2])
+def test_mamba3_states_and_output_in_one_kernel(T, G):
+    """More (batch, head) pairs than SMs take one kernel for states and output, fewer take two: the same bits, and the states it
+    keeps serve the backward as the recomputed ones do."""
+    B, nheads = 5, 32
+    a = inputs.mamba3_inputs(B, T, nheads, 64, 128, G=G, seed=61, io_dtype=BF16, per_head=True)
+    names = ("x", "dt_raw", "lambda_raw", "theta", "a_log", "b", "c")
+    args = [_dev(a[n]) for n in names]
+    y = ops.mamba3_selective_scan(*args, nheads=nheads, save_for_backward=True)
+    dy = _dev(a["dy"])
+    saved = ops.mamba3_selective_scan_backward(*args, dy, nheads=nheads, use_saved=True)
+    again = ops.mamba3_selective_scan_backward(*args, dy, nheads=nheads)
+    for n in saved:
+        assert torch.equal(saved[n], again[n]), n
+    assert torch.equal(y, ops.mamba3_selective_scan(*args, nheads=nheads))
+    for b in (0, B - 1):
+        row = [t if n == "a_log" else t[b:b + 1].contiguous() for n, t in zip(names, args)]
+        assert torch.equal(y[b:b + 1], ops.mamba3_selective_scan(*row, nheads=nheads))
