@@ -313,23 +313,10 @@ __global__ void __launch_bounds__(256) mamba3_bwd_kernel(M3P p) {
 
 // dB[b,t,g,:] = the S slice rows of the group added in slice order, in the tensors' dtype.
 template <typename IO>
-__global__ void __launch_bounds__(256) m3_bc_sum_kernel(const float* __restrict__ pb, const float* __restrict__ pc,
-                                                        IO* __restrict__ db, IO* __restrict__ dc, size_t rows, int S, int N) {
+__global__ void __launch_bounds__(256) m3_bc_sum_kernel(M3P p) {
   begin_dependent();
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < rows * N; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t r = i / N;
-    const int n = (int)(i - r * N);
-    float sb = 0.f, sc = 0.f;
-    for (int s = 0; s < S; ++s) {
-      sb += pb[(r * S + s) * N + n];
-      sc += pc[(r * S + s) * N + n];
-    }
-    db[i] = from_f32<IO>(sb);
-    dc[i] = from_f32<IO>(sc);
-  }
+  m3_bc_sum<IO>(p, blockIdx.x, gridDim.x);
 }
-
-// Head-broadcast layout: ddt, dlam, dtheta [B,T,NH] = the per-channel values of a head added in channel order.
 __global__ void __launch_bounds__(256) m3_head_sum_kernel(const float* __restrict__ hd, float* __restrict__ ddt,
                                                           float* __restrict__ dlam, float* __restrict__ dtheta,
                                                           size_t rows, int D, int NH) {
@@ -354,27 +341,9 @@ __global__ void __launch_bounds__(256) m3_head_sum_kernel(const float* __restric
 
 // da_log = the per-batch (or per-window) partials added in a fixed order ([D,N]), and over the channels of a head ([NH]):
 // 16 slices of the rows per output, then the slices in order.
-constexpr int kDalogSlices = 16;
-__global__ void __launch_bounds__(32 * kDalogSlices) m3_dalog_sum_kernel(const float* __restrict__ part, float* __restrict__ out,
-                                                                         int rows, int D, int N, int NH) {
+__global__ void __launch_bounds__(32 * kDalogSlices) m3_dalog_sum_kernel(M3P p, int rows) {
   begin_dependent();
-  __shared__ float red[kDalogSlices][32];
-  const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
-  const int cph = NH > 0 ? D / NH : 1, outs = NH > 0 ? NH : D * N, total = rows * cph;
-  float s = 0.f;
-  if (i < outs) {
-#pragma unroll 8
-    for (int r = slice; r < total; r += kDalogSlices)
-      s += NH > 0 ? part[(size_t)(r / cph) * D + i * cph + r % cph] : part[(size_t)r * outs + i];
-  }
-  red[slice][lane] = s;
-  __syncthreads();
-  if (slice == 0 && i < outs) {
-    s = 0.f;
-#pragma unroll
-    for (int k = 0; k < kDalogSlices; ++k) s += red[k][lane];
-    out[i] = s;
-  }
+  m3_dalog_sum(p, rows, blockIdx.x);
 }
 
 // --------------------------------------------------------------------- host
@@ -581,7 +550,7 @@ mxb_status mamba3_bwd(const mxb_mamba3_desc* d, const void* x, const float* dt, 
   M3P p = make_m3(d);
   const bool f32 = d->io_dtype == MXB_F32;
   p.x = x; p.dt = dt; p.lam = lam; p.theta = theta; p.a_log = a_log; p.b = b; p.c = c;
-  p.dy = dy; p.dx = dx; p.ddt = ddt; p.dlam = dlam; p.dtheta = dtheta; p.da_log = da_log;
+  p.dy = dy; p.dx = dx; p.ddt = ddt; p.dlam = dlam; p.dtheta = dtheta; p.da_log = da_log; p.db = db; p.dc = dc;
   const bool head_bwd = !(d->flags & MXB_MAMBA3_CHANNEL_KERNELS) && mamba3_head_bwd_supported(d);
   float *pb = nullptr, *pc = nullptr, *hscal = nullptr;
   if (head_bwd) p.nW = (d->T + mamba3_head_window() - 1) / mamba3_head_window();
@@ -608,19 +577,17 @@ mxb_status mamba3_bwd(const mxb_mamba3_desc* d, const void* x, const float* dt, 
     s = f32 ? m3_bwd_serial<float>(p, st) : m3_bwd_serial<__nv_bfloat16>(p, st);
   }
   if (s != MXB_OK) return s;
-  const size_t rows = (size_t)p.B * p.T * p.G;
-  const int grid = (int)std::min<size_t>((rows * p.N + 255) / 256, 148 * 8);
-  if (f32)
-    MXB_LAUNCH("m3_bc_sum_kernel", st, (launch_kernel(m3_bc_sum_kernel<float>, grid, 256, 0, st, p.pb32, p.pc32, static_cast<float*>(db), static_cast<float*>(dc), rows, p.S, p.N)));
-  else
-    MXB_LAUNCH("m3_bc_sum_kernel", st, (launch_kernel(m3_bc_sum_kernel<__nv_bfloat16>, grid, 256, 0, st, p.pb32, p.pc32, static_cast<__nv_bfloat16*>(db), static_cast<__nv_bfloat16*>(dc), rows, p.S, p.N)));
+  if (!windows) {  // (the window kernels have added them up)
+    const int grid = m3_bc_sum_blocks(p, 256);
+    if (f32) MXB_LAUNCH("m3_bc_sum_kernel", st, (launch_kernel(m3_bc_sum_kernel<float>, grid, 256, 0, st, p)));
+    else MXB_LAUNCH("m3_bc_sum_kernel", st, (launch_kernel(m3_bc_sum_kernel<__nv_bfloat16>, grid, 256, 0, st, p)));
+    MXB_LAUNCH("m3_dalog_sum_kernel", st, (launch_kernel(m3_dalog_sum_kernel, m3_dalog_blocks(p), 32 * kDalogSlices, 0, st, p, p.B)));
+  }
   if (p.NH > 0) {
     const size_t bt = (size_t)p.B * p.T;
     const int gh = (int)std::min<size_t>((bt * p.NH + 255) / 256, 148 * 8);
     MXB_LAUNCH("m3_head_sum_kernel", st, (launch_kernel(m3_head_sum_kernel, gh, 256, 0, st, p.hd, ddt, dlam, dtheta, bt, p.D, p.NH)));
   }
-  const int nal = p.NH > 0 ? p.NH : p.D * p.N;
-  MXB_LAUNCH("m3_dalog_sum_kernel", st, (launch_kernel(m3_dalog_sum_kernel, (nal + 31) / 32, 32 * kDalogSlices, 0, st, p.dal_part, da_log, windows ? p.B * p.nW : p.B, p.D, p.N, p.NH)));
   return check_launch("mamba3 channel backward sums");
 }
 

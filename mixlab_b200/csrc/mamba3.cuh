@@ -17,6 +17,7 @@ struct M3P {
   const void* dy;
   void* dx;
   float *ddt, *dlam, *dtheta, *da_log;
+  void *db, *dc;
   // channel kernels: CW channels (warps) per CTA, S = channels per group / CW slices per group
   int CW, S;
   float *pb32, *pc32;  // [B,T,G,S,N] rows summed over the CW channels of a CTA
@@ -63,6 +64,50 @@ struct M3Idx {
   __device__ size_t alog(int d, int n) const { return NH > 0 ? (size_t)(d / cph) : (size_t)d * N + n; }
   __device__ size_t grp(size_t row, int d, int n) const { return (row * G + d / cpg) * N + n; }
 };
+
+// Sums of the partials the reverse walks leave, in a fixed order, by the block-th of `blocks` blocks.
+// dB, dC: rows over the slices of a group.
+template <typename IO>
+__device__ __forceinline__ void m3_bc_sum(const M3P& p, int block, int blocks) {
+  const size_t total = (size_t)p.B * p.T * p.G * p.N;
+  for (size_t i = block * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)blocks * blockDim.x) {
+    const size_t r = i / p.N;
+    const int n = (int)(i - r * p.N);
+    float sb = 0.f, sc = 0.f;
+    for (int s = 0; s < p.S; ++s) {
+      sb += p.pb32[(r * p.S + s) * p.N + n];
+      sc += p.pc32[(r * p.S + s) * p.N + n];
+    }
+    static_cast<IO*>(p.db)[i] = from_f32<IO>(sb);
+    static_cast<IO*>(p.dc)[i] = from_f32<IO>(sc);
+  }
+}
+inline int m3_bc_sum_blocks(const M3P& p, int threads) {
+  const size_t want = ((size_t)p.B * p.T * p.G * p.N + threads - 1) / threads, most = 148 * 2048 / threads;
+  return (int)(want < most ? want : most);
+}
+// da_log over the batch (and windows: `rows`), and the channels of a head; 32 outputs a block of 16 warps, each with a slice.
+constexpr int kDalogSlices = 16;
+__device__ __forceinline__ void m3_dalog_sum(const M3P& p, int rows, int block) {
+  __shared__ float red[kDalogSlices][32];
+  const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, i = block * 32 + lane;
+  const int cph = p.NH > 0 ? p.D / p.NH : 1, outs = p.NH > 0 ? p.NH : p.D * p.N, total = rows * cph;
+  float s = 0.f;
+  if (i < outs) {
+#pragma unroll 8
+    for (int r = slice; r < total; r += kDalogSlices)
+      s += p.NH > 0 ? p.dal_part[(size_t)(r / cph) * p.D + i * cph + r % cph] : p.dal_part[(size_t)r * outs + i];
+  }
+  red[slice][lane] = s;
+  __syncthreads();
+  if (slice == 0 && i < outs) {
+    s = 0.f;
+#pragma unroll
+    for (int k = 0; k < kDalogSlices; ++k) s += red[k][lane];
+    p.da_log[i] = s;
+  }
+}
+inline int m3_dalog_blocks(const M3P& p) { return ((p.NH > 0 ? p.NH : p.D * p.N) + 31) / 32; }
 
 constexpr int kM3WinSteps = 8;  // steps per window of the window-parallel kernels
 struct M3WinShape { int lanes, warps; };  // lanes per channel; warps per CTA, all of one group

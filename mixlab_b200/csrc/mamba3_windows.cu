@@ -10,14 +10,15 @@
 //             also what the trapezoid's look-back sends to the window's last step: exp(A dt) up of the step behind)
 //   walk      forward: the true walk writes y;  backward: replay into shared memory, then the true reverse walk with
 //             window-local angle-gradient sums
-//   scan, fix reverse scan of those sums; the later windows' sums are added to ddt and dtheta
+//   sums, fix reverse scan of those sums (and the sums of dB, dC and da_log over CTAs and windows); the later windows' sums are
+//             added to ddt and dtheta
 //
 // What bounds it: instruction issue (a sine, a cosine and two exponentials per state pair and pass).  So everything
 // that belongs to a (step, channel) is computed once and not by every lane and pass; the two states of a pair and two
 // pairs per lane go through packed arithmetic; a pass keeps sine, cosine and decay in shared memory for its reverse
 // half; rows of dB, dC are added over the channels of a warp by halving exchanges and over the warps once per window.
 // Scans run 16 segments of windows side by side.  2 x 1024 x 128 channels of 16 states, forward + backward:
-// 70 us a call; 4096 x 448 channels: 0.42 ms.
+// 65 us a call; 4096 x 448 channels: 0.41 ms.
 //
 // Every sum has a fixed order: the same inputs give the same bits.
 #include <algorithm>
@@ -293,12 +294,12 @@ __device__ __forceinline__ uint32_t turns(float x) {
 }
 constexpr int kChains = 16, kSegs = 32, kScanThreads = kChains * kSegs;
 template <int MODE, int PER>
-__device__ __forceinline__ void scan_chain(const M3P& p, int chains) {
+__device__ __forceinline__ void scan_chain(const M3P& p, int chains, int block, int b) {
   constexpr bool linear = MODE == kState || MODE == kDh, back = MODE == kDh || MODE == kAngle;
   using Sum = std::conditional_t<MODE == kPhase, uint32_t, float>;
   __shared__ Sum s_add[kSegs][kChains];
   __shared__ float s_dec[kSegs][kChains];
-  const int lane = threadIdx.x % kChains, seg = threadIdx.x / kChains, b = blockIdx.y, i = blockIdx.x * kChains + lane;
+  const int lane = threadIdx.x % kChains, seg = threadIdx.x / kChains, i = block * kChains + lane;
   const bool in = i < chains;
   float* buf = MODE == kPhase ? p.ck_phi : MODE == kState ? p.ck_h : MODE == kDh ? p.dhk : p.ang;
   const int d = linear ? i / p.N : 0;
@@ -360,19 +361,26 @@ __device__ __forceinline__ void scan_chain(const M3P& p, int chains) {
 template <int PER>
 __global__ void __launch_bounds__(kScanThreads) m3w_phase_scan_kernel(M3P p) {
   begin_dependent();
-  scan_chain<kPhase, PER>(p, p.D * p.Kp);
+  scan_chain<kPhase, PER>(p, p.D * p.Kp, blockIdx.x, blockIdx.y);
 }
-template <int PER>
-__global__ void __launch_bounds__(kScanThreads) m3w_angle_scan_kernel(M3P p) {
+// What follows the gradient walk and does not wait for each other, in one launch (three took 12 us at 2 x 1024 x 128 channels,
+// 5 together): the first `scans` blocks scan the angle gradients, the next `dalogs` add the shares of da_log, the others
+// the rows of dB and dC.
+template <typename IO, int PER>
+__global__ void __launch_bounds__(kScanThreads) m3w_sums_kernel(M3P p, int scans, int dalogs) {
+  static_assert(kScanThreads == 32 * kDalogSlices, "one block size");
   begin_dependent();
-  scan_chain<kAngle, PER>(p, p.D * p.Kp);
+  const int block = blockIdx.x;
+  if (block < scans) scan_chain<kAngle, PER>(p, p.D * p.Kp, block / p.B, block % p.B);
+  else if (block < scans + dalogs) m3_dalog_sum(p, p.B * p.nW, block - scans);
+  else m3_bc_sum<IO>(p, block - scans - dalogs, gridDim.x - scans - dalogs);
 }
 // blockIdx.z: 0 the states, 1 dh (first: the one to start with)
 template <int PER>
 __global__ void __launch_bounds__(kScanThreads) m3w_linear_scan_kernel(M3P p, int first) {
   begin_dependent();
-  if (first + (int)blockIdx.z == 0) scan_chain<kState, PER>(p, p.D * p.N);
-  else scan_chain<kDh, PER>(p, p.D * p.N);
+  if (first + (int)blockIdx.z == 0) scan_chain<kState, PER>(p, p.D * p.N, blockIdx.x, blockIdx.y);
+  else scan_chain<kDh, PER>(p, p.D * p.N, blockIdx.x, blockIdx.y);
 }
 
 // -------------------------------------------------------------- local walks
@@ -948,9 +956,11 @@ static mxb_status backward(const M3P& p, bool have_states, cudaStream_t st) {
   linear_scan(p, first, 2 - first, st);
   M3W_DISPATCH(g.shape.lanes, p, (s = launch_grad<IO, PRV, LPCV, PL>(p, g, st)));
   if (s != MXB_OK) return s;
+  const int scans = chain_grid(p, p.D * p.Kp, 1).x * p.B, dalogs = m3_dalog_blocks(p);
   by_segment(p, [&](auto per) {
-    MXB_LAUNCH("m3w_angle_scan_kernel", st,
-               (launch_kernel(m3w_angle_scan_kernel<decltype(per)::value>, chain_grid(p, p.D * p.Kp, 1), kScanThreads, 0, st, p)));
+    MXB_LAUNCH("m3w_sums_kernel", st,
+               (launch_kernel(m3w_sums_kernel<IO, decltype(per)::value>, scans + dalogs + m3_bc_sum_blocks(p, kScanThreads), kScanThreads, 0,
+                              st, p, scans, dalogs)));
   });
   m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
     M3W_DISPATCH(g.shape.lanes, p, MXB_LAUNCH("m3w_fix_kernel", st, (launch_kernel(m3w_fix_kernel<IO, PRV, LPCV, PL>, grid, g.threads, 0, st, q))));
