@@ -680,10 +680,12 @@ static int blk_tiles(const mxb_gdn_desc* d) {
   const int tile = blk::kPreRuns * blk_run(d);
   return (d->T + tile - 1) / tile;
 }
-static int blk_post_ctas(const mxb_gdn_desc* d) {
+// CTAs of the output stage: what is on the GPU at once (eight an SM forward, six backward), so that no second round of a few CTAs
+// follows (backward, 16 x 2048 x 16 heads of 64: 73 us with eight an SM asked for, 60 with six).
+static int blk_post_ctas(const mxb_gdn_desc* d, bool bwd) {
   const size_t rows = (size_t)d->B * d->T * d->H, per = 128 / blk_lanes(d->Dv, 8);
-  const size_t want = (rows + per - 1) / per;
-  return (int)(want < 148 * 8 ? want : 148 * 8);
+  const size_t want = (rows + per - 1) / per, most = 148 * (bwd ? 6 : 8);
+  return (int)(want < most ? want : most);
 }
 static int blk_gate_ctas(const mxb_gdn_desc* d) {
   const size_t n = (size_t)d->B * d->T * d->H;
@@ -693,7 +695,7 @@ static int blk_gate_ctas(const mxb_gdn_desc* d) {
 size_t gdn_block_workspace_bytes(const mxb_gdn_desc* d) {
   const size_t rows = (size_t)d->B * blk_tiles(d);
   const size_t pre = rows * 4 * ((size_t)2 * d->H * d->Dk + (size_t)d->H * d->Dv) * sizeof(float);
-  const size_t post = (size_t)blk_post_ctas(d) * d->Dv * sizeof(float);
+  const size_t post = (size_t)blk_post_ctas(d, true) * d->Dv * sizeof(float);
   const size_t gate = 2 * (size_t)blk_gate_ctas(d) * d->H * sizeof(float);
   return (pre + gate > post ? pre + gate : post) + 256;
 }
@@ -844,7 +846,7 @@ template <typename IO>
 static mxb_status blk_post(const mxb_gdn_desc* d, const void* o, const void* z, const float* wn, void* y,
                            const void* dy, void* d_o, void* dz, float* dwn, void* ws, cudaStream_t st) {
   BlockP p = make_blk(d);
-  const int ctas = blk_post_ctas(d);
+  const int ctas = blk_post_ctas(d, dy != nullptr);
   const int lanes = blk_lanes(d->Dv, 8);
   if (!dy) {
     with_lanes(lanes, [&](auto lpr) {

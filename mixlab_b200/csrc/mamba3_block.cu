@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(256) m3b_post_fwd_warp_kernel(BlkP p, const IO
   }
 }
 template <typename IO>
-__global__ void __launch_bounds__(256) m3b_post_bwd_warp_kernel(BlkP p, const IO* __restrict__ y, const IO* __restrict__ z,
+__global__ void __launch_bounds__(256, 2) m3b_post_bwd_warp_kernel(BlkP p, const IO* __restrict__ y, const IO* __restrict__ z,
                                                                 const float* __restrict__ wn, const IO* __restrict__ dout,
                                                                 IO* __restrict__ dy, IO* __restrict__ dz,
                                                                 float* __restrict__ dwp) {
@@ -505,14 +505,16 @@ static int m3b_bc_ctas(const mxb_mamba3_desc* d) {
   const size_t per = 128 / m3b_bc_lanes(d), want = ((size_t)d->B * d->T + per - 1) / per;
   return (int)std::min<size_t>(want, 148 * 4);
 }
-static int m3b_post_ctas(const mxb_mamba3_desc* d) {
+// CTAs of the output stage: what is on the GPU at once.
+static int m3b_post_ctas(const mxb_mamba3_desc* d, bool bwd) {
   const size_t rows = (size_t)d->B * d->T;
-  return (int)(d->D <= m3b::kWarpRow ? std::min<size_t>((rows + 7) / 8, 148 * 4) : std::min<size_t>(rows, 148 * 8));
+  if (d->D <= m3b::kWarpRow) return (int)std::min<size_t>((rows + 7) / 8, 148 * (bwd ? 2 : 3));
+  return (int)std::min<size_t>(rows, 148 * (bwd ? 3 : 5));
 }
 size_t mamba3_block_workspace_bytes(const mxb_mamba3_desc* d) {
   const size_t conv = (size_t)d->B * m3b_runs(d) * m3b::kMaxK * d->D * sizeof(float);
   const size_t bc = 2 * (size_t)m3b_bc_ctas(d) * d->G * 2 * d->N * sizeof(float);
-  const size_t post = (size_t)m3b_post_ctas(d) * d->D * sizeof(float);
+  const size_t post = (size_t)m3b_post_ctas(d, true) * d->D * sizeof(float);
   size_t m = conv > bc ? conv : bc;
   m = m > post ? m : post;
   return m + 256;
@@ -605,7 +607,7 @@ template <typename IO>
 static mxb_status m3b_post(const mxb_mamba3_desc* d, float eps, const void* y, const void* z, const float* wn, void* out,
                            const void* dout, void* dy, void* dz, float* dwn, void* ws, cudaStream_t st) {
   BlkP p = make_m3b(d, 0, eps);
-  const int ctas = m3b_post_ctas(d);
+  const int ctas = m3b_post_ctas(d, dout != nullptr);
   const bool narrow = d->D <= m3b::kWarpRow;
   const IO *yv = static_cast<const IO*>(y), *zv = static_cast<const IO*>(z);
   if (!dout) {
