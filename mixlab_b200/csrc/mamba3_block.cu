@@ -15,15 +15,17 @@ namespace mxb {
 namespace m3b {
 
 using bf16 = __nv_bfloat16;
-constexpr int kRun = 16;     // steps per lane for the convolution
+constexpr int kRun = 16;     // steps per lane for the convolution: a whole number of these
 constexpr int kMaxK = 4;     // taps
 
 struct BlkP {
   int B, T, D, N, G, K;
   float eps;
+  int runs;   // convolution: a lane's steps / kRun
+  int wvec;   // convolution: the four taps of a channel can be read at once
 };
 
-// C consecutive channels: 8 of either type, or 4 floats.
+// C consecutive channels: 8 or 4.
 template <typename IO, int C>
 __device__ __forceinline__ void load_n(const IO* p, float (&e)[C]) {
   if constexpr (sizeof(IO) == 4) {
@@ -33,10 +35,11 @@ __device__ __forceinline__ void load_n(const IO* p, float (&e)[C]) {
       e[4 * i] = a.x; e[4 * i + 1] = a.y; e[4 * i + 2] = a.z; e[4 * i + 3] = a.w;
     }
   } else {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+    using V = std::conditional_t<C == 8, uint4, uint2>;
+    const V v = __ldg(reinterpret_cast<const V*>(p));
     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { e[2 * i] = __low2float(h[i]); e[2 * i + 1] = __high2float(h[i]); }
+    for (int i = 0; i < C / 2; ++i) { e[2 * i] = __low2float(h[i]); e[2 * i + 1] = __high2float(h[i]); }
   }
 }
 template <typename IO, int C>
@@ -46,11 +49,12 @@ __device__ __forceinline__ void store_n(IO* p, const float (&e)[C]) {
     for (int i = 0; i < C / 4; ++i)
       reinterpret_cast<float4*>(p)[i] = make_float4(e[4 * i], e[4 * i + 1], e[4 * i + 2], e[4 * i + 3]);
   } else {
-    uint4 v;
+    using V = std::conditional_t<C == 8, uint4, uint2>;
+    V v;
     __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(e[2 * i], e[2 * i + 1]);
-    *reinterpret_cast<uint4*>(p) = v;
+    for (int i = 0; i < C / 2; ++i) h[i] = __floats2bfloat162_rn(e[2 * i], e[2 * i + 1]);
+    *reinterpret_cast<V*>(p) = v;
   }
 }
 template <typename IO>
@@ -60,12 +64,30 @@ __device__ __forceinline__ void store8(IO* p, const float (&e)[8]) { store_n<IO,
 __device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 
 // ------------------------------------------------------------------ depthwise convolution
-// grid (ceil(D/C / 128), ceil(T / kRun), B) x 128: thread = C channels (16 bytes of a row, so that the lanes of a warp read whole
-// lines), kRun steps; weights w[d][k], k < K <= 4.  Loads in flight bound small calls: 4096 x 448 float32 channels, forward /
-// backward 12.8 / 13.9 us with eight channels a thread (two loads of 16 bytes, 32 apart; 56 threads of a CTA at work),
-// 8.3 / 11.7 with four.
+// grid (ceil(D/C / 128), ceil(T / (runs kRun)), B) x 128: thread = C channels (16 bytes of a row, so that the lanes of a warp read
+// whole lines), runs kRun steps; weights w[d][k], k < K <= 4.  Loads in flight bound small calls: 4096 x 448 float32 channels,
+// forward / backward 12.8 / 13.9 us with eight channels a thread (two loads of 16 bytes, 32 apart; 56 threads of a CTA at work), 8.3
+// / 11.7 with four.  In large ones the weights did: 32 loads a thread, each of 32 lines, for 19 of x (8 x 4096 x 2048 bf16, forward
+// / backward with the column sums 114 / 203 us); read tap by tap only where they must be, and for up to 64 steps: 65 / 187.  The
+// backward takes four channels of bf16 too, so that six CTAs fit an SM: 95.
 template <typename IO>
 constexpr int kConvC = 16 / sizeof(IO);
+constexpr int kConvBwdC = 4;  // (the backward's weights, their gradients and six rows of eight channels do not fit a thread's registers)
+template <int C>
+__device__ __forceinline__ void conv_weights(float (&wk)[kMaxK][C], const float* __restrict__ w, const BlkP& p, int ch) {
+  if (p.wvec) {
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const float4 x = __ldg(reinterpret_cast<const float4*>(w) + ch + c);
+      wk[0][c] = x.x; wk[1][c] = x.y; wk[2][c] = x.z; wk[3][c] = x.w;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < kMaxK; ++k)
+#pragma unroll
+      for (int c = 0; c < C; ++c) wk[k][c] = k < p.K ? w[(size_t)(ch + c) * p.K + k] : 0.f;
+  }
+}
 template <typename IO>
 __global__ void __launch_bounds__(128) m3b_conv_fwd_kernel(BlkP p, const IO* __restrict__ x, const float* __restrict__ w,
                                                            IO* __restrict__ y) {
@@ -73,89 +95,95 @@ __global__ void __launch_bounds__(128) m3b_conv_fwd_kernel(BlkP p, const IO* __r
   constexpr int C = kConvC<IO>;
   const int cg = blockIdx.x * 128 + threadIdx.x, ch = cg * C;
   if (ch >= p.D) return;
-  const int t0 = blockIdx.y * kRun, b = blockIdx.z;
+  const int first = blockIdx.y * p.runs * kRun, b = blockIdx.z;
   float wk[kMaxK][C];
-#pragma unroll
-  for (int k = 0; k < kMaxK; ++k)
-#pragma unroll
-    for (int c = 0; c < C; ++c) wk[k][c] = k < p.K ? w[(size_t)(ch + c) * p.K + k] : 0.f;
+  conv_weights<C>(wk, w, p, ch);
   const IO* __restrict__ xb = x + (size_t)b * p.T * p.D + ch;
   IO* __restrict__ yb = y + (size_t)b * p.T * p.D + ch;
   float x1[C], x2[C], x3[C];
 #pragma unroll
   for (int c = 0; c < C; ++c) x1[c] = x2[c] = x3[c] = 0.f;
-  if (t0 - 1 >= 0) load_n<IO, C>(xb + (size_t)(t0 - 1) * p.D, x1);
-  if (t0 - 2 >= 0) load_n<IO, C>(xb + (size_t)(t0 - 2) * p.D, x2);
-  if (t0 - 3 >= 0) load_n<IO, C>(xb + (size_t)(t0 - 3) * p.D, x3);
+  if (first - 1 >= 0) load_n<IO, C>(xb + (size_t)(first - 1) * p.D, x1);
+  if (first - 2 >= 0) load_n<IO, C>(xb + (size_t)(first - 2) * p.D, x2);
+  if (first - 3 >= 0) load_n<IO, C>(xb + (size_t)(first - 3) * p.D, x3);
+  for (int t0 = first; t0 < min(p.T, first + p.runs * kRun); t0 += kRun) {
 #pragma unroll
-  for (int r = 0; r < kRun; ++r) {
-    const int t = t0 + r;
-    const bool in = t < p.T;
-    float x0[C], o[C];
-    load_n<IO, C>(xb + (size_t)(in ? t : t0) * p.D, x0);  // clamped address: the loads of the run can all be in flight
+    for (int r = 0; r < kRun; ++r) {
+      const int t = t0 + r;
+      const bool in = t < p.T;
+      float x0[C], o[C];
+      load_n<IO, C>(xb + (size_t)(in ? t : t0) * p.D, x0);  // clamped address: the loads of the run can all be in flight
 #pragma unroll
-    for (int c = 0; c < C; ++c) o[c] = wk[0][c] * x0[c] + wk[1][c] * x1[c] + wk[2][c] * x2[c] + wk[3][c] * x3[c];
-    if (in) store_n<IO, C>(yb + (size_t)t * p.D, o);
+      for (int c = 0; c < C; ++c) o[c] = wk[0][c] * x0[c] + wk[1][c] * x1[c] + wk[2][c] * x2[c] + wk[3][c] * x3[c];
+      if (in) store_n<IO, C>(yb + (size_t)t * p.D, o);
 #pragma unroll
-    for (int c = 0; c < C; ++c) { x3[c] = x2[c]; x2[c] = x1[c]; x1[c] = x0[c]; }
+      for (int c = 0; c < C; ++c) { x3[c] = x2[c]; x2[c] = x1[c]; x1[c] = x0[c]; }
+    }
   }
 }
-// dx[t] = sum_k w[k] dy[t+k];  dw[d][k] partial = sum over this run of x[t-k] dy[t]  -> dwp[(b, run)][k][D]
+// dx[t] = sum_k w[k] dy[t+k];  dw[d][k] partial = sum over this lane's steps of x[t-k] dy[t]  -> dwp[(b, lane of steps)][k][D]
 template <typename IO>
-__global__ void __launch_bounds__(128) m3b_conv_bwd_kernel(BlkP p, const IO* __restrict__ x, const float* __restrict__ w,
+__global__ void __launch_bounds__(128, sizeof(IO) == 2 ? 6 : 4) m3b_conv_bwd_kernel(BlkP p, const IO* __restrict__ x, const float* __restrict__ w,
                                                            const IO* __restrict__ dy, IO* __restrict__ dx,
                                                            float* __restrict__ dwp) {
   begin_dependent();
-  constexpr int C = kConvC<IO>;
+  constexpr int C = kConvBwdC;
   const int cg = blockIdx.x * 128 + threadIdx.x, ch = cg * C;
   if (ch >= p.D) return;
-  const int t0 = blockIdx.y * kRun, b = blockIdx.z;
+  const int first = blockIdx.y * p.runs * kRun, b = blockIdx.z;
   float wk[kMaxK][C], dw[kMaxK][C];
+  conv_weights<C>(wk, w, p, ch);
 #pragma unroll
   for (int k = 0; k < kMaxK; ++k)
 #pragma unroll
-    for (int c = 0; c < C; ++c) { wk[k][c] = k < p.K ? w[(size_t)(ch + c) * p.K + k] : 0.f; dw[k][c] = 0.f; }
+    for (int c = 0; c < C; ++c) dw[k][c] = 0.f;
   const IO* __restrict__ xb = x + (size_t)b * p.T * p.D + ch;
   const IO* __restrict__ gb = dy + (size_t)b * p.T * p.D + ch;
   IO* __restrict__ ob = dx + (size_t)b * p.T * p.D + ch;
   float x1[C], x2[C], x3[C], g1[C], g2[C], g3[C];  // previous inputs; previous three dy
 #pragma unroll
   for (int c = 0; c < C; ++c) x1[c] = x2[c] = x3[c] = g1[c] = g2[c] = g3[c] = 0.f;
-  if (t0 - 1 >= 0) load_n<IO, C>(xb + (size_t)(t0 - 1) * p.D, x1);
-  if (t0 - 2 >= 0) load_n<IO, C>(xb + (size_t)(t0 - 2) * p.D, x2);
-  if (t0 - 3 >= 0) load_n<IO, C>(xb + (size_t)(t0 - 3) * p.D, x3);
-#pragma unroll
-  for (int r = 0; r < kRun + 3; ++r) {
-    const int t = t0 + r;
-    const bool in = t < p.T;
-    float x0[C], g0[C];
-    load_n<IO, C>(gb + (size_t)(in ? t : t0) * p.D, g0);  // clamped addresses, masked below
-    if (r < kRun) load_n<IO, C>(xb + (size_t)(in ? t : t0) * p.D, x0);
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      g0[c] = in ? g0[c] : 0.f;
-      x0[c] = (in && r < kRun) ? x0[c] : 0.f;
-    }
-    if (r < kRun) {
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        dw[0][c] = fmaf(x0[c], g0[c], dw[0][c]);
-        dw[1][c] = fmaf(x1[c], g0[c], dw[1][c]);
-        dw[2][c] = fmaf(x2[c], g0[c], dw[2][c]);
-        dw[3][c] = fmaf(x3[c], g0[c], dw[3][c]);
-      }
-    }
-    if (r >= 3 && t - 3 < p.T) {  // dx[t-3] = w0 dy[t-3] + w1 dy[t-2] + w2 dy[t-1] + w3 dy[t]
+  if (first - 1 >= 0) load_n<IO, C>(xb + (size_t)(first - 1) * p.D, x1);
+  if (first - 2 >= 0) load_n<IO, C>(xb + (size_t)(first - 2) * p.D, x2);
+  if (first - 3 >= 0) load_n<IO, C>(xb + (size_t)(first - 3) * p.D, x3);
+  auto emit = [&](int t, const float (&g0)[C]) {  // dx[t-3] = w0 dy[t-3] + w1 dy[t-2] + w2 dy[t-1] + w3 dy[t]
+    if (t - 3 >= first && t - 3 < p.T) {
       float o[C];
 #pragma unroll
       for (int c = 0; c < C; ++c) o[c] = wk[0][c] * g3[c] + wk[1][c] * g2[c] + wk[2][c] * g1[c] + wk[3][c] * g0[c];
       store_n<IO, C>(ob + (size_t)(t - 3) * p.D, o);
     }
 #pragma unroll
-    for (int c = 0; c < C; ++c) {
-      x3[c] = x2[c]; x2[c] = x1[c]; x1[c] = x0[c];
-      g3[c] = g2[c]; g2[c] = g1[c]; g1[c] = g0[c];
+    for (int c = 0; c < C; ++c) { g3[c] = g2[c]; g2[c] = g1[c]; g1[c] = g0[c]; }
+  };
+  auto loaded = [&](const IO* src, int t, float (&v)[C]) {  // clamped address, masked
+    load_n<IO, C>(src + (size_t)min(t, p.T - 1) * p.D, v);
+#pragma unroll
+    for (int c = 0; c < C; ++c) v[c] = t < p.T ? v[c] : 0.f;
+  };
+  int t0 = first;
+  for (; t0 < min(p.T, first + p.runs * kRun); t0 += kRun) {
+#pragma unroll
+    for (int r = 0; r < kRun; ++r) {
+      float x0[C], g0[C];
+      loaded(gb, t0 + r, g0);
+      loaded(xb, t0 + r, x0);
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        dw[0][c] = fmaf(x0[c], g0[c], dw[0][c]);
+        dw[1][c] = fmaf(x1[c], g0[c], dw[1][c]);
+        dw[2][c] = fmaf(x2[c], g0[c], dw[2][c]);
+        dw[3][c] = fmaf(x3[c], g0[c], dw[3][c]);
+        x3[c] = x2[c]; x2[c] = x1[c]; x1[c] = x0[c];
+      }
+      emit(t0 + r, g0);
     }
+  }
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {  // the three steps behind, for dx alone
+    float g0[C];
+    loaded(gb, t0 + r, g0);
+    emit(t0 + r, g0);
   }
   float* dst = dwp + ((size_t)(b * gridDim.y + blockIdx.y) * kMaxK) * p.D + ch;
 #pragma unroll
@@ -495,7 +523,17 @@ static BlkP make_m3b(const mxb_mamba3_desc* d, int K, float eps) {
 bool mamba3_block_supported(const mxb_mamba3_desc* d) {
   return d->D % 8 == 0 && d->D <= 2048 && d->N % 8 == 0 && d->N <= 128 && d->G > 0;
 }
-static int m3b_runs(const mxb_mamba3_desc* d) { return (d->T + m3b::kRun - 1) / m3b::kRun; }
+// Steps of a lane of the convolution, in units of kRun: up to four while that gives three CTAs an SM.
+static int m3b_run_units(const mxb_mamba3_desc* d) {
+  const int c = d->io_dtype == MXB_F32 ? m3b::kConvC<float> : m3b::kConvC<m3b::bf16>;
+  int u = 4;
+  while (u > 1 && (size_t)d->B * ((d->D / c + 127) / 128) * ((d->T + u * m3b::kRun - 1) / (u * m3b::kRun)) < 3 * 148) u /= 2;
+  return u;
+}
+static int m3b_runs(const mxb_mamba3_desc* d) {
+  const int steps = m3b::kRun * m3b_run_units(d);
+  return (d->T + steps - 1) / steps;
+}
 static int m3b_bc_lanes(const mxb_mamba3_desc* d) {
   int n = 2;
   while (8 * n < d->N) n *= 2;
@@ -534,7 +572,10 @@ template <typename IO>
 static mxb_status m3b_conv(const mxb_mamba3_desc* d, int K, const void* x, const float* w, void* y, const void* dy,
                            void* dx, float* dw, void* ws, cudaStream_t st) {
   BlkP p = make_m3b(d, K, 0.f);
-  const dim3 grid((d->D / m3b::kConvC<IO> + 127) / 128, m3b_runs(d), d->B);
+  p.runs = m3b_run_units(d);
+  p.wvec = K == 4 && reinterpret_cast<uintptr_t>(w) % 16 == 0;
+  const int c = dy ? m3b::kConvBwdC : m3b::kConvC<IO>;
+  const dim3 grid((d->D / c + 127) / 128, m3b_runs(d), d->B);
   if (!dy) {
     MXB_LAUNCH("m3b_conv_fwd_kernel", st,
                (launch_kernel(m3b::m3b_conv_fwd_kernel<IO>, grid, 128, 0, st, p, static_cast<const IO*>(x), w, static_cast<IO*>(y))));

@@ -357,3 +357,25 @@ def test_mamba3_states_and_output_in_one_kernel(T, G):
     for b in (0, B - 1):
         row = [t if n == "a_log" else t[b:b + 1].contiguous() for n, t in zip(names, args)]
         assert torch.equal(y[b:b + 1], ops.mamba3_selective_scan(*row, nheads=nheads))
+
+
+@pytest.mark.parametrize("io", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T", [1, 16, 63, 64, 67, 130])
+def test_block_conv_long_runs(T, io):
+    """Enough sequences that a lane takes 64 steps: runs that end inside, at and just behind the sequence; weights that can be read
+    four taps at a time and ones that cannot (three taps, or a base that is not 16-byte aligned)."""
+    from oracle import mamba3_block
+    B, D = 444, 8
+    g = torch.Generator().manual_seed(T)
+    x, dy = torch.randn(B, T, D, generator=g).to(io), torch.randn(B, T, D, generator=g).to(io)
+    flat = 0.4 * torch.randn(4 * D + 1, generator=g)
+    for K, first in ((4, 0), (4, 1), (3, 0)):
+        w = flat[first:first + K * D].view(D, K)
+        x64, w64 = x.double().requires_grad_(True), w.double().requires_grad_(True)
+        y = mamba3_block.depthwise_conv(x64, w64)
+        gx, gw = torch.autograd.grad((y * dy.double()).sum(), [x64, w64])
+        dw = flat.to("cuda")[first:first + K * D].view(D, K)
+        assert_close(ops.mamba3_block_conv(_dev(x), dw), y.detach(), TOL[io], f"y {K} {first}")
+        got = ops.mamba3_block_conv_backward(_dev(x), dw, _dev(dy))
+        assert_close(got["dx"], gx, TOL[io], f"dx {K} {first}")
+        assert_close(got["dw"], gw, TOL[io], f"dw {K} {first}")
