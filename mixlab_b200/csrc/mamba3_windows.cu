@@ -567,10 +567,12 @@ struct GradSmem {  // bytes per thread and per warp
 };
 // grid (D / channels of a CTA, windows, B).  What a step needs of its channel waits in shared memory, one read for all lanes (four
 // shuffles and the products of three scalars a step and pass before), and its results take the place; the decay is computed again
-// on the way back.  That makes room for three CTAs of seven warps an SM (two before): 4096 x 448 channels of 16 states 190 us ->
-// 161.
-template <typename IO, int PR, int LPC, bool PLAIN>
-__global__ void __maxnreg__(PR == 2 ? 96 : 168) m3w_grad_kernel(M3P p) {
+// on the way back.  Of 96 registers (no spills to speak of) a quarter of an SM holds five warps, of 80 six: the fewer where a CTA
+// more fits an SM for it (launch_grad).  4096 x 448 channels of 16 states, seven warps a CTA: 190 us, two CTAs an SM; 161 with two
+// CTAs still; 141 with three and 80 registers (76 bytes spilled).  2 x 1024 x 128 channels, four warps and five CTAs either way:
+// 26.9 with 96 registers, 28.8 with 80.
+template <typename IO, int PR, int LPC, bool PLAIN, int REGS>
+__global__ void __maxnreg__(REGS) m3w_grad_kernel(M3P p) {
   begin_dependent();
   using K = Walker<IO, PR, LPC, PLAIN>;
   constexpr int UN = K::UN, CPW = K::CPW, KEEP = 4 * PR / CPW > 0 ? 4 * PR / CPW : 1, NR = 2 * K::NP;
@@ -901,12 +903,21 @@ static mxb_status launch_local(const M3P& p, const M3WGrid& g, cudaStream_t st) 
 template <typename IO, int PR, int LPC, bool PLAIN>
 static mxb_status launch_grad(const M3P& p, const M3WGrid& g, cudaStream_t st) {
   constexpr int per_warp = 32 * GradSmem<PR, LPC>::kThread + GradSmem<PR, LPC>::kWarp, rows = kRowBytes<PR, LPC>;
-  if (MXB_ALLOW_SMEM((PR == 4 ? 4 : 8) * per_warp + rows, m3w_grad_kernel<IO, PR, LPC, PLAIN>) != MXB_OK) return MXB_ERR_CUDA;
   const int sm = g.shape.warps * per_warp + rows;
-  m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
-    MXB_LAUNCH("m3w_grad_kernel", st, (launch_kernel(m3w_grad_kernel<IO, PR, LPC, PLAIN>, grid, g.threads, sm, st, q)));
-  });
-  return MXB_OK;
+  auto launch = [&](auto regs) {
+    constexpr int REGS = decltype(regs)::value;
+    if (MXB_ALLOW_SMEM((PR == 4 ? 4 : 8) * per_warp + rows, m3w_grad_kernel<IO, PR, LPC, PLAIN, REGS>) != MXB_OK) return MXB_ERR_CUDA;
+    m3w_walk(p, g, [&](const M3P& q, dim3 grid) {
+      MXB_LAUNCH("m3w_grad_kernel", st, (launch_kernel(m3w_grad_kernel<IO, PR, LPC, PLAIN, REGS>, grid, g.threads, sm, st, q)));
+    });
+    return MXB_OK;
+  };
+  if constexpr (PR == 4) {
+    return launch(std::integral_constant<int, 168>{});
+  } else {
+    auto ctas = [&](int warps) { return std::min(warps / g.shape.warps, 228 * 1024 / (sm + 1024)); };  // of an SM that holds so many warps
+    return ctas(24) > ctas(20) ? launch(std::integral_constant<int, 80>{}) : launch(std::integral_constant<int, 96>{});
+  }
 }
 template <typename IO>
 static mxb_status prepare(const M3P& p, const M3WGrid& g, cudaStream_t st) {
