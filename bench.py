@@ -64,8 +64,8 @@ GDN_NCU_TRAFFIC_MB = {
 }
 GDN_NCU_TRAFFIC_UNITS = 8192     # (batch, head, chunk) units of the captured step
 M3_NCU_TRAFFIC_MB = {
-    "m3s_scalars_kernel": 15.8, "m3s_chunk_scalars_kernel": 17.5, "m3s_state_pass_kernel": 861.5,
-    "m3s_chunk_out_kernel": 615.5, "m3s_chunk_grad_kernel": 1077.5, "m3s_tail_kernel": 80.1,
+    "m3s_scalars_kernel": 15.1, "m3s_chunk_scalars_kernel": 16.1, "m3s_scan_out_kernel": 583.4,
+    "m3s_state_pass_kernel": 443.7, "m3s_chunk_grad_kernel": 1078.1, "m3s_tail_kernel": 80.0,
     "m3s_dalog_kernel": 0.0,
 }
 M3_NCU_TRAFFIC_UNITS = 16384
