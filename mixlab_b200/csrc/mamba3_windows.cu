@@ -15,10 +15,10 @@
 //
 // What bounds it: instruction issue (a sine, a cosine and two exponentials per state pair and pass).  So everything
 // that belongs to a (step, channel) is computed once and not by every lane and pass; the two states of a pair and two
-// pairs per lane go through packed arithmetic; a pass keeps sine, cosine and decay in shared memory for its reverse
-// half; rows of dB, dC are added over the channels of a warp by halving exchanges and over the warps once per window.
-// Scans run 16 segments of windows side by side.  2 x 1024 x 128 channels of 16 states, forward + backward:
-// 65 us a call; 4096 x 448 channels: 0.41 ms.
+// pairs per lane go through packed arithmetic; a pass keeps sine and cosine (the local walk the decay too) in shared memory
+// for its reverse half; rows of dB, dC are added over the channels of a warp by halving exchanges and over the warps once per
+// window.  Scans run 32 segments of windows side by side.  2 x 1024 x 128 channels of 16 states, forward + backward:
+// 65 us a call; 4096 x 448 channels: 0.37 ms.
 //
 // Every sum has a fixed order: the same inputs give the same bits.
 #include <algorithm>
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(256, 7) m3w_prepare_kernel(M3P p) {
 // 16 chains x 32 segments of PER windows per CTA: a segment is loaded once and folded, the folds of the earlier segments give
 // what enters it, and the registers are walked again to write (longer sequences in rounds of 32 PER windows).  Latency and, with
 // a decay, its exponentials bound it.  4096 x 448 channels of 16 states, us: one linear scan / both 20.5 / 51 with every value
-// loaded twice and two or three exponentials, 19.5 / 33 now.
+// loaded twice and two or three exponentials, 19.5 / 33 without, 15.6 a scan since two CTAs of 64 registers share an SM.
 //   kPhase  ck_phi: window sums -> wrapped angle at each window start, summed in 32-bit turns, which wrap by themselves and round
 //           nothing: the rounding of float sums, wrapped one by one, was a good part of the distance of every result from
 //           float64 (y 3.19e-7, dtheta 9.5e-7 over six
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kScanThreads) m3w_sums_kernel(M3P p, int scans
 }
 // blockIdx.z: 0 the states, 1 dh (first: the one to start with)
 template <int PER>
-__global__ void __launch_bounds__(kScanThreads) m3w_linear_scan_kernel(M3P p, int first) {
+__global__ void __launch_bounds__(kScanThreads, 2) m3w_linear_scan_kernel(M3P p, int first) {
   begin_dependent();
   if (first + (int)blockIdx.z == 0) scan_chain<kState, PER>(p, p.D * p.N, blockIdx.x, blockIdx.y);
   else scan_chain<kDh, PER>(p, p.D * p.N, blockIdx.x, blockIdx.y);
