@@ -292,11 +292,17 @@ __device__ __forceinline__ uint32_t turns(float x) {
   const float p = x * 683565248.f, e = fmaf(x, 27.5764316f, fmaf(x, 683565248.f, -p));
   return (uint32_t)__float2int_rn(p) + (uint32_t)__float2int_rn(e);
 }
+// The sum of angles: turns, and 0 or, once an angle was not finite, NaN: integers carry no NaN, and every later window has one.
+struct Angle {
+  uint32_t turns;
+  float bad;
+};
+__device__ __forceinline__ Angle operator+(Angle a, Angle b) { return {a.turns + b.turns, a.bad + b.bad}; }
 constexpr int kChains = 16, kSegs = 32, kScanThreads = kChains * kSegs;
 template <int MODE, int PER>
 __device__ __forceinline__ void scan_chain(const M3P& p, int chains, int block, int b) {
   constexpr bool linear = MODE == kState || MODE == kDh, back = MODE == kDh || MODE == kAngle;
-  using Sum = std::conditional_t<MODE == kPhase, uint32_t, float>;
+  using Sum = std::conditional_t<MODE == kPhase, Angle, float>;
   __shared__ Sum s_add[kSegs][kChains];
   __shared__ float s_dec[kSegs][kChains];
   const int lane = threadIdx.x % kChains, seg = threadIdx.x / kChains, i = block * kChains + lane;
@@ -306,18 +312,18 @@ __device__ __forceinline__ void scan_chain(const M3P& p, int chains, int block, 
   const float A = linear && in ? -expf(p.a_log[M3Idx(p).alog(d, i % p.N)]) : 0.f;
   auto win = [&](int x) { return (size_t)b * p.nW + (back ? p.nW - 1 - x : x); };  // x-th window in walking order
   auto value = [](float x) -> Sum {
-    if constexpr (MODE == kPhase) return turns(x);
+    if constexpr (MODE == kPhase) return {turns(x), 0.f * x};
     else return x;
   };
   auto result = [](Sum run) -> float {
-    if constexpr (MODE == kPhase) return (float)(int)run * 1.4629180792671596e-9f;  // 2 pi / 2^32
+    if constexpr (MODE == kPhase) return fmaf((float)(int)run.turns, 1.4629180792671596e-9f, run.bad);  // 2 pi / 2^32
     else return run;
   };
   auto fold = [](float dec, Sum run, Sum add) -> Sum {
     if constexpr (linear) return fmaf(dec, run, add);
     else return run + add;
   };
-  Sum carry = 0;
+  Sum carry{};
   for (int x0 = 0; x0 < p.nW; x0 += kSegs * PER) {
     const int lo = x0 + seg * PER;
     Sum loc[PER];
@@ -328,7 +334,7 @@ __device__ __forceinline__ void scan_chain(const M3P& p, int chains, int block, 
       loc[x] = value(ok ? buf[win(lo + x) * chains + i] : 0.f);
       dec[x] = ok && linear ? p.dtsum[win(lo + x) * p.D + d] : 0.f;
     }
-    Sum run = 0;
+    Sum run{};
     float dts = 0.f;
 #pragma unroll
     for (int x = 0; x < PER; ++x) {

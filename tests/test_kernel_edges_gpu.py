@@ -379,3 +379,18 @@ def test_block_conv_long_runs(T, io):
         got = ops.mamba3_block_conv_backward(_dev(x), dw, _dev(dy))
         assert_close(got["dx"], gx, TOL[io], f"dx {K} {first}")
         assert_close(got["dw"], gw, TOL[io], f"dw {K} {first}")
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("T,step", [(40, 3), (200, 77), (1300, 900)])
+def test_mamba3_windows_pass_on_angles_that_are_not_finite(T, step, bad):
+    """An angle that is not finite makes the same results NaN as in the serial walk: every later angle of its pair is NaN, in its own
+    window and in all that follow (one, some and all segments of the scan)."""
+    a = inputs.mamba3_inputs(1, T, 16, 1, 8, G=2, seed=71, per_head=False)
+    a["theta"][0, step, 5, 2] = bad
+    args = [_dev(a[n]) for n in ("x", "dt_raw", "lambda_raw", "theta", "a_log", "b", "c")]
+    got, want = ({"y": ops.mamba3_selective_scan(*args, flags=f), **ops.mamba3_selective_scan_backward(*args, _dev(a["dy"]), flags=f)}
+                 for f in (_lib.MXB_MAMBA3_WINDOW_PARALLEL, _lib.MXB_MAMBA3_SERIAL_WALK))
+    assert bool(torch.isnan(want["dx"][0, step:, 5]).all()) and not bool(torch.isnan(want["dx"][0, :, 4]).any())
+    for n in want:
+        assert torch.equal(torch.isnan(got[n]), torch.isnan(want[n])), n
