@@ -278,19 +278,20 @@ __global__ void __launch_bounds__(256, 7) m3w_prepare_kernel(M3P p) {
 // what enters it, and the registers are walked again to write (longer sequences in rounds of 32 PER windows).  Latency and, with
 // a decay, its exponentials bound it.  4096 x 448 channels of 16 states, us: one linear scan / both 20.5 / 51 with every value
 // loaded twice and two or three exponentials, 19.5 / 33 without, 15.6 a scan since two CTAs of 64 registers share an SM.
-//   kPhase  ck_phi: window sums -> wrapped angle at each window start, summed in 32-bit turns, which wrap by themselves and round
-//           nothing: the rounding of float sums, wrapped one by one, was a good part of the distance of every result from
+//   kPhase  ck_phi: window sums -> wrapped angle at each window start, summed in 32-bit turns: additions that wrap by themselves and
+//           do not round, of terms good to 1.5e-9.  The rounding of float sums, wrapped one by one, was a good part of the distance of every result from
 //           float64 (y 3.19e-7, dtheta 9.5e-7 over six
 //           problems of 257 to 1200 steps; 2.82e-7 and 7.9e-7 now)
 //   kState  ck_h: local end states -> state at each window start
 //   kDh     dhk: local dh -> dh entering each window from later steps
 //   kAngle  ang: window sums -> sum over all later windows
 enum { kPhase, kState, kDh, kAngle };
-// An angle in units of 2^-32 of a turn: the rounded product, and what its rounding left.
+// An angle in units of 2^-32 of a turn: the rounded product, and what its rounding left, each to the nearest integer (1.5e-9 of
+// angle together).  64 bits, of which the upper half are whole turns, hold window sums of up to 1.3e10, where a float no longer
+// knows its angle; one wrapped to 32 bits in float before is rounded by up to 1e-7, or cut off where it comes out above pi.
 __device__ __forceinline__ uint32_t turns(float x) {
-  x = m3_wrap(x);
   const float p = x * 683565248.f, e = fmaf(x, 27.5764316f, fmaf(x, 683565248.f, -p));
-  return (uint32_t)__float2int_rn(p) + (uint32_t)__float2int_rn(e);
+  return (uint32_t)__float2ll_rn(p) + (uint32_t)__float2ll_rn(e);
 }
 // The sum of angles: turns, and 0 or, once an angle was not finite, NaN: integers carry no NaN, and every later window has one.
 struct Angle {
@@ -365,7 +366,7 @@ __device__ __forceinline__ void scan_chain(const M3P& p, int chains, int block, 
   }
 }
 template <int PER>
-__global__ void __launch_bounds__(kScanThreads) m3w_phase_scan_kernel(M3P p) {
+__global__ void __launch_bounds__(kScanThreads, 2) m3w_phase_scan_kernel(M3P p) {
   begin_dependent();
   scan_chain<kPhase, PER>(p, p.D * p.Kp, blockIdx.x, blockIdx.y);
 }

@@ -394,3 +394,21 @@ def test_mamba3_windows_pass_on_angles_that_are_not_finite(T, step, bad):
     assert bool(torch.isnan(want["dx"][0, step:, 5]).all()) and not bool(torch.isnan(want["dx"][0, :, 4]).any())
     for n in want:
         assert torch.equal(torch.isnan(got[n]), torch.isnan(want[n])), n
+
+
+def test_mamba3_window_angles_around_odd_multiples_of_pi():
+    """The angle at a window start, read off as the sine by which the row of c has turned against the state (no decay, one input).
+    Bound: the sum back in float32 2.4e-7 (as a float, and its product with 2 pi / 2^32) and that constant 1e-7, the wrap of the first
+    step 2.4e-7, the sine 1.2e-7: 7e-7."""
+    pi = torch.tensor([k * torch.pi for k in range(1, 256, 2)], dtype=torch.float64).float()
+    above, below = torch.nextafter(pi, pi + 1), torch.nextafter(pi, pi - 1)
+    X = torch.cat([pi, above, below, torch.nextafter(above, above + 1)])
+    X = torch.cat([X, -X])
+    D, T = X.numel(), 9
+    x, theta = torch.zeros(1, T, D), torch.zeros(1, T, D, 1)
+    x[:, 0], theta[0, 1, :, 0] = 1, X / 32
+    dt, lam, a_log = torch.full((1, T, D), 32.0), torch.full((1, T, D), 60.0), torch.full((D, 2), -float("inf"))
+    b, c = torch.tensor([1.0, 0.0]).expand(1, T, 1, 2), torch.tensor([0.0, 1.0]).expand(1, T, 1, 2)
+    y = ops.mamba3_selective_scan(*map(_dev, (x, dt, lam, theta, a_log, b, c)), flags=_lib.MXB_MAMBA3_WINDOW_PARALLEL)
+    err = float((y[0, 8].cpu().double() / 32 - torch.sin(X.double())).abs().max())
+    assert err <= 7e-7, err
