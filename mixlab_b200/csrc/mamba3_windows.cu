@@ -90,18 +90,12 @@ __global__ void __launch_bounds__(256) m3w_sincos_kernel(const float* __restrict
   }
 }
 __device__ __forceinline__ f2 neg2(f2 v) { return v ^ 0x8000000080000000ull; }
-__device__ __forceinline__ float ex2(float x) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
+// exp(dt a) of two states.  (One ex2 of a product with rates in base 2 would save 1 to 11 % of a call and is less exact: rms distance
+// from float64 9.3e-8 for 6.8e-8 at exponents of 1 to 4, 3.5e-7 for 2.2e-7 at 4 to 16.)
+__device__ __forceinline__ f2 decay2(f2 a, f2 dt) {
+  const float2 x = unpack2(mul2(a, dt));
+  return pack2(expf(x.x), expf(x.y));
 }
-// exp(-r dt) of two states, r their decay rates times log2 e.  (expf spends instructions on a range that decays do not have; what
-// ex2 is further off, 2 % of the outputs' distance from float64, is less than the angles at the window starts have gained.)
-__device__ __forceinline__ f2 decay2(f2 r, f2 dt) {
-  const float2 x = unpack2(mul2(r, dt));
-  return pack2(ex2(-x.x), ex2(-x.y));
-}
-constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
 
 // One walker: the lanes of one channel in one window.  A lane owns PR state pairs kp = sl PR + r in units of two; a
 // packed value holds the same quantity of both pairs of a unit, even and odd states apart, so that the rotations are
@@ -216,12 +210,12 @@ struct Walker {
     if (act(2 * u)) { s[0] = x.x; s[1] = y.x; }
     if (act(2 * u + 1)) { s[2] = x.y; s[3] = y.y; }
   }
-  __device__ void rates(f2 (&A)[PR]) const {  // decay rates times log2 e; A[2 u]: even states of unit u, A[2 u + 1]: odd
+  __device__ void rates(f2 (&A)[PR]) const {  // decay rates; A[2 u]: even states of unit u, A[2 u + 1]: odd
 #pragma unroll
     for (int u = 0; u < UN; ++u) {
       float a[4];
 #pragma unroll
-      for (int x = 0; x < 4; ++x) a[x] = act(2 * u + x / 2) ? kLog2e * expf(p.a_log[ix.alog(d, 2 * (sl * PR + 2 * u) + x)]) : 0.f;
+      for (int x = 0; x < 4; ++x) a[x] = act(2 * u + x / 2) ? -expf(p.a_log[ix.alog(d, 2 * (sl * PR + 2 * u) + x)]) : 0.f;
       A[2 * u] = pack2(a[0], a[2]);
       A[2 * u + 1] = pack2(a[1], a[3]);
     }
@@ -279,9 +273,8 @@ __global__ void __launch_bounds__(256, 7) m3w_prepare_kernel(M3P p) {
 // a decay, its exponentials bound it.  4096 x 448 channels of 16 states, us: one linear scan / both 20.5 / 51 with every value
 // loaded twice and two or three exponentials, 19.5 / 33 without, 15.6 a scan since two CTAs of 64 registers share an SM.
 //   kPhase  ck_phi: window sums -> wrapped angle at each window start, summed in 32-bit turns: additions that wrap by themselves and
-//           do not round, of terms good to 1.5e-9.  The rounding of float sums, wrapped one by one, was a good part of the distance of every result from
-//           float64 (y 3.19e-7, dtheta 9.5e-7 over six
-//           problems of 257 to 1200 steps; 2.82e-7 and 7.9e-7 now)
+//           do not round, of terms good to 1.5e-9.  The rounding of float sums, wrapped one by one, was a good part of the
+//           distance of every result from float64 (900 steps: y 4.2e-7, dtheta 1.25e-6; 3.4e-7 and 9.8e-7 now)
 //   kState  ck_h: local end states -> state at each window start
 //   kDh     dhk: local dh -> dh entering each window from later steps
 //   kAngle  ang: window sums -> sum over all later windows
@@ -678,7 +671,7 @@ __global__ void __maxnreg__(REGS) m3w_grad_kernel(M3P p) {
     const float4 f = fin[at(s)];
     const float bf = fin5[at(s)];
     const f2 dt2 = dup2(f.x), gx = dup2(f.y), bx = dup2(f.z), dy2 = dup2(f.w);
-    f2 s_bu = 0ull, s_qv = 0ull, s_a = 0ull, s_w = 0ull, s_ca = 0ull;  // (s_w: times -log2 e)
+    f2 s_bu = 0ull, s_qv = 0ull, s_a = 0ull, s_w = 0ull, s_ca = 0ull;
     float rows[4 * PR];  // this lane's values of dB (first half) and dC of the step
 #pragma unroll
     for (int u = 0; u < UN; ++u) {
@@ -719,7 +712,7 @@ __global__ void __maxnreg__(REGS) m3w_grad_kernel(M3P p) {
       if (per_head) s_ca = add2(s_ca, carry[u]);
       else if (k.in(s)) k.put_two(p.dtheta + ((k.row0 + s) * p.D + k.d) * p.Kp, u, mul2(carry[u], dt2));
     }
-    s_a = mad2(dup2(-kLn2), s_w, s_a);
+    s_a = add2(s_a, s_w);
     const float v = sum_lanes4<LPC>(sum2(s_bu), sum2(s_qv), sum2(s_a), sum2(pend), k.sl);
     __syncwarp();
     if (k.sl < 4) reinterpret_cast<float*>(fin + at(s))[k.sl] = v;
@@ -738,9 +731,7 @@ __global__ void __maxnreg__(REGS) m3w_grad_kernel(M3P p) {
   }
 #pragma unroll
   for (int u = 0; u < UN; ++u) k.put_two(p.ang + k.wrow() * p.Kp, u, carry[u]);
-  // da_log: d/d a_log = d/dA * A  (A = -exp(a_log)); the closed form above already carries A (times -log2 e)
-#pragma unroll
-  for (int r = 0; r < PR; ++r) dal[r] = mul2(dup2(-kLn2), dal[r]);
+  // da_log: d/d a_log = d/dA * A  (A = -exp(a_log)); the closed form above already carries A
   if (per_head) {
     f2 sum = 0ull;
 #pragma unroll

@@ -412,3 +412,18 @@ def test_mamba3_window_angles_around_odd_multiples_of_pi():
     y = ops.mamba3_selective_scan(*map(_dev, (x, dt, lam, theta, a_log, b, c)), flags=_lib.MXB_MAMBA3_WINDOW_PARALLEL)
     err = float((y[0, 8].cpu().double() / 32 - torch.sin(X.double())).abs().max())
     assert err <= 7e-7, err
+
+
+def test_mamba3_window_decays_are_as_exact_as_expf():
+    """The decay of one step, read off as the state of a step that adds nothing (A = -1, so that dt is the exponent without rounding).
+    Bound: two units in the last place of float32, 2.4e-7."""
+    D = 1 << 14
+    x, theta, lam = torch.zeros(1, 2, D), torch.zeros(1, 2, D, 1), torch.full((1, 2, D), 60.0)
+    x[:, 0] = 1
+    dt = torch.full((1, 2, D), 32.0)          # softplus(dt) = dt above 20
+    dt[0, 1] = torch.linspace(20.5, 87, D)
+    b = torch.tensor([1.0, 0.0]).expand(1, 2, 1, 2)
+    y = ops.mamba3_selective_scan(*map(_dev, (x, dt, lam, theta, torch.zeros(D, 2), b, b)), flags=_lib.MXB_MAMBA3_WINDOW_PARALLEL)
+    want = 32 * torch.exp(-dt[0, 1].double())
+    err = float(((y[0, 1].cpu().double() - want) / want).abs().max())
+    assert err <= 2.4e-7, err
