@@ -340,12 +340,14 @@ __device__ __forceinline__ void scan_chain(const M3P& p, int chains, int block, 
     if (linear) s_dec[seg][lane] = expf(A * dts);
     __syncthreads();
     run = carry;
-    for (int s = 0; s < kSegs; ++s) {
-      if (s == seg) {
-        carry = run;
-        if (x0 + kSegs * PER >= p.nW) break;  // (the last round)
+    const bool last = x0 + kSegs * PER >= p.nW;
+    const int upto = last ? min(seg + 1, (p.nW - x0 + PER - 1) / PER) : kSegs;  // what comes behind enters no window
+    for (int s0 = 0; s0 < upto; s0 += 8) {  // (eight reads ahead of the chain; all 32 segments cost short sequences 1 us a scan)
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        if (s0 + x == seg) carry = run;
+        run = fold(linear ? s_dec[s0 + x][lane] : 0.f, run, s_add[s0 + x][lane]);
       }
-      run = fold(linear ? s_dec[s][lane] : 0.f, run, s_add[s][lane]);
     }
     const Sum through = run;
     run = carry;

@@ -7,6 +7,7 @@ import torch
 import mixlab_b200
 from mixlab_b200 import _lib, ops
 from oracle import gdn, inputs
+from oracle import mamba3 as oracle_mamba3
 from tests import test_gdn_block_gpu as blocks
 from tests import test_mamba3_gpu as mamba
 from tests.util import assert_close
@@ -427,3 +428,20 @@ def test_mamba3_window_decays_are_as_exact_as_expf():
     want = 32 * torch.exp(-dt[0, 1].double())
     err = float(((y[0, 1].cpu().double() - want) / want).abs().max())
     assert err <= 2.4e-7, err
+
+
+def _check_windows(B, T, D, N, G, io):
+    a = inputs.mamba3_inputs(B, T, D, 1, N, G=G, seed=73, io_dtype=io, per_head=False)
+    names = ("x", "dt_raw", "lambda_raw", "theta", "a_log", "b", "c")
+    args, kw = [_dev(a[n]) for n in names], dict(flags=_lib.MXB_MAMBA3_WINDOW_PARALLEL)
+    y_ref, want = oracle_mamba3.scan_vjp(*(a[n].double() for n in names), a["dy"].double())
+    assert_close(ops.mamba3_selective_scan(*args, **kw), y_ref, TOL[io], "y")
+    got = ops.mamba3_selective_scan_backward(*args, _dev(a["dy"]), **kw)
+    for n in want:
+        assert_close(got[n], want[n], TOL[io], n)
+
+
+@pytest.mark.parametrize("T", [1025, 1100, 2048])
+def test_mamba3_windows_eight_to_a_segment(T):
+    """Forward and reverse scans whose segments hold eight windows, the last segment whole, partly filled and the last of all."""
+    _check_windows(1, T, 16, 8, 2, F32)
