@@ -572,7 +572,8 @@ struct GradSmem {  // bytes per thread and per warp
 // grid (D / channels of a CTA, windows, B).  What a step needs of its channel waits in shared memory, one read for all lanes (four
 // shuffles and the products of three scalars a step and pass before), and its results take the place; the decay is computed again
 // on the way back.  Of 96 registers (no spills to speak of) a quarter of an SM holds five warps, of 80 six: the fewer where a CTA
-// more fits an SM for it (launch_grad).  4096 x 448 channels of 16 states, seven warps a CTA: 190 us, two CTAs an SM; 161 with two
+// more fits an SM for it and the grid takes a round of CTAs less (launch_grad; CTAs of seven warps alone; 256 x 448 channels with
+// 96 registers a call of 39.4 us, 40.4 with 80; 2048 x 448 171 and 164).  4096 x 448 channels of 16 states, seven warps a CTA: 190 us, two CTAs an SM; 161 with two
 // CTAs still; 141 with three and 80 registers (76 bytes spilled).  2 x 1024 x 128 channels, four warps and five CTAs either way:
 // 26.9 with 96 registers, 28.8 with 80.
 template <typename IO, int PR, int LPC, bool PLAIN, int REGS>
@@ -917,8 +918,15 @@ static mxb_status launch_grad(const M3P& p, const M3WGrid& g, cudaStream_t st) {
   if constexpr (PR == 4) {
     return launch(std::integral_constant<int, 255>{});  // (shared memory leaves one CTA of four warps an SM)
   } else {
-    auto ctas = [&](int warps) { return std::min(warps / g.shape.warps, 228 * 1024 / (sm + 1024)); };  // of an SM that holds so many warps
-    return ctas(24) > ctas(20) ? launch(std::integral_constant<int, 80>{}) : launch(std::integral_constant<int, 96>{});
+    if constexpr (LPC == 4) {  // (no other lane count has a number of warps for which it matters)
+      const size_t grid = (size_t)p.D / (g.shape.warps * 8) * p.nW * p.B;
+      auto rounds = [&](int warps) {  // of CTAs over the GPU, where an SM's registers hold so many warps
+        const size_t at_once = 148 * std::min(warps / g.shape.warps, 228 * 1024 / (sm + 1024));
+        return (grid + at_once - 1) / at_once;
+      };
+      if (rounds(24) < rounds(20)) return launch(std::integral_constant<int, 80>{});
+    }
+    return launch(std::integral_constant<int, 96>{});
   }
 }
 template <typename IO>

@@ -445,3 +445,11 @@ def _check_windows(B, T, D, N, G, io):
 def test_mamba3_windows_eight_to_a_segment(T):
     """Forward and reverse scans whose segments hold eight windows, the last segment whole, partly filled and the last of all."""
     _check_windows(1, T, 16, 8, 2, F32)
+
+
+@pytest.mark.parametrize("io", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N", [16, 14])
+def test_mamba3_windows_of_seven_warps(N, io):
+    """Groups of 112 channels make CTAs of seven warps, and 304 of them a gradient walk that fits the GPU at once with the fewer
+    registers; states that can be read two pairs at a time and ones that cannot."""
+    _check_windows(1, 300, 448, N, 4, io)
