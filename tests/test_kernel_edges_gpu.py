@@ -453,3 +453,20 @@ def test_mamba3_windows_of_seven_warps(N, io):
     """Groups of 112 channels make CTAs of seven warps, and 304 of them a gradient walk that fits the GPU at once with the fewer
     registers; states that can be read two pairs at a time and ones that cannot."""
     _check_windows(1, 300, 448, N, 4, io)
+
+
+@pytest.mark.parametrize("io", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,T,D", [(444, 67, 136), (444, 64, 136), (444, 130, 136), (444, 67, 72), (444, 16, 128), (740, 64, 32), (741, 64, 64), (444, 67, 64),
+                                   (1480, 33, 8), (16, 300, 24)])
+def test_block_conv_runs_of_narrow_rows(B, T, D, io):
+    """bf16 rows of up to sixteen lanes and the first wider ones, with 16, 32 and 64 steps a lane."""
+    from oracle import mamba3_block
+    g = torch.Generator().manual_seed(D)
+    x, dy, w = torch.randn(B, T, D, generator=g).to(io), torch.randn(B, T, D, generator=g).to(io), 0.4 * torch.randn(D, 4, generator=g)
+    x64, w64 = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    y = mamba3_block.depthwise_conv(x64, w64)
+    gx, gw = torch.autograd.grad((y * dy.double()).sum(), [x64, w64])
+    assert_close(ops.mamba3_block_conv(_dev(x), _dev(w)), y.detach(), TOL[io], "y")
+    got = ops.mamba3_block_conv_backward(_dev(x), _dev(w), _dev(dy))
+    assert_close(got["dx"], gx, TOL[io], "dx")
+    assert_close(got["dw"], gw, TOL[io], "dw")
