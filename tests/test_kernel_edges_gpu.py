@@ -470,3 +470,22 @@ def test_block_conv_runs_of_narrow_rows(B, T, D, io):
     got = ops.mamba3_block_conv_backward(_dev(x), _dev(w), _dev(dy))
     assert_close(got["dx"], gx, TOL[io], "dx")
     assert_close(got["dw"], gw, TOL[io], "dw")
+
+
+@pytest.mark.parametrize("B,NH,one", [(4, 37, False), (149, 1, True), (5, 32, True), (10, 30, True)])
+def test_mamba3_states_and_output_kernels_by_pairs(B, NH, one):
+    """Up to 148 (batch, head) pairs take a kernel for the states and one for the output, more take one for both (also in a second
+    round of CTAs, from 297 on); a single sequence of the same inputs gives the same bits through the two."""
+    a = inputs.mamba3_inputs(B, 130, NH, 64, 128, G=1, seed=62, io_dtype=BF16, per_head=True)
+    names = ("x", "dt_raw", "lambda_raw", "theta", "a_log", "b", "c")
+    args = [_dev(a[n]) for n in names]
+
+    def run(args):
+        n0 = mixlab_b200.lib().mxb_launch_count()
+        y = ops.mamba3_selective_scan(*args, nheads=NH)
+        return y, mixlab_b200.lib().mxb_launch_count() - n0
+
+    row = [t if n == "a_log" else t[B - 1:].contiguous() for n, t in zip(names, args)]
+    (y, launches), (y_row, launches_row) = run(args), run(row)
+    assert launches_row - launches == (1 if one else 0)
+    assert torch.equal(y[B - 1:], y_row)
