@@ -680,8 +680,9 @@ static int blk_tiles(const mxb_gdn_desc* d) {
   const int tile = blk::kPreRuns * blk_run(d);
   return (d->T + tile - 1) / tile;
 }
-// CTAs of the output stage: what is on the GPU at once (eight an SM forward, six backward), so that no second round of a few CTAs
-// follows (backward, 16 x 2048 x 16 heads of 64: 73 us with eight an SM asked for, 60 with six).
+// CTAs of the output stage: what is on the GPU at once (eight an SM forward, six backward: 61 to 64 and 76 to 78 registers in every
+// variant, 128 threads), so that no second round of a few CTAs follows (backward, 16 x 2048 x 16 heads of 64: 73 us with eight an SM
+// asked for, 60 with six).
 static int blk_post_ctas(const mxb_gdn_desc* d, bool bwd) {
   const size_t rows = (size_t)d->B * d->T * d->H, per = 128 / blk_lanes(d->Dv, 8);
   const size_t want = (rows + per - 1) / per, most = 148 * (bwd ? 6 : 8);
@@ -773,7 +774,6 @@ static void blk_colsum(blk::ColSums& c, cudaStream_t st) {
   if (col_sum_tall(columns)) launch(std::true_type{});
   else launch(std::false_type{});
 }
-
 
 template <typename IO>
 static mxb_status blk_pre_bwd(const mxb_gdn_desc* d, const void* qp, const void* kp, const void* vp, const float* cq,

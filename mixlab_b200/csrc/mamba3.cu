@@ -317,6 +317,8 @@ __global__ void __launch_bounds__(256) m3_bc_sum_kernel(M3P p) {
   begin_dependent();
   m3_bc_sum<IO>(p, blockIdx.x, gridDim.x);
 }
+
+// Head-broadcast layout: ddt, dlam, dtheta [B,T,NH] = the per-channel values of a head added in channel order.
 __global__ void __launch_bounds__(256) m3_head_sum_kernel(const float* __restrict__ hd, float* __restrict__ ddt,
                                                           float* __restrict__ dlam, float* __restrict__ dtheta,
                                                           size_t rows, int D, int NH) {

@@ -69,7 +69,9 @@ __device__ __forceinline__ float sigmoid_f(float x) { return __fdividef(1.f, 1.f
 // forward / backward 12.8 / 13.9 us with eight channels a thread (two loads of 16 bytes, 32 apart; 56 threads of a CTA at work), 8.3
 // / 11.7 with four.  In large ones the weights did: 32 loads a thread, each of 32 lines, for 19 of x (8 x 4096 x 2048 bf16, forward
 // / backward with the column sums 114 / 203 us); read tap by tap only where they must be, and for up to 64 steps: 65 / 187.  The
-// backward takes four channels of bf16 too, so that six CTAs fit an SM: 95.
+// backward takes four channels of bf16 too, so that six CTAs fit an SM (16 bytes spilled): 95.  Of float32 four CTAs of 128 registers
+// (96 bytes spilled); with the 241 that it would take, 8 x 4096 x 2048 165 -> 137 us, but 8 x 1024 x 256 8.0 -> 9.1 and 30000 x 5 x 8
+// 85 -> 179.
 template <typename IO>
 constexpr int kConvC = 16 / sizeof(IO);
 constexpr int kConvBwdC = 4;  // (the backward's weights, their gradients and six rows of eight channels do not fit a thread's registers)
@@ -315,7 +317,7 @@ __global__ void __launch_bounds__(kSumThreads<true>) m3b_bc_sum_kernel(BlkP p, B
 // ------------------------------------------------------------------ post: RMSNorm over D x SiLU gate
 // Rows of up to 512 channels: a warp per token row, 16 bytes of a row per lane and piece, no barrier.  (A CTA per row of 448 float32
 // channels had 56 of 256 threads at work and three barriers a row: 4096 rows forward / backward 11.2 / 17.4 us, 6.5 / 11.9
-// now.)
+// now.  The backward spills 56 bytes at two CTAs an SM; with one, 8 x 4096 rows of 512 bf16 channels take 46 us for 35.)
 constexpr int kWarpRow = 512;
 template <typename IO>
 struct WarpRow {
@@ -557,7 +559,8 @@ static int m3b_bc_ctas(const mxb_mamba3_desc* d) {
   const size_t per = 128 / m3b_bc_lanes(d), want = ((size_t)d->B * d->T + per - 1) / per;
   return (int)std::min<size_t>(want, 148 * 4);
 }
-// CTAs of the output stage: what is on the GPU at once.
+// CTAs of the output stage: what is on the GPU at once by the registers of the kernels (bf16 and float32: rows of a warp 70 and 73
+// forward, 128 backward; wider ones 48 and 47, 80 backward; 256 threads).
 static int m3b_post_ctas(const mxb_mamba3_desc* d, bool bwd) {
   const size_t rows = (size_t)d->B * d->T;
   if (d->D <= m3b::kWarpRow) return (int)std::min<size_t>((rows + 7) / 8, 148 * (bwd ? 2 : 3));

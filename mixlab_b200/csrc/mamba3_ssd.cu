@@ -694,8 +694,9 @@ __global__ void __launch_bounds__(128, 4) m3s_chunk_out_kernel(SsdP p, const __g
 // is counted per stage stays within two chunks, and of every other barrier the next phase needs its waiters to have passed.
 // G*M takes the place of Brot, y that of x.
 // TMEM: the state's contribution [0, 64) and [64, 128) by turns, G [128, 160), Crot H0 [160, 192), (G*M) X [192, 224).
-// Bound by instruction issue (50 % of the slots; rotation, masks and the state's update), with 69 + 16 KB a chunk through shared
-// memory beside it: 8 x 4096 x 32 heads 222 us where the two kernels take 102 + 184 (without keeping the states 200).
+// No unit is at its limit (5 x 2048 x 32 heads: 25 % of the issue slots, shared memory 29 %, tensor pipe 8 %, DRAM 14 %): what takes
+// the time is the chain of hand-overs of a chunk (rotation, product, state; G, mask, product, y) with two CTAs an SM to fill it.
+// 8 x 4096 x 32 heads 222 us where the two kernels take 102 + 184 (without keeping the states 200).
 constexpr int kScanThreads = 512;
 constexpr int kScanStage = 2 * 16384 + 8192;
 constexpr int kScanSmem = 2 * kScanStage + 8192 + 16384 + 2 * (int)sizeof(ChunkScal) + 21 * 8 + 16 + 1024;
@@ -1639,9 +1640,12 @@ static mxb_status ssd_state_pass(SsdP& p, int mode, cudaStream_t st) {
 }
 
 // States and output by one kernel where the CTAs of the state pass would share SMs; false where a tensor map cannot be made.  Of
-// fewer (batch, head) pairs the chain of chunks is what counts, and the output kernel spreads over all SMs.  Forward, us, two
-// kernels / one: 1 x 4096 x 32 heads 76 / 140, 4 x 4096 x 32 147 / 164, 5 x 2000 x 32 114 / 115 (108 without keeping the states),
-// 6 x 2000 x 32 126 / 119, 8 x 1024 x 32 81 / 68, 8 x 4096 x 32 286 / 238 (215).  The bits are the same.
+// fewer (batch, head) pairs the chain of chunks is what counts, and the output kernel spreads over all SMs.  A forward with its
+// scalars, us, two kernels / one that keeps the states / one that does not: 1 x 4096 x 32 heads 74 / 136 / 125, 4 x 4096 x 32 145 / 163
+// / 158, 4 x 1024 x 37 47.7 / 51.2 / 51.3, 149 x 512 x 1 36.3 / 33.6 / 32.5, 5 x 512 x 30 34.6 / 32.3 / 31.5, 5 x 4096 x 32 213 / 220 /
+// 204 (long sequences that keep their states lose a little at 160 pairs and gain at 192), 6 x 4096 x 32 237 / 225 / 209, 8 x 4096 x 32 284 / 235 / 213;
+// in a second round of CTAs 9 x 4096 x 33 368 / 355 / 324, 10 x 2048 x 32 196 / 185 / 187, 16 x 2048 x 32 285 / 233 / 211.  The bits
+// are the same.
 static bool ssd_scan_maps(const SsdP& p, m3s::ScanMaps& maps) {
   std::memset(&maps, 0, sizeof maps);
   return !p.no_tma && make_tma_map_bthd(&maps.b, p.b, p.B, p.T, p.G, m3s::N) && make_tma_map_bthd(&maps.c, p.c, p.B, p.T, p.G, m3s::N) &&

@@ -18,7 +18,7 @@
 // pairs per lane go through packed arithmetic; a pass keeps sine and cosine (the local walk the decay too) in shared memory
 // for its reverse half; rows of dB, dC are added over the channels of a warp by halving exchanges and over the warps once per
 // window.  Scans run 32 segments of windows side by side.  2 x 1024 x 128 channels of 16 states, forward + backward:
-// 65 us a call; 4096 x 448 channels: 0.37 ms.
+// 71 us a call; 4096 x 448 channels: 140 us forward, 313 a backward with its recompute.
 //
 // Every sum has a fixed order: the same inputs give the same bits.
 #include <algorithm>
@@ -573,9 +573,9 @@ struct GradSmem {  // bytes per thread and per warp
 // shuffles and the products of three scalars a step and pass before), and its results take the place; the decay is computed again
 // on the way back.  Of 96 registers (no spills to speak of) a quarter of an SM holds five warps, of 80 six: the fewer where a CTA
 // more fits an SM for it and the grid takes a round of CTAs less (launch_grad; CTAs of seven warps alone; 256 x 448 channels with
-// 96 registers a call of 39.4 us, 40.4 with 80; 2048 x 448 171 and 164).  4096 x 448 channels of 16 states, seven warps a CTA: 190 us, two CTAs an SM; 161 with two
-// CTAs still; 141 with three and 80 registers (76 bytes spilled).  2 x 1024 x 128 channels, four warps and five CTAs either way:
-// 26.9 with 96 registers, 28.8 with 80.
+// 96 registers a call of 39.4 us, 40.4 with 80; 2048 x 448 171 and 164).  4096 x 448 channels of 16 states, seven warps a CTA: 170 us with two CTAs an SM and 96
+// registers, 154 with three and 80 (76 bytes spilled).  2 x 1024 x 128 channels, four warps and five CTAs either way: 29.2 with 96
+// registers, 30.8 with 80.
 template <typename IO, int PR, int LPC, bool PLAIN, int REGS>
 __global__ void __maxnreg__(REGS) m3w_grad_kernel(M3P p) {
   begin_dependent();
