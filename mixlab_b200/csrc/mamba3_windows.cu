@@ -234,10 +234,12 @@ template <int PR, int LPC>
 constexpr int kRowBytes = (2 * W + 1) * 2 * PR * LPC * 4;
 
 // ------------------------------------------------------------------ prepare
-// Seven CTAs an SM where rows are read two pairs at a time (32 registers, 24 bytes spilled; 4096 x 448 channels 2 us less than with
-// 56).  Without that the loads in flight want the registers: N 30, 512 steps of 64 channels 0.3 us less, N 256 0.5 to 1.2 us.
+// CTAs an SM: seven (32 registers) of four lanes a channel, or where rows are read two pairs at a time (4096 x 448 channels 2 us less
+// than with 56 registers, 65 x 64 channels of 6 states 0.7); five (48 registers) of more lanes (18 to 128 states, against 32 registers
+// and against no bound: up to 4 % of a forward); no bound with four pairs a lane, whose CTAs have at most
+// 128 threads (256 states, 512 steps of 256 channels 248 us, 252 with 32 registers and 156 bytes spilled).
 template <typename IO, int PR, int LPC, bool PLAIN>
-__global__ void __launch_bounds__(256, PLAIN ? 7 : 1) m3w_prepare_kernel(M3P p) {
+__global__ void __launch_bounds__(256, LPC == 4 || PLAIN ? 7 : PR == 4 ? 1 : 5) m3w_prepare_kernel(M3P p) {
   begin_dependent();
   using K = Walker<IO, PR, LPC, PLAIN>;
   const K k(p, nullptr);
